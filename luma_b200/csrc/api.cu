@@ -6,6 +6,7 @@
 //   luma-flash-attn/kernels/flash_attn_func.cu:267-304
 //   luma-flash-attn/kernels/flash_attn_varlen_func.cu:243-304
 //   luma-flash-attn/kernels/flash_attn_with_kvcache.cu:313-386
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstring>
@@ -76,8 +77,8 @@ namespace {
 struct WsEntry {
     int dev = -1;
     cudaStream_t stream = nullptr;
-    void* ptr = nullptr;
-    size_t bytes = 0;
+    void* ptr = nullptr;          // the counters, then the partials
+    size_t bytes = 0, counters = 0;
     unsigned long long last_use = 0;
 };
 constexpr size_t kMaxWorkspaces = 32;
@@ -97,11 +98,11 @@ void release_entry(WsEntry& e) {
     }
     if (cur != e.dev && cur >= 0) cudaSetDevice(cur);
     e.ptr = nullptr;
-    e.bytes = 0;
+    e.bytes = e.counters = 0;
 }
 }  // namespace
 
-void* decode_workspace(cudaStream_t stream, size_t bytes) {
+void* decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_bytes, unsigned** counters) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
     std::lock_guard<std::mutex> lock(g_ws_mutex);
@@ -122,22 +123,31 @@ void* decode_workspace(cudaStream_t stream, size_t bytes) {
         e->stream = stream;
     }
     e->last_use = ++g_ws_clock;
-    if (e->bytes >= bytes && e->ptr != nullptr) return e->ptr;
-    release_entry(*e);   // ordered after the work that still reads the old buffer
-    size_t want = bytes + bytes / 4;
-    if (want < (size_t(1) << 20)) want = size_t(1) << 20;
-    void* ptr = nullptr;
-    if (cudaMallocAsync(&ptr, want, stream) != cudaSuccess) {
-        cudaGetLastError();
-        want = bytes;
+    if (e->ptr == nullptr || e->bytes < e->counters + bytes || e->counters < counter_bytes) {
+        const size_t want_counters = std::max({(counter_bytes + 4095) / 4096 * 4096, e->counters, size_t(1) << 16});
+        const size_t old = e->bytes > e->counters ? e->bytes - e->counters : 0;
+        release_entry(*e);   // ordered after the work that still reads the old buffer
+        size_t want = want_counters + std::max({bytes + bytes / 4, old, size_t(1) << 20});
+        void* ptr = nullptr;
         if (cudaMallocAsync(&ptr, want, stream) != cudaSuccess) {
             cudaGetLastError();
+            want = want_counters + bytes;
+            if (cudaMallocAsync(&ptr, want, stream) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+        }
+        e->ptr = ptr;
+        e->bytes = want;
+        e->counters = want_counters;
+        if (cudaMemsetAsync(ptr, 0, want_counters, stream) != cudaSuccess) {   // once: every launch leaves them at zero again
+            cudaGetLastError();
+            release_entry(*e);
             return nullptr;
         }
     }
-    e->ptr = ptr;
-    e->bytes = want;
-    return ptr;
+    *counters = static_cast<unsigned*>(e->ptr);
+    return static_cast<unsigned char*>(e->ptr) + e->counters;
 }
 
 int release_workspaces() {

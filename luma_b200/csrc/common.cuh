@@ -154,6 +154,12 @@ int check_launch(const char* what);
 // family supports (the dispatcher then tries the next one).
 int launch_tile_simt(const AttnParams& p, cudaStream_t stream);
 int launch_decode_splitk(const AttnParams& p, cudaStream_t stream);
+// The same kernel for a few query rows per sequence through any entry point.
+int launch_few_rows(const AttnParams& p, cudaStream_t stream);
+// The same kernel for those sequences of a packed batch that have few query rows (the host does not know which):
+// launched beside the prefill kernel, which leaves out sequences of at most the returned number of rows (query tokens x
+// group); 0 = nothing was launched.
+int launch_mixed_few_rows(const AttnParams& p, cudaStream_t stream);
 int launch_prefill_tcgen05(const AttnParams& p, cudaStream_t stream);
 int launch_debug_block_slots(const int* block_tables, const int* context_lens, const int* offsets,
                              int num_seqs, int block_size, int max_blocks, int* out_slots,
@@ -172,8 +178,9 @@ int prefill_device_status();
 // to host memory; returns the bytes copied or -1.
 int prefill_debug_read(void* dst, int bytes);
 
-// Split-K scratch of the decode path: one buffer per (device, stream), grown on demand.
-void* decode_workspace(cudaStream_t stream, size_t bytes);
+// Split-K scratch of the decode path: one buffer per (device, stream), grown on demand. `counters`: at
+// least counter_bytes that are zero at the first use and that every launch leaves at zero.
+void* decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_bytes, unsigned** counters);
 // Releases every workspace (stream-ordered); returns how many buffers were held.
 int release_workspaces();
 

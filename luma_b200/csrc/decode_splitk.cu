@@ -1,21 +1,30 @@
-// Paged-KV single-token decode for f16/bf16 storage, head_size 32, 64 or 128.
+// Attention of a few query rows per sequence over a long K/V range, f16/bf16 storage, head_size 32, 64 or 128:
+// single-token decode over the paged cache above all, and also a handful of speculated tokens, decoding over
+// contiguous K/V, and the decoding sequences of a packed mixed batch.
 //
 // Replaces flash_attn_decode_kernel (luma-flash-attn/kernels/flash_attn_with_kvcache.cu:22-116;
 // launch :123-145), which walks the context one token at a time with one warp per query head and
 // re-reads K/V once per query head of a GQA group.
 //
 // Here the path is HBM-bound by construction:
-//   * work item = (chunk of the context, KV head, sequence); a CTA reads each K/V row of its chunk
-//     exactly once and serves every query head of the GQA group from it;
+//   * the query rows that share a KV head (every head of the GQA group x every query token) are the rows of
+//     one tensor-core tile: a CTA reads each K/V row once and serves all of them, 16 rows at a time;
+//   * the K/V ranges of all sequences are laid end to end in units of 64 tokens and cut into equal
+//     shares, one per CTA slot of the device ("columns"; every KV head has its own CTA per column): all CTAs do
+//     the same number of units whatever the lengths are, and each reads its share through one copy pipeline
+//     that runs on across the sequence boundaries. The host knows only the width of the block table, so the
+//     cut is made on the device, by every warp for itself, from the lengths;
 //   * rows are gathered through the block table with 16-byte cp.async copies into a per-warp ring
 //     of shared-memory stages (3 tiles of 16 tokens in flight per warp, 2 CTAs per SM), no
-//     CTA-wide barrier inside the loop;
-//   * Q.K^T and P.V run on tensor cores (mma.sync m16n8k16, f32 accumulate) with the group's
-//     query heads as the 16-row M dimension — at 8 query heads per KV head scalar FMA could not
-//     keep up with the memory system;
-//   * split-K over the context: every chunk writes an unnormalised f32 partial (acc, m, l) to a
-//     workspace and a second kernel merges the chunks of a sequence with log-sum-exp weights.
-// Token -> slot arithmetic is block_slot() from common.cuh (reference: kernels/common.cuh:89-108).
+//     CTA-wide barrier inside a sequence;
+//   * Q.K^T and P.V run on tensor cores (mma.sync m16n8k16, f32 accumulate) — at 8 query heads per KV
+//     head scalar FMA could not keep up with the memory system;
+//   * a sequence that lies inside one column is finished there; one that is cut leaves unnormalised f32
+//     partials (acc, m, l) in a workspace, and the CTA that finishes its part last merges them, always in
+//     column order, with log-sum-exp weights.
+// Token -> slot arithmetic is that of block_slot() in common.cuh (reference: kernels/common.cuh:89-108).
+#include <algorithm>
+#include <atomic>
 #include <mutex>
 
 #include "common.cuh"
@@ -27,22 +36,37 @@ namespace {
 constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
 constexpr int kTile = 16;    // tokens per tile (one mma K step for P.V, two N blocks for Q.K^T)
+constexpr int kUnit = kWarps * kTile;   // tokens that the CTA's warps take at a time, the unit of the cut
 constexpr int kStages = 3;   // tiles in flight per warp
-constexpr int kMaxHeads = 16;  // query heads served per CTA (M of the mma)
+constexpr int kRows = 16;    // query rows served per CTA (M of the mma)
 
-struct DecodeArgs {
+// Where the finished rows go: one buffer of (rows, o_heads, D), or — head-sharded decode with
+// the output all-gather fused in — the same tensor on every GPU of the group (peer memory, plain
+// stores over NVLink), each receiving this call's heads at head offset o_head0.
+struct RowsOut {
+    void* o[8];
+    int n_out, o_heads, o_head0, peer0;
+    float* lse;      // MODE_BATCH: (num_seqs, q_heads, q_seq_len) or null
+};
+
+struct RowsArgs {
     const void* q;
     const void* k;
     const void* v;
     const int* block_tables;
-    const int* context_lens;
-    float* ws_acc;   // (num_seqs, q_heads, max_splits, D) f32, unnormalised
-    float2* ws_ml;   // (num_seqs, q_heads, max_splits) {m (log2 domain), l}
-    int num_seqs, q_heads, kv_heads, block_size, max_blocks;
-    int chunk;       // tokens per work item, multiple of kWarps * kTile
-    int max_splits;
-    int head_blocks; // ceil(group / kMaxHeads)
-    float scale_log2;  // scale * log2(e)
+    const int* context_lens;   // MODE_KVCACHE
+    const int* cu_q;           // MODE_VARLEN
+    const int* cu_k;           // MODE_VARLEN
+    float* ws_acc;       // (2 * CTAs, kRows, D) f32, unnormalised; slot 0 of a CTA: the sequence that began in an earlier column, slot 1: the one that goes on in the next
+    float2* ws_ml;       // (2 * CTAs, kRows) {m (log2 domain), l}
+    unsigned* arrived;   // (gridDim.x, num_seqs) parts of a cut sequence that are in the workspace; zero between calls
+    int mode, num_seqs, q_seq_len, kv_seq_len, start_pos;
+    int q_heads, kv_heads, block_size, block_shift, max_blocks, paged;   // block_shift: log2 of the page size, -1 where it is no power of two
+    int row_blocks;      // blocks of kRows query rows per KV head (blockIdx.x = KV head x row block)
+    int max_rows;        // sequences with more query rows than this (per KV head) are not this launch's
+    int forced_units;    // > 0: units per column (option "decode_chunk_tokens"); 0: equal shares
+    float scale_log2;    // scale * log2(e)
+    RowsOut out;
 };
 
 __device__ __forceinline__ void cp_async_16(void* smem, const void* gmem, bool valid) {
@@ -115,7 +139,8 @@ __device__ __forceinline__ float fast_exp2(float x) {
 //   ring : kWarps x kStages x {K tile, V tile}, each tile kTile rows of D elements, 16-byte chunks
 //          XOR-swizzled by the row (row & 7; row & 3 at head_size 32, whose rows hold only four chunks) against
 //          ldmatrix bank conflicts
-//   after the loop the same bytes hold the per-warp partials for the cross-warp merge.
+//   merge: the warps' partials of a finished sequence, kMergeCols columns at a time — beside the ring, which
+//          already holds tiles of the next sequence by then
 template <int D>
 struct Smem {
     static constexpr int kRowBytes = D * 2;
@@ -124,12 +149,184 @@ struct Smem {
     static constexpr int kStageBytes = 2 * kTileBytes;
     static constexpr int kWarpBytes = kStages * kStageBytes;
     static constexpr int kRingBytes = kWarps * kWarpBytes;
-    static constexpr int kMergeBytes = kWarps * kMaxHeads * (D + 2) * 4;
-    static constexpr int kBytes = kRingBytes > kMergeBytes ? kRingBytes : kMergeBytes;
+    static constexpr int kMergeCols = D < 64 ? D : 64;
+    static constexpr int kMergePitch = kMergeCols + 2;   // the row's m and l in the last two
+    static constexpr int kMergeBytes = kWarps * kRows * kMergePitch * 4;
+    static constexpr int kBytes = kRingBytes + kMergeBytes + 16;
+    // CTAs per SM by shared memory (228 KiB, 1 KiB of it reserved per CTA) and registers
+    static constexpr int kCtasPerSm = D == 128 ? 2 : (D == 64 ? 3 : 4);
 };
 
+// Extents of one sequence: its query rows and the keys it sees. Query token i sits at global position
+// pos_off + i and sees keys j < kv_len with j <= pos_off + i.
+struct RowsSeq {
+    int q_len, kv_len, pos_off;
+    long long q_row0, kv_row0;
+};
+
+__device__ __forceinline__ RowsSeq rows_seq(const RowsArgs& a, int s) {
+    RowsSeq r;
+    if (a.mode == MODE_KVCACHE) {
+        r.q_len = a.q_seq_len;
+        r.kv_len = a.context_lens[s];
+        r.pos_off = r.kv_len - r.q_len;
+        r.q_row0 = (long long)s * a.q_seq_len;
+        r.kv_row0 = 0;
+    } else if (a.mode == MODE_BATCH) {
+        r.q_len = a.q_seq_len;
+        r.kv_len = a.kv_seq_len;
+        r.pos_off = a.start_pos;
+        r.q_row0 = (long long)s * a.q_seq_len;
+        r.kv_row0 = (long long)s * a.kv_seq_len;
+    } else {
+        const int q0 = a.cu_q[s], k0 = a.cu_k[s];
+        r.q_len = a.cu_q[s + 1] - q0;
+        r.kv_len = a.cu_k[s + 1] - k0;
+        r.pos_off = r.kv_len - r.q_len;
+        r.q_row0 = q0;
+        r.kv_row0 = k0;
+    }
+    return r;
+}
+
+// Keys that the last query token sees.
+__device__ __forceinline__ int rows_visible(const RowsSeq& r) {
+    const long long v = min((long long)r.kv_len, (long long)r.pos_off + r.q_len);
+    return v > 0 ? (int)v : 0;
+}
+
+// Units of the sequence for the row block that starts at query row `row0`; 0: nothing to do there. A sequence
+// whose rows see no key has one unit all the same: somebody has to write its zeros.
+__device__ __forceinline__ int rows_units(const RowsArgs& a, const RowsSeq& r, int group, int row0) {
+    const int rows = r.q_len * group;
+    if (rows <= row0 || rows > a.max_rows) return 0;
+    return max(1, (rows_visible(r) + kUnit - 1) / kUnit);
+}
+
+// The cut of `total` units into columns: the first `more` columns have share + 1 units, the others share
+// (or, forced, every column `share` units). All in 32 bits: a 64-bit division here cost a microsecond of a small call.
+struct Cut {
+    unsigned share, more;
+    __device__ __forceinline__ Cut(unsigned total, unsigned columns, unsigned forced) {
+        share = forced > 0 ? forced : total / columns;
+        more = forced > 0 ? 0u : total - share * columns;
+    }
+    __device__ __forceinline__ unsigned first(unsigned c) const { return share * c + min(c, more); }
+    __device__ __forceinline__ unsigned column_of(unsigned unit) const {
+        const unsigned split = more * (share + 1u);
+        return unit < split ? unit / (share + 1u) : more + (unit - split) / share;
+    }
+};
+
+// One arrival: everything the CTA's threads wrote before their last barrier is visible to whoever sees the count
+// (release), and what earlier arrivals published is visible to this CTA after its next barrier (acquire).
+__device__ __forceinline__ unsigned arrive_acq_rel(unsigned* count) {
+    unsigned before;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;\n" : "=r"(before) : "l"(count) : "memory");
+    return before;
+}
+
+// Two finished neighbours of an output row, to every output buffer.
+template <typename T>
+__device__ __forceinline__ void store_pair(const RowsOut& out, long long row, int head, int D, int d, unsigned both) {
+    const long long off = (row * out.o_heads + out.o_head0 + head) * D + d;
+    int pe = out.peer0;
+    for (int n = 0; n < out.n_out; ++n) {
+        *reinterpret_cast<unsigned*>(static_cast<T*>(out.o[pe]) + off) = both;
+        pe = pe + 1 == out.n_out ? 0 : pe + 1;
+    }
+}
+
+// Merges the parts of a cut sequence: warp w takes rows w, w + 4, ..., RW of them, a lane D / 32 neighbouring
+// elements of each. The CTA runs alone at the end of its column here, so what counts is the number of dependent
+// trips to L2 (about 0.8 us each): one for every part's (m, l), then 16 rows of partials in flight per lane.
+// 22 parts of 8 rows: 10 us with one row and 8 partials at a time, 3 us so.
+template <int D, int RW, typename Finish>
+__device__ __forceinline__ void merge_parts(const float* acc0, const float2* ml0, float* scratch, int nrows, int c_first, int parts,
+                                            unsigned grid_x, int warp, int lane, const Finish& finish) {
+    constexpr int E = D / 32;
+    constexpr int kAtOnce = 16 / RW;      // parts in flight per row
+    constexpr int kChunk = 64;            // parts whose weights sit in shared memory at a time
+    static_assert(kRows * kChunk * 4 <= Smem<D>::kMergeBytes, "weights of a chunk fit the merge buffer");
+    auto slot_of = [&](int c) { return (long long)c * grid_x * 2 + (c == c_first ? 1 : 0); };
+    float o[RW][E], m[RW], l[RW];
+#pragma unroll
+    for (int k = 0; k < RW; ++k) {
+        m[k] = -INFINITY;
+        l[k] = 0.0f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) o[k][e] = 0.0f;
+    }
+    for (int p0 = 0; p0 < parts; p0 += kChunk) {
+        const int n = min(kChunk, parts - p0);
+#pragma unroll
+        for (int k = 0; k < RW; ++k) {
+            const int r = warp + k * kWarps;
+            float2 x[2] = {make_float2(-INFINITY, 0.0f), make_float2(-INFINITY, 0.0f)};
+            if (r < nrows) {
+                if (lane < n) x[0] = __ldcg(&ml0[slot_of(c_first + p0 + lane) * kRows + r]);
+                if (lane + 32 < n) x[1] = __ldcg(&ml0[slot_of(c_first + p0 + 32 + lane) * kRows + r]);
+            }
+            float mx = fmaxf(x[0].x, x[1].x);
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+            mx = fmaxf(mx, m[k]);
+            const float before = m[k] == -INFINITY ? 0.0f : fast_exp2(m[k] - mx);
+            m[k] = mx;
+            l[k] *= before;
+#pragma unroll
+            for (int e = 0; e < E; ++e) o[k][e] *= before;
+            const float w0 = x[0].x == -INFINITY ? 0.0f : fast_exp2(x[0].x - mx);
+            const float w1 = x[1].x == -INFINITY ? 0.0f : fast_exp2(x[1].x - mx);
+            scratch[(k * kWarps + warp) * kChunk + lane] = w0;
+            scratch[(k * kWarps + warp) * kChunk + 32 + lane] = w1;
+            l[k] += w0 * x[0].y + w1 * x[1].y;   // this lane's share
+        }
+        __syncwarp();
+        for (int i0 = 0; i0 < n; i0 += kAtOnce) {
+            float x[RW][kAtOnce][E];
+#pragma unroll
+            for (int k = 0; k < RW; ++k) {
+                const int r = warp + k * kWarps;
+#pragma unroll
+                for (int i = 0; i < kAtOnce; ++i) {
+#pragma unroll
+                    for (int e = 0; e < E; ++e) x[k][i][e] = 0.0f;
+                    if (r < nrows && i0 + i < n) {
+                        const float* src = acc0 + (slot_of(c_first + p0 + i0 + i) * kRows + r) * D + lane * E;
+                        if constexpr (E == 4) {
+                            const float4 y = __ldcg(reinterpret_cast<const float4*>(src));
+                            x[k][i][0] = y.x; x[k][i][1] = y.y; x[k][i][2] = y.z; x[k][i][3] = y.w;
+                        } else if constexpr (E == 2) {
+                            const float2 y = __ldcg(reinterpret_cast<const float2*>(src));
+                            x[k][i][0] = y.x; x[k][i][1] = y.y;
+                        } else {
+                            x[k][i][0] = __ldcg(src);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < RW; ++k)
+#pragma unroll
+                for (int i = 0; i < kAtOnce; ++i) {
+                    const float w = scratch[(k * kWarps + warp) * kChunk + min(i0 + i, n - 1)];
+#pragma unroll
+                    for (int e = 0; e < E; ++e) o[k][e] = fmaf(w, x[k][i][e], o[k][e]);
+                }
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int k = 0; k < RW; ++k) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) l[k] += __shfl_xor_sync(0xffffffffu, l[k], off);
+        if (warp + k * kWarps < nrows) finish(warp + k * kWarps, o[k], m[k], l[k]);
+    }
+}
+
 template <typename T, int D>
-__global__ void __launch_bounds__(kThreads, 2) decode_splitk_kernel(const DecodeArgs a) {
+__global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_kernel(const __grid_constant__ RowsArgs a) {
     using S = Smem<D>;
     constexpr int kChunksPerRow = D / 8;          // 16-byte chunks per K/V row
     constexpr int kCopiesPerLane = kChunksPerRow / 2;  // a lane copies half a row of K and of V
@@ -142,401 +339,623 @@ __global__ void __launch_bounds__(kThreads, 2) decode_splitk_kernel(const Decode
     const int g = lane >> 2;   // mma row group
     const int c4 = lane & 3;
 
-    // A merge kernel launched with programmatic stream serialisation may take its place on the SMs as
-    // soon as every CTA of this grid has started (it still waits for this grid to finish before it reads).
+    // Launched with programmatic stream serialisation: the grid may be set up while the kernel before it
+    // drains, and touches nothing in global memory before that kernel has finished (returns at once
+    // when the launch carries no programmatic dependency). The next kernel may be set up likewise.
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
 
     // KV heads vary fastest across the grid: the CTAs that read the adjacent 256-byte slices of the
     // same token rows (one slice per KV head) are launched together, which keeps DRAM pages open.
-    const int kvh = blockIdx.x / a.head_blocks;
-    const int hb = blockIdx.x - kvh * a.head_blocks;
-    const int split = blockIdx.y;
-    const int s = blockIdx.z;
-
-    const int L = a.context_lens[s];
-    const int chunk_begin = split * a.chunk;
-    if (chunk_begin >= L) return;  // nothing cached here (L <= 0 included): the merge kernel writes zeros
-    const int chunk_end = min(L, chunk_begin + a.chunk);
-
+    const int kvh = blockIdx.x / a.row_blocks;
+    const int row0 = (blockIdx.x - kvh * a.row_blocks) * kRows;   // first query row of this CTA (row = token x group + head in group)
+    const int column = blockIdx.y;
+    int columns = gridDim.y;
     const int group = a.q_heads / a.kv_heads;
-    const int head0 = kvh * group + hb * kMaxHeads;            // first query head of this CTA
-    const int nheads = min(kMaxHeads, group - hb * kMaxHeads);  // query heads served
+
+    // The cut: total units, this column's share of them, and the sequence its first unit lies in.
+    unsigned total = 0, seq_first = 0;   // seq_first: unit at which sequence `s` begins
+    int s = 0;
+    unsigned u_begin, u_end;
+    if (a.mode == MODE_BATCH) {
+        const unsigned per = (unsigned)rows_units(a, rows_seq(a, 0), group, row0);
+        total = per * (unsigned)a.num_seqs;
+        columns = (int)min((unsigned)columns, max(total, 1u));   // never an empty column between two others
+        const Cut cut(total, (unsigned)columns, (unsigned)a.forced_units);
+        u_begin = cut.first(column);
+        u_end = min(total, cut.first(column + 1));
+        if (column >= columns || u_begin >= u_end) return;   // fewer units than columns
+        s = (int)(u_begin / per);
+        seq_first = per * (unsigned)s;
+    } else {
+        // four neighbouring sequences per lane, 128 at a time; the last 128's counts stay in registers
+        int mine[4], lane_sum = 0, upto = 0;
+        int s0 = 0;
+        for (;; s0 += 128) {
+            lane_sum = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int si = s0 + lane * 4 + i;
+                mine[i] = si < a.num_seqs ? rows_units(a, rows_seq(a, si), group, row0) : 0;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) lane_sum += mine[i];
+            upto = lane_sum;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int o = __shfl_up_sync(0xffffffffu, upto, off);
+                if (lane >= off) upto += o;
+            }
+            total += (unsigned)__shfl_sync(0xffffffffu, upto, 31);
+            if (s0 + 128 >= a.num_seqs) break;
+        }
+        columns = (int)min((unsigned)columns, max(total, 1u));   // never an empty column between two others
+        const Cut cut(total, (unsigned)columns, (unsigned)a.forced_units);
+        u_begin = cut.first(column);
+        u_end = min(total, cut.first(column + 1));
+        if (column >= columns || u_begin >= u_end) return;   // fewer units than columns
+        if (s0 > 0) s0 = 0;          // more than 128 sequences: walk them again from the start
+        else s0 = -1;
+        for (;;) {
+            if (s0 >= 0) {
+                lane_sum = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int si = s0 + lane * 4 + i;
+                    mine[i] = si < a.num_seqs ? rows_units(a, rows_seq(a, si), group, row0) : 0;
+                    lane_sum += mine[i];
+                }
+                upto = lane_sum;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const int o = __shfl_up_sync(0xffffffffu, upto, off);
+                    if (lane >= off) upto += o;
+                }
+            }
+            const unsigned past = __ballot_sync(0xffffffffu, seq_first + (unsigned)upto > u_begin);
+            if (past != 0u) {   // always before the sequences run out: u_begin < total
+                const int at = __ffs(past) - 1;
+                unsigned f = seq_first + (unsigned)(upto - lane_sum);
+                int si = max(s0, 0) + lane * 4;
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                    if (f + (unsigned)mine[i] <= u_begin && si == max(s0, 0) + lane * 4 + i) { f += (unsigned)mine[i]; ++si; }
+                s = __shfl_sync(0xffffffffu, si, at);
+                seq_first = __shfl_sync(0xffffffffu, f, at);
+                break;
+            }
+            seq_first += (unsigned)__shfl_sync(0xffffffffu, upto, 31);
+            s0 += 128;
+        }
+    }
 
     const T* __restrict__ qg = static_cast<const T*>(a.q);
     const T* __restrict__ kg = static_cast<const T*>(a.k);
     const T* __restrict__ vg = static_cast<const T*>(a.v);
     const long long kv_pitch = (long long)a.kv_heads * D;
 
-    // Q fragments of the A operand, straight from global: row g and g+8 of the head block.
-    unsigned qa[kKSteps][4];
-    {
-        const unsigned* q0 = reinterpret_cast<const unsigned*>(qg + ((long long)s * a.q_heads + head0 + g) * D);
-        const unsigned* q1 = reinterpret_cast<const unsigned*>(qg + ((long long)s * a.q_heads + head0 + g + 8) * D);
-        const bool v0 = g < nheads, v1 = g + 8 < nheads;
-#pragma unroll
-        for (int kk = 0; kk < kKSteps; ++kk) {
-            qa[kk][0] = v0 ? q0[kk * 8 + c4] : 0u;
-            qa[kk][1] = v1 ? q1[kk * 8 + c4] : 0u;
-            qa[kk][2] = v0 ? q0[kk * 8 + 4 + c4] : 0u;
-            qa[kk][3] = v1 ? q1[kk * 8 + 4 + c4] : 0u;
-        }
-    }
-
-    float acc[kDBlocks][4];
-#pragma unroll
-    for (int n = 0; n < kDBlocks; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
-    float m0 = -INFINITY, m1 = -INFINITY;  // running max of rows g and g+8 (log2 domain)
-    float l0 = 0.0f, l1 = 0.0f;            // this lane's share of the running sums
-
     unsigned char* ring = smem_raw + warp * S::kWarpBytes;
-    const int n_tiles = (chunk_end - chunk_begin + kTile - 1) / kTile;   // tiles in the chunk
-    const int my_tiles = (n_tiles - warp + kWarps - 1) / kWarps;         // tiles warp takes: warp, warp+4, ...
 
+    // ---- copy side: a cursor of its own over the CTA's units ------------------------------------------
     // Copies of one tile: a K/V row (D*2 bytes) is moved by kChunksPerRow adjacent lanes, 16 bytes
     // each, so one warp instruction reads whole rows (full 128-byte lines). Lane r < 16 looks up the
-    // slot of token row r once per tile; the other lanes get it by shuffle.
+    // slot of token row r once per tile, two tiles ahead (the look-up is a load of its own, of a
+    // microsecond under load); the other lanes get it by shuffle.
     constexpr int kRowsPerInstr = 32 / kChunksPerRow;      // 2 (D=128) or 4 (D=64)
     constexpr int kInstrPerTile = kTile / kRowsPerInstr;   // 8 or 4
     static_assert(kCopiesPerLane == kInstrPerTile, "a lane issues one 16-byte copy per instruction");
     const int cp_ch = lane % kChunksPerRow;
     const int cp_sub = lane / kChunksPerRow;
-    auto issue = [&](int it) {
-        if (it < my_tiles) {
-            const int tile = warp + it * kWarps;
-            const int j = chunk_begin + tile * kTile + (lane & 15);
-            long long my_off = -1;   // element offset of token row (lane & 15), -1 when past the chunk
-            if (j < chunk_end) {
-                const int slot = block_slot(a.block_tables, s, a.max_blocks, j, a.block_size);
-                my_off = (long long)slot * kv_pitch + (long long)kvh * D;
+    int cp_left = (int)(u_end - u_begin);
+    int cp_s = s;
+    RowsSeq cp_seq = rows_seq(a, s);
+    int cp_vis = rows_visible(cp_seq);
+    int cp_tok = (int)(u_begin - seq_first) * kUnit;   // first token of the unit to copy next
+    int cp_end = rows_units(a, cp_seq, group, row0) * kUnit;
+    auto look_up = [&]() -> long long {   // element offset of this lane's token row in the caches, -1 past the visible keys
+        const int j = cp_tok + warp * kTile + (lane & 15);
+        if (j >= cp_vis) return -1;
+        long long slot;
+        if (a.paged) {
+            const int page = a.block_shift >= 0 ? j >> a.block_shift : j / a.block_size;
+            slot = a.block_tables[cp_s * a.max_blocks + page] * a.block_size + (j - page * a.block_size);
+        } else {
+            slot = cp_seq.kv_row0 + j;
+        }
+        return slot * kv_pitch + (long long)kvh * D;
+    };
+    int cp_ahead = (int)(u_end - u_begin);   // units whose slots have not been looked up yet
+    auto look_up_next = [&]() -> long long {
+        if (cp_ahead <= 0) return -1;
+        const long long off = look_up();
+        if (--cp_ahead > 0) {
+            cp_tok += kUnit;
+            if (cp_tok >= cp_end) {   // on to the next sequence that has rows here
+                do {
+                    cp_seq = rows_seq(a, ++cp_s);
+                    cp_end = rows_units(a, cp_seq, group, row0) * kUnit;
+                } while (cp_end == 0);
+                cp_vis = rows_visible(cp_seq);
+                cp_tok = 0;
             }
-            unsigned char* kst = ring + (it % kStages) * S::kStageBytes;
+        }
+        return off;
+    };
+    long long cp_off = look_up_next();
+    long long cp_off2 = look_up_next();
+    int cp_stage = 0;
+    auto issue = [&]() {
+        if (cp_left > 0) {
+            unsigned char* kst = ring + cp_stage * S::kStageBytes;
             unsigned char* vst = kst + S::kTileBytes;
 #pragma unroll
             for (int i = 0; i < kInstrPerTile; ++i) {
                 const int row = i * kRowsPerInstr + cp_sub;
-                const long long off = __shfl_sync(0xffffffffu, my_off, row);
+                const long long off = __shfl_sync(0xffffffffu, cp_off, row);
                 const bool valid = off >= 0;
                 const long long src = (valid ? off : 0) + cp_ch * 8;
                 const int dst = row * S::kRowBytes + ((cp_ch ^ (row & S::kSwz)) << 4);
                 cp_async_16(kst + dst, kg + src, valid);
                 cp_async_16(vst + dst, vg + src, valid);
             }
+            cp_stage = cp_stage + 1 == kStages ? 0 : cp_stage + 1;
+            --cp_left;
+            cp_off = cp_off2;
+            cp_off2 = look_up_next();
         }
         cp_async_commit();  // committed even when empty so that group counting stays uniform
     };
 
 #pragma unroll
-    for (int it = 0; it < kStages - 1; ++it) issue(it);
+    for (int it = 0; it < kStages - 1; ++it) issue();
 
-    for (int it = 0; it < my_tiles; ++it) {
-        issue(it + kStages - 1);
-        cp_async_wait<kStages - 1>();
-        __syncwarp();
+    // ---- compute side: sequence after sequence ----------------------------------------------------------
+    float* const merge = reinterpret_cast<float*>(smem_raw + S::kRingBytes);
+    auto merge_ml = [&](int w, int r) { return reinterpret_cast<float2*>(merge + (w * kRows + r) * S::kMergePitch + S::kMergeCols); };
+    int* const last_flag = reinterpret_cast<int*>(smem_raw + S::kRingBytes + S::kMergeBytes);
+    const int cta = blockIdx.y * gridDim.x + blockIdx.x;
+    int stage = 0;
+    unsigned u = u_begin;
+    while (u < u_end) {
+        RowsSeq seq = rows_seq(a, s);
+        int units = rows_units(a, seq, group, row0);
+        while (units == 0) {   // not this launch's
+            seq = rows_seq(a, ++s);
+            units = rows_units(a, seq, group, row0);
+        }
+        const int vis = rows_visible(seq);
+        const int nrows = min(kRows, seq.q_len * group - row0);   // query rows served here
+        const unsigned seg_end = min(u_end, seq_first + (unsigned)units);
+        const bool starts = u == seq_first, ends = seg_end == seq_first + (unsigned)units;
 
-        const unsigned char* kst = ring + (it % kStages) * S::kStageBytes;
-        const unsigned char* vst = kst + S::kTileBytes;
-        const int tile_tok0 = chunk_begin + (warp + it * kWarps) * kTile;
-
-        // S = Q K^T : 16 heads x 16 tokens as two N blocks of 8 tokens
-        float sc[2][4];
-#pragma unroll
-        for (int nb = 0; nb < 2; ++nb) sc[nb][0] = sc[nb][1] = sc[nb][2] = sc[nb][3] = 0.0f;
+        // Q fragments of the A operand, straight from global: rows g and g+8; and the last key each of them sees.
+        unsigned qa[kKSteps][4];
+        int lim0 = -1, lim1 = -1;
         {
-            const int mi = lane >> 3;                    // which 8x8 matrix this lane addresses
-            const int tok = ((mi >> 1) << 3) + (lane & 7);  // token row
+            const bool v0 = g < nrows, v1 = g + 8 < nrows;
+            const int r0 = row0 + g, r1 = row0 + g + 8;
+            const int t0 = r0 / group, t1 = r1 / group;
+            const unsigned* q0 = reinterpret_cast<const unsigned*>(qg + ((seq.q_row0 + t0) * a.q_heads + kvh * group + (r0 - t0 * group)) * D);
+            const unsigned* q1 = reinterpret_cast<const unsigned*>(qg + ((seq.q_row0 + t1) * a.q_heads + kvh * group + (r1 - t1 * group)) * D);
 #pragma unroll
             for (int kk = 0; kk < kKSteps; ++kk) {
-                const int ch = 2 * kk + (mi & 1);
-                unsigned b0, b1, b2, b3;
-                ldmatrix_x4(b0, b1, b2, b3, kst + tok * S::kRowBytes + ((ch ^ (tok & S::kSwz)) << 4));
-                mma_16816<T>(sc[0], qa[kk], b0, b1);
-                mma_16816<T>(sc[1], qa[kk], b2, b3);
+                qa[kk][0] = v0 ? q0[kk * 8 + c4] : 0u;
+                qa[kk][1] = v1 ? q1[kk * 8 + c4] : 0u;
+                qa[kk][2] = v0 ? q0[kk * 8 + 4 + c4] : 0u;
+                qa[kk][3] = v1 ? q1[kk * 8 + 4 + c4] : 0u;
             }
+            lim0 = (int)min((long long)seq.kv_len - 1, (long long)seq.pos_off + t0);
+            lim1 = (int)min((long long)seq.kv_len - 1, (long long)seq.pos_off + t1);
+        }
+        const int lim_all = min(seq.kv_len, seq.pos_off + 1);   // keys below this are seen by every row
+
+        float acc[kDBlocks][4];
+#pragma unroll
+        for (int n = 0; n < kDBlocks; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+        float m0 = -INFINITY, m1 = -INFINITY;  // running max of rows g and g+8 (log2 domain)
+        float l0 = 0.0f, l1 = 0.0f;            // this lane's share of the running sums
+
+        int tok = (int)(u - seq_first) * kUnit + warp * kTile;   // first token of this warp's tile
+        for (; u < seg_end; ++u, tok += kUnit) {
+            issue();
+            cp_async_wait<kStages - 1>();
+            __syncwarp();
+            const unsigned char* kst = ring + stage * S::kStageBytes;
+            const unsigned char* vst = kst + S::kTileBytes;
+            stage = stage + 1 == kStages ? 0 : stage + 1;
+            if (tok >= vis) continue;   // past the last visible key: this warp has no tile in the sequence's last unit
+
+            // S = Q K^T : 16 query rows x 16 tokens as two N blocks of 8 tokens
+            float sc[2][4];
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb) sc[nb][0] = sc[nb][1] = sc[nb][2] = sc[nb][3] = 0.0f;
+            {
+                const int mi = lane >> 3;                    // which 8x8 matrix this lane addresses
+                const int tr = ((mi >> 1) << 3) + (lane & 7);  // token row
+#pragma unroll
+                for (int kk = 0; kk < kKSteps; ++kk) {
+                    const int ch = 2 * kk + (mi & 1);
+                    unsigned b0, b1, b2, b3;
+                    ldmatrix_x4(b0, b1, b2, b3, kst + tr * S::kRowBytes + ((ch ^ (tr & S::kSwz)) << 4));
+                    mma_16816<T>(sc[0], qa[kk], b0, b1);
+                    mma_16816<T>(sc[1], qa[kk], b2, b3);
+                }
+            }
+
+            // scale, mask (only tiles that reach past the first query token's position need it), online
+            // softmax over this tile's 16 tokens
+            const bool cut = tok + kTile > lim_all;
+            float tmax0 = -INFINITY, tmax1 = -INFINITY;
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int j = tok + nb * 8 + 2 * c4 + e;
+                    sc[nb][e] *= a.scale_log2;
+                    sc[nb][2 + e] *= a.scale_log2;
+                    if (cut) {
+                        if (j > lim0) sc[nb][e] = -INFINITY;
+                        if (j > lim1) sc[nb][2 + e] = -INFINITY;
+                    }
+                    tmax0 = fmaxf(tmax0, sc[nb][e]);
+                    tmax1 = fmaxf(tmax1, sc[nb][2 + e]);
+                }
+            }
+            tmax0 = fmaxf(tmax0, __shfl_xor_sync(0xffffffffu, tmax0, 1));
+            tmax0 = fmaxf(tmax0, __shfl_xor_sync(0xffffffffu, tmax0, 2));
+            tmax1 = fmaxf(tmax1, __shfl_xor_sync(0xffffffffu, tmax1, 1));
+            tmax1 = fmaxf(tmax1, __shfl_xor_sync(0xffffffffu, tmax1, 2));
+            const float mp0 = m0, mp1 = m1;
+            m0 = fmaxf(m0, tmax0);
+            m1 = fmaxf(m1, tmax1);
+            // a row that has seen no key yet keeps m = -inf: exp2(-inf - 0) is an exact zero
+            const float mu0 = m0 == -INFINITY ? 0.0f : m0, mu1 = m1 == -INFINITY ? 0.0f : m1;
+            const float alpha0 = fast_exp2(mp0 - mu0), alpha1 = fast_exp2(mp1 - mu1);
+            float ps0 = 0.0f, ps1 = 0.0f;
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    sc[nb][e] = fast_exp2(sc[nb][e] - mu0);
+                    sc[nb][2 + e] = fast_exp2(sc[nb][2 + e] - mu1);
+                    ps0 += sc[nb][e];
+                    ps1 += sc[nb][2 + e];
+                }
+            }
+            l0 = l0 * alpha0 + ps0;
+            l1 = l1 * alpha1 + ps1;
+#pragma unroll
+            for (int n = 0; n < kDBlocks; ++n) {
+                acc[n][0] *= alpha0;
+                acc[n][1] *= alpha0;
+                acc[n][2] *= alpha1;
+                acc[n][3] *= alpha1;
+            }
+
+            // O += P V : P (16 rows x 16 tokens) re-used from the accumulator layout as the A operand
+            unsigned pa[4];
+            pa[0] = pack2<T>(sc[0][0], sc[0][1]);
+            pa[1] = pack2<T>(sc[0][2], sc[0][3]);
+            pa[2] = pack2<T>(sc[1][0], sc[1][1]);
+            pa[3] = pack2<T>(sc[1][2], sc[1][3]);
+            {
+                const int mi = lane >> 3;
+                const int tr = ((mi & 1) << 3) + (lane & 7);
+#pragma unroll
+                for (int n = 0; n < kDBlocks; n += 2) {
+                    const int ch = n + (mi >> 1);
+                    unsigned b0, b1, b2, b3;
+                    ldmatrix_x4_trans(b0, b1, b2, b3, vst + tr * S::kRowBytes + ((ch ^ (tr & S::kSwz)) << 4));
+                    mma_16816<T>(acc[n], pa, b0, b1);
+                    mma_16816<T>(acc[n + 1], pa, b2, b3);
+                }
+            }
+            __syncwarp();  // the stage may be refilled by the next issue()
         }
 
-        // scale, mask the tail of the chunk, online softmax over this tile's 16 tokens
-        float tmax0 = -INFINITY, tmax1 = -INFINITY;
-#pragma unroll
-        for (int nb = 0; nb < 2; ++nb) {
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int j = tile_tok0 + nb * 8 + 2 * c4 + e;
-                const bool vis = j < chunk_end;
-                sc[nb][e] = vis ? sc[nb][e] * a.scale_log2 : -INFINITY;
-                sc[nb][2 + e] = vis ? sc[nb][2 + e] * a.scale_log2 : -INFINITY;
-                tmax0 = fmaxf(tmax0, sc[nb][e]);
-                tmax1 = fmaxf(tmax1, sc[nb][2 + e]);
-            }
+        // ---- the warps' parts of this sequence, merged through shared memory ----------------------------
+        // row sums: fold the four lanes that share a row
+        l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+        l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+        l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+        l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+        if (c4 == 0) {
+            *merge_ml(warp, g) = make_float2(m0, l0);
+            *merge_ml(warp, g + 8) = make_float2(m1, l1);
         }
-        tmax0 = fmaxf(tmax0, __shfl_xor_sync(0xffffffffu, tmax0, 1));
-        tmax0 = fmaxf(tmax0, __shfl_xor_sync(0xffffffffu, tmax0, 2));
-        tmax1 = fmaxf(tmax1, __shfl_xor_sync(0xffffffffu, tmax1, 1));
-        tmax1 = fmaxf(tmax1, __shfl_xor_sync(0xffffffffu, tmax1, 2));
-        // every tile inside the chunk has at least its first token visible, so the maxima are finite
-        const float mn0 = fmaxf(m0, tmax0), mn1 = fmaxf(m1, tmax1);
-        const float alpha0 = fast_exp2(m0 - mn0), alpha1 = fast_exp2(m1 - mn1);
-        m0 = mn0;
-        m1 = mn1;
-        float ps0 = 0.0f, ps1 = 0.0f;
+        const int slot = 2 * cta + (starts ? 1 : 0);
+        float* const mine = merge + warp * kRows * S::kMergePitch;
 #pragma unroll
-        for (int nb = 0; nb < 2; ++nb) {
+        for (int pass = 0; pass < D / S::kMergeCols; ++pass) {
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                sc[nb][e] = fast_exp2(sc[nb][e] - mn0);
-                sc[nb][2 + e] = fast_exp2(sc[nb][2 + e] - mn1);
-                ps0 += sc[nb][e];
-                ps1 += sc[nb][2 + e];
+            for (int n = 0; n < S::kMergeCols / 8; ++n) {
+                const int d = n * 8 + 2 * c4;
+                const float(&x)[4] = acc[pass * (S::kMergeCols / 8) + n];
+                *reinterpret_cast<float2*>(mine + g * S::kMergePitch + d) = make_float2(x[0], x[1]);
+                *reinterpret_cast<float2*>(mine + (g + 8) * S::kMergePitch + d) = make_float2(x[2], x[3]);
             }
-        }
-        l0 = l0 * alpha0 + ps0;
-        l1 = l1 * alpha1 + ps1;
+            __syncthreads();
+            for (int idx = threadIdx.x; idx < nrows * (S::kMergeCols / 2); idx += kThreads) {
+                const int r = idx / (S::kMergeCols / 2);
+                const int d = (idx - r * (S::kMergeCols / 2)) * 2;
+                float2 ml[kWarps];
+                float mstar = -INFINITY;
 #pragma unroll
-        for (int n = 0; n < kDBlocks; ++n) {
-            acc[n][0] *= alpha0;
-            acc[n][1] *= alpha0;
-            acc[n][2] *= alpha1;
-            acc[n][3] *= alpha1;
+                for (int w = 0; w < kWarps; ++w) {
+                    ml[w] = *merge_ml(w, r);
+                    mstar = fmaxf(mstar, ml[w].x);
+                }
+                float ox = 0.0f, oy = 0.0f, l = 0.0f;
+#pragma unroll
+                for (int w = 0; w < kWarps; ++w) {
+                    const float wgt = ml[w].x == -INFINITY ? 0.0f : fast_exp2(ml[w].x - mstar);
+                    const float2 x = *reinterpret_cast<const float2*>(merge + (w * kRows + r) * S::kMergePitch + d);
+                    ox += wgt * x.x;
+                    oy += wgt * x.y;
+                    l += wgt * ml[w].y;
+                }
+                const int dd = pass * S::kMergeCols + d;
+                if (starts && ends) {   // the whole sequence: finished here
+                    const float inv = l > 0.0f ? 1.0f / l : 0.0f;   // reference: flash_attn_with_kvcache.cu:109
+                    const int t = (row0 + r) / group, h = kvh * group + (row0 + r) - t * group;
+                    const unsigned w2 = pack2<T>(ox * inv, oy * inv);
+                    store_pair<T>(a.out, seq.q_row0 + t, h, D, dd, w2);
+                    if (dd == 0 && a.out.lse != nullptr)
+                        a.out.lse[((long long)s * a.q_heads + h) * a.q_seq_len + t] = l > 0.0f ? (mstar + log2f(l)) * 0.6931471805599453f : -INFINITY;
+                } else {
+                    *reinterpret_cast<float2*>(a.ws_acc + ((long long)slot * kRows + r) * D + dd) = make_float2(ox, oy);
+                    if (dd == 0) a.ws_ml[(long long)slot * kRows + r] = make_float2(mstar, l);
+                }
+            }
+            __syncthreads();   // the buffer is written again by the next pass or sequence
         }
 
-        // O += P V : P (16 heads x 16 tokens) re-used from the accumulator layout as the A operand
-        unsigned pa[4];
-        pa[0] = pack2<T>(sc[0][0], sc[0][1]);
-        pa[1] = pack2<T>(sc[0][2], sc[0][3]);
-        pa[2] = pack2<T>(sc[1][0], sc[1][1]);
-        pa[3] = pack2<T>(sc[1][2], sc[1][3]);
-        {
-            const int mi = lane >> 3;
-            const int tok = ((mi & 1) << 3) + (lane & 7);
+        if (!(starts && ends)) {
+            // ---- a cut sequence: whoever brings the last part merges all of them, in column order --------
+            const Cut cut(total, (unsigned)columns, (unsigned)a.forced_units);
+            const int c_first = (int)cut.column_of(seq_first);
+            const int parts = (int)cut.column_of(seq_first + (unsigned)units - 1u) - c_first + 1;
+            // (the last pass of the merge above ended with a barrier: every thread's partials are before this)
+            if (threadIdx.x == 0) {
+                unsigned* cnt = a.arrived + (long long)blockIdx.x * a.num_seqs + s;
+                const int last = arrive_acq_rel(cnt) == (unsigned)(parts - 1);
+                if (last) *cnt = 0u;   // as it was found, for the next call
+                *last_flag = last;
+            }
+            __syncthreads();
+            if (*last_flag) {
+                const float* acc0 = a.ws_acc + (long long)blockIdx.x * (2 * kRows * D);
+                const float2* ml0 = a.ws_ml + (long long)blockIdx.x * (2 * kRows);
+                auto finish = [&](int r, const float (&o)[D / 32], float m, float l) {
+                    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+                    const int t = (row0 + r) / group, h = kvh * group + (row0 + r) - t * group;
+                    if constexpr (D >= 64) {
 #pragma unroll
-            for (int n = 0; n < kDBlocks; n += 2) {
-                const int ch = n + (mi >> 1);
-                unsigned b0, b1, b2, b3;
-                ldmatrix_x4_trans(b0, b1, b2, b3, vst + tok * S::kRowBytes + ((ch ^ (tok & S::kSwz)) << 4));
-                mma_16816<T>(acc[n], pa, b0, b1);
-                mma_16816<T>(acc[n + 1], pa, b2, b3);
+                        for (int e = 0; e < D / 32; e += 2)
+                            store_pair<T>(a.out, seq.q_row0 + t, h, D, lane * (D / 32) + e, pack2<T>(o[e] * inv, o[e + 1] * inv));
+                    } else {
+                        const float up = __shfl_down_sync(0xffffffffu, o[0], 1);
+                        if ((lane & 1) == 0) store_pair<T>(a.out, seq.q_row0 + t, h, D, lane, pack2<T>(o[0] * inv, up * inv));
+                    }
+                    if (lane == 0 && a.out.lse != nullptr)
+                        a.out.lse[((long long)s * a.q_heads + h) * a.q_seq_len + t] = l > 0.0f ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
+                };
+                const int rows_per_warp = (nrows + kWarps - 1) / kWarps;
+                if (rows_per_warp == 1) merge_parts<D, 1>(acc0, ml0, merge, nrows, c_first, parts, gridDim.x, warp, lane, finish);
+                else if (rows_per_warp == 2) merge_parts<D, 2>(acc0, ml0, merge, nrows, c_first, parts, gridDim.x, warp, lane, finish);
+                else merge_parts<D, 4>(acc0, ml0, merge, nrows, c_first, parts, gridDim.x, warp, lane, finish);
+                __syncthreads();   // the merge buffer is written again by the next sequence
             }
         }
-        __syncwarp();  // the stage may be refilled by the next issue()
+        if (ends) {
+            seq_first += (unsigned)units;
+            ++s;
+        }
     }
     cp_async_wait<0>();
-
-    // row sums: fold the four lanes that share a row
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-
-    // cross-warp merge through shared memory (the ring is dead now)
-    __syncthreads();
-    float* merge = reinterpret_cast<float*>(smem_raw);
-    float* macc = merge + warp * kMaxHeads * (D + 2);  // [head][D + 2]: acc, m, l
-#pragma unroll
-    for (int n = 0; n < kDBlocks; ++n) {
-        const int d = n * 8 + 2 * c4;
-        macc[g * (D + 2) + d] = acc[n][0];
-        macc[g * (D + 2) + d + 1] = acc[n][1];
-        macc[(g + 8) * (D + 2) + d] = acc[n][2];
-        macc[(g + 8) * (D + 2) + d + 1] = acc[n][3];
-    }
-    if (c4 == 0) {
-        macc[g * (D + 2) + D] = m0;
-        macc[g * (D + 2) + D + 1] = l0;
-        macc[(g + 8) * (D + 2) + D] = m1;
-        macc[(g + 8) * (D + 2) + D + 1] = l1;
-    }
-    __syncthreads();
-
-    for (int idx = threadIdx.x; idx < nheads * D; idx += kThreads) {
-        const int hh = idx / D;
-        const int d = idx - hh * D;
-        float mw[kWarps];
-        float mstar = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            mw[w] = merge[(w * kMaxHeads + hh) * (D + 2) + D];
-            mstar = fmaxf(mstar, mw[w]);
-        }
-        float o = 0.0f, l = 0.0f;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const float wgt = (mw[w] == -INFINITY) ? 0.0f : fast_exp2(mw[w] - mstar);
-            o += wgt * merge[(w * kMaxHeads + hh) * (D + 2) + d];
-            l += wgt * merge[(w * kMaxHeads + hh) * (D + 2) + D + 1];
-        }
-        const long long row = ((long long)s * a.q_heads + head0 + hh) * a.max_splits + split;
-        a.ws_acc[row * D + d] = o;
-        if (d == 0) a.ws_ml[row] = make_float2(mstar, l);
-    }
 }
 
-// Where the merged rows go: one buffer of (num_seqs, 1, o_heads, D), or — head-sharded decode with
-// the output all-gather fused in — the same tensor on every GPU of the group (peer memory, plain
-// stores over NVLink), each receiving this call's heads at head offset o_head0.
-struct MergeOut {
-    void* o[8];
-    int n_out, o_heads, o_head0, peer0;
+// The grid: one CTA per KV head (x row block) and column, as many columns as fill the device's CTA slots in
+// one wave or, where that leaves too many slots empty (many KV heads), in two.
+int num_columns(int per_column, int ctas_per_sm, int sms) {
+    const long long slots = (long long)ctas_per_sm * sms;
+    const int one = (int)std::max<long long>(1, slots / per_column);
+    const int two = (int)std::max<long long>(1, 2 * slots / per_column);
+    const bool one_fills = (long long)one * per_column * 100 >= slots * 95 || 2LL * one * per_column >= (long long)two * per_column;
+    return one_fills ? one : two;
+}
+
+int sm_count() {
+    static std::atomic<int> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    int n = known[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        known[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+struct RowsPlan {
+    int row_blocks, columns, forced_units;
+    size_t partial_bytes, counter_bytes, acc_bytes;
 };
 
-// Merges the split-K partials of one (sequence, query head) and writes the output row.
-template <typename T, int D>
-__global__ void __launch_bounds__(D) decode_merge_kernel(const float* __restrict__ ws_acc,
-                                                         const float2* __restrict__ ws_ml,
-                                                         const int* __restrict__ context_lens,
-                                                         const MergeOut out, int q_heads, int chunk,
-                                                         int max_splits) {
-    const int h = blockIdx.x;
-    const int s = blockIdx.y;
-    const int d = threadIdx.x;
-    const int L = context_lens[s];
-    const int n = L > 0 ? min(max_splits, (L + chunk - 1) / chunk) : 0;
-    // the split-K grid this one depends on has finished and its partials are visible (returns at once
-    // when the launch carries no programmatic dependency)
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    const long long row0 = ((long long)s * q_heads + h) * max_splits;
-    float mstar = -INFINITY;
-    for (int i = 0; i < n; ++i) mstar = fmaxf(mstar, ws_ml[row0 + i].x);
-    float acc = 0.0f, l = 0.0f;
-    for (int i = 0; i < n; ++i) {
-        const float2 ml = ws_ml[row0 + i];
-        const float w = (ml.x == -INFINITY) ? 0.0f : fast_exp2(ml.x - mstar);
-        acc += w * ws_acc[(row0 + i) * D + d];
-        l += w * ml.y;
+// `rows`: query rows per KV head at most; `max_tokens`: upper bound of a sequence's visible keys.
+template <int D>
+RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, bool allow_forced) {
+    RowsPlan r{};
+    r.row_blocks = (rows + kRows - 1) / kRows;
+    const long long per_column = (long long)kv_heads * r.row_blocks;
+    if (per_column > 0x7fffffffLL) return r;   // columns == 0: not this kernel's
+    r.columns = num_columns((int)per_column, Smem<D>::kCtasPerSm, sm_count());
+    const long long most_units = (long long)num_seqs * std::max(1LL, (max_tokens + kUnit - 1) / kUnit);
+    if (allow_forced && get_option_decode_chunk() > 0) {
+        r.forced_units = (get_option_decode_chunk() + kUnit - 1) / kUnit;
+        while ((most_units + r.forced_units - 1) / r.forced_units > 4096) r.forced_units *= 2;
+        r.columns = (int)((most_units + r.forced_units - 1) / r.forced_units);
     }
-    // reference: inv = l > 0 ? 1/l : 0 (flash_attn_with_kvcache.cu:109)
-    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-    const T val = from_f32<T>(acc * inv);
-    const long long off = ((long long)s * out.o_heads + out.o_head0 + h) * D + d;
-    int pe = out.peer0;
-    for (int n = 0; n < out.n_out; ++n) {
-        static_cast<T*>(out.o[pe])[off] = val;
-        pe = pe + 1 == out.n_out ? 0 : pe + 1;
-    }
-}
-
-MergeOut merge_out_single(void* o, int q_heads) {
-    MergeOut m{};
-    m.o[0] = o;
-    m.n_out = 1;
-    m.o_heads = q_heads;
-    return m;
-}
-
-// Tokens per work item. A CTA needs several microseconds to fill its copy pipeline, so long
-// chunks win as long as there are enough of them: the largest of 4096/2048/1024 that still yields
-// >= 1500 work items (about 5 waves of 2 CTAs x 148 SMs, counted at the maximum length), else the
-// largest chunk >= 256 that yields at least 256. `base` = work items per split.
-static int auto_chunk(long long base, long long max_tokens) {
-    auto items = [&](int c) { return base * ((max_tokens + c - 1) / c); };
-    for (int c = 4096; c >= 1024; c >>= 1)
-        if (items(c) >= 1500) return c;
-    for (int c = 4096; c >= 256; c >>= 1)
-        if (items(c) >= 256) return c;
-    return 256;
+    r.columns = (int)std::min<long long>(std::min(r.columns, 65535), most_units);
+    const size_t slots = (size_t)2 * per_column * r.columns;
+    r.acc_bytes = slots * kRows * D * sizeof(float);
+    r.partial_bytes = r.acc_bytes + slots * kRows * sizeof(float2);
+    r.counter_bytes = (size_t)per_column * num_seqs * sizeof(unsigned);
+    return r;
 }
 
 template <typename T, int D>
-int launch_typed(const AttnParams& p, cudaStream_t stream) {
+int launch_rows(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
     using S = Smem<D>;
-    const int group = p.q_heads / p.kv_heads;
-    const int head_blocks = (group + kMaxHeads - 1) / kMaxHeads;
-    const long long max_tokens = (long long)p.max_blocks * p.block_size;
-    if (max_tokens <= 0) return -1;
-
-    const int unit = kWarps * kTile;
-    int chunk = get_option_decode_chunk();
-    if (chunk <= 0) chunk = auto_chunk((long long)p.num_seqs * p.kv_heads * head_blocks, max_tokens);
-    chunk = ((chunk + unit - 1) / unit) * unit;
-    const long long max_splits_ll = (max_tokens + chunk - 1) / chunk;
-    if (max_splits_ll > 65535 || p.num_seqs > 65535 || (long long)p.kv_heads * head_blocks > 65535) return -1;
-    const int max_splits = (int)max_splits_ll;
-
-    const size_t rows = (size_t)p.num_seqs * p.q_heads * max_splits;
-    const size_t acc_bytes = rows * D * sizeof(float);
-    const size_t ml_bytes = rows * sizeof(float2);
-    unsigned char* ws = static_cast<unsigned char*>(decode_workspace(stream, acc_bytes + ml_bytes));
-    if (ws == nullptr) {
-        set_last_errorf("flash_attn_with_kvcache: could not allocate %zu bytes of split-K workspace",
-                        acc_bytes + ml_bytes);
-        return FLASH_ATTN_ERR_CUDA;
+    a.row_blocks = plan.row_blocks;
+    a.forced_units = plan.forced_units;
+    static std::atomic<unsigned long long> ready{0};   // devices whose copy of this kernel has its shared-memory limit raised
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err == cudaSuccess && (dev >= 64 || !((ready.load(std::memory_order_acquire) >> dev) & 1ULL))) {
+        err = cudaFuncSetAttribute(decode_splitk_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
+        if (err == cudaSuccess && dev < 64) ready.fetch_or(1ULL << dev, std::memory_order_release);
     }
-
-    DecodeArgs a{};
-    a.q = p.q; a.k = p.k; a.v = p.v;
-    a.block_tables = p.block_tables;
-    a.context_lens = p.context_lens;
-    a.ws_acc = reinterpret_cast<float*>(ws);
-    a.ws_ml = reinterpret_cast<float2*>(ws + acc_bytes);
-    a.num_seqs = p.num_seqs;
-    a.q_heads = p.q_heads;
-    a.kv_heads = p.kv_heads;
-    a.block_size = p.block_size;
-    a.max_blocks = p.max_blocks;
-    a.chunk = chunk;
-    a.max_splits = max_splits;
-    a.head_blocks = head_blocks;
-    a.scale_log2 = p.scale * 1.4426950408889634f;
-
-    cudaError_t err = cudaFuncSetAttribute(decode_splitk_kernel<T, D>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
     if (err != cudaSuccess) {
         set_last_errorf("decode_splitk_kernel: %s", cudaGetErrorString(err));
         cudaGetLastError();
         return FLASH_ATTN_ERR_CUDA;
     }
-    dim3 grid(p.kv_heads * head_blocks, max_splits, p.num_seqs);
-    decode_splitk_kernel<T, D><<<grid, kThreads, S::kBytes, stream>>>(a);
-    int rc = check_launch("decode_splitk_kernel");
-    if (rc != FLASH_ATTN_OK) return rc;
-    dim3 mgrid(p.q_heads, p.num_seqs);
-    MergeOut mo = merge_out_single(p.o, p.q_heads);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(a.kv_heads * plan.row_blocks), (unsigned)plan.columns);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = S::kBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, decode_splitk_kernel<T, D>, a);
+    return check_launch("decode_splitk_kernel");
+}
+
+int log2_or_minus1(int v) {
+    for (int i = 0; i < 31; ++i)
+        if (v == (1 << i)) return i;
+    return -1;
+}
+
+template <typename T, int D>
+int launch_typed(const AttnParams& p, int rows, int max_rows, cudaStream_t stream) {
+    const long long max_tokens = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
+    if (max_tokens <= 0) return -1;
+    const RowsPlan plan = plan_rows<D>(p.num_seqs, p.kv_heads, rows, max_tokens, true);
+    if (plan.columns <= 0) return -1;
+
+    unsigned* arrived = nullptr;
+    unsigned char* ws = static_cast<unsigned char*>(decode_workspace(stream, plan.partial_bytes, plan.counter_bytes, &arrived));
+    if (ws == nullptr) {
+        set_last_errorf("flash_attn_with_kvcache: could not allocate %zu bytes of split-K workspace",
+                        plan.partial_bytes + plan.counter_bytes);
+        return FLASH_ATTN_ERR_CUDA;
+    }
+
+    RowsArgs a{};
+    a.q = p.q; a.k = p.k; a.v = p.v;
+    a.block_tables = p.block_tables;
+    a.context_lens = p.context_lens;
+    a.cu_q = p.cu_q;
+    a.cu_k = p.cu_k;
+    a.ws_acc = reinterpret_cast<float*>(ws);
+    a.ws_ml = reinterpret_cast<float2*>(ws + plan.acc_bytes);
+    a.arrived = arrived;
+    a.mode = p.mode;
+    a.num_seqs = p.num_seqs;
+    a.q_seq_len = p.q_seq_len;
+    a.kv_seq_len = p.kv_seq_len;
+    a.start_pos = p.start_pos;
+    a.q_heads = p.q_heads;
+    a.kv_heads = p.kv_heads;
+    a.block_size = p.block_size;
+    a.block_shift = log2_or_minus1(p.block_size);
+    a.max_blocks = p.max_blocks;
+    a.paged = p.paged;
+    a.max_rows = max_rows;
+    a.scale_log2 = p.scale * 1.4426950408889634f;
     if (p.n_out > 0) {
-        for (int i = 0; i < p.n_out && i < 8; ++i) mo.o[i] = p.o_peers[i];
-        mo.n_out = p.n_out;
-        mo.o_heads = p.o_heads;
-        mo.o_head0 = p.o_head0;
-        mo.peer0 = (p.o_head0 / p.q_heads + 1) % p.n_out;
+        for (int i = 0; i < p.n_out && i < 8; ++i) a.out.o[i] = p.o_peers[i];
+        a.out.n_out = p.n_out;
+        a.out.o_heads = p.o_heads;
+        a.out.o_head0 = p.o_head0;
+        a.out.peer0 = (p.o_head0 / p.q_heads + 1) % p.n_out;
+    } else {
+        a.out.o[0] = p.o;
+        a.out.n_out = 1;
+        a.out.o_heads = p.q_heads;
     }
-    {
-        // programmatic dependent launch: the merge grid is set up while the split-K grid drains
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = mgrid;
-        cfg.blockDim = dim3(D);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr.val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        const float* ws_acc = a.ws_acc;
-        const float2* ws_ml = a.ws_ml;
-        const int* lens = p.context_lens;
-        const int q_heads = p.q_heads;
-        cudaLaunchKernelEx(&cfg, decode_merge_kernel<T, D>, ws_acc, ws_ml, lens, mo, q_heads, chunk, max_splits);
-    }
-    rc = check_launch("decode_merge_kernel");
-    if (rc == FLASH_ATTN_OK) note_path("decode_splitk", 2);
+    a.out.lse = p.lse;
+    const int rc = launch_rows<T, D>(a, plan, stream);
+    if (rc == FLASH_ATTN_OK) note_path("decode_splitk", 1);
     return rc;
 }
 
 }  // namespace
 
-int launch_decode_splitk(const AttnParams& p, cudaStream_t stream) {
-    if (p.mode != MODE_KVCACHE || p.q_seq_len != 1) return -1;
-    if (p.dtype != DT_F16 && p.dtype != DT_BF16) return -1;
-    if (p.head_size != 32 && p.head_size != 64 && p.head_size != 128) return -1;
-    if (p.q_heads > 65535) return -1;
-    // 16-byte cp.async needs 16-byte aligned rows
-    if ((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) return -1;
-    if (reinterpret_cast<uintptr_t>(p.q) & 3) return -1;
+namespace {
+
+// 16-bit storage, 16-byte aligned K/V rows (cp.async); q is read and o written four bytes at a time.
+bool rows_kernel_takes(const AttnParams& p) {
+    if (p.dtype != DT_F16 && p.dtype != DT_BF16) return false;
+    if (p.head_size != 32 && p.head_size != 64 && p.head_size != 128) return false;
+    if (p.mask != nullptr || p.n_lse > 0 || p.multicast) return false;
+    if ((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) return false;
+    uintptr_t qo = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.o);
+    for (int i = 0; i < p.n_out && i < 8; ++i) qo |= reinterpret_cast<uintptr_t>(p.o_peers[i]);
+    return (qo & 3) == 0;
+}
+
+int launch_rows_typed(const AttnParams& p, int rows, int max_rows, cudaStream_t stream) {
     if (p.dtype == DT_BF16) {
-        return p.head_size == 128 ? launch_typed<__nv_bfloat16, 128>(p, stream)
-               : p.head_size == 64 ? launch_typed<__nv_bfloat16, 64>(p, stream)
-                                   : launch_typed<__nv_bfloat16, 32>(p, stream);
+        return p.head_size == 128 ? launch_typed<__nv_bfloat16, 128>(p, rows, max_rows, stream)
+               : p.head_size == 64 ? launch_typed<__nv_bfloat16, 64>(p, rows, max_rows, stream)
+                                   : launch_typed<__nv_bfloat16, 32>(p, rows, max_rows, stream);
     }
-    return p.head_size == 128 ? launch_typed<__half, 128>(p, stream)
-           : p.head_size == 64 ? launch_typed<__half, 64>(p, stream)
-                               : launch_typed<__half, 32>(p, stream);
+    return p.head_size == 128 ? launch_typed<__half, 128>(p, rows, max_rows, stream)
+           : p.head_size == 64 ? launch_typed<__half, 64>(p, rows, max_rows, stream)
+                               : launch_typed<__half, 32>(p, rows, max_rows, stream);
+}
+
+}  // namespace
+
+int launch_decode_splitk(const AttnParams& p, cudaStream_t stream) {
+    if (p.mode != MODE_KVCACHE || p.q_seq_len != 1 || !rows_kernel_takes(p)) return -1;
+    const int rows = p.q_heads / p.kv_heads;
+    return launch_rows_typed(p, rows, rows, stream);
+}
+
+// Whether few query rows (per KV head) over a range of `keys` are better off here than on the tensor-core prefill
+// kernel, whose CTAs walk a whole K/V range each, for one or two 128-row tiles of which almost all rows are empty.
+// That kernel takes about 5 us plus 1.7 us per 128 keys, times the waves of its CTAs: up to 12 tiles in one
+// wave (25 us at most) it keeps the call; beyond, the cut of the K/V ranges over the whole device wins at any
+// size (16 sequences x 4 tokens x 4 heads over 512-8192 keys: 63 us against 175; 8 rows of 4000 keys, f16: 27 against
+// 62; 26 single tokens over 802 keys: 21 against 58).
+static bool worth_cutting(const AttnParams& p, long long rows) {
+    const long long keys = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
+    const long long tile_pairs = ((long long)(p.q_heads / p.kv_heads) * ((p.q_seq_len + 127) / 128) + 1) / 2 * p.kv_heads * p.num_seqs;
+    return rows > 0 && (keys > 12 * 128 || tile_pairs > sm_count());
+}
+
+int launch_few_rows(const AttnParams& p, cudaStream_t stream) {
+    if (p.n_out > 0 || !rows_kernel_takes(p)) return -1;
+    const long long rows = (long long)p.q_seq_len * (p.q_heads / p.kv_heads);
+    // up to four row blocks: each reads the K/V rows again, from L2 (28 rows of 7 x 1355-5421 keys: 43 us against
+    // 87 on the prefill kernel; 32 rows of 8 x 3108: 45 against 109)
+    if (rows > 4 * kRows || !worth_cutting(p, rows)) return -1;
+    return launch_rows_typed(p, (int)rows, (int)rows, stream);
+}
+
+int launch_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {
+    if (p.mode != MODE_VARLEN || p.num_seqs < 2 || p.n_out > 0 || !rows_kernel_takes(p)) return 0;
+    const int group = p.q_heads / p.kv_heads;
+    // one row block: the CTA slots are shared out before anybody knows how many rows the sequences have
+    if (group > kRows || !worth_cutting(p, kRows)) return 0;
+    return launch_rows_typed(p, kRows, kRows, stream) == FLASH_ATTN_OK ? kRows : 0;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -557,11 +976,12 @@ int launch_decode_splitk(const AttnParams& p, cudaStream_t stream) {
 //
 // In host code `g_static_scratch` is only a handle for the symbol, not a device address; the
 // device address is fetched once per device with cudaGetSymbolAddress (with that device current)
-// and passed to the same two kernels the ordinary path launches.
+// and passed to the same kernel the ordinary path launches.
 // ---------------------------------------------------------------------------------------------
 namespace {
 
 constexpr size_t kStaticScratchBytes = size_t(16) << 20;   // 16 MiB per GPU
+constexpr size_t kStaticCounterBytes = size_t(1) << 20;    // of these, the arrival counters (at most 63 550 x 4 bytes within the entry point's limit)
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
 constexpr int kMaxDevices = 64;
@@ -603,13 +1023,10 @@ int launch_static(const void* q, const void* k, const void* v, void* o, const in
                   const int* context_lens, int num_seqs, int q_heads, int kv_heads, int block_size,
                   int max_blocks, float scale, cudaStream_t stream) {
     using T = __nv_bfloat16;
-    using S = Smem<D>;
     const int group = q_heads / kv_heads;
-    const int head_blocks = (group + kMaxHeads - 1) / kMaxHeads;
     const long long max_tokens = (long long)max_blocks * block_size;
-    const int unit = kWarps * kTile;
 
-    // one split must always fit; beyond that the chunk grows until the partials fit the array
+    // the documented limit of this entry point: one (acc, m, l) row per (sequence, head)
     const size_t row_bytes = (size_t)D * sizeof(float) + sizeof(float2);
     const size_t rows1 = (size_t)num_seqs * q_heads;
     if (rows1 * row_bytes > kStaticScratchBytes) {
@@ -618,56 +1035,47 @@ int launch_static(const void* q, const void* k, const void* v, void* o, const in
                         rows1, kStaticScratchBytes, kStaticScratchBytes / row_bytes, D);
         return FLASH_ATTN_ERR_INVALID_SHAPE;
     }
-    long long chunk = auto_chunk((long long)num_seqs * kv_heads * head_blocks, max_tokens);
-    {
-        while (rows1 * (size_t)((max_tokens + chunk - 1) / chunk) * row_bytes > kStaticScratchBytes) chunk <<= 1;
+    // Within that limit the counters (one per sequence and row block of a KV head, at most one per row)
+    // fit their part of the array; the partials are bounded by the device's CTA slots, not by the call
+    // (two waves of 2 x 148 CTAs at head size 128: 9.8 MB).
+    RowsPlan plan = plan_rows<D>(num_seqs, kv_heads, group, max_tokens, false);
+    while (plan.columns > 1 && plan.partial_bytes > kStaticScratchBytes - kStaticCounterBytes) {
+        const size_t per = plan.partial_bytes / plan.columns;
+        --plan.columns;
+        plan.partial_bytes -= per;
+        plan.acc_bytes = (size_t)2 * kv_heads * plan.row_blocks * plan.columns * kRows * D * sizeof(float);
     }
-    chunk = ((chunk + unit - 1) / unit) * unit;
-    const long long max_splits_ll = (max_tokens + chunk - 1) / chunk;
-    if (chunk > 0x40000000LL || max_splits_ll > 65535 || num_seqs > 65535 || (long long)kv_heads * head_blocks > 65535 ||
-        q_heads > 65535) {
+    if (plan.columns <= 0 || plan.counter_bytes > kStaticCounterBytes) {
         set_last_error("flash_attn_decode_bf16_noalloc: grid dimensions out of range");
         return FLASH_ATTN_ERR_INVALID_SHAPE;
     }
-    const int max_splits = (int)max_splits_ll;
-    const size_t rows = rows1 * max_splits;
-    const size_t acc_bytes = rows * D * sizeof(float);   // a multiple of 256 bytes, so the float2 part stays aligned
 
     unsigned char* ws = static_scratch_ptr();
     if (ws == nullptr) return FLASH_ATTN_ERR_CUDA;
 
-    DecodeArgs a{};
+    RowsArgs a{};
     a.q = q; a.k = k; a.v = v;
     a.block_tables = block_tables;
     a.context_lens = context_lens;
-    a.ws_acc = reinterpret_cast<float*>(ws);
-    a.ws_ml = reinterpret_cast<float2*>(ws + acc_bytes);
+    a.arrived = reinterpret_cast<unsigned*>(ws);   // zero in the library image, and again after every call
+    a.ws_acc = reinterpret_cast<float*>(ws + kStaticCounterBytes);
+    a.ws_ml = reinterpret_cast<float2*>(ws + kStaticCounterBytes + plan.acc_bytes);
+    a.mode = MODE_KVCACHE;
     a.num_seqs = num_seqs;
+    a.q_seq_len = 1;
     a.q_heads = q_heads;
     a.kv_heads = kv_heads;
     a.block_size = block_size;
+    a.block_shift = log2_or_minus1(block_size);
     a.max_blocks = max_blocks;
-    a.chunk = (int)chunk;
-    a.max_splits = max_splits;
-    a.head_blocks = head_blocks;
+    a.paged = 1;
+    a.max_rows = group;
     a.scale_log2 = scale * 1.4426950408889634f;
-
-    cudaError_t err = cudaFuncSetAttribute(decode_splitk_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           S::kBytes);
-    if (err != cudaSuccess) {
-        set_last_errorf("decode_splitk_kernel: %s", cudaGetErrorString(err));
-        cudaGetLastError();
-        return FLASH_ATTN_ERR_CUDA;
-    }
-    dim3 grid(kv_heads * head_blocks, max_splits, num_seqs);
-    decode_splitk_kernel<T, D><<<grid, kThreads, S::kBytes, stream>>>(a);
-    int rc = check_launch("decode_splitk_kernel");
-    if (rc != FLASH_ATTN_OK) return rc;
-    dim3 mgrid(q_heads, num_seqs);
-    decode_merge_kernel<T, D><<<mgrid, D, 0, stream>>>(a.ws_acc, a.ws_ml, context_lens, merge_out_single(o, q_heads), q_heads,
-                                                      (int)chunk, max_splits);
-    rc = check_launch("decode_merge_kernel");
-    if (rc == FLASH_ATTN_OK) note_path("decode_splitk_static", 2);
+    a.out.o[0] = o;
+    a.out.n_out = 1;
+    a.out.o_heads = q_heads;
+    const int rc = launch_rows<T, D>(a, plan, stream);
+    if (rc == FLASH_ATTN_OK) note_path("decode_splitk_static", 1);
     return rc;
 }
 
@@ -696,8 +1104,8 @@ extern "C" int flash_attn_decode_bf16_noalloc(const flash_attn_bf16_t* q, const 
         return FLASH_ATTN_ERR_INVALID_SHAPE;
     }
     if (((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) ||
-        (reinterpret_cast<uintptr_t>(q) & 3)) {
-        set_last_error("flash_attn_decode_bf16_noalloc: k_cache/v_cache must be 16-byte aligned, q 4-byte aligned");
+        ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(o)) & 3)) {
+        set_last_error("flash_attn_decode_bf16_noalloc: k_cache/v_cache must be 16-byte aligned, q and o 4-byte aligned");
         return FLASH_ATTN_ERR_INVALID_SHAPE;
     }
     // launch on the device that owns q, and resolve the scratch address on that same device
