@@ -222,6 +222,8 @@ int dispatch(const AttnParams& p, cudaStream_t stream) {
     if (!get_option_force_generic()) {
         int rc = launch_decode_splitk(p, stream);
         if (rc >= 0) return rc;
+        rc = launch_few_rows(p, stream);
+        if (rc >= 0) return rc;
         rc = launch_prefill_tcgen05(p, stream);
         if (rc >= 0) return rc;
     }

@@ -129,6 +129,7 @@ struct PrefillArgs {
     const int* context_lens;    // MODE_KVCACHE: cached length per sequence, query tokens included
     const int* block_tables;    // paged K/V: (batch, max_blocks) logical -> physical block
     int paged, block_size, max_blocks;
+    int skip_rows;              // MODE_VARLEN: sequences of at most this many (query token, group head) rows are not this launch's; 0: none
     float scale_log2;
 };
 
@@ -512,6 +513,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     const int stream_id = (int)blockIdx.z * (int)(gridDim.x / a.band) + (int)(blockIdx.x / a.band);
     if (stream_id >= a.kv_heads * a.batch) return;   // the last group may be short
     const SeqExtent sq = seq_extent(a, stream_id / a.kv_heads);
+    if (sq.q_len * group <= a.skip_rows) return;   // the few-row kernel's
     const int num_mb = (sq.q_len + kBlockM - 1) / kBlockM;
     const int kvh = stream_id % a.kv_heads;
     const int b = stream_id / a.kv_heads;
@@ -1426,9 +1428,10 @@ int launch_typed(const AttnParams& p, cudaStream_t stream) {
     }
     const int streams_per_group = (int)(((long long)p.kv_heads * p.num_seqs + groups - 1) / groups);
     dim3 grid(streams_per_group * band, (pairs + band - 1) / band, groups);
+    a.skip_rows = launch_mixed_few_rows(p, stream);
     prefill_tcgen05_kernel<T, D, kMask><<<grid, kThreads, smem, stream>>>(qm, km, vm, om, a);
     const int rc = check_launch("prefill_tcgen05_kernel");
-    if (rc == FLASH_ATTN_OK) note_path("prefill_tcgen05", 1);
+    if (rc == FLASH_ATTN_OK) note_path("prefill_tcgen05", a.skip_rows > 0 ? 2 : 1);
     return rc;
 }
 
