@@ -1,6 +1,6 @@
 """Builds the attention library for sm_100a with nvcc, in-tree (luma_b200/lib/): the static archive
-libflash_attn.a the reference crate links (`static=flash_attn`, luma-flash-attn/build.rs:147-148)
-and libflash_attn.so for ctypes.
+libflash_attn.a the reference crate links (`static=flash_attn`, luma-flash-attn/build.rs:147-148),
+libflash_attn.so for ctypes, and _host.so, the Python front end's native host path.
 
 Mirrors what luma-flash-attn/build.rs:47-253 does for the reference crate — find nvcc
 (CUDA_HOME / CUDA_PATH / CUDA_ROOT, then PATH), compile every kernels translation unit, `ar rcs`
@@ -24,6 +24,7 @@ LIB_DIR = ROOT / "lib"
 LIB_PATH = LIB_DIR / "libflash_attn.so"
 
 ARCHIVE_PATH = LIB_DIR / "libflash_attn.a"
+HOST_PATH = LIB_DIR / "_host.so"   # the Python front end's native host path (csrc/host_fast.cpp)
 
 SOURCES = ["api.cu", "tile_simt.cu", "decode_splitk.cu", "prefill_tcgen05.cu", "kv_append.cu", "softmax_lastdim.cu", "comm.cu", "host_pipe.cu"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -49,6 +50,19 @@ def _stale(target: Path, deps: list[Path]) -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
+def _host_command(src: Path) -> list[str]:
+    """g++ line of the extension module: CPython's and torch's headers, torch's libraries (the front end has torch
+    loaded before it, so they need no run path)."""
+    import importlib.util
+    import sysconfig
+    torch_dir = Path(importlib.util.find_spec("torch").origin).parent
+    cuda = Path(find_nvcc()).resolve().parent.parent
+    includes = [torch_dir / "include", torch_dir / "include" / "torch" / "csrc" / "api" / "include", cuda / "include",
+                Path(sysconfig.get_paths()["include"])]
+    return ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", *[f"-I{p}" for p in includes], str(src), "-o", str(HOST_PATH),
+            f"-L{torch_dir / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+
+
 def build(force: bool = False, verbose: bool = False, trace: bool = False) -> Path:
     nvcc = find_nvcc()
     LIB_DIR.mkdir(exist_ok=True)
@@ -71,7 +85,16 @@ def build(force: bool = False, verbose: bool = False, trace: bool = False) -> Pa
                    *(["-DFA_TRACE"] if trace else []),
                    "-Xptxas", "-v" if verbose else "-O3", "-c", str(src), "-o", str(obj)]
             procs.append((name, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+    host = None
+    host_src = CSRC / "host_fast.cpp"
+    if force or _stale(HOST_PATH, [host_src]):
+        host = subprocess.Popen(_host_command(host_src), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     failed = False
+    if host is not None:
+        out, _ = host.communicate()
+        if host.returncode != 0 or verbose:
+            sys.stderr.write(f"--- g++ {host_src.name} ---\n{out}\n")
+        failed = host.returncode != 0
     for name, proc in procs:
         out, _ = proc.communicate()
         if proc.returncode != 0 or verbose:

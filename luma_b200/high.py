@@ -14,7 +14,7 @@ from typing import Optional
 import torch
 
 from . import error as E
-from . import ffi, low
+from . import ffi, host_path, low
 
 
 def _check_float(t: torch.Tensor, what: str) -> None:
@@ -31,6 +31,10 @@ def flash_attn_func(q, k, v, softmax_scale: Optional[float] = None, causal: bool
     Query token i sits at global position start_pos + i (high.rs:15-52). `return_lse` is this
     library's addition: also returns the fp32 log-sum-exp (B, Hq, Sq).
     """
+    if causal:
+        got = host_path.attn(q, k, v, softmax_scale, start_pos, return_lse)
+        if got is not None:
+            return got
     if not causal:
         raise E.Unsupported("flash_attn_func: non-causal is not supported yet (kernels are causal-only)")
     _check_float(q, "flash_attn_func")
@@ -56,6 +60,10 @@ def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q: in
     """Packed variable-length attention (high.rs:54-109). q (total_q, Hq, d); k, v
     (total_kv, Hkv, d) or, with `block_table` (batch, max_blocks), a paged cache
     (num_blocks, block_size, Hkv, d)."""
+    if causal:
+        o = host_path.varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, softmax_scale, block_table)
+        if o is not None:
+            return o
     if not causal:
         raise E.Unsupported("flash_attn_varlen_func: non-causal is not supported yet (kernels are causal-only)")
     _check_float(q, "flash_attn_varlen_func")
@@ -91,6 +99,9 @@ def flash_attn_with_kvcache(q, k_cache, v_cache, cache_seqlens, block_table,
     """Attention over a paged KV cache (high.rs:111-149). q (B, Sq, Hq, d); caches
     (num_blocks, block_size, Hkv, d); cache_seqlens (B,) i32 including the q tokens; block_table
     (B, max_blocks) i32. Sq == 1 decodes, Sq > 1 is chunked prefill (bottom-right causal)."""
+    o = host_path.kvcache(q, k_cache, v_cache, cache_seqlens, block_table, softmax_scale)
+    if o is not None:
+        return o
     _check_float(q, "flash_attn_with_kvcache")
     if q.dim() != 4 or k_cache.dim() != 4 or v_cache.dim() != 4:
         raise E.InvalidShape("flash_attn_with_kvcache: q and caches must be rank 4")

@@ -10,7 +10,7 @@ from __future__ import annotations
 import torch
 
 from . import error as E
-from . import ffi
+from . import ffi, host_path
 
 _SUFFIX = {torch.float32: "f32", torch.float16: "f16", torch.bfloat16: "bf16"}
 
@@ -72,6 +72,9 @@ def flash_attn(q, k, v, o, batch, q_seq_len, kv_seq_len, q_num_heads, kv_num_hea
     head_size), attn_mask (batch, kv_seq_len) uint8. `lse` (optional f32 buffer of
     batch*q_num_heads*q_seq_len) is this library's additive output.
     """
+    if stream is None and host_path.low_attn(q, k, v, o, batch, q_seq_len, kv_seq_len, q_num_heads, kv_num_heads, head_size,
+                                             start_pos, scale, attn_mask, lse):
+        return
     _validate(q, k, v, o, batch, q_seq_len, kv_seq_len, q_num_heads, kv_num_heads, head_size,
               start_pos, attn_mask)
     sfx = _suffix(q)
@@ -220,6 +223,9 @@ def kvcache_append(k_new, v_new, k_cache, v_cache, block_tables, context_lens, n
     """Writes the K/V rows of the n_new newest tokens of every sequence into their pages
     (`context_lens` = lengths after the append). Additive: the reference leaves this to the caller
     (luma-flash-attn/src/api/high.rs:123-125)."""
+    if stream is None and host_path.append(k_new, v_new, k_cache, v_cache, block_tables, context_lens, num_seqs, n_new, kv_heads,
+                                           head_size, block_size, max_blocks):
+        return
     need = num_seqs * n_new * kv_heads * head_size
     _check_len("k_new", k_new.numel(), need)
     _check_len("v_new", v_new.numel(), need)
@@ -234,6 +240,10 @@ def softmax_last_dim(x, out=None, stream=None):
     """Softmax over the last dimension of a dense device tensor (f32 / f16 / bf16), f32 arithmetic;
     the role of luma-cuda's softmax_<T> kernels (luma-cuda/kernels/nn.cu:21-76, launched from
     luma-cuda/src/ops/nn_provide.rs:10-70) on the math path. `out` may be `x` itself."""
+    if out is None and stream is None:
+        y = host_path.softmax(x)
+        if y is not None:
+            return y
     if not x.is_contiguous():
         raise E.Unsupported("softmax_last_dim: the input must be contiguous (nn_provide.rs:11-13)")
     if out is None:
