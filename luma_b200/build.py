@@ -26,7 +26,7 @@ LIB_PATH = LIB_DIR / "libflash_attn.so"
 ARCHIVE_PATH = LIB_DIR / "libflash_attn.a"
 HOST_PATH = LIB_DIR / "_host.so"   # the Python front end's native host path (csrc/host_fast.cpp)
 
-SOURCES = ["api.cu", "tile_simt.cu", "decode_splitk.cu", "prefill_tcgen05.cu", "kv_append.cu", "softmax_lastdim.cu", "comm.cu", "host_pipe.cu"]
+SOURCES = ["api.cu", "tile_simt.cu", "tile_f32.cu", "decode_splitk.cu", "prefill_tcgen05.cu", "kv_append.cu", "softmax_lastdim.cu", "comm.cu", "host_pipe.cu"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -226,6 +226,8 @@ int dispatch(const AttnParams& p, cudaStream_t stream) {
         if (rc >= 0) return rc;
         rc = launch_prefill_tcgen05(p, stream);
         if (rc >= 0) return rc;
+        rc = launch_tile_f32(p, stream);
+        if (rc >= 0) return rc;
     }
     return launch_tile_simt(p, stream);
 }

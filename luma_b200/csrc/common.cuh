@@ -153,6 +153,7 @@ int check_launch(const char* what);
 // Kernel families. Each returns a flash_attn_status, or -1 when the problem is outside what that
 // family supports (the dispatcher then tries the next one).
 int launch_tile_simt(const AttnParams& p, cudaStream_t stream);
+int launch_tile_f32(const AttnParams& p, cudaStream_t stream);
 int launch_decode_splitk(const AttnParams& p, cudaStream_t stream);
 // The same kernel for a few query rows per sequence through any entry point.
 int launch_few_rows(const AttnParams& p, cudaStream_t stream);
