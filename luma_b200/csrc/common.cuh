@@ -157,9 +157,10 @@ int launch_tile_f32(const AttnParams& p, cudaStream_t stream);
 int launch_decode_splitk(const AttnParams& p, cudaStream_t stream);
 // The same kernel for a few query rows per sequence through any entry point.
 int launch_few_rows(const AttnParams& p, cudaStream_t stream);
-// The same kernel for those sequences of a packed batch that have few query rows (the host does not know which):
-// launched beside the prefill kernel, which leaves out sequences of at most the returned number of rows (query tokens x
-// group); 0 = nothing was launched.
+// The same kernel for those sequences of a packed batch that have few query rows (the host does not know which),
+// launched behind the prefill kernel, which leaves out sequences of at most the number of rows (query tokens x group)
+// that prepare_mixed_few_rows() returns; 0 = not for this call. Once it has returned more, the launch has to follow.
+int prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream);
 int launch_mixed_few_rows(const AttnParams& p, cudaStream_t stream);
 int launch_prefill_tcgen05(const AttnParams& p, cudaStream_t stream);
 int launch_debug_block_slots(const int* block_tables, const int* context_lens, const int* offsets,

@@ -64,6 +64,7 @@ struct RowsArgs {
     int q_heads, kv_heads, block_size, block_shift, max_blocks, paged;   // block_shift: log2 of the page size, -1 where it is no power of two
     int row_blocks;      // blocks of kRows query rows per KV head (blockIdx.x = KV head x row block)
     int max_rows;        // sequences with more query rows than this (per KV head) are not this launch's
+    int behind_prefill;  // launched behind the prefill kernel of the same call, which it does not depend on
     int forced_units;    // > 0: units per column (option "decode_chunk_tokens"); 0: equal shares
     float scale_log2;    // scale * log2(e)
     RowsOut out;
@@ -342,8 +343,12 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
     // Launched with programmatic stream serialisation: the grid may be set up while the kernel before it
     // drains, and touches nothing in global memory before that kernel has finished (returns at once
     // when the launch carries no programmatic dependency). The next kernel may be set up likewise.
+    // Behind a prefill kernel (packed mixed batch) it starts when that kernel's last CTAs have started and fills
+    // the SMs that they leave: what both read was written before the prefill kernel began. Every CTA then waits at
+    // its end instead, so that this grid's completion stands for both.
+    const bool behind = a.behind_prefill != 0;
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    if (!behind) asm volatile("griddepcontrol.wait;\n" ::: "memory");
 
     // KV heads vary fastest across the grid: the CTAs that read the adjacent 256-byte slices of the
     // same token rows (one slice per KV head) are launched together, which keeps DRAM pages open.
@@ -364,7 +369,10 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
         const Cut cut(total, (unsigned)columns, (unsigned)a.forced_units);
         u_begin = cut.first(column);
         u_end = min(total, cut.first(column + 1));
-        if (column >= columns || u_begin >= u_end) return;   // fewer units than columns
+        if (column >= columns || u_begin >= u_end) {   // fewer units than columns
+            if (behind) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+            return;
+        }
         s = (int)(u_begin / per);
         seq_first = per * (unsigned)s;
     } else {
@@ -393,7 +401,10 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
         const Cut cut(total, (unsigned)columns, (unsigned)a.forced_units);
         u_begin = cut.first(column);
         u_end = min(total, cut.first(column + 1));
-        if (column >= columns || u_begin >= u_end) return;   // fewer units than columns
+        if (column >= columns || u_begin >= u_end) {   // fewer units than columns
+            if (behind) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+            return;
+        }
         if (s0 > 0) s0 = 0;          // more than 128 sequences: walk them again from the start
         else s0 = -1;
         for (;;) {
@@ -753,6 +764,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
         }
     }
     cp_async_wait<0>();
+    if (behind) asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 
 // The grid: one CTA per KV head (x row block) and column, as many columns as fill the device's CTA slots in
@@ -782,14 +794,14 @@ struct RowsPlan {
     size_t partial_bytes, counter_bytes, acc_bytes;
 };
 
-// `rows`: query rows per KV head at most; `max_tokens`: upper bound of a sequence's visible keys.
+// `rows`: query rows per KV head at most; `max_tokens`: upper bound of a sequence's visible keys; `waves`: CTAs per slot.
 template <int D>
-RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, bool allow_forced) {
+RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, int waves, bool allow_forced) {
     RowsPlan r{};
     r.row_blocks = (rows + kRows - 1) / kRows;
     const long long per_column = (long long)kv_heads * r.row_blocks;
     if (per_column > 0x7fffffffLL) return r;   // columns == 0: not this kernel's
-    r.columns = num_columns((int)per_column, Smem<D>::kCtasPerSm, sm_count());
+    r.columns = num_columns((int)per_column, Smem<D>::kCtasPerSm, sm_count()) * waves;
     const long long most_units = (long long)num_seqs * std::max(1LL, (max_tokens + kUnit - 1) / kUnit);
     if (allow_forced && get_option_decode_chunk() > 0) {
         r.forced_units = (get_option_decode_chunk() + kUnit - 1) / kUnit;
@@ -841,11 +853,16 @@ int log2_or_minus1(int v) {
     return -1;
 }
 
+// What a call does: a launch of its own; or, behind a prefill kernel, first whatever can fail (the plan and its
+// workspace, before that kernel is launched) and then the launch.
+enum class Step { kAlone, kPrepare, kBehindPrefill };
+
 template <typename T, int D>
-int launch_typed(const AttnParams& p, int rows, int max_rows, cudaStream_t stream) {
+int launch_typed(const AttnParams& p, int rows, int max_rows, Step step, cudaStream_t stream) {
     const long long max_tokens = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
     if (max_tokens <= 0) return -1;
-    const RowsPlan plan = plan_rows<D>(p.num_seqs, p.kv_heads, rows, max_tokens, true);
+    // Behind a prefill kernel the CTA slots come free one after the other: smaller shares, three per slot, level that out.
+    const RowsPlan plan = plan_rows<D>(p.num_seqs, p.kv_heads, rows, max_tokens, step == Step::kAlone ? 1 : 3, true);
     if (plan.columns <= 0) return -1;
 
     unsigned* arrived = nullptr;
@@ -855,8 +872,10 @@ int launch_typed(const AttnParams& p, int rows, int max_rows, cudaStream_t strea
                         plan.partial_bytes + plan.counter_bytes);
         return FLASH_ATTN_ERR_CUDA;
     }
+    if (step == Step::kPrepare) return FLASH_ATTN_OK;
 
     RowsArgs a{};
+    a.behind_prefill = step == Step::kBehindPrefill ? 1 : 0;
     a.q = p.q; a.k = p.k; a.v = p.v;
     a.block_tables = p.block_tables;
     a.context_lens = p.context_lens;
@@ -910,15 +929,15 @@ bool rows_kernel_takes(const AttnParams& p) {
     return (qo & 3) == 0;
 }
 
-int launch_rows_typed(const AttnParams& p, int rows, int max_rows, cudaStream_t stream) {
+int launch_rows_typed(const AttnParams& p, int rows, int max_rows, Step step, cudaStream_t stream) {
     if (p.dtype == DT_BF16) {
-        return p.head_size == 128 ? launch_typed<__nv_bfloat16, 128>(p, rows, max_rows, stream)
-               : p.head_size == 64 ? launch_typed<__nv_bfloat16, 64>(p, rows, max_rows, stream)
-                                   : launch_typed<__nv_bfloat16, 32>(p, rows, max_rows, stream);
+        return p.head_size == 128 ? launch_typed<__nv_bfloat16, 128>(p, rows, max_rows, step, stream)
+               : p.head_size == 64 ? launch_typed<__nv_bfloat16, 64>(p, rows, max_rows, step, stream)
+                                   : launch_typed<__nv_bfloat16, 32>(p, rows, max_rows, step, stream);
     }
-    return p.head_size == 128 ? launch_typed<__half, 128>(p, rows, max_rows, stream)
-           : p.head_size == 64 ? launch_typed<__half, 64>(p, rows, max_rows, stream)
-                               : launch_typed<__half, 32>(p, rows, max_rows, stream);
+    return p.head_size == 128 ? launch_typed<__half, 128>(p, rows, max_rows, step, stream)
+           : p.head_size == 64 ? launch_typed<__half, 64>(p, rows, max_rows, step, stream)
+                               : launch_typed<__half, 32>(p, rows, max_rows, step, stream);
 }
 
 }  // namespace
@@ -926,7 +945,7 @@ int launch_rows_typed(const AttnParams& p, int rows, int max_rows, cudaStream_t 
 int launch_decode_splitk(const AttnParams& p, cudaStream_t stream) {
     if (p.mode != MODE_KVCACHE || p.q_seq_len != 1 || !rows_kernel_takes(p)) return -1;
     const int rows = p.q_heads / p.kv_heads;
-    return launch_rows_typed(p, rows, rows, stream);
+    return launch_rows_typed(p, rows, rows, Step::kAlone, stream);
 }
 
 // Whether few query rows (per KV head) over a range of `keys` are better off here than on the tensor-core prefill
@@ -947,15 +966,20 @@ int launch_few_rows(const AttnParams& p, cudaStream_t stream) {
     // up to four row blocks: each reads the K/V rows again, from L2 (28 rows of 7 x 1355-5421 keys: 43 us against
     // 87 on the prefill kernel; 32 rows of 8 x 3108: 45 against 109)
     if (rows > 4 * kRows || !worth_cutting(p, rows)) return -1;
-    return launch_rows_typed(p, (int)rows, (int)rows, stream);
+    return launch_rows_typed(p, (int)rows, (int)rows, Step::kAlone, stream);
 }
 
-int launch_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {
+int prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {
     if (p.mode != MODE_VARLEN || p.num_seqs < 2 || p.n_out > 0 || !rows_kernel_takes(p)) return 0;
     const int group = p.q_heads / p.kv_heads;
     // one row block: the CTA slots are shared out before anybody knows how many rows the sequences have
-    if (group > kRows || !worth_cutting(p, kRows)) return 0;
-    return launch_rows_typed(p, kRows, kRows, stream) == FLASH_ATTN_OK ? kRows : 0;
+    // prompts packed back to back with their own K/V: few rows would see few keys
+    if (group > kRows || !worth_cutting(p, kRows) || (!p.paged && p.kv_seq_len <= p.q_seq_len)) return 0;
+    return launch_rows_typed(p, kRows, kRows, Step::kPrepare, stream) == FLASH_ATTN_OK ? kRows : 0;
+}
+
+int launch_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {
+    return launch_rows_typed(p, kRows, kRows, Step::kBehindPrefill, stream);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1038,7 +1062,7 @@ int launch_static(const void* q, const void* k, const void* v, void* o, const in
     // Within that limit the counters (one per sequence and row block of a KV head, at most one per row)
     // fit their part of the array; the partials are bounded by the device's CTA slots, not by the call
     // (two waves of 2 x 148 CTAs at head size 128: 9.8 MB).
-    RowsPlan plan = plan_rows<D>(num_seqs, kv_heads, group, max_tokens, false);
+    RowsPlan plan = plan_rows<D>(num_seqs, kv_heads, group, max_tokens, 1, false);
     while (plan.columns > 1 && plan.partial_bytes > kStaticScratchBytes - kStaticCounterBytes) {
         const size_t per = plan.partial_bytes / plan.columns;
         --plan.columns;

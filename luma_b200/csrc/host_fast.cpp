@@ -27,6 +27,8 @@ using BatchFn = int (*)(const void*, const void*, const void*, void*, int, int, 
 using BatchLseFn = int (*)(const void*, const void*, const void*, void*, float*, int, int, int, int, int, int, int, float, const uint8_t*, void*);
 using VarlenFn = int (*)(const void*, const void*, const void*, void*, const int*, const int*, const int*, int, int, int, int, int, int,
                          int, int, int, float, void*);
+using VarlenTotalFn = int (*)(const void*, const void*, const void*, void*, const int*, const int*, const int*, int, int, int, int, int, int,
+                         int, int, int, float, int, int, void*);
 using KvFn = int (*)(const void*, const void*, const void*, void*, const int*, const int*, int, int, int, int, int, int, int, float, void*);
 using AppendFn = int (*)(const void*, const void*, void*, void*, const int*, const int*, int, int, int, int, int, int, int, void*);
 using SoftmaxFn = int (*)(const void*, void*, long long, int, void*);
@@ -36,6 +38,7 @@ struct Library {
     BatchFn batch[3];
     BatchLseFn batch_lse[3];
     VarlenFn varlen[3];
+    VarlenTotalFn varlen_total[2];   // f16, bf16: with the row counts of the packed buffers
     KvFn kv[3];
     AppendFn append;
     SoftmaxFn softmax[3];
@@ -195,9 +198,17 @@ PyObject* varlen(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Tensor o = at::empty_like(*q);
     void* st = stream_of(dev);
     int code;
-    WITHOUT_GIL(code = lib.varlen[ti](q->const_data_ptr(), k->const_data_ptr(), v->const_data_ptr(), o.data_ptr(), cu_q->const_data_ptr<int>(),
-                                      cu_k->const_data_ptr<int>(), table != nullptr ? table->const_data_ptr<int>() : nullptr, (int)num_seqs, max_q,
-                                      max_k, (int)hq, (int)hkv, (int)d, (int)block_size, (int)max_blocks, table != nullptr ? 1 : 0, scale, st));
+    const int* tab = table != nullptr ? table->const_data_ptr<int>() : nullptr;
+    const int paged = table != nullptr ? 1 : 0;
+    if (ti > 0 && q->size(0) <= INT32_MAX && (paged || k->size(0) <= INT32_MAX)) {
+        WITHOUT_GIL(code = lib.varlen_total[ti - 1](q->const_data_ptr(), k->const_data_ptr(), v->const_data_ptr(), o.data_ptr(), cu_q->const_data_ptr<int>(),
+                                                    cu_k->const_data_ptr<int>(), tab, (int)num_seqs, max_q, max_k, (int)hq, (int)hkv, (int)d, (int)block_size,
+                                                    (int)max_blocks, paged, scale, (int)q->size(0), paged ? 0 : (int)k->size(0), st));
+    } else {
+        WITHOUT_GIL(code = lib.varlen[ti](q->const_data_ptr(), k->const_data_ptr(), v->const_data_ptr(), o.data_ptr(), cu_q->const_data_ptr<int>(),
+                                          cu_k->const_data_ptr<int>(), tab, (int)num_seqs, max_q, max_k, (int)hq, (int)hkv, (int)d, (int)block_size,
+                                          (int)max_blocks, paged, scale, st));
+    }
     return finish(code, code == 0 ? THPVariable_Wrap(std::move(o)) : nullptr);
 }
 

@@ -27,7 +27,8 @@ _loader.exec_module(_native)
 
 def _addresses():
     names = ([f"flash_attn_{s}" for s in ffi.DTYPE_SUFFIX] + [f"flash_attn_{s}_lse" for s in ffi.DTYPE_SUFFIX]
-             + [f"flash_attn_varlen_{s}" for s in ffi.DTYPE_SUFFIX] + [f"flash_attn_with_kvcache_{s}" for s in ffi.DTYPE_SUFFIX]
+             + [f"flash_attn_varlen_{s}" for s in ffi.DTYPE_SUFFIX]
+             + ["flash_attn_varlen_f16_total", "flash_attn_varlen_bf16_total"] + [f"flash_attn_with_kvcache_{s}" for s in ffi.DTYPE_SUFFIX]
              + ["flash_attn_kvcache_append"] + [f"luma_softmax_{s}" for s in ffi.DTYPE_SUFFIX] + ["flash_attn_last_error"])
     return tuple(ctypes.cast(getattr(ffi.lib, n), ctypes.c_void_p).value for n in names)
 
