@@ -12,10 +12,17 @@ namespace fa {
 namespace {
 
 template <int ELEM_BYTES>
-__global__ void kv_append_kernel(const unsigned char* __restrict__ k_new, const unsigned char* __restrict__ v_new,
-                                 unsigned char* __restrict__ k_cache, unsigned char* __restrict__ v_cache,
-                                 const int* __restrict__ block_tables, const int* __restrict__ context_lens,
+__global__ void kv_append_kernel(const unsigned char* k_new, const unsigned char* v_new,
+                                 unsigned char* k_cache, unsigned char* v_cache,
+                                 const int* block_tables, const int* context_lens,
                                  int n_new, int row_elems, int block_size, int max_blocks) {
+    // Launched with programmatic stream serialisation, on both sides: its blocks are set up while the kernel before it
+    // drains, and the attention kernel that follows may be set up while it runs (and waits for its end before
+    // it reads anything). The trigger stands behind the wait: before it, the attention kernel's CTAs came in while the last step's
+    // were still leaving, and 16 sequences x 4 tokens took 68.7 us a step. So 65.8, with ordinary launches 67.4; one
+    // sequence of 777 tokens 9.8 against 12.3.
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     const int s = blockIdx.y;
     const int t = blockIdx.x;                       // new token index within the sequence
     const int L = context_lens[s];                  // length AFTER the append
@@ -44,19 +51,18 @@ int launch_kv_append(int elem_bytes, const void* k_new, const void* v_new, void*
         return FLASH_ATTN_ERR_INVALID_SHAPE;
     }
     const int row_elems = kv_heads * head_size;
-    const int threads = 128;
-    dim3 grid(n_new, num_seqs);
-    if (elem_bytes == 4) {
-        kv_append_kernel<4><<<grid, threads, 0, stream>>>(
-            static_cast<const unsigned char*>(k_new), static_cast<const unsigned char*>(v_new),
-            static_cast<unsigned char*>(k_cache), static_cast<unsigned char*>(v_cache), block_tables, context_lens, n_new,
-            row_elems, block_size, max_blocks);
-    } else {
-        kv_append_kernel<2><<<grid, threads, 0, stream>>>(
-            static_cast<const unsigned char*>(k_new), static_cast<const unsigned char*>(v_new),
-            static_cast<unsigned char*>(k_cache), static_cast<unsigned char*>(v_cache), block_tables, context_lens, n_new,
-            row_elems, block_size, max_blocks);
-    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)n_new, (unsigned)num_seqs);
+    cfg.blockDim = dim3(128);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, elem_bytes == 4 ? kv_append_kernel<4> : kv_append_kernel<2>, static_cast<const unsigned char*>(k_new),
+                       static_cast<const unsigned char*>(v_new), static_cast<unsigned char*>(k_cache), static_cast<unsigned char*>(v_cache),
+                       block_tables, context_lens, n_new, row_elems, block_size, max_blocks);
     const int rc = check_launch("kv_append_kernel");
     if (rc == FLASH_ATTN_OK) note_path("kv_append", 1);
     return rc;
