@@ -77,3 +77,33 @@ def test_packed_and_chunked(bs):
     torch.cuda.synchronize()
     assert ffi.last_path() == "tile_f32"
     _close(o.cpu().numpy(), want, f"packed, page {bs}")
+
+
+@pytest.mark.parametrize("d,sq", [(32, 40), (64, 70), (128, 33)])
+@pytest.mark.parametrize("what", ["k -inf", "k inf", "v inf", "v nan", "q nan", "k large", "v large"])
+def test_values_that_do_not_split(d, sq, what):
+    """Infinities, NaN and values that round to a bf16 infinity: what the scalar kernel gives, row by row (a row that does
+    not see the value is not touched by it)."""
+    b, hq, hkv, at = 2, 4, 2, 21
+    q, k, v = H.normal((b, sq, hq, d), 11), H.normal((b, sq, hkv, d), 12), H.normal((b, sq, hkv, d), 13)
+    x = {"q": q, "k": k, "v": v}[what[0]]
+    x[1, at, 0, 3] = {"-inf": -np.inf, "inf": np.inf, "nan": np.nan, "large": 3.4e38}[what.split()[1]]
+    if what == "k -inf":
+        q[1, :, :, 3] = np.abs(q[1, :, :, 3]) + 0.1      # the scores are -inf: the key has no weight
+
+    def call():
+        o, lse = torch.full((b, sq, hq, d), 7.0, device="cuda"), torch.full((b, hq, sq), 7.0, device="cuda")
+        low.flash_attn(H.to_dev(q, "f32"), H.to_dev(k, "f32"), H.to_dev(v, "f32"), o, b, sq, sq, hq, hkv, d, 0, 1.0 / np.sqrt(d), None, None, lse)
+        torch.cuda.synchronize()
+        return o.cpu().numpy(), lse.cpu().numpy(), ffi.last_path()
+
+    o, lse, path = call()
+    ffi.lib.flash_attn_set_option(b"force_generic", 1)
+    try:
+        want, lse_want, generic = call()
+    finally:
+        ffi.lib.flash_attn_set_option(b"force_generic", 0)
+    assert (path, generic) == ("tile_f32", "tile_simt")
+    np.testing.assert_allclose(o, want, rtol=1e-4, atol=TOL)          # NaN and infinities in the same places
+    np.testing.assert_allclose(lse, lse_want, rtol=1e-4, atol=TOL)
+    assert np.isfinite(o[1, :at]).all() and np.isfinite(o[0]).all()
