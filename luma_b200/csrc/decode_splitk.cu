@@ -794,14 +794,14 @@ struct RowsPlan {
     size_t partial_bytes, counter_bytes, acc_bytes;
 };
 
-// `rows`: query rows per KV head at most; `max_tokens`: upper bound of a sequence's visible keys; `waves`: CTAs per slot.
+// `rows`: query rows per KV head at most; `max_tokens`: upper bound of a sequence's visible keys.
 template <int D>
-RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, int waves, bool allow_forced) {
+RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, bool allow_forced) {
     RowsPlan r{};
     r.row_blocks = (rows + kRows - 1) / kRows;
     const long long per_column = (long long)kv_heads * r.row_blocks;
     if (per_column > 0x7fffffffLL) return r;   // columns == 0: not this kernel's
-    r.columns = num_columns((int)per_column, Smem<D>::kCtasPerSm, sm_count()) * waves;
+    r.columns = num_columns((int)per_column, Smem<D>::kCtasPerSm, sm_count());
     const long long most_units = (long long)num_seqs * std::max(1LL, (max_tokens + kUnit - 1) / kUnit);
     if (allow_forced && get_option_decode_chunk() > 0) {
         r.forced_units = (get_option_decode_chunk() + kUnit - 1) / kUnit;
@@ -861,8 +861,9 @@ template <typename T, int D>
 int launch_typed(const AttnParams& p, int rows, int max_rows, Step step, cudaStream_t stream) {
     const long long max_tokens = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
     if (max_tokens <= 0) return -1;
-    // Behind a prefill kernel the CTA slots come free one after the other: smaller shares, three per slot, level that out.
-    const RowsPlan plan = plan_rows<D>(p.num_seqs, p.kv_heads, rows, max_tokens, step == Step::kAlone ? 1 : 3, true);
+    // (behind a prefill kernel, whose SMs come free one after the other, smaller shares were no faster: 4 chunks of 512 with 32
+    // decoding sequences 248-252 us with one share per CTA slot, 256 with two, 253-257 with three)
+    const RowsPlan plan = plan_rows<D>(p.num_seqs, p.kv_heads, rows, max_tokens, true);
     if (plan.columns <= 0) return -1;
 
     unsigned* arrived = nullptr;
@@ -1062,7 +1063,7 @@ int launch_static(const void* q, const void* k, const void* v, void* o, const in
     // Within that limit the counters (one per sequence and row block of a KV head, at most one per row)
     // fit their part of the array; the partials are bounded by the device's CTA slots, not by the call
     // (two waves of 2 x 148 CTAs at head size 128: 9.8 MB).
-    RowsPlan plan = plan_rows<D>(num_seqs, kv_heads, group, max_tokens, 1, false);
+    RowsPlan plan = plan_rows<D>(num_seqs, kv_heads, group, max_tokens, false);
     while (plan.columns > 1 && plan.partial_bytes > kStaticScratchBytes - kStaticCounterBytes) {
         const size_t per = plan.partial_bytes / plan.columns;
         --plan.columns;
