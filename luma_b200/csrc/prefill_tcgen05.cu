@@ -119,8 +119,8 @@ struct PrefillArgs {
     // first spread_w rows of the grid are every spread_m-th band (a first wave that mixes all weights,
     // so that CTAs end at spread-out times from the start), the other bands follow heaviest first.
     int spread_w, spread_m;
-    // kOrdered instantiations: the CTA finds its tile pair on the device (find_item); pairs: tile pairs per (sequence, KV head) at most.
-    int pairs;
+    // Paged calls: ordered != 0: the CTA finds its tile pair on the device (find_item); pairs: tile pairs per (sequence, KV head) at most.
+    int ordered, pairs;
     // which entry point the problem came from (fa::Mode) and its per-sequence descriptors
     int mode;                   // MODE_BATCH: uniform q_seq_len / kv_seq_len / start_pos
     const void* q;              // MODE_VARLEN: the packed q / k / v buffers themselves, for the tiles at their very end
@@ -537,35 +537,36 @@ __device__ __forceinline__ int3 find_item(const PrefillArgs& a, int group, int i
     return make_int3(__shfl_sync(0xffffffffu, s, owner), __shfl_sync(0xffffffffu, kvh, owner), __shfl_sync(0xffffffffu, pair, owner));
 }
 
-// One K or V tile (128 keys x D dims, D / 64 halves of 64 columns), tile index j, requested by one whole warp.
+// One K or V tile (128 keys x D dims, D / 64 halves of 64 columns), tile index j.
 //   contiguous: boxes of 128 rows starting at the sequence's row kv_crow + 128 j;
-//   paged     : one box per page and half (block_size rows); lane i holds the tile's page i (page_of_lane) and requests
-//               it. Pages past the sequence's last one are requested at block -1, which is out of range for the
+//   paged     : one box per page and half (block_size rows), requested by one whole warp; lane i holds the tile's page i
+//               (page_of_lane) and requests it. Pages past the sequence's last one are requested at block -1, which is out of range for the
 //               tensor map and therefore arrives as zeros.
 // A paged tile is 16 copies at a page of 16 tokens: the lanes look their pages up before the ring stage is free, so
 // that the request follows the release at once. Looked up and requested page by page by one thread after the release,
 // a tile came about a thousand clocks later, which the two-stage rings do not hide: 4 chunks of 512 over 1024-8192 tokens
 // (page 16) took 167 us a step, 161 so.
 __device__ __forceinline__ int page_of_lane(const PrefillArgs& a, int kv_len, int s, int j, int lane) {
-    if (!a.paged) return -1;
     const int per_tile = kBlockN / a.block_size;
     const int pg = j * per_tile + lane;
     return lane < per_tile && pg < (kv_len + a.block_size - 1) / a.block_size ? a.block_tables[(long long)s * a.max_blocks + pg] : -1;
 }
 
-template <int D>
+// Contiguous K/V: called by one lane.
+template <int D, bool kPaged>
 __device__ __forceinline__ void load_kv_tile(const PrefillArgs& a, const SeqExtent& sq, int kvh, unsigned char* dst,
                                              const CUtensorMap* map, unsigned long long* bar, int j, int page, int lane) {
-    if (lane == 0) mbar_expect_tx(bar, TileBytes<D>::value);
-    __syncwarp();
-    if (a.paged) {
-        if (lane < kBlockN / a.block_size) {
-            tma_load_4d(dst + lane * a.block_size * 128, map, bar, 0, kvh, 0, page);
-            if (D == 128) tma_load_4d(dst + kHalfBytes + lane * a.block_size * 128, map, bar, 64, kvh, 0, page);
-        }
-    } else if (lane == 0) {
+    if (!kPaged) {
+        mbar_expect_tx(bar, TileBytes<D>::value);
         tma_load_4d(dst, map, bar, 0, kvh, sq.kv_crow + j * kBlockN, sq.kv_cb);
         if (D == 128) tma_load_4d(dst + kHalfBytes, map, bar, 64, kvh, sq.kv_crow + j * kBlockN, sq.kv_cb);
+        return;
+    }
+    if (lane == 0) mbar_expect_tx(bar, TileBytes<D>::value);
+    __syncwarp();
+    if (lane < kBlockN / a.block_size) {
+        tma_load_4d(dst + lane * a.block_size * 128, map, bar, 0, kvh, 0, page);
+        if (D == 128) tma_load_4d(dst + kHalfBytes + lane * a.block_size * 128, map, bar, 64, kvh, 0, page);
     }
     __syncwarp();
 }
@@ -597,9 +598,9 @@ __device__ __forceinline__ void edge_tile_copy(unsigned char* dst, const void* b
 
 // kMask: the call carries a key-padding mask (a separate instantiation, so that calls without one
 // pay nothing for it in the softmax loop)
-// kOrdered: sequences of different lengths, launched heaviest first (see find_item; a separate instantiation as well:
-// its code in the batched calls' kernel cost those 2-3 %)
-template <typename T, int D, bool kMask, bool kOrdered>
+// kPaged: paged K/V, whose tiles are gathered page by page and whose tile pairs may be ordered on the device (a separate instantiation as
+// well: the code of the two in the contiguous calls' kernel cost those 2-3 %)
+template <typename T, int D, bool kMask, bool kPaged>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                        const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap o_map, const PrefillArgs a) {
@@ -617,7 +618,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     // A few-row kernel launched behind this one may start once every CTA here has: it fills the SMs that run out of tile pairs.
     if (a.skip_rows > 0) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     int b, kvh, pair;
-    if (kOrdered) {
+    if (kPaged && a.ordered) {
         if (warp == kLoadWarp) {
             const int3 item = find_item(a, group, (int)blockIdx.x, lane);
             if (lane == 0) { sm.item[0] = item.x; sm.item[1] = item.y; sm.item[2] = item.z; }
@@ -659,10 +660,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     const long long tot_k = (packed && !a.paged) ? (long long)a.cu_k[a.batch] : 0;
     auto q_edge = [&](const TileInfo& ti) { return packed && ti.valid && (long long)sq.q_crow + ti.row0 + kBlockM > tot_q; };
     auto kv_edge = [&](int j) { return packed && !a.paged && (long long)sq.kv_crow + (long long)(j + 1) * kBlockN > tot_k; };
-    if (warp == kLoadWarp) {
+    if (warp == kLoadWarp && (kPaged || lane == 0)) {
         int pages[kStages];   // of the tiles requested here, looked up together
 #pragma unroll
-        for (int j = 0; j < kStages; ++j) pages[j] = j < n_pre ? page_of_lane(a, sq.kv_len, b, j, lane) : -1;
+        for (int j = 0; j < kStages; ++j) pages[j] = kPaged && j < n_pre ? page_of_lane(a, sq.kv_len, b, j, lane) : -1;
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];\n" ::"l"(&q_map) : "memory");
             asm volatile("prefetch.tensormap [%0];\n" ::"l"(&k_map) : "memory");
@@ -688,9 +689,9 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         }
-        __syncwarp();
+        if (kPaged) __syncwarp();
         auto load_q = [&](const TileInfo& ti, int t) {
-            if (lane != 0 || !ti.valid || q_edge(ti)) return;
+            if ((kPaged && lane != 0) || !ti.valid || q_edge(ti)) return;
             mbar_expect_tx(&sm.q_full[t], TileBytes<D>::value);
             tma_load_4d(sm.q[t], &q_map, &sm.q_full[t], 0, ti.head, sq.q_crow + ti.row0, sq.q_cb);
             if (D == 128) tma_load_4d(sm.q[t] + kHalfBytes, &q_map, &sm.q_full[t], 64, ti.head, sq.q_crow + ti.row0, sq.q_cb);
@@ -698,7 +699,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         load_q(t0, 0);
 #pragma unroll
         for (int j = 0; j < kStages; ++j) {
-            if (j < n_pre && !kv_edge(j) && a.test_skip_k != j + 1) load_kv_tile<D>(a, sq, kvh, sm.k[j], &k_map, &sm.k_full[j], j, pages[j], lane);
+            if (j < n_pre && !kv_edge(j) && a.test_skip_k != j + 1) load_kv_tile<D, kPaged>(a, sq, kvh, sm.k[j], &k_map, &sm.k_full[j], j, pages[j], lane);
             if (j == 0) load_q(t1, 1);
         }
         // the V tiles come from a producer thread of their own (warp kLoadWarpV), after the set-up barrier
@@ -761,7 +762,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             int issued = is_v ? 0 : n_pre;   // K tiles 0 .. n_pre-1 were issued during set-up
             for (int j = issued; j < n_max && alive; ++j) {
                 const int s = j % n_stages;
-                const int page = page_of_lane(a, sq.kv_len, b, j, lane);
+                const int page = kPaged ? page_of_lane(a, sq.kv_len, b, j, lane) : -1;
                 if (j >= n_stages) {
                     alive = __all_sync(0xffffffffu, mbar_wait(sm, &empty[s], ((unsigned)(j / n_stages) & 1u) ^ 1u, a, is_v ? 2 : 1));
                     if (!alive) break;
@@ -772,8 +773,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     // test hook: this tile is never requested, the issuer's wait for it runs out
                 } else if (kv_edge(j)) {
                     edge_tile_copy<D>(ring[s], kv_base, a.kv_heads, kvh, (long long)sq.kv_crow + (long long)j * kBlockN, tot_k, bar, lane, a.d_real);
-                } else {
-                    load_kv_tile<D>(a, sq, kvh, ring[s], map, bar, j, page, lane);
+                } else if (kPaged || lane == 0) {
+                    load_kv_tile<D, kPaged>(a, sq, kvh, ring[s], map, bar, j, page, lane);
                 }
                 issued = j + 1;
                 if (fix) {
@@ -1409,7 +1410,7 @@ unsigned char* debug_area() {
 }
 #endif
 
-template <typename T, int D, bool kMask, bool kOrdered>
+template <typename T, int D, bool kMask, bool kPaged>
 int launch_variant(const AttnParams& p, cudaStream_t stream) {
     CUtensorMap qm, km, vm, om;
     // packed varlen buffers are one "batch" of total rows
@@ -1492,7 +1493,7 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     const int num_mb = (p.q_seq_len + kBlockM - 1) / kBlockM;
     const int pairs = (group * num_mb + 1) / 2;
     const size_t smem = sizeof(SharedStorage<D>) + 1024;
-    cudaError_t err = cudaFuncSetAttribute(prefill_tcgen05_kernel<T, D, kMask, kOrdered>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = cudaFuncSetAttribute(prefill_tcgen05_kernel<T, D, kMask, kPaged>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) {
         set_last_errorf("prefill_tcgen05_kernel: %s", cudaGetErrorString(err));
         cudaGetLastError();
@@ -1557,7 +1558,13 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     const int streams_per_group = (int)(((long long)p.kv_heads * p.num_seqs + groups - 1) / groups);
     dim3 grid(streams_per_group * band, (pairs + band - 1) / band, groups);
     a.pairs = pairs;
-    if (kOrdered) {
+    // Ordered: chunks of prompts, at most half as long as the context may be. Whole prompts keep grid order, which is heaviest
+    // first for them already: finding the pair costs a CTA about 1 us, and a packed batch of prompts has thousands of short
+    // ones (24 prompts of 17-2000 tokens: 394 us ordered, 376 in grid order).
+    const long long kv_rows = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
+    if (kPaged && p.num_seqs >= 2 && p.num_seqs <= kOrderMax && 2LL * p.q_seq_len <= kv_rows && get_option_prefill_band() <= 0 &&
+        get_option_prefill_groups() <= 0) {
+        a.ordered = 1;
         long long ctas = (long long)p.num_seqs * p.kv_heads * pairs;
         if (p.total_q > 0)   // a sequence of n rows has (group * ceil(n / 128) + 1) / 2 pairs
             ctas = std::min(ctas, p.kv_heads * ((group * (((long long)p.total_q + 127LL * p.num_seqs) / 128) + p.num_seqs) / 2));
@@ -1565,23 +1572,17 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
         grid = dim3((unsigned)ctas);
     }
     a.skip_rows = prepare_mixed_few_rows(p, stream);
-    prefill_tcgen05_kernel<T, D, kMask, kOrdered><<<grid, kThreads, smem, stream>>>(qm, km, vm, om, a);
+    prefill_tcgen05_kernel<T, D, kMask, kPaged><<<grid, kThreads, smem, stream>>>(qm, km, vm, om, a);
     int rc = check_launch("prefill_tcgen05_kernel");
     if (rc == FLASH_ATTN_OK && a.skip_rows > 0) rc = launch_mixed_few_rows(p, stream);
     if (rc == FLASH_ATTN_OK) note_path("prefill_tcgen05", a.skip_rows > 0 ? 2 : 1);
     return rc;
 }
 
-// Ordered: chunks of prompts, at most half as long as the context may be. Whole prompts keep grid order, which is heaviest
-// first for them already: finding the pair costs a CTA about 1 us, and a packed batch of prompts has thousands of short
-// ones (24 prompts of 17-2000 tokens: 394 us ordered, 376 in grid order).
 template <typename T, int D>
 int launch_typed(const AttnParams& p, cudaStream_t stream) {
     if (p.mask != nullptr) return launch_variant<T, D, true, false>(p, stream);
-    const long long kv_rows = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
-    const bool ordered = p.mode != MODE_BATCH && p.num_seqs >= 2 && p.num_seqs <= kOrderMax && 2LL * p.q_seq_len <= kv_rows &&
-                         get_option_prefill_band() <= 0 && get_option_prefill_groups() <= 0;
-    return ordered ? launch_variant<T, D, false, true>(p, stream) : launch_variant<T, D, false, false>(p, stream);
+    return p.paged ? launch_variant<T, D, false, true>(p, stream) : launch_variant<T, D, false, false>(p, stream);
 }
 
 }  // namespace
