@@ -599,7 +599,8 @@ __device__ __forceinline__ void edge_tile_copy(unsigned char* dst, const void* b
 // kMask: the call carries a key-padding mask (a separate instantiation, so that calls without one
 // pay nothing for it in the softmax loop)
 // kPaged: paged K/V, whose tiles are gathered page by page and whose tile pairs may be ordered on the device (a separate instantiation as
-// well: the code of the two in the contiguous calls' kernel cost those 2-3 %)
+// well: with the code of the two in it the contiguous calls' kernel took 375 us for 24 prompts of 17-2000 tokens at d = 64,
+// 364 without; 2 x 8192 GQA 1047 against 1027)
 template <typename T, int D, bool kMask, bool kPaged>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
