@@ -10,6 +10,7 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -66,24 +67,30 @@ int check_launch(const char* what) {
     return FLASH_ATTN_OK;
 }
 
-// ---- decode split-K workspace: one buffer per (device, stream) ---------------------------
+// ---- split-K workspace: one buffer per (device, stream) -----------------------------------
 // Allocation and release are stream-ordered (cudaMallocAsync / cudaFreeAsync on the stream that
 // uses the buffer): growing a workspace neither takes a device-wide synchronisation nor frees
-// memory under work that still reads it. The table is bounded: beyond kMaxWorkspaces entries the
+// memory under work that still reads it. Stream order alone does not protect a call that has the
+// address and has not launched yet, so a buffer belongs to one call from the look-up until its kernels are in the
+// stream (Workspace holds the entry's mutex): another host thread on the same stream waits for that long, and an
+// entry in use is never the one that is released. The table is bounded: beyond kMaxWorkspaces entries the
 // least recently used one is released, so a program that keeps creating streams does not keep
 // one buffer per stream it ever had (a stream handle that is destroyed and handed out again simply
 // finds a scratch buffer that nobody else uses).
-namespace {
 struct WsEntry {
+    std::mutex in_use;            // held by the call that works with the buffer
     int dev = -1;
     cudaStream_t stream = nullptr;
     void* ptr = nullptr;          // the counters, then the partials
     size_t bytes = 0, counters = 0;
-    unsigned long long last_use = 0;
+    unsigned long long last_use = 0;   // under g_ws_mutex
+    bool gone = false;            // taken out of the table (under in_use)
 };
+
+namespace {
 constexpr size_t kMaxWorkspaces = 32;
-std::mutex g_ws_mutex;
-std::vector<WsEntry> g_ws;
+std::mutex g_ws_mutex;            // the table; never waited for while an entry is held
+std::vector<std::shared_ptr<WsEntry>> g_ws;
 unsigned long long g_ws_clock = 0;
 
 void release_entry(WsEntry& e) {
@@ -100,29 +107,54 @@ void release_entry(WsEntry& e) {
     e.ptr = nullptr;
     e.bytes = e.counters = 0;
 }
+
+// The entry of (dev, stream), made where there is none, in the hands of the caller.
+std::shared_ptr<WsEntry> lock_entry(int dev, cudaStream_t stream, std::unique_lock<std::mutex>& held) {
+    for (;;) {
+        std::shared_ptr<WsEntry> e;
+        {
+            std::lock_guard<std::mutex> lock(g_ws_mutex);
+            for (const auto& w : g_ws)
+                if (w->dev == dev && w->stream == stream) e = w;
+            if (e == nullptr) {
+                if (g_ws.size() >= kMaxWorkspaces) {
+                    std::unique_lock<std::mutex> lru_held;
+                    size_t lru = g_ws.size();
+                    for (size_t i = 0; i < g_ws.size(); ++i) {
+                        if (lru < g_ws.size() && g_ws[i]->last_use >= g_ws[lru]->last_use) continue;
+                        std::unique_lock<std::mutex> idle(g_ws[i]->in_use, std::try_to_lock);
+                        if (!idle.owns_lock()) continue;
+                        lru_held = std::move(idle);
+                        lru = i;
+                    }
+                    if (lru < g_ws.size()) {   // (all in use: the table is one longer for a while)
+                        const std::shared_ptr<WsEntry> old = g_ws[lru];
+                        release_entry(*old);
+                        old->gone = true;
+                        g_ws.erase(g_ws.begin() + (long)lru);
+                        lru_held.unlock();
+                    }
+                }
+                e = std::make_shared<WsEntry>();
+                e->dev = dev;
+                e->stream = stream;
+                g_ws.push_back(e);
+            }
+            e->last_use = ++g_ws_clock;
+        }
+        held = std::unique_lock<std::mutex>(e->in_use);
+        if (!e->gone) return e;
+        held.unlock();   // released between the look-up and here: look again
+    }
+}
 }  // namespace
 
-void* decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_bytes, unsigned** counters) {
+Workspace decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_bytes) {
+    Workspace ws;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-    std::lock_guard<std::mutex> lock(g_ws_mutex);
-    WsEntry* e = nullptr;
-    for (WsEntry& w : g_ws)
-        if (w.dev == dev && w.stream == stream) e = &w;
-    if (e == nullptr) {
-        if (g_ws.size() >= kMaxWorkspaces) {
-            size_t lru = 0;
-            for (size_t i = 1; i < g_ws.size(); ++i)
-                if (g_ws[i].last_use < g_ws[lru].last_use) lru = i;
-            release_entry(g_ws[lru]);
-            g_ws.erase(g_ws.begin() + (long)lru);
-        }
-        g_ws.emplace_back();
-        e = &g_ws.back();
-        e->dev = dev;
-        e->stream = stream;
-    }
-    e->last_use = ++g_ws_clock;
+    if (cudaGetDevice(&dev) != cudaSuccess) return ws;
+    std::unique_lock<std::mutex> held;
+    const std::shared_ptr<WsEntry> e = lock_entry(dev, stream, held);
     if (e->ptr == nullptr || e->bytes < e->counters + bytes || e->counters < counter_bytes) {
         const size_t want_counters = std::max({(counter_bytes + 4095) / 4096 * 4096, e->counters, size_t(1) << 16});
         const size_t old = e->bytes > e->counters ? e->bytes - e->counters : 0;
@@ -134,7 +166,7 @@ void* decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_bytes, 
             want = want_counters + bytes;
             if (cudaMallocAsync(&ptr, want, stream) != cudaSuccess) {
                 cudaGetLastError();
-                return nullptr;
+                return ws;
             }
         }
         e->ptr = ptr;
@@ -143,21 +175,29 @@ void* decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_bytes, 
         if (cudaMemsetAsync(ptr, 0, want_counters, stream) != cudaSuccess) {   // once: every launch leaves them at zero again
             cudaGetLastError();
             release_entry(*e);
-            return nullptr;
+            return ws;
         }
     }
-    *counters = static_cast<unsigned*>(e->ptr);
-    return static_cast<unsigned char*>(e->ptr) + e->counters;
+    ws.counters = static_cast<unsigned*>(e->ptr);
+    ws.partials = static_cast<unsigned char*>(e->ptr) + e->counters;
+    ws.entry = e;
+    ws.held = std::move(held);
+    return ws;
 }
 
 int release_workspaces() {
-    std::lock_guard<std::mutex> lock(g_ws_mutex);
-    int n = 0;
-    for (WsEntry& w : g_ws) {
-        if (w.ptr != nullptr) ++n;
-        release_entry(w);
+    std::vector<std::shared_ptr<WsEntry>> all;
+    {
+        std::lock_guard<std::mutex> lock(g_ws_mutex);
+        all.swap(g_ws);
     }
-    g_ws.clear();
+    int n = 0;
+    for (const auto& w : all) {
+        std::lock_guard<std::mutex> held(w->in_use);
+        if (w->ptr != nullptr) ++n;
+        release_entry(*w);
+        w->gone = true;
+    }
     return n;
 }
 

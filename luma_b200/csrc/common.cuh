@@ -8,6 +8,8 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <memory>
+#include <mutex>
 
 #include "../../include/flash_attn.h"
 
@@ -150,6 +152,24 @@ int get_option_prefill_test_skip_k();   // test hook: 1 + index of a K tile the 
 // Returns FLASH_ATTN_OK or FLASH_ATTN_ERR_CUDA (with last error set) after a launch.
 int check_launch(const char* what);
 
+// Split-K scratch of one call: the buffer of its (device, stream), grown on demand, this call's alone until the Workspace goes,
+// which is to be after its launches. partials == nullptr: not to be had. `counters`: at least counter_bytes that
+// are zero at the first use and that every launch leaves at zero.
+struct WsEntry;
+struct Workspace {
+    unsigned char* partials = nullptr;
+    unsigned* counters = nullptr;
+    std::shared_ptr<WsEntry> entry;         // (before `held`: outlives its mutex's lock)
+    std::unique_lock<std::mutex> held;
+};
+Workspace decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_bytes);
+
+// How the split-K kernel runs a call.
+struct RowsPlan {
+    int row_blocks = 0, columns = 0, forced_units = 0;
+    size_t partial_bytes = 0, counter_bytes = 0, acc_bytes = 0;
+};
+
 // Kernel families. Each returns a flash_attn_status, or -1 when the problem is outside what that
 // family supports (the dispatcher then tries the next one).
 int launch_tile_simt(const AttnParams& p, cudaStream_t stream);
@@ -158,10 +178,15 @@ int launch_decode_splitk(const AttnParams& p, cudaStream_t stream);
 // The same kernel for a few query rows per sequence through any entry point.
 int launch_few_rows(const AttnParams& p, cudaStream_t stream);
 // The same kernel for those sequences of a packed batch that have few query rows (the host does not know which),
-// launched behind the prefill kernel, which leaves out sequences of at most the number of rows (query tokens x group)
-// that prepare_mixed_few_rows() returns; 0 = not for this call. Once it has returned more, the launch has to follow.
-int prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream);
-int launch_mixed_few_rows(const AttnParams& p, cudaStream_t stream);
+// launched behind the prefill kernel, which leaves out sequences of at most max_rows rows (query tokens x group).
+// prepare_mixed_few_rows() does what can fail, before that kernel is launched; max_rows == 0: not for this call.
+struct MixedFewRows {
+    int max_rows = 0;
+    RowsPlan plan;
+    Workspace ws;
+};
+MixedFewRows prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream);
+int launch_mixed_few_rows(const AttnParams& p, const MixedFewRows& few, cudaStream_t stream);
 int launch_prefill_tcgen05(const AttnParams& p, cudaStream_t stream);
 int launch_debug_block_slots(const int* block_tables, const int* context_lens, const int* offsets,
                              int num_seqs, int block_size, int max_blocks, int* out_slots,
@@ -180,9 +205,6 @@ int prefill_device_status();
 // to host memory; returns the bytes copied or -1.
 int prefill_debug_read(void* dst, int bytes);
 
-// Split-K scratch of the decode path: one buffer per (device, stream), grown on demand. `counters`: at
-// least counter_bytes that are zero at the first use and that every launch leaves at zero.
-void* decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_bytes, unsigned** counters);
 // Releases every workspace (stream-ordered); returns how many buffers were held.
 int release_workspaces();
 

@@ -789,15 +789,10 @@ int sm_count() {
     return n;
 }
 
-struct RowsPlan {
-    int row_blocks, columns, forced_units;
-    size_t partial_bytes, counter_bytes, acc_bytes;
-};
-
 // `rows`: query rows per KV head at most; `max_tokens`: upper bound of a sequence's visible keys.
 template <int D>
 RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, bool allow_forced) {
-    RowsPlan r{};
+    RowsPlan r;
     r.row_blocks = (rows + kRows - 1) / kRows;
     const long long per_column = (long long)kv_heads * r.row_blocks;
     if (per_column > 0x7fffffffLL) return r;   // columns == 0: not this kernel's
@@ -853,38 +848,36 @@ int log2_or_minus1(int v) {
     return -1;
 }
 
-// What a call does: a launch of its own; or, behind a prefill kernel, first whatever can fail (the plan and its
-// workspace, before that kernel is launched) and then the launch.
-enum class Step { kAlone, kPrepare, kBehindPrefill };
-
-template <typename T, int D>
-int launch_typed(const AttnParams& p, int rows, int max_rows, Step step, cudaStream_t stream) {
+// What can fail before anything is launched: the plan and its workspace. -1: not this kernel's.
+template <int D>
+int prepare_typed(const AttnParams& p, int rows, cudaStream_t stream, RowsPlan& plan, Workspace& ws) {
     const long long max_tokens = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
     if (max_tokens <= 0) return -1;
     // (behind a prefill kernel, whose SMs come free one after the other, smaller shares were no faster: 4 chunks of 512 with 32
     // decoding sequences 248-252 us with one share per CTA slot, 256 with two, 253-257 with three)
-    const RowsPlan plan = plan_rows<D>(p.num_seqs, p.kv_heads, rows, max_tokens, true);
+    plan = plan_rows<D>(p.num_seqs, p.kv_heads, rows, max_tokens, true);
     if (plan.columns <= 0) return -1;
-
-    unsigned* arrived = nullptr;
-    unsigned char* ws = static_cast<unsigned char*>(decode_workspace(stream, plan.partial_bytes, plan.counter_bytes, &arrived));
-    if (ws == nullptr) {
+    ws = decode_workspace(stream, plan.partial_bytes, plan.counter_bytes);
+    if (ws.partials == nullptr) {
         set_last_errorf("flash_attn_with_kvcache: could not allocate %zu bytes of split-K workspace",
                         plan.partial_bytes + plan.counter_bytes);
         return FLASH_ATTN_ERR_CUDA;
     }
-    if (step == Step::kPrepare) return FLASH_ATTN_OK;
+    return FLASH_ATTN_OK;
+}
 
+template <typename T, int D>
+int launch_typed(const AttnParams& p, int max_rows, bool behind_prefill, const RowsPlan& plan, const Workspace& ws, cudaStream_t stream) {
     RowsArgs a{};
-    a.behind_prefill = step == Step::kBehindPrefill ? 1 : 0;
+    a.behind_prefill = behind_prefill ? 1 : 0;
     a.q = p.q; a.k = p.k; a.v = p.v;
     a.block_tables = p.block_tables;
     a.context_lens = p.context_lens;
     a.cu_q = p.cu_q;
     a.cu_k = p.cu_k;
-    a.ws_acc = reinterpret_cast<float*>(ws);
-    a.ws_ml = reinterpret_cast<float2*>(ws + plan.acc_bytes);
-    a.arrived = arrived;
+    a.ws_acc = reinterpret_cast<float*>(ws.partials);
+    a.ws_ml = reinterpret_cast<float2*>(ws.partials + plan.acc_bytes);
+    a.arrived = ws.counters;
     a.mode = p.mode;
     a.num_seqs = p.num_seqs;
     a.q_seq_len = p.q_seq_len;
@@ -930,23 +923,36 @@ bool rows_kernel_takes(const AttnParams& p) {
     return (qo & 3) == 0;
 }
 
-int launch_rows_typed(const AttnParams& p, int rows, int max_rows, Step step, cudaStream_t stream) {
+int prepare_rows(const AttnParams& p, int rows, cudaStream_t stream, RowsPlan& plan, Workspace& ws) {
+    return p.head_size == 128 ? prepare_typed<128>(p, rows, stream, plan, ws)
+           : p.head_size == 64 ? prepare_typed<64>(p, rows, stream, plan, ws)
+                               : prepare_typed<32>(p, rows, stream, plan, ws);
+}
+
+int launch_prepared(const AttnParams& p, int max_rows, bool behind_prefill, const RowsPlan& plan, const Workspace& ws, cudaStream_t stream) {
     if (p.dtype == DT_BF16) {
-        return p.head_size == 128 ? launch_typed<__nv_bfloat16, 128>(p, rows, max_rows, step, stream)
-               : p.head_size == 64 ? launch_typed<__nv_bfloat16, 64>(p, rows, max_rows, step, stream)
-                                   : launch_typed<__nv_bfloat16, 32>(p, rows, max_rows, step, stream);
+        return p.head_size == 128 ? launch_typed<__nv_bfloat16, 128>(p, max_rows, behind_prefill, plan, ws, stream)
+               : p.head_size == 64 ? launch_typed<__nv_bfloat16, 64>(p, max_rows, behind_prefill, plan, ws, stream)
+                                   : launch_typed<__nv_bfloat16, 32>(p, max_rows, behind_prefill, plan, ws, stream);
     }
-    return p.head_size == 128 ? launch_typed<__half, 128>(p, rows, max_rows, step, stream)
-           : p.head_size == 64 ? launch_typed<__half, 64>(p, rows, max_rows, step, stream)
-                               : launch_typed<__half, 32>(p, rows, max_rows, step, stream);
+    return p.head_size == 128 ? launch_typed<__half, 128>(p, max_rows, behind_prefill, plan, ws, stream)
+           : p.head_size == 64 ? launch_typed<__half, 64>(p, max_rows, behind_prefill, plan, ws, stream)
+                               : launch_typed<__half, 32>(p, max_rows, behind_prefill, plan, ws, stream);
+}
+
+// The whole of a call whose sequences have at most `rows` query rows per KV head.
+int run_rows(const AttnParams& p, int rows, cudaStream_t stream) {
+    RowsPlan plan;
+    Workspace ws;
+    const int rc = prepare_rows(p, rows, stream, plan, ws);
+    return rc == FLASH_ATTN_OK ? launch_prepared(p, rows, false, plan, ws, stream) : rc;
 }
 
 }  // namespace
 
 int launch_decode_splitk(const AttnParams& p, cudaStream_t stream) {
     if (p.mode != MODE_KVCACHE || p.q_seq_len != 1 || !rows_kernel_takes(p)) return -1;
-    const int rows = p.q_heads / p.kv_heads;
-    return launch_rows_typed(p, rows, rows, Step::kAlone, stream);
+    return run_rows(p, p.q_heads / p.kv_heads, stream);
 }
 
 // Whether few query rows (per KV head) over a range of `keys` are better off here than on the tensor-core prefill
@@ -967,20 +973,22 @@ int launch_few_rows(const AttnParams& p, cudaStream_t stream) {
     // up to four row blocks: each reads the K/V rows again, from L2 (28 rows of 7 x 1355-5421 keys: 43 us against
     // 87 on the prefill kernel; 32 rows of 8 x 3108: 45 against 109)
     if (rows > 4 * kRows || !worth_cutting(p, rows)) return -1;
-    return launch_rows_typed(p, (int)rows, (int)rows, Step::kAlone, stream);
+    return run_rows(p, (int)rows, stream);
 }
 
-int prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {
-    if (p.mode != MODE_VARLEN || p.num_seqs < 2 || p.n_out > 0 || !rows_kernel_takes(p)) return 0;
+MixedFewRows prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {
+    MixedFewRows few;
+    if (p.mode != MODE_VARLEN || p.num_seqs < 2 || p.n_out > 0 || !rows_kernel_takes(p)) return few;
     const int group = p.q_heads / p.kv_heads;
     // one row block: the CTA slots are shared out before anybody knows how many rows the sequences have
     // prompts packed back to back with their own K/V: few rows would see few keys
-    if (group > kRows || !worth_cutting(p, kRows) || (!p.paged && p.kv_seq_len <= p.q_seq_len)) return 0;
-    return launch_rows_typed(p, kRows, kRows, Step::kPrepare, stream) == FLASH_ATTN_OK ? kRows : 0;
+    if (group > kRows || !worth_cutting(p, kRows) || (!p.paged && p.kv_seq_len <= p.q_seq_len)) return few;
+    if (prepare_rows(p, kRows, stream, few.plan, few.ws) == FLASH_ATTN_OK) few.max_rows = kRows;
+    return few;
 }
 
-int launch_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {
-    return launch_rows_typed(p, kRows, kRows, Step::kBehindPrefill, stream);
+int launch_mixed_few_rows(const AttnParams& p, const MixedFewRows& few, cudaStream_t stream) {
+    return launch_prepared(p, few.max_rows, true, few.plan, few.ws, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

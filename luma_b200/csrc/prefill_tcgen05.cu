@@ -1572,10 +1572,11 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
         if (ctas <= 0 || ctas > 0x7fffffffLL) return -1;
         grid = dim3((unsigned)ctas);
     }
-    a.skip_rows = prepare_mixed_few_rows(p, stream);
+    const MixedFewRows few = prepare_mixed_few_rows(p, stream);   // its workspace is this call's until both kernels are launched
+    a.skip_rows = few.max_rows;
     prefill_tcgen05_kernel<T, D, kMask, kPaged><<<grid, kThreads, smem, stream>>>(qm, km, vm, om, a);
     int rc = check_launch("prefill_tcgen05_kernel");
-    if (rc == FLASH_ATTN_OK && a.skip_rows > 0) rc = launch_mixed_few_rows(p, stream);
+    if (rc == FLASH_ATTN_OK && a.skip_rows > 0) rc = launch_mixed_few_rows(p, few, stream);
     if (rc == FLASH_ATTN_OK) note_path("prefill_tcgen05", a.skip_rows > 0 ? 2 : 1);
     return rc;
 }
