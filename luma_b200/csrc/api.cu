@@ -147,12 +147,161 @@ std::shared_ptr<WsEntry> lock_entry(int dev, cudaStream_t stream, std::unique_lo
         held.unlock();   // released between the look-up and here: look again
     }
 }
+
+// ---- workspaces of captured calls: one per (graph, stream of the capture) -----------------
+// A captured launch may run again at any time, beside anything, after the buffer of its stream has been grown or
+// released; and an allocation made on the capturing stream would belong to that one graph. So a graph gets buffers of its
+// own, allocated outside the capture and kept by the graph itself (a CUDA user object): they come back when the
+// graph and everything instantiated from it are gone, and serve the next capture; at most kMaxIdle wait for one.
+struct GraphBuffer {
+    int dev = -1;
+    unsigned char* ptr = nullptr;      // the counters, then the partials
+    size_t bytes = 0, counters = 0;
+    unsigned long long capture = 0;
+    cudaStream_t stream = nullptr;
+};
+constexpr size_t kMaxIdle = 4;
+
+// Buffers whose graph is gone. The destructor of a user object may run on any thread and must not call CUDA: it leaves the
+// buffer here and somebody else collects it. (Never destroyed: graphs may outlive the library's other statics.)
+struct Retired {
+    std::mutex mutex;
+    std::vector<GraphBuffer*> list;
+    std::atomic<int> count{0};
+};
+Retired& retired() {
+    static Retired* r = new Retired();
+    return *r;
+}
+void CUDART_CB retire(void* buffer) {
+    Retired& r = retired();
+    std::lock_guard<std::mutex> lock(r.mutex);
+    r.list.push_back(static_cast<GraphBuffer*>(buffer));
+    r.count.fetch_add(1, std::memory_order_release);
+}
+
+std::mutex g_graph_mutex;
+std::vector<GraphBuffer*> g_graph_live;   // kept by a graph
+std::vector<GraphBuffer*> g_graph_idle;
+
+// Allocations and synchronisation of a stream that is not captured are allowed to this thread while another stream captures.
+struct OutsideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// A stream of the library's own on the current device, for what must not be in the captured stream.
+cudaStream_t side_stream(int dev) {
+    static cudaStream_t streams[64] = {nullptr};   // under g_graph_mutex
+    if (dev < 0 || dev >= 64) return nullptr;
+    if (streams[dev] == nullptr && cudaStreamCreateWithFlags(&streams[dev], cudaStreamNonBlocking) != cudaSuccess) {
+        cudaGetLastError();
+        streams[dev] = nullptr;
+    }
+    return streams[dev];
+}
+
+void free_graph_buffer(GraphBuffer* b) {   // under g_graph_mutex; nothing uses it any more
+    int cur = -1;
+    cudaGetDevice(&cur);
+    if (cur != b->dev) cudaSetDevice(b->dev);
+    if (cudaFreeAsync(b->ptr, side_stream(b->dev)) != cudaSuccess) cudaGetLastError();
+    if (cur != b->dev && cur >= 0) cudaSetDevice(cur);
+    delete b;
+}
+
+int collect_retired(size_t keep) {   // under g_graph_mutex; returns how many were given back
+    Retired& r = retired();
+    std::vector<GraphBuffer*> got;
+    {
+        std::lock_guard<std::mutex> lock(r.mutex);
+        got.swap(r.list);
+        r.count.store(0, std::memory_order_relaxed);
+    }
+    for (GraphBuffer* b : got) {
+        g_graph_live.erase(std::remove(g_graph_live.begin(), g_graph_live.end(), b), g_graph_live.end());
+        g_graph_idle.push_back(b);
+    }
+    int freed = 0;
+    if (g_graph_idle.size() > keep) {
+        OutsideCapture outside;
+        for (; g_graph_idle.size() > keep; ++freed) {
+            free_graph_buffer(g_graph_idle.front());
+            g_graph_idle.erase(g_graph_idle.begin());
+        }
+    }
+    return freed;
+}
+
+Workspace graph_workspace(cudaStream_t stream, int dev, unsigned long long capture, cudaGraph_t graph, size_t bytes, size_t counter_bytes) {
+    Workspace ws;
+    std::lock_guard<std::mutex> lock(g_graph_mutex);
+    collect_retired(kMaxIdle);
+    auto large_enough = [&](const GraphBuffer* b) { return b->dev == dev && b->counters >= counter_bytes && b->bytes >= b->counters + bytes; };
+    GraphBuffer* mine = nullptr;
+    for (GraphBuffer* b : g_graph_live)   // launches of one stream follow one another in the graph as well
+        if (b->capture == capture && b->stream == stream && large_enough(b)) mine = b;
+    if (mine == nullptr) {
+        OutsideCapture outside;
+        cudaStream_t side = side_stream(dev);
+        if (side == nullptr) return ws;
+        for (size_t i = 0; i < g_graph_idle.size() && mine == nullptr; ++i) {
+            if (!large_enough(g_graph_idle[i])) continue;
+            mine = g_graph_idle[i];
+            g_graph_idle.erase(g_graph_idle.begin() + (long)i);
+        }
+        if (mine == nullptr) {
+            const size_t counters = std::max((counter_bytes + 4095) / 4096 * 4096, size_t(1) << 16);
+            void* ptr = nullptr;
+            if (cudaMallocAsync(&ptr, counters + bytes, side) != cudaSuccess) {
+                cudaGetLastError();
+                return ws;
+            }
+            mine = new GraphBuffer();
+            mine->dev = dev;
+            mine->ptr = static_cast<unsigned char*>(ptr);
+            mine->bytes = counters + bytes;
+            mine->counters = counters;
+        }
+        cudaUserObject_t owner = nullptr;
+        bool ok = cudaMemsetAsync(mine->ptr, 0, mine->counters, side) == cudaSuccess && cudaStreamSynchronize(side) == cudaSuccess;
+        ok = ok && cudaUserObjectCreate(&owner, mine, retire, 1, cudaUserObjectNoDestructorSync) == cudaSuccess;
+        if (!ok) {
+            cudaGetLastError();
+            g_graph_idle.push_back(mine);
+            return ws;
+        }
+        mine->capture = capture;
+        mine->stream = stream;
+        g_graph_live.push_back(mine);
+        if (cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+            cudaGetLastError();
+            mine->capture = 0;                    // nobody finds it
+            cudaUserObjectRelease(owner, 1);      // ... and it is retired
+            return ws;
+        }
+    }
+    ws.counters = reinterpret_cast<unsigned*>(mine->ptr);
+    ws.partials = mine->ptr + mine->counters;
+    return ws;
+}
 }  // namespace
 
 Workspace decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_bytes) {
     Workspace ws;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return ws;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long capture = 0;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo_v2(stream, &status, &capture, &graph) != cudaSuccess) cudaGetLastError();   // the launch will say what is wrong
+    if (status == cudaStreamCaptureStatusActive) return graph_workspace(stream, dev, capture, graph, bytes, counter_bytes);
+    if (status != cudaStreamCaptureStatusNone) return ws;
+    if (retired().count.load(std::memory_order_acquire) > 0) {
+        std::lock_guard<std::mutex> lock(g_graph_mutex);
+        collect_retired(kMaxIdle);
+    }
     std::unique_lock<std::mutex> held;
     const std::shared_ptr<WsEntry> e = lock_entry(dev, stream, held);
     if (e->ptr == nullptr || e->bytes < e->counters + bytes || e->counters < counter_bytes) {
@@ -198,7 +347,8 @@ int release_workspaces() {
         release_entry(*w);
         w->gone = true;
     }
-    return n;
+    std::lock_guard<std::mutex> lock(g_graph_mutex);
+    return n + collect_retired(0);   // (buffers that a graph keeps are the graph's)
 }
 
 namespace {

@@ -153,8 +153,8 @@ int get_option_prefill_test_skip_k();   // test hook: 1 + index of a K tile the 
 int check_launch(const char* what);
 
 // Split-K scratch of one call: the buffer of its (device, stream), grown on demand, this call's alone until the Workspace goes,
-// which is to be after its launches. partials == nullptr: not to be had. `counters`: at least counter_bytes that
-// are zero at the first use and that every launch leaves at zero.
+// which is to be after its launches; on a capturing stream, a buffer that the graph keeps. partials == nullptr: not to be had.
+// `counters`: at least counter_bytes that are zero at the first use and that every launch leaves at zero.
 struct WsEntry;
 struct Workspace {
     unsigned char* partials = nullptr;

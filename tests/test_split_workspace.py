@@ -74,3 +74,95 @@ def test_more_streams_than_workspaces_from_two_threads():
     for t in threads:
         t.join()
     assert not wrong
+
+
+def _dense(b, s, kv, hq=32, hkv=8, d=128, seed=0, dtype=torch.bfloat16):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    q, k, v = (torch.randn(b, n, h, d, generator=g, device="cuda").to(dtype) for n, h in ((s, hq), (kv, hkv), (kv, hkv)))
+    return lambda: high.flash_attn_func(q, k, v, start_pos=kv - s)
+
+
+def _mixed(ones, prompts, new, kv, hq=32, hkv=8, d=128, page=16, seed=0, dtype=torch.bfloat16):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    q_lens, k_lens = [new] * prompts + [1] * ones, [kv] * (prompts + ones)
+    pages = -(-kv // page)
+    k, v = (torch.randn(len(k_lens) * pages, page, hkv, d, generator=g, device="cuda").to(dtype) for _ in range(2))
+    q = torch.randn(sum(q_lens), hq, d, generator=g, device="cuda").to(dtype)
+    table = torch.randperm(len(k_lens) * pages, generator=torch.Generator().manual_seed(seed)).int().view(len(k_lens), pages).cuda()
+    cu = [torch.tensor([0] + n, dtype=torch.int32).cumsum(0).int().cuda() for n in (q_lens, k_lens)]
+    return lambda: high.flash_attn_varlen_func(q, k, v, *cu, new, kv, block_table=table)
+
+
+def _capture(call, stream):
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        out = call()
+    return graph, out
+
+
+CAPTURED = {"decode": lambda seed: _decode([3000, 40, 700], seed=seed), "speculate": lambda seed: _decode([5000, 2600], new=4, seed=seed),
+            "contiguous": lambda seed: _dense(3, 1, 4000, seed=seed), "mixed": lambda seed: _mixed(24, 3, 256, 3000, seed=seed)}
+
+
+@pytest.mark.parametrize("kind", CAPTURED)
+def test_graphs_captured_on_one_stream_without_a_call_before(kind):
+    # the stream has no workspace yet; two graphs of it and plain calls there must not depend on each other, in any order,
+    # nor on what becomes of the stream's own workspace
+    first, second = CAPTURED[kind](1), CAPTURED[kind](2)
+    want1, want2 = first(), second()
+    torch.cuda.synchronize()
+    ffi.lib.flash_attn_release_workspaces()
+    st = torch.cuda.Stream()
+    graph1, out1 = _capture(first, st)
+    graph2, out2 = _capture(second, st)
+
+    def check(graph, out, want):
+        out.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    check(graph2, out2, want2)          # before the first graph has ever run
+    with torch.cuda.stream(st):
+        got = second()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want2)
+    check(graph1, out1, want1)
+    ffi.lib.flash_attn_release_workspaces()
+    check(graph2, out2, want2)
+    other = torch.cuda.Stream()         # side by side, again and again
+    for o in (out1, out2):
+        o.fill_(float("nan"))
+    torch.cuda.synchronize()
+    for _ in range(20):
+        with torch.cuda.stream(other):
+            graph1.replay()
+        with torch.cuda.stream(st):
+            graph2.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out1, want1) and torch.equal(out2, want2)
+    del graph1, out1
+    torch.cuda.synchronize()
+    third, want3 = CAPTURED[kind](3), CAPTURED[kind](3)()
+    graph3, out3 = _capture(third, st)  # may take what the first graph gave back
+    check(graph2, out2, want2)
+    check(graph3, out3, want3)
+    check(graph2, out2, want2)
+
+
+def test_buffers_of_graphs_come_back():
+    call = _decode([4000] * 8, seed=4)
+    call()
+    st = torch.cuda.Stream()
+
+    def cycle(n):
+        for _ in range(n):
+            graph, out = _capture(call, st)
+            graph.replay()
+            torch.cuda.synchronize()
+            del graph, out
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+    before = cycle(8)
+    after = cycle(40)
+    assert before - after < 64 << 20, "each of 40 graphs that are gone kept its buffer (about 6 MB each)"
+    assert ffi.lib.flash_attn_release_workspaces() >= 1
