@@ -848,7 +848,8 @@ int log2_or_minus1(int v) {
     return -1;
 }
 
-// What can fail before anything is launched: the plan and its workspace. -1: not this kernel's.
+// What can fail before anything is launched: the plan and its workspace. -1: not this kernel's; FLASH_ATTN_ERR_CUDA (no
+// message yet): no memory for it, which is a failure only where no other kernel can take the call.
 template <int D>
 int prepare_typed(const AttnParams& p, int rows, cudaStream_t stream, RowsPlan& plan, Workspace& ws) {
     const long long max_tokens = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
@@ -858,12 +859,7 @@ int prepare_typed(const AttnParams& p, int rows, cudaStream_t stream, RowsPlan& 
     plan = plan_rows<D>(p.num_seqs, p.kv_heads, rows, max_tokens, true);
     if (plan.columns <= 0) return -1;
     ws = decode_workspace(stream, plan.partial_bytes, plan.counter_bytes);
-    if (ws.partials == nullptr) {
-        set_last_errorf("flash_attn_with_kvcache: could not allocate %zu bytes of split-K workspace",
-                        plan.partial_bytes + plan.counter_bytes);
-        return FLASH_ATTN_ERR_CUDA;
-    }
-    return FLASH_ATTN_OK;
+    return ws.partials != nullptr ? FLASH_ATTN_OK : FLASH_ATTN_ERR_CUDA;
 }
 
 template <typename T, int D>
@@ -940,19 +936,17 @@ int launch_prepared(const AttnParams& p, int max_rows, bool behind_prefill, cons
                                : launch_typed<__half, 32>(p, max_rows, behind_prefill, plan, ws, stream);
 }
 
-// The whole of a call whose sequences have at most `rows` query rows per KV head.
-int run_rows(const AttnParams& p, int rows, cudaStream_t stream) {
-    RowsPlan plan;
-    Workspace ws;
-    const int rc = prepare_rows(p, rows, stream, plan, ws);
-    return rc == FLASH_ATTN_OK ? launch_prepared(p, rows, false, plan, ws, stream) : rc;
-}
-
 }  // namespace
 
 int launch_decode_splitk(const AttnParams& p, cudaStream_t stream) {
     if (p.mode != MODE_KVCACHE || p.q_seq_len != 1 || !rows_kernel_takes(p)) return -1;
-    return run_rows(p, p.q_heads / p.kv_heads, stream);
+    const int rows = p.q_heads / p.kv_heads;
+    RowsPlan plan;
+    Workspace ws;
+    const int rc = prepare_rows(p, rows, stream, plan, ws);
+    if (rc == FLASH_ATTN_ERR_CUDA)
+        set_last_errorf("flash_attn_with_kvcache: could not allocate %zu bytes of split-K workspace", plan.partial_bytes + plan.counter_bytes);
+    return rc == FLASH_ATTN_OK ? launch_prepared(p, rows, false, plan, ws, stream) : rc;
 }
 
 // Whether few query rows (per KV head) over a range of `keys` are better off here than on the tensor-core prefill
@@ -973,7 +967,10 @@ int launch_few_rows(const AttnParams& p, cudaStream_t stream) {
     // up to four row blocks: each reads the K/V rows again, from L2 (28 rows of 7 x 1355-5421 keys: 43 us against
     // 87 on the prefill kernel; 32 rows of 8 x 3108: 45 against 109)
     if (rows > 4 * kRows || !worth_cutting(p, rows)) return -1;
-    return run_rows(p, (int)rows, stream);
+    RowsPlan plan;
+    Workspace ws;
+    if (prepare_rows(p, (int)rows, stream, plan, ws) != FLASH_ATTN_OK) return -1;   // the prefill kernel needs no memory of the library's
+    return launch_prepared(p, (int)rows, false, plan, ws, stream);
 }
 
 MixedFewRows prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {

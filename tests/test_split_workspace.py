@@ -166,3 +166,61 @@ def test_buffers_of_graphs_come_back():
     after = cycle(40)
     assert before - after < 64 << 20, "each of 40 graphs that are gone kept its buffer (about 6 MB each)"
     assert ffi.lib.flash_attn_release_workspaces() >= 1
+
+
+@pytest.fixture
+def no_pool_memory():
+    """cudaMallocAsync finds less than 1 MiB: the device's current pool is a small one that is full."""
+    from cuda.bindings import runtime as rt
+
+    def ok(ret):
+        assert int(ret[0]) == 0, ret
+        return ret[1] if len(ret) > 1 else None
+    dev = torch.cuda.current_device()
+    torch.cuda.synchronize()
+    ffi.lib.flash_attn_release_workspaces()
+    before = ok(rt.cudaDeviceGetMemPool(dev))
+    props = rt.cudaMemPoolProps()
+    props.allocType = rt.cudaMemAllocationType.cudaMemAllocationTypePinned
+    props.location.type = rt.cudaMemLocationType.cudaMemLocationTypeDevice
+    props.location.id = dev
+    props.maxSize = 32 << 20
+    pool = ok(rt.cudaMemPoolCreate(props))
+    ok(rt.cudaDeviceSetMemPool(dev, pool))
+    held = []
+    while len(held) < 4096:
+        err, ptr = rt.cudaMallocAsync(1 << 20, 0)
+        if int(err) != 0:
+            rt.cudaGetLastError()
+            break
+        held.append(ptr)
+    assert 0 < len(held) < 4096
+    yield
+    torch.cuda.synchronize()
+    ffi.lib.flash_attn_release_workspaces()
+    for ptr in held:
+        ok(rt.cudaFreeAsync(ptr, 0))
+    torch.cuda.synchronize()
+    ok(rt.cudaDeviceSetMemPool(dev, before))
+    ok(rt.cudaMemPoolDestroy(pool))
+
+
+@pytest.mark.parametrize("kind", ["speculate", "contiguous", "mixed"])
+def test_calls_that_have_another_kernel_run_without_a_workspace(kind, no_pool_memory):
+    ffi.lib.flash_attn_set_option(b"force_generic", 1)
+    try:
+        want = CAPTURED[kind](5)().float()
+    finally:
+        ffi.lib.flash_attn_set_option(b"force_generic", 0)
+    got = CAPTURED[kind](5)().float()
+    assert ffi.last_path() == "prefill_tcgen05" and ffi.lib.flash_attn_last_launches() == 1
+    assert ffi.last_error() == ""       # nothing went wrong
+    torch.cuda.synchronize()
+    diff = (got - want).abs()           # two bf16 results of the same f32 sums: the bar of bf16 outputs
+    assert diff.max() <= 2e-2 and diff.mean() <= 2e-3
+
+
+def test_decoding_without_a_workspace_says_so(no_pool_memory):
+    from luma_b200 import error
+    with pytest.raises(error.CudaError, match="flash_attn_with_kvcache: could not allocate"):
+        CAPTURED["decode"](6)()
