@@ -282,7 +282,7 @@ Workspace graph_workspace(cudaStream_t stream, int dev, unsigned long long captu
             return ws;
         }
     }
-    ws.counters = reinterpret_cast<unsigned*>(mine->ptr);
+    ws.counters = reinterpret_cast<unsigned long long*>(mine->ptr);
     ws.partials = mine->ptr + mine->counters;
     return ws;
 }
@@ -327,7 +327,7 @@ Workspace decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_byt
             return ws;
         }
     }
-    ws.counters = static_cast<unsigned*>(e->ptr);
+    ws.counters = static_cast<unsigned long long*>(e->ptr);
     ws.partials = static_cast<unsigned char*>(e->ptr) + e->counters;
     ws.entry = e;
     ws.held = std::move(held);

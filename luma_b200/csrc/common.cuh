@@ -154,11 +154,12 @@ int check_launch(const char* what);
 
 // Split-K scratch of one call: the buffer of its (device, stream), grown on demand, this call's alone until the Workspace goes,
 // which is to be after its launches; on a capturing stream, a buffer that the graph keeps. partials == nullptr: not to be had.
-// `counters`: at least counter_bytes that are zero at the first use and that every launch leaves at zero.
+// `counters`: at least counter_bytes that are zero at the first use and that every launch leaves at zero (unless calls overlap on
+// one buffer, which only a stream handle that stands for several streams can bring about).
 struct WsEntry;
 struct Workspace {
     unsigned char* partials = nullptr;
-    unsigned* counters = nullptr;
+    unsigned long long* counters = nullptr;
     std::shared_ptr<WsEntry> entry;         // (before `held`: outlives its mutex's lock)
     std::unique_lock<std::mutex> held;
 };

@@ -49,6 +49,9 @@ struct RowsOut {
     float* lse;      // MODE_BATCH: (num_seqs, q_heads, q_seq_len) or null
 };
 
+constexpr int kMaxColumns = 65535;
+constexpr int kCountBits = 20;   // of an arrival counter; the number of the call is above
+
 struct RowsArgs {
     const void* q;
     const void* k;
@@ -59,7 +62,8 @@ struct RowsArgs {
     const int* cu_k;           // MODE_VARLEN
     float* ws_acc;       // (2 * CTAs, kRows, D) f32, unnormalised; slot 0 of a CTA: the sequence that began in an earlier column, slot 1: the one that goes on in the next
     float2* ws_ml;       // (2 * CTAs, kRows) {m (log2 domain), l}
-    unsigned* arrived;   // (gridDim.x, num_seqs) parts of a cut sequence that are in the workspace; zero between calls
+    unsigned long long* arrived;   // (gridDim.x, num_seqs): `call` + the parts of a cut sequence that are in the workspace; zero between calls
+    unsigned long long call;       // number of this call, in the bits above the count
     int mode, num_seqs, q_seq_len, kv_seq_len, start_pos;
     int q_heads, kv_heads, block_size, block_shift, max_blocks, paged;   // block_shift: log2 of the page size, -1 where it is no power of two
     int row_blocks;      // blocks of kRows query rows per KV head (blockIdx.x = KV head x row block)
@@ -219,12 +223,16 @@ struct Cut {
     }
 };
 
-// One arrival: everything the CTA's threads wrote before their last barrier is visible to whoever sees the count
-// (release), and what earlier arrivals published is visible to this CTA after its next barrier (acquire).
-__device__ __forceinline__ unsigned arrive_acq_rel(unsigned* count) {
-    unsigned before;
-    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;\n" : "=r"(before) : "l"(count) : "memory");
-    return before;
+// One arrival; returns how many came before it. Everything the CTA's threads wrote before their last barrier is visible to
+// whoever sees the count (release), and what earlier arrivals published is visible to this CTA after its next barrier (acquire).
+// Whatever an earlier call left there (calls that overlapped on one buffer, which spoils their results, leave counts that are
+// not zero) is below this call's number and does not count: the maximum lifts it, ahead of the addition to the same word,
+// and costs no trip of its own, as nothing waits for it.
+__device__ __forceinline__ unsigned long long arrive_acq_rel(unsigned long long* count, unsigned long long call) {
+    unsigned long long before;
+    asm volatile("red.relaxed.gpu.global.max.u64 [%0], %1;\n" ::"l"(count), "l"(call) : "memory");
+    asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;\n" : "=l"(before) : "l"(count) : "memory");
+    return before - call;
 }
 
 // Two finished neighbours of an output row, to every output buffer.
@@ -728,9 +736,9 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
             const int parts = (int)cut.column_of(seq_first + (unsigned)units - 1u) - c_first + 1;
             // (the last pass of the merge above ended with a barrier: every thread's partials are before this)
             if (threadIdx.x == 0) {
-                unsigned* cnt = a.arrived + (long long)blockIdx.x * a.num_seqs + s;
-                const int last = arrive_acq_rel(cnt) == (unsigned)(parts - 1);
-                if (last) *cnt = 0u;   // as it was found, for the next call
+                unsigned long long* cnt = a.arrived + (long long)blockIdx.x * a.num_seqs + s;
+                const int last = arrive_acq_rel(cnt, a.call) == (unsigned long long)(parts - 1);
+                if (last) *cnt = 0ull;   // as it was found: a captured launch runs again under the same number
                 *last_flag = last;
             }
             __syncthreads();
@@ -803,17 +811,21 @@ RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, b
         while ((most_units + r.forced_units - 1) / r.forced_units > 4096) r.forced_units *= 2;
         r.columns = (int)((most_units + r.forced_units - 1) / r.forced_units);
     }
-    r.columns = (int)std::min<long long>(std::min(r.columns, 65535), most_units);
+    r.columns = (int)std::min<long long>(std::min(r.columns, kMaxColumns), most_units);
     const size_t slots = (size_t)2 * per_column * r.columns;
     r.acc_bytes = slots * kRows * D * sizeof(float);
     r.partial_bytes = r.acc_bytes + slots * kRows * sizeof(float2);
-    r.counter_bytes = (size_t)per_column * num_seqs * sizeof(unsigned);
+    r.counter_bytes = (size_t)per_column * num_seqs * sizeof(unsigned long long);
     return r;
 }
+
+std::atomic<unsigned long long> g_calls{0};   // launches of this kernel, of any type and on any device
 
 template <typename T, int D>
 int launch_rows(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
     using S = Smem<D>;
+    static_assert(kMaxColumns < (1 << kCountBits), "the parts of a sequence fit the count");
+    a.call = (g_calls.fetch_add(1, std::memory_order_relaxed) + 1) << kCountBits;
     a.row_blocks = plan.row_blocks;
     a.forced_units = plan.forced_units;
     static std::atomic<unsigned long long> ready{0};   // devices whose copy of this kernel has its shared-memory limit raised
@@ -1011,7 +1023,7 @@ int launch_mixed_few_rows(const AttnParams& p, const MixedFewRows& few, cudaStre
 namespace {
 
 constexpr size_t kStaticScratchBytes = size_t(16) << 20;   // 16 MiB per GPU
-constexpr size_t kStaticCounterBytes = size_t(1) << 20;    // of these, the arrival counters (at most 63 550 x 4 bytes within the entry point's limit)
+constexpr size_t kStaticCounterBytes = size_t(1) << 20;    // of these, the arrival counters (at most 63 550 x 8 bytes within the entry point's limit)
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
 constexpr int kMaxDevices = 64;
@@ -1087,7 +1099,7 @@ int launch_static(const void* q, const void* k, const void* v, void* o, const in
     a.q = q; a.k = k; a.v = v;
     a.block_tables = block_tables;
     a.context_lens = context_lens;
-    a.arrived = reinterpret_cast<unsigned*>(ws);   // zero in the library image, and again after every call
+    a.arrived = reinterpret_cast<unsigned long long*>(ws);   // zero in the library image, and again after every call
     a.ws_acc = reinterpret_cast<float*>(ws + kStaticCounterBytes);
     a.ws_ml = reinterpret_cast<float2*>(ws + kStaticCounterBytes + plan.acc_bytes);
     a.mode = MODE_KVCACHE;
@@ -1104,6 +1116,10 @@ int launch_static(const void* q, const void* k, const void* v, void* o, const in
     a.out.o[0] = o;
     a.out.n_out = 1;
     a.out.o_heads = q_heads;
+    // A captured launch keeps its number, which is lower than that of calls made since: the graph clears the counters itself.
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) cudaGetLastError();
+    if (status == cudaStreamCaptureStatusActive) cudaMemsetAsync(ws, 0, plan.counter_bytes, stream);
     const int rc = launch_rows<T, D>(a, plan, stream);
     if (rc == FLASH_ATTN_OK) note_path("decode_splitk_static", 1);
     return rc;

@@ -224,3 +224,58 @@ def test_decoding_without_a_workspace_says_so(no_pool_memory):
     from luma_b200 import error
     with pytest.raises(error.CudaError, match="flash_attn_with_kvcache: could not allocate"):
         CAPTURED["decode"](6)()
+
+
+def _noalloc(lens, hq, hkv, d, seed, page=16):
+    """(call on a stream, its output buffer, f64 result) of the allocation-free entry point."""
+    import numpy as np
+    from oracle import binding as ob
+    from tests import helpers as H
+    kc, vc, table = H.make_paged_cache(lens, page, hkv, d, seed=seed)
+    q = H.normal((len(lens), 1, hq, d), seed + 3)
+    dq, dk, dv = (H.to_dev(x, "bf16") for x in (q, kc, vc))
+    bt, cl, o = torch.from_numpy(table).cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda"), torch.empty_like(dq)
+    scale = float(1.0 / np.sqrt(d))
+
+    def call(stream=None):
+        st = stream if stream is not None else torch.cuda.current_stream()
+        rc = ffi.lib.flash_attn_decode_bf16_noalloc(dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), o.data_ptr(), bt.data_ptr(), cl.data_ptr(),
+                                                    len(lens), hq, hkv, d, page, bt.shape[1], scale, st.cuda_stream)
+        assert rc == 0, ffi.last_error()
+    want = ob.attn_f64_kvcache(H.round_to(q, "bf16"), H.round_to(kc, "bf16"), H.round_to(vc, "bf16"), lens, table, scale=scale)
+
+    def check(what):
+        torch.cuda.synchronize()
+        H.assert_bf16_close(H.to_np(o), want, what)
+        o.fill_(float("nan"))
+    return call, check
+
+
+def test_allocation_free_calls_after_calls_that_overlapped():
+    # the documented misuse, two calls at once on the shared array (in bounds, but their results are spoiled), must not reach the calls
+    # that follow, plain or captured before
+    problems = [_noalloc(lens, hq, hkv, d, 50 + i) for i, (lens, hq, hkv, d) in enumerate(
+        [([9000, 300, 5000], 8, 2, 128), ([2500] * 7, 16, 4, 64), ([40000], 8, 8, 128), ([64, 1, 0, 700], 8, 2, 128)])]
+    st = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for call, check in problems:
+        call()
+        check("before")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=st[0]):
+        problems[0][0](st[0])
+    for _ in range(50):
+        for i, j in ((0, 1), (2, 0), (1, 2)):
+            problems[i][0](st[0])
+            problems[j][0](st[1])
+    torch.cuda.synchronize()
+    for _, check in problems:
+        try:
+            check("spoiled")
+        except AssertionError:
+            pass
+    for _ in range(2):
+        for n, (call, check) in enumerate(problems):
+            call()
+            check(f"problem {n} after overlapping calls")
+        graph.replay()
+        problems[0][1]("captured before, replayed after overlapping calls")
