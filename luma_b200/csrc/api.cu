@@ -298,6 +298,25 @@ Workspace decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_byt
     if (cudaStreamGetCaptureInfo_v2(stream, &status, &capture, &graph) != cudaSuccess) cudaGetLastError();   // the launch will say what is wrong
     if (status == cudaStreamCaptureStatusActive) return graph_workspace(stream, dev, capture, graph, bytes, counter_bytes);
     if (status != cudaStreamCaptureStatusNone) return ws;
+    if (stream == cudaStreamPerThread) {
+        // One handle, a stream of its own in every thread: no key of the table. Memory of this call alone, given back
+        // in stream order behind its launch.
+        void* ptr = nullptr;
+        const size_t counters = (counter_bytes + 255) / 256 * 256;
+        if (cudaMallocAsync(&ptr, counters + bytes, stream) != cudaSuccess) {
+            cudaGetLastError();
+            return ws;
+        }
+        if (cudaMemsetAsync(ptr, 0, counters, stream) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFreeAsync(ptr, stream);
+            return ws;
+        }
+        ws.own = ptr;
+        ws.counters = static_cast<unsigned long long*>(ptr);
+        ws.partials = static_cast<unsigned char*>(ptr) + counters;
+        return ws;
+    }
     if (retired().count.load(std::memory_order_acquire) > 0) {
         std::lock_guard<std::mutex> lock(g_graph_mutex);
         collect_retired(kMaxIdle);
@@ -332,6 +351,10 @@ Workspace decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_byt
     ws.entry = e;
     ws.held = std::move(held);
     return ws;
+}
+
+Workspace::~Workspace() {
+    if (own != nullptr) cudaFreeAsync(own, cudaStreamPerThread);
 }
 
 int release_workspaces() {

@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <memory>
 #include <mutex>
+#include <utility>
 
 #include "../../include/flash_attn.h"
 
@@ -154,12 +155,24 @@ int check_launch(const char* what);
 
 // Split-K scratch of one call: the buffer of its (device, stream), grown on demand, this call's alone until the Workspace goes,
 // which is to be after its launches; on a capturing stream, a buffer that the graph keeps. partials == nullptr: not to be had.
-// `counters`: at least counter_bytes that are zero at the first use and that every launch leaves at zero (unless calls overlap on
-// one buffer, which only a stream handle that stands for several streams can bring about).
+// `counters`: at least counter_bytes that are zero at the first use and that every launch leaves at zero.
 struct WsEntry;
 struct Workspace {
+    Workspace() = default;
+    Workspace(Workspace&& o) noexcept
+        : partials(o.partials), counters(o.counters), own(std::exchange(o.own, nullptr)), entry(std::move(o.entry)), held(std::move(o.held)) {}
+    Workspace& operator=(Workspace&& o) noexcept {
+        partials = o.partials;
+        counters = o.counters;
+        std::swap(own, o.own);
+        entry.swap(o.entry);
+        held.swap(o.held);
+        return *this;
+    }
+    ~Workspace();
     unsigned char* partials = nullptr;
     unsigned long long* counters = nullptr;
+    void* own = nullptr;                    // a buffer of this call's, given back to the per-thread stream
     std::shared_ptr<WsEntry> entry;         // (before `held`: outlives its mutex's lock)
     std::unique_lock<std::mutex> held;
 };

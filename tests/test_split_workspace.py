@@ -279,3 +279,43 @@ def test_allocation_free_calls_after_calls_that_overlapped():
             check(f"problem {n} after overlapping calls")
         graph.replay()
         problems[0][1]("captured before, replayed after overlapping calls")
+
+
+def test_the_per_thread_stream_is_another_stream_in_every_thread():
+    # one handle value (2), a stream of its own per thread: the threads' kernels run side by side
+    from luma_b200 import low
+    import types
+    per_thread = types.SimpleNamespace(cuda_stream=2)
+
+    def problem(lens, hq, hkv, seed):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        n, pages = len(lens), -(-max(lens) // 16)
+        k, v = (torch.randn(n * pages, 16, hkv, 128, generator=g, device="cuda").bfloat16() for _ in range(2))
+        q = torch.randn(n, 1, hq, 128, generator=g, device="cuda").bfloat16()
+        table = torch.randperm(n * pages, generator=torch.Generator().manual_seed(seed)).int().view(n, pages).cuda()
+        cl = torch.tensor(lens, dtype=torch.int32, device="cuda")
+
+        def call(outs, stream=None):
+            for o in outs:
+                low.flash_attn_with_kvcache(q, k, v, o, table, cl, n, 1, hq, hkv, 128, 16, pages, 0.1, stream)
+            if stream is not None:   # nothing of the thread's stream is in flight when the thread ends
+                torch.cuda.ExternalStream(stream.cuda_stream).synchronize()
+        return call, q
+    problems = [problem([20000, 300], 32, 8, 1), problem([9000] * 12, 32, 8, 2), problem([30000], 8, 8, 3)]
+    want = []
+    for call, q in problems:
+        want.append(torch.empty_like(q))
+        call([want[-1]])
+    torch.cuda.synchronize()
+    ffi.lib.flash_attn_release_workspaces()
+    for _ in range(12):      # more threads in all than the table has entries
+        outs = [[torch.full_like(q, float("nan")) for _ in range(8)] for _, q in problems]
+        torch.cuda.synchronize()
+        threads = [threading.Thread(target=call, args=(o, per_thread)) for (call, _), o in zip(problems, outs)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        torch.cuda.synchronize()
+        for w, out in zip(want, outs):
+            assert all(torch.equal(w, o) for o in out)
