@@ -46,6 +46,7 @@ constexpr int kRows = 16;    // query rows served per CTA (M of the mma)
 struct RowsOut {
     void* o[8];
     int n_out, o_heads, o_head0, peer0;
+    int halves;      // a buffer is aligned to its 2-byte elements only: no 4-byte stores
     float* lse;      // MODE_BATCH: (num_seqs, q_heads, q_seq_len) or null
 };
 
@@ -241,7 +242,13 @@ __device__ __forceinline__ void store_pair(const RowsOut& out, long long row, in
     const long long off = (row * out.o_heads + out.o_head0 + head) * D + d;
     int pe = out.peer0;
     for (int n = 0; n < out.n_out; ++n) {
-        *reinterpret_cast<unsigned*>(static_cast<T*>(out.o[pe]) + off) = both;
+        T* const at = static_cast<T*>(out.o[pe]) + off;
+        if (out.halves) {
+            reinterpret_cast<unsigned short*>(at)[0] = (unsigned short)both;
+            reinterpret_cast<unsigned short*>(at)[1] = (unsigned short)(both >> 16);
+        } else {
+            *reinterpret_cast<unsigned*>(at) = both;
+        }
         pe = pe + 1 == out.n_out ? 0 : pe + 1;
     }
 }
@@ -825,6 +832,8 @@ template <typename T, int D>
 int launch_rows(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
     using S = Smem<D>;
     static_assert(kMaxColumns < (1 << kCountBits), "the parts of a sequence fit the count");
+    for (int i = 0; i < a.out.n_out; ++i)
+        if (reinterpret_cast<uintptr_t>(a.out.o[i]) & 3) a.out.halves = 1;
     a.call = (g_calls.fetch_add(1, std::memory_order_relaxed) + 1) << kCountBits;
     a.row_blocks = plan.row_blocks;
     a.forced_units = plan.forced_units;
@@ -920,15 +929,13 @@ int launch_typed(const AttnParams& p, int max_rows, bool behind_prefill, const R
 
 namespace {
 
-// 16-bit storage, 16-byte aligned K/V rows (cp.async); q is read and o written four bytes at a time.
+// 16-bit storage, 16-byte aligned K/V rows (cp.async); q is read four bytes at a time.
 bool rows_kernel_takes(const AttnParams& p) {
     if (p.dtype != DT_F16 && p.dtype != DT_BF16) return false;
     if (p.head_size != 32 && p.head_size != 64 && p.head_size != 128) return false;
     if (p.mask != nullptr || p.n_lse > 0 || p.multicast) return false;
     if ((reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) return false;
-    uintptr_t qo = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.o);
-    for (int i = 0; i < p.n_out && i < 8; ++i) qo |= reinterpret_cast<uintptr_t>(p.o_peers[i]);
-    return (qo & 3) == 0;
+    return (reinterpret_cast<uintptr_t>(p.q) & 3) == 0;
 }
 
 int prepare_rows(const AttnParams& p, int rows, cudaStream_t stream, RowsPlan& plan, Workspace& ws) {
@@ -1150,8 +1157,8 @@ extern "C" int flash_attn_decode_bf16_noalloc(const flash_attn_bf16_t* q, const 
         return FLASH_ATTN_ERR_INVALID_SHAPE;
     }
     if (((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) ||
-        ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(o)) & 3)) {
-        set_last_error("flash_attn_decode_bf16_noalloc: k_cache/v_cache must be 16-byte aligned, q and o 4-byte aligned");
+        (reinterpret_cast<uintptr_t>(q) & 3)) {
+        set_last_error("flash_attn_decode_bf16_noalloc: k_cache/v_cache must be 16-byte aligned, q 4-byte aligned");
         return FLASH_ATTN_ERR_INVALID_SHAPE;
     }
     // launch on the device that owns q, and resolve the scratch address on that same device

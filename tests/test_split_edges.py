@@ -1,0 +1,40 @@
+"""What the split-K kernel takes at the edges of its arguments: output alignment, lengths beyond the block table."""
+import numpy as np
+import pytest
+import torch
+
+from luma_b200 import ffi, low
+from oracle import binding as ob
+from tests import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("d", [32, 64, 128])
+@pytest.mark.parametrize("entry", ["decode", "noalloc", "allgather"])
+def test_output_aligned_to_its_elements_only(entry, d):
+    # an output that starts two bytes off a word: a whole sequence (finished by one CTA) and a cut one (merged)
+    if entry == "noalloc" and d == 32:
+        pytest.skip("the entry point takes head sizes 64 and 128")
+    lens, hq, hkv, bs = [5000, 33], 8, 2, 16
+    kc, vc, table = H.make_paged_cache(lens, bs, hkv, d, seed=80 + d)
+    q = H.normal((2, 1, hq, d), 83)
+    dq, dk, dv = (H.to_dev(x, "bf16") for x in (q, kc, vc))
+    bt, cl = torch.from_numpy(table).cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda")
+    room = torch.zeros(dq.numel() + 2, dtype=torch.bfloat16, device="cuda")
+    o = room[1:-1]
+    assert o.data_ptr() % 4 == 2
+    scale = float(1 / np.sqrt(d))
+    if entry == "decode":
+        low.flash_attn_with_kvcache(dq, dk, dv, o, bt, cl, 2, 1, hq, hkv, d, bs, bt.shape[1], scale)
+    elif entry == "allgather":
+        low.flash_attn_with_kvcache_allgather(dq, dk, dv, [o.data_ptr()], hq, 0, bt, cl, 2, hq, hkv, d, bs, bt.shape[1], scale)
+    else:
+        rc = ffi.lib.flash_attn_decode_bf16_noalloc(dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), o.data_ptr(), bt.data_ptr(), cl.data_ptr(), 2,
+                                                    hq, hkv, d, bs, bt.shape[1], scale, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0, ffi.last_error()
+    torch.cuda.synchronize()
+    assert ffi.last_path() in ("decode_splitk", "decode_splitk_static")
+    want = ob.attn_f64_kvcache(H.round_to(q, "bf16"), H.round_to(kc, "bf16"), H.round_to(vc, "bf16"), lens, table, scale=scale)
+    H.assert_bf16_close(H.to_np(o).reshape(want.shape), want, entry)
+    assert room[0] == 0 and room[-1] == 0      # and nothing beside it
