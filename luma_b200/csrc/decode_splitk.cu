@@ -68,6 +68,7 @@ struct RowsArgs {
     int mode, num_seqs, q_seq_len, kv_seq_len, start_pos;
     int q_heads, kv_heads, block_size, block_shift, max_blocks, paged;   // block_shift: log2 of the page size, -1 where it is no power of two
     int row_blocks;      // blocks of kRows query rows per KV head (blockIdx.x = KV head x row block)
+    int capacity;        // keys that a sequence's row of the block table has room for; contiguous K/V: no limit
     int max_rows;        // sequences with more query rows than this (per KV head) are not this launch's
     int behind_prefill;  // launched behind the prefill kernel of the same call, which it does not depend on
     int forced_units;    // > 0: units per column (option "decode_chunk_tokens"); 0: equal shares
@@ -195,9 +196,9 @@ __device__ __forceinline__ RowsSeq rows_seq(const RowsArgs& a, int s) {
     return r;
 }
 
-// Keys that the last query token sees.
-__device__ __forceinline__ int rows_visible(const RowsSeq& r) {
-    const long long v = min((long long)r.kv_len, (long long)r.pos_off + r.q_len);
+// Keys that the last query token sees: of a length beyond what the block table holds, the part that it holds.
+__device__ __forceinline__ int rows_visible(const RowsArgs& a, const RowsSeq& r) {
+    const long long v = min((long long)min(r.kv_len, a.capacity), (long long)r.pos_off + r.q_len);
     return v > 0 ? (int)v : 0;
 }
 
@@ -206,16 +207,20 @@ __device__ __forceinline__ int rows_visible(const RowsSeq& r) {
 __device__ __forceinline__ int rows_units(const RowsArgs& a, const RowsSeq& r, int group, int row0) {
     const int rows = r.q_len * group;
     if (rows <= row0 || rows > a.max_rows) return 0;
-    return max(1, (rows_visible(r) + kUnit - 1) / kUnit);
+    return max(1, (rows_visible(a, r) + kUnit - 1) / kUnit);
 }
 
 // The cut of `total` units into columns: the first `more` columns have share + 1 units, the others share
-// (or, forced, every column `share` units). All in 32 bits: a 64-bit division here cost a microsecond of a small call.
+// (or, forced, every column at least `forced` units). All in 32 bits: a 64-bit division here cost a microsecond of a small call.
 struct Cut {
     unsigned share, more;
     __device__ __forceinline__ Cut(unsigned total, unsigned columns, unsigned forced) {
-        share = forced > 0 ? forced : total / columns;
-        more = forced > 0 ? 0u : total - share * columns;
+        share = total / columns;
+        more = total - share * columns;
+        if (share < forced || (share == forced && more == 0u)) {   // (never less than covers them all, whatever bound the host had)
+            share = forced;
+            more = 0u;
+        }
     }
     __device__ __forceinline__ unsigned first(unsigned c) const { return share * c + min(c, more); }
     __device__ __forceinline__ unsigned column_of(unsigned unit) const {
@@ -475,7 +480,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
     int cp_left = (int)(u_end - u_begin);
     int cp_s = s;
     RowsSeq cp_seq = rows_seq(a, s);
-    int cp_vis = rows_visible(cp_seq);
+    int cp_vis = rows_visible(a, cp_seq);
     int cp_tok = (int)(u_begin - seq_first) * kUnit;   // first token of the unit to copy next
     int cp_end = rows_units(a, cp_seq, group, row0) * kUnit;
     auto look_up = [&]() -> long long {   // element offset of this lane's token row in the caches, -1 past the visible keys
@@ -501,7 +506,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
                     cp_seq = rows_seq(a, ++cp_s);
                     cp_end = rows_units(a, cp_seq, group, row0) * kUnit;
                 } while (cp_end == 0);
-                cp_vis = rows_visible(cp_seq);
+                cp_vis = rows_visible(a, cp_seq);
                 cp_tok = 0;
             }
         }
@@ -549,7 +554,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
             seq = rows_seq(a, ++s);
             units = rows_units(a, seq, group, row0);
         }
-        const int vis = rows_visible(seq);
+        const int vis = rows_visible(a, seq);
         const int nrows = min(kRows, seq.q_len * group - row0);   // query rows served here
         const unsigned seg_end = min(u_end, seq_first + (unsigned)units);
         const bool starts = u == seq_first, ends = seg_end == seq_first + (unsigned)units;
@@ -570,10 +575,10 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
                 qa[kk][2] = v0 ? q0[kk * 8 + 4 + c4] : 0u;
                 qa[kk][3] = v1 ? q1[kk * 8 + 4 + c4] : 0u;
             }
-            lim0 = (int)min((long long)seq.kv_len - 1, (long long)seq.pos_off + t0);
-            lim1 = (int)min((long long)seq.kv_len - 1, (long long)seq.pos_off + t1);
+            lim0 = (int)min((long long)min(seq.kv_len, a.capacity) - 1, (long long)seq.pos_off + t0);
+            lim1 = (int)min((long long)min(seq.kv_len, a.capacity) - 1, (long long)seq.pos_off + t1);
         }
-        const int lim_all = min(seq.kv_len, seq.pos_off + 1);   // keys below this are seen by every row
+        const int lim_all = min(min(seq.kv_len, a.capacity), seq.pos_off + 1);   // keys below this are seen by every row
 
         float acc[kDBlocks][4];
 #pragma unroll
@@ -906,6 +911,7 @@ int launch_typed(const AttnParams& p, int max_rows, bool behind_prefill, const R
     a.block_shift = log2_or_minus1(p.block_size);
     a.max_blocks = p.max_blocks;
     a.paged = p.paged;
+    a.capacity = p.paged ? (int)std::min(0x7fffffffLL, (long long)p.max_blocks * p.block_size) : 0x7fffffff;
     a.max_rows = max_rows;
     a.scale_log2 = p.scale * 1.4426950408889634f;
     if (p.n_out > 0) {
@@ -1118,6 +1124,7 @@ int launch_static(const void* q, const void* k, const void* v, void* o, const in
     a.block_shift = log2_or_minus1(block_size);
     a.max_blocks = max_blocks;
     a.paged = 1;
+    a.capacity = (int)std::min(0x7fffffffLL, max_tokens);
     a.max_rows = group;
     a.scale_log2 = scale * 1.4426950408889634f;
     a.out.o[0] = o;

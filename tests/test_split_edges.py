@@ -38,3 +38,37 @@ def test_output_aligned_to_its_elements_only(entry, d):
     want = ob.attn_f64_kvcache(H.round_to(q, "bf16"), H.round_to(kc, "bf16"), H.round_to(vc, "bf16"), lens, table, scale=scale)
     H.assert_bf16_close(H.to_np(o).reshape(want.shape), want, entry)
     assert room[0] == 0 and room[-1] == 0      # and nothing beside it
+
+
+@pytest.mark.parametrize("chunk", [0, 64, 1024])
+@pytest.mark.parametrize("new", [1, 4])
+def test_length_beyond_the_block_table_is_cut_at_its_capacity(chunk, new):
+    hq, hkv, d, bs = 8, 2, 128, 16
+    table_lens, lens = [2048, 2048, 2048], [2048 + 5000, 700, 2049]
+    kc, vc, table = H.make_paged_cache(table_lens, bs, hkv, d, seed=90)
+    q = H.normal((3, new, hq, d), 93)
+    dq, dk, dv = (H.to_dev(x, "bf16") for x in (q, kc, vc))
+    bt = torch.from_numpy(table).cuda()
+    scale = float(1 / np.sqrt(d))
+
+    def run(lens):
+        o = torch.full_like(dq, float("nan"))
+        low.flash_attn_with_kvcache(dq, dk, dv, o, bt, torch.tensor(lens, dtype=torch.int32, device="cuda"), 3, new, hq, hkv, d, bs, bt.shape[1], scale)
+        assert ffi.last_path() == "decode_splitk"
+        return H.to_np(o)
+    rq, rk, rv = (H.round_to(x, "bf16") for x in (q, kc, vc))
+    ffi.lib.flash_attn_set_option(b"decode_chunk_tokens", chunk)
+    try:
+        for _ in range(2):
+            got = run(lens)
+            for s, n in enumerate(lens):
+                # a row at a position past the table sees all that the table holds
+                pos = [n - new + t for t in range(new)]
+                want = np.concatenate([ob.attn_f64_kvcache(rq[s:s + 1, t:t + 1], rk, rv, [min(2048, p + 1)], table[s:s + 1], scale=scale)
+                                       for t, p in enumerate(pos)], axis=1)
+                H.assert_bf16_close(got[s:s + 1], want, f"sequence {s} of {n} tokens")
+            got = run([2048, 30, 900])        # and the next call finds everything in order
+            want = ob.attn_f64_kvcache(rq, rk, rv, [2048, 30, 900], table, scale=scale)
+            H.assert_bf16_close(got, want, "after")
+    finally:
+        ffi.lib.flash_attn_set_option(b"decode_chunk_tokens", 0)
