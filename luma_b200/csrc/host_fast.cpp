@@ -86,6 +86,9 @@ void* stream_of(int device) { return (void*)c10::cuda::getCurrentCUDAStream((c10
 
 bool fits(int64_t v) { return v >= 1 && v <= INT32_MAX; }
 
+// Whether the buffer holds a * b * c * d elements; four ints multiply to 124 bits, which 64 do not hold.
+bool holds(const Tensor& t, int64_t a, int64_t b, int64_t c, int64_t d) { return (__int128)a * b * c * d <= (__int128)t.numel(); }
+
 bool head_size_ok(int64_t d) { return d == 32 || d == 64 || d == 128; }
 
 // The library's status as the front end reports it: nullptr with the exception set, or `result`.
@@ -154,9 +157,9 @@ PyObject* low_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
     scale = (float)PyFloat_AS_DOUBLE(a[11]);
     const int ti = type_index(*q);
     PLAIN(ti >= 0 && k->scalar_type() == q->scalar_type() && v->scalar_type() == q->scalar_type() && o->scalar_type() == q->scalar_type());
-    PLAIN(q->numel() >= b * sq * hq * d && o->numel() >= b * sq * hq * d && k->numel() >= b * skv * hkv * d && v->numel() >= b * skv * hkv * d);
-    if (a[12] != Py_None) PLAIN(plain(a[12], mask, dev) && mask->element_size() == 1 && mask->numel() >= b * skv);
-    if (a[13] != Py_None) PLAIN(plain(a[13], lse, dev) && lse->scalar_type() == at::kFloat && lse->numel() >= b * hq * sq);
+    PLAIN(holds(*q, b, sq, hq, d) && holds(*o, b, sq, hq, d) && holds(*k, b, skv, hkv, d) && holds(*v, b, skv, hkv, d));
+    if (a[12] != Py_None) PLAIN(plain(a[12], mask, dev) && mask->element_size() == 1 && holds(*mask, b, skv, 1, 1));
+    if (a[13] != Py_None) PLAIN(plain(a[13], lse, dev) && lse->scalar_type() == at::kFloat && holds(*lse, b, hq, sq, 1));
     const uint8_t* mp = mask != nullptr ? (const uint8_t*)mask->const_data_ptr() : nullptr;
     void* st = stream_of(dev);
     int code;
@@ -242,8 +245,7 @@ PyObject* append(PyObject*, PyObject* const* a, Py_ssize_t n) {
     int dev = -1, x[6];
     PLAIN(plain(a[0], kn, dev) && plain(a[1], vn, dev) && plain(a[2], kc, dev) && plain(a[3], vc, dev) && plain(a[4], table, dev) && plain(a[5], lens, dev));
     for (int i = 0; i < 6; ++i) PLAIN(as_int(a[6 + i], x[i]) && x[i] >= 1);
-    const int64_t need = (int64_t)x[0] * x[1] * x[2] * x[3];
-    PLAIN(kn->numel() >= need && vn->numel() >= need && table->scalar_type() == at::kInt && lens->scalar_type() == at::kInt);
+    PLAIN(holds(*kn, x[0], x[1], x[2], x[3]) && holds(*vn, x[0], x[1], x[2], x[3]) && table->scalar_type() == at::kInt && lens->scalar_type() == at::kInt);
     void* st = stream_of(dev);
     int code;
     WITHOUT_GIL(code = lib.append(kn->const_data_ptr(), vn->const_data_ptr(), kc->data_ptr(), vc->data_ptr(), table->const_data_ptr<int>(),
