@@ -1,6 +1,6 @@
 """Builds the attention library for sm_100a with nvcc, in-tree (luma_b200/lib/): the static archive
 libflash_attn.a the reference crate links (`static=flash_attn`, luma-flash-attn/build.rs:147-148),
-libflash_attn.so for ctypes, and _host.so, the Python front end's native host path.
+libflash_attn.so for ctypes, and _host.*.so, the Python front end's native host path.
 
 Mirrors what luma-flash-attn/build.rs:47-253 does for the reference crate — find nvcc
 (CUDA_HOME / CUDA_PATH / CUDA_ROOT, then PATH), compile every kernels translation unit, `ar rcs`
@@ -24,7 +24,15 @@ LIB_DIR = ROOT / "lib"
 LIB_PATH = LIB_DIR / "libflash_attn.so"
 
 ARCHIVE_PATH = LIB_DIR / "libflash_attn.a"
-HOST_PATH = LIB_DIR / "_host.so"   # the Python front end's native host path (csrc/host_fast.cpp)
+
+
+def host_path_file() -> Path:
+    """The Python front end's native host path (csrc/host_fast.cpp), built against this Python's and this torch's headers: both
+    are in the name, so that an extension of another installation is neither loaded nor taken for built."""
+    import importlib.metadata
+    import sysconfig
+    return LIB_DIR / f"_host.{sysconfig.get_config_var('SOABI')}.torch-{importlib.metadata.version('torch')}.so"
+
 
 SOURCES = ["api.cu", "tile_simt.cu", "tile_f32.cu", "decode_splitk.cu", "prefill_tcgen05.cu", "kv_append.cu", "softmax_lastdim.cu", "comm.cu", "host_pipe.cu"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -59,7 +67,7 @@ def _host_command(src: Path) -> list[str]:
     cuda = Path(find_nvcc()).resolve().parent.parent
     includes = [torch_dir / "include", torch_dir / "include" / "torch" / "csrc" / "api" / "include", cuda / "include",
                 Path(sysconfig.get_paths()["include"])]
-    return ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", *[f"-I{p}" for p in includes], str(src), "-o", str(HOST_PATH),
+    return ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", *[f"-I{p}" for p in includes], str(src), "-o", str(host_path_file()),
             f"-L{torch_dir / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
 
 
@@ -87,7 +95,9 @@ def build(force: bool = False, verbose: bool = False, trace: bool = False) -> Pa
             procs.append((name, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     host = None
     host_src = CSRC / "host_fast.cpp"
-    if force or _stale(HOST_PATH, [host_src]):
+    if force or _stale(host_path_file(), [host_src, *(ROOT.parent / "include").glob("*.h")]):
+        for old in LIB_DIR.glob("_host*.so"):
+            old.unlink()
         host = subprocess.Popen(_host_command(host_src), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     failed = False
     if host is not None:

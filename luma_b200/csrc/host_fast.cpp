@@ -16,23 +16,40 @@
 #include <cstdint>
 #include <cstring>
 #include <exception>
+#include <type_traits>
+
+#include "../../include/flash_attn.h"
+#include "../../include/luma_nn_kernels.h"
 
 namespace {
 
 using Tensor = at::Tensor;
 
-// The C ABI (include/flash_attn.h, include/luma_nn_kernels.h), by storage type: f32, f16, bf16. Addresses come from
+// The C ABI's functions by storage type (f32, f16, bf16), with every pointer as void*: the types are made from the
+// headers' declarations, so that a changed argument list does not compile here. Addresses come from
 // the ctypes handle of the library, so that both front ends drive the same copy of it.
-using BatchFn = int (*)(const void*, const void*, const void*, void*, int, int, int, int, int, int, int, float, const uint8_t*, void*);
-using BatchLseFn = int (*)(const void*, const void*, const void*, void*, float*, int, int, int, int, int, int, int, float, const uint8_t*, void*);
-using VarlenFn = int (*)(const void*, const void*, const void*, void*, const int*, const int*, const int*, int, int, int, int, int, int,
-                         int, int, int, float, void*);
-using VarlenTotalFn = int (*)(const void*, const void*, const void*, void*, const int*, const int*, const int*, int, int, int, int, int, int,
-                         int, int, int, float, int, int, void*);
-using KvFn = int (*)(const void*, const void*, const void*, void*, const int*, const int*, int, int, int, int, int, int, int, float, void*);
-using AppendFn = int (*)(const void*, const void*, void*, void*, const int*, const int*, int, int, int, int, int, int, int, void*);
-using SoftmaxFn = int (*)(const void*, void*, long long, int, void*);
-using ErrorFn = const char* (*)();
+template <class A> struct Erased { using type = A; };
+template <class A> struct Erased<A*> { using type = void*; };
+template <class A> struct Erased<const A*> { using type = const void*; };
+template <class F> struct ErasedFn;
+template <class... A> struct ErasedFn<int(A...)> { using type = int (*)(typename Erased<A>::type...); };
+#define ERASED(fn) ErasedFn<decltype(fn)>::type
+#define SAME(T, ...) static_assert(all_same<T, __VA_ARGS__>, #T)
+template <class T, class... U> constexpr bool all_same = (std::is_same_v<T, U> && ...);
+using BatchFn = ERASED(flash_attn_f32);
+using BatchLseFn = ERASED(flash_attn_f32_lse);
+using VarlenFn = ERASED(flash_attn_varlen_f32);
+using VarlenTotalFn = ERASED(flash_attn_varlen_f16_total);
+using KvFn = ERASED(flash_attn_with_kvcache_f32);
+using AppendFn = ERASED(flash_attn_kvcache_append);
+using SoftmaxFn = ERASED(luma_softmax_f32);
+using ErrorFn = decltype(&flash_attn_last_error);
+SAME(BatchFn, ERASED(flash_attn_f16), ERASED(flash_attn_bf16));
+SAME(BatchLseFn, ERASED(flash_attn_f16_lse), ERASED(flash_attn_bf16_lse));
+SAME(VarlenFn, ERASED(flash_attn_varlen_f16), ERASED(flash_attn_varlen_bf16));
+SAME(VarlenTotalFn, ERASED(flash_attn_varlen_bf16_total));
+SAME(KvFn, ERASED(flash_attn_with_kvcache_f16), ERASED(flash_attn_with_kvcache_bf16));
+SAME(SoftmaxFn, ERASED(luma_softmax_f16), ERASED(luma_softmax_bf16));
 
 struct Library {
     BatchFn batch[3];

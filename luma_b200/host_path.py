@@ -1,28 +1,22 @@
-"""Loads luma_b200/lib/_host.so (csrc/host_fast.cpp), the native host path of the calls whose arguments are exactly
-what an entry point takes, and hands it the C ABI's addresses from the ctypes handle in `ffi`.
+"""Loads the native host path (csrc/host_fast.cpp, built into luma_b200/lib/ with the library) of the calls whose arguments are
+exactly what an entry point takes, and hands it the C ABI's addresses from the ctypes handle in `ffi`.
 
 Each function returns None, having done nothing, for anything it does not take; `high` and `low` then go
-on in Python. The extension is built with the library (luma_b200/build.py); a missing one is an ImportError.
+on in Python. An extension that was not built for this Python and this torch is not loaded: every call then takes the Python
+path, with the same results and more host time, after one warning.
 """
 from __future__ import annotations
 
 import ctypes
 import importlib.machinery
 import importlib.util
-from pathlib import Path
+import warnings
 
 import torch  # noqa: F401  (the extension links against the libraries that this import loads)
 
-from . import error, ffi
+from . import build, error, ffi
 
-PATH = Path(__file__).resolve().parent / "lib" / "_host.so"
-
-if not PATH.exists():
-    raise ImportError(f"{PATH} is missing: build it with `python -m luma_b200.build`")
-
-_loader = importlib.machinery.ExtensionFileLoader("_host", str(PATH))
-_native = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host", _loader))
-_loader.exec_module(_native)
+PATH = build.host_path_file()
 
 
 def _addresses():
@@ -33,11 +27,24 @@ def _addresses():
     return tuple(ctypes.cast(getattr(ffi.lib, n), ctypes.c_void_p).value for n in names)
 
 
-_native.bind(error.from_status, _addresses())
+def _load():
+    try:
+        loader = importlib.machinery.ExtensionFileLoader("_host", str(PATH))
+        native = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host", loader))
+        loader.exec_module(native)
+        native.bind(error.from_status, _addresses())
+        return native
+    except ImportError as e:
+        warnings.warn(f"luma_b200: the native host path is not available ({e}); calls go through Python. "
+                      "Build it with `python -m luma_b200.build`.", RuntimeWarning, stacklevel=2)
+        return None
 
-attn = _native.attn
-low_attn = _native.low_attn
-varlen = _native.varlen
-kvcache = _native.kvcache
-append = _native.append
-softmax = _native.softmax
+
+def _not_taken(*_):
+    return None
+
+
+_native = _load()
+
+attn, low_attn, varlen, kvcache, append, softmax = (getattr(_native, name, _not_taken)
+                                                    for name in ("attn", "low_attn", "varlen", "kvcache", "append", "softmax"))

@@ -18,3 +18,26 @@ def test_sizes_whose_product_does_not_fit_64_bits_are_too_large_for_any_buffer()
     i = torch.zeros(4, dtype=torch.int32, device="cuda")
     with pytest.raises(E.BufferTooSmall):
         low.kvcache_append(t, t, t, t, i, i, 1 << 16, 1 << 16, 1 << 25, 128, 16, 1)
+
+
+def test_an_extension_of_another_installation_is_not_loaded(monkeypatch, tmp_path):
+    # the file's name says which Python and which torch it was built for; without it the front end works, in Python
+    import importlib.metadata
+    import sysconfig
+
+    from luma_b200 import build, host_path
+    assert sysconfig.get_config_var("SOABI") in build.host_path_file().name and importlib.metadata.version("torch") in build.host_path_file().name
+    assert host_path.PATH == build.host_path_file() and host_path._load() is not None
+    monkeypatch.setattr(host_path, "PATH", tmp_path / "_host.other.so")
+    with pytest.warns(RuntimeWarning, match="python -m luma_b200.build"):
+        assert host_path._load() is None
+    assert host_path._not_taken(1, 2, 3) is None
+
+
+def test_the_extension_is_rebuilt_when_a_declaration_changes(monkeypatch, tmp_path):
+    from luma_b200 import build
+    asked = []
+    monkeypatch.setattr(build, "_stale", lambda target, deps: asked.append((target, [d.name for d in deps])) or False)
+    build.build()
+    deps = dict(asked)[build.host_path_file()]
+    assert {"host_fast.cpp", "flash_attn.h", "luma_nn_kernels.h"} <= set(deps)
