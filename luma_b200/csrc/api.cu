@@ -435,9 +435,11 @@ int dispatch(const AttnParams& p, cudaStream_t stream) {
     if (!get_option_force_generic()) {
         int rc = launch_decode_splitk(p, stream);
         if (rc >= 0) return rc;
-        rc = launch_few_rows(p, stream);
+        rc = launch_few_rows(p, true, stream);
         if (rc >= 0) return rc;
         rc = launch_prefill_tcgen05(p, stream);
+        if (rc >= 0) return rc;
+        rc = launch_few_rows(p, false, stream);   // (e.g. pages that do not divide 128 keys)
         if (rc >= 0) return rc;
         rc = launch_tile_f32(p, stream);
         if (rc >= 0) return rc;

@@ -189,8 +189,8 @@ struct RowsPlan {
 int launch_tile_simt(const AttnParams& p, cudaStream_t stream);
 int launch_tile_f32(const AttnParams& p, cudaStream_t stream);
 int launch_decode_splitk(const AttnParams& p, cudaStream_t stream);
-// The same kernel for a few query rows per sequence through any entry point.
-int launch_few_rows(const AttnParams& p, cudaStream_t stream);
+// The same kernel for a few query rows per sequence through any entry point, where it is the faster one.
+int launch_few_rows(const AttnParams& p, bool prefill_takes_it, cudaStream_t stream);
 // The same kernel for those sequences of a packed batch that have few query rows (the host does not know which),
 // launched behind the prefill kernel, which leaves out sequences of at most max_rows rows (query tokens x group).
 // prepare_mixed_few_rows() does what can fail, before that kernel is launched; max_rows == 0: not for this call.

@@ -974,24 +974,35 @@ int launch_decode_splitk(const AttnParams& p, cudaStream_t stream) {
     return rc == FLASH_ATTN_OK ? launch_prepared(p, rows, false, plan, ws, stream) : rc;
 }
 
-// Whether few query rows (per KV head) over a range of `keys` are better off here than on the tensor-core prefill
-// kernel, whose CTAs walk a whole K/V range each, for one or two 128-row tiles of which almost all rows are empty.
-// That kernel takes about 5 us plus 1.7 us per 128 keys, times the waves of its CTAs: up to 12 tiles in one
-// wave (25 us at most) it keeps the call; beyond, the cut of the K/V ranges over the whole device wins at any
-// size (16 sequences x 4 tokens x 4 heads over 512-8192 keys: 63 us against 175; 8 rows of 4000 keys, f16: 27 against
-// 62; 26 single tokens over 802 keys: 21 against 58).
-static bool worth_cutting(const AttnParams& p, long long rows) {
-    const long long keys = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
-    const long long tile_pairs = ((long long)(p.q_heads / p.kv_heads) * ((p.q_seq_len + 127) / 128) + 1) / 2 * p.kv_heads * p.num_seqs;
-    return rows > 0 && (keys > 12 * 128 || tile_pairs > sm_count());
+// ---- this kernel or the prefill kernel, for calls that both take: the time of each, in microseconds, from what the host knows.
+// Prefill kernel: a CTA per pair of 128-row tiles, one per SM; a CTA walks its K/V range at 1.7 us per 128 keys after 5 us of set-up.
+static long long longest_keys(const AttnParams& p) { return p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len; }
+static long long tile_pairs(const AttnParams& p, long long q_len) { return ((long long)(p.q_heads / p.kv_heads) * ((q_len + 127) / 128) + 1) / 2 * p.kv_heads; }
+static double prefill_us(const AttnParams& p, double pairs) {
+    return std::max(1.0, pairs / sm_count()) * (5.0 + 1.7 * (double)((longest_keys(p) + 127) / 128));
+}
+// This kernel: a CTA slot takes 1.2 us per unit of 64 keys (16 rows of one KV head) and 3 us + 0.2 us a row per sequence, most of it the merge of its
+// warps' parts; where sequences are cut, the merge of their parts is another 0.4 us a row.
+static double rows_us(const AttnParams& p, long long seqs, long long rows) {
+    const long long slots = (long long)sm_count() * (p.head_size == 128 ? Smem<128>::kCtasPerSm : p.head_size == 64 ? Smem<64>::kCtasPerSm : Smem<32>::kCtasPerSm);
+    const double units = (double)((longest_keys(p) + kUnit - 1) / kUnit), nrows = (double)std::min<long long>(kRows, rows);
+    const double blocks_per_slot = (double)(seqs * p.kv_heads * ((rows + kRows - 1) / kRows)) / (double)slots;
+    return 5.0 + (1.2 * units + 3.0 + 0.2 * nrows) * blocks_per_slot + (units * blocks_per_slot < units ? 0.4 * nrows : 0.0);
 }
 
-int launch_few_rows(const AttnParams& p, cudaStream_t stream) {
+// Up to four row blocks of 16 (query token x group head) rows, each of which reads the K/V rows again, from L2. The prefill kernel's one or two
+// tiles per CTA are almost empty, but it reads K/V once: over up to 12 tiles in one wave of its CTAs (25 us at most) it keeps the call,
+// else the estimates decide. Both kernels over 286 shapes (1-64 sequences x 1-64 tokens, 64-8192 keys, groups of 1, 4
+// and 8): the choice is at most 3 % slower than the prefill kernel anywhere and 1.3 % off the better one on average. 64 rows:
+// 64 x 64 tokens x 1600 keys, 32 heads without GQA 275 us on the prefill kernel, 743 here; 1 x 16 x 8192, 32/8 heads 110 and 31. 16 rows: 16 x 4 x
+// 8192, 32/8: 180 and 63.
+int launch_few_rows(const AttnParams& p, bool prefill_takes_it, cudaStream_t stream) {
     if (p.n_out > 0 || !rows_kernel_takes(p)) return -1;
     const long long rows = (long long)p.q_seq_len * (p.q_heads / p.kv_heads);
-    // up to four row blocks: each reads the K/V rows again, from L2 (28 rows of 7 x 1355-5421 keys: 43 us against
-    // 87 on the prefill kernel; 32 rows of 8 x 3108: 45 against 109)
-    if (rows > 4 * kRows || !worth_cutting(p, rows)) return -1;
+    if (rows <= 0 || rows > 4 * kRows) return -1;
+    const double pairs = (double)tile_pairs(p, p.q_seq_len) * p.num_seqs;
+    if (longest_keys(p) <= 12 * 128 && pairs <= sm_count()) return -1;
+    if (prefill_takes_it && rows_us(p, p.num_seqs, rows) >= prefill_us(p, pairs)) return -1;
     RowsPlan plan;
     Workspace ws;
     if (prepare_rows(p, (int)rows, stream, plan, ws) != FLASH_ATTN_OK) return -1;   // the prefill kernel needs no memory of the library's
@@ -1004,7 +1015,8 @@ MixedFewRows prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {
     const int group = p.q_heads / p.kv_heads;
     // one row block: the CTA slots are shared out before anybody knows how many rows the sequences have
     // prompts packed back to back with their own K/V: few rows would see few keys
-    if (group > kRows || !worth_cutting(p, kRows) || (!p.paged && p.kv_seq_len <= p.q_seq_len)) return few;
+    if (group > kRows || (longest_keys(p) <= 12 * 128 && tile_pairs(p, p.q_seq_len) * p.num_seqs <= sm_count()) || (!p.paged && p.kv_seq_len <= p.q_seq_len))
+        return few;
     if (prepare_rows(p, kRows, stream, few.plan, few.ws) == FLASH_ATTN_OK) few.max_rows = kRows;
     return few;
 }
