@@ -67,6 +67,18 @@ int check_launch(const char* what) {
     return FLASH_ATTN_OK;
 }
 
+int sm_count() {
+    static std::atomic<int> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    int n = known[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        known[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 // ---- split-K workspace: one buffer per (device, stream) -----------------------------------
 // Allocation and release are stream-ordered (cudaMallocAsync / cudaFreeAsync on the stream that
 // uses the buffer): growing a workspace neither takes a device-wide synchronisation nor frees

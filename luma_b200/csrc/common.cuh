@@ -150,6 +150,8 @@ int get_option_prefill_order();         // 1 = heaviest-first launch order even 
 int get_option_prefill_wait_us();       // bound of the tcgen05 kernel's waits in microseconds (0 = the default, 2 s)
 int get_option_prefill_test_skip_k();   // test hook: 1 + index of a K tile the producer never requests (0 = off)
 
+int sm_count();   // of the current device
+
 // Returns FLASH_ATTN_OK or FLASH_ATTN_ERR_CUDA (with last error set) after a launch.
 int check_launch(const char* what);
 

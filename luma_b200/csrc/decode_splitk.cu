@@ -797,18 +797,6 @@ int num_columns(int per_column, int ctas_per_sm, int sms) {
     return one_fills ? one : two;
 }
 
-int sm_count() {
-    static std::atomic<int> known[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    int n = known[dev].load(std::memory_order_relaxed);
-    if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        known[dev].store(n, std::memory_order_relaxed);
-    }
-    return n;
-}
-
 // `rows`: query rows per KV head at most; `max_tokens`: upper bound of a sequence's visible keys.
 template <int D>
 RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, bool allow_forced) {

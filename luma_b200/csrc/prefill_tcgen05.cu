@@ -1519,10 +1519,7 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     {
         const int rows = (pairs + band - 1) / band;
         const int per_row = p.kv_heads * p.num_seqs * band;
-        int sms = 148;
-        int dev = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int w = (sms + per_row - 1) / per_row;
+        const int w = (sm_count() + per_row - 1) / per_row;
         const int m = w > 0 ? rows / w : 0;
         const bool spread = p.n_out > 1 && get_option_prefill_order() != 1 && m >= 2;
         a.spread_w = spread ? w : 0;

@@ -461,7 +461,7 @@ int launch_tile_f32(const AttnParams& p, cudaStream_t stream) {
         return -1;
     const long long rows = (long long)p.q_seq_len * (p.q_heads / p.kv_heads);
     if (rows > 0x7fffffffLL - 64) return -1;
-    const bool large = (rows + 63) / 64 * p.kv_heads * p.num_seqs >= 2 * 148;
+    const bool large = (rows + 63) / 64 * p.kv_heads * p.num_seqs >= 2LL * sm_count();   // two CTAs per SM
     if (p.head_size == 128) return large ? launch_one<128, 4>(p, stream) : launch_one<128, 2>(p, stream);
     if (p.head_size == 64) return large ? launch_one<64, 4>(p, stream) : launch_one<64, 1>(p, stream);
     return large ? launch_one<32, 4>(p, stream) : launch_one<32, 1>(p, stream);
