@@ -201,6 +201,10 @@ struct MixedFewRows {
     RowsPlan plan;
     Workspace ws;
 };
+struct PackedMix {
+    long long prompts, few;   // sequences of a packed batch, an estimate from its number of rows (not known: all prompts)
+};
+PackedMix packed_mix(const AttnParams& p);
 MixedFewRows prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream);
 int launch_mixed_few_rows(const AttnParams& p, const MixedFewRows& few, cudaStream_t stream);
 int launch_prefill_tcgen05(const AttnParams& p, cudaStream_t stream);

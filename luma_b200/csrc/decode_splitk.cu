@@ -997,14 +997,39 @@ int launch_few_rows(const AttnParams& p, bool prefill_takes_it, cudaStream_t str
     return launch_prepared(p, (int)rows, false, plan, ws, stream);
 }
 
+// A packed batch of prompts (or chunks of them) and sequences with few rows: from the number of rows, as many sequences with max_seqlen_q
+// rows as they make; the others may have few.
+PackedMix packed_mix(const AttnParams& p) {
+    PackedMix m{p.num_seqs, 0};
+    if (p.mode != MODE_VARLEN || p.total_q <= 0) return m;
+    if (p.q_seq_len > 1) m.prompts = std::min<long long>(p.num_seqs, std::max<long long>(1, ((long long)p.total_q - p.num_seqs + p.q_seq_len - 2) / (p.q_seq_len - 1)));
+    else m.prompts = 0;
+    m.few = p.num_seqs - m.prompts;
+    return m;
+}
+
+// Whether the few-row sequences of a packed batch are better off behind the prefill kernel than in its grid, where each takes a
+// CTA per two heads of its group: only where they make waves of those, by the estimates above and a fifth more, since the second launch
+// starts when that kernel's last CTA has. Over 238 paged mixes (1-6 prompts, chunks of 64 or 512, 0-128 single tokens, contexts of
+// 64-8192, four head layouts) no mix is then slower than with everything in the prefill grid, and the choice is 3 % off the better one on average:
+// 4 x 512 with 32 tokens over 512-8192, 32/8 heads: 435 us in one grid, 231 so; with 1 token: 131 in one grid, 152 with two kernels, which
+// one grid keeps. Without the row count of the packed buffers (the C ABI's plain entry point) nothing is known of the mix, and
+// long contexts go to two kernels.
+static bool mixed_few_rows_are_better(const AttnParams& p) {
+    if (p.total_q <= 0) return longest_keys(p) > 12 * 128 || tile_pairs(p, p.q_seq_len) * p.num_seqs > sm_count();
+    const PackedMix m = packed_mix(p);
+    if (m.few <= 0) return false;
+    const double prompts = (double)m.prompts * tile_pairs(p, p.q_seq_len), few = (double)m.few * tile_pairs(p, 1);
+    return prefill_us(p, prompts + few) > 1.2 * (prefill_us(p, prompts) + rows_us(p, m.few, p.q_heads / p.kv_heads));
+}
+
 MixedFewRows prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {
     MixedFewRows few;
     if (p.mode != MODE_VARLEN || p.num_seqs < 2 || p.n_out > 0 || !rows_kernel_takes(p)) return few;
     const int group = p.q_heads / p.kv_heads;
     // one row block: the CTA slots are shared out before anybody knows how many rows the sequences have
     // prompts packed back to back with their own K/V: few rows would see few keys
-    if (group > kRows || (longest_keys(p) <= 12 * 128 && tile_pairs(p, p.q_seq_len) * p.num_seqs <= sm_count()) || (!p.paged && p.kv_seq_len <= p.q_seq_len))
-        return few;
+    if (group > kRows || (!p.paged && p.kv_seq_len <= p.q_seq_len) || !mixed_few_rows_are_better(p)) return few;
     if (prepare_rows(p, kRows, stream, few.plan, few.ws) == FLASH_ATTN_OK) few.max_rows = kRows;
     return few;
 }

@@ -90,7 +90,8 @@ def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q: in
     q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
     o = torch.empty_like(q)
     low.flash_attn_varlen(q, k, v, o, cu_seqlens_q.contiguous(), cu_seqlens_k.contiguous(), num_seqs,
-                          int(max_seqlen_q), int(max_seqlen_k), hq, hkv, d, scale, block_table, block_size)
+                          int(max_seqlen_q), int(max_seqlen_k), hq, hkv, d, scale, block_table, block_size,
+                          total_q=total_q, total_k=None if block_table is not None else k.shape[0])
     return o
 
 

@@ -103,8 +103,8 @@ def flash_attn_varlen(q, k, v, o, cu_seqlens_q, cu_seqlens_k, num_seqs, max_seql
     cache and max_blocks is inferred as block_tables.numel() // num_seqs (low.rs:266-269).
     The call goes through the reference's symbol. When the caller gives the row counts of the packed
     buffers (`total_q`, and `total_k` unless paged) and the storage is 16-bit, they go along through
-    the additive `flash_attn_varlen_<T>_total` entry point and bound the tensor maps as well; the
-    results are bit-identical either way."""
+    the additive `flash_attn_varlen_<T>_total` entry point: they bound the tensor maps, and tell a batch
+    of prompts from one with many decoding sequences, which then run on a kernel of their own."""
     sfx = _suffix(q)
     k_paged = 1 if block_tables is not None else 0
     max_blocks = (block_tables.numel() // num_seqs) if (block_tables is not None and num_seqs > 0) else 0

@@ -24,3 +24,28 @@ def test_few_rows_go_to_the_faster_kernel(b, s, kv, hq, hkv, d, path):
     high.flash_attn_func(q, k, k, start_pos=kv - s)
     torch.cuda.synchronize()
     assert ffi.last_path() == path
+
+
+def _packed(q_lens, k_lens, hq, hkv, d, page=16):
+    cu = [torch.tensor([0] + x, dtype=torch.int32).cumsum(0).int().cuda() for x in (q_lens, k_lens)]
+    pages = -(-max(k_lens) // page)
+    k = torch.zeros(len(k_lens) * pages, page, hkv, d, dtype=torch.bfloat16, device="cuda")
+    table = torch.arange(len(k_lens) * pages, dtype=torch.int32, device="cuda").view(len(k_lens), pages)
+    q = torch.zeros(sum(q_lens), hq, d, dtype=torch.bfloat16, device="cuda")
+    high.flash_attn_varlen_func(q, k, k, *cu, max(q_lens), max(k_lens), block_table=table)
+    torch.cuda.synchronize()
+    assert ffi.last_path() == "prefill_tcgen05"
+    return ffi.last_launches()
+
+
+@pytest.mark.parametrize("q_lens,keys,hq,hkv,d,launches", [
+    ([512] * 4, 8192, 32, 8, 128, 1),                # no room for few rows next to the prompts
+    ([512] * 4 + [1], 8192, 32, 8, 128, 1),          # a few that fill up the prefill grid's last wave
+    ([64] + [1] * 8, 2048, 32, 8, 128, 1),           # all in one wave
+    ([64] * 2 + [1] * 32, 2048, 8, 2, 64, 1),
+    ([512] * 4 + [1] * 32, 8192, 32, 8, 128, 2),     # waves of almost empty tiles
+    ([64] + [1] * 128, 512, 32, 8, 128, 2),
+    ([512] + [1] * 32, 2048, 64, 8, 64, 2),
+])
+def test_few_rows_of_a_packed_batch_leave_the_prefill_grid_where_they_make_waves(q_lens, keys, hq, hkv, d, launches):
+    assert _packed(q_lens, [max(keys, n) for n in q_lens], hq, hkv, d) == launches
