@@ -1556,12 +1556,19 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     const int streams_per_group = (int)(((long long)p.kv_heads * p.num_seqs + groups - 1) / groups);
     dim3 grid(streams_per_group * band, (pairs + band - 1) / band, groups);
     a.pairs = pairs;
+    const MixedFewRows few = prepare_mixed_few_rows(p, stream);   // its workspace is this call's until both kernels are launched
+    a.skip_rows = few.max_rows;
     // Ordered: chunks of prompts, at most half as long as the context may be. Whole prompts keep grid order, which is heaviest
-    // first for them already: finding the pair costs a CTA about 1 us, and a packed batch of prompts has thousands of short
-    // ones (24 prompts of 17-2000 tokens: 394 us ordered, 376 in grid order).
+    // first for them already. Finding its pair costs a CTA 1 to 2 us; what it wins is one late long pair, about a fifth of the longest pair's
+    // 1.7 us per K/V tile, and nothing where all pairs start at once. So: more than one wave of pairs, and at least five tiles in the longest for
+    // each. 4 chunks of 300 over 2048-8192 keys, 32/8 heads (1.3 waves) 148 us in grid order, 116 ordered; 16 chunks of 300 over 512-2048,
+    // 32/32 heads (7 waves) 159 and 170; 4 chunks of 64 over 128-512 (less than a wave) 14.7 and 16.2.
     const long long kv_rows = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
+    const PackedMix mix = packed_mix(p);
+    const double waves = (double)(mix.prompts * pairs + (a.skip_rows > 0 ? 0 : mix.few * ((group + 1) / 2))) * p.kv_heads / sm_count();
+    const bool worth_ordering = waves > 1.0 && (double)((kv_rows + kBlockN - 1) / kBlockN) > 5.0 * waves;
     if (kPaged && p.num_seqs >= 2 && p.num_seqs <= kOrderMax && 2LL * p.q_seq_len <= kv_rows && get_option_prefill_band() <= 0 &&
-        get_option_prefill_groups() <= 0) {
+        get_option_prefill_groups() <= 0 && (worth_ordering || get_option_prefill_order() == 2)) {
         a.ordered = 1;
         long long ctas = (long long)p.num_seqs * p.kv_heads * pairs;
         if (p.total_q > 0)   // a sequence of n rows has (group * ceil(n / 128) + 1) / 2 pairs
@@ -1569,8 +1576,6 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
         if (ctas <= 0 || ctas > 0x7fffffffLL) return -1;
         grid = dim3((unsigned)ctas);
     }
-    const MixedFewRows few = prepare_mixed_few_rows(p, stream);   // its workspace is this call's until both kernels are launched
-    a.skip_rows = few.max_rows;
     prefill_tcgen05_kernel<T, D, kMask, kPaged><<<grid, kThreads, smem, stream>>>(qm, km, vm, om, a);
     int rc = check_launch("prefill_tcgen05_kernel");
     if (rc == FLASH_ATTN_OK && a.skip_rows > 0) rc = launch_mixed_few_rows(p, few, stream);
