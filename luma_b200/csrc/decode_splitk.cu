@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -146,8 +147,8 @@ __device__ __forceinline__ float fast_exp2(float x) {
 //   ring : kWarps x kStages x {K tile, V tile}, each tile kTile rows of D elements, 16-byte chunks
 //          XOR-swizzled by the row (row & 7; row & 3 at head_size 32, whose rows hold only four chunks) against
 //          ldmatrix bank conflicts
-//   merge: the warps' partials of a finished sequence, kMergeCols columns at a time — beside the ring, which
-//          already holds tiles of the next sequence by then
+//   merge: the warps' partials of a finished sequence, up to 8 rows whole or 16 rows kMergeCols columns at a time — beside
+//          the ring, which already holds tiles of the next sequence by then
 template <int D>
 struct Smem {
     static constexpr int kRowBytes = D * 2;
@@ -268,6 +269,7 @@ __device__ __forceinline__ void merge_parts(const float* acc0, const float2* ml0
     constexpr int E = D / 32;
     constexpr int kAtOnce = 16 / RW;      // parts in flight per row
     constexpr int kChunk = 64;            // parts whose weights sit in shared memory at a time
+    static_assert(kRows / 2 * (D + 2) <= kRows * Smem<D>::kMergePitch, "half of the rows fit the merge buffer whole");
     static_assert(kRows * kChunk * 4 <= Smem<D>::kMergeBytes, "weights of a chunk fit the merge buffer");
     auto slot_of = [&](int c) { return (long long)c * grid_x * 2 + (c == c_first ? 1 : 0); };
     float o[RW][E], m[RW], l[RW];
@@ -542,7 +544,6 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
 
     // ---- compute side: sequence after sequence ----------------------------------------------------------
     float* const merge = reinterpret_cast<float*>(smem_raw + S::kRingBytes);
-    auto merge_ml = [&](int w, int r) { return reinterpret_cast<float2*>(merge + (w * kRows + r) * S::kMergePitch + S::kMergeCols); };
     int* const last_flag = reinterpret_cast<int*>(smem_raw + S::kRingBytes + S::kMergeBytes);
     const int cta = blockIdx.y * gridDim.x + blockIdx.x;
     int stage = 0;
@@ -690,56 +691,67 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
         l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
         l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
         l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-        if (c4 == 0) {
-            *merge_ml(warp, g) = make_float2(m0, l0);
-            *merge_ml(warp, g + 8) = make_float2(m1, l1);
-        }
+        // Up to 8 rows fit the buffer whole; 16 go through it 64 columns at a time. Rows that do not exist are not written: a CTA does this once per
+        // sequence with nothing of its own in flight but the ring, which is what batches of short contexts are made of
+        // (256 x 128-512 tokens: 32/32 heads 294 us with all 16 rows in two passes, 259 so; 32/8 heads 86.5 and 82). The two are
+        // separate code: with the pitch in a variable 16 sequences x 4 tokens x 4 heads lost 1.5 %.
         const int slot = 2 * cta + (starts ? 1 : 0);
-        float* const mine = merge + warp * kRows * S::kMergePitch;
-#pragma unroll
-        for (int pass = 0; pass < D / S::kMergeCols; ++pass) {
-#pragma unroll
-            for (int n = 0; n < S::kMergeCols / 8; ++n) {
-                const int d = n * 8 + 2 * c4;
-                const float(&x)[4] = acc[pass * (S::kMergeCols / 8) + n];
-                *reinterpret_cast<float2*>(mine + g * S::kMergePitch + d) = make_float2(x[0], x[1]);
-                *reinterpret_cast<float2*>(mine + (g + 8) * S::kMergePitch + d) = make_float2(x[2], x[3]);
+        auto merge_warps = [&](auto few) {
+            constexpr bool kFew = decltype(few)::value;
+            constexpr int kCols = kFew ? D : S::kMergeCols, kPitch = kCols + 2, kSlots = kFew ? kRows / 2 : kRows;
+            auto merge_ml = [&](int w, int r) { return reinterpret_cast<float2*>(merge + (w * kSlots + r) * kPitch + kCols); };
+            float* const mine = merge + warp * kSlots * kPitch;
+            if (c4 == 0) {
+                if (!kFew || g < nrows) *merge_ml(warp, g) = make_float2(m0, l0);
+                if (!kFew) *merge_ml(warp, g + 8) = make_float2(m1, l1);
             }
-            __syncthreads();
-            for (int idx = threadIdx.x; idx < nrows * (S::kMergeCols / 2); idx += kThreads) {
-                const int r = idx / (S::kMergeCols / 2);
-                const int d = (idx - r * (S::kMergeCols / 2)) * 2;
-                float2 ml[kWarps];
-                float mstar = -INFINITY;
 #pragma unroll
-                for (int w = 0; w < kWarps; ++w) {
-                    ml[w] = *merge_ml(w, r);
-                    mstar = fmaxf(mstar, ml[w].x);
-                }
-                float ox = 0.0f, oy = 0.0f, l = 0.0f;
+            for (int pass = 0; pass < D / kCols; ++pass) {
 #pragma unroll
-                for (int w = 0; w < kWarps; ++w) {
-                    const float wgt = ml[w].x == -INFINITY ? 0.0f : fast_exp2(ml[w].x - mstar);
-                    const float2 x = *reinterpret_cast<const float2*>(merge + (w * kRows + r) * S::kMergePitch + d);
-                    ox += wgt * x.x;
-                    oy += wgt * x.y;
-                    l += wgt * ml[w].y;
+                for (int n = 0; n < kCols / 8; ++n) {
+                    const int d = n * 8 + 2 * c4;
+                    const float(&x)[4] = acc[pass * (kCols / 8) + n];
+                    if (!kFew || g < nrows) *reinterpret_cast<float2*>(mine + g * kPitch + d) = make_float2(x[0], x[1]);
+                    if (!kFew) *reinterpret_cast<float2*>(mine + (g + 8) * kPitch + d) = make_float2(x[2], x[3]);
                 }
-                const int dd = pass * S::kMergeCols + d;
-                if (starts && ends) {   // the whole sequence: finished here
-                    const float inv = l > 0.0f ? 1.0f / l : 0.0f;   // reference: flash_attn_with_kvcache.cu:109
-                    const int t = (row0 + r) / group, h = kvh * group + (row0 + r) - t * group;
-                    const unsigned w2 = pack2<T>(ox * inv, oy * inv);
-                    store_pair<T>(a.out, seq.q_row0 + t, h, D, dd, w2);
-                    if (dd == 0 && a.out.lse != nullptr)
-                        a.out.lse[((long long)s * a.q_heads + h) * a.q_seq_len + t] = l > 0.0f ? (mstar + log2f(l)) * 0.6931471805599453f : -INFINITY;
-                } else {
-                    *reinterpret_cast<float2*>(a.ws_acc + ((long long)slot * kRows + r) * D + dd) = make_float2(ox, oy);
-                    if (dd == 0) a.ws_ml[(long long)slot * kRows + r] = make_float2(mstar, l);
+                __syncthreads();
+                for (int idx = threadIdx.x; idx < nrows * (kCols / 2); idx += kThreads) {
+                    const int r = idx / (kCols / 2);
+                    const int d = (idx - r * (kCols / 2)) * 2;
+                    float2 ml[kWarps];
+                    float mstar = -INFINITY;
+#pragma unroll
+                    for (int w = 0; w < kWarps; ++w) {
+                        ml[w] = *merge_ml(w, r);
+                        mstar = fmaxf(mstar, ml[w].x);
+                    }
+                    float ox = 0.0f, oy = 0.0f, l = 0.0f;
+#pragma unroll
+                    for (int w = 0; w < kWarps; ++w) {
+                        const float wgt = ml[w].x == -INFINITY ? 0.0f : fast_exp2(ml[w].x - mstar);
+                        const float2 x = *reinterpret_cast<const float2*>(merge + (w * kSlots + r) * kPitch + d);
+                        ox += wgt * x.x;
+                        oy += wgt * x.y;
+                        l += wgt * ml[w].y;
+                    }
+                    const int dd = pass * kCols + d;
+                    if (starts && ends) {   // the whole sequence: finished here
+                        const float inv = l > 0.0f ? 1.0f / l : 0.0f;   // reference: flash_attn_with_kvcache.cu:109
+                        const int t = (row0 + r) / group, h = kvh * group + (row0 + r) - t * group;
+                        const unsigned w2 = pack2<T>(ox * inv, oy * inv);
+                        store_pair<T>(a.out, seq.q_row0 + t, h, D, dd, w2);
+                        if (dd == 0 && a.out.lse != nullptr)
+                            a.out.lse[((long long)s * a.q_heads + h) * a.q_seq_len + t] = l > 0.0f ? (mstar + log2f(l)) * 0.6931471805599453f : -INFINITY;
+                    } else {
+                        *reinterpret_cast<float2*>(a.ws_acc + ((long long)slot * kRows + r) * D + dd) = make_float2(ox, oy);
+                        if (dd == 0) a.ws_ml[(long long)slot * kRows + r] = make_float2(mstar, l);
+                    }
                 }
+                __syncthreads();   // the buffer is written again by the next pass or sequence
             }
-            __syncthreads();   // the buffer is written again by the next pass or sequence
-        }
+        };
+        if (nrows <= kRows / 2) merge_warps(std::true_type{});
+        else merge_warps(std::false_type{});
 
         if (!(starts && ends)) {
             // ---- a cut sequence: whoever brings the last part merges all of them, in column order --------

@@ -72,3 +72,43 @@ def test_length_beyond_the_block_table_is_cut_at_its_capacity(chunk, new):
             H.assert_bf16_close(got, want, "after")
     finally:
         ffi.lib.flash_attn_set_option(b"decode_chunk_tokens", 0)
+
+
+def test_more_kv_heads_than_cta_slots_without_a_cut():
+    # 1200 KV heads leave one column: every sequence is finished by one CTA, and the allocation-free entry point needs no partials
+    lens, h, d, bs = [300, 65], 1200, 64, 16
+    kc, vc, table = H.make_paged_cache(lens, bs, h, d, seed=70)
+    q = H.normal((2, 1, h, d), 71)
+    dq, dk, dv = (H.to_dev(x, "bf16") for x in (q, kc, vc))
+    bt, cl, o = torch.from_numpy(table).cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda"), torch.full_like(dq, float("nan"))
+    want = ob.attn_f64_kvcache(H.round_to(q, "bf16"), H.round_to(kc, "bf16"), H.round_to(vc, "bf16"), lens, table, scale=0.125)
+    for _ in range(2):
+        rc = ffi.lib.flash_attn_decode_bf16_noalloc(dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), o.data_ptr(), bt.data_ptr(), cl.data_ptr(), 2, h, h, d,
+                                                    bs, bt.shape[1], 0.125, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0, ffi.last_error()
+        torch.cuda.synchronize()
+        H.assert_bf16_close(H.to_np(o), want, "noalloc")
+        o.fill_(float("nan"))
+        low.flash_attn_with_kvcache(dq, dk, dv, o, bt, cl, 2, 1, h, h, d, bs, bt.shape[1], 0.125)
+        torch.cuda.synchronize()
+        H.assert_bf16_close(H.to_np(o), want, "workspace")
+
+
+@pytest.mark.parametrize("new,hq,hkv,d", [(4, 8, 2, 128), (9, 2, 2, 64), (3, 8, 1, 32)])
+def test_several_rows_over_pages_with_nan_in_every_unwritten_slot(new, hq, hkv, d):
+    lens, bs = [1701, 65, 2049, 16, new], 16
+    kc, vc, table = H.make_paged_cache(lens, bs, hkv, d, seed=60 + d)
+    q = H.normal((len(lens), new, hq, d), 61)
+    want = ob.attn_f64_kvcache(H.round_to(q, "bf16"), H.round_to(kc, "bf16"), H.round_to(vc, "bf16"), lens, table)
+    written = np.zeros(kc.shape[:2], dtype=bool)
+    for s, n in enumerate(lens):
+        j = np.arange(n)
+        written[table[s, j // bs], j % bs] = True
+    kc[~written] = np.nan
+    vc[~written] = np.nan
+    o = torch.empty(len(lens), new, hq, d, device="cuda", dtype=torch.bfloat16)
+    low.flash_attn_with_kvcache(H.to_dev(q, "bf16"), H.to_dev(kc, "bf16"), H.to_dev(vc, "bf16"), o, torch.from_numpy(table).cuda(),
+                                torch.tensor(lens, dtype=torch.int32, device="cuda"), len(lens), new, hq, hkv, d, bs, table.shape[1], 1.0 / np.sqrt(d))
+    torch.cuda.synchronize()
+    assert ffi.last_path() == "decode_splitk"
+    H.assert_bf16_close(H.to_np(o), want, f"{new} tokens")
