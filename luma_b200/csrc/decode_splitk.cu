@@ -47,7 +47,6 @@ constexpr int kRows = 16;    // query rows served per CTA (M of the mma)
 struct RowsOut {
     void* o[8];
     int n_out, o_heads, o_head0, peer0;
-    int halves;      // a buffer is aligned to its 2-byte elements only: no 4-byte stores
     float* lse;      // MODE_BATCH: (num_seqs, q_heads, q_seq_len) or null
 };
 
@@ -166,7 +165,8 @@ struct Smem {
 };
 
 // Extents of one sequence: its query rows and the keys it sees. Query token i sits at global position
-// pos_off + i and sees keys j < kv_len with j <= pos_off + i.
+// pos_off + i and sees keys j < kv_len with j <= pos_off + i; of a length beyond what the block table holds, kv_len is the part
+// that it holds.
 struct RowsSeq {
     int q_len, kv_len, pos_off;
     long long q_row0, kv_row0;
@@ -176,8 +176,9 @@ __device__ __forceinline__ RowsSeq rows_seq(const RowsArgs& a, int s) {
     RowsSeq r;
     if (a.mode == MODE_KVCACHE) {
         r.q_len = a.q_seq_len;
-        r.kv_len = a.context_lens[s];
-        r.pos_off = r.kv_len - r.q_len;
+        const int len = a.context_lens[s];
+        r.kv_len = min(len, a.capacity);
+        r.pos_off = len - r.q_len;
         r.q_row0 = (long long)s * a.q_seq_len;
         r.kv_row0 = 0;
     } else if (a.mode == MODE_BATCH) {
@@ -189,17 +190,18 @@ __device__ __forceinline__ RowsSeq rows_seq(const RowsArgs& a, int s) {
     } else {
         const int q0 = a.cu_q[s], k0 = a.cu_k[s];
         r.q_len = a.cu_q[s + 1] - q0;
-        r.kv_len = a.cu_k[s + 1] - k0;
-        r.pos_off = r.kv_len - r.q_len;
+        const int len = a.cu_k[s + 1] - k0;
+        r.kv_len = min(len, a.capacity);
+        r.pos_off = len - r.q_len;
         r.q_row0 = q0;
         r.kv_row0 = k0;
     }
     return r;
 }
 
-// Keys that the last query token sees: of a length beyond what the block table holds, the part that it holds.
-__device__ __forceinline__ int rows_visible(const RowsArgs& a, const RowsSeq& r) {
-    const long long v = min((long long)min(r.kv_len, a.capacity), (long long)r.pos_off + r.q_len);
+// Keys that the last query token sees.
+__device__ __forceinline__ int rows_visible(const RowsSeq& r) {
+    const long long v = min((long long)r.kv_len, (long long)r.pos_off + r.q_len);
     return v > 0 ? (int)v : 0;
 }
 
@@ -208,7 +210,7 @@ __device__ __forceinline__ int rows_visible(const RowsArgs& a, const RowsSeq& r)
 __device__ __forceinline__ int rows_units(const RowsArgs& a, const RowsSeq& r, int group, int row0) {
     const int rows = r.q_len * group;
     if (rows <= row0 || rows > a.max_rows) return 0;
-    return max(1, (rows_visible(a, r) + kUnit - 1) / kUnit);
+    return max(1, (rows_visible(r) + kUnit - 1) / kUnit);
 }
 
 // The cut of `total` units into columns: the first `more` columns have share + 1 units, the others share
@@ -243,13 +245,13 @@ __device__ __forceinline__ unsigned long long arrive_acq_rel(unsigned long long*
 }
 
 // Two finished neighbours of an output row, to every output buffer.
-template <typename T>
+template <typename T, bool kHalves>
 __device__ __forceinline__ void store_pair(const RowsOut& out, long long row, int head, int D, int d, unsigned both) {
     const long long off = (row * out.o_heads + out.o_head0 + head) * D + d;
     int pe = out.peer0;
     for (int n = 0; n < out.n_out; ++n) {
         T* const at = static_cast<T*>(out.o[pe]) + off;
-        if (out.halves) {
+        if (kHalves) {
             reinterpret_cast<unsigned short*>(at)[0] = (unsigned short)both;
             reinterpret_cast<unsigned short*>(at)[1] = (unsigned short)(both >> 16);
         } else {
@@ -348,7 +350,9 @@ __device__ __forceinline__ void merge_parts(const float* acc0, const float2* ml0
     }
 }
 
-template <typename T, int D>
+// kHalves: an output buffer is aligned to its 2-byte elements only, rows are stored element by element (a separate instantiation: the
+// branch at each store, and a minimum with the table's capacity at each mask, cost 1 us of the 18 of one sequence with 16 rows to merge).
+template <typename T, int D, bool kHalves>
 __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_kernel(const __grid_constant__ RowsArgs a) {
     using S = Smem<D>;
     constexpr int kChunksPerRow = D / 8;          // 16-byte chunks per K/V row
@@ -482,7 +486,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
     int cp_left = (int)(u_end - u_begin);
     int cp_s = s;
     RowsSeq cp_seq = rows_seq(a, s);
-    int cp_vis = rows_visible(a, cp_seq);
+    int cp_vis = rows_visible(cp_seq);
     int cp_tok = (int)(u_begin - seq_first) * kUnit;   // first token of the unit to copy next
     int cp_end = rows_units(a, cp_seq, group, row0) * kUnit;
     auto look_up = [&]() -> long long {   // element offset of this lane's token row in the caches, -1 past the visible keys
@@ -508,7 +512,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
                     cp_seq = rows_seq(a, ++cp_s);
                     cp_end = rows_units(a, cp_seq, group, row0) * kUnit;
                 } while (cp_end == 0);
-                cp_vis = rows_visible(a, cp_seq);
+                cp_vis = rows_visible(cp_seq);
                 cp_tok = 0;
             }
         }
@@ -555,7 +559,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
             seq = rows_seq(a, ++s);
             units = rows_units(a, seq, group, row0);
         }
-        const int vis = rows_visible(a, seq);
+        const int vis = rows_visible(seq);
         const int nrows = min(kRows, seq.q_len * group - row0);   // query rows served here
         const unsigned seg_end = min(u_end, seq_first + (unsigned)units);
         const bool starts = u == seq_first, ends = seg_end == seq_first + (unsigned)units;
@@ -576,10 +580,10 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
                 qa[kk][2] = v0 ? q0[kk * 8 + 4 + c4] : 0u;
                 qa[kk][3] = v1 ? q1[kk * 8 + 4 + c4] : 0u;
             }
-            lim0 = (int)min((long long)min(seq.kv_len, a.capacity) - 1, (long long)seq.pos_off + t0);
-            lim1 = (int)min((long long)min(seq.kv_len, a.capacity) - 1, (long long)seq.pos_off + t1);
+            lim0 = (int)min((long long)seq.kv_len - 1, (long long)seq.pos_off + t0);
+            lim1 = (int)min((long long)seq.kv_len - 1, (long long)seq.pos_off + t1);
         }
-        const int lim_all = min(min(seq.kv_len, a.capacity), seq.pos_off + 1);   // keys below this are seen by every row
+        const int lim_all = min(seq.kv_len, seq.pos_off + 1);   // keys below this are seen by every row
 
         float acc[kDBlocks][4];
 #pragma unroll
@@ -739,7 +743,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
                         const float inv = l > 0.0f ? 1.0f / l : 0.0f;   // reference: flash_attn_with_kvcache.cu:109
                         const int t = (row0 + r) / group, h = kvh * group + (row0 + r) - t * group;
                         const unsigned w2 = pack2<T>(ox * inv, oy * inv);
-                        store_pair<T>(a.out, seq.q_row0 + t, h, D, dd, w2);
+                        store_pair<T, kHalves>(a.out, seq.q_row0 + t, h, D, dd, w2);
                         if (dd == 0 && a.out.lse != nullptr)
                             a.out.lse[((long long)s * a.q_heads + h) * a.q_seq_len + t] = l > 0.0f ? (mstar + log2f(l)) * 0.6931471805599453f : -INFINITY;
                     } else {
@@ -775,10 +779,10 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
                     if constexpr (D >= 64) {
 #pragma unroll
                         for (int e = 0; e < D / 32; e += 2)
-                            store_pair<T>(a.out, seq.q_row0 + t, h, D, lane * (D / 32) + e, pack2<T>(o[e] * inv, o[e + 1] * inv));
+                            store_pair<T, kHalves>(a.out, seq.q_row0 + t, h, D, lane * (D / 32) + e, pack2<T>(o[e] * inv, o[e + 1] * inv));
                     } else {
                         const float up = __shfl_down_sync(0xffffffffu, o[0], 1);
-                        if ((lane & 1) == 0) store_pair<T>(a.out, seq.q_row0 + t, h, D, lane, pack2<T>(o[0] * inv, up * inv));
+                        if ((lane & 1) == 0) store_pair<T, kHalves>(a.out, seq.q_row0 + t, h, D, lane, pack2<T>(o[0] * inv, up * inv));
                     }
                     if (lane == 0 && a.out.lse != nullptr)
                         a.out.lse[((long long)s * a.q_heads + h) * a.q_seq_len + t] = l > 0.0f ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
@@ -833,20 +837,17 @@ RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, b
 
 std::atomic<unsigned long long> g_calls{0};   // launches of this kernel, of any type and on any device
 
-template <typename T, int D>
-int launch_rows(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
+template <typename T, int D, bool kHalves>
+int launch_rows_as(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
     using S = Smem<D>;
     static_assert(kMaxColumns < (1 << kCountBits), "the parts of a sequence fit the count");
-    for (int i = 0; i < a.out.n_out; ++i)
-        if (reinterpret_cast<uintptr_t>(a.out.o[i]) & 3) a.out.halves = 1;
-    a.call = (g_calls.fetch_add(1, std::memory_order_relaxed) + 1) << kCountBits;
     a.row_blocks = plan.row_blocks;
     a.forced_units = plan.forced_units;
     static std::atomic<unsigned long long> ready{0};   // devices whose copy of this kernel has its shared-memory limit raised
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err == cudaSuccess && (dev >= 64 || !((ready.load(std::memory_order_acquire) >> dev) & 1ULL))) {
-        err = cudaFuncSetAttribute(decode_splitk_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
+        err = cudaFuncSetAttribute(decode_splitk_kernel<T, D, kHalves>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
         if (err == cudaSuccess && dev < 64) ready.fetch_or(1ULL << dev, std::memory_order_release);
     }
     if (err != cudaSuccess) {
@@ -864,8 +865,15 @@ int launch_rows(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, decode_splitk_kernel<T, D>, a);
+    cudaLaunchKernelEx(&cfg, decode_splitk_kernel<T, D, kHalves>, a);
     return check_launch("decode_splitk_kernel");
+}
+
+template <typename T, int D>
+int launch_rows(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
+    bool halves = false;
+    for (int i = 0; i < a.out.n_out; ++i) halves |= (reinterpret_cast<uintptr_t>(a.out.o[i]) & 3) != 0;
+    return halves ? launch_rows_as<T, D, true>(a, plan, stream) : launch_rows_as<T, D, false>(a, plan, stream);
 }
 
 int log2_or_minus1(int v) {
