@@ -580,7 +580,7 @@ def run_sharded_prefill(torch, low, ffi, dev, dist, world, rank, name, steps, wa
 
 def run_sharded_decode(torch, low, ffi, dev, dist, world, rank, name, steps, warmup, peaks):
     """Strong scaling of paged decode: every rank holds the cache slice of its KV heads
-    (num_blocks, page, hkv/world, d); block tables and lengths are replicated; the merge kernel stores
+    (num_blocks, page, hkv/world, d); block tables and lengths are replicated; the kernel stores
     its heads into every rank's (batch, 1, hq, d) output. All ranks build their cache slice from the
     same seed and differ in their query rows, so a rank can recompute another rank's heads alone."""
     from luma_b200 import dist as fdist

@@ -695,7 +695,7 @@ int kvcache_impl(int dtype, const void* q, const void* k_cache, const void* v_ca
     p.paged = 1;
     p.scale = scale;
     if (o_peers != nullptr) {
-        // head-sharded single-token decode with the output all-gather fused into the merge kernel
+        // head-sharded single-token decode with the output all-gather fused into the kernel
         if (n_peers < 1 || n_peers > 8 || q_head_offset < 0 || q_heads_total <= 0 || q_head_offset + q_heads > q_heads_total) {
             set_last_error("flash_attn_with_kvcache_allgather: n_peers must be in 1..8 and q_head_offset + q_heads inside q_heads_total");
             return FLASH_ATTN_ERR_INVALID_SHAPE;

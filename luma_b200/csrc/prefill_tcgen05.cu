@@ -443,8 +443,7 @@ __device__ __forceinline__ TileInfo tile_info(const SeqExtent& a, int pair, int 
 // The launch order of chunks of prompts over long contexts, whose lengths the host does not know: CTA `index`
 // of the grid takes the index-th tile pair of the call, heaviest first (K/V tiles, in classes of an eighth of the longest
 // range, so that the pairs of one K/V stream stay neighbours and meet in L2). In grid order (sequences as they
-// come) a long context that comes late ends alone: 4 chunks of 512 over 1024-8192 tokens 161 us a step, 155 so; with 32
-// decoding sequences beside them 264, 253 so.
+// come) a long context that comes late ends alone (times beside the rule that asks for it, in launch_variant).
 // Run by one whole warp; a lane holds 8 neighbouring sequences at most.
 constexpr int kOrderPerLane = 8;
 constexpr int kOrderMax = 32 * kOrderPerLane;
@@ -544,8 +543,8 @@ __device__ __forceinline__ int3 find_item(const PrefillArgs& a, int group, int i
 //               tensor map and therefore arrives as zeros.
 // A paged tile is 16 copies at a page of 16 tokens: the lanes look their pages up before the ring stage is free, so
 // that the request follows the release at once. Looked up and requested page by page by one thread after the release,
-// a tile came about a thousand clocks later, which the two-stage rings do not hide: 4 chunks of 512 over 1024-8192 tokens
-// (page 16) took 167 us a step, 161 so.
+// a tile came about a thousand clocks later, which the two-stage rings do not hide: 3.6 % of a step of 4 chunks of 512 over
+// 1024-8192 tokens (page 16).
 __device__ __forceinline__ int page_of_lane(const PrefillArgs& a, int kv_len, int s, int j, int lane) {
     const int per_tile = kBlockN / a.block_size;
     const int pg = j * per_tile + lane;
@@ -1646,8 +1645,8 @@ int launch_prefill_tcgen05(const AttnParams& p, cudaStream_t stream) {
     if (p.dtype != DT_F16 && p.dtype != DT_BF16) return -1;
     if (p.head_size != 32 && p.head_size != 64 && p.head_size != 128) return -1;
     if (!(p.scale > 0.0f)) return -1;
-    // (single-token calls of the kv-cache entry point never get here: the dispatcher tries the split-K
-    // decode kernel first; single rows through the batched or packed entry points do)
+    // (the dispatcher tries the split-K kernel first: single-token calls of the kv-cache entry point never get here, other calls
+    // with few query rows where this kernel is the faster one for them)
     uintptr_t align = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) |
                       reinterpret_cast<uintptr_t>(p.v) | reinterpret_cast<uintptr_t>(p.o);
     for (int i = 0; i < p.n_out && i < 8; ++i) align |= reinterpret_cast<uintptr_t>(p.o_peers[i]);

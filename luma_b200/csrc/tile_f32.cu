@@ -1,4 +1,5 @@
-// f32 storage on the tensor cores without giving up f32: every operand is split into three bf16 terms that together
+// f32 storage on the tensor cores without giving up f32 (the splitting is that of Henry, Tang and Heinecke, "Leveraging the
+// bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations", 2019): every operand is split into three bf16 terms that together
 // hold its 24 bits (x = hi + mid + lo exactly, each term the rounded rest of the one before), and a product of two
 // operands is the six term products of at least 2^-16 of the largest (hi hi, hi mid, mid hi, mid mid, hi lo,
 // lo hi; what is left out is below 2^-24). Replaces the scalar kernel (tile_simt.cu) for f32 tensors through the

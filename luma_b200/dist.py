@@ -84,7 +84,7 @@ class PeerOutput:
     multicast is not on offer (`self.mc_ptr == 0`, agreed across the group) the peer-pointer path is used.
 
     `fused_attention` runs the head-sharded prefill with the gather fused into its epilogue,
-    `fused_decode` the head-sharded single-token decode with the gather fused into its merge kernel;
+    `fused_decode` the head-sharded single-token decode with the gather fused into its kernel;
     `sync()` then synchronises the group, after which `self.out` (and `self.lse`) hold every rank's heads.
     """
 
@@ -178,7 +178,7 @@ class PeerOutput:
 
     def fused_decode(self, q, k_cache, v_cache, block_tables, context_lens, q_heads_total, q_head_offset, scale=None):
         """q (B, 1, Hq_local, d) and this rank's cache slice (num_blocks, page, Hkv_local, d): one
-        decode step whose merge kernel writes this rank's heads into every rank's (B, 1, Hq_total, d)."""
+        decode step whose kernel writes this rank's heads into every rank's (B, 1, Hq_total, d)."""
         from . import low
         b, one, hq_l, d = q.shape
         assert one == 1 and tuple(self.out.shape) == (b, 1, q_heads_total, d)

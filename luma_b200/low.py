@@ -202,7 +202,7 @@ def flash_attn_allgather_multicast(q, k, v, o_multicast_ptr, q_heads_total, q_he
 def flash_attn_with_kvcache_allgather(q, k_cache, v_cache, o_peer_ptrs, q_heads_total, q_head_offset, block_tables,
                                       context_lens, num_seqs, q_heads, kv_heads, head_size, block_size, max_blocks,
                                       scale, stream=None) -> None:
-    """Head-sharded single-token paged decode whose merge kernel stores this rank's heads into the
+    """Head-sharded single-token paged decode whose kernel stores this rank's heads into the
     (num_seqs, 1, q_heads_total, head_size) output of every GPU of the group. Additive."""
     import ctypes
     sfx = _suffix(q)

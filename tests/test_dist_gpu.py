@@ -7,7 +7,7 @@ every rank (luma-dist/src/backends/nccl/tests.rs:60-90):
   through an NVSwitch multicast address (one multimem.st per 16 bytes) where the box offers one;
 * prefill, two-step: attention on the shard, then the all-gather along the head axis
   (torch.distributed's NCCL, and this library's own communicator: luma_comm_all_gather);
-* decode, fused: the split-K merge kernel stores into every rank's output; and two-step.
+* decode, fused: the split-K kernel stores into every rank's output; and two-step.
 
 One process per GPU over NCCL; skipped on a box with a single GPU."""
 import os
