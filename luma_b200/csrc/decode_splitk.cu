@@ -871,6 +871,7 @@ int launch_rows_as(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
 
 template <typename T, int D>
 int launch_rows(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
+    a.call = (g_calls.fetch_add(1, std::memory_order_relaxed) + 1) << kCountBits;
     bool halves = false;
     for (int i = 0; i < a.out.n_out; ++i) halves |= (reinterpret_cast<uintptr_t>(a.out.o[i]) & 3) != 0;
     return halves ? launch_rows_as<T, D, true>(a, plan, stream) : launch_rows_as<T, D, false>(a, plan, stream);
