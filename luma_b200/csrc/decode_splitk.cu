@@ -984,25 +984,26 @@ int launch_decode_splitk(const AttnParams& p, cudaStream_t stream) {
 }
 
 // ---- this kernel or the prefill kernel, for calls that both take: the time of each, in microseconds, from what the host knows.
-// Prefill kernel: a CTA per pair of 128-row tiles, one per SM; a CTA walks its K/V range at 1.7 us per 128 keys after 5 us of set-up.
+// Prefill kernel: a CTA per pair of 128-row tiles, one per SM; a CTA walks its K/V range at 1.5 us per 128 keys after 6.6 us of set-up.
 static long long longest_keys(const AttnParams& p) { return p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len; }
 static long long tile_pairs(const AttnParams& p, long long q_len) { return ((long long)(p.q_heads / p.kv_heads) * ((q_len + 127) / 128) + 1) / 2 * p.kv_heads; }
 static double prefill_us(const AttnParams& p, double pairs) {
-    return std::max(1.0, pairs / sm_count()) * (5.0 + 1.7 * (double)((longest_keys(p) + 127) / 128));
+    return std::max(1.0, pairs / sm_count()) * (6.6 + 1.5 * (double)((longest_keys(p) + 127) / 128));
 }
-// This kernel: a CTA slot takes 1.2 us per unit of 64 keys (16 rows of one KV head) and 3 us + 0.2 us a row per sequence, most of it the merge of its
-// warps' parts; where sequences are cut, the merge of their parts is another 0.5 us a row.
+// This kernel: a CTA slot takes 1.04 us per unit of 64 keys (16 rows of one KV head; 0.91 where several row blocks read the same K/V) and 2.2 us
+// + 0.15 us a row per sequence, most of it the merge of its warps' parts; some sequence of more than one unit is always cut, and the merge of its
+// parts is another 0.6 us a row.
 static double rows_us(const AttnParams& p, long long seqs, long long rows) {
     const long long slots = (long long)sm_count() * (p.head_size == 128 ? Smem<128>::kCtasPerSm : p.head_size == 64 ? Smem<64>::kCtasPerSm : Smem<32>::kCtasPerSm);
     const double units = (double)((longest_keys(p) + kUnit - 1) / kUnit), nrows = (double)std::min<long long>(kRows, rows);
     const double blocks_per_slot = (double)(seqs * p.kv_heads * ((rows + kRows - 1) / kRows)) / (double)slots;
-    return 5.0 + (1.2 * units + 3.0 + 0.2 * nrows) * blocks_per_slot + (blocks_per_slot < 1.0 ? 0.5 * nrows : 0.0);
+    return 4.4 + ((rows > kRows ? 0.91 : 1.04) * units + 2.2 + 0.15 * nrows) * blocks_per_slot + (units > 1.0 ? 0.6 * nrows : 0.0);
 }
 
 // Up to four row blocks of 16 (query token x group head) rows, each of which reads the K/V rows again, from L2. The prefill kernel's one or two
 // tiles per CTA are almost empty, but it reads K/V once: over up to 12 tiles in one wave of its CTAs (25 us at most) it keeps the call,
-// else the estimates decide. Both kernels over 298 shapes (1-64 sequences x 1-64 tokens, 64-8192 keys, groups of 1, 4
-// and 8): the choice is at most 3 % slower than the prefill kernel anywhere. 64 rows:
+// else the estimates decide. Both kernels over the 235 of 298 shapes that get this far (1-64 sequences x 1-64 tokens, 64-8192 keys, groups of 1, 4
+// and 8): the choice is at most 5 % slower than the prefill kernel and at most 9 % slower than this one. 64 rows:
 // 64 x 64 tokens x 1600 keys, 32 heads without GQA 275 us on the prefill kernel, 743 here; 1 x 16 x 8192, 32/8 heads 110 and 31. 16 rows: 16 x 4 x
 // 8192, 32/8: 180 and 63.
 int launch_few_rows(const AttnParams& p, bool prefill_takes_it, cudaStream_t stream) {

@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
     (1, 64, 8192, 32, 32, 128, "decode_splitk"), (1, 16, 8192, 32, 8, 128, "decode_splitk"), (4, 16, 8192, 32, 8, 128, "decode_splitk"),
     # one or two row blocks: whatever leaves the prefill kernel's CTAs a long walk or several waves
     (16, 4, 8192, 32, 8, 128, "decode_splitk"), (8, 1, 4000, 32, 8, 128, "decode_splitk"), (64, 4, 1600, 64, 8, 128, "decode_splitk"),
-    (64, 1, 64, 32, 32, 128, "decode_splitk"), (1, 4, 512, 32, 8, 128, "prefill_tcgen05"), (4, 4, 64, 32, 8, 128, "prefill_tcgen05"),
+    (64, 1, 64, 32, 32, 128, "decode_splitk"), (16, 4, 64, 32, 8, 128, "decode_splitk"), (4, 16, 1600, 32, 8, 128, "decode_splitk"), (1, 4, 512, 32, 8, 128, "prefill_tcgen05"), (4, 4, 64, 32, 8, 128, "prefill_tcgen05"),
 ])
 def test_few_rows_go_to_the_faster_kernel(b, s, kv, hq, hkv, d, path):
     q = torch.zeros(b, s, hq, d, dtype=torch.bfloat16, device="cuda")
