@@ -987,8 +987,8 @@ int launch_decode_splitk(const AttnParams& p, cudaStream_t stream) {
 // Prefill kernel: a CTA per pair of 128-row tiles, one per SM; a CTA walks its K/V range at 1.5 us per 128 keys after 6.6 us of set-up.
 static long long longest_keys(const AttnParams& p) { return p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len; }
 static long long tile_pairs(const AttnParams& p, long long q_len) { return ((long long)(p.q_heads / p.kv_heads) * ((q_len + 127) / 128) + 1) / 2 * p.kv_heads; }
-static double prefill_us(const AttnParams& p, double pairs) {
-    return std::max(1.0, pairs / sm_count()) * (6.6 + 1.5 * (double)((longest_keys(p) + 127) / 128));
+static double prefill_us(const AttnParams& p, double pairs, double setup = 6.6) {
+    return std::max(1.0, pairs / sm_count()) * (setup + 1.5 * (double)((longest_keys(p) + 127) / 128));
 }
 // This kernel: a CTA slot takes 1.04 us per unit of 64 keys (16 rows of one KV head; 0.91 where several row blocks read the same K/V) and 2.2 us
 // + 0.15 us a row per sequence, most of it the merge of its warps' parts; some sequence of more than one unit is always cut, and the merge of its
@@ -1031,9 +1031,10 @@ PackedMix packed_mix(const AttnParams& p) {
 }
 
 // Whether the few-row sequences of a packed batch are better off behind the prefill kernel than in its grid, where each takes a
-// CTA per two heads of its group: only where they make waves of those, by the estimates above and a fifth more, since the second launch
+// CTA per two heads of its group: only where they make waves of those, by the estimates above (14 us of set-up for a CTA of a packed batch) and a
+// seventh more, since the second launch
 // starts when that kernel's last CTA has. Over 238 paged mixes (1-6 prompts, chunks of 64 or 512, 0-128 single tokens, contexts of
-// 64-8192, four head layouts) no mix is then slower than with everything in the prefill grid, and the choice is 3 % off the better one on average:
+// 64-8192, four head layouts) no mix is then slower than with everything in the prefill grid, and the choice is 2 % off the better one on average:
 // 4 x 512 with 32 tokens over 512-8192, 32/8 heads: 435 us in one grid, 231 so; with 1 token: 131 in one grid, 152 with two kernels, which
 // one grid keeps. Without the row count of the packed buffers (the C ABI's plain entry point) nothing is known of the mix, and
 // long contexts go to two kernels.
@@ -1042,7 +1043,7 @@ static bool mixed_few_rows_are_better(const AttnParams& p) {
     const PackedMix m = packed_mix(p);
     if (m.few <= 0) return false;
     const double prompts = (double)m.prompts * tile_pairs(p, p.q_seq_len), few = (double)m.few * tile_pairs(p, 1);
-    return prefill_us(p, prompts + few) > 1.2 * (prefill_us(p, prompts) + rows_us(p, m.few, p.q_heads / p.kv_heads));
+    return prefill_us(p, prompts + few, 14.0) > 1.15 * (prefill_us(p, prompts, 14.0) + rows_us(p, m.few, p.q_heads / p.kv_heads));
 }
 
 MixedFewRows prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {

@@ -1565,13 +1565,16 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     const long long kv_rows = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
     const PackedMix mix = packed_mix(p);
     const double waves = (double)(mix.prompts * pairs + (a.skip_rows > 0 ? 0 : mix.few * ((group + 1) / 2))) * p.kv_heads / sm_count();
-    const bool worth_ordering = waves > 1.0 && (double)((kv_rows + kBlockN - 1) / kBlockN) > 5.0 * waves;
+    const long long all = (long long)p.num_seqs * p.kv_heads * pairs;
+    long long ctas = all;
+    if (p.total_q > 0)   // a sequence of n rows has (group * ceil(n / 128) + 1) / 2 pairs
+        ctas = std::min(ctas, p.kv_heads * ((group * (((long long)p.total_q + 127LL * p.num_seqs) / 128) + p.num_seqs) / 2));
+    // ... and where most of the grid would be empty CTAs of sequences that are left to the few-row kernel: a launch in order has no more than
+    // the rows can make (one chunk of 512 with 128 tokens over 128-2048, 32/8 heads: 8256 CTAs or 2644, 200 us or 173).
+    const bool worth_ordering = (waves > 1.0 && (double)((kv_rows + kBlockN - 1) / kBlockN) > 5.0 * waves) || (a.skip_rows > 0 && all > 2 * ctas);
     if (kPaged && p.num_seqs >= 2 && p.num_seqs <= kOrderMax && 2LL * p.q_seq_len <= kv_rows && get_option_prefill_band() <= 0 &&
         get_option_prefill_groups() <= 0 && (worth_ordering || get_option_prefill_order() == 2)) {
         a.ordered = 1;
-        long long ctas = (long long)p.num_seqs * p.kv_heads * pairs;
-        if (p.total_q > 0)   // a sequence of n rows has (group * ceil(n / 128) + 1) / 2 pairs
-            ctas = std::min(ctas, p.kv_heads * ((group * (((long long)p.total_q + 127LL * p.num_seqs) / 128) + p.num_seqs) / 2));
         if (ctas <= 0 || ctas > 0x7fffffffLL) return -1;
         grid = dim3((unsigned)ctas);
     }
