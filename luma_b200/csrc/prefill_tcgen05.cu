@@ -48,11 +48,8 @@ constexpr int kBlockM = 128;   // query rows per tile
 constexpr int kBlockN = 128;   // keys per K/V tile
 // head size D (64 or 128) is a template parameter of the kernel
 constexpr int kStages = 2;     // K ring depth
-// V ring depth. Two, like K: a third stage fits the 227 KiB of shared memory and takes the MMA
-// issuer's ~350-clock wait for V out of every step (a bulk copy needs about 2 us to land while 148
-// CTAs stream their tiles out of L2, and a V stage is released later than a K stage), but measured
-// 5 % slower on every prefill workload (1165 against 1228 TFLOP/s at S = 8192, same box).
-constexpr int kStagesV = 2;
+// The rings are two tiles deep. A third V stage fits the shared memory and measured 5 % slower on every prefill workload (1165
+// against 1228 TFLOP/s at S = 8192); the issuer does not wait for the copies.
 constexpr int kThreads = 384;   // three warpgroups: softmax 0, softmax 1, and producer + issuer (+ two idle warps)
 constexpr int kLoadWarp = 8;
 constexpr int kMmaWarp = 9;
@@ -71,13 +68,13 @@ template <int D>
 struct SharedStorage {
     alignas(1024) unsigned char q[2][TileBytes<D>::value];
     alignas(1024) unsigned char k[kStages][TileBytes<D>::value];
-    alignas(1024) unsigned char v[kStagesV][TileBytes<D>::value];
+    alignas(1024) unsigned char v[kStages][TileBytes<D>::value];
     alignas(8) unsigned long long q_full[2];
-    unsigned long long k_full[kStages], k_empty[kStages];
-    unsigned long long v_full[kStagesV], v_empty[kStagesV];
+    unsigned long long k_first;     // copy engine -> MMA: K tile 0
+    unsigned long long step_full[2];    // copy engine -> MMA: what step j reads, V tile j and K tile j + 1, in entry j & 1
+    unsigned long long step_done[2];    // MMA -> producers: the products of step j - 1 (j = 0: the first S) have finished, in entry j & 1
     unsigned long long s_full[2];   // MMA -> softmax: S_t ready (and every earlier MMA finished)
-    unsigned long long p_lo[2];     // softmax -> MMA: keys 0-63 of P_t written, O_t rescaled
-    unsigned long long p_hi[2];     // softmax -> MMA: keys 64-127 of P_t written
+    unsigned long long p_ready[2][2];   // softmax -> MMA: keys 0-63 of P_t written and O_t rescaled ([0][t]), keys 64-127 written ([1][t])
     unsigned long long v_tail;      // copy engine -> V producer: the sequence's last, partly filled V tile has landed
     unsigned long long drain;       // MMA issuer, error path only: every product issued so far has finished
     unsigned int tmem_base;
@@ -149,15 +146,17 @@ __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned
     asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}\n" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
+__device__ __forceinline__ bool mbar_try_wait_at(unsigned bar, unsigned parity) {
     unsigned ok;
     asm volatile(
         "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(bar), "r"(parity)
         : "memory");
     return ok != 0;
 }
+__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) { return mbar_try_wait_at(smem_u32(bar), parity); }
+__device__ __forceinline__ void set_shared_flag(unsigned addr) { asm volatile("st.volatile.shared.s32 [%0], 1;\n" ::"r"(addr) : "memory"); }
 __device__ __forceinline__ unsigned long long global_timer_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t));
@@ -166,16 +165,17 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
 
 // Bounded wait. Returns false when the wait was abandoned (time limit, or another thread of the
 // CTA already gave up); the caller then falls through to the end of the kernel.
+// The bound is counted in SM clocks (cheap to read, unlike the global nanosecond timer): wait_ns x 2 clocks, i.e. at least
+// wait_ns of wall time at any SM clock up to 2 GHz.
 // The status word lives in mapped host memory (the host reads it without touching the device), so it
 // is written with a plain store: the code of one of the waits that expired.
 template <typename Storage>
 __device__ __forceinline__ bool mbar_wait(Storage& sm, unsigned long long* bar, unsigned parity, const PrefillArgs& a,
                                           int where) {
     if (mbar_try_wait(bar, parity)) return true;
-    // the bound is counted in SM clocks (cheap to read, unlike the global nanosecond timer):
-    // wait_ns x 2 clocks, i.e. at least wait_ns of wall time at any SM clock up to 2 GHz
     const long long t0 = clock64();
     const long long limit = (long long)(a.wait_ns * 2ULL);
+#pragma unroll 1
     for (unsigned spin = 1;; ++spin) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((spin & 63u) == 0u) {
@@ -216,39 +216,26 @@ __device__ __forceinline__ void multimem_st16(void* mc_addr, const uint4& w) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 
-// Executed by the whole (converged) issuer warp; one elected lane commits.
-__device__ __forceinline__ void tc_commit(unsigned long long* bar) {
-    asm volatile("{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\n@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // The products as the issuer warp runs them: the whole warp executes the instruction stream
 // converged and one elected lane issues. Keeping the warp uniform lets the descriptors live in
-// uniform registers, so a product costs a handful of issue slots; issued from a single diverged
-// lane each needs register-to-uniform moves and, next to ALU-heavy warps on the same scheduler,
-// took ~130 clocks instead of the tensor pipe's 64. The accumulate flag is a compile-time constant.
+// uniform registers: a product is 5 instructions inside an elected branch, 7 with an election of its own and 12 to 14 where the compiler
+// cannot see that its operands are the same for the whole warp.
+__device__ __forceinline__ bool elect_one() {
+    unsigned e;
+    asm volatile("{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\nselp.u32 %0, 1, 0, e;\n}\n" : "=r"(e));
+    return e != 0;
+}
 // D[tmem] (+)= A[smem] * B[smem]
-template <bool kAccumulate>
-__device__ __forceinline__ void tc_mma_ss_imm(unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc) {
-    if (kAccumulate)
-        asm volatile("{\n.reg .pred p, e;\nelect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, 1, 0;\n@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-                     "l"(a_desc), "l"(b_desc), "r"(idesc)
-                     : "memory");
-    else
-        asm volatile("{\n.reg .pred p, e;\nelect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, 0, 0;\n@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-                     "l"(a_desc), "l"(b_desc), "r"(idesc)
-                     : "memory");
+__device__ __forceinline__ void tc_mma_ss(unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc, bool accumulate) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc),
+                 "r"(idesc), "r"((unsigned)accumulate)
+                 : "memory");
 }
 // D[tmem] (+)= A[tmem] * B[smem]
-template <bool kAccumulate>
-__device__ __forceinline__ void tc_mma_ts_imm(unsigned d_tmem, unsigned a_tmem, unsigned long long b_desc, unsigned idesc) {
-    if (kAccumulate)
-        asm volatile("{\n.reg .pred p, e;\nelect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, 1, 0;\n@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
-                     "r"(a_tmem), "l"(b_desc), "r"(idesc)
-                     : "memory");
-    else
-        asm volatile("{\n.reg .pred p, e;\nelect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, 0, 0;\n@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
-                     "r"(a_tmem), "l"(b_desc), "r"(idesc)
-                     : "memory");
+__device__ __forceinline__ void tc_mma_ts(unsigned d_tmem, unsigned a_tmem, unsigned long long b_desc, unsigned idesc, bool accumulate) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc),
+                 "r"(idesc), "r"((unsigned)accumulate)
+                 : "memory");
 }
 // 32 lanes x 32 consecutive 32-bit columns: thread i of the warp <-> TMEM lane (base + i)
 __device__ __forceinline__ void tc_ld32(unsigned taddr, float (&r)[32]) {
@@ -383,8 +370,12 @@ __device__ __forceinline__ void trace_event(long long* trace, int role, int j, i
     if (trace != nullptr && j < kTraceSteps) trace[(role * kTraceSteps + j) * 8 + ev] = clock64();
 }
 #define FA_TRACE_EVENT(role, j, ev) trace_event(trace, role, j, ev)
+#define FA_TRACE_PARAM(x) , long long* x
+#define FA_TRACE_ARG(x) , x
 #else
 #define FA_TRACE_EVENT(role, j, ev) ((void)0)
+#define FA_TRACE_PARAM(x)
+#define FA_TRACE_ARG(x)
 #endif
 
 struct TileInfo {
@@ -595,6 +586,132 @@ __device__ __forceinline__ void edge_tile_copy(unsigned char* dst, const void* b
     if (lane == 0) mbar_arrive(bar);
 }
 
+__device__ __forceinline__ unsigned clock_lo() {
+    unsigned t;
+    asm volatile("mov.u32 %0, %%clock;\n" : "=r"(t));
+    return t;
+}
+
+// The MMA issuer, run by one whole warp (converged). Its loop is written for few instructions: about 400 a step where it had 780 (12.5 KiB).
+// What a scheduler executes in a loop comes at full rate up to 8 KiB, beyond that at an instruction in 3 clocks, beyond 32 KiB in 6 (a
+// straight-line loop of multiply-adds); the softmax warps' 10 KiB pass between two steps of the issuer, so that it is fetched anew every time.
+// The tensor pipe stood still meanwhile: 300 clocks from the issuer's last commit of a step to its first look at the next barrier, 150 for
+// a look at one that had long completed (45 alone), with or without the copies. Step of 128 keys at S = 8192 GQA 3100 -> 2840 clocks,
+// 884 -> 833 us; 4 x 2048 MHA 157.5 -> 147.8 us; head size 64, 2 x 8192 GQA 755 -> 699 us.
+//   * a function of its own, so that the compiler sees what is the same for the whole warp (everything is, or is broadcast here): inside
+//     the kernel, whose early returns and per-sequence loads it takes for divergent, a product was 11 instructions, here it is 6;
+//   * a wait that runs out is looked after once a step: the loop goes on, without waiting for anything more, on what happens to be in
+//     shared memory (the softmax warps leave at the abort flag; nothing is written). Leaving at each wait doubled the code after it.
+// n0, n1: K/V tiles that query tile 0 and 1 need (0: none, or no such tile).
+template <typename T, int D>
+__device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int n0, int n1, int* status, unsigned long long wait_ns
+                                            FA_TRACE_PARAM(trace)) {
+    using Storage = SharedStorage<D>;
+    sm_addr = __shfl_sync(0xffffffffu, sm_addr, 0);
+    n0 = __shfl_sync(0xffffffffu, n0, 0);
+    n1 = __shfl_sync(0xffffffffu, n1, 0);
+    tmem = __shfl_sync(0xffffffffu, tmem, 0);
+    const int n_max = max(n0, n1);
+    const unsigned idesc_qk = make_idesc<T>(false, kBlockN);
+    const unsigned idesc_pv = make_idesc<T>(true, D);   // N = head size
+    const unsigned long long dq = make_desc(sm_addr + (unsigned)offsetof(Storage, q), 16, 1024);
+    const unsigned long long dk = make_desc(sm_addr + (unsigned)offsetof(Storage, k), 16, 1024);
+    const unsigned long long dv = make_desc(sm_addr + (unsigned)offsetof(Storage, v), kHalfBytes, 1024);
+    constexpr unsigned kTileStep = TileBytes<D>::value >> 4;   // from one tile's descriptor to the next one's
+    // the bound in SM clocks, as in mbar_wait, in the 32 bits of the clock's lower half (which wraps after 2.1 s at the least)
+    unsigned patience = (unsigned)(wait_ns < 2000000000ULL ? wait_ns * 2ULL : 4000000000ULL);
+    int expired = 0;   // code of a wait that ran out
+    auto wait = [&](size_t bar, unsigned parity, int where) {
+        const unsigned t0 = clock_lo();
+#pragma unroll 1
+        while (!__any_sync(0xffffffffu, mbar_try_wait_at(sm_addr + (unsigned)bar, parity))) {
+            if (__any_sync(0xffffffffu, clock_lo() - t0 >= patience)) {
+                expired = where;
+                break;
+            }
+        }
+    };
+    // S_t = Q_t K^T : D / 16 K-steps over d; both operands K-major, 128 B swizzle
+    auto issue_s = [&](int t, unsigned long long kd) {
+        const unsigned long long qd = dq + t * kTileStep;
+        if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < D / 16; ++kk) {
+                const unsigned inc = ((kk >> 2) * kHalfBytes + (kk & 3) * 32) >> 4;
+                tc_mma_ss(tmem + t * 128, qd + inc, kd + inc, idesc_qk, kk > 0);
+            }
+        }
+    };
+    // O_t += P_t V : 4 K-steps of 16 keys; A = P from tensor memory (packed 16-bit, 8 columns
+    // per step), B = V MN-major: 64-column halves 16 KiB apart, 8-key groups 1 KiB apart
+    auto issue_pv = [&](int t, int half, unsigned long long vd, bool accumulate) {
+        if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+                tc_mma_ts(tmem + 256 + t * 128, tmem + t * 128 + half * 32 + kk * 8, vd + half * 512 + kk * (2048 >> 4), idesc_pv, kk > 0 || accumulate);
+        }
+    };
+    auto commit = [&](size_t bar) {
+        if (elect_one()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(sm_addr + (unsigned)bar) : "memory");
+    };
+    if (n_max > 0) {
+        // The copies were requested in the order Q0, K0, Q1: the first S of tile 0 is issued as soon as
+        // its two operands are there, without waiting for the other tile's Q.
+#pragma unroll 1
+        for (int t = 0; t < 2; ++t) {
+            if ((t == 0 ? n0 : n1) <= 0) continue;
+            wait(offsetof(Storage, q_full) + 8 * t, 0, 10);
+            wait(offsetof(Storage, k_first), 0, 11);
+            tc_fence_after();
+            issue_s(t, dk);
+            commit(offsetof(Storage, s_full) + 8 * t);
+        }
+        commit(offsetof(Storage, step_done));
+    }
+    FA_TRACE_EVENT(2, kTraceSteps - 1, 2);       // Q and the first K tile have landed
+#pragma unroll 1
+    for (int j = 0; j < n_max; ++j) {
+        const unsigned s = j & 1;   // stage of V(j); K(j + 1) is in the other one
+        const unsigned long long vd = dv + s * kTileStep, kd = dk + (s ^ 1) * kTileStep;
+        wait(offsetof(Storage, step_full) + 8 * s, (unsigned)(j >> 1) & 1u, 13);
+        FA_TRACE_EVENT(2, j, 4);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const int n_kv = t == 0 ? n0 : n1;
+            if (j < n_kv) {
+                // the first 64 keys of P_t arrive while the softmax still works on the other 64:
+                // their half of P.V leaves the critical path
+                wait(offsetof(Storage, p_ready) + 8 * t, s, 14 + t);
+                FA_TRACE_EVENT(2, j, t * 2);
+                tc_fence_after();
+                issue_pv(t, 0, vd, j > 0);
+                wait(offsetof(Storage, p_ready) + 16 + 8 * t, s, 16 + t);
+                FA_TRACE_EVENT(2, j, 5 + t);
+                tc_fence_after();
+                issue_pv(t, 1, vd, true);
+                if (j + 1 < n_kv) issue_s(t, kd);
+                commit(offsetof(Storage, s_full) + 8 * t);   // S_t(j+1) ready, or after the last PV: O_t final
+                FA_TRACE_EVENT(2, j, t * 2 + 1);
+            }
+        }
+        commit(offsetof(Storage, step_done) + 8 * (s ^ 1));
+        if (expired != 0) {
+            set_shared_flag(sm_addr + (unsigned)offsetof(Storage, abort_flag));
+            *reinterpret_cast<volatile int*>(status) = expired;
+            __threadfence_system();
+            patience = 0;
+        }
+    }
+    if (expired != 0) {
+        // error path: tensor memory is freed at the end of the kernel, so let every product issued
+        // so far finish first (bounded; depends on the tensor pipe alone)
+        __syncwarp();
+        commit(offsetof(Storage, drain));
+        const unsigned long long t_begin = global_timer_ns();
+        while (!mbar_try_wait_at(sm_addr + (unsigned)offsetof(Storage, drain), 0u) && global_timer_ns() - t_begin < 100000000ULL) {}
+    }
+}
+
 // kMask: the call carries a key-padding mask (a separate instantiation, so that calls without one
 // pay nothing for it in the softmax loop)
 // kPaged: paged K/V, whose tiles are gathered page by page and whose tile pairs may be ordered on the device (a separate instantiation as
@@ -612,7 +729,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     const unsigned long long ns_entry = a.cta_log != nullptr ? global_timer_ns() : 0ULL;
 #endif
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // (the same for the whole warp, which the compiler sees only so)
     const int lane = threadIdx.x & 31;
     const int group = a.q_heads / a.kv_heads;
     // A few-row kernel launched behind this one may start once every CTA here has: it fills the SMs that run out of tile pairs.
@@ -673,17 +790,12 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             for (int i = 0; i < 2; ++i) {
                 mbar_init(&sm.q_full[i], 1);
                 mbar_init(&sm.s_full[i], 1);
-                mbar_init(&sm.p_lo[i], 128);
-                mbar_init(&sm.p_hi[i], 128);
+                mbar_init(&sm.p_ready[0][i], 128);
+                mbar_init(&sm.p_ready[1][i], 128);
+                mbar_init(&sm.step_full[i], 2);
+                mbar_init(&sm.step_done[i], 1);
             }
-            for (int i = 0; i < kStages; ++i) {
-                mbar_init(&sm.k_full[i], 1);
-                mbar_init(&sm.k_empty[i], 1);
-            }
-            for (int i = 0; i < kStagesV; ++i) {
-                mbar_init(&sm.v_full[i], 1);
-                mbar_init(&sm.v_empty[i], 1);
-            }
+            mbar_init(&sm.k_first, 1);
             mbar_init(&sm.v_tail, 1);
             mbar_init(&sm.drain, 1);
             asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -699,7 +811,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         load_q(t0, 0);
 #pragma unroll
         for (int j = 0; j < kStages; ++j) {
-            if (j < n_pre && !kv_edge(j) && a.test_skip_k != j + 1) load_kv_tile<D, kPaged>(a, sq, kvh, sm.k[j], &k_map, &sm.k_full[j], j, pages[j], lane);
+            if (j < n_pre && !kv_edge(j) && a.test_skip_k != j + 1) load_kv_tile<D, kPaged>(a, sq, kvh, sm.k[j], &k_map, j == 0 ? &sm.k_first : &sm.step_full[0], j, pages[j], lane);
             if (j == 0) load_q(t1, 1);
         }
         // the V tiles come from a producer thread of their own (warp kLoadWarpV), after the set-up barrier
@@ -737,17 +849,17 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         {
             const bool is_v = warp == kLoadWarpV;
             unsigned char (*ring)[TileBytes<D>::value] = is_v ? sm.v : sm.k;
-            unsigned long long* full = is_v ? sm.v_full : sm.k_full;
-            unsigned long long* empty = is_v ? sm.v_empty : sm.k_empty;
             const CUtensorMap* map = is_v ? &v_map : &k_map;
             const void* kv_base = is_v ? a.v : a.k;
-            const int n_stages = is_v ? kStagesV : kStages;
             bool alive = true;
+            // V tile j and K tile j + 1 are what step j reads: both arrive on its barrier
+            auto full_of = [&](int j) { return is_v ? &sm.step_full[j & 1] : (j == 0 ? &sm.k_first : &sm.step_full[(j - 1) & 1]); };
+            auto full_parity = [&](int j) { return is_v ? (unsigned)(j >> 1) & 1u : (j == 0 ? 0u : (unsigned)((j - 1) >> 1) & 1u); };
             if (!is_v) {   // what the set-up left out: Q tiles and first K tiles at the end of the packed buffers
                 if (q_edge(t0)) edge_tile_copy<D>(sm.q[0], a.q, a.q_heads, t0.head, (long long)sq.q_crow + t0.row0, tot_q, &sm.q_full[0], lane, a.d_real);
                 if (q_edge(t1)) edge_tile_copy<D>(sm.q[1], a.q, a.q_heads, t1.head, (long long)sq.q_crow + t1.row0, tot_q, &sm.q_full[1], lane, a.d_real);
                 for (int j = 0; j < n_pre; ++j)
-                    if (kv_edge(j)) edge_tile_copy<D>(sm.k[j], a.k, a.kv_heads, kvh, (long long)sq.kv_crow + (long long)j * kBlockN, tot_k, &sm.k_full[j], lane, a.d_real);
+                    if (kv_edge(j)) edge_tile_copy<D>(sm.k[j], a.k, a.kv_heads, kvh, (long long)sq.kv_crow + (long long)j * kBlockN, tot_k, full_of(j), lane, a.d_real);
             }
             // The sequence's last V tile, when the sequence does not end on a tile boundary, holds rows
             // that are not this sequence's: the unwritten rest of its last page, or the next sequence
@@ -760,15 +872,22 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             const int tail_j = sq.kv_len > 0 ? (sq.kv_len - 1) / kBlockN : -1;
             bool tail_pending = false;   // the tail tile's copy was issued and v_tail not yet seen complete
             int issued = is_v ? 0 : n_pre;   // K tiles 0 .. n_pre-1 were issued during set-up
-            for (int j = issued; j < n_max && alive; ++j) {
-                const int s = j % n_stages;
-                const int page = kPaged ? page_of_lane(a, sq.kv_len, b, j, lane) : -1;
-                if (j >= n_stages) {
-                    alive = __all_sync(0xffffffffu, mbar_wait(sm, &empty[s], ((unsigned)(j / n_stages) & 1u) ^ 1u, a, is_v ? 2 : 1));
+            // (the K producer goes one past the last tile: the last step's barrier wants its arrival too)
+            for (int j = issued; j < n_max + (is_v ? 0 : 1) && alive; ++j) {
+                if (!is_v && j == 0) break;   // no tile at all
+                const int s = j % kStages;
+                const int page = kPaged && j < n_max ? page_of_lane(a, sq.kv_len, b, j, lane) : -1;
+                if (j >= kStages) {   // the stage's tile: V(j - 2) was last read in step j - 2, K(j - 2) by the S of step j - 3
+                    const int e = is_v ? j - 1 : j - 2;
+                    alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.step_done[e & 1], (unsigned)(e >> 1) & 1u, a, is_v ? 2 : 1));
                     if (!alive) break;
                 }
+                if (j == n_max) {
+                    if (lane == 0) mbar_arrive(full_of(j));
+                    break;
+                }
                 const bool fix = tail_fix && j == tail_j;
-                unsigned long long* const bar = fix ? &sm.v_tail : &full[s];
+                unsigned long long* const bar = fix ? &sm.v_tail : full_of(j);
                 if (!is_v && a.test_skip_k == j + 1) {
                     // test hook: this tile is never requested, the issuer's wait for it runs out
                 } else if (kv_edge(j)) {
@@ -790,7 +909,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                             *reinterpret_cast<uint4*>(ring[s] + h * kHalfBytes + first * 128 + idx * 16) = make_uint4(0u, 0u, 0u, 0u);
                     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // generic-proxy writes -> tensor-core reads
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&full[s]);
+                    if (lane == 0) mbar_arrive(full_of(j));
                 }
             }
             // Make sure none of this warp's copies is still in flight when the CTA exits: wait
@@ -802,122 +921,21 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     if (t1.valid) mbar_wait(sm, &sm.q_full[1], 0, a, 3);
                 }
                 const unsigned long long t_begin = global_timer_ns();
-                for (int s = 0; s < n_stages; ++s) {
-                    if (issued <= s) continue;   // never filled
-                    const int last = issued - 1 - (issued - 1 - s) % n_stages;   // last issued tile of this stage
+                // (K: where the loop went one past the last tile, the tile before the last has been read, and its barrier used again)
+                for (int last = max(0, issued - (!is_v && alive ? 1 : kStages)); last < issued; ++last) {
                     if (!is_v && a.test_skip_k == last + 1) continue;          // test hook: never requested
                     if (tail_fix && last == tail_j) {
                         // that tile's copy completes on v_tail; the ring's barrier got (or, after an abort, never gets) a plain arrival
                         while (tail_pending && !mbar_try_wait(&sm.v_tail, 0u) && global_timer_ns() - t_begin < 100000000ULL) {}
                         continue;
                     }
-                    while (!mbar_try_wait(&full[s], (unsigned)(last / n_stages) & 1u) && global_timer_ns() - t_begin < 100000000ULL) {}
+                    // (after an abort the other ring's arrival may be missing; the copies have landed long before the limit then)
+                    while (!mbar_try_wait(full_of(last), full_parity(last)) && global_timer_ns() - t_begin < 100000000ULL) {}
                 }
             }
         }
     } else if (warp == kMmaWarp) {
-        // ------------------------------ MMA issuer ------------------------------
-        {   // the whole warp runs this block converged (see tc_mma_ss_imm)
-            const unsigned idesc_qk = make_idesc<T>(false, kBlockN);
-            const unsigned idesc_pv = make_idesc<T>(true, D);   // N = head size
-            const TileInfo ts[2] = {t0, t1};
-            bool alive = true;
-            // Descriptors are built once; inside the loops an MMA costs one 64-bit add per operand. A
-            // single thread then issues a 128x128x16 product every ~64 clocks, the tensor pipe's own
-            // rate — rebuilding the descriptors per product held it at ~90.
-            const unsigned long long dq[2] = {make_desc(smem_u32(sm.q[0]), 16, 1024), make_desc(smem_u32(sm.q[1]), 16, 1024)};
-            const unsigned long long dk[2] = {make_desc(smem_u32(sm.k[0]), 16, 1024), make_desc(smem_u32(sm.k[1]), 16, 1024)};
-            const unsigned long long dv[3] = {make_desc(smem_u32(sm.v[0]), kHalfBytes, 1024), make_desc(smem_u32(sm.v[1]), kHalfBytes, 1024),
-                                              make_desc(smem_u32(sm.v[kStagesV - 1]), kHalfBytes, 1024)};
-            static_assert(kStages == 2 && (kStagesV == 3 || kStagesV == 2), "descriptor tables hold two K stages and up to three V stages");
-            auto issue_s = [&](int t, int stage) {
-                // S_t = Q_t K^T : D / 16 K-steps over d; both operands K-major, 128 B swizzle
-                const unsigned long long qd = t ? dq[1] : dq[0];
-                const unsigned long long kd = stage ? dk[1] : dk[0];
-                const unsigned d_tmem = tmem + t * 128;
-#pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    const unsigned long long inc = (unsigned long long)(((kk >> 2) * kHalfBytes + (kk & 3) * 32) >> 4);
-                    if (kk == 0) tc_mma_ss_imm<false>(d_tmem, qd + inc, kd + inc, idesc_qk);
-                    else tc_mma_ss_imm<true>(d_tmem, qd + inc, kd + inc, idesc_qk);
-                }
-            };
-            auto issue_pv = [&](int t, int stage, bool accumulate, int half) {
-                // O_t += P_t V : 8 K-steps of 16 keys; A = P from tensor memory (packed 16-bit, 8 columns
-                // per step), B = V MN-major: 64-column halves 16 KiB apart, 8-key groups 1 KiB apart
-                const unsigned long long vd = stage == 0 ? dv[0] : (stage == 1 ? dv[1] : dv[2]);
-                const unsigned d_tmem = tmem + 256 + t * 128;
-                const unsigned p_tmem = tmem + t * 128;
-#pragma unroll
-                for (int kk = half * 4; kk < half * 4 + 4; ++kk) {
-                    const unsigned long long inc = (unsigned long long)((kk * 2048) >> 4);
-                    if (kk == 0 && !accumulate) tc_mma_ts_imm<false>(d_tmem, p_tmem + kk * 8, vd + inc, idesc_pv);
-                    else tc_mma_ts_imm<true>(d_tmem, p_tmem + kk * 8, vd + inc, idesc_pv);
-                }
-            };
-            // The copies were requested in the order Q0, K0, Q1: the first S of tile 0 is issued as soon as
-            // its two operands are there, without waiting for the other tile's Q.
-            if (ts[0].valid) alive = (mbar_wait(sm, &sm.q_full[0], 0, a, 10));
-            if (alive && n_max > 0) alive = (mbar_wait(sm, &sm.k_full[0], 0, a, 11));
-            if (alive && ts[0].n_kv > 0) {
-                tc_fence_after();
-                issue_s(0, 0);
-                tc_commit(&sm.s_full[0]);
-            }
-            if (alive && ts[1].valid) alive = (mbar_wait(sm, &sm.q_full[1], 0, a, 10));
-            FA_TRACE_EVENT(2, kTraceSteps - 1, 2);       // Q and the first K tile have landed
-            if (alive && n_max > 0) {
-                tc_fence_after();
-                if (ts[1].n_kv > 0) {
-                    issue_s(1, 0);
-                    tc_commit(&sm.s_full[1]);
-                }
-                tc_commit(&sm.k_empty[0]);
-            }
-            for (int j = 0; j < n_max && alive; ++j) {
-                const int s = j % kStagesV;                              // V stage of this step
-                const unsigned ph = (unsigned)(j / kStagesV) & 1u;
-                const int s1 = (j + 1) % kStages;                        // K stage of the next step
-                const unsigned ph1 = (unsigned)((j + 1) / kStages) & 1u;
-                alive = (mbar_wait(sm, &sm.v_full[s], ph, a, 13));
-                if (!alive) break;
-                FA_TRACE_EVENT(2, j, 4);
-                bool k_seen = j + 1 >= n_max;   // K(j+1) is first needed for S(j+1): looked at while P's second half is awaited
-                for (int t = 0; t < 2; ++t) {
-                    if (j >= ts[t].n_kv) continue;
-                    // the first 64 keys of P_t arrive while the softmax still works on the other 64:
-                    // their half of P.V leaves the critical path
-                    alive = (mbar_wait(sm, &sm.p_lo[t], (unsigned)j & 1u, a, 14 + t));
-                    if (!alive) break;
-                    FA_TRACE_EVENT(2, j, t * 2);
-                    tc_fence_after();
-                    issue_pv(t, s, j > 0, 0);
-                    if (!k_seen) {
-                        alive = (mbar_wait(sm, &sm.k_full[s1], ph1, a, 12));
-                        if (!alive) break;
-                        k_seen = true;
-                    }
-                    alive = (mbar_wait(sm, &sm.p_hi[t], (unsigned)j & 1u, a, 16 + t));
-                    if (!alive) break;
-                    FA_TRACE_EVENT(2, j, 5 + t);
-                    tc_fence_after();
-                    issue_pv(t, s, true, 1);
-                    if (j + 1 < ts[t].n_kv) issue_s(t, s1);
-                    tc_commit(&sm.s_full[t]);   // S_t(j+1) ready, or after the last PV: O_t final
-                    FA_TRACE_EVENT(2, j, t * 2 + 1);
-                }
-                if (!alive) break;
-                tc_commit(&sm.v_empty[s]);
-                if (j + 1 < n_max) tc_commit(&sm.k_empty[s1]);
-            }
-            if (!alive) {
-                // error path: tensor memory is freed at the end of the kernel, so let every product issued
-                // so far finish first (bounded; depends on the tensor pipe alone)
-                tc_commit(&sm.drain);
-                const unsigned long long t_begin = global_timer_ns();
-                while (!mbar_try_wait(&sm.drain, 0u) && global_timer_ns() - t_begin < 100000000ULL) {}
-            }
-        }
+        issue_products<T, D>(smem_u32(&sm), tmem, t0.n_kv, t1.n_kv, a.status, a.wait_ns FA_TRACE_ARG(trace));
     }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 208;\n");
@@ -1056,9 +1074,9 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 }
                 tc_wait_st();
                 tc_fence_before();
-                mbar_arrive(&sm.p_lo[t]);
+                mbar_arrive(&sm.p_ready[0][t]);
                 FA_TRACE_EVENT(t, j, 2);
-                mbar_arrive(&sm.p_hi[t]);
+                mbar_arrive(&sm.p_ready[1][t]);
                 float sum_lo, sum_hi;
                 unpack2(sum2, sum_lo, sum_hi);
                 l = l * alpha + (sum_lo + sum_hi);
@@ -1143,7 +1161,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                         tc_st32(s_addr + c * 32, pu);
                         tc_wait_st();
                         tc_fence_before();
-                        mbar_arrive(c == 0 ? &sm.p_lo[t] : &sm.p_hi[t]);
+                        mbar_arrive(&sm.p_ready[c][t]);
                         if (c == 0) FA_TRACE_EVENT(t, j, 2);
                     }
                 };
