@@ -76,7 +76,7 @@ struct SharedStorage {
     unsigned long long s_full[2];   // MMA -> softmax: S_t ready (and every earlier MMA finished)
     unsigned long long p_ready[2][2];   // softmax -> MMA: keys 0-63 of P_t written and O_t rescaled ([0][t]), keys 64-127 written ([1][t])
     unsigned long long v_tail;      // copy engine -> V producer: the sequence's last, partly filled V tile has landed
-    unsigned long long drain;       // MMA issuer, error path only: every product issued so far has finished
+    unsigned long long drain;       // MMA issuer, at its end: every product issued has finished
     unsigned int tmem_base;
     volatile int abort_flag;
     int item[3];                    // ordered launches: sequence (-1: none left), KV head, tile pair of this CTA
@@ -600,8 +600,8 @@ __device__ __forceinline__ unsigned clock_lo() {
 // 884 -> 833 us; 4 x 2048 MHA 157.5 -> 147.8 us; head size 64, 2 x 8192 GQA 755 -> 699 us.
 //   * a function of its own, so that the compiler sees what is the same for the whole warp (everything is, or is broadcast here): inside
 //     the kernel, whose early returns and per-sequence loads it takes for divergent, a product was 11 instructions, here it is 6;
-//   * a wait that runs out is looked after once a step: the loop goes on, without waiting for anything more, on what happens to be in
-//     shared memory (the softmax warps leave at the abort flag; nothing is written). Leaving at each wait doubled the code after it.
+//   * a wait that runs out is looked after at the end of its step, which goes on without waiting on what happens to be in shared memory and
+//     reports nothing as done. Leaving at each wait doubled the code after it.
 // n0, n1: K/V tiles that query tile 0 and 1 need (0: none, or no such tile).
 template <typename T, int D>
 __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int n0, int n1, int* status, unsigned long long wait_ns
@@ -627,6 +627,7 @@ __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int
         while (!__any_sync(0xffffffffu, mbar_try_wait_at(sm_addr + (unsigned)bar, parity))) {
             if (__any_sync(0xffffffffu, clock_lo() - t0 >= patience)) {
                 expired = where;
+                patience = 0;
                 break;
             }
         }
@@ -651,8 +652,10 @@ __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int
                 tc_mma_ts(tmem + 256 + t * 128, tmem + t * 128 + half * 32 + kk * 8, vd + half * 512 + kk * (2048 >> 4), idesc_pv, kk > 0 || accumulate);
         }
     };
+    // Nothing is reported as done after a wait has run out: a producer that took a stage for free out of turn would arrive on a barrier whose phase
+    // has both its arrivals but not all its bytes, which the hardware takes for an error.
     auto commit = [&](size_t bar) {
-        if (elect_one()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(sm_addr + (unsigned)bar) : "memory");
+        if (expired == 0 && elect_one()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(sm_addr + (unsigned)bar) : "memory");
     };
     if (n_max > 0) {
         // The copies were requested in the order Q0, K0, Q1: the first S of tile 0 is issued as soon as
@@ -699,17 +702,16 @@ __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int
             set_shared_flag(sm_addr + (unsigned)offsetof(Storage, abort_flag));
             *reinterpret_cast<volatile int*>(status) = expired;
             __threadfence_system();
-            patience = 0;
+            break;
         }
     }
-    if (expired != 0) {
-        // error path: tensor memory is freed at the end of the kernel, so let every product issued
-        // so far finish first (bounded; depends on the tensor pipe alone)
-        __syncwarp();
-        commit(offsetof(Storage, drain));
-        const unsigned long long t_begin = global_timer_ns();
-        while (!mbar_try_wait_at(sm_addr + (unsigned)offsetof(Storage, drain), 0u) && global_timer_ns() - t_begin < 100000000ULL) {}
-    }
+    // Tensor memory is freed at the end of the kernel, in error paths while the softmax warps have long left: every product issued here has to
+    // finish first (bounded; depends on the tensor pipe alone). Otherwise the last P.V is what the epilogue waits for as well.
+    __syncwarp();
+    expired = 0;
+    commit(offsetof(Storage, drain));
+    const unsigned long long t_begin = global_timer_ns();
+    while (!mbar_try_wait_at(sm_addr + (unsigned)offsetof(Storage, drain), 0u) && global_timer_ns() - t_begin < 100000000ULL) {}
 }
 
 // kMask: the call carries a key-padding mask (a separate instantiation, so that calls without one

@@ -53,6 +53,35 @@ def test_expired_wait_is_reported_by_the_next_call_and_then_cleared():
     H.assert_bf16_close(H.to_np(o), ob.attn_f64_batch(q, k, v), "call after the reported expiry")
 
 
+@pytest.mark.parametrize("d", [128, 64])
+@pytest.mark.parametrize("tile", [0, 1, 2, 5])
+def test_expiry_at_every_part_of_the_key_loop(tile, d):
+    # the first tile, the two that the set-up requests, one behind the rings' first round: the issuer reports nothing as done after its wait has
+    # run out, so no producer takes a stage out of turn, and the kernel ends; the call after the report is right
+    b, s, hq, hkv = 1, 1024, 2, 1
+    q = H.round_to(H.normal((b, s, hq, d), 1), "bf16")
+    k = H.round_to(H.normal((b, s, hkv, d), 2), "bf16")
+    v = H.round_to(H.normal((b, s, hkv, d), 3), "bf16")
+    qd, kd, vd = (H.to_dev(x, "bf16") for x in (q, k, v))
+    o = torch.empty_like(qd)
+    args = (qd, kd, vd, o, b, s, s, hq, hkv, d, 0, 1.0 / math.sqrt(d))
+    assert ffi.device_status() == 0
+    try:
+        ffi.set_option("prefill_wait_us", 1000)
+        ffi.set_option("prefill_test_skip_k", tile + 1)
+        low.flash_attn(*args)
+    finally:
+        ffi.set_option("prefill_test_skip_k", 0)
+        ffi.set_option("prefill_wait_us", 0)
+    torch.cuda.synchronize()
+    with pytest.raises(E.CudaError):
+        low.flash_attn(*args)
+    low.flash_attn(*args)
+    torch.cuda.synchronize()
+    assert ffi.device_status() == 0
+    H.assert_bf16_close(H.to_np(o), ob.attn_f64_batch(q, k, v), "call after the reported expiry")
+
+
 def test_workspaces_are_bounded_and_releasable():
     # the decode path keeps one split-K workspace per (device, stream), at most 32, and gives them back on request
     hq, hkv, d, bs = 8, 2, 128, 16
