@@ -88,6 +88,20 @@ constexpr int kCtaLogEntries = 2048;
 #endif
 constexpr unsigned long long kWaitLimitNs = 2000000000ULL;   // default bound of every mbarrier wait
 
+// Division of n < 2^31 by a divisor the host knows, as a product with its rounded-up inverse (Granlund and Montgomery, "Division by
+// invariant integers using multiplication"): three instructions. The compiler's division is some forty dependent ones, and a CTA made ten before its
+// first copy was requested: 1700 clocks from its start, on every SM with nothing else to do.
+struct FastDiv {
+    unsigned mul, shift;
+    int d;
+    FastDiv() = default;
+    __host__ explicit FastDiv(int divisor) : mul(0), shift(0), d(divisor) {
+        while ((1u << shift) < (unsigned)d) ++shift;
+        mul = (unsigned)((((1ULL << shift) - (unsigned)d) << 32) / (unsigned)d) + 1u;
+    }
+    __device__ __forceinline__ int div(int n) const { return (int)((__umulhi((unsigned)n, mul) + (unsigned)n) >> shift); }
+};
+
 struct PrefillArgs {
     // Output: n_out buffers of (batch, q_seq_len, o_heads, 128), each receiving this launch's heads
     // at head offset o_head0. n_out == 1 with o_heads == q_heads is the ordinary call; with n_out > 1
@@ -111,6 +125,8 @@ struct PrefillArgs {
 #endif
     int batch, q_seq_len, kv_seq_len, q_heads, kv_heads, start_pos;
     int d_real;     // head size of the tensors: D, or 32 when the D = 64 kernel runs a head size of 32 on zero-padded tiles
+    FastDiv by_group, by_kv_heads, by_band;   // query heads per KV head; KV heads; band
+    int streams_z;  // (batch, KV head) streams per blockIdx.z
     int band;       // tile pairs of one (batch, KV head) that sit next to each other in blockIdx.x
     // Launch order of the bands (blockIdx.y), heaviest = 0. spread_w == 0: heaviest first. Otherwise the
     // first spread_w rows of the grid are every spread_m-th band (a first wave that mixes all weights,
@@ -413,7 +429,7 @@ __device__ __forceinline__ SeqExtent seq_extent(const PrefillArgs& a, int s) {
     return e;
 }
 
-__device__ __forceinline__ TileInfo tile_info(const SeqExtent& a, int pair, int t, int kvh, int group, int num_mb) {
+__device__ __forceinline__ TileInfo tile_info(const SeqExtent& a, int pair, int t, int kvh, const FastDiv& by_group, int num_mb) {
     TileInfo ti;
     // Tile 0 takes the later index of the pair: where the pair is two consecutive row blocks of one head
     // (group 1), that is the longer tile, and tile 0 is the one whose copies are requested first and whose
@@ -421,8 +437,9 @@ __device__ __forceinline__ TileInfo tile_info(const SeqExtent& a, int pair, int 
     // the one that waits (S = 2048 MHA: 887-892 against 851 TFLOP/s; no difference for GQA pairs, whose
     // two tiles are equally long).
     const int idx = pair * 2 + (1 - t);
+    const int group = by_group.d;
     ti.valid = idx < group * num_mb;
-    const int mb = ti.valid ? idx / group : 0;
+    const int mb = ti.valid ? by_group.div(idx) : 0;
     ti.head = kvh * group + (ti.valid ? idx - mb * group : 0);
     ti.row0 = mb * kBlockM;
     const int last_row = min(ti.row0 + kBlockM, a.q_len) - 1;
@@ -733,7 +750,26 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // (the same for the whole warp, which the compiler sees only so)
     const int lane = threadIdx.x & 31;
-    const int group = a.q_heads / a.kv_heads;
+    const int group = a.by_group.d;
+    if (warp == kLoadWarp && lane == 0) {   // (what needs no extents goes first: their loads are on the way meanwhile)
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&q_map) : "memory");
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&k_map) : "memory");
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&v_map) : "memory");
+        sm.abort_flag = 0;
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&sm.q_full[i], 1);
+            mbar_init(&sm.s_full[i], 1);
+            mbar_init(&sm.p_ready[0][i], 128);
+            mbar_init(&sm.p_ready[1][i], 128);
+            mbar_init(&sm.step_full[i], 2);
+            mbar_init(&sm.step_done[i], 1);
+        }
+        mbar_init(&sm.k_first, 1);
+        mbar_init(&sm.v_tail, 1);
+        mbar_init(&sm.drain, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    }
     // A few-row kernel launched behind this one may start once every CTA here has: it fills the SMs that run out of tile pairs.
     if (a.skip_rows > 0) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     int b, kvh, pair;
@@ -752,25 +788,25 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         // HBM, while the order across bands stays heaviest first.
         // blockIdx.z = group of K/V streams: the grid runs group after group (each heaviest first), so that the
         // K/V of the streams in flight stay within L2 when every tile pair of a stream re-reads its stream's prefix
-        const int stream_id = (int)blockIdx.z * (int)(gridDim.x / a.band) + (int)(blockIdx.x / a.band);
+        const int x_band = a.by_band.div((int)blockIdx.x);
+        const int stream_id = (int)blockIdx.z * a.streams_z + x_band;
         if (stream_id >= a.kv_heads * a.batch) return;   // the last group may be short
-        kvh = stream_id % a.kv_heads;
-        b = stream_id / a.kv_heads;
+        b = a.by_kv_heads.div(stream_id);
+        kvh = stream_id - b * a.kv_heads;
         const int rank_y = launch_rank((int)blockIdx.y, a.spread_w, a.spread_m);   // this row's rank by weight, 0 = heaviest
-        pair = ((int)gridDim.y - 1 - rank_y) * a.band + (a.band - 1 - (int)(blockIdx.x % a.band));
+        pair = ((int)gridDim.y - 1 - rank_y) * a.band + (a.band - 1 - ((int)blockIdx.x - x_band * a.band));
     }
     const SeqExtent sq = seq_extent(a, b);
     if (sq.q_len * group <= a.skip_rows) return;   // the few-row kernel's
     const int num_mb = (sq.q_len + kBlockM - 1) / kBlockM;
 
-    const TileInfo t0 = tile_info(sq, pair, 0, kvh, group, num_mb);
-    const TileInfo t1 = tile_info(sq, pair, 1, kvh, group, num_mb);
+    const TileInfo t0 = tile_info(sq, pair, 0, kvh, a.by_group, num_mb);
+    const TileInfo t1 = tile_info(sq, pair, 1, kvh, a.by_group, num_mb);
     if (!t0.valid && !t1.valid) return;   // this sequence is shorter than the grid's row range (whole CTA leaves)
     const int n_max = max(t0.n_kv, t1.n_kv);
 
-    // The producer thread initialises the barriers itself and issues the first loads right away (Q,
-    // and the K/V tiles that fill the empty ring), before the CTA-wide set-up barrier: the copies
-    // then fly while tensor memory is being allocated and the other warps start up.
+    // The first copies are requested before the CTA-wide set-up barrier, by the two producer warps (Q and the K tiles that fill the empty ring; the
+    // V tiles likewise): they fly while tensor memory is being allocated and the other warps start up.
     const int n_pre = min(kStages, n_max);
     // Packed buffers end at row cu_seqlens[num_seqs]; a tile that reaches past that row is not asked
     // of the copy engine (see edge_tile_copy) but fetched by the producer warp after the set-up.
@@ -779,31 +815,11 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     const long long tot_k = (packed && !a.paged) ? (long long)a.cu_k[a.batch] : 0;
     auto q_edge = [&](const TileInfo& ti) { return packed && ti.valid && (long long)sq.q_crow + ti.row0 + kBlockM > tot_q; };
     auto kv_edge = [&](int j) { return packed && !a.paged && (long long)sq.kv_crow + (long long)(j + 1) * kBlockN > tot_k; };
+    if (warp == kLoadWarp) asm volatile("barrier.cta.arrive 1, 64;\n" ::: "memory");
     if (warp == kLoadWarp && (kPaged || lane == 0)) {
         int pages[kStages];   // of the tiles requested here, looked up together
 #pragma unroll
         for (int j = 0; j < kStages; ++j) pages[j] = kPaged && j < n_pre ? page_of_lane(a, sq.kv_len, b, j, lane) : -1;
-        if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&q_map) : "memory");
-            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&k_map) : "memory");
-            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&v_map) : "memory");
-            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&o_map) : "memory");
-            sm.abort_flag = 0;
-            for (int i = 0; i < 2; ++i) {
-                mbar_init(&sm.q_full[i], 1);
-                mbar_init(&sm.s_full[i], 1);
-                mbar_init(&sm.p_ready[0][i], 128);
-                mbar_init(&sm.p_ready[1][i], 128);
-                mbar_init(&sm.step_full[i], 2);
-                mbar_init(&sm.step_done[i], 1);
-            }
-            mbar_init(&sm.k_first, 1);
-            mbar_init(&sm.v_tail, 1);
-            mbar_init(&sm.drain, 1);
-            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        }
-        if (kPaged) __syncwarp();
         auto load_q = [&](const TileInfo& ti, int t) {
             if ((kPaged && lane != 0) || !ti.valid || q_edge(ti)) return;
             mbar_expect_tx(&sm.q_full[t], TileBytes<D>::value);
@@ -816,7 +832,17 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             if (j < n_pre && !kv_edge(j) && a.test_skip_k != j + 1) load_kv_tile<D, kPaged>(a, sq, kvh, sm.k[j], &k_map, j == 0 ? &sm.k_first : &sm.step_full[0], j, pages[j], lane);
             if (j == 0) load_q(t1, 1);
         }
-        // the V tiles come from a producer thread of their own (warp kLoadWarpV), after the set-up barrier
+        if (lane == 0) asm volatile("prefetch.tensormap [%0];\n" ::"l"(&o_map) : "memory");
+    }
+    int v_issued = 0;
+    if (warp == kLoadWarpV) {
+        asm volatile("barrier.cta.sync 1, 64;\n" ::: "memory");   // the barriers have been initialised
+        // (the tiles that need more than a copy are left to the producer loop)
+        while (v_issued < n_pre && !kv_edge(v_issued) && !((a.paged || packed) && (v_issued + 1) * kBlockN > sq.kv_len)) {
+            if (kPaged || lane == 0)
+                load_kv_tile<D, kPaged>(a, sq, kvh, sm.v[v_issued], &v_map, &sm.step_full[v_issued], v_issued, kPaged ? page_of_lane(a, sq.kv_len, b, v_issued, lane) : -1, lane);
+            ++v_issued;
+        }
     }
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(&sm.tmem_base)) : "memory");
@@ -873,7 +899,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             const bool tail_fix = is_v && (a.paged || packed) && (sq.kv_len % kBlockN) != 0;
             const int tail_j = sq.kv_len > 0 ? (sq.kv_len - 1) / kBlockN : -1;
             bool tail_pending = false;   // the tail tile's copy was issued and v_tail not yet seen complete
-            int issued = is_v ? 0 : n_pre;   // K tiles 0 .. n_pre-1 were issued during set-up
+            int issued = is_v ? v_issued : n_pre;   // tiles that were requested during set-up
             // (the K producer goes one past the last tile: the last step's barrier wants its arrival too)
             for (int j = issued; j < n_max + (is_v ? 0 : 1) && alive; ++j) {
                 if (!is_v && j == 0) break;   // no tile at all
@@ -1203,39 +1229,34 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 // of 32 different rows per instruction would fill the SM's memory pipeline for thousands
                 // of clocks and hold up the barrier traffic of the other tile's last steps. Rows past the
                 // end of the sequence are outside the tensor map and are not written.
-                float ov[D / 32][32];
-#pragma unroll
-                for (int c = 0; c < D / 32; ++c) tc_ld32(o_addr + c * 32, ov[c]);
-                tc_wait_ld();
-                if (ti.n_kv == 0) {   // the tile saw no key: tensor memory holds nothing of ours, the rows are zeros
-#pragma unroll
-                    for (int c = 0; c < D / 32; ++c)
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) ov[c][i] = 0.0f;
-                }
                 unsigned char* stage = sm.q[t];
+#pragma unroll 1
+                for (int h = 0; h < D / 64; ++h) {   // a half's copy is on its way while the next one is packed
+                    float ov[2][32];
+                    tc_ld32(o_addr + h * 64, ov[0]);
+                    tc_ld32(o_addr + h * 64 + 32, ov[1]);
+                    tc_wait_ld();
+                    if (ti.n_kv == 0) {   // the tile saw no key: tensor memory holds nothing of ours, the rows are zeros
 #pragma unroll
-                for (int c = 0; c < D / 32; ++c) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        uint4 w;
-                        w.x = pack16<T>(ov[c][8 * i] * inv, ov[c][8 * i + 1] * inv);
-                        w.y = pack16<T>(ov[c][8 * i + 2] * inv, ov[c][8 * i + 3] * inv);
-                        w.z = pack16<T>(ov[c][8 * i + 4] * inv, ov[c][8 * i + 5] * inv);
-                        w.w = pack16<T>(ov[c][8 * i + 6] * inv, ov[c][8 * i + 7] * inv);
-                        const int ch = (c & 1) * 4 + i;   // 16-byte chunk within the 64-column half c >> 1
-                        *reinterpret_cast<uint4*>(stage + (c >> 1) * kHalfBytes + r * 128 + ((ch ^ (r & 7)) << 4)) = w;
+                        for (int i = 0; i < 32; ++i) ov[0][i] = ov[1][i] = 0.0f;
                     }
-                }
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // generic-proxy writes -> bulk copy reads
-                __syncwarp();
-                if (lane == 0) {
-                    const int warp_row0 = (warp & 3) * 32;
-                    tma_store_4d(&o_map, stage + warp_row0 * 128, 0, a.o_head0 + ti.head, sq.q_crow + ti.row0 + warp_row0, sq.q_cb);
-                    if (D == 128)
-                        tma_store_4d(&o_map, stage + kHalfBytes + warp_row0 * 128, 64, a.o_head0 + ti.head, sq.q_crow + ti.row0 + warp_row0, sq.q_cb);
-                    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
-                    asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // shared memory stays valid until read
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {   // 16-byte chunk i of the 64-column half
+                        const float* o8 = &ov[i >> 2][8 * (i & 3)];
+                        uint4 w;
+                        w.x = pack16<T>(o8[0] * inv, o8[1] * inv);
+                        w.y = pack16<T>(o8[2] * inv, o8[3] * inv);
+                        w.z = pack16<T>(o8[4] * inv, o8[5] * inv);
+                        w.w = pack16<T>(o8[6] * inv, o8[7] * inv);
+                        *reinterpret_cast<uint4*>(stage + h * kHalfBytes + r * 128 + ((i ^ (r & 7)) << 4)) = w;
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // generic-proxy writes -> bulk copy reads
+                    __syncwarp();
+                    if (lane == 0) {
+                        const int warp_row0 = (warp & 3) * 32;
+                        tma_store_4d(&o_map, stage + h * kHalfBytes + warp_row0 * 128, h * 64, a.o_head0 + ti.head, sq.q_crow + ti.row0 + warp_row0, sq.q_cb);
+                        asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+                    }
                 }
             } else {
                 // Stage this warp's 32 rows (2 D bytes each) in the Q tile's shared memory — every MMA that read
@@ -1300,6 +1321,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 const long long g_off = ((long long)b * a.o_heads + a.o_head0 + ti.head) * a.q_seq_len + row;
                 for (int n = 0; n < a.n_lse; ++n) a.lse_peers[n][g_off] = lse_val;
             }
+            if (bulk_ok && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // shared memory stays valid until read
             FA_TRACE_EVENT(t, kTraceSteps - 1, 0);       // epilogue stores issued
         }
     }
@@ -1531,6 +1553,9 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
         if (get_option_prefill_band() > 0) band = std::min(get_option_prefill_band(), pairs);
     }
     a.band = band;
+    a.by_band = FastDiv(band);
+    a.by_kv_heads = FastDiv(p.kv_heads);
+    a.by_group = FastDiv(group);
     // Head-sharded call (every CTA ends with stores to the other GPUs): heaviest-first makes the SMs end
     // their CTAs in waves, each wave a burst on the links that stalls every SM in it. A first wave that
     // mixes all weights staggers the SMs for the rest of the launch; the rest stays heaviest first, which
@@ -1573,6 +1598,7 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
         if (groups < 1) groups = 1;
     }
     const int streams_per_group = (int)(((long long)p.kv_heads * p.num_seqs + groups - 1) / groups);
+    a.streams_z = streams_per_group;
     dim3 grid(streams_per_group * band, (pairs + band - 1) / band, groups);
     a.pairs = pairs;
     const MixedFewRows few = prepare_mixed_few_rows(p, stream);   // its workspace is this call's until both kernels are launched
