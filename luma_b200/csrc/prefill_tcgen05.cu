@@ -58,10 +58,9 @@ constexpr int kHalfBytes = kBlockN * 64 * 2;   // 16 KiB: one 64-column half, 12
 template <int D> struct TileBytes { static constexpr int value = kBlockN * D * 2; };   // one half at D = 64, two at D = 128
 constexpr float kRescaleThreshold = 8.0f;            // log2 units
 
-// Which element pairs of an unmasked chunk take their exponential on the FMA pipe (a cubic) instead
-// of the special-function unit: one pair in eight. Measured on the S = 8192 GQA prefill, same box:
-// none 1231, one in eight 1237, one in four 1207, three in eight 1128, one in two 1058 TFLOP/s — the
-// cubic costs about as many issue slots as the special-function unit saves, so the share is small.
+// Which element pairs take their exponential on the FMA pipe (a quartic) instead of the special-function unit: one in eight. It costs issue slots
+// and registers that the special-function unit's time does not buy back at a larger share where CTAs are short. us a pass for a share of 1/16, 1/8,
+// 1/6, 1/4: 2 x 8192 GQA 961, 947, 945, 954; 4 x 2048 MHA 163.4, 161.3, 162.2, 163.1; 4 chunks of 512 155.8, 155.0, 156.3, 158.5.
 __device__ __forceinline__ constexpr bool fma_pipe_exp(int i) { return (i & 7) == 7; }
 
 template <int D>
@@ -318,25 +317,29 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
     asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-// 2^x for two finite x on the FMA pipe instead of the special-function unit: x = n + f with n the
-// nearest integer (magic-number rounding), a cubic for 2^f on [-0.5, 0.5] (relative error 7.5e-5,
-// far below the 16-bit rounding of P), and n added to the exponent field. x is clamped at -126,
-// so the result is never below 2^-126 — callers use this only where no element is masked.
+// 2^x for two x on the FMA pipe instead of the special-function unit: x = n + f with n the
+// nearest integer (magic-number rounding), a quartic for 2^f on [-0.5, 0.5] (minimax by the Remez exchange, relative error 2.6e-6), and n
+// added to the exponent field. x is clamped at -200, where that addition gives a negative integer, and those become zeros: 2^x for x
+// below -126.5, -inf (a masked score) among them, is an exact zero or below 2^-126. A NaN is not clamped and gives no finite result.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float d;
+    asm("max.NaN.f32 %0, %1, %2;\n" : "=f"(d) : "f"(a), "f"(b));
+    return d;
+}
 __device__ __forceinline__ void ex2_fma2(float x0, float x1, float& p0, float& p1) {
-    x0 = fmaxf(x0, -126.0f);
-    x1 = fmaxf(x1, -126.0f);
-    const unsigned long long x2 = pack2(x0, x1);
+    const unsigned long long x2 = pack2(max_nan(x0, -200.0f), max_nan(x1, -200.0f));
     const unsigned long long t2 = add2(x2, pack2(12582912.0f, 12582912.0f));   // 1.5 * 2^23
     const unsigned long long n2 = add2(t2, pack2(-12582912.0f, -12582912.0f));
     const unsigned long long f2 = fma2(n2, pack2(-1.0f, -1.0f), x2);
-    unsigned long long p2 = fma2(pack2(0.05517084f, 0.05517084f), f2, pack2(0.24260908f, 0.24260908f));
-    p2 = fma2(p2, f2, pack2(0.69326109f, 0.69326109f));
-    p2 = fma2(p2, f2, pack2(0.99992847f, 0.99992847f));
+    unsigned long long p2 = fma2(pack2(0.009570101911f, 0.009570101911f), f2, pack2(0.05591786032f, 0.05591786032f));
+    p2 = fma2(p2, f2, pack2(0.2402474483f, 0.2402474483f));
+    p2 = fma2(p2, f2, pack2(0.6931218147f, 0.6931218147f));
+    p2 = fma2(p2, f2, pack2(0.9999992614f, 0.9999992614f));
     float t0, t1, q0, q1;
     unpack2(t2, t0, t1);
     unpack2(p2, q0, q1);
-    p0 = __uint_as_float(__float_as_uint(q0) + (__float_as_uint(t0) << 23));
-    p1 = __uint_as_float(__float_as_uint(q1) + (__float_as_uint(t1) << 23));
+    p0 = __int_as_float(max(__float_as_int(q0) + (__float_as_int(t0) << 23), 0));
+    p1 = __int_as_float(max(__float_as_int(q1) + (__float_as_int(t1) << 23), 0));
 }
 
 template <typename T> __device__ __forceinline__ unsigned pack16(float lo, float hi);
@@ -991,215 +994,98 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             const bool need_mask = (long long)(key0 + kBlockN - 1) > min((long long)sq.pos_off + ti.row0, (long long)sq.kv_len - 1);
             const int limit = need_mask ? (int)max(-1LL, min(limit_ll, (long long)kBlockN)) : kBlockN;
 
-            // An aligned diagonal tile (row i of the tile sees exactly keys 0..i of it) has a fixed shape
-            // per warp: warp w sees chunks 0..w-1 of 32 columns in full, chunk w up to its own lane,
-            // nothing after it. It is handled with the chunks rotated so that the diagonal one sits in
-            // register slot 0 (the tensor-memory addresses are run-time values, the slots are not):
-            // 32 compares instead of 128, FMA-pipe exponentials in the full chunks, no work in the
-            // unseen ones. Any other masked tile (cut by the end of K/V, unaligned start) takes the
-            // general code below.
-            // Key-padding mask (batched entry point): the tile's 128 validity bytes become four ballots;
-            // a tile whose keys are all valid — the usual case, padding sits at one end — runs as if
-            // there were no mask, any other takes the general step with the bits applied first.
-            unsigned kb0 = 0xffffffffu, kb1 = 0xffffffffu, kb2 = 0xffffffffu, kb3 = 0xffffffffu;
-            bool pad = false;
+            // Masked scores become -inf, whose P is an exact zero from either exponential, so a masked tile runs the code of the others. (A form of its own
+            // for the aligned diagonal, which left out the chunks of 32 keys that a warp does not see, and one for other masked tiles were 17 KiB of
+            // straight-line code run once per tile: 2 x 8192 GQA 967 us with them, 948 without. Leaving unseen chunks out behind a branch in this
+            // code: 990 us, for what the compiler no longer interleaves.)
+            // Key-padding mask (batched entry point): the tile's validity bytes become a ballot per chunk of 32; a tile whose real keys are all
+            // valid (the usual case, padding sits at one end) runs as if there were no mask.
+            unsigned valid[4];
+            bool masked = need_mask;
             if (kMask) {
-                const unsigned char* mrow = a.mask + (long long)b * a.kv_seq_len;
-                const int kk = key0 + lane;
-                kb0 = __ballot_sync(0xffffffffu, kk < sq.kv_len && mrow[kk < sq.kv_len ? kk : 0] != 0);
-                kb1 = __ballot_sync(0xffffffffu, kk + 32 < sq.kv_len && mrow[kk + 32 < sq.kv_len ? kk + 32 : 0] != 0);
-                kb2 = __ballot_sync(0xffffffffu, kk + 64 < sq.kv_len && mrow[kk + 64 < sq.kv_len ? kk + 64 : 0] != 0);
-                kb3 = __ballot_sync(0xffffffffu, kk + 96 < sq.kv_len && mrow[kk + 96 < sq.kv_len ? kk + 96 : 0] != 0);
-                // keys past kv_len are cut by `limit` already; only padding among the real keys counts here
-                const int real = min(kBlockN, sq.kv_len - key0);
-                const unsigned w0 = real >= 32 ? 0xffffffffu : ((1u << max(real, 0)) - 1u);
-                const unsigned w1 = real >= 64 ? 0xffffffffu : (real <= 32 ? 0u : ((1u << (real - 32)) - 1u));
-                const unsigned w2 = real >= 96 ? 0xffffffffu : (real <= 64 ? 0u : ((1u << (real - 64)) - 1u));
-                const unsigned w3 = real >= 128 ? 0xffffffffu : (real <= 96 ? 0u : ((1u << (real - 96)) - 1u));
-                pad = ((kb0 & w0) != w0) || ((kb1 & w1) != w1) || ((kb2 & w2) != w2) || ((kb3 & w3) != w3);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int kk = key0 + c * 32 + lane;
+                    const bool real = kk < sq.kv_len;
+                    valid[c] = __ballot_sync(0xffffffffu, real && a.mask[(long long)b * a.kv_seq_len + (real ? kk : 0)] != 0);
+                    masked = masked || valid[c] != __ballot_sync(0xffffffffu, real);
+                }
             }
-            const bool diag_tile = !(kMask && pad) && need_mask && (long long)sq.pos_off + ti.row0 == (long long)key0 &&
-                                   (long long)sq.pos_off + ti.row0 + kBlockM - 1 <= (long long)sq.kv_len - 1;
-            if (diag_tile) {
-                const int w = warp & 3;
-                float dv[4][32];   // slot k holds chunk (w + k) & 3
+            float sv[4][32];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) tc_ld32(s_addr + ((w + k) & 3) * 32, dv[k]);
-                tc_wait_ld();
+            for (int c = 0; c < 4; ++c) tc_ld32(s_addr + c * 32, sv[c]);
+            tc_wait_ld();
+            if (masked) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    if (i > lane) dv[0][i] = -INFINITY;
-                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+                for (int c = 0; c < 4; ++c) {
+                    const int n = limit + 1 - c * 32;
+                    unsigned seen = n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : (1u << n) - 1u);   // keys that this row sees of the chunk
+                    if (kMask) seen &= valid[c];
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], dv[0][i], dv[0][i + 1]);
-#pragma unroll
-                for (int k = 1; k < 4; ++k) {
-                    if (((w + k) & 3) < w) {   // a chunk before the diagonal one: seen in full
-#pragma unroll
-                        for (int i = 0; i < 32; i += 2) mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], dv[k][i], dv[k][i + 1]);
-                    }
+                    for (int i = 0; i < 32; ++i)
+                        if (!((seen >> i) & 1u)) sv[c][i] = -INFINITY;
                 }
-                float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * a.scale_log2;
-                FA_TRACE_EVENT(t, j, 1);
-                float alpha = 1.0f;
-                bool changed = false;
-                if (mx > m + kRescaleThreshold) {
-                    alpha = ex2(m - mx);
-                    m = mx;
-                    changed = true;
-                }
-                if (j > 0 && __any_sync(0xffffffffu, changed)) {
+            }
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], sv[c][i], sv[c][i + 1]);
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * a.scale_log2;   // scale > 0 is guaranteed by the dispatcher
+            FA_TRACE_EVENT(t, j, 1);
+
+            float alpha = 1.0f;
+            bool changed = false;
+            if (mx > m + kRescaleThreshold) {   // also true for the first finite max (m == -inf)
+                alpha = ex2(m - mx);            // 0 when m == -inf
+                m = mx;
+                changed = true;
+            }
+            if (j > 0 && __any_sync(0xffffffffu, changed)) {
+                // rescale this warp's 32 rows of O in tensor memory (rows that did not move use 1.0)
 #pragma unroll 1
-                    for (int c = 0; c < D / 32; ++c) {
-                        float ov[32];
-                        tc_ld32(o_addr + c * 32, ov);
-                        tc_wait_ld();
-                        unsigned ou[32];
+                for (int c = 0; c < D / 32; ++c) {
+                    float ov[32];
+                    tc_ld32(o_addr + c * 32, ov);
+                    tc_wait_ld();
+                    unsigned ou[32];
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) ou[i] = __float_as_uint(ov[i] * alpha);
-                        tc_st32(o_addr + c * 32, ou);
-                    }
+                    for (int i = 0; i < 32; ++i) ou[i] = __float_as_uint(ov[i] * alpha);
+                    tc_st32(o_addr + c * 32, ou);
                 }
-                const float m_use = (m == -INFINITY) ? 0.0f : m;
-                const unsigned long long scale2 = pack2(a.scale_log2, a.scale_log2);
-                const unsigned long long neg_m2 = pack2(-m_use, -m_use);
-                unsigned long long sum2 = pack2(0.0f, 0.0f);
-                {   // the diagonal chunk: every exponential on the special-function unit (-inf gives an exact zero)
-                    unsigned pu[16];
+            }
+            const float m_use = (m == -INFINITY) ? 0.0f : m;
+            // exp2(s * scale - m) two columns at a time: packed FMA for the argument and the row sum
+            const unsigned long long scale2 = pack2(a.scale_log2, a.scale_log2);
+            const unsigned long long neg_m2 = pack2(-m_use, -m_use);
+            unsigned long long sum2 = pack2(0.0f, 0.0f);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        float x0, x1;
-                        unpack2(fma2(pack2(dv[0][2 * i], dv[0][2 * i + 1]), scale2, neg_m2), x0, x1);
-                        const float p0 = ex2(x0), p1 = ex2(x1);
-                        sum2 = add2(sum2, pack2(p0, p1));
-                        pu[i] = pack16<T>(p0, p1);
-                    }
-                    tc_st16(s_addr + w * 16, pu);   // P of chunk c lives in 16 packed columns at c * 16
-                }
+            for (int h = 0; h < 2; ++h) {   // 64 keys
+                unsigned pu[32];
 #pragma unroll
-                for (int k = 1; k < 4; ++k) {
-                    const int c = (w + k) & 3;
-                    unsigned pu[16];
-                    if (c < w) {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            float x0, x1, p0, p1;
-                            unpack2(fma2(pack2(dv[k][2 * i], dv[k][2 * i + 1]), scale2, neg_m2), x0, x1);
-                            if (fma_pipe_exp(i)) {
-                                ex2_fma2(x0, x1, p0, p1);
-                            } else {
-                                p0 = ex2(x0);
-                                p1 = ex2(x1);
-                            }
-                            sum2 = add2(sum2, pack2(p0, p1));
-                            pu[i] = pack16<T>(p0, p1);
-                        }
+                for (int i = 0; i < 32; ++i) {
+                    const float(&x)[32] = sv[h * 2 + (i >> 4)];
+                    const int ii = (i & 15) * 2;
+                    float x0, x1, e0, e1;
+                    unpack2(fma2(pack2(x[ii], x[ii + 1]), scale2, neg_m2), x0, x1);
+                    if (fma_pipe_exp(i)) {
+                        ex2_fma2(x0, x1, e0, e1);
                     } else {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) pu[i] = 0u;
+                        e0 = ex2(x0);
+                        e1 = ex2(x1);
                     }
-                    tc_st16(s_addr + c * 16, pu);
+                    sum2 = add2(sum2, pack2(e0, e1));
+                    pu[i] = pack16<T>(e0, e1);
                 }
+                tc_st32(s_addr + h * 32, pu);
                 tc_wait_st();
                 tc_fence_before();
-                mbar_arrive(&sm.p_ready[0][t]);
-                FA_TRACE_EVENT(t, j, 2);
-                mbar_arrive(&sm.p_ready[1][t]);
-                float sum_lo, sum_hi;
-                unpack2(sum2, sum_lo, sum_hi);
-                l = l * alpha + (sum_lo + sum_hi);
-            } else {
-                float sv[4][32];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) tc_ld32(s_addr + c * 32, sv[c]);
-                tc_wait_ld();
-                if (kMask && pad) {   // padded keys first: the bits are dead after this
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        if (!((kb0 >> i) & 1u)) sv[0][i] = -INFINITY;
-                        if (!((kb1 >> i) & 1u)) sv[1][i] = -INFINITY;
-                        if (!((kb2 >> i) & 1u)) sv[2][i] = -INFINITY;
-                        if (!((kb3 >> i) & 1u)) sv[3][i] = -INFINITY;
-                    }
-                }
-                if (need_mask) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (c * 32 + i > limit) sv[c][i] = -INFINITY;
-                }
-                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], sv[c][i], sv[c][i + 1]);
-                float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-                mx *= a.scale_log2;   // scale > 0 is guaranteed by the dispatcher
-                FA_TRACE_EVENT(t, j, 1);
-
-                float alpha = 1.0f;
-                bool changed = false;
-                if (mx > m + kRescaleThreshold) {   // also true for the first finite max (m == -inf)
-                    alpha = ex2(m - mx);            // 0 when m == -inf
-                    m = mx;
-                    changed = true;
-                }
-                if (j > 0 && __any_sync(0xffffffffu, changed)) {
-                    // rescale this warp's 32 rows of O in tensor memory (rows that did not move use 1.0)
-#pragma unroll 1
-                    for (int c = 0; c < D / 32; ++c) {
-                        float ov[32];
-                        tc_ld32(o_addr + c * 32, ov);
-                        tc_wait_ld();
-                        unsigned ou[32];
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) ou[i] = __float_as_uint(ov[i] * alpha);
-                        tc_st32(o_addr + c * 32, ou);
-                    }
-                }
-                const float m_use = (m == -INFINITY) ? 0.0f : m;
-                // exp2(s * scale - m) two columns at a time: packed FMA for the argument and the row sum;
-                // one pair in four takes its exponential on the FMA pipe (unmasked tiles only), which
-                // relieves the special-function unit the two warpgroups compete for.
-                const unsigned long long scale2 = pack2(a.scale_log2, a.scale_log2);
-                const unsigned long long neg_m2 = pack2(-m_use, -m_use);
-                unsigned long long sum2 = pack2(0.0f, 0.0f);
-                // two straight-line copies (masked tiles keep every exponential on the special-function
-                // unit, where -inf gives an exact zero) rather than a branch inside the unrolled loop
-                auto exp_phase = [&](auto fma_pipe_share) {
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        unsigned pu[32];
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const int cc = c * 2 + (i >> 4);
-                            const int ii = (i & 15) * 2;
-                            float x0, x1, p0, p1;
-                            unpack2(fma2(pack2(sv[cc][ii], sv[cc][ii + 1]), scale2, neg_m2), x0, x1);
-                            if (decltype(fma_pipe_share)::value && fma_pipe_exp(i)) {
-                                ex2_fma2(x0, x1, p0, p1);
-                            } else {
-                                p0 = ex2(x0);
-                                p1 = ex2(x1);
-                            }
-                            sum2 = add2(sum2, pack2(p0, p1));
-                            pu[i] = pack16<T>(p0, p1);
-                        }
-                        tc_st32(s_addr + c * 32, pu);
-                        tc_wait_st();
-                        tc_fence_before();
-                        mbar_arrive(&sm.p_ready[c][t]);
-                        if (c == 0) FA_TRACE_EVENT(t, j, 2);
-                    }
-                };
-                if (need_mask || (kMask && pad)) exp_phase(std::false_type{});
-                else exp_phase(std::true_type{});
-                float sum_lo, sum_hi;
-                unpack2(sum2, sum_lo, sum_hi);
-                const float sum = sum_lo + sum_hi;
-                l = l * alpha + sum;
+                mbar_arrive(&sm.p_ready[h][t]);
+                if (h == 0) FA_TRACE_EVENT(t, j, 2);
             }
+            float sum_lo, sum_hi;
+            unpack2(sum2, sum_lo, sum_hi);
+            l = l * alpha + (sum_lo + sum_hi);
             FA_TRACE_EVENT(t, j, 3);
         }
 

@@ -191,3 +191,28 @@ def test_key_padding_mask_on_the_tensor_core_kernel(kind, shape):
     H.assert_bf16_close(got, want, f"padding mask {kind} {shape}")
     if kind == "one_row_all_masked":
         assert np.all(got[0] == 0.0)
+
+
+@pytest.mark.parametrize("padded", [False, True])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("s", [128, 200, 300])
+def test_masked_keys_weigh_exactly_nothing(s, d, padded):
+    # the largest finite V behind a row's keys must not reach it, whichever unit computes the exponential: with any weight above zero, 2^-126 even,
+    # it would show; both calls then give the same bits
+    b, hq, hkv, cut = 2, 4, 2, s - 40
+    q, k = (H.to_dev(H.round_to(H.normal((b, s, h, d), i), "bf16"), "bf16") for i, h in ((1, hq), (2, hkv)))
+    v = H.to_dev(H.round_to(H.normal((b, s, hkv, d), 3), "bf16"), "bf16")
+    mask = torch.ones(b, s, dtype=torch.uint8, device="cuda")
+    if padded:
+        mask[1, cut:] = 0
+        mask[0, :7] = 0
+    outs = []
+    for huge in (0.0, torch.finfo(torch.bfloat16).max):
+        vv = v.clone()
+        vv[:, cut:] = huge
+        o = torch.empty_like(q)
+        low.flash_attn(q, k, vv, o, b, s, s, hq, hkv, d, 0, 1.0 / d**0.5, mask if padded else None)
+        outs.append(o[:, :cut].clone())
+    assert ffi.last_path() == "prefill_tcgen05"
+    assert torch.isfinite(outs[0]).all()
+    assert torch.equal(outs[0], outs[1])
