@@ -816,7 +816,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     const bool packed = a.mode == MODE_VARLEN;
     const long long tot_q = packed ? (long long)a.cu_q[a.batch] : 0;
     const long long tot_k = (packed && !a.paged) ? (long long)a.cu_k[a.batch] : 0;
-    auto q_edge = [&](const TileInfo& ti) { return packed && ti.valid && (long long)sq.q_crow + ti.row0 + kBlockM > tot_q; };
+    // (a tile that sees no key needs no Q: the issuer leaves it out, and its softmax warps lay zeros down in Q's shared memory without waiting for anybody)
+    auto q_edge = [&](const TileInfo& ti) { return packed && ti.n_kv > 0 && (long long)sq.q_crow + ti.row0 + kBlockM > tot_q; };
     auto kv_edge = [&](int j) { return packed && !a.paged && (long long)sq.kv_crow + (long long)(j + 1) * kBlockN > tot_k; };
     if (warp == kLoadWarp) asm volatile("barrier.cta.arrive 1, 64;\n" ::: "memory");
     if (warp == kLoadWarp && (kPaged || lane == 0)) {
@@ -824,7 +825,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 #pragma unroll
         for (int j = 0; j < kStages; ++j) pages[j] = kPaged && j < n_pre ? page_of_lane(a, sq.kv_len, b, j, lane) : -1;
         auto load_q = [&](const TileInfo& ti, int t) {
-            if ((kPaged && lane != 0) || !ti.valid || q_edge(ti)) return;
+            if ((kPaged && lane != 0) || ti.n_kv <= 0 || q_edge(ti)) return;
             mbar_expect_tx(&sm.q_full[t], TileBytes<D>::value);
             tma_load_4d(sm.q[t], &q_map, &sm.q_full[t], 0, ti.head, sq.q_crow + ti.row0, sq.q_cb);
             if (D == 128) tma_load_4d(sm.q[t] + kHalfBytes, &q_map, &sm.q_full[t], 64, ti.head, sq.q_crow + ti.row0, sq.q_cb);
@@ -948,8 +949,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             // abort flag: they only depend on the copy engine.
             if (lane == 0) {
                 if (!is_v) {
-                    if (t0.valid) mbar_wait(sm, &sm.q_full[0], 0, a, 3);
-                    if (t1.valid) mbar_wait(sm, &sm.q_full[1], 0, a, 3);
+                    if (t0.n_kv > 0) mbar_wait(sm, &sm.q_full[0], 0, a, 3);
+                    if (t1.n_kv > 0) mbar_wait(sm, &sm.q_full[1], 0, a, 3);
                 }
                 const unsigned long long t_begin = global_timer_ns();
                 // (K: where the loop went one past the last tile, the tile before the last has been read, and its barrier used again)
