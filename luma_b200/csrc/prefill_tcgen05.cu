@@ -293,9 +293,15 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
-__device__ __forceinline__ float max3(float a, float b, float c) {
+// Maxima that are NaN where an operand is.
+__device__ __forceinline__ float max_nan(float a, float b) {
     float d;
-    asm("max.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    asm("max.NaN.f32 %0, %1, %2;\n" : "=f"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+    float d;
+    asm("max.NaN.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
 // Two f32 lanes in one 64-bit register for the packed FMA-pipe instructions of sm_100.
@@ -323,12 +329,8 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
 // f32 evaluation. 1.9e-7 at most, 2.2e-8 low on average, against ex2.approx's measured 1.4e-7 and 4.6e-8. A quartic (2.7e-6) showed in the f32 sums of the
 // rows' first tile: error of LSE over 128 tokens with scores N(0,1) at most 9.9e-7, rms 2.4e-7, instead of 7.9e-7 and 2.2e-7 (8 x 128 x 8 rows,
 // bf16, against 64 bits), and 7e-7 where one key takes all of a row's weight. x is clamped at -200, where that addition gives a negative integer, and those become zeros: 2^x for x
-// below -126.5, -inf (a masked score) among them, is an exact zero or below 2^-126. A NaN is not clamped and gives no finite result.
-__device__ __forceinline__ float max_nan(float a, float b) {
-    float d;
-    asm("max.NaN.f32 %0, %1, %2;\n" : "=f"(d) : "f"(a), "f"(b));
-    return d;
-}
+// below -126.5, -inf (a masked score) among them, is an exact zero or below 2^-126. A NaN becomes the largest finite number (the addition takes one from
+// its exponent): infinite in 16 bits, but not in the row's sum, so the caller looks for NaN and +inf among the scores itself (see the row maximum).
 __device__ __forceinline__ void ex2_fma2(float x0, float x1, float& p0, float& p1) {
     const unsigned long long x2 = pack2(max_nan(x0, -200.0f), max_nan(x1, -200.0f));
     const unsigned long long t2 = add2(x2, pack2(12582912.0f, 12582912.0f));   // 1.5 * 2^23
@@ -1035,14 +1037,16 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 #pragma unroll
             for (int c = 0; c < 4; ++c)
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], sv[c][i], sv[c][i + 1]);
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * a.scale_log2;   // scale > 0 is guaranteed by the dispatcher
+                for (int i = 0; i < 32; i += 2) mx4[(i >> 1) & 3] = max3_nan(mx4[(i >> 1) & 3], sv[c][i], sv[c][i + 1]);
+            // A row that sees a NaN outputs NaN whichever unit takes that key's exponential: its maximum is NaN, and with it the reference below, every
+            // exponential of the tile and the row's sum from here on. A +inf stays the reference to the end, where the epilogue sees it.
+            const float mx = max_nan(max3_nan(mx4[0], mx4[1], mx4[2]), mx4[3]) * a.scale_log2;   // scale > 0 is guaranteed by the dispatcher
             FA_TRACE_EVENT(t, j, 1);
 
             float alpha = 1.0f;
             bool changed = false;
-            if (mx > m + kRescaleThreshold) {   // also true for the first finite max (m == -inf)
-                alpha = ex2(m - mx);            // 0 when m == -inf
+            if (!(mx <= m + kRescaleThreshold)) {   // also for the first finite max (m == -inf) and where either is NaN
+                alpha = ex2(m - mx);                // 0 when m == -inf
                 m = mx;
                 changed = true;
             }
@@ -1103,7 +1107,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             // with a padding mask a query row at a padded (or out-of-range) position outputs zeros (flash_attn_func.cu:77-84)
             bool q_ok = true;
             if (kMask) q_ok = row_ok && pos >= 0 && pos < (long long)sq.kv_len && a.mask[(long long)b * a.kv_seq_len + pos] != 0;
-            const float inv = (l > 0.0f && q_ok) ? 1.0f / l : 0.0f;
+            const bool seen = l > 0.0f && m < INFINITY && q_ok;   // (false where a score was NaN, l NaN, or +inf, m +inf: 0 times that row's NaN or infinity is NaN)
+            const float inv = seen ? 1.0f / l : 0.0f;
             // a bulk store writes every row of its box that lies inside the tensor: in a packed buffer the
             // rows after this sequence belong to the next one, so a tile that overhangs the end of its
             // sequence takes the row-guarded path
@@ -1206,7 +1211,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 }
             }
             if (row_ok && (a.lse != nullptr || a.n_lse > 0)) {
-                const float lse_val = (l > 0.0f && q_ok) ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
+                const float lse_val = seen ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
                 if (a.lse != nullptr) a.lse[((long long)b * a.q_heads + ti.head) * a.q_seq_len + row] = lse_val;
                 // head-sharded call: the same value into the (batch, o_heads, q_seq_len) LSE of every GPU of the group
                 const long long g_off = ((long long)b * a.o_heads + a.o_head0 + ti.head) * a.q_seq_len + row;
