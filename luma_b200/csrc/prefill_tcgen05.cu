@@ -171,6 +171,11 @@ __device__ __forceinline__ bool mbar_try_wait_at(unsigned bar, unsigned parity) 
     return ok != 0;
 }
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) { return mbar_try_wait_at(smem_u32(bar), parity); }
+__device__ __forceinline__ bool shared_flag(unsigned addr) {
+    int f;
+    asm volatile("ld.volatile.shared.s32 %0, [%1];\n" : "=r"(f) : "r"(addr) : "memory");
+    return f != 0;
+}
 __device__ __forceinline__ void set_shared_flag(unsigned addr) { asm volatile("st.volatile.shared.s32 [%0], 1;\n" ::"r"(addr) : "memory"); }
 __device__ __forceinline__ unsigned long long global_timer_ns() {
     unsigned long long t;
@@ -612,11 +617,8 @@ __device__ __forceinline__ void edge_tile_copy(unsigned char* dst, const void* b
     if (lane == 0) mbar_arrive(bar);
 }
 
-__device__ __forceinline__ unsigned clock_lo() {
-    unsigned t;
-    asm volatile("mov.u32 %0, %%clock;\n" : "=r"(t));
-    return t;
-}
+// The SM clock in units of 1024: 32 bits hold 36 minutes at 2 GHz, more than the longest bound of a wait.
+__device__ __forceinline__ unsigned clock_1024() { return (unsigned)(clock64() >> 10); }
 
 // The MMA issuer, run by one whole warp (converged). Its loop is written for few instructions: about 400 a step where it had 780 (12.5 KiB).
 // What a scheduler executes in a loop comes at full rate up to 8 KiB, beyond that at an instruction in 3 clocks, beyond 32 KiB in 6 (a
@@ -644,15 +646,14 @@ __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int
     const unsigned long long dk = make_desc(sm_addr + (unsigned)offsetof(Storage, k), 16, 1024);
     const unsigned long long dv = make_desc(sm_addr + (unsigned)offsetof(Storage, v), kHalfBytes, 1024);
     constexpr unsigned kTileStep = TileBytes<D>::value >> 4;   // from one tile's descriptor to the next one's
-    // the bound in SM clocks, as in mbar_wait, in the 32 bits of the clock's lower half (which wraps after 2.1 s at the least)
-    unsigned patience = (unsigned)(wait_ns < 2000000000ULL ? wait_ns * 2ULL : 4000000000ULL);
-    int expired = 0;   // code of a wait that ran out
+    unsigned patience = (unsigned)(wait_ns >> 9) + 1u;   // the bound as in mbar_wait, in units of 1024 SM clocks
+    int expired = 0;   // code of the wait that was the first to be given up; none has any patience from then on
     auto wait = [&](size_t bar, unsigned parity, int where) {
-        const unsigned t0 = clock_lo();
+        const unsigned t0 = clock_1024();
 #pragma unroll 1
         while (!__any_sync(0xffffffffu, mbar_try_wait_at(sm_addr + (unsigned)bar, parity))) {
-            if (__any_sync(0xffffffffu, clock_lo() - t0 >= patience)) {
-                expired = where;
+            if (__any_sync(0xffffffffu, clock_1024() - t0 >= patience || shared_flag(sm_addr + (unsigned)offsetof(Storage, abort_flag)))) {
+                if (expired == 0) expired = where;
                 patience = 0;
                 break;
             }
@@ -725,9 +726,11 @@ __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int
         }
         commit(offsetof(Storage, step_done) + 8 * (s ^ 1));
         if (expired != 0) {
-            set_shared_flag(sm_addr + (unsigned)offsetof(Storage, abort_flag));
-            *reinterpret_cast<volatile int*>(status) = expired;
-            __threadfence_system();
+            if (!shared_flag(sm_addr + (unsigned)offsetof(Storage, abort_flag))) {   // (else another warp of the CTA gave up and reported it)
+                set_shared_flag(sm_addr + (unsigned)offsetof(Storage, abort_flag));
+                *reinterpret_cast<volatile int*>(status) = expired;
+                __threadfence_system();
+            }
             break;
         }
     }

@@ -10,6 +10,7 @@ The expiry is provoked the permitted way: the limit is shortened to about a mill
 hook makes the K producer leave out one tile, so that the issuer's wait for it runs out and the
 kernel returns. Nothing traps, faults or spins without bound."""
 import math
+import re
 
 import numpy as np
 import pytest
@@ -74,12 +75,37 @@ def test_expiry_at_every_part_of_the_key_loop(tile, d):
         ffi.set_option("prefill_test_skip_k", 0)
         ffi.set_option("prefill_wait_us", 0)
     torch.cuda.synchronize()
-    with pytest.raises(E.CudaError):
+    with pytest.raises(E.CudaError) as exc:
         low.flash_attn(*args)
+    # the issuer's wait for the tile (K tile 0: 11, a step's tiles: 13), or one that waits on what follows from it (the next scores: 20, 21; a
+    # free stage: 1, 2); never one that the issuer came to after it had given up (P: 14 to 17)
+    assert int(re.search(r"code (-?\d+)", str(exc.value)).group(1)) in ({11, 20, 21, 1, 2} if tile == 0 else {13, 20, 21, 1, 2})
     low.flash_attn(*args)
     torch.cuda.synchronize()
     assert ffi.device_status() == 0
     H.assert_bf16_close(H.to_np(o), ob.attn_f64_batch(q, k, v), "call after the reported expiry")
+
+
+def test_a_bound_above_two_seconds_is_kept():
+    # the bound is counted in clocks, two to the nanosecond, so that it is no shorter than asked for at any SM clock up to 2 GHz
+    b, s, h, d = 1, 256, 1, 128
+    q = H.to_dev(H.normal((b, s, h, d), 1), "bf16")
+    o = torch.empty_like(q)
+    args = (q, q, q, o, b, s, s, h, h, d, 0, 1.0 / math.sqrt(d))
+    torch.cuda.synchronize()
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    try:
+        ffi.set_option("prefill_wait_us", 2300000)
+        ffi.set_option("prefill_test_skip_k", 1)
+        begin.record()
+        low.flash_attn(*args)
+        end.record()
+    finally:
+        ffi.set_option("prefill_test_skip_k", 0)
+        ffi.set_option("prefill_wait_us", 0)
+    torch.cuda.synchronize()
+    assert ffi.device_status() != 0                  # (read and cleared)
+    assert begin.elapsed_time(end) >= 2300
 
 
 def test_workspaces_are_bounded_and_releasable():
