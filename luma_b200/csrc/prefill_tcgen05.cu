@@ -47,10 +47,11 @@ namespace {
 constexpr int kBlockM = 128;   // query rows per tile
 constexpr int kBlockN = 128;   // keys per K/V tile
 // head size D (64 or 128) is a template parameter of the kernel
-constexpr int kStages = 2;     // K ring depth
-// The rings are two tiles deep. A third V stage fits the shared memory and measured 5 % slower on every prefill workload (1165
+constexpr int kStages = 2;     // depth of the K and V rings
+static_assert(kStages == 2, "step_full and step_done have an entry per stage, found by the parity of the step (j & 1, phase j >> 1) throughout the kernel");
+// A third V stage fits the shared memory and measured 5 % slower on every prefill workload (1165
 // against 1228 TFLOP/s at S = 8192); the issuer does not wait for the copies.
-constexpr int kThreads = 384;   // three warpgroups: softmax 0, softmax 1, and producer + issuer (+ two idle warps)
+constexpr int kThreads = 384;   // three warpgroups: softmax 0, softmax 1, and producers + issuer (+ an idle warp)
 constexpr int kLoadWarp = 8;
 constexpr int kMmaWarp = 9;
 constexpr int kLoadWarpV = 10;   // V-ring producer (K ring and Q: kLoadWarp)
@@ -279,14 +280,6 @@ __device__ __forceinline__ void tc_st32(unsigned taddr, const unsigned (&u)[32])
         "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15]), "r"(u[16]), "r"(u[17]), "r"(u[18]),
         "r"(u[19]), "r"(u[20]), "r"(u[21]), "r"(u[22]), "r"(u[23]), "r"(u[24]), "r"(u[25]), "r"(u[26]), "r"(u[27]),
         "r"(u[28]), "r"(u[29]), "r"(u[30]), "r"(u[31])
-        : "memory");
-}
-// 32 lanes x 16 consecutive 32-bit columns
-__device__ __forceinline__ void tc_st16(unsigned taddr, const unsigned (&u)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr),
-        "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]), "r"(u[9]),
-        "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15])
         : "memory");
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }

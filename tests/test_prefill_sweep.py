@@ -1,6 +1,6 @@
 """Seeded sweep of the tcgen05 prefill kernel against the f64 oracle over shapes drawn at random:
 batch, GQA widths, ragged and tile-aligned lengths, start positions that are and are not multiples
-of the tile (aligned diagonal tiles take a specialised softmax step), kv longer than needed, head
+of the tile (the diagonal cuts one tile of a row block or two), kv longer than needed, head
 sizes 64 and 128, bf16 and f16 — a guard against shape-dependent slips in the tile, band and mask arithmetic."""
 import numpy as np
 import pytest
