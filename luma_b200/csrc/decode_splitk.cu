@@ -984,7 +984,9 @@ int launch_decode_splitk(const AttnParams& p, cudaStream_t stream) {
 }
 
 // ---- this kernel or the prefill kernel, for calls that both take: the time of each, in microseconds, from what the host knows.
-// Prefill kernel: a CTA per pair of 128-row tiles, one per SM; a CTA walks its K/V range at 1.5 us per 128 keys after 6.6 us of set-up.
+// Prefill kernel: a CTA per pair of 128-row tiles, one per SM; a CTA walks its K/V range at 1.5 us per 128 keys after 6.6 us of set-up. (Measured again
+// since that kernel's issuer, set-up and softmax step got shorter, calls of one wave: 27-31 us at 2048 keys, 41-55 at 4096, 95-109 at 8192, where this says
+// 31, 55 and 103.)
 static long long longest_keys(const AttnParams& p) { return p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len; }
 static long long tile_pairs(const AttnParams& p, long long q_len) { return ((long long)(p.q_heads / p.kv_heads) * ((q_len + 127) / 128) + 1) / 2 * p.kv_heads; }
 static double prefill_us(const AttnParams& p, double pairs, double setup = 6.6) {
@@ -1005,7 +1007,9 @@ static double rows_us(const AttnParams& p, long long seqs, long long rows) {
 // else the estimates decide. Both kernels over the 235 of 298 shapes that get this far (1-64 sequences x 1-64 tokens, 64-8192 keys, groups of 1, 4
 // and 8): the choice is at most 5 % slower than the prefill kernel and at most 9 % slower than this one. 64 rows:
 // 64 x 64 tokens x 1600 keys, 32 heads without GQA 275 us on the prefill kernel, 743 here; 1 x 16 x 8192, 32/8 heads 110 and 31. 16 rows: 16 x 4 x
-// 8192, 32/8: 180 and 63.
+// 8192, 32/8: 180 and 63. With the prefill kernel as it is now, 135 calls drawn anew: the 102 that get this far at most 0.1 % slower than it and
+// 2.5 % slower than this one; of the 33 that it keeps for their short K/V the slowest takes 27 us where this kernel would take 11 (4 x 1 token over 256-1024, 64/8
+// heads).
 int launch_few_rows(const AttnParams& p, bool prefill_takes_it, cudaStream_t stream) {
     if (p.n_out > 0 || !rows_kernel_takes(p)) return -1;
     const long long rows = (long long)p.q_seq_len * (p.q_heads / p.kv_heads);
@@ -1036,7 +1040,8 @@ PackedMix packed_mix(const AttnParams& p) {
 // starts when that kernel's last CTA has. Over 238 paged mixes (1-6 prompts, chunks of 64 or 512, 0-128 single tokens, contexts of
 // 64-8192, four head layouts) no mix is then slower than with everything in the prefill grid, and the choice is 2 % off the better one on average:
 // 4 x 512 with 32 tokens over 512-8192, 32/8 heads: 435 us in one grid, 231 so; with 1 token: 131 in one grid, 152 with two kernels, which
-// one grid keeps. Without the row count of the packed buffers (the C ABI's plain entry point) nothing is known of the mix, and
+// one grid keeps. With the prefill kernel as it is now, 102 mixes drawn anew: two are more than 1.2 % slower than one grid (5.5 %: 53 us for 50; 2.7 %), two more than
+// 5 % slower than with two kernels always (29 us for 23, 24.3 for 22.8, both 512 keys at most). Without the row count of the packed buffers (the C ABI's plain entry point) nothing is known of the mix, and
 // long contexts go to two kernels.
 static bool mixed_few_rows_are_better(const AttnParams& p) {
     if (p.total_q <= 0) return longest_keys(p) > 12 * 128 || tile_pairs(p, p.q_seq_len) * p.num_seqs > sm_count();

@@ -61,7 +61,8 @@ constexpr float kRescaleThreshold = 8.0f;            // log2 units
 
 // Which element pairs take their exponential on the FMA pipe (a quintic) instead of the special-function unit: one in eight. It costs issue slots
 // and registers that the special-function unit's time does not buy back at a larger share where CTAs are short. us a pass for a share of 1/16, 1/8,
-// 1/6, 1/4: 2 x 8192 GQA 961, 947, 945, 954; 4 x 2048 MHA 163.4, 161.3, 162.2, 163.1; 4 chunks of 512 155.8, 155.0, 156.3, 158.5.
+// 1/6, 1/4: 2 x 8192 GQA 932, 903, 895, 881; 4 x 2048 MHA 155.0, 151.6, 148.9, 148.1; 24 packed prompts at head size 64 337, 335, 329, 332; 4 chunks of 512
+// 145.1, 142.5, 143.8, 144.7; chunks with 32 decoding sequences 225.9, 225.0, 226.8, 230.4; 7 packed prompts of 7-125 tokens 27.4, 27.0, 27.3, 28.1.
 __device__ __forceinline__ constexpr bool fma_pipe_exp(int i) { return (i & 7) == 7; }
 
 template <int D>
@@ -89,8 +90,8 @@ constexpr int kCtaLogEntries = 2048;
 constexpr unsigned long long kWaitLimitNs = 2000000000ULL;   // default bound of every mbarrier wait
 
 // Division of n < 2^31 by a divisor the host knows, as a product with its rounded-up inverse (Granlund and Montgomery, "Division by
-// invariant integers using multiplication"): three instructions. The compiler's division is some forty dependent ones, and a CTA made ten before its
-// first copy was requested: 1700 clocks from its start, on every SM with nothing else to do.
+// invariant integers using multiplication"): a product, a sum and a shift. With the division operator, a CTA made ten divisions by run-time values one after
+// the other before its first copy was requested, and knew its extents 1700 clocks from its start (timeline), on an SM with nothing else to do.
 struct FastDiv {
     unsigned mul, shift;
     int d;
@@ -239,8 +240,8 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 
 // The products as the issuer warp runs them: the whole warp executes the instruction stream
 // converged and one elected lane issues. Keeping the warp uniform lets the descriptors live in
-// uniform registers: a product is 5 instructions inside an elected branch, 7 with an election of its own and 12 to 14 where the compiler
-// cannot see that its operands are the same for the whole warp.
+// uniform registers; an election for each group of products instead of each product, and operands that the compiler can see to be the same for the
+// whole warp, take moves between the register files out (times at issue_products).
 __device__ __forceinline__ bool elect_one() {
     unsigned e;
     asm volatile("{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\nselp.u32 %0, 1, 0, e;\n}\n" : "=r"(e));
@@ -613,14 +614,13 @@ __device__ __forceinline__ void edge_tile_copy(unsigned char* dst, const void* b
 // The SM clock in units of 1024: 32 bits hold 36 minutes at 2 GHz, more than the longest bound of a wait.
 __device__ __forceinline__ unsigned clock_1024() { return (unsigned)(clock64() >> 10); }
 
-// The MMA issuer, run by one whole warp (converged). Its loop is written for few instructions: about 400 a step where it had 780 (12.5 KiB).
-// What a scheduler executes in a loop comes at full rate up to 8 KiB, beyond that at an instruction in 3 clocks, beyond 32 KiB in 6 (a
-// straight-line loop of multiply-adds); the softmax warps' 10 KiB pass between two steps of the issuer, so that it is fetched anew every time.
-// The tensor pipe stood still meanwhile: 300 clocks from the issuer's last commit of a step to its first look at the next barrier, 150 for
+// The MMA issuer, run by one whole warp (converged). Its loop is written for few instructions. What a scheduler executes in a loop comes at full rate
+// up to 512 instructions (8 KiB), beyond that at one in 3 clocks, beyond 2048 in 6 (`clock64` around loops of that many independent multiply-adds); the
+// softmax warps' unrolled steps pass between two steps of the issuer, which finds its own anew every time. The tensor pipe stood still meanwhile: 300 clocks from the issuer's last commit of a step to its first look at the next barrier, 150 for
 // a look at one that had long completed (45 alone), with or without the copies. Step of 128 keys at S = 8192 GQA 3100 -> 2840 clocks,
 // 884 -> 833 us; 4 x 2048 MHA 157.5 -> 147.8 us; head size 64, 2 x 8192 GQA 755 -> 699 us.
 //   * a function of its own, so that the compiler sees what is the same for the whole warp (everything is, or is broadcast here): inside
-//     the kernel, whose early returns and per-sequence loads it takes for divergent, a product was 11 instructions, here it is 6;
+//     the kernel it takes them for divergent, for the early returns and per-sequence loads before them;
 //   * a wait that runs out is looked after at the end of its step, which goes on without waiting on what happens to be in shared memory and
 //     reports nothing as done. Leaving at each wait doubled the code after it.
 // n0, n1: K/V tiles that query tile 0 and 1 need (0: none, or no such tile).
@@ -998,8 +998,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             const int limit = need_mask ? (int)max(-1LL, min(limit_ll, (long long)kBlockN)) : kBlockN;
 
             // Masked scores become -inf, whose P is an exact zero from either exponential, so a masked tile runs the code of the others. (A form of its own
-            // for the aligned diagonal, which left out the chunks of 32 keys that a warp does not see, and one for other masked tiles were 17 KiB of
-            // straight-line code run once per tile: 2 x 8192 GQA 967 us with them, 948 without. Leaving unseen chunks out behind a branch in this
+            // for the aligned diagonal, which left out the chunks of 32 keys that a warp does not see, and one for other masked tiles were straight-line
+            // code run once per tile: 2 x 8192 GQA 967 us with them, 948 without. Leaving unseen chunks out behind a branch in this
             // code: 990 us, for what the compiler no longer interleaves.)
             // Key-padding mask (batched entry point): the tile's validity bytes become a ballot per chunk of 32; a tile whose real keys are all
             // valid (the usual case, padding sits at one end) runs as if there were no mask.
@@ -1497,9 +1497,9 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     a.skip_rows = few.max_rows;
     // Ordered: chunks of prompts, at most half as long as the context may be. Whole prompts keep grid order, which is heaviest
     // first for them already. Finding its pair costs a CTA 1 to 2 us; what it wins is one late long pair, about a fifth of the longest pair's
-    // 1.7 us per K/V tile, and nothing where all pairs start at once. So: more than one wave of pairs, and at least five tiles in the longest for
-    // each. 4 chunks of 300 over 2048-8192 keys, 32/8 heads (1.3 waves) 148 us in grid order, 116 ordered; 16 chunks of 300 over 512-2048,
-    // 32/32 heads (7 waves) 159 and 170; 4 chunks of 64 over 128-512 (less than a wave) 14.7 and 16.2.
+    // 1.5 to 1.7 us per K/V tile, and nothing where all pairs start at once. So: more than one wave of pairs, and at least five tiles in the longest for
+    // each. 4 chunks of 300 over 2048-8192 keys (the longest last), 32/8 heads (1.3 waves) 138-152 us in grid order, 110 ordered; 16 chunks of 300 over
+    // 512-2048, 32/32 heads (7 waves) 161-172 and 166-186; 4 chunks of 64 over 128-512 (less than a wave) 17-19 and 19-21.
     const long long kv_rows = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
     const PackedMix mix = packed_mix(p);
     const double waves = (double)(mix.prompts * pairs + (a.skip_rows > 0 ? 0 : mix.few * ((group + 1) / 2))) * p.kv_heads / sm_count();
@@ -1508,7 +1508,7 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     if (p.total_q > 0)   // a sequence of n rows has (group * ceil(n / 128) + 1) / 2 pairs
         ctas = std::min(ctas, p.kv_heads * ((group * (((long long)p.total_q + 127LL * p.num_seqs) / 128) + p.num_seqs) / 2));
     // ... and where most of the grid would be empty CTAs of sequences that are left to the few-row kernel: a launch in order has no more than
-    // the rows can make (one chunk of 512 with 128 tokens over 128-2048, 32/8 heads: 8256 CTAs or 2644, 200 us or 173).
+    // the rows can make (one chunk of 512 with 128 tokens over 128-2048, 32/8 heads: 8256 CTAs or 2644, 191 us or 153).
     const bool worth_ordering = (waves > 1.0 && (double)((kv_rows + kBlockN - 1) / kBlockN) > 5.0 * waves) || (a.skip_rows > 0 && all > 2 * ctas);
     if (kPaged && p.num_seqs >= 2 && p.num_seqs <= kOrderMax && 2LL * p.q_seq_len <= kv_rows && get_option_prefill_band() <= 0 &&
         get_option_prefill_groups() <= 0 && (worth_ordering || get_option_prefill_order() == 2)) {
