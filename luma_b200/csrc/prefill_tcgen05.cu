@@ -146,6 +146,7 @@ struct PrefillArgs {
     const int* context_lens;    // MODE_KVCACHE: cached length per sequence, query tokens included
     const int* block_tables;    // paged K/V: (batch, max_blocks) logical -> physical block
     int paged, block_size, max_blocks;
+    int q_bounded, kv_bounded;  // MODE_VARLEN: the caller gave the packed buffers' rows, their tensor maps end there
     int skip_rows;              // MODE_VARLEN: sequences of at most this many (query token, group head) rows are not this launch's; 0: none
     float scale_log2;
 };
@@ -592,6 +593,9 @@ __device__ __forceinline__ void load_kv_tile(const PrefillArgs& a, const SeqExte
 // rows that may not exist. Rows past the end are written as zeros (what an out-of-range bulk copy
 // delivers). Same shared-memory image as the bulk copies: 64-column halves, 128 B per row, 16-byte
 // chunks XOR-swizzled by the row. The barrier's phase is completed by one plain arrival.
+// All of a lane's copies are in flight together (cp.async): one trip to memory for a tile. As loads into registers, four at a time, a
+// tile was 16 trips one after the other, and a CTA at the end of the buffers waited for two Q tiles, K and V so: 4 prompts of 38-155 tokens, 32/8 heads, through the
+// plain entry point 27 us, 23 so; 4 of 235-941, 8/2 heads, 39 and 31. (With the row counts given nothing comes this way, see q_open: 36 and 12 us, 38 and 22.)
 template <int D>
 __device__ __forceinline__ void edge_tile_copy(unsigned char* dst, const void* base, int heads, int head, long long row_start,
                                                long long total_rows, unsigned long long* bar, int lane, int d_real) {
@@ -599,13 +603,17 @@ __device__ __forceinline__ void edge_tile_copy(unsigned char* dst, const void* b
     const long long left = total_rows - row_start;
     const int nrows = left < 0 ? 0 : (left > kBlockN ? kBlockN : (int)left);
     const unsigned char* src = static_cast<const unsigned char*>(base);
+    const unsigned to = smem_u32(dst);
 #pragma unroll 4
     for (int idx = lane; idx < kBlockN * kChunksPerRow; idx += 32) {
         const int r = idx / kChunksPerRow, cc = idx % kChunksPerRow;
-        uint4 w = make_uint4(0u, 0u, 0u, 0u);
-        if (r < nrows && cc * 8 < d_real) w = *reinterpret_cast<const uint4*>(src + ((row_start + r) * heads + head) * (long long)(d_real * 2) + cc * 16);
-        *reinterpret_cast<uint4*>(dst + (cc >> 3) * kHalfBytes + r * 128 + (((cc & 7) ^ (r & 7)) << 4)) = w;
+        const bool real = r < nrows && cc * 8 < d_real;
+        const unsigned char* from = real ? src + ((row_start + r) * heads + head) * (long long)(d_real * 2) + cc * 16 : src;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to + (cc >> 3) * kHalfBytes + r * 128 + (((cc & 7) ^ (r & 7)) << 4)), "l"(from),
+                     "r"(real ? 16 : 0)   // 0: nothing is read, zeros are written
+                     : "memory");
     }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // generic-proxy writes -> tensor-core reads
     __syncwarp();
     if (lane == 0) mbar_arrive(bar);
@@ -813,14 +821,15 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     // The first copies are requested before the CTA-wide set-up barrier, by the two producer warps (Q and the K tiles that fill the empty ring; the
     // V tiles likewise): they fly while tensor memory is being allocated and the other warps start up.
     const int n_pre = min(kStages, n_max);
-    // Packed buffers end at row cu_seqlens[num_seqs]; a tile that reaches past that row is not asked
-    // of the copy engine (see edge_tile_copy) but fetched by the producer warp after the set-up.
+    // Packed buffers end at row cu_seqlens[num_seqs]; where the tensor map does not end with the buffer, a tile that reaches past that row is not asked
+    // of the copy engine (see edge_tile_copy) but fetched by the producer warp after the set-up. A map that does gives zeros there like any other.
     const bool packed = a.mode == MODE_VARLEN;
-    const long long tot_q = packed ? (long long)a.cu_q[a.batch] : 0;
-    const long long tot_k = (packed && !a.paged) ? (long long)a.cu_k[a.batch] : 0;
+    const bool q_open = packed && !a.q_bounded, kv_open = packed && !a.paged && !a.kv_bounded;
+    const long long tot_q = q_open ? (long long)a.cu_q[a.batch] : 0;
+    const long long tot_k = kv_open ? (long long)a.cu_k[a.batch] : 0;
     // (a tile that sees no key needs no Q: the issuer leaves it out, and its softmax warps lay zeros down in Q's shared memory without waiting for anybody)
-    auto q_edge = [&](const TileInfo& ti) { return packed && ti.n_kv > 0 && (long long)sq.q_crow + ti.row0 + kBlockM > tot_q; };
-    auto kv_edge = [&](int j) { return packed && !a.paged && (long long)sq.kv_crow + (long long)(j + 1) * kBlockN > tot_k; };
+    auto q_edge = [&](const TileInfo& ti) { return q_open && ti.n_kv > 0 && (long long)sq.q_crow + ti.row0 + kBlockM > tot_q; };
+    auto kv_edge = [&](int j) { return kv_open && (long long)sq.kv_crow + (long long)(j + 1) * kBlockN > tot_k; };
     if (warp == kLoadWarp) asm volatile("barrier.cta.arrive 1, 64;\n" ::: "memory");
     if (warp == kLoadWarp && (kPaged || lane == 0)) {
         int pages[kStages];   // of the tiles requested here, looked up together
@@ -1421,6 +1430,8 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     a.paged = p.paged;
     a.block_size = p.block_size;
     a.max_blocks = p.max_blocks;
+    a.q_bounded = p.total_q > 0;
+    a.kv_bounded = p.total_k > 0;
     a.scale_log2 = p.scale * 1.4426950408889634f;
 
     const int group = p.q_heads / p.kv_heads;

@@ -172,3 +172,38 @@ def test_single_row_batched_entry_point_with_start_pos():
     torch.cuda.synchronize()
     assert ffi.last_path() == "prefill_tcgen05" and ffi.device_status() == 0
     H.assert_bf16_close(H.to_np(o), ob.attn_f64_batch(q, k, v, start_pos=skv - 1), "single row, batched")
+
+
+@pytest.mark.parametrize("d,page", [(128, 0), (64, 0), (32, 0), (128, 16)])
+@pytest.mark.parametrize("lens", [[1], [127, 1], [128, 129, 3], [60, 40, 27, 300]])
+def test_row_counts_end_the_tensor_maps(lens, d, page):
+    """With the buffers' row counts given, the tiles that reach past the last row come in by bulk copies that end there: the same bits as through the plain
+    entry point, whose last tiles come in row by row, with NaN behind both buffers and behind the rows that are counted but belong to no sequence."""
+    hq, hkv, spare = 4, 2, 5
+    cu = _cu(lens)
+    t = int(cu[-1])
+    cq = torch.from_numpy(cu).cuda()
+    table, kv_shape = None, (t, hkv, d)
+    if page:
+        need = [-(-n // page) for n in lens]
+        table = torch.full((len(lens), max(need)), -1, dtype=torch.int32)
+        for i, n in enumerate(need):
+            table[i, :n] = torch.arange(n, dtype=torch.int32) + sum(need[:i])
+        table, kv_shape = table.cuda(), (sum(need), page, hkv, d)
+
+    def fill(shape, seed):
+        buf = torch.full((shape[0] + 200, *shape[1:]), float("nan"), device="cuda", dtype=torch.bfloat16)
+        buf[:shape[0]] = H.to_dev(H.normal(shape, seed), "bf16")
+        return buf
+
+    q, k, v = fill((t, hq, d), 1), fill(kv_shape, 2), fill(kv_shape, 3)
+    got = []
+    for total in (None, t, t + spare):
+        o = torch.full((t + spare, hq, d), -7.0, device="cuda", dtype=torch.bfloat16)
+        low.flash_attn_varlen(q, k, v, o, cq, cq, len(lens), max(lens), max(lens), hq, hkv, d, 1.0 / np.sqrt(d), table, page or 1,
+                              total_q=total, total_k=None if page else total)
+        torch.cuda.synchronize()
+        assert ffi.last_path() == "prefill_tcgen05" and ffi.device_status() == 0
+        assert bool((o[t:] == -7.0).all()) and not bool(torch.isnan(o[:t]).any())
+        got.append(o[:t])
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
