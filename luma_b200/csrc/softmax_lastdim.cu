@@ -8,7 +8,11 @@
 // 32 elements per thread throughout (4 vectors of 16-bit storage, 8 of f32):
 //   rows of up to 1024 elements  : one warp per row (several short rows at a time), no shared memory
 //   rows of up to 32768 elements : one CTA of 64 .. 1024 threads per row, one shared-memory exchange
-//   longer or unaligned rows     : one CTA per row, two passes over the row (read twice)
+//   longer rows                  : one CTA per row, two passes over the row (read twice)
+// Where rows begin on no 16-byte boundary, the first and the last kind read as wide as every row's beginning allows, two elements or one (template
+// parameter V; a warp's loads still cover whole lines), the second kind in the aligned vectors that cover the row (RAGGED). Until then all such rows
+// went through the last kind in single elements. Before and now, us: 42983 rows of 162 bf16 223 and 14, 20000 of 1001 f32 152 and 28 (of 1000: 27), 60000 of 4099 bf16 789 and 189,
+// 8000 of 16383 bf16 340 and 105.
 #include "common.cuh"
 #include "../../include/luma_nn_kernels.h"
 
@@ -17,26 +21,87 @@ namespace {
 
 constexpr float kLog2e = 1.4426950408889634f;
 
-template <typename T> struct VecOf;
-template <> struct VecOf<float> { static constexpr int n = 4; };
-template <> struct VecOf<__half> { static constexpr int n = 8; };
-template <> struct VecOf<__nv_bfloat16> { static constexpr int n = 8; };
+template <int BYTES> struct Word;
+template <> struct Word<2> { using type = unsigned short; };
+template <> struct Word<4> { using type = unsigned; };
+template <> struct Word<8> { using type = uint2; };
+template <> struct Word<16> { using type = uint4; };
 
-template <typename T>
-__device__ __forceinline__ void load_vec(const T* p, float (&x)[VecOf<T>::n]) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(p);
+template <typename T, int V>
+__device__ __forceinline__ void load_vec(const T* p, float (&x)[V]) {
+    const auto raw = *reinterpret_cast<const typename Word<V * (int)sizeof(T)>::type*>(p);
     const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-    for (int i = 0; i < VecOf<T>::n; ++i) x[i] = to_f32<T>(e[i]);
+    for (int i = 0; i < V; ++i) x[i] = to_f32<T>(e[i]);
 }
-template <typename T>
-__device__ __forceinline__ void store_vec(T* p, const float (&x)[VecOf<T>::n]) {
-    uint4 raw;
+template <typename T, int V>
+__device__ __forceinline__ void store_vec(T* p, const float (&x)[V]) {
+    typename Word<V * (int)sizeof(T)>::type raw;
     T* e = reinterpret_cast<T*>(&raw);
 #pragma unroll
-    for (int i = 0; i < VecOf<T>::n; ++i) e[i] = from_f32<T>(x[i]);
-    *reinterpret_cast<uint4*>(p) = raw;
+    for (int i = 0; i < V; ++i) e[i] = from_f32<T>(x[i]);
+    *reinterpret_cast<typename Word<V * (int)sizeof(T)>::type*>(p) = raw;
 }
+
+// Where a row that begins anywhere lies in aligned vectors: vector v of it begins at element v * V of `src` and `dst`, and its own elements are
+// [head, end) of those; head == 0 and end % V == 0 unless RAGGED. All loads come first and `unpack` after, so that what the ends of a row cost stays
+// behind the last load.
+template <typename T, bool RAGGED>
+struct RowWindow {
+    static constexpr int V = 16 / (int)sizeof(T);
+    const T* src;
+    T* dst;
+    int head, end;
+    int first, last;   // vectors at [first, last) lie inside the tensor whole; the others are read element by element
+    bool whole_stores;
+    // [in, stop): the whole tensor, outside of which nothing is read
+    __device__ __forceinline__ RowWindow(const T* in, const T* stop, T* out, long long row, int n) : src(in + row * n), dst(out + row * n), head(0), end(n) {
+        if (RAGGED) {
+            head = (int)((reinterpret_cast<uintptr_t>(src) & 15) / sizeof(T));
+            src -= head;
+            dst -= head;
+            end += head;
+            first = src < in ? V : 0;
+            last = stop - src < end + V ? (int)(stop - src) / V * V : end + V;
+            whole_stores = (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+        }
+    }
+    __device__ __forceinline__ uint4 load(int col) const {
+        uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+        if (col >= first && col < last && col < end) raw = *reinterpret_cast<const uint4*>(src + col);
+        return raw;
+    }
+    // one bit per element of the vector at col that is the row's
+    __device__ __forceinline__ unsigned own(int col) const {
+        return (((1u << V) - 1u) << max(head - col, 0)) & ((1u << min(max(end - col, 0), V)) - 1u);
+    }
+    __device__ __forceinline__ void unpack(int col, const uint4& raw, float (&x)[V]) const {
+        const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+        for (int i = 0; i < V; ++i) x[i] = to_f32<T>(e[i]);
+        if (col < head || col + V > end) {
+            const unsigned mine = own(col);
+            if (col < first || col >= last) {
+#pragma unroll
+                for (int i = 0; i < V; ++i)
+                    if ((mine >> i) & 1u) x[i] = to_f32<T>(src[col + i]);
+            }
+#pragma unroll
+            for (int i = 0; i < V; ++i)
+                if (!((mine >> i) & 1u)) x[i] = -INFINITY;
+        }
+    }
+    __device__ __forceinline__ void store(int col, const float (&x)[V]) const {
+        if (!RAGGED || (col >= head && col + V <= end && whole_stores)) {
+            store_vec<T, V>(dst + col, x);
+            return;
+        }
+        const unsigned mine = own(col);
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+            if ((mine >> i) & 1u) dst[col + i] = from_f32<T>(x[i]);
+    }
+};
 
 __device__ __forceinline__ float fast_ex2(float x) {
     float y;
@@ -74,9 +139,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // One warp works on R rows at a time, each row in VPT vectors per lane (R * VPT vectors = 32 elements per lane).
-template <typename T, int VPT, int R>
+template <typename T, int V, int VPT, int R>
 __global__ void __launch_bounds__(256) softmax_warp_kernel(const T* __restrict__ in, T* __restrict__ out, long long rows, int n) {
-    constexpr int V = VecOf<T>::n;
     const int lane = threadIdx.x & 31;
     const long long row0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R;
     if (row0 >= rows) return;
@@ -91,7 +155,7 @@ __global__ void __launch_bounds__(256) softmax_warp_kernel(const T* __restrict__
         for (int v = 0; v < VPT; ++v) {
             const int col = (v * 32 + lane) * V;
             if (live && col < n) {
-                load_vec<T>(src + col, x[r][v]);
+                load_vec<T, V>(src + col, x[r][v]);
             } else {
 #pragma unroll
                 for (int i = 0; i < V; ++i) x[r][v][i] = -INFINITY;
@@ -127,30 +191,37 @@ __global__ void __launch_bounds__(256) softmax_warp_kernel(const T* __restrict__
                 if (col < n) {
 #pragma unroll
                     for (int i = 0; i < V; ++i) x[r][v][i] *= f;
-                    store_vec<T>(dst + col, x[r][v]);
+                    store_vec<T, V>(dst + col, x[r][v]);
                 }
             }
         }
     }
 }
 
-// One CTA of THREADS threads per row; VPT vectors per thread; one exchange through shared memory.
-template <typename T, int VPT, int THREADS>
+// One CTA of THREADS threads per row, or (RAGGED) of as many warps as the row's vectors need; VPT vectors per thread; one exchange through shared memory.
+template <typename T, bool RAGGED, int VPT, int THREADS>
 __global__ void __launch_bounds__(THREADS) softmax_block_kernel(const T* __restrict__ in, T* __restrict__ out, int n) {
-    constexpr int V = VecOf<T>::n;
+    constexpr int V = 16 / (int)sizeof(T);
     __shared__ float sh_m[THREADS / 32], sh_s[THREADS / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const T* src = in + (long long)blockIdx.x * n;
-    T* dst = out + (long long)blockIdx.x * n;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, threads = RAGGED ? blockDim.x : THREADS, warps = threads >> 5;
+    const RowWindow<T, RAGGED> w(in, in + (long long)gridDim.x * n, out, (long long)blockIdx.x, n);
     float x[VPT][V];
+    if constexpr (RAGGED) {
+        uint4 raw[VPT];
 #pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-        const int col = (v * THREADS + threadIdx.x) * V;
-        if (col < n) {
-            load_vec<T>(src + col, x[v]);
-        } else {
+        for (int v = 0; v < VPT; ++v) raw[v] = w.load((v * threads + threadIdx.x) * V);
 #pragma unroll
-            for (int i = 0; i < V; ++i) x[v][i] = -INFINITY;
+        for (int v = 0; v < VPT; ++v) w.unpack((v * threads + threadIdx.x) * V, raw[v], x[v]);
+    } else {
+#pragma unroll
+        for (int v = 0; v < VPT; ++v) {
+            const int col = (v * THREADS + threadIdx.x) * V;
+            if (col < n) {
+                load_vec<T, V>(w.src + col, x[v]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < V; ++i) x[v][i] = -INFINITY;
+            }
         }
     }
     float m = -INFINITY;
@@ -171,40 +242,37 @@ __global__ void __launch_bounds__(THREADS) softmax_block_kernel(const T* __restr
     float mw = warp_max(m);
     if (lane == 0) sh_m[warp] = mw;
     __syncthreads();
-    const float mr = warp_max(lane < THREADS / 32 ? sh_m[lane] : -INFINITY);
+    const float mr = warp_max(lane < warps ? sh_m[lane] : -INFINITY);
     const float rescale = (m == -INFINITY && mr != -INFINITY) ? 0.0f : fast_ex2((m - mr) * kLog2e);
     const float sw = warp_sum(s * rescale);
     if (lane == 0) sh_s[warp] = sw;
     __syncthreads();
-    const float sr = warp_sum(lane < THREADS / 32 ? sh_s[lane] : 0.0f);
+    const float sr = warp_sum(lane < warps ? sh_s[lane] : 0.0f);
     const float f = rescale / sr;
 #pragma unroll
     for (int v = 0; v < VPT; ++v) {
-        const int col = (v * THREADS + threadIdx.x) * V;
-        if (col < n) {
+        const int col = (v * threads + threadIdx.x) * V;
+        if (col < w.end) {
 #pragma unroll
             for (int i = 0; i < V; ++i) x[v][i] *= f;
-            store_vec<T>(dst + col, x[v]);
+            w.store(col, x[v]);
         }
     }
 }
 
 constexpr int kStreamThreads = 512;
 
-// Any row length: one CTA per row, pass 1 reduces (m, s) online, pass 2 re-reads and writes. VEC = true
-// reads 16 bytes per load (rows and base 16-byte aligned), else one element.
-template <typename T, bool VEC>
+// Any row length: one CTA per row, pass 1 reduces (m, s) online, pass 2 re-reads and writes.
+template <typename T, int V>
 __global__ void __launch_bounds__(kStreamThreads) softmax_stream_kernel(const T* __restrict__ in, T* __restrict__ out, int n) {
-    constexpr int V = VEC ? VecOf<T>::n : 1;
     __shared__ float sh_m[kStreamThreads / 32], sh_s[kStreamThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const T* src = in + (long long)blockIdx.x * n;
     T* dst = out + (long long)blockIdx.x * n;
     float m = -INFINITY, s = 0.0f;
     for (int c = threadIdx.x * V; c < n; c += kStreamThreads * V) {
-        float x[VecOf<T>::n];
-        if (VEC) load_vec<T>(src + c, x);
-        else x[0] = to_f32<T>(src[c]);
+        float x[V];
+        load_vec<T, V>(src + c, x);
         float mv = x[0];
 #pragma unroll
         for (int i = 1; i < V; ++i) mv = fmaxf(mv, x[i]);
@@ -222,45 +290,58 @@ __global__ void __launch_bounds__(kStreamThreads) softmax_stream_kernel(const T*
     warp_merge(m, s);
     const float ml = m * kLog2e, inv = 1.0f / s;
     for (int c = threadIdx.x * V; c < n; c += kStreamThreads * V) {
-        float x[VecOf<T>::n];
-        if (VEC) load_vec<T>(src + c, x);
-        else x[0] = to_f32<T>(src[c]);
+        float x[V];
+        load_vec<T, V>(src + c, x);
 #pragma unroll
         for (int i = 0; i < V; ++i) x[i] = fast_ex2(fmaf(x[i], kLog2e, -ml)) * inv;
-        if (VEC) store_vec<T>(dst + c, x);
-        else dst[c] = from_f32<T>(x[0]);
+        store_vec<T, V>(dst + c, x);
     }
 }
 
-template <typename T>
+template <typename T, int V>
 int launch_softmax(const T* in, T* out, long long rows, int n, cudaStream_t stream) {
-    constexpr int V = VecOf<T>::n;
     // 32 elements per thread (4 vectors of 16-bit, 8 of f32): few enough registers for 4 CTAs of 256
     // threads per SM, whose loads, arithmetic and stores then overlap; with 128 elements per thread
     // (one resident CTA) a bf16 row of 4096 reached 0.54 of the copy bandwidth
     constexpr int P = 32 / V;
-    const bool aligned = (n % V) == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-    const int vecs = (n + V - 1) / V;
+    const int vecs = n / V;
     const int warps = 8;
-    auto warp_grid = [&](int r) { return (unsigned)((rows + (long long)warps * r - 1) / ((long long)warps * r)); };
     const unsigned grid = (unsigned)rows;
-    if (aligned && vecs <= 32 * P) {
-        const int vpt = (vecs + 31) / 32;
-        if (vpt <= 1) softmax_warp_kernel<T, 1, P><<<warp_grid(P), warps * 32, 0, stream>>>(in, out, rows, n);
-        else if (vpt <= 2) softmax_warp_kernel<T, 2, P / 2><<<warp_grid(P / 2), warps * 32, 0, stream>>>(in, out, rows, n);
-        else if (vpt <= 4) softmax_warp_kernel<T, 4, P / 4><<<warp_grid(P / 4), warps * 32, 0, stream>>>(in, out, rows, n);
-        else softmax_warp_kernel<T, P, 1><<<warp_grid(1), warps * 32, 0, stream>>>(in, out, rows, n);
+    if (vecs <= 32 * P) {
+        // a warp takes R rows of P / R vectors per lane at a time
+        auto per_warp = [&](auto kernel, int r) {
+            kernel<<<(unsigned)((rows + (long long)warps * r - 1) / ((long long)warps * r)), warps * 32, 0, stream>>>(in, out, rows, n);
+        };
+        if (P >= 8 && vecs <= 32 * (P / 8)) per_warp(softmax_warp_kernel<T, V, P >= 8 ? P / 8 : P, P >= 8 ? 8 : 1>, 8);
+        else if (vecs <= 32 * (P / 4)) per_warp(softmax_warp_kernel<T, V, P / 4, 4>, 4);
+        else if (vecs <= 32 * (P / 2)) per_warp(softmax_warp_kernel<T, V, P / 2, 2>, 2);
+        else per_warp(softmax_warp_kernel<T, V, P, 1>, 1);
         note_path("softmax_warp", 1);
-    } else if (aligned && vecs <= 1024 * P) {
-        if (vecs <= 64 * P) softmax_block_kernel<T, P, 64><<<grid, 64, 0, stream>>>(in, out, n);
-        else if (vecs <= 128 * P) softmax_block_kernel<T, P, 128><<<grid, 128, 0, stream>>>(in, out, n);
-        else if (vecs <= 256 * P) softmax_block_kernel<T, P, 256><<<grid, 256, 0, stream>>>(in, out, n);
-        else if (vecs <= 512 * P) softmax_block_kernel<T, P, 512><<<grid, 512, 0, stream>>>(in, out, n);
-        else softmax_block_kernel<T, P, 1024><<<grid, 1024, 0, stream>>>(in, out, n);
+    } else if (V * sizeof(T) == 16 ? n <= 32768 : (n + 30 / (int)sizeof(T)) / (16 / (int)sizeof(T)) <= 32768 / (16 / (int)sizeof(T))) {
+        if constexpr (V * sizeof(T) == 16) {
+            if (vecs <= 64 * P) softmax_block_kernel<T, false, P, 64><<<grid, 64, 0, stream>>>(in, out, n);
+            else if (vecs <= 128 * P) softmax_block_kernel<T, false, P, 128><<<grid, 128, 0, stream>>>(in, out, n);
+            else if (vecs <= 256 * P) softmax_block_kernel<T, false, P, 256><<<grid, 256, 0, stream>>>(in, out, n);
+            else if (vecs <= 512 * P) softmax_block_kernel<T, false, P, 512><<<grid, 512, 0, stream>>>(in, out, n);
+            else softmax_block_kernel<T, false, P, 1024><<<grid, 1024, 0, stream>>>(in, out, n);
+        } else {
+            // Rows as long as this pay for aligned vectors with masked ends; in single elements a bf16 row of 4099 took 415 us where this takes 189
+            // (60000 rows), one of 1413 86 and 57 (f16, 46713 rows). CTAs of just as many warps as a row needs: in CTAs of a power of two,
+            // lengths just above one had twice the threads. Two CTAs of more than 512 threads do not fit an SM's registers: up to an eighth
+            // above, each thread takes a vector more (8000 rows of 16383 bf16: 105 us, 155 without).
+            constexpr int kWide = 16 / (int)sizeof(T), kEach = 32 / kWide;
+            const unsigned all = (unsigned)(n + 2 * kWide - 2) / kWide;   // (a row begins up to kWide - 1 elements into its first vector)
+            auto fit = [&](unsigned each) { return (all + each * 32 - 1) / (each * 32) * 32; };
+            const unsigned threads = fit(kEach);
+            if (threads <= 128) softmax_block_kernel<T, true, kEach, 128><<<grid, threads, 0, stream>>>(in, out, n);
+            else if (threads <= 256) softmax_block_kernel<T, true, kEach, 256><<<grid, threads, 0, stream>>>(in, out, n);
+            else if (threads <= 512) softmax_block_kernel<T, true, kEach, 512><<<grid, threads, 0, stream>>>(in, out, n);
+            else if (fit(kEach + 1) <= 512) softmax_block_kernel<T, true, kEach + 1, 512><<<grid, fit(kEach + 1), 0, stream>>>(in, out, n);
+            else softmax_block_kernel<T, true, kEach, 1024><<<grid, threads, 0, stream>>>(in, out, n);
+        }
         note_path("softmax_block", 1);
     } else {
-        if (aligned) softmax_stream_kernel<T, true><<<grid, kStreamThreads, 0, stream>>>(in, out, n);
-        else softmax_stream_kernel<T, false><<<grid, kStreamThreads, 0, stream>>>(in, out, n);
+        softmax_stream_kernel<T, V><<<grid, kStreamThreads, 0, stream>>>(in, out, n);
         note_path("softmax_stream", 1);
     }
     return check_launch("softmax_last_dim");
@@ -287,7 +368,14 @@ int softmax_impl(const void* in, void* out, long long rows, int n, void* stream)
     } else {
         cudaGetLastError();
     }
-    const int rc = launch_softmax<T>(static_cast<const T*>(in), static_cast<T*>(out), rows, n, static_cast<cudaStream_t>(stream));
+    const T* const src = static_cast<const T*>(in);
+    T* const dst = static_cast<T*>(out);
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    constexpr int kWide = 16 / (int)sizeof(T);
+    const uintptr_t both = reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out) | (uintptr_t)((size_t)n * sizeof(T));   // every row's beginning
+    const int rc = both % 16 == 0 ? launch_softmax<T, kWide>(src, dst, rows, n, st)
+                   : both % (2 * sizeof(T)) == 0 ? launch_softmax<T, 2>(src, dst, rows, n, st)
+                                                 : launch_softmax<T, 1>(src, dst, rows, n, st);
     if (prev >= 0) cudaSetDevice(prev);
     return rc;
 }

@@ -24,7 +24,7 @@ def test_oracle_softmax_matches_f64_formula():
     assert np.all(got[3, 10:] == 0.0) and abs(got[3].sum() - 1.0) < 1e-6
 
 
-# (rows, row_size): up to 1024 -> warp kernel; up to 32768 -> CTA kernel; beyond or unaligned -> two-pass
+# (rows, row_size): up to 1024 -> warp kernel; up to 32768 -> CTA kernel; beyond -> two-pass
 SHAPES = [(64, 8), (33, 256), (5, 1000), (17, 2048), (9, 4096), (3, 16384), (2, 40000), (7, 1001), (4, 77), (2, 33000)]
 
 
@@ -56,6 +56,37 @@ def test_softmax_kernel_matches_oracle(shape, dt):
     low.softmax_last_dim(y, out=y)
     torch.cuda.synchronize()
     assert torch.equal(y, got)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+def test_softmax_rows_that_begin_anywhere(dt):
+    """Rows that begin on no 16-byte boundary: odd and even sizes at both sides of every kernel's longest row, bases off the boundary by one
+    element, by two and more, input and output alike or not. Guard elements around both stay as they are, the NaN around the input reaches no
+    row, and a row's own NaN reaches its whole row."""
+    from luma_b200 import low
+    V = 4 if dt == "f32" else 8
+    sizes = sorted({1, 2, 3, 7, 162, 1413} | {n + o for n in (128, 256, 512, 1024, 2048, 4096, 8192, 16384, 16400, 18432, 20480, 32768) for o in (-1, 0, 1, 2)})
+    for n in sizes:
+        rows = 9 if n < 5000 else 3
+        for off_in, off_out in ((0, 0), (1, 1), (V - 1, V - 1), (0, 1), (3, 0)):
+            x = H.round_to(H.normal((rows, n), 7 + n) * 2.5, dt)
+            x[0, n // 2 + 1:] = -np.inf
+            if n > 40:
+                x[-1, n - 1] = np.nan
+            src = torch.full((rows * n + 2 * V,), float("nan"), device="cuda", dtype=H.to_dev(x[:1, :1], dt).dtype)
+            dst = torch.full_like(src, -3.0)
+            xd, yd = src[off_in:off_in + rows * n].view(rows, n), dst[off_out:off_out + rows * n].view(rows, n)
+            xd.copy_(H.to_dev(x, dt))
+            low.softmax_last_dim(xd, out=yd)
+            torch.cuda.synchronize()
+            g = H.to_np(yd)
+            want = _ref64(np.nan_to_num(x, nan=0.0, neginf=-np.inf)) if n <= 40 else np.concatenate([_ref64(x[:-1]), np.full((1, n), np.nan)])
+            # f32: sums of n terms in another order, ex2.approx, an argument rounded at |x| up to 12; 16 bits: one rounding of the result
+            rel, atol = {"f32": (1e-5, 1e-9), "bf16": (2.0 ** -8 + 1e-5, 1e-9), "f16": (2.0 ** -11 + 1e-5, 4e-8)}[dt]
+            np.testing.assert_allclose(g, want, rtol=rel, atol=atol, err_msg=f"{n} {off_in} {off_out}")
+            around = torch.cat([dst[:off_out], dst[off_out + rows * n:]])
+            assert bool((around == -3.0).all()), (n, off_in, off_out)
 
 
 @pytest.mark.gpu
