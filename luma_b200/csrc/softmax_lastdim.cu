@@ -276,10 +276,10 @@ __global__ void __launch_bounds__(kStreamThreads) softmax_stream_kernel(const T*
         float mv = x[0];
 #pragma unroll
         for (int i = 1; i < V; ++i) mv = fmaxf(mv, x[i]);
-        if (mv == -INFINITY) continue;
+        const float ref = mv == -INFINITY ? 0.0f : mv;   // (a NaN beside -inf reaches the sum so)
         float sv = 0.0f;
 #pragma unroll
-        for (int i = 0; i < V; ++i) sv += fast_ex2((x[i] - mv) * kLog2e);
+        for (int i = 0; i < V; ++i) sv += fast_ex2((x[i] - ref) * kLog2e);
         merge(m, s, mv, sv);
     }
     warp_merge(m, s);
