@@ -8,25 +8,29 @@
 // (kernels/flash_attn_with_kvcache.cu:157-277) and flash_attn_varlen_kernel
 // (kernels/flash_attn_varlen_func.cu:35-199), one-thread-per-query-row scalar kernels.
 //
-// One CTA (384 threads, 1 per SM) owns up to two query tiles of 128 rows that share a batch
+// One CTA (384 threads, 1 per SM) works on a pair of query tiles of 128 rows that share a batch
 // element and a KV head — two query heads of one GQA group at the same row block, or two
 // consecutive row blocks of one head when the group is 1 (tile 0 the later one) — and streams that KV head's K/V tiles
-// (128 keys) past both:
+// (128 keys) past both; then it takes over the pair of a CTA of the grid that has not started (clusterlaunchcontrol), until none is left:
 //   warps 0-3 / 4-7 : softmax warpgroup of query tile 0 / 1 — one thread per query row: read S
 //                     from tensor memory (tcgen05.ld), running max / sum in registers (exp2 with
 //                     the scale folded in), write P as packed 16-bit back over S (tcgen05.st),
 //                     rescale O in tensor memory only when the row max moved by more than 2^8,
-//                     final normalisation of O, staged in Q's shared memory and written with bulk
+//                     final normalisation of O, staged in shared memory and written with bulk
 //                     tensor stores (and LSE); setmaxnreg gives these warps 208 registers
-//   warp 8 / 10     : TMA producers — warp 8 loads Q once, then the K tiles; warp 10 the V tiles; two 2-stage rings
+//   warp 8 / 10     : TMA producers — warp 8 finds the tile pairs, loads Q and the K tiles; warp 10 the V tiles; two 2-stage rings
+//                     that run on across the pairs
 //   warp 9          : MMA issuer — S_t = Q_t K^T (SS form), O_t += P_t V (P from tensor memory),
 //                     completion signalled with tcgen05.commit on mbarriers; the warp runs converged
 //                     and one elected lane issues
-//   warp 11         : idle (completes the third warpgroup, which setmaxnreg needs whole)
-// While one warpgroup runs its softmax the tensor core works on the other tile.
+//   warp 11         : sets the barriers up
+// While one warpgroup runs its softmax the tensor core works on the other tile; while the warpgroups normalise and write O, the next
+// pair's Q and first K and V tiles arrive and its first S is computed. With a CTA for every pair, 4 to 5 us of each were set-up, first copies and
+// last stores with nothing beside them: 24 packed prompts of 17-2000 tokens at head size 64 332 us, 267 so; 8 x 1000 at head size 64, 32/8 heads 77 and 64; 4 x 2048
+// MHA 160 and 155; 2 x 8192 GQA, 64 steps to a pair, 937-948 and 945-952.
 // Tensor memory (512 columns): S0 | S1 | O0 | O1, 128 fp32 columns each; P_t aliases S_t.
 // Shared memory: Q 2 x 32 KiB, K ring 2 x 32 KiB, V ring 2 x 32 KiB, all 128-byte swizzled
-// exactly as TMA writes them, so the MMA descriptors address them in place.
+// exactly as TMA writes them, so the MMA descriptors address them in place; 32 KiB for the softmax warps' rows on their way out.
 //
 // Every wait on an mbarrier is bounded (about 2 s of wall clock); on expiry the CTA records a
 // status word in global memory, stops waiting everywhere, drains its own TMA copies, frees its
@@ -65,23 +69,60 @@ constexpr float kRescaleThreshold = 8.0f;            // log2 units
 // 145.1, 142.5, 143.8, 144.7; chunks with 32 decoding sequences 225.9, 225.0, 226.8, 230.4; 7 packed prompts of 7-125 tokens 27.4, 27.0, 27.3, 28.1.
 __device__ __forceinline__ constexpr bool fma_pipe_exp(int i) { return (i & 7) == 7; }
 
+// Extents of one sequence. Query row i sits at global position pos_off + i and sees keys
+// j < kv_len with j <= pos_off + i (bottom-right aligned for the varlen and kv-cache entry points).
+struct SeqExtent {
+    int q_len, kv_len, pos_off;
+    long long o_row0;     // first row of this sequence in o (rows of o_heads * 128 elements)
+    int q_crow, q_cb;     // TMA coordinates (row, batch) of the sequence's first q row
+    int kv_crow, kv_cb;   // same for contiguous K/V (unused when paged)
+};
+
+struct TileInfo {
+    int valid;    // this query tile exists
+    int head;     // query head
+    int row0;     // first query row
+    int n_kv;     // K/V tiles it needs
+};
+
+// One tile pair, as the CTA's roles find it in shared memory.
+struct Item {
+    int some;            // 0: nothing is left, the CTA ends
+    int seq, kv_head;
+    SeqExtent sq;
+    TileInfo t[2];
+};
+
+constexpr int kOutBytes = 4096;     // a softmax warp's rows on their way out: 32 of 128 bytes
+constexpr int kDone = 4;            // entries of step_done, see there
+
 template <int D>
 struct SharedStorage {
     alignas(1024) unsigned char q[2][TileBytes<D>::value];
     alignas(1024) unsigned char k[kStages][TileBytes<D>::value];
     alignas(1024) unsigned char v[kStages][TileBytes<D>::value];
-    alignas(8) unsigned long long q_full[2];
-    unsigned long long k_first;     // copy engine -> MMA: K tile 0
-    unsigned long long step_full[2];    // copy engine -> MMA: what step j reads, V tile j and K tile j + 1, in entry j & 1
-    unsigned long long step_done[2];    // MMA -> producers: the products of step j - 1 (j = 0: the first S) have finished, in entry j & 1
-    unsigned long long s_full[2];   // MMA -> softmax: S_t ready (and every earlier MMA finished)
+    alignas(1024) unsigned char out[8][kOutBytes];
+    alignas(16) unsigned char answer[16];   // what the request for another tile pair brought (written by the hardware)
+    Item item[2];                   // tile pair i of the CTA in entry i & 1
+    alignas(8) unsigned long long item_full[2];   // K producer -> all roles: the entry holds the next tile pair
+    unsigned long long item_empty[2];   // V producer, issuer, softmax warps -> K producer: it has been read
+    unsigned long long answered;    // hardware -> K producer: `answer` is there
+    unsigned long long q_full[2];
+    unsigned long long k_first;     // copy engine -> MMA: K tile 0 of a tile pair
+    unsigned long long step_full[2];    // copy engine -> MMA: what a step reads, its V tile and the tile pair's next K tile; step g of the CTA in entry g & 1
+    // MMA -> producers: what was issued before this has finished. The issuer commits once per tile pair for the first S and once for every step; commit c is in
+    // entry c & 3. A producer that waits for commit c can fall behind by up to three (tile pairs of one step: a step, the next pair's first S, its step), with two
+    // entries it would find the phase it waits for gone, and wait for good.
+    unsigned long long step_done[kDone];
+    unsigned long long s_full[2];   // MMA -> softmax: S_t ready
+    unsigned long long o_full[2];   // MMA -> softmax: O_t final (a barrier of its own: the next pair's first S_t may be ready before anybody has looked at this)
     unsigned long long p_ready[2][2];   // softmax -> MMA: keys 0-63 of P_t written and O_t rescaled ([0][t]), keys 64-127 written ([1][t])
     unsigned long long v_tail;      // copy engine -> V producer: the sequence's last, partly filled V tile has landed
     unsigned long long drain;       // MMA issuer, at its end: every product issued has finished
     unsigned int tmem_base;
     volatile int abort_flag;
-    int item[3];                    // ordered launches: sequence (-1: none left), KV head, tile pair of this CTA
 };
+static_assert(sizeof(SharedStorage<128>) + 1024 <= 232448, "fits the shared memory of an SM");
 
 constexpr int kMaxPeers = 8;
 #ifdef FA_TRACE
@@ -110,6 +151,7 @@ struct PrefillArgs {
     // NVLink), which makes the output all-gather part of the epilogue.
     void* o[kMaxPeers];
     int n_out, o_heads, o_head0;
+    int o_by_32;        // o[0] is 32-byte aligned (and so is every row of every head)
     int peer0;          // n_out > 1: the buffer this CTA's rows go to first; each CTA walks the buffers from there
     int multicast;      // o[0] is an NVSwitch multicast address of the group's output tensors: one multimem.st reaches all of them
     float* lse;         // (batch, q_heads, q_seq_len) of this call, or null
@@ -173,11 +215,28 @@ __device__ __forceinline__ bool mbar_try_wait_at(unsigned bar, unsigned parity) 
         : "memory");
     return ok != 0;
 }
+__device__ __forceinline__ bool mbar_test_at(unsigned bar, unsigned parity) {   // (does not suspend)
+    unsigned ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) { return mbar_try_wait_at(smem_u32(bar), parity); }
 __device__ __forceinline__ bool shared_flag(unsigned addr) {
     int f;
     asm volatile("ld.volatile.shared.s32 %0, [%1];\n" : "=r"(f) : "r"(addr) : "memory");
     return f != 0;
+}
+__device__ __forceinline__ int shared_int(unsigned addr) {
+    int f;
+    asm volatile("ld.shared.s32 %0, [%1];\n" : "=r"(f) : "r"(addr) : "memory");
+    return f;
+}
+__device__ __forceinline__ void mbar_arrive_at(unsigned bar) {
+    asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void set_shared_flag(unsigned addr) { asm volatile("st.volatile.shared.s32 [%0], 1;\n" ::"r"(addr) : "memory"); }
 __device__ __forceinline__ unsigned long long global_timer_ns() {
@@ -222,6 +281,11 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
         : "memory");
 }
 
+// The same box as far as L2.
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n" ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
+
 // Bulk tensor store shared -> global of one box, tracked by the issuing thread's bulk group.
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* src, int c0, int c1, int c2, int c3) {
     asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];\n" ::"l"(map),
@@ -234,6 +298,36 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void*
 __device__ __forceinline__ void multimem_st16(void* mc_addr, const uint4& w) {
     asm volatile("multimem.st.global.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(mc_addr), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w)
                  : "memory");
+}
+
+// Asks for a tile pair of a CTA that has not started (which then never does); the answer arrives as 16 bytes on the barrier.
+__device__ __forceinline__ void request_pair(void* answer, unsigned long long* bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];\n" ::"r"(smem_u32(answer)), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ bool read_answer(const void* answer, int& x, int& y, int& z) {
+    unsigned got;
+    asm volatile(
+        "{\n.reg .pred p;\n.reg .b128 h;\nld.shared.b128 h, [%4];\n"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\nselp.u32 %0, 1, 0, p;\n"
+        "mov.b32 %1, 0;\nmov.b32 %2, 0;\nmov.b32 %3, 0;\n"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, %3, _}, h;\n}\n"
+        : "=r"(got), "=r"(x), "=r"(y), "=r"(z)
+        : "r"(smem_u32(answer))
+        : "memory");
+    return got != 0;
+}
+
+// 32 bytes from registers, in one store where the buffer is aligned to them, else in two of 16.
+__device__ __forceinline__ void store_32(void* to, const unsigned (&w)[8], bool whole) {
+    if (whole) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(to), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]),
+                     "r"(w[7])
+                     : "memory");
+    } else {
+        *static_cast<uint4*>(to) = make_uint4(w[0], w[1], w[2], w[3]);
+        *(static_cast<uint4*>(to) + 1) = make_uint4(w[4], w[5], w[6], w[7]);
+    }
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
@@ -387,7 +481,7 @@ __device__ __forceinline__ unsigned make_idesc(bool b_mn_major, int n) {
     return d;
 }
 
-// Timeline slots: role (0/1 = softmax warpgroup, 2 = MMA issuer) x kv step (< 60) x event (< 8).
+// Timeline slots: role (0/1 = softmax warpgroup, 2 = MMA issuer, 3 = K producer, by tile pair) x step of the CTA, over its tile pairs (< 60) x event (< 8).
 // Compiled in with -DFA_TRACE only; the default build carries none of it.
 [[maybe_unused]] constexpr int kTraceSteps = 60;
 #ifdef FA_TRACE
@@ -402,22 +496,6 @@ __device__ __forceinline__ void trace_event(long long* trace, int role, int j, i
 #define FA_TRACE_PARAM(x)
 #define FA_TRACE_ARG(x)
 #endif
-
-struct TileInfo {
-    int valid;    // this query tile exists
-    int head;     // query head
-    int row0;     // first query row
-    int n_kv;     // K/V tiles it needs
-};
-
-// Extents of one sequence. Query row i sits at global position pos_off + i and sees keys
-// j < kv_len with j <= pos_off + i (bottom-right aligned for the varlen and kv-cache entry points).
-struct SeqExtent {
-    int q_len, kv_len, pos_off;
-    long long o_row0;     // first row of this sequence in o (rows of o_heads * 128 elements)
-    int q_crow, q_cb;     // TMA coordinates (row, batch) of the sequence's first q row
-    int kv_crow, kv_cb;   // same for contiguous K/V (unused when paged)
-};
 
 __device__ __forceinline__ SeqExtent seq_extent(const PrefillArgs& a, int s) {
     SeqExtent e;
@@ -570,12 +648,12 @@ __device__ __forceinline__ int page_of_lane(const PrefillArgs& a, int kv_len, in
 
 // Contiguous K/V: called by one lane.
 template <int D, bool kPaged>
-__device__ __forceinline__ void load_kv_tile(const PrefillArgs& a, const SeqExtent& sq, int kvh, unsigned char* dst,
+__device__ __forceinline__ void load_kv_tile(const PrefillArgs& a, int kv_crow, int kv_cb, int kvh, unsigned char* dst,
                                              const CUtensorMap* map, unsigned long long* bar, int j, int page, int lane) {
     if (!kPaged) {
         mbar_expect_tx(bar, TileBytes<D>::value);
-        tma_load_4d(dst, map, bar, 0, kvh, sq.kv_crow + j * kBlockN, sq.kv_cb);
-        if (D == 128) tma_load_4d(dst + kHalfBytes, map, bar, 64, kvh, sq.kv_crow + j * kBlockN, sq.kv_cb);
+        tma_load_4d(dst, map, bar, 0, kvh, kv_crow + j * kBlockN, kv_cb);
+        if (D == 128) tma_load_4d(dst + kHalfBytes, map, bar, 64, kvh, kv_crow + j * kBlockN, kv_cb);
         return;
     }
     if (lane == 0) mbar_expect_tx(bar, TileBytes<D>::value);
@@ -622,6 +700,8 @@ __device__ __forceinline__ void edge_tile_copy(unsigned char* dst, const void* b
 // The SM clock in units of 1024: 32 bits hold 36 minutes at 2 GHz, more than the longest bound of a wait.
 __device__ __forceinline__ unsigned clock_1024() { return (unsigned)(clock64() >> 10); }
 
+constexpr unsigned kApart = 950;   // clocks between the two tiles' first S at head size 64
+
 // The MMA issuer, run by one whole warp (converged). Its loop is written for few instructions. What a scheduler executes in a loop comes at full rate
 // up to 512 instructions (8 KiB), beyond that at one in 3 clocks, beyond 2048 in 6 (`clock64` around loops of that many independent multiply-adds); the
 // softmax warps' unrolled steps pass between two steps of the issuer, which finds its own anew every time. The tensor pipe stood still meanwhile: 300 clocks from the issuer's last commit of a step to its first look at the next barrier, 150 for
@@ -629,18 +709,15 @@ __device__ __forceinline__ unsigned clock_1024() { return (unsigned)(clock64() >
 // 884 -> 833 us; 4 x 2048 MHA 157.5 -> 147.8 us; head size 64, 2 x 8192 GQA 755 -> 699 us.
 //   * a function of its own, so that the compiler sees what is the same for the whole warp (everything is, or is broadcast here): inside
 //     the kernel it takes them for divergent, for the early returns and per-sequence loads before them;
+//   * nothing is in the loop for the sake of the next tile pair: with a look for it behind a tile's last step (so that its first S would be issued beside the other
+//     tile's last products) 24 packed prompts took 299 us instead of 275, 4 x 2048 MHA 159 instead of 154.5, 2 x 8192 GQA 965 instead of 947;
 //   * a wait that runs out is looked after at the end of its step, which goes on without waiting on what happens to be in shared memory and
 //     reports nothing as done. Leaving at each wait doubled the code after it.
-// n0, n1: K/V tiles that query tile 0 and 1 need (0: none, or no such tile).
 template <typename T, int D>
-__device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int n0, int n1, int* status, unsigned long long wait_ns
-                                            FA_TRACE_PARAM(trace)) {
+__device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int* status, unsigned long long wait_ns FA_TRACE_PARAM(trace)) {
     using Storage = SharedStorage<D>;
     sm_addr = __shfl_sync(0xffffffffu, sm_addr, 0);
-    n0 = __shfl_sync(0xffffffffu, n0, 0);
-    n1 = __shfl_sync(0xffffffffu, n1, 0);
     tmem = __shfl_sync(0xffffffffu, tmem, 0);
-    const int n_max = max(n0, n1);
     const unsigned idesc_qk = make_idesc<T>(false, kBlockN);
     const unsigned idesc_pv = make_idesc<T>(true, D);   // N = head size
     const unsigned long long dq = make_desc(sm_addr + (unsigned)offsetof(Storage, q), 16, 1024);
@@ -685,55 +762,78 @@ __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int
     auto commit = [&](size_t bar) {
         if (expired == 0 && elect_one()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(sm_addr + (unsigned)bar) : "memory");
     };
-    if (n_max > 0) {
+    unsigned s0_at = 0;
+    unsigned g = 0, done = 0, pairs = 0;      // steps, commits on step_done and tile pairs with a step so far
+    unsigned loads0 = 0, loads1 = 0, steps0 = 0, steps1 = 0;   // tiles of Q, steps of each query tile
+#pragma unroll 1
+    for (unsigned it = 0; expired == 0; ++it) {
+        const unsigned entry = sm_addr + (unsigned)offsetof(Storage, item) + (it & 1u) * (unsigned)sizeof(Item);
+        wait(offsetof(Storage, item_full) + 8 * (it & 1u), (it >> 1) & 1u, 18);
+        if (expired != 0) break;
+        // n0, n1: K/V tiles that query tile 0 and 1 need (0: none, or no such tile)
+        const int some = __shfl_sync(0xffffffffu, shared_int(entry + (unsigned)offsetof(Item, some)), 0);
+        const int n0 = __shfl_sync(0xffffffffu, shared_int(entry + (unsigned)(offsetof(Item, t) + offsetof(TileInfo, n_kv))), 0);
+        const int n1 = __shfl_sync(0xffffffffu, shared_int(entry + (unsigned)(offsetof(Item, t) + sizeof(TileInfo) + offsetof(TileInfo, n_kv))), 0);
+        if (elect_one()) mbar_arrive_at(sm_addr + (unsigned)offsetof(Storage, item_empty) + 8 * (it & 1u));
+        if (some == 0) break;
+        const int n_max = max(n0, n1);
+        if (n_max <= 0) continue;
         // The copies were requested in the order Q0, K0, Q1: the first S of tile 0 is issued as soon as
         // its two operands are there, without waiting for the other tile's Q.
+        const unsigned long long kd0 = dk + (g & 1u) * kTileStep;
 #pragma unroll 1
         for (int t = 0; t < 2; ++t) {
             if ((t == 0 ? n0 : n1) <= 0) continue;
-            wait(offsetof(Storage, q_full) + 8 * t, 0, 10);
-            wait(offsetof(Storage, k_first), 0, 11);
+            wait(offsetof(Storage, q_full) + 8 * t, (t == 0 ? loads0++ : loads1++) & 1u, 10);
+            wait(offsetof(Storage, k_first), pairs & 1u, 11);
+            if (D == 64) {
+                // Two tiles that start together stay together, in each other's way at the exponentials (2900 clocks a step); near half a step apart they stay
+                // so as well and take 2570. Where the pair has the steps to win the delay back.
+                if (t == 1 && n0 >= 4)
+                    while ((unsigned)clock64() - s0_at < kApart) {}
+                s0_at = (unsigned)clock64();
+            }
             tc_fence_after();
-            issue_s(t, dk);
+            issue_s(t, kd0);
             commit(offsetof(Storage, s_full) + 8 * t);
         }
-        commit(offsetof(Storage, step_done));
-    }
-    FA_TRACE_EVENT(2, kTraceSteps - 1, 2);       // Q and the first K tile have landed
+        ++pairs;
+        commit(offsetof(Storage, step_done) + 8 * (done++ & (kDone - 1)));
+        FA_TRACE_EVENT(2, (int)g, 7);       // Q and the first K tile have landed
 #pragma unroll 1
-    for (int j = 0; j < n_max; ++j) {
-        const unsigned s = j & 1;   // stage of V(j); K(j + 1) is in the other one
-        const unsigned long long vd = dv + s * kTileStep, kd = dk + (s ^ 1) * kTileStep;
-        wait(offsetof(Storage, step_full) + 8 * s, (unsigned)(j >> 1) & 1u, 13);
-        FA_TRACE_EVENT(2, j, 4);
+        for (int j = 0; j < n_max && expired == 0; ++j, ++g) {
+            const unsigned s = g & 1u;   // stage of this step's V tile; the next K tile is in the other one
+            const unsigned long long vd = dv + s * kTileStep, kd = dk + (s ^ 1u) * kTileStep;
+            wait(offsetof(Storage, step_full) + 8 * s, (g >> 1) & 1u, 13);
+            FA_TRACE_EVENT(2, (int)g, 4);
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const int n_kv = t == 0 ? n0 : n1;
-            if (j < n_kv) {
-                // the first 64 keys of P_t arrive while the softmax still works on the other 64:
-                // their half of P.V leaves the critical path
-                wait(offsetof(Storage, p_ready) + 8 * t, s, 14 + t);
-                FA_TRACE_EVENT(2, j, t * 2);
-                tc_fence_after();
-                issue_pv(t, 0, vd, j > 0);
-                wait(offsetof(Storage, p_ready) + 16 + 8 * t, s, 16 + t);
-                FA_TRACE_EVENT(2, j, 5 + t);
-                tc_fence_after();
-                issue_pv(t, 1, vd, true);
-                if (j + 1 < n_kv) issue_s(t, kd);
-                commit(offsetof(Storage, s_full) + 8 * t);   // S_t(j+1) ready, or after the last PV: O_t final
-                FA_TRACE_EVENT(2, j, t * 2 + 1);
+            for (int t = 0; t < 2; ++t) {
+                const int n_kv = t == 0 ? n0 : n1;
+                if (j < n_kv) {
+                    // the first 64 keys of P_t arrive while the softmax still works on the other 64:
+                    // their half of P.V leaves the critical path
+                    const unsigned ph = (t == 0 ? steps0++ : steps1++) & 1u;
+                    wait(offsetof(Storage, p_ready) + 8 * t, ph, 14 + t);
+                    FA_TRACE_EVENT(2, (int)g, t * 2);
+                    tc_fence_after();
+                    issue_pv(t, 0, vd, j > 0);
+                    wait(offsetof(Storage, p_ready) + 16 + 8 * t, ph, 16 + t);
+                    FA_TRACE_EVENT(2, (int)g, 5 + t);
+                    tc_fence_after();
+                    issue_pv(t, 1, vd, true);
+                    const bool more = j + 1 < n_kv;
+                    if (more) issue_s(t, kd);
+                    commit((more ? offsetof(Storage, s_full) : offsetof(Storage, o_full)) + 8 * t);
+                    FA_TRACE_EVENT(2, (int)g, t * 2 + 1);
+                }
             }
+            commit(offsetof(Storage, step_done) + 8 * (done++ & (kDone - 1)));
         }
-        commit(offsetof(Storage, step_done) + 8 * (s ^ 1));
-        if (expired != 0) {
-            if (!shared_flag(sm_addr + (unsigned)offsetof(Storage, abort_flag))) {   // (else another warp of the CTA gave up and reported it)
-                set_shared_flag(sm_addr + (unsigned)offsetof(Storage, abort_flag));
-                *reinterpret_cast<volatile int*>(status) = expired;
-                __threadfence_system();
-            }
-            break;
-        }
+    }
+    if (expired != 0 && !shared_flag(sm_addr + (unsigned)offsetof(Storage, abort_flag))) {   // (else another warp of the CTA gave up and reported it)
+        set_shared_flag(sm_addr + (unsigned)offsetof(Storage, abort_flag));
+        *reinterpret_cast<volatile int*>(status) = expired;
+        __threadfence_system();
     }
     // Tensor memory is freed at the end of the kernel, in error paths while the softmax warps have long left: every product issued here has to
     // finish first (bounded; depends on the tensor pipe alone). Otherwise the last P.V is what the epilogue waits for as well.
@@ -742,6 +842,38 @@ __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int
     commit(offsetof(Storage, drain));
     const unsigned long long t_begin = global_timer_ns();
     while (!mbar_try_wait_at(sm_addr + (unsigned)offsetof(Storage, drain), 0u) && global_timer_ns() - t_begin < 100000000ULL) {}
+}
+
+// The tile pair that CTA (bx, by, bz) of the grid stands for; false: there is none, or nothing to do for it. Run by one whole warp.
+template <bool kPaged>
+__device__ __forceinline__ bool find_pair(const PrefillArgs& a, int bx, int by, int bz, int lane, Item& w) {
+    const int group = a.by_group.d;
+    int pair;
+    if (kPaged && a.ordered) {
+        const int3 item = find_item(a, group, bx, lane);
+        w.seq = item.x; w.kv_head = item.y; pair = item.z;
+        if (w.seq < 0) return false;
+    } else {
+        // x = (batch element, KV head) x `band` neighbouring tile pairs, y = band of pairs,
+        // heaviest (latest rows) first. Pairs are handed out in index order, so the `band` pairs that walk
+        // the same K/V stream start together and meet its tiles in L2 instead of each pulling them from
+        // HBM, while the order across bands stays heaviest first.
+        // z = group of K/V streams: the grid runs group after group (each heaviest first), so that the
+        // K/V of the streams in flight stay within L2 when every tile pair of a stream re-reads its stream's prefix
+        const int x_band = a.by_band.div(bx);
+        const int stream_id = bz * a.streams_z + x_band;
+        if (stream_id >= a.kv_heads * a.batch) return false;   // the last group may be short
+        w.seq = a.by_kv_heads.div(stream_id);
+        w.kv_head = stream_id - w.seq * a.kv_heads;
+        const int rank_y = launch_rank(by, a.spread_w, a.spread_m);   // this row's rank by weight, 0 = heaviest
+        pair = ((int)gridDim.y - 1 - rank_y) * a.band + (a.band - 1 - (bx - x_band * a.band));
+    }
+    w.sq = seq_extent(a, w.seq);
+    if (w.sq.q_len * group <= a.skip_rows) return false;   // the few-row kernel's
+    const int num_mb = (w.sq.q_len + kBlockM - 1) / kBlockM;
+    w.t[0] = tile_info(w.sq, pair, 0, w.kv_head, a.by_group, num_mb);
+    w.t[1] = tile_info(w.sq, pair, 1, w.kv_head, a.by_group, num_mb);
+    return w.t[0].valid || w.t[1].valid;   // (a sequence may be shorter than the grid's row range)
 }
 
 // kMask: the call carries a key-padding mask (a separate instantiation, so that calls without one
@@ -763,147 +895,209 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // (the same for the whole warp, which the compiler sees only so)
     const int lane = threadIdx.x & 31;
-    const int group = a.by_group.d;
-    if (warp == kLoadWarp && lane == 0) {   // (what needs no extents goes first: their loads are on the way meanwhile)
-        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&q_map) : "memory");
-        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&k_map) : "memory");
-        asm volatile("prefetch.tensormap [%0];\n" ::"l"(&v_map) : "memory");
-        sm.abort_flag = 0;
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&sm.q_full[i], 1);
-            mbar_init(&sm.s_full[i], 1);
-            mbar_init(&sm.p_ready[0][i], 128);
-            mbar_init(&sm.p_ready[1][i], 128);
-            mbar_init(&sm.step_full[i], 2);
-            mbar_init(&sm.step_done[i], 1);
-        }
-        mbar_init(&sm.k_first, 1);
-        mbar_init(&sm.v_tail, 1);
-        mbar_init(&sm.drain, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    }
-    // A few-row kernel launched behind this one may start once every CTA here has: it fills the SMs that run out of tile pairs.
+    // A few-row kernel launched behind this one may start once every tile pair here is taken: it fills the SMs that run out of them.
     if (a.skip_rows > 0) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    int b, kvh, pair;
-    if (kPaged && a.ordered) {
-        if (warp == kLoadWarp) {
-            const int3 item = find_item(a, group, (int)blockIdx.x, lane);
-            if (lane == 0) { sm.item[0] = item.x; sm.item[1] = item.y; sm.item[2] = item.z; }
-        }
-        __syncthreads();
-        b = sm.item[0]; kvh = sm.item[1]; pair = sm.item[2];
-        if (b < 0) return;   // no pair is left for this CTA
-    } else {
-        // blockIdx.x = (batch element, KV head) x `band` neighbouring tile pairs, blockIdx.y = band of pairs,
-        // heaviest (latest rows) first. CTAs are dispatched in index order, so the `band` CTAs that walk
-        // the same K/V stream start together and meet its tiles in L2 instead of each pulling them from
-        // HBM, while the order across bands stays heaviest first.
-        // blockIdx.z = group of K/V streams: the grid runs group after group (each heaviest first), so that the
-        // K/V of the streams in flight stay within L2 when every tile pair of a stream re-reads its stream's prefix
-        const int x_band = a.by_band.div((int)blockIdx.x);
-        const int stream_id = (int)blockIdx.z * a.streams_z + x_band;
-        if (stream_id >= a.kv_heads * a.batch) return;   // the last group may be short
-        b = a.by_kv_heads.div(stream_id);
-        kvh = stream_id - b * a.kv_heads;
-        const int rank_y = launch_rank((int)blockIdx.y, a.spread_w, a.spread_m);   // this row's rank by weight, 0 = heaviest
-        pair = ((int)gridDim.y - 1 - rank_y) * a.band + (a.band - 1 - ((int)blockIdx.x - x_band * a.band));
-    }
-    const SeqExtent sq = seq_extent(a, b);
-    if (sq.q_len * group <= a.skip_rows) return;   // the few-row kernel's
-    const int num_mb = (sq.q_len + kBlockM - 1) / kBlockM;
-
-    const TileInfo t0 = tile_info(sq, pair, 0, kvh, a.by_group, num_mb);
-    const TileInfo t1 = tile_info(sq, pair, 1, kvh, a.by_group, num_mb);
-    if (!t0.valid && !t1.valid) return;   // this sequence is shorter than the grid's row range (whole CTA leaves)
-    const int n_max = max(t0.n_kv, t1.n_kv);
-
-    // The first copies are requested before the CTA-wide set-up barrier, by the two producer warps (Q and the K tiles that fill the empty ring; the
-    // V tiles likewise): they fly while tensor memory is being allocated and the other warps start up.
-    const int n_pre = min(kStages, n_max);
     // Packed buffers end at row cu_seqlens[num_seqs]; where the tensor map does not end with the buffer, a tile that reaches past that row is not asked
-    // of the copy engine (see edge_tile_copy) but fetched by the producer warp after the set-up. A map that does gives zeros there like any other.
+    // of the copy engine but fetched by the producer warp (see edge_tile_copy). A map that does gives zeros there like any other.
     const bool packed = a.mode == MODE_VARLEN;
-    const bool q_open = packed && !a.q_bounded, kv_open = packed && !a.paged && !a.kv_bounded;
-    const long long tot_q = q_open ? (long long)a.cu_q[a.batch] : 0;
-    const long long tot_k = kv_open ? (long long)a.cu_k[a.batch] : 0;
-    // (a tile that sees no key needs no Q: the issuer leaves it out, and its softmax warps lay zeros down in Q's shared memory without waiting for anybody)
-    auto q_edge = [&](const TileInfo& ti) { return q_open && ti.n_kv > 0 && (long long)sq.q_crow + ti.row0 + kBlockM > tot_q; };
-    auto kv_edge = [&](int j) { return kv_open && (long long)sq.kv_crow + (long long)(j + 1) * kBlockN > tot_k; };
-    if (warp == kLoadWarp) asm volatile("barrier.cta.arrive 1, 64;\n" ::: "memory");
-    if (warp == kLoadWarp && (kPaged || lane == 0)) {
-        int pages[kStages];   // of the tiles requested here, looked up together
-#pragma unroll
-        for (int j = 0; j < kStages; ++j) pages[j] = kPaged && j < n_pre ? page_of_lane(a, sq.kv_len, b, j, lane) : -1;
-        auto load_q = [&](const TileInfo& ti, int t) {
-            if ((kPaged && lane != 0) || ti.n_kv <= 0 || q_edge(ti)) return;
-            mbar_expect_tx(&sm.q_full[t], TileBytes<D>::value);
-            tma_load_4d(sm.q[t], &q_map, &sm.q_full[t], 0, ti.head, sq.q_crow + ti.row0, sq.q_cb);
-            if (D == 128) tma_load_4d(sm.q[t] + kHalfBytes, &q_map, &sm.q_full[t], 64, ti.head, sq.q_crow + ti.row0, sq.q_cb);
-        };
-        load_q(t0, 0);
-#pragma unroll
-        for (int j = 0; j < kStages; ++j) {
-            if (j < n_pre && !kv_edge(j) && a.test_skip_k != j + 1) load_kv_tile<D, kPaged>(a, sq, kvh, sm.k[j], &k_map, j == 0 ? &sm.k_first : &sm.step_full[0], j, pages[j], lane);
-            if (j == 0) load_q(t1, 1);
-        }
-        if (lane == 0) asm volatile("prefetch.tensormap [%0];\n" ::"l"(&o_map) : "memory");
-    }
-    int v_issued = 0;
-    if (warp == kLoadWarpV) {
-        asm volatile("barrier.cta.sync 1, 64;\n" ::: "memory");   // the barriers have been initialised
-        // (the tiles that need more than a copy are left to the producer loop)
-        while (v_issued < n_pre && !kv_edge(v_issued) && !((a.paged || packed) && (v_issued + 1) * kBlockN > sq.kv_len)) {
-            if (kPaged || lane == 0)
-                load_kv_tile<D, kPaged>(a, sq, kvh, sm.v[v_issued], &v_map, &sm.step_full[v_issued], v_issued, kPaged ? page_of_lane(a, sq.kv_len, b, v_issued, lane) : -1, lane);
-            ++v_issued;
-        }
-    }
-    if (warp == kMmaWarp) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(&sm.tmem_base)) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const unsigned tmem = sm.tmem_base;
-#ifdef FA_TRACE
-    // only the heaviest CTA of the first (batch, KV head) records its timeline, one thread per role
-    long long* const trace = (a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == (unsigned)a.trace_y && lane == 0 && (warp == kMmaWarp || (warp & 3) == 0)) ? a.trace : nullptr;
-    // slot kTraceSteps - 1 of each role holds the CTA's life cycle instead of a kv step
-    if (trace != nullptr && warp == kMmaWarp) {
-        trace[(2 * kTraceSteps + kTraceSteps - 1) * 8 + 0] = t_entry;
-        FA_TRACE_EVENT(2, kTraceSteps - 1, 1);   // set-up (barriers, tensor memory) done
-    }
-#endif
 
     // Register budget: the kernel is compiled for 168 registers per thread (384 threads); the
     // producer/issuer warpgroup hands most of its share to the two softmax warpgroups, which
     // keep a whole 128-column score row per thread in registers.
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n");
-    if (warp == kLoadWarp || warp == kLoadWarpV) {
-        // ------------------------------ TMA producers ------------------------------
-        // One thread streams the K tiles (and loaded Q before), one the V tiles: with a paged cache a
-        // tile is one copy per page and 64-column half plus a block-table read per page, and a single
-        // thread issuing both rings cannot keep up with the tensor pipe at small page sizes.
-        // The warps run their loops whole; lane 0 issues the bulk copies, and all lanes share the
+    if (warp == kLoadWarp) {
+        // ------------------------------ tile pairs, Q and K tiles ------------------------------
+        // The warps run their loops whole; lane 0 issues the bulk copies (a paged tile: a lane per page), and all lanes share the
         // plain-load copy of a tile at the very end of a packed buffer.
-        {
-            const bool is_v = warp == kLoadWarpV;
-            unsigned char (*ring)[TileBytes<D>::value] = is_v ? sm.v : sm.k;
-            const CUtensorMap* map = is_v ? &v_map : &k_map;
-            const void* kv_base = is_v ? a.v : a.k;
-            bool alive = true;
-            // V tile j and K tile j + 1 are what step j reads: both arrive on its barrier
-            auto full_of = [&](int j) { return is_v ? &sm.step_full[j & 1] : (j == 0 ? &sm.k_first : &sm.step_full[(j - 1) & 1]); };
-            auto full_parity = [&](int j) { return is_v ? (unsigned)(j >> 1) & 1u : (j == 0 ? 0u : (unsigned)((j - 1) >> 1) & 1u); };
-            if (!is_v) {   // what the set-up left out: Q tiles and first K tiles at the end of the packed buffers
-                if (q_edge(t0)) edge_tile_copy<D>(sm.q[0], a.q, a.q_heads, t0.head, (long long)sq.q_crow + t0.row0, tot_q, &sm.q_full[0], lane, a.d_real);
-                if (q_edge(t1)) edge_tile_copy<D>(sm.q[1], a.q, a.q_heads, t1.head, (long long)sq.q_crow + t1.row0, tot_q, &sm.q_full[1], lane, a.d_real);
-                for (int j = 0; j < n_pre; ++j)
-                    if (kv_edge(j)) edge_tile_copy<D>(sm.k[j], a.k, a.kv_heads, kvh, (long long)sq.kv_crow + (long long)j * kBlockN, tot_k, full_of(j), lane, a.d_real);
+        const bool q_open = packed && !a.q_bounded, kv_open = packed && !a.paged && !a.kv_bounded;
+        const long long tot_q = q_open ? (long long)a.cu_q[a.batch] : 0;
+        const long long tot_k = kv_open ? (long long)a.cu_k[a.batch] : 0;
+        int g = 0, commits = 0;              // steps and commits on step_done of the tile pairs before this one
+        int k_free0 = -1, k_free1 = -1;      // the commit that frees each K stage (-1: free)
+        unsigned scores0 = 0, scores1 = 0;   // S of each query tile so far: its Q is free when the last one has finished
+        bool q_used0 = false, q_used1 = false;   // (and has to be waited for: by the pair before this one)
+        int first_s = -1;                    // the commit of the last pair's first S, where that pair had one step (else it has been waited for)
+        int k_asked = 0, n_before = 0;       // K tiles of this pair that have been requested; tiles of the pair before
+        unsigned q_loads0 = 0, q_loads1 = 0, pairs = 0, requests = 0, answers = 0;
+        bool alive = true, own = true;
+#ifdef FA_TRACE
+        long long* const trace = (a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == (unsigned)a.trace_y && blockIdx.z == 0 && lane == 0) ? a.trace : nullptr;
+#endif
+        auto wait_commit = [&](int c) { return c < 0 || __all_sync(0xffffffffu, mbar_wait(sm, &sm.step_done[c & (kDone - 1)], (unsigned)(c / kDone) & 1u, a, 1)); };
+        auto ask = [&]() {
+            if (lane == 0) {
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // (the answer before has been read)
+                mbar_expect_tx(&sm.answered, 16);
+                request_pair(sm.answer, &sm.answered);
             }
+            ++requests;
+            FA_TRACE_EVENT(3, (int)requests, 0);
+        };
+        bool owed = false;                   // the arrival that the last step of the pair before waits for, in place of another K tile
+        auto owed_commit = [&]() { return (g & 1) ? k_free1 : k_free0; };
+        for (unsigned it = 0;; ++it) {
+            if (owed) {
+                const int c = owed_commit();
+                if (c < 0 || __all_sync(0xffffffffu, mbar_test_at(smem_u32(&sm.step_done[c & (kDone - 1)]), (unsigned)(c / kDone) & 1u))) {
+                    if (lane == 0) mbar_arrive(&sm.step_full[(g - 1) & 1]);
+                    owed = false;
+                }
+            }
+            // The next tile pair with something to do: this CTA's own first, then those of CTAs that have not started. Asked for when the pair at hand has its
+            // last K tile requested, two to three steps before its end: whoever comes to its end first takes the next one. Asked for at a
+            // pair's beginning, the order heaviest first was lost for the second half of 4 chunks of 512 (256 pairs on 148 SMs): 174 us instead of
+            // 153. The answer takes 1100 to 3100 clocks, what follows from it until the first copy 2000 more.
+            if (!own && requests == answers) ask();
+            Item w;
+            w.some = 0;
+            if (it >= 2) alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.item_empty[it & 1u], ((it >> 1) - 1u) & 1u, a, 5));
+            while (alive) {
+                int bx = (int)blockIdx.x, by = (int)blockIdx.y, bz = (int)blockIdx.z;
+                if (!own) {
+                    alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.answered, answers & 1u, a, 6));
+                    if (!alive) break;
+                    ++answers;
+                    FA_TRACE_EVENT(3, (int)answers, 1);
+                    const bool got = read_answer(sm.answer, bx, by, bz);
+                    __syncwarp();
+                    if (!got) break;   // every tile pair is taken
+                }
+                w.some = find_pair<kPaged>(a, bx, by, bz, lane, w);
+                if (own) asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
+                own = false;
+                if (w.some) break;
+                ask();
+            }
+            if (!alive) break;
+            if (!w.some) w.t[0].n_kv = w.t[1].n_kv = 0;
+            if (lane == 0) {
+                sm.item[it & 1u] = w;
+                mbar_arrive(&sm.item_full[it & 1u]);
+            }
+            FA_TRACE_EVENT(3, (int)it, 2);
+            if (owed) {
+                alive = wait_commit(owed_commit());
+                if (!alive) break;
+                if (lane == 0) mbar_arrive(&sm.step_full[(g - 1) & 1]);
+                owed = false;
+            }
+            if (!w.some) break;
+            const int kv_len = w.sq.kv_len, kv_crow = w.sq.kv_crow, kv_cb = w.sq.kv_cb, seq = w.seq, kv_head = w.kv_head;
+            const int n0 = w.t[0].n_kv, n1 = w.t[1].n_kv, n_max = max(n0, n1);
+            if (n_max <= 0) {
+                ask();
+                continue;
+            }
+            if (it > 0 && !q_open && lane == 0) {   // its Q on the way to L2 while the tiles before it are still in use
+                if (n0 > 0) {
+                    tma_prefetch_4d(&q_map, 0, w.t[0].head, w.sq.q_crow + w.t[0].row0, w.sq.q_cb);
+                    if (D == 128) tma_prefetch_4d(&q_map, 64, w.t[0].head, w.sq.q_crow + w.t[0].row0, w.sq.q_cb);
+                }
+                if (n1 > 0) {
+                    tma_prefetch_4d(&q_map, 0, w.t[1].head, w.sq.q_crow + w.t[1].row0, w.sq.q_cb);
+                    if (D == 128) tma_prefetch_4d(&q_map, 64, w.t[1].head, w.sq.q_crow + w.t[1].row0, w.sq.q_cb);
+                }
+            }
+            int page = kPaged ? page_of_lane(a, kv_len, seq, 0, lane) : -1;
+            auto load_k = [&](int j) {   // K tile j of the pair is what step g + j - 1 reads besides its V tile, and arrives on its barrier (tile 0: on its own)
+                const int e = (g + j) & 1;
+                unsigned long long* const bar = j == 0 ? &sm.k_first : &sm.step_full[e ^ 1];
+                if (a.test_skip_k != j + 1) {   // (the test hook's tile is never requested, the issuer's wait for it runs out)
+                    if (kv_open && (long long)kv_crow + (long long)(j + 1) * kBlockN > tot_k)
+                        edge_tile_copy<D>(sm.k[e], a.k, a.kv_heads, kv_head, (long long)kv_crow + (long long)j * kBlockN, tot_k, bar, lane, a.d_real);
+                    else if (kPaged || lane == 0) load_kv_tile<D, kPaged>(a, kv_crow, kv_cb, kv_head, sm.k[e], &k_map, bar, j, page, lane);
+                }
+                (e ? k_free1 : k_free0) = commits + j;
+                k_asked = j + 1;
+                if (kPaged && j + 1 < n_max) page = page_of_lane(a, kv_len, seq, j + 1, lane);
+            };
+            // (a tile that sees no key needs no Q: the issuer leaves it out)
+            auto load_q = [&](const TileInfo ti, unsigned char* to, unsigned long long* bar, unsigned& loads) {
+                if (ti.n_kv <= 0) return;
+                ++loads;
+                if (q_open && (long long)w.sq.q_crow + ti.row0 + kBlockM > tot_q) {
+                    edge_tile_copy<D>(to, a.q, a.q_heads, ti.head, (long long)w.sq.q_crow + ti.row0, tot_q, bar, lane, a.d_real);
+                } else if (lane == 0) {
+                    mbar_expect_tx(bar, TileBytes<D>::value);
+                    tma_load_4d(to, &q_map, bar, 0, ti.head, w.sq.q_crow + ti.row0, w.sq.q_cb);
+                    if (D == 128) tma_load_4d(to + kHalfBytes, &q_map, bar, 64, ti.head, w.sq.q_crow + ti.row0, w.sq.q_cb);
+                }
+            };
+            k_asked = 0;
+            alive = wait_commit(first_s) &&   // the last pair's K tile 0 has left its barrier
+                    wait_commit((g & 1) ? k_free1 : k_free0);
+            if (!alive) break;
+            load_k(0);
+            FA_TRACE_EVENT(3, (int)it, 3);
+            // (the first pair's tile 0 first, whose products are; else the one that comes free first, of two row blocks of one head the shorter one, tile 1)
+            auto wait_q = [&](int t, unsigned scores) { return __all_sync(0xffffffffu, mbar_wait(sm, &sm.s_full[t], (scores - 1u) & 1u, a, 8)); };
+#pragma unroll 1
+            for (int n = 0; n < 2; ++n) {
+                const int t = it == 0 ? n : n ^ 1;
+                if (t ? q_used1 : q_used0) alive = wait_q(t, t ? scores1 : scores0);
+                if (!alive) break;
+                load_q(t ? w.t[1] : w.t[0], sm.q[t], &sm.q_full[t], t ? q_loads1 : q_loads0);
+                FA_TRACE_EVENT(3, (int)it, 4 + t);
+            }
+            if (!alive) break;
+            for (int j = 1; j < n_max; ++j) {
+                alive = wait_commit(((g + j) & 1) ? k_free1 : k_free0);
+                if (!alive) break;
+                load_k(j);
+            }
+            if (!alive) break;
+            owed = true;
+            ++pairs;
+            n_before = n_max;
+            // (waits are for commits of late only, see step_done: where this pair had no use for a Q tile, that has long been free)
+            first_s = n_max == 1 ? commits : -1;
+            q_used0 = n0 > 0;
+            q_used1 = n1 > 0;
+            scores0 += (unsigned)max(n0, 0);
+            scores1 += (unsigned)max(n1, 0);
+            commits += n_max + 1;
+            g += n_max;
+        }
+        // After an abort none of this warp's copies may be in flight when the CTA ends (otherwise every tile has been read): wait (bounded) for
+        // the last ones. These waits ignore the abort flag: they only depend on the copy engine; the other ring's arrival may be missing, and the
+        // copies have landed long before the limit then.
+        if (lane == 0 && !alive) {
+            const unsigned long long t_begin = global_timer_ns();
+            auto settle = [&](unsigned long long* bar, unsigned parity) {
+                while (!mbar_try_wait(bar, parity) && global_timer_ns() - t_begin < 100000000ULL) {}
+            };
+            if (answers != requests) settle(&sm.answered, answers & 1u);
+            if (q_loads0 > 0) settle(&sm.q_full[0], (q_loads0 - 1u) & 1u);
+            if (q_loads1 > 0) settle(&sm.q_full[1], (q_loads1 - 1u) & 1u);
+            for (int j = k_asked - 2; j < k_asked; ++j) {   // (j = -1, -2: of the pair before)
+                if (j < -1 || (j == -1 && n_before == 0) || (j >= 0 && a.test_skip_k == j + 1)) continue;
+                if (j == 0 || (j == -1 && n_before == 1)) settle(&sm.k_first, (pairs + (j == 0 ? 0u : 1u)) & 1u);
+                else settle(&sm.step_full[(g + j - 1) & 1], (unsigned)((g + j - 1) >> 1) & 1u);
+            }
+        }
+    } else if (warp == kLoadWarpV) {
+        // ------------------------------ V tiles ------------------------------
+        // A producer of its own: with a paged cache a tile is one copy per page and 64-column half plus a block-table read per page, and a single
+        // thread issuing both rings cannot keep up with the tensor pipe at small page sizes.
+        asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
+        const bool kv_open = packed && !a.paged && !a.kv_bounded;
+        const long long tot_k = kv_open ? (long long)a.cu_k[a.batch] : 0;
+        int g = 0, commits = 0;
+        int v_free0 = -1, v_free1 = -1;
+        unsigned tails = 0;
+        bool alive = true, tail_pending = false;   // tail_pending: the tail tile's copy was issued and v_tail not yet seen complete
+        int last_g[2] = {-1, -1};              // the last two steps whose V tile arrives on step_full by a copy: before last, last
+        for (unsigned it = 0;; ++it) {
+            alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.item_full[it & 1u], (it >> 1) & 1u, a, 7));
+            if (!alive) break;
+            const Item w = sm.item[it & 1u];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.item_empty[it & 1u]);
+            if (!w.some) break;
+            const SeqExtent& sq = w.sq;
+            const int n_max = max(w.t[0].n_kv, w.t[1].n_kv);
+            if (n_max <= 0) continue;
             // The sequence's last V tile, when the sequence does not end on a tile boundary, holds rows
             // that are not this sequence's: the unwritten rest of its last page, or the next sequence
             // of a packed buffer. P is exactly zero there, but 0 x NaN (an uninitialised pool, a page
@@ -911,94 +1105,136 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             // cleared in shared memory before the tile is handed to the MMA issuer: its copy completes
             // on a barrier of its own, the producer warp zeroes the rows and then completes the
             // ring's barrier with a plain arrival. (Garbage in K is harmless: the score mask is a select.)
-            const bool tail_fix = is_v && (a.paged || packed) && (sq.kv_len % kBlockN) != 0;
+            const bool tail_fix = (a.paged || packed) && (sq.kv_len % kBlockN) != 0;
             const int tail_j = sq.kv_len > 0 ? (sq.kv_len - 1) / kBlockN : -1;
-            bool tail_pending = false;   // the tail tile's copy was issued and v_tail not yet seen complete
-            int issued = is_v ? v_issued : n_pre;   // tiles that were requested during set-up
-            // (the K producer goes one past the last tile: the last step's barrier wants its arrival too)
-            for (int j = issued; j < n_max + (is_v ? 0 : 1) && alive; ++j) {
-                if (!is_v && j == 0) break;   // no tile at all
-                const int s = j % kStages;
-                const int page = kPaged && j < n_max ? page_of_lane(a, sq.kv_len, b, j, lane) : -1;
-                if (j >= kStages) {   // the stage's tile: V(j - 2) was last read in step j - 2, K(j - 2) by the S of step j - 3
-                    const int e = is_v ? j - 1 : j - 2;
-                    alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.step_done[e & 1], (unsigned)(e >> 1) & 1u, a, is_v ? 2 : 1));
-                    if (!alive) break;
-                }
-                if (j == n_max) {
-                    if (lane == 0) mbar_arrive(full_of(j));
-                    break;
-                }
+            int page = kPaged ? page_of_lane(a, sq.kv_len, w.seq, 0, lane) : -1;
+            for (int j = 0; j < n_max; ++j) {
+                const int e = (g + j) & 1;
+                const int c = e ? v_free1 : v_free0;
+                if (c >= 0) alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.step_done[c & (kDone - 1)], (unsigned)(c / kDone) & 1u, a, 2));
+                if (!alive) break;
                 const bool fix = tail_fix && j == tail_j;
-                unsigned long long* const bar = fix ? &sm.v_tail : full_of(j);
-                if (!is_v && a.test_skip_k == j + 1) {
-                    // test hook: this tile is never requested, the issuer's wait for it runs out
-                } else if (kv_edge(j)) {
-                    edge_tile_copy<D>(ring[s], kv_base, a.kv_heads, kvh, (long long)sq.kv_crow + (long long)j * kBlockN, tot_k, bar, lane, a.d_real);
-                } else if (kPaged || lane == 0) {
-                    load_kv_tile<D, kPaged>(a, sq, kvh, ring[s], map, bar, j, page, lane);
+                unsigned long long* const bar = fix ? &sm.v_tail : &sm.step_full[e];
+                if (kv_open && (long long)sq.kv_crow + (long long)(j + 1) * kBlockN > tot_k)
+                    edge_tile_copy<D>(sm.v[e], a.v, a.kv_heads, w.kv_head, (long long)sq.kv_crow + (long long)j * kBlockN, tot_k, bar, lane, a.d_real);
+                else if (kPaged || lane == 0)
+                    load_kv_tile<D, kPaged>(a, sq.kv_crow, sq.kv_cb, w.kv_head, sm.v[e], &v_map, bar, j, page, lane);
+                (e ? v_free1 : v_free0) = commits + j + 1;
+                if (kPaged && j + 1 < n_max) page = page_of_lane(a, sq.kv_len, w.seq, j + 1, lane);
+                if (!fix) {
+                    last_g[0] = last_g[1];
+                    last_g[1] = g + j;
+                    continue;
                 }
-                issued = j + 1;
-                if (fix) {
-                    tail_pending = true;
-                    alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.v_tail, 0u, a, 4));
-                    if (!alive) break;
-                    tail_pending = false;
-                    const int first = sq.kv_len - j * kBlockN;   // first row of the tile that is not this sequence's
-                    constexpr int kChunksPerHalfRow = 8;        // 128 B per row and 64-column half
-                    const int n_chunks = (kBlockN - first) * kChunksPerHalfRow;
-                    for (int h = 0; h < D / 64; ++h)
-                        for (int idx = lane; idx < n_chunks; idx += 32)
-                            *reinterpret_cast<uint4*>(ring[s] + h * kHalfBytes + first * 128 + idx * 16) = make_uint4(0u, 0u, 0u, 0u);
-                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // generic-proxy writes -> tensor-core reads
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(full_of(j));
-                }
+                tail_pending = true;
+                alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.v_tail, tails & 1u, a, 4));
+                if (!alive) break;
+                tail_pending = false;
+                ++tails;
+                const int first = sq.kv_len - j * kBlockN;   // first row of the tile that is not this sequence's
+                constexpr int kChunksPerHalfRow = 8;        // 128 B per row and 64-column half
+                const int n_chunks = (kBlockN - first) * kChunksPerHalfRow;
+                for (int h = 0; h < D / 64; ++h)
+                    for (int idx = lane; idx < n_chunks; idx += 32)
+                        *reinterpret_cast<uint4*>(sm.v[e] + h * kHalfBytes + first * 128 + idx * 16) = make_uint4(0u, 0u, 0u, 0u);
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // generic-proxy writes -> tensor-core reads
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.step_full[e]);
             }
-            // Make sure none of this warp's copies is still in flight when the CTA exits: wait
-            // (bounded) for the last fill of every stage (and of the Q tiles). These waits ignore the
-            // abort flag: they only depend on the copy engine.
-            if (lane == 0) {
-                if (!is_v) {
-                    if (t0.n_kv > 0) mbar_wait(sm, &sm.q_full[0], 0, a, 3);
-                    if (t1.n_kv > 0) mbar_wait(sm, &sm.q_full[1], 0, a, 3);
-                }
-                const unsigned long long t_begin = global_timer_ns();
-                // (K: where the loop went one past the last tile, the tile before the last has been read, and its barrier used again)
-                for (int last = max(0, issued - (!is_v && alive ? 1 : kStages)); last < issued; ++last) {
-                    if (!is_v && a.test_skip_k == last + 1) continue;          // test hook: never requested
-                    if (tail_fix && last == tail_j) {
-                        // that tile's copy completes on v_tail; the ring's barrier got (or, after an abort, never gets) a plain arrival
-                        while (tail_pending && !mbar_try_wait(&sm.v_tail, 0u) && global_timer_ns() - t_begin < 100000000ULL) {}
-                        continue;
-                    }
-                    // (after an abort the other ring's arrival may be missing; the copies have landed long before the limit then)
-                    while (!mbar_try_wait(full_of(last), full_parity(last)) && global_timer_ns() - t_begin < 100000000ULL) {}
-                }
-            }
+            if (!alive) break;
+            commits += n_max + 1;
+            g += n_max;
+        }
+        if (lane == 0 && !alive) {   // (else every V tile has been read; the waits as at the end of the K producer)
+            const unsigned long long t_begin = global_timer_ns();
+            while (tail_pending && !mbar_try_wait(&sm.v_tail, tails & 1u) && global_timer_ns() - t_begin < 100000000ULL) {}
+            for (int i = 0; i < 2; ++i)
+                if (last_g[i] >= 0)
+                    while (!mbar_try_wait(&sm.step_full[last_g[i] & 1], (unsigned)(last_g[i] >> 1) & 1u) && global_timer_ns() - t_begin < 100000000ULL) {}
         }
     } else if (warp == kMmaWarp) {
-        issue_products<T, D>(smem_u32(&sm), tmem, t0.n_kv, t1.n_kv, a.status, a.wait_ns FA_TRACE_ARG(trace));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(&sm.tmem_base)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+        tc_fence_before();
+        asm volatile("barrier.cta.sync 2, 320;\n" ::: "memory");
+        tc_fence_after();
+#ifdef FA_TRACE
+        // only the heaviest CTA of the first (batch, KV head) records its timeline, one thread per role
+        long long* const trace = (a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == (unsigned)a.trace_y && blockIdx.z == 0 && lane == 0) ? a.trace : nullptr;
+        // slot kTraceSteps - 1 of each role holds the CTA's life cycle instead of a kv step
+        if (trace != nullptr) {
+            trace[(2 * kTraceSteps + kTraceSteps - 1) * 8 + 0] = t_entry;
+            FA_TRACE_EVENT(2, kTraceSteps - 1, 1);   // set-up (barriers, tensor memory) done
+        }
+#endif
+        issue_products<T, D>(smem_u32(&sm), sm.tmem_base, a.status, a.wait_ns FA_TRACE_ARG(trace));
+    } else {
+        // ------------------------------ set-up ------------------------------
+        // (by the warp that has nothing else to do, while the K producer finds out what the CTA's first tile pair is)
+        if (lane == 0) {
+            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&q_map) : "memory");
+            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&k_map) : "memory");
+            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&v_map) : "memory");
+            sm.abort_flag = 0;
+            for (int i = 0; i < 2; ++i) {
+                mbar_init(&sm.item_full[i], 1);
+                mbar_init(&sm.item_empty[i], 10);
+                mbar_init(&sm.q_full[i], 1);
+                mbar_init(&sm.s_full[i], 1);
+                mbar_init(&sm.o_full[i], 1);
+                mbar_init(&sm.p_ready[0][i], 128);
+                mbar_init(&sm.p_ready[1][i], 128);
+                mbar_init(&sm.step_full[i], 2);
+            }
+            for (int i = 0; i < kDone; ++i) mbar_init(&sm.step_done[i], 1);
+            mbar_init(&sm.answered, 1);
+            mbar_init(&sm.k_first, 1);
+            mbar_init(&sm.v_tail, 1);
+            mbar_init(&sm.drain, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        }
+        __syncwarp();
+        asm volatile("barrier.cta.arrive 1, 96;\n" ::: "memory");    // the producers
+        asm volatile("barrier.cta.arrive 2, 320;\n" ::: "memory");   // issuer and softmax warps, which wait for tensor memory as well
     }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 208;\n");
         // ------------------------------ softmax warpgroups ------------------------------
+        asm volatile("barrier.cta.sync 2, 320;\n" ::: "memory");   // barriers and tensor memory
+        tc_fence_after();
+        const unsigned tmem = sm.tmem_base;
         const int t = warp >> 2;
-        const TileInfo ti = t == 0 ? t0 : t1;
         const int r = (warp & 3) * 32 + lane;                  // row within the tile == TMEM lane
         const unsigned lane_base = (unsigned)((warp & 3) * 32) << 16;
         const unsigned s_addr = tmem + lane_base + t * 128;
         const unsigned o_addr = tmem + lane_base + 256 + t * 128;
+        unsigned steps = 0, tiles = 0;    // of this query tile so far: steps, and tiles with a step
+        bool alive = true;
+#ifdef FA_TRACE
+        long long* trace = (a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == (unsigned)a.trace_y && blockIdx.z == 0 && lane == 0 && (warp & 3) == 0) ? a.trace : nullptr;
+#endif
+#pragma unroll 1
+        for (unsigned it = 0; alive; ++it) {
+        alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.item_full[it & 1u], (it >> 1) & 1u, a, 22 + t));
+        if (!alive) break;
+        const bool some = sm.item[it & 1u].some != 0;
+        const int b = sm.item[it & 1u].seq;
+        const SeqExtent sq = sm.item[it & 1u].sq;
+        const TileInfo ti = sm.item[it & 1u].t[t];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.item_empty[it & 1u]);
+        if (!some) break;
         const int row = ti.row0 + r;
         const long long pos = (long long)sq.pos_off + row;      // global position of this query row
         float m = -INFINITY;   // reference max, log2 domain (may lag the true max by <= 2^8)
         float l = 0.0f;
-        bool alive = true;
 
         for (int j = 0; j < ti.n_kv && alive; ++j) {
-            alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.s_full[t], (unsigned)j & 1u, a, 20 + t));
+            alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.s_full[t], steps & 1u, a, 20 + t));
             if (!alive) break;
-            FA_TRACE_EVENT(t, j, 0);
+            ++steps;
+            FA_TRACE_EVENT(t, (int)steps - 1, 0);
             tc_fence_after();
             const int key0 = j * kBlockN;
             // mask only where the causal diagonal or the end of K/V cuts through this tile
@@ -1046,7 +1282,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             // A row that sees a NaN outputs NaN whichever unit takes that key's exponential: its maximum is NaN, and with it the reference below, every
             // exponential of the tile and the row's sum from here on. A +inf stays the reference to the end, where the epilogue sees it.
             const float mx = max_nan(max3_nan(mx4[0], mx4[1], mx4[2]), mx4[3]) * a.scale_log2;   // scale > 0 is guaranteed by the dispatcher
-            FA_TRACE_EVENT(t, j, 1);
+            FA_TRACE_EVENT(t, (int)steps - 1, 1);
 
             float alpha = 1.0f;
             bool changed = false;
@@ -1095,17 +1331,18 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 tc_wait_st();
                 tc_fence_before();
                 mbar_arrive(&sm.p_ready[h][t]);
-                if (h == 0) FA_TRACE_EVENT(t, j, 2);
+                if (h == 0) FA_TRACE_EVENT(t, (int)steps - 1, 2);
             }
             float sum_lo, sum_hi;
             unpack2(sum2, sum_lo, sum_hi);
             l = l * alpha + (sum_lo + sum_hi);
-            FA_TRACE_EVENT(t, j, 3);
+            FA_TRACE_EVENT(t, (int)steps - 1, 3);
         }
 
         // epilogue: O_t is final once the commit after the last P.V has arrived
         if (alive && ti.n_kv > 0)
-            alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.s_full[t], (unsigned)ti.n_kv & 1u, a, 30 + t));
+            alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.o_full[t], tiles++ & 1u, a, 30 + t));
+        FA_TRACE_EVENT(t, max(0, (int)steps - 1), 4);
         if (alive && ti.valid) {
             tc_fence_after();
             const bool row_ok = row < sq.q_len;
@@ -1116,23 +1353,22 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             const float inv = seen ? 1.0f / l : 0.0f;
             // a bulk store writes every row of its box that lies inside the tensor: in a packed buffer the
             // rows after this sequence belong to the next one, so a tile that overhangs the end of its
-            // sequence takes the row-guarded path
+            // sequence is written row by row
 #ifdef FA_TRACE
             const bool staged_only = a.staged_store != 0;
 #else
             constexpr bool staged_only = false;
 #endif
+            unsigned char* const stage = sm.out[warp];
             const bool bulk_ok = a.n_out == 1 && !a.multicast && !staged_only && (a.mode != MODE_VARLEN || ti.row0 + kBlockM <= sq.q_len);
             if (bulk_ok) {
                 // Single output: the rows go out as bulk tensor stores. Each warp lays its 32 rows down in
-                // the Q tile's shared memory (every MMA that read Q_t has finished) in the 128-byte-swizzled
-                // box layout and one lane issues one store of 32 rows x 64 columns per half. Plain 16-byte stores
+                // shared memory in the 128-byte-swizzled box layout, 64 columns at a time, and one lane issues one store of 32 rows x 64 columns. Plain 16-byte stores
                 // of 32 different rows per instruction would fill the SM's memory pipeline for thousands
                 // of clocks and hold up the barrier traffic of the other tile's last steps. Rows past the
                 // end of the sequence are outside the tensor map and are not written.
-                unsigned char* stage = sm.q[t];
 #pragma unroll 1
-                for (int h = 0; h < D / 64; ++h) {   // a half's copy is on its way while the next one is packed
+                for (int h = 0; h < D / 64; ++h) {   // a half's copy is on its way while the next one is read and scaled
                     float ov[2][32];
                     tc_ld32(o_addr + h * 64, ov[0]);
                     tc_ld32(o_addr + h * 64 + 32, ov[1]);
@@ -1141,6 +1377,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 #pragma unroll
                         for (int i = 0; i < 32; ++i) ov[0][i] = ov[1][i] = 0.0f;
                     }
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // what was laid down here before has been read
+                    __syncwarp();
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {   // 16-byte chunk i of the 64-column half
                         const float* o8 = &ov[i >> 2][8 * (i & 3)];
@@ -1149,23 +1387,43 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                         w.y = pack16<T>(o8[2] * inv, o8[3] * inv);
                         w.z = pack16<T>(o8[4] * inv, o8[5] * inv);
                         w.w = pack16<T>(o8[6] * inv, o8[7] * inv);
-                        *reinterpret_cast<uint4*>(stage + h * kHalfBytes + r * 128 + ((i ^ (r & 7)) << 4)) = w;
+                        *reinterpret_cast<uint4*>(stage + lane * 128 + ((i ^ (lane & 7)) << 4)) = w;
                     }
                     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // generic-proxy writes -> bulk copy reads
                     __syncwarp();
                     if (lane == 0) {
-                        const int warp_row0 = (warp & 3) * 32;
-                        tma_store_4d(&o_map, stage + h * kHalfBytes + warp_row0 * 128, h * 64, a.o_head0 + ti.head, sq.q_crow + ti.row0 + warp_row0, sq.q_cb);
+                        tma_store_4d(&o_map, stage, h * 64, a.o_head0 + ti.head, sq.q_crow + ti.row0 + (warp & 3) * 32, sq.q_cb);
                         asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
                     }
                 }
+            } else if (a.n_out == 1 && !a.multicast && !staged_only) {
+                // A tile that overhangs its sequence: the rows that exist, from registers in 32-byte stores (whole sectors).
+#pragma unroll 1
+                for (int c = 0; c < D / 32; ++c) {
+                    float ov[32];
+                    tc_ld32(o_addr + c * 32, ov);
+                    tc_wait_ld();
+                    T* const to = static_cast<T*>(a.o[0]) + ((sq.o_row0 + row) * a.o_heads + a.o_head0 + ti.head) * a.d_real + c * 32;
+                    if (row_ok && c * 32 < a.d_real) {
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            unsigned w[8];
+#pragma unroll
+                            for (int x = 0; x < 8; ++x) w[x] = ti.n_kv == 0 ? 0u : pack16<T>(ov[16 * i + 2 * x] * inv, ov[16 * i + 2 * x + 1] * inv);
+                            store_32(to + i * 16, w, a.o_by_32 != 0);
+                        }
+                    }
+                }
             } else {
-                // Stage this warp's 32 rows (2 D bytes each) in the Q tile's shared memory — every MMA that read
-                // Q_t has finished — so that the global stores are whole rows: D / 8 lanes x 16 B contiguous,
+                // Several GPUs' buffers: this warp's rows (2 D bytes each, 16 at a time at D = 128) through shared memory, so that the global stores are whole rows: D / 8 lanes x 16 B contiguous,
                 // 256 / D rows per instruction. That matters most for the peer copies, which cross NVLink.
                 constexpr int kRowBytes = D * 2;
                 constexpr int kChunks = D / 8;          // 16-byte chunks per row
-                unsigned char* stage = sm.q[t];
+                constexpr int kRowsAtOnce = kOutBytes / kRowBytes;
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // (an earlier tile's bulk stores)
+                __syncwarp();
+    #pragma unroll 1
+                for (int part = 0; part < 32 / kRowsAtOnce; ++part) {
     #pragma unroll 1
                 for (int c = 0; c < D / 32; ++c) {
                     float ov[32];
@@ -1175,6 +1433,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     #pragma unroll
                         for (int i = 0; i < 32; ++i) ov[i] = 0.0f;
                     }
+                    if (lane / kRowsAtOnce != part) continue;
+                    const int rr = lane % kRowsAtOnce;
     #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         uint4 w;
@@ -1183,7 +1443,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                         w.z = pack16<T>(ov[8 * i + 4] * inv, ov[8 * i + 5] * inv);
                         w.w = pack16<T>(ov[8 * i + 6] * inv, ov[8 * i + 7] * inv);
                         const int ch = c * 4 + i;   // 16-byte chunk of the row, XOR-swizzled against bank conflicts
-                        *reinterpret_cast<uint4*>(stage + r * kRowBytes + ((ch ^ (r & (kChunks - 1))) << 4)) = w;
+                        *reinterpret_cast<uint4*>(stage + rr * kRowBytes + ((ch ^ (rr & (kChunks - 1))) << 4)) = w;
                     }
                 }
                 __syncwarp();
@@ -1191,11 +1451,11 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     const int ch = lane & (kChunks - 1);
                     const int sub = lane / kChunks;
                     constexpr int kRowsPerStep = 32 / kChunks;
-                    const int warp_row0 = (warp & 3) * 32;
+                    const int part_row0 = ti.row0 + (warp & 3) * 32 + part * kRowsAtOnce;
     #pragma unroll 4
-                    for (int it = 0; it < 32 / kRowsPerStep; ++it) {
-                        const int rr = warp_row0 + it * kRowsPerStep + sub;
-                        const int grow = ti.row0 + rr;
+                    for (int n = 0; n < kRowsAtOnce / kRowsPerStep; ++n) {
+                        const int rr = n * kRowsPerStep + sub;
+                        const int grow = part_row0 + rr;
                         if (grow < sq.q_len && ch * 8 < a.d_real) {
                             const uint4 w = *reinterpret_cast<const uint4*>(stage + rr * kRowBytes + ((ch ^ (rr & (kChunks - 1))) << 4));
                             const long long o_off = ((sq.o_row0 + grow) * a.o_heads + a.o_head0 + ti.head) * a.d_real + ch * 8;
@@ -1206,13 +1466,15 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                                 multimem_st16(static_cast<T*>(a.o[0]) + o_off, w);
                             } else {
                                 int pe = a.peer0;
-                                for (int n = 0; n < a.n_out; ++n) {
+                                for (int n_pe = 0; n_pe < a.n_out; ++n_pe) {
                                     *reinterpret_cast<uint4*>(static_cast<T*>(a.o[pe]) + o_off) = w;
                                     pe = pe + 1 == a.n_out ? 0 : pe + 1;
                                 }
                             }
                         }
                     }
+                }
+                __syncwarp();   // the rows are written again by the next part
                 }
             }
             if (row_ok && (a.lse != nullptr || a.n_lse > 0)) {
@@ -1222,17 +1484,17 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 const long long g_off = ((long long)b * a.o_heads + a.o_head0 + ti.head) * a.q_seq_len + row;
                 for (int n = 0; n < a.n_lse; ++n) a.lse_peers[n][g_off] = lse_val;
             }
-            if (bulk_ok && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // shared memory stays valid until read
-            FA_TRACE_EVENT(t, kTraceSteps - 1, 0);       // epilogue stores issued
+            FA_TRACE_EVENT(t, max(0, (int)steps - 1), 5);       // epilogue stores issued
         }
+        }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // shared memory stays valid until read
     }
 
     tc_fence_before();
     __syncthreads();
-    FA_TRACE_EVENT(2, kTraceSteps - 1, 3);               // every role done
     if (warp == kMmaWarp) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(sm.tmem_base) : "memory");
     }
 #ifdef FA_TRACE
     if (a.cta_log != nullptr && threadIdx.x == 0) {
@@ -1269,10 +1531,10 @@ EncodeFn get_encode_fn() {
     return fn;
 }
 
-// (batch, seq, heads, 128) 16-bit tensor viewed as 4-D {d, head, seq, batch}; box = 64 x 1 x 128 x 1
+// (batch, seq, heads, 128) 16-bit tensor viewed as 4-D {d, head, seq, batch}; box = 64 x 1 x 128 x 1 (out: 64 x 1 x 32 x 1, what a softmax warp lays down at a time)
 // seq <= 0: a packed buffer whose row count the caller did not give (batch is 1 then). The row extent is
 // set beyond any buffer and the kernel never asks for a box that reaches past the real last row.
-bool encode_map(CUtensorMap* map, const void* base, int dtype, int d, int batch, int seq, int heads, int box_rows = kBlockM) {
+bool encode_map(CUtensorMap* map, const void* base, int dtype, int d, int batch, int seq, int heads, bool out = false) {
     EncodeFn fn = get_encode_fn();
     if (fn == nullptr) return false;
     const bool unbounded = seq <= 0;
@@ -1281,7 +1543,7 @@ bool encode_map(CUtensorMap* map, const void* base, int dtype, int d, int batch,
     // the stride of the batch axis is never used when batch is 1; it only has to be a legal value
     const cuuint64_t strides[3] = {(cuuint64_t)d * 2, (cuuint64_t)heads * d * 2,
                                    unbounded ? (cuuint64_t)heads * d * 2 * 128 : (cuuint64_t)seq * heads * d * 2};
-    const cuuint32_t box[4] = {64, 1, (cuuint32_t)box_rows, 1};
+    const cuuint32_t box[4] = {64, 1, out ? 32u : (cuuint32_t)kBlockM, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUtensorMapDataType dt = dtype == DT_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     const CUresult rc = fn(map, dt, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1364,11 +1626,11 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     // boxes read zeros past it and bulk stores write nothing there
     const int d_real = p.head_size;
     bool ok = encode_map(&qm, p.q, p.dtype, d_real, q_batch, q_rows, p.q_heads);
-    // The output as 32-row boxes (one per softmax warp). Bulk stores are used for a single, local output
+    // The output as boxes of 32 rows. Bulk stores are used for a single, local output
     // only: a head-sharded call (n_out > 0) stores every copy with plain stores, and no tensor map is
     // ever made over another GPU's memory — the kernel's fourth map is then a second one over q, unused.
     if (p.n_out > 0) om = qm;
-    else ok = ok && encode_map(&om, p.o, p.dtype, d_real, q_batch, q_rows, p.q_heads, 32);
+    else ok = ok && encode_map(&om, p.o, p.dtype, d_real, q_batch, q_rows, p.q_heads, true);
     if (p.paged) {
         ok = ok && encode_paged_map(&km, p.k, p.dtype, d_real, p.block_size, p.kv_heads) &&
              encode_paged_map(&vm, p.v, p.dtype, d_real, p.block_size, p.kv_heads);
@@ -1394,6 +1656,7 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
         a.multicast = p.multicast;
     } else {
         a.o[0] = p.o;
+        a.o_by_32 = (reinterpret_cast<uintptr_t>(p.o) & 31) == 0;
         a.n_out = 1;
         a.o_heads = p.q_heads;
         a.o_head0 = 0;
