@@ -789,7 +789,7 @@ __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int
             if (D == 64) {
                 // Two tiles that start together stay together, in each other's way at the exponentials (2900 clocks a step); near half a step apart they stay
                 // so as well and take 2570. Where the pair has the steps to win the delay back.
-                if (t == 1 && n0 >= 4)
+                if (t == 1 && n0 >= 6)
                     while ((unsigned)clock64() - s0_at < kApart) {}
                 s0_at = (unsigned)clock64();
             }
@@ -905,7 +905,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     // producer/issuer warpgroup hands most of its share to the two softmax warpgroups, which
     // keep a whole 128-column score row per thread in registers.
     if (warp >= 8) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n");
+    if (warp != kLoadWarp) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n");
     if (warp == kLoadWarp) {
         // ------------------------------ tile pairs, Q and K tiles ------------------------------
         // The warps run their loops whole; lane 0 issues the bulk copies (a paged tile: a lane per page), and all lanes share the
@@ -920,7 +920,29 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         int first_s = -1;                    // the commit of the last pair's first S, where that pair had one step (else it has been waited for)
         int k_asked = 0, n_before = 0;       // K tiles of this pair that have been requested; tiles of the pair before
         unsigned q_loads0 = 0, q_loads1 = 0, pairs = 0, requests = 0, answers = 0;
-        bool alive = true, own = true;
+        bool alive = true;
+        // The CTA's own tile pair, and its first copies at once, in as few instructions as that takes: all of them come in for the first time here, and
+        // in the loop below, with its waits and cases, the first S came 1600 to 2300 clocks later (a fifth of a call of one short wave).
+        Item w;
+        w.some = find_pair<kPaged>(a, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, lane, w);
+        asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
+        const bool begun = w.some && max(w.t[0].n_kv, w.t[1].n_kv) > 0 && !q_open && !kv_open && a.test_skip_k != 1;
+        if (begun && (kPaged || lane == 0)) {
+            const int page = kPaged ? page_of_lane(a, w.sq.kv_len, w.seq, 0, lane) : -1;
+            if (lane == 0 && w.t[0].n_kv > 0) {
+                mbar_expect_tx(&sm.q_full[0], TileBytes<D>::value);
+                tma_load_4d(sm.q[0], &q_map, &sm.q_full[0], 0, w.t[0].head, w.sq.q_crow + w.t[0].row0, w.sq.q_cb);
+                if (D == 128) tma_load_4d(sm.q[0] + kHalfBytes, &q_map, &sm.q_full[0], 64, w.t[0].head, w.sq.q_crow + w.t[0].row0, w.sq.q_cb);
+            }
+            load_kv_tile<D, kPaged>(a, w.sq.kv_crow, w.sq.kv_cb, w.kv_head, sm.k[0], &k_map, &sm.k_first, 0, page, lane);
+            if (lane == 0 && w.t[1].n_kv > 0) {
+                mbar_expect_tx(&sm.q_full[1], TileBytes<D>::value);
+                tma_load_4d(sm.q[1], &q_map, &sm.q_full[1], 0, w.t[1].head, w.sq.q_crow + w.t[1].row0, w.sq.q_cb);
+                if (D == 128) tma_load_4d(sm.q[1] + kHalfBytes, &q_map, &sm.q_full[1], 64, w.t[1].head, w.sq.q_crow + w.t[1].row0, w.sq.q_cb);
+            }
+        }
+        __syncwarp();
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n");
 #ifdef FA_TRACE
         long long* const trace = (a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == (unsigned)a.trace_y && blockIdx.z == 0 && lane == 0) ? a.trace : nullptr;
 #endif
@@ -948,28 +970,25 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             // last K tile requested, two to three steps before its end: whoever comes to its end first takes the next one. Asked for at a
             // pair's beginning, the order heaviest first was lost for the second half of 4 chunks of 512 (256 pairs on 148 SMs): 174 us instead of
             // 153. The answer takes 1100 to 3100 clocks, what follows from it until the first copy 2000 more.
-            if (!own && requests == answers) ask();
-            Item w;
+            if (it > 0 || !w.some) {
             w.some = 0;
+            if (requests == answers) ask();
             if (it >= 2) alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.item_empty[it & 1u], ((it >> 1) - 1u) & 1u, a, 5));
             while (alive) {
-                int bx = (int)blockIdx.x, by = (int)blockIdx.y, bz = (int)blockIdx.z;
-                if (!own) {
-                    alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.answered, answers & 1u, a, 6));
-                    if (!alive) break;
-                    ++answers;
-                    FA_TRACE_EVENT(3, (int)answers, 1);
-                    const bool got = read_answer(sm.answer, bx, by, bz);
-                    __syncwarp();
-                    if (!got) break;   // every tile pair is taken
-                }
+                int bx, by, bz;
+                alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.answered, answers & 1u, a, 6));
+                if (!alive) break;
+                ++answers;
+                FA_TRACE_EVENT(3, (int)answers, 1);
+                const bool got = read_answer(sm.answer, bx, by, bz);
+                __syncwarp();
+                if (!got) break;   // every tile pair is taken
                 w.some = find_pair<kPaged>(a, bx, by, bz, lane, w);
-                if (own) asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
-                own = false;
                 if (w.some) break;
                 ask();
             }
             if (!alive) break;
+            }
             if (!w.some) w.t[0].n_kv = w.t[1].n_kv = 0;
             if (lane == 0) {
                 sm.item[it & 1u] = w;
@@ -1025,20 +1044,31 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 }
             };
             k_asked = 0;
-            alive = wait_commit(first_s) &&   // the last pair's K tile 0 has left its barrier
-                    wait_commit((g & 1) ? k_free1 : k_free0);
-            if (!alive) break;
-            load_k(0);
-            FA_TRACE_EVENT(3, (int)it, 3);
-            // (the first pair's tile 0 first, whose products are; else the one that comes free first, of two row blocks of one head the shorter one, tile 1)
+            // K tile 0 and the Q tiles: of the first pair in the order that the issuer wants them; else K first, which comes free first, then the Q tile that does, of
+            // two row blocks of one head the shorter one, tile 1.
             auto wait_q = [&](int t, unsigned scores) { return __all_sync(0xffffffffu, mbar_wait(sm, &sm.s_full[t], (scores - 1u) & 1u, a, 8)); };
+            if (it == 0 && begun) {
+                k_free0 = 0;
+                k_asked = 1;
+                q_loads0 = n0 > 0;
+                q_loads1 = n1 > 0;
+                if (kPaged && n_max > 1) page = page_of_lane(a, kv_len, seq, 1, lane);
+            } else
 #pragma unroll 1
-            for (int n = 0; n < 2; ++n) {
-                const int t = it == 0 ? n : n ^ 1;
-                if (t ? q_used1 : q_used0) alive = wait_q(t, t ? scores1 : scores0);
-                if (!alive) break;
-                load_q(t ? w.t[1] : w.t[0], sm.q[t], &sm.q_full[t], t ? q_loads1 : q_loads0);
-                FA_TRACE_EVENT(3, (int)it, 4 + t);
+            for (int n = 0; n < 3; ++n) {
+                if (n == (it == 0 ? 1 : 0)) {
+                    alive = wait_commit(first_s) &&   // the last pair's K tile 0 has left its barrier
+                            wait_commit((g & 1) ? k_free1 : k_free0);
+                    if (!alive) break;
+                    load_k(0);
+                    FA_TRACE_EVENT(3, (int)it, 3);
+                } else {
+                    const int t = it == 0 ? n >> 1 : 2 - n;
+                    if (t ? q_used1 : q_used0) alive = wait_q(t, t ? scores1 : scores0);
+                    if (!alive) break;
+                    load_q(t ? w.t[1] : w.t[0], sm.q[t], &sm.q_full[t], t ? q_loads1 : q_loads0);
+                    FA_TRACE_EVENT(3, (int)it, 4 + t);
+                }
             }
             if (!alive) break;
             for (int j = 1; j < n_max; ++j) {
@@ -1367,8 +1397,11 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 // of 32 different rows per instruction would fill the SM's memory pipeline for thousands
                 // of clocks and hold up the barrier traffic of the other tile's last steps. Rows past the
                 // end of the sequence are outside the tensor map and are not written.
+                // Where no tile pair follows, the second half goes through the Q tile's shared memory and need not wait until the first has been read (0.4 us).
+                const bool last = D == 128 && __all_sync(0xffffffffu, mbar_test_at(smem_u32(&sm.item_full[(it + 1u) & 1u]), ((it + 1u) >> 1) & 1u) && sm.item[(it + 1u) & 1u].some == 0);
 #pragma unroll 1
                 for (int h = 0; h < D / 64; ++h) {   // a half's copy is on its way while the next one is read and scaled
+                    unsigned char* const half = h > 0 && last ? sm.q[t] + (warp & 3) * kOutBytes : stage;
                     float ov[2][32];
                     tc_ld32(o_addr + h * 64, ov[0]);
                     tc_ld32(o_addr + h * 64 + 32, ov[1]);
@@ -1377,7 +1410,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 #pragma unroll
                         for (int i = 0; i < 32; ++i) ov[0][i] = ov[1][i] = 0.0f;
                     }
-                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // what was laid down here before has been read
+                    if (lane == 0 && !(h > 0 && last)) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // what was laid down here before has been read
                     __syncwarp();
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {   // 16-byte chunk i of the 64-column half
@@ -1387,12 +1420,12 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                         w.y = pack16<T>(o8[2] * inv, o8[3] * inv);
                         w.z = pack16<T>(o8[4] * inv, o8[5] * inv);
                         w.w = pack16<T>(o8[6] * inv, o8[7] * inv);
-                        *reinterpret_cast<uint4*>(stage + lane * 128 + ((i ^ (lane & 7)) << 4)) = w;
+                        *reinterpret_cast<uint4*>(half + lane * 128 + ((i ^ (lane & 7)) << 4)) = w;
                     }
                     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // generic-proxy writes -> bulk copy reads
                     __syncwarp();
                     if (lane == 0) {
-                        tma_store_4d(&o_map, stage, h * 64, a.o_head0 + ti.head, sq.q_crow + ti.row0 + (warp & 3) * 32, sq.q_cb);
+                        tma_store_4d(&o_map, half, h * 64, a.o_head0 + ti.head, sq.q_crow + ti.row0 + (warp & 3) * 32, sq.q_cb);
                         asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
                     }
                 }

@@ -61,3 +61,19 @@ def test_rows_of_a_batch_are_those_of_each_element_alone(b, s, hq, hkv, d):
                 low.flash_attn(q[i:i + 1, :, h * per:(h + 1) * per].contiguous(), k[i:i + 1, :, h:h + 1].contiguous(), v[i:i + 1, :, h:h + 1].contiguous(), o1, 1, s, s, per, 1, d, 0,
                                1.0 / np.sqrt(d), None if m is None else m[i:i + 1], None, l1)
                 assert torch.equal(o1, o[i:i + 1, :, h * per:(h + 1) * per]) and torch.equal(l1, lse[i:i + 1, h * per:(h + 1) * per])
+
+
+@pytest.mark.parametrize("d", [128, 64])
+def test_rows_to_several_buffers(d):
+    # the head-sharded epilogue with two buffers of this GPU: a shard's heads in both, the others' left alone
+    b, s, hq, hkv, first, total = 2, 700, 16, 4, 8, 32
+    g = torch.Generator(device="cuda").manual_seed(d)
+    q, k, v = (torch.randn((b, s, h, d), generator=g, device="cuda", dtype=torch.bfloat16) for h in (hq, hkv, hkv))
+    outs = [torch.full((b, s, total, d), -7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    low.flash_attn_allgather(q, k, v, [x.data_ptr() for x in outs], total, first, b, s, s, hq, hkv, d, 0, 1.0 / np.sqrt(d))
+    torch.cuda.synchronize()
+    want = high.flash_attn_func(q, k, v)
+    for x in outs:
+        assert torch.equal(x[:, :, first:first + hq], want)
+        assert bool((x[:, :, :first] == -7.0).all()) and bool((x[:, :, first + hq:] == -7.0).all())
+    assert ffi.device_status() == 0
