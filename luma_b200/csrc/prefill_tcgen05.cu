@@ -121,6 +121,7 @@ struct SharedStorage {
     unsigned long long drain;       // MMA issuer, at its end: every product issued has finished
     unsigned int tmem_base;
     volatile int abort_flag;
+    int left_out;                   // test hook: 1 + the step whose K tile was never requested, 0: none
 };
 static_assert(sizeof(SharedStorage<128>) + 1024 <= 232448, "fits the shared memory of an SM");
 
@@ -270,6 +271,41 @@ __device__ __forceinline__ bool mbar_wait(Storage& sm, unsigned long long* bar, 
             }
         }
     }
+}
+
+// The end of a producer after an abort: none of its copies may be in flight when the CTA ends. These waits ignore the abort flag and depend on the copy engine
+// alone (bounded all the same). A step's barrier also wants the arrival of the other ring's producer, which may have given up before that step, so each of them
+// makes its arrivals for the two steps after its last one here. Two are enough: a stage is filled for step x once step x - 2 has finished, so neither ring is more
+// than two steps ahead. And no phase gets a third arrival, which the hardware would take for an error while bytes are missing: one per ring and step,
+// the one for step x when the phase of step x - 2 has been seen complete.
+//   given    : steps that have this ring's arrival, or a copy that brings it
+//   left_out : 1 + a step before them that the test hook left without, or 0
+//   single   : what else is on its way, two bits each from bit 0: whether, and the parity of its phase (answer, Q of tile 0 and 1, K tile 0, V tail)
+template <typename Storage>
+__device__ __noinline__ void settle_copies(Storage& sm, int given, int left_out, unsigned single) {
+    const unsigned long long begin = global_timer_ns();
+    auto landed = [&](unsigned long long* bar, unsigned parity) {
+#pragma unroll 1
+        while (!mbar_try_wait(bar, parity & 1u))
+            if (global_timer_ns() - begin >= 100000000ULL) return false;
+        return true;
+    };
+#pragma unroll 1
+    for (int i = 0; i < 5; ++i) {
+        unsigned long long* const bar = i == 0 ? &sm.answered : i < 3 ? &sm.q_full[i - 1] : i == 3 ? &sm.k_first : &sm.v_tail;
+        if ((single >> (2 * i)) & 1u) landed(bar, single >> (2 * i + 1));
+    }
+#pragma unroll 1
+    for (int i = left_out > 0 ? -1 : 0; i < 2; ++i) {
+        const int x = i < 0 ? left_out - 1 : given + i;
+        if (x < 2 || landed(&sm.step_full[x & 1], (unsigned)((x - 2) >> 1))) mbar_arrive(&sm.step_full[x & 1]);
+    }
+}
+
+// The end of a producer: false where its copies have to be looked after (above). As long as nobody gives up, every copy has landed when the issuer has come to its end.
+template <typename Storage>
+__device__ __forceinline__ bool all_read(Storage& sm, bool alive, const PrefillArgs& a, int where) {
+    return alive && mbar_wait(sm, &sm.drain, 0u, a, where) && !sm.abort_flag;   // (an issuer that gives up says so before it ends)
 }
 
 __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, unsigned long long* bar, int c0, int c1,
@@ -918,8 +954,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         unsigned scores0 = 0, scores1 = 0;   // S of each query tile so far: its Q is free when the last one has finished
         bool q_used0 = false, q_used1 = false;   // (and has to be waited for: by the pair before this one)
         int first_s = -1;                    // the commit of the last pair's first S, where that pair had one step (else it has been waited for)
-        int k_asked = 0, n_before = 0;       // K tiles of this pair that have been requested; tiles of the pair before
-        unsigned q_loads0 = 0, q_loads1 = 0, pairs = 0, requests = 0, answers = 0;
+        int given = 0;                       // steps whose K arrival has been made or comes with a copy that has been requested
+        unsigned q_loads0 = 0, q_loads1 = 0, firsts = 0, requests = 0, answers = 0;   // firsts: K tiles 0 that have been requested
         bool alive = true;
         // The CTA's own tile pair, and its first copies at once, in as few instructions as that takes: all of them come in for the first time here, and
         // in the loop below, with its waits and cases, the first S came 1600 to 2300 clocks later (a fifth of a call of one short wave).
@@ -963,6 +999,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 const int c = owed_commit();
                 if (c < 0 || __all_sync(0xffffffffu, mbar_test_at(smem_u32(&sm.step_done[c & (kDone - 1)]), (unsigned)(c / kDone) & 1u))) {
                     if (lane == 0) mbar_arrive(&sm.step_full[(g - 1) & 1]);
+                    given = g;
                     owed = false;
                 }
             }
@@ -999,6 +1036,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 alive = wait_commit(owed_commit());
                 if (!alive) break;
                 if (lane == 0) mbar_arrive(&sm.step_full[(g - 1) & 1]);
+                given = g;
                 owed = false;
             }
             if (!w.some) break;
@@ -1022,13 +1060,17 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             auto load_k = [&](int j) {   // K tile j of the pair is what step g + j - 1 reads besides its V tile, and arrives on its barrier (tile 0: on its own)
                 const int e = (g + j) & 1;
                 unsigned long long* const bar = j == 0 ? &sm.k_first : &sm.step_full[e ^ 1];
-                if (a.test_skip_k != j + 1) {   // (the test hook's tile is never requested, the issuer's wait for it runs out)
-                    if (kv_open && (long long)kv_crow + (long long)(j + 1) * kBlockN > tot_k)
-                        edge_tile_copy<D>(sm.k[e], a.k, a.kv_heads, kv_head, (long long)kv_crow + (long long)j * kBlockN, tot_k, bar, lane, a.d_real);
-                    else if (kPaged || lane == 0) load_kv_tile<D, kPaged>(a, kv_crow, kv_cb, kv_head, sm.k[e], &k_map, bar, j, page, lane);
+                const bool skip = a.test_skip_k == j + 1;   // (the test hook's tile is never requested, the issuer's wait for it runs out)
+                if (skip) {
+                    if (lane == 0) sm.left_out = j > 0 ? g + j : 0;
+                } else if (kv_open && (long long)kv_crow + (long long)(j + 1) * kBlockN > tot_k) {
+                    edge_tile_copy<D>(sm.k[e], a.k, a.kv_heads, kv_head, (long long)kv_crow + (long long)j * kBlockN, tot_k, bar, lane, a.d_real);
+                } else if (kPaged || lane == 0) {
+                    load_kv_tile<D, kPaged>(a, kv_crow, kv_cb, kv_head, sm.k[e], &k_map, bar, j, page, lane);
                 }
                 (e ? k_free1 : k_free0) = commits + j;
-                k_asked = j + 1;
+                if (j > 0) given = g + j;
+                else if (!skip) ++firsts;
                 if (kPaged && j + 1 < n_max) page = page_of_lane(a, kv_len, seq, j + 1, lane);
             };
             // (a tile that sees no key needs no Q: the issuer leaves it out)
@@ -1043,13 +1085,12 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     if (D == 128) tma_load_4d(to + kHalfBytes, &q_map, bar, 64, ti.head, w.sq.q_crow + ti.row0, w.sq.q_cb);
                 }
             };
-            k_asked = 0;
             // K tile 0 and the Q tiles: of the first pair in the order that the issuer wants them; else K first, which comes free first, then the Q tile that does, of
             // two row blocks of one head the shorter one, tile 1.
             auto wait_q = [&](int t, unsigned scores) { return __all_sync(0xffffffffu, mbar_wait(sm, &sm.s_full[t], (scores - 1u) & 1u, a, 8)); };
             if (it == 0 && begun) {
                 k_free0 = 0;
-                k_asked = 1;
+                firsts = 1;
                 q_loads0 = n0 > 0;
                 q_loads1 = n1 > 0;
                 if (kPaged && n_max > 1) page = page_of_lane(a, kv_len, seq, 1, lane);
@@ -1078,8 +1119,6 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             }
             if (!alive) break;
             owed = true;
-            ++pairs;
-            n_before = n_max;
             // (waits are for commits of late only, see step_done: where this pair had no use for a Q tile, that has long been free)
             first_s = n_max == 1 ? commits : -1;
             q_used0 = n0 > 0;
@@ -1089,22 +1128,11 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             commits += n_max + 1;
             g += n_max;
         }
-        // After an abort none of this warp's copies may be in flight when the CTA ends (otherwise every tile has been read): wait (bounded) for
-        // the last ones. These waits ignore the abort flag: they only depend on the copy engine; the other ring's arrival may be missing, and the
-        // copies have landed long before the limit then.
-        if (lane == 0 && !alive) {
-            const unsigned long long t_begin = global_timer_ns();
-            auto settle = [&](unsigned long long* bar, unsigned parity) {
-                while (!mbar_try_wait(bar, parity) && global_timer_ns() - t_begin < 100000000ULL) {}
-            };
-            if (answers != requests) settle(&sm.answered, answers & 1u);
-            if (q_loads0 > 0) settle(&sm.q_full[0], (q_loads0 - 1u) & 1u);
-            if (q_loads1 > 0) settle(&sm.q_full[1], (q_loads1 - 1u) & 1u);
-            for (int j = k_asked - 2; j < k_asked; ++j) {   // (j = -1, -2: of the pair before)
-                if (j < -1 || (j == -1 && n_before == 0) || (j >= 0 && a.test_skip_k == j + 1)) continue;
-                if (j == 0 || (j == -1 && n_before == 1)) settle(&sm.k_first, (pairs + (j == 0 ? 0u : 1u)) & 1u);
-                else settle(&sm.step_full[(g + j - 1) & 1], (unsigned)((g + j - 1) >> 1) & 1u);
-            }
+        if (lane == 0) {
+            if (!all_read(sm, alive, a, 3))
+                settle_copies(sm, given, sm.left_out,
+                              (unsigned)(answers != requests) | (answers & 1u) << 1 | (unsigned)(q_loads0 > 0) << 2 | ((q_loads0 - 1u) & 1u) << 3 |
+                                  (unsigned)(q_loads1 > 0) << 4 | ((q_loads1 - 1u) & 1u) << 5 | (unsigned)(firsts > 0) << 6 | ((firsts - 1u) & 1u) << 7);
         }
     } else if (warp == kLoadWarpV) {
         // ------------------------------ V tiles ------------------------------
@@ -1117,7 +1145,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         int v_free0 = -1, v_free1 = -1;
         unsigned tails = 0;
         bool alive = true, tail_pending = false;   // tail_pending: the tail tile's copy was issued and v_tail not yet seen complete
-        int last_g[2] = {-1, -1};              // the last two steps whose V tile arrives on step_full by a copy: before last, last
+        int given = 0;                         // as in the K producer
         for (unsigned it = 0;; ++it) {
             alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.item_full[it & 1u], (it >> 1) & 1u, a, 7));
             if (!alive) break;
@@ -1152,8 +1180,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 (e ? v_free1 : v_free0) = commits + j + 1;
                 if (kPaged && j + 1 < n_max) page = page_of_lane(a, sq.kv_len, w.seq, j + 1, lane);
                 if (!fix) {
-                    last_g[0] = last_g[1];
-                    last_g[1] = g + j;
+                    given = g + j + 1;
                     continue;
                 }
                 tail_pending = true;
@@ -1170,17 +1197,14 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // generic-proxy writes -> tensor-core reads
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sm.step_full[e]);
+                given = g + j + 1;
             }
             if (!alive) break;
             commits += n_max + 1;
             g += n_max;
         }
-        if (lane == 0 && !alive) {   // (else every V tile has been read; the waits as at the end of the K producer)
-            const unsigned long long t_begin = global_timer_ns();
-            while (tail_pending && !mbar_try_wait(&sm.v_tail, tails & 1u) && global_timer_ns() - t_begin < 100000000ULL) {}
-            for (int i = 0; i < 2; ++i)
-                if (last_g[i] >= 0)
-                    while (!mbar_try_wait(&sm.step_full[last_g[i] & 1], (unsigned)(last_g[i] >> 1) & 1u) && global_timer_ns() - t_begin < 100000000ULL) {}
+        if (lane == 0) {
+            if (!all_read(sm, alive, a, 9)) settle_copies(sm, given, 0, (unsigned)tail_pending << 8 | (tails & 1u) << 9);
         }
     } else if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(&sm.tmem_base)) : "memory");
@@ -1206,6 +1230,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             asm volatile("prefetch.tensormap [%0];\n" ::"l"(&k_map) : "memory");
             asm volatile("prefetch.tensormap [%0];\n" ::"l"(&v_map) : "memory");
             sm.abort_flag = 0;
+            sm.left_out = 0;
             for (int i = 0; i < 2; ++i) {
                 mbar_init(&sm.item_full[i], 1);
                 mbar_init(&sm.item_empty[i], 10);

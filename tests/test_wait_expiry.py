@@ -86,6 +86,59 @@ def test_expiry_at_every_part_of_the_key_loop(tile, d):
     H.assert_bf16_close(H.to_np(o), ob.attn_f64_batch(q, k, v), "call after the reported expiry")
 
 
+@pytest.mark.parametrize("d", [128, 64])
+@pytest.mark.parametrize("how", ["packed", "packed, rows unknown", "packed over pages", "chunks over pages"])
+@pytest.mark.parametrize("tile", [0, 3, 6])
+def test_expiry_in_a_tile_pair_that_a_cta_has_taken_over(tile, how, d):
+    # pairs of one to three tiles, some twenty for every SM, before a few of eight that alone have tiles 3 and 6. The call ends soon after the limit: what the producers wait for
+    # at their end has arrived by then, and their last waits would otherwise run 100 ms
+    hq, hkv, page, dt = 16, 8, 16, torch.bfloat16
+    rng = np.random.Generator(np.random.Philox(d + tile))
+    lens = (128 * rng.integers(1, 4, size=400) - 50 * rng.integers(0, 2, size=400)).tolist() + [1024] * 6
+    new = [128 if how == "chunks over pages" else min(x, 128) for x in lens]
+    lens = [max(x, n) for x, n in zip(lens, new)]
+    g = torch.Generator(device="cuda").manual_seed(tile)
+    cu_q, cu_k = (torch.tensor(np.concatenate([[0], np.cumsum(x)]), dtype=torch.int32, device="cuda") for x in (new, lens))
+    n, q = len(lens), torch.randn((sum(new), hq, d), generator=g, device="cuda", dtype=dt)
+    o, scale = torch.empty_like(q), 1.0 / math.sqrt(d)
+    if how.startswith("packed,") or how == "packed":
+        k, v = (torch.randn((sum(lens), hkv, d), generator=g, device="cuda", dtype=dt) for _ in range(2))
+        totals = dict(total_q=sum(new), total_k=sum(lens)) if how == "packed" else {}
+        call = lambda: low.flash_attn_varlen(q, k, v, o, cu_q, cu_k, n, max(new), max(lens), hq, hkv, d, scale, **totals)
+    else:
+        width = -(-max(lens) // page)
+        k, v = (torch.randn((n * width, page, hkv, d), generator=g, device="cuda", dtype=dt) for _ in range(2))
+        table = torch.randperm(n * width, generator=g, device="cuda").to(torch.int32).view(n, width)
+        if how == "packed over pages":
+            call = lambda: low.flash_attn_varlen(q, k, v, o, cu_q, cu_k, n, max(new), max(lens), hq, hkv, d, scale, table, page, total_q=sum(new))
+        else:
+            ctx = torch.tensor(lens, dtype=torch.int32, device="cuda")
+            call = lambda: low.flash_attn_with_kvcache(q, k, v, o, table, ctx, n, 128, hq, hkv, d, page, width, scale)
+    call()
+    torch.cuda.synchronize()
+    assert ffi.last_path() == "prefill_tcgen05" and ffi.device_status() == 0
+    want = o.clone()
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    try:
+        ffi.set_option("prefill_wait_us", 1000)
+        ffi.set_option("prefill_test_skip_k", tile + 1)
+        begin.record()
+        call()
+        end.record()
+    finally:
+        ffi.set_option("prefill_test_skip_k", 0)
+        ffi.set_option("prefill_wait_us", 0)
+    torch.cuda.synchronize()
+    code = ffi.device_status()                       # (read and cleared)
+    assert code != 0
+    # 1 ms from the tile that does not come, and so for every CTA that starts after one has given up: all pairs have a tile 0, 22 to an SM
+    assert begin.elapsed_time(end) < (100 if tile == 0 else 30)
+    o.fill_(float("nan"))
+    call()
+    torch.cuda.synchronize()
+    assert ffi.device_status() == 0 and torch.equal(o, want)
+
+
 def test_a_bound_above_two_seconds_is_kept():
     # the bound is counted in clocks, two to the nanosecond, so that it is no shorter than asked for at any SM clock up to 2 GHz
     b, s, h, d = 1, 256, 1, 128
