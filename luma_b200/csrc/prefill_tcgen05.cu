@@ -941,28 +941,16 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     // producer/issuer warpgroup hands most of its share to the two softmax warpgroups, which
     // keep a whole 128-column score row per thread in registers.
     if (warp >= 8) {
-    if (warp != kLoadWarp) asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n");
+    // The packed buffers' ends that the tensor maps do not know.
+    const bool q_open = packed && !a.q_bounded, kv_open = packed && !a.paged && !a.kv_bounded;
+    Item w;                // K producer: the tile pair at hand
+    bool begun = false;    // ... and whether the first one's first copies have been requested
     if (warp == kLoadWarp) {
-        // ------------------------------ tile pairs, Q and K tiles ------------------------------
-        // The warps run their loops whole; lane 0 issues the bulk copies (a paged tile: a lane per page), and all lanes share the
-        // plain-load copy of a tile at the very end of a packed buffer.
-        const bool q_open = packed && !a.q_bounded, kv_open = packed && !a.paged && !a.kv_bounded;
-        const long long tot_q = q_open ? (long long)a.cu_q[a.batch] : 0;
-        const long long tot_k = kv_open ? (long long)a.cu_k[a.batch] : 0;
-        int g = 0, commits = 0;              // steps and commits on step_done of the tile pairs before this one
-        int k_free0 = -1, k_free1 = -1;      // the commit that frees each K stage (-1: free)
-        unsigned scores0 = 0, scores1 = 0;   // S of each query tile so far: its Q is free when the last one has finished
-        bool q_used0 = false, q_used1 = false;   // (and has to be waited for: by the pair before this one)
-        int first_s = -1;                    // the commit of the last pair's first S, where that pair had one step (else it has been waited for)
-        int given = 0;                       // steps whose K arrival has been made or comes with a copy that has been requested
-        unsigned q_loads0 = 0, q_loads1 = 0, firsts = 0, requests = 0, answers = 0;   // firsts: K tiles 0 that have been requested
-        bool alive = true;
         // The CTA's own tile pair, and its first copies at once, in as few instructions as that takes: all of them come in for the first time here, and
         // in the loop below, with its waits and cases, the first S came 1600 to 2300 clocks later (a fifth of a call of one short wave).
-        Item w;
         w.some = find_pair<kPaged>(a, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, lane, w);
         asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
-        const bool begun = w.some && max(w.t[0].n_kv, w.t[1].n_kv) > 0 && !q_open && !kv_open && a.test_skip_k != 1;
+        begun = w.some && max(w.t[0].n_kv, w.t[1].n_kv) > 0 && !q_open && !kv_open && a.test_skip_k != 1;
         if (begun && (kPaged || lane == 0)) {
             const int page = kPaged ? page_of_lane(a, w.sq.kv_len, w.seq, 0, lane) : -1;
             if (lane == 0 && w.t[0].n_kv > 0) {
@@ -978,7 +966,55 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             }
         }
         __syncwarp();
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n");
+    } else if (warp == kLoadWarpV) {
+        asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
+    } else if (warp != kMmaWarp) {
+        // Set-up, by the warp that has nothing else to do, while the K producer finds out what the CTA's first tile pair is.
+        if (lane == 0) {
+            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&q_map) : "memory");
+            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&k_map) : "memory");
+            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&v_map) : "memory");
+            sm.abort_flag = 0;
+            sm.left_out = 0;
+            for (int i = 0; i < 2; ++i) {
+                mbar_init(&sm.item_full[i], 1);
+                mbar_init(&sm.item_empty[i], 10);
+                mbar_init(&sm.q_full[i], 1);
+                mbar_init(&sm.s_full[i], 1);
+                mbar_init(&sm.o_full[i], 1);
+                mbar_init(&sm.p_ready[0][i], 128);
+                mbar_init(&sm.p_ready[1][i], 128);
+                mbar_init(&sm.step_full[i], 2);
+            }
+            for (int i = 0; i < kDone; ++i) mbar_init(&sm.step_done[i], 1);
+            mbar_init(&sm.answered, 1);
+            mbar_init(&sm.k_first, 1);
+            mbar_init(&sm.v_tail, 1);
+            mbar_init(&sm.drain, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        }
+        __syncwarp();
+        asm volatile("barrier.cta.arrive 1, 96;\n" ::: "memory");    // the producers
+        asm volatile("barrier.cta.arrive 2, 320;\n" ::: "memory");   // issuer and softmax warps, which wait for tensor memory as well
+    }
+    // One instruction for the four warps, as the instruction wants it. The softmax warps get the registers that all four give back: none before the first copies have been
+    // requested, and there is nothing to do for them before.
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n");
+    if (warp == kLoadWarp) {
+        // ------------------------------ tile pairs, Q and K tiles ------------------------------
+        // The warps run their loops whole; lane 0 issues the bulk copies (a paged tile: a lane per page), and all lanes share the
+        // plain-load copy of a tile at the very end of a packed buffer.
+        const long long tot_q = q_open ? (long long)a.cu_q[a.batch] : 0;
+        const long long tot_k = kv_open ? (long long)a.cu_k[a.batch] : 0;
+        int g = 0, commits = 0;              // steps and commits on step_done of the tile pairs before this one
+        int k_free0 = -1, k_free1 = -1;      // the commit that frees each K stage (-1: free)
+        unsigned scores0 = 0, scores1 = 0;   // S of each query tile so far: its Q is free when the last one has finished
+        bool q_used0 = false, q_used1 = false;   // (and has to be waited for: by the pair before this one)
+        int first_s = -1;                    // the commit of the last pair's first S, where that pair had one step (else it has been waited for)
+        int given = 0;                       // steps whose K arrival has been made or comes with a copy that has been requested
+        unsigned q_loads0 = 0, q_loads1 = 0, firsts = 0, requests = 0, answers = 0;   // firsts: K tiles 0 that have been requested
+        bool alive = true;
 #ifdef FA_TRACE
         long long* const trace = (a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == (unsigned)a.trace_y && blockIdx.z == 0 && lane == 0) ? a.trace : nullptr;
 #endif
@@ -1138,8 +1174,6 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         // ------------------------------ V tiles ------------------------------
         // A producer of its own: with a paged cache a tile is one copy per page and 64-column half plus a block-table read per page, and a single
         // thread issuing both rings cannot keep up with the tensor pipe at small page sizes.
-        asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
-        const bool kv_open = packed && !a.paged && !a.kv_bounded;
         const long long tot_k = kv_open ? (long long)a.cu_k[a.batch] : 0;
         int g = 0, commits = 0;
         int v_free0 = -1, v_free1 = -1;
@@ -1222,36 +1256,6 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         }
 #endif
         issue_products<T, D>(smem_u32(&sm), sm.tmem_base, a.status, a.wait_ns FA_TRACE_ARG(trace));
-    } else {
-        // ------------------------------ set-up ------------------------------
-        // (by the warp that has nothing else to do, while the K producer finds out what the CTA's first tile pair is)
-        if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&q_map) : "memory");
-            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&k_map) : "memory");
-            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&v_map) : "memory");
-            sm.abort_flag = 0;
-            sm.left_out = 0;
-            for (int i = 0; i < 2; ++i) {
-                mbar_init(&sm.item_full[i], 1);
-                mbar_init(&sm.item_empty[i], 10);
-                mbar_init(&sm.q_full[i], 1);
-                mbar_init(&sm.s_full[i], 1);
-                mbar_init(&sm.o_full[i], 1);
-                mbar_init(&sm.p_ready[0][i], 128);
-                mbar_init(&sm.p_ready[1][i], 128);
-                mbar_init(&sm.step_full[i], 2);
-            }
-            for (int i = 0; i < kDone; ++i) mbar_init(&sm.step_done[i], 1);
-            mbar_init(&sm.answered, 1);
-            mbar_init(&sm.k_first, 1);
-            mbar_init(&sm.v_tail, 1);
-            mbar_init(&sm.drain, 1);
-            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        }
-        __syncwarp();
-        asm volatile("barrier.cta.arrive 1, 96;\n" ::: "memory");    // the producers
-        asm volatile("barrier.cta.arrive 2, 320;\n" ::: "memory");   // issuer and softmax warps, which wait for tensor memory as well
     }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 208;\n");
