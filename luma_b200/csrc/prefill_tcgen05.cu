@@ -1432,6 +1432,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 for (int h = 0; h < D / 64; ++h) {   // a half's copy is on its way while the next one is read and scaled
                     unsigned char* const half = h > 0 && last ? sm.q[t] + (warp & 3) * kOutBytes : stage;
                     float ov[2][32];
+                    __syncwarp();   // (one lane has stored)
                     tc_ld32(o_addr + h * 64, ov[0]);
                     tc_ld32(o_addr + h * 64 + 32, ov[1]);
                     tc_wait_ld();
@@ -1463,6 +1464,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 #pragma unroll 1
                 for (int c = 0; c < D / 32; ++c) {
                     float ov[32];
+                    __syncwarp();   // (lanes whose rows exist have stored)
                     tc_ld32(o_addr + c * 32, ov);
                     tc_wait_ld();
                     T* const to = static_cast<T*>(a.o[0]) + ((sq.o_row0 + row) * a.o_heads + a.o_head0 + ti.head) * a.d_real + c * 32;
@@ -1489,23 +1491,25 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     #pragma unroll 1
                 for (int c = 0; c < D / 32; ++c) {
                     float ov[32];
+                    __syncwarp();   // (some lanes have written their rows)
                     tc_ld32(o_addr + c * 32, ov);
                     tc_wait_ld();
                     if (ti.n_kv == 0) {   // the tile saw no key: tensor memory holds nothing of ours, the rows are zeros
                     #pragma unroll
                         for (int i = 0; i < 32; ++i) ov[i] = 0.0f;
                     }
-                    if (lane / kRowsAtOnce != part) continue;
-                    const int rr = lane % kRowsAtOnce;
+                    if (lane / kRowsAtOnce == part) {
+                        const int rr = lane % kRowsAtOnce;
     #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        uint4 w;
-                        w.x = pack16<T>(ov[8 * i] * inv, ov[8 * i + 1] * inv);
-                        w.y = pack16<T>(ov[8 * i + 2] * inv, ov[8 * i + 3] * inv);
-                        w.z = pack16<T>(ov[8 * i + 4] * inv, ov[8 * i + 5] * inv);
-                        w.w = pack16<T>(ov[8 * i + 6] * inv, ov[8 * i + 7] * inv);
-                        const int ch = c * 4 + i;   // 16-byte chunk of the row, XOR-swizzled against bank conflicts
-                        *reinterpret_cast<uint4*>(stage + rr * kRowBytes + ((ch ^ (rr & (kChunks - 1))) << 4)) = w;
+                        for (int i = 0; i < 4; ++i) {
+                            uint4 w;
+                            w.x = pack16<T>(ov[8 * i] * inv, ov[8 * i + 1] * inv);
+                            w.y = pack16<T>(ov[8 * i + 2] * inv, ov[8 * i + 3] * inv);
+                            w.z = pack16<T>(ov[8 * i + 4] * inv, ov[8 * i + 5] * inv);
+                            w.w = pack16<T>(ov[8 * i + 6] * inv, ov[8 * i + 7] * inv);
+                            const int ch = c * 4 + i;   // 16-byte chunk of the row, XOR-swizzled against bank conflicts
+                            *reinterpret_cast<uint4*>(stage + rr * kRowBytes + ((ch ^ (rr & (kChunks - 1))) << 4)) = w;
+                        }
                     }
                 }
                 __syncwarp();
