@@ -273,6 +273,31 @@ __device__ __forceinline__ bool mbar_wait(Storage& sm, unsigned long long* bar, 
     }
 }
 
+// The same for the producers. A look suspends until the phase is complete, or some 8000 clocks, so what follows the first one is seldom reached: it is a function of its own, out of the
+// producers' loops, whose instructions share the SM's instruction cache with the softmax steps. 24 packed prompts of 17-2000 tokens, head size 64 267 us with it in each of the loops'
+// waits, 254 so; 4 chunks of 512 143.3 and 142.5; 4 x 2048 MHA 129.8 and 129.2.
+__device__ __noinline__ bool mbar_wait_on(unsigned bar, unsigned parity, unsigned abort_flag, long long limit, int* status, int where) {
+    const long long t0 = clock64();
+#pragma unroll 1
+    for (unsigned spin = 1;; ++spin) {
+        if (mbar_try_wait_at(bar, parity)) return true;
+        if ((spin & 63u) == 0u) {
+            if (shared_flag(abort_flag)) return false;
+            if (clock64() - t0 > limit) {
+                set_shared_flag(abort_flag);
+                *reinterpret_cast<volatile int*>(status) = where;
+                __threadfence_system();
+                return false;
+            }
+        }
+    }
+}
+template <typename Storage>
+__device__ __forceinline__ bool producer_wait(Storage& sm, unsigned long long* bar, unsigned parity, const PrefillArgs& a, int where) {
+    if (mbar_try_wait(bar, parity)) return true;
+    return mbar_wait_on(smem_u32(bar), parity, smem_u32((const void*)&sm.abort_flag), (long long)(a.wait_ns * 2ULL), a.status, where);
+}
+
 // The end of a producer after an abort: none of its copies may be in flight when the CTA ends. These waits ignore the abort flag and depend on the copy engine
 // alone (bounded all the same). A step's barrier also wants the arrival of the other ring's producer, which may have given up before that step, so each of them
 // makes its arrivals for the two steps after its last one here. Two are enough: a stage is filled for step x once step x - 2 has finished, so neither ring is more
@@ -305,7 +330,7 @@ __device__ __noinline__ void settle_copies(Storage& sm, int given, int left_out,
 // The end of a producer: false where its copies have to be looked after (above). As long as nobody gives up, every copy has landed when the issuer has come to its end.
 template <typename Storage>
 __device__ __forceinline__ bool all_read(Storage& sm, bool alive, const PrefillArgs& a, int where) {
-    return alive && mbar_wait(sm, &sm.drain, 0u, a, where) && !sm.abort_flag;   // (an issuer that gives up says so before it ends)
+    return alive && producer_wait(sm, &sm.drain, 0u, a, where) && !sm.abort_flag;   // (an issuer that gives up says so before it ends)
 }
 
 __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, unsigned long long* bar, int c0, int c1,
@@ -1018,7 +1043,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 #ifdef FA_TRACE
         long long* const trace = (a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == (unsigned)a.trace_y && blockIdx.z == 0 && lane == 0) ? a.trace : nullptr;
 #endif
-        auto wait_commit = [&](int c) { return c < 0 || __all_sync(0xffffffffu, mbar_wait(sm, &sm.step_done[c & (kDone - 1)], (unsigned)(c / kDone) & 1u, a, 1)); };
+        auto wait_commit = [&](int c) { return c < 0 || __all_sync(0xffffffffu, producer_wait(sm, &sm.step_done[c & (kDone - 1)], (unsigned)(c / kDone) & 1u, a, 1)); };
         auto ask = [&]() {
             if (lane == 0) {
                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // (the answer before has been read)
@@ -1046,10 +1071,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             if (it > 0 || !w.some) {
             w.some = 0;
             if (requests == answers) ask();
-            if (it >= 2) alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.item_empty[it & 1u], ((it >> 1) - 1u) & 1u, a, 5));
+            if (it >= 2) alive = __all_sync(0xffffffffu, producer_wait(sm, &sm.item_empty[it & 1u], ((it >> 1) - 1u) & 1u, a, 5));
             while (alive) {
                 int bx, by, bz;
-                alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.answered, answers & 1u, a, 6));
+                alive = __all_sync(0xffffffffu, producer_wait(sm, &sm.answered, answers & 1u, a, 6));
                 if (!alive) break;
                 ++answers;
                 FA_TRACE_EVENT(3, (int)answers, 1);
@@ -1123,7 +1148,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             };
             // K tile 0 and the Q tiles: of the first pair in the order that the issuer wants them; else K first, which comes free first, then the Q tile that does, of
             // two row blocks of one head the shorter one, tile 1.
-            auto wait_q = [&](int t, unsigned scores) { return __all_sync(0xffffffffu, mbar_wait(sm, &sm.s_full[t], (scores - 1u) & 1u, a, 8)); };
+            auto wait_q = [&](int t, unsigned scores) { return __all_sync(0xffffffffu, producer_wait(sm, &sm.s_full[t], (scores - 1u) & 1u, a, 8)); };
             if (it == 0 && begun) {
                 k_free0 = 0;
                 firsts = 1;
@@ -1181,7 +1206,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         bool alive = true, tail_pending = false;   // tail_pending: the tail tile's copy was issued and v_tail not yet seen complete
         int given = 0;                         // as in the K producer
         for (unsigned it = 0;; ++it) {
-            alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.item_full[it & 1u], (it >> 1) & 1u, a, 7));
+            alive = __all_sync(0xffffffffu, producer_wait(sm, &sm.item_full[it & 1u], (it >> 1) & 1u, a, 7));
             if (!alive) break;
             const Item w = sm.item[it & 1u];
             __syncwarp();
@@ -1203,7 +1228,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             for (int j = 0; j < n_max; ++j) {
                 const int e = (g + j) & 1;
                 const int c = e ? v_free1 : v_free0;
-                if (c >= 0) alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.step_done[c & (kDone - 1)], (unsigned)(c / kDone) & 1u, a, 2));
+                if (c >= 0) alive = __all_sync(0xffffffffu, producer_wait(sm, &sm.step_done[c & (kDone - 1)], (unsigned)(c / kDone) & 1u, a, 2));
                 if (!alive) break;
                 const bool fix = tail_fix && j == tail_j;
                 unsigned long long* const bar = fix ? &sm.v_tail : &sm.step_full[e];
@@ -1218,7 +1243,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     continue;
                 }
                 tail_pending = true;
-                alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.v_tail, tails & 1u, a, 4));
+                alive = __all_sync(0xffffffffu, producer_wait(sm, &sm.v_tail, tails & 1u, a, 4));
                 if (!alive) break;
                 tail_pending = false;
                 ++tails;
