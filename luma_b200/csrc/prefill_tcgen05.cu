@@ -774,7 +774,7 @@ constexpr unsigned kApart = 950;   // clocks between the two tiles' first S at h
 //     tile's last products) 24 packed prompts took 299 us instead of 275, 4 x 2048 MHA 159 instead of 154.5, 2 x 8192 GQA 965 instead of 947;
 //   * a wait that runs out is looked after at the end of its step, which goes on without waiting on what happens to be in shared memory and
 //     reports nothing as done. Leaving at each wait doubled the code after it.
-template <typename T, int D>
+template <typename T, int D, bool kOnePair>
 __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int* status, unsigned long long wait_ns FA_TRACE_PARAM(trace)) {
     using Storage = SharedStorage<D>;
     sm_addr = __shfl_sync(0xffffffffu, sm_addr, 0);
@@ -838,7 +838,10 @@ __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int
         if (elect_one()) mbar_arrive_at(sm_addr + (unsigned)offsetof(Storage, item_empty) + 8 * (it & 1u));
         if (some == 0) break;
         const int n_max = max(n0, n1);
-        if (n_max <= 0) continue;
+        if (n_max <= 0) {
+            if (kOnePair) break;
+            continue;
+        }
         // The copies were requested in the order Q0, K0, Q1: the first S of tile 0 is issued as soon as
         // its two operands are there, without waiting for the other tile's Q.
         const unsigned long long kd0 = dk + (g & 1u) * kTileStep;
@@ -890,6 +893,7 @@ __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int
             }
             commit(offsetof(Storage, step_done) + 8 * (done++ & (kDone - 1)));
         }
+        if (kOnePair) break;
     }
     if (expired != 0 && !shared_flag(sm_addr + (unsigned)offsetof(Storage, abort_flag))) {   // (else another warp of the CTA gave up and reported it)
         set_shared_flag(sm_addr + (unsigned)offsetof(Storage, abort_flag));
@@ -942,7 +946,8 @@ __device__ __forceinline__ bool find_pair(const PrefillArgs& a, int bx, int by, 
 // kPaged: paged K/V, whose tiles are gathered page by page and whose tile pairs may be ordered on the device (a separate instantiation as
 // well: with the code of the two in it the contiguous calls' kernel took 375 us for 24 prompts of 17-2000 tokens at d = 64,
 // 364 without; 2 x 8192 GQA 1047 against 1027)
-template <typename T, int D, bool kMask, bool kPaged>
+// kOnePair: a CTA works on its own tile pair and no other; nobody looks for a next one.
+template <typename T, int D, bool kMask, bool kPaged, bool kOnePair>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                        const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap o_map, const PrefillArgs a) {
@@ -1068,27 +1073,27 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             // last K tile requested, two to three steps before its end: whoever comes to its end first takes the next one. Asked for at a
             // pair's beginning, the order heaviest first was lost for the second half of 4 chunks of 512 (256 pairs on 148 SMs): 174 us instead of
             // 153. The answer takes 1100 to 3100 clocks, what follows from it until the first copy 2000 more.
-            if (it > 0 || !w.some) {
-            w.some = 0;
-            if (requests == answers) ask();
-            if (it >= 2) alive = __all_sync(0xffffffffu, producer_wait(sm, &sm.item_empty[it & 1u], ((it >> 1) - 1u) & 1u, a, 5));
-            while (alive) {
-                int bx, by, bz;
-                alive = __all_sync(0xffffffffu, producer_wait(sm, &sm.answered, answers & 1u, a, 6));
+            if (it > 0) w.some = 0;
+            if (!kOnePair && !w.some) {
+                if (requests == answers) ask();
+                if (it >= 2) alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.item_empty[it & 1u], ((it >> 1) - 1u) & 1u, a, 5));
+                while (alive) {
+                    int bx, by, bz;
+                    alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.answered, answers & 1u, a, 6));
+                    if (!alive) break;
+                    ++answers;
+                    FA_TRACE_EVENT(3, (int)answers, 1);
+                    const bool got = read_answer(sm.answer, bx, by, bz);
+                    __syncwarp();
+                    if (!got) break;   // every tile pair is taken
+                    w.some = find_pair<kPaged>(a, bx, by, bz, lane, w);
+                    if (w.some) break;
+                    ask();
+                }
                 if (!alive) break;
-                ++answers;
-                FA_TRACE_EVENT(3, (int)answers, 1);
-                const bool got = read_answer(sm.answer, bx, by, bz);
-                __syncwarp();
-                if (!got) break;   // every tile pair is taken
-                w.some = find_pair<kPaged>(a, bx, by, bz, lane, w);
-                if (w.some) break;
-                ask();
-            }
-            if (!alive) break;
             }
             if (!w.some) w.t[0].n_kv = w.t[1].n_kv = 0;
-            if (lane == 0) {
+            if (lane == 0 && (!kOnePair || it == 0)) {
                 sm.item[it & 1u] = w;
                 mbar_arrive(&sm.item_full[it & 1u]);
             }
@@ -1104,6 +1109,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             const int kv_len = w.sq.kv_len, kv_crow = w.sq.kv_crow, kv_cb = w.sq.kv_cb, seq = w.seq, kv_head = w.kv_head;
             const int n0 = w.t[0].n_kv, n1 = w.t[1].n_kv, n_max = max(n0, n1);
             if (n_max <= 0) {
+                if (kOnePair) break;
                 ask();
                 continue;
             }
@@ -1214,7 +1220,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             if (!w.some) break;
             const SeqExtent& sq = w.sq;
             const int n_max = max(w.t[0].n_kv, w.t[1].n_kv);
-            if (n_max <= 0) continue;
+            if (n_max <= 0) {
+                if (kOnePair) break;
+                continue;
+            }
             // The sequence's last V tile, when the sequence does not end on a tile boundary, holds rows
             // that are not this sequence's: the unwritten rest of its last page, or the next sequence
             // of a packed buffer. P is exactly zero there, but 0 x NaN (an uninitialised pool, a page
@@ -1259,6 +1268,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 given = g + j + 1;
             }
             if (!alive) break;
+            if (kOnePair) break;
             commits += n_max + 1;
             g += n_max;
         }
@@ -1280,7 +1290,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             FA_TRACE_EVENT(2, kTraceSteps - 1, 1);   // set-up (barriers, tensor memory) done
         }
 #endif
-        issue_products<T, D>(smem_u32(&sm), sm.tmem_base, a.status, a.wait_ns FA_TRACE_ARG(trace));
+        issue_products<T, D, kOnePair>(smem_u32(&sm), sm.tmem_base, a.status, a.wait_ns FA_TRACE_ARG(trace));
     }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 208;\n");
@@ -1299,7 +1309,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         long long* trace = (a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == (unsigned)a.trace_y && blockIdx.z == 0 && lane == 0 && (warp & 3) == 0) ? a.trace : nullptr;
 #endif
 #pragma unroll 1
-        for (unsigned it = 0; alive; ++it) {
+        for (unsigned it = 0; alive && (!kOnePair || it == 0); ++it) {
         alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.item_full[it & 1u], (it >> 1) & 1u, a, 22 + t));
         if (!alive) break;
         const bool some = sm.item[it & 1u].some != 0;
@@ -1452,7 +1462,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 // of clocks and hold up the barrier traffic of the other tile's last steps. Rows past the
                 // end of the sequence are outside the tensor map and are not written.
                 // Where no tile pair follows, the second half goes through the Q tile's shared memory and need not wait until the first has been read (0.4 us).
-                const bool last = D == 128 && __all_sync(0xffffffffu, mbar_test_at(smem_u32(&sm.item_full[(it + 1u) & 1u]), ((it + 1u) >> 1) & 1u) && sm.item[(it + 1u) & 1u].some == 0);
+                const bool last = D == 128 && (kOnePair || __all_sync(0xffffffffu, mbar_test_at(smem_u32(&sm.item_full[(it + 1u) & 1u]), ((it + 1u) >> 1) & 1u) && sm.item[(it + 1u) & 1u].some == 0));
 #pragma unroll 1
                 for (int h = 0; h < D / 64; ++h) {   // a half's copy is on its way while the next one is read and scaled
                     unsigned char* const half = h > 0 && last ? sm.q[t] + (warp & 3) * kOutBytes : stage;
@@ -1792,12 +1802,6 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     const int num_mb = (p.q_seq_len + kBlockM - 1) / kBlockM;
     const int pairs = (group * num_mb + 1) / 2;
     const size_t smem = sizeof(SharedStorage<D>) + 1024;
-    cudaError_t err = cudaFuncSetAttribute(prefill_tcgen05_kernel<T, D, kMask, kPaged>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) {
-        set_last_errorf("prefill_tcgen05_kernel: %s", cudaGetErrorString(err));
-        cudaGetLastError();
-        return FLASH_ATTN_ERR_CUDA;
-    }
     // Band width: the pairs of a band start together, so their work must be about equal or the
     // heaviest-first order is lost (at S = 2048 without GQA, bands of 2 cost 13 %). A band of w
     // pairs spans 2w / group row blocks, i.e. that many K/V tiles of difference between its lightest
@@ -1881,7 +1885,24 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
         if (ctas <= 0 || ctas > 0x7fffffffLL) return -1;
         grid = dim3((unsigned)ctas);
     }
-    prefill_tcgen05_kernel<T, D, kMask, kPaged><<<grid, kThreads, smem, stream>>>(qm, km, vm, om, a);
+    // Where the grid has no more CTAs than the device has SMs there is no pair to take over, and such a call runs without the loop over pairs, whose counters and cases cost the
+    // first copies, the step (2 to 3 %) and, over pages, the producers' registers. us with the loop and without, from a graph: 1 x 658, 32/8 heads 15.6 and 15.3; 2 x 433 MHA 11.4 and
+    // 11.0; 1 x 4096, 4/4 heads 52.4 and 51.6; 3 x 5 tokens over 46-747 18.9 and 17.7; 16 x 64 tokens over 1024-8192, 8/8 heads 108 and 100. Not asking for a pair alone, in the same
+    // code, gave 0.1 us. Nor has a call in order much to take over: a CTA that has asked starts a pair about 2 us later, and those that start by themselves take
+    // the next one just as well (4 chunks of 512 over 1024-8192 142 and 139.5, 4 of 300 over 2048-8192 125.5 and 122.6, 8 of 512 247 either way). With few-row sequences left out
+    // a grid in order has empty CTAs, which are cheaper to take over (serve steps of 4 chunks with 32 tokens 225 and 229, 6 with 40 308 and 317), and so are short pairs at head size
+    // 64 (8 x 200 over 512-4096, 32/8 heads 69 and 71). Contiguous K/V at head size 64: no difference (1 x 449, 64/8 heads of 32 11.6 either way; 1 x 2048, 8/8 heads 26.8 and 27.3), and
+    // none is built.
+    constexpr bool kOneWave = D == 128 || kPaged;
+    const bool one_pair = kOneWave && ((long long)grid.x * grid.y * grid.z <= sm_count() || (D == 128 && a.ordered && a.skip_rows == 0));
+    const auto kernel = one_pair ? prefill_tcgen05_kernel<T, D, kMask, kPaged, kOneWave> : prefill_tcgen05_kernel<T, D, kMask, kPaged, false>;
+    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) {
+        set_last_errorf("prefill_tcgen05_kernel: %s", cudaGetErrorString(err));
+        cudaGetLastError();
+        return FLASH_ATTN_ERR_CUDA;
+    }
+    kernel<<<grid, kThreads, smem, stream>>>(qm, km, vm, om, a);
     int rc = check_launch("prefill_tcgen05_kernel");
     if (rc == FLASH_ATTN_OK && a.skip_rows > 0) rc = launch_mixed_few_rows(p, few, stream);
     if (rc == FLASH_ATTN_OK) note_path("prefill_tcgen05", a.skip_rows > 0 ? 2 : 1);

@@ -77,3 +77,32 @@ def test_rows_to_several_buffers(d):
         assert torch.equal(x[:, :, first:first + hq], want)
         assert bool((x[:, :, :first] == -7.0).all()) and bool((x[:, :, first + hq:] == -7.0).all())
     assert ffi.device_status() == 0
+
+
+@pytest.mark.parametrize("d", [128, 64])
+@pytest.mark.parametrize("paged", [False, True])
+@pytest.mark.parametrize("s", [100, 256, 700])
+def test_a_grid_of_one_wave_and_one_with_a_tile_pair_more(s, paged, d):
+    # as many CTAs as the device has SMs, each on its own pair, and one pair more, which somebody takes over: the same bits for what they have in common
+    sms, page = torch.cuda.get_device_properties(0).multi_processor_count, 16
+    per_seq = -(-s // 256)                         # without GQA a pair is two row blocks of one head
+    g = torch.Generator(device="cuda").manual_seed(s + d)
+    width = -(-s // page)
+    most = sms // per_seq + 1
+    q = torch.randn((most, s, 1, d), generator=g, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.randn((most * width, page, 1, d) if paged else (most, s, 1, d), generator=g, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    table = torch.randperm(most * width, generator=g, device="cuda").to(torch.int32).view(most, width)
+    outs = []
+    for b in (sms // per_seq, most):
+        o = torch.full_like(q[:b], float("nan"))
+        if paged:
+            lens = torch.full((b,), s, dtype=torch.int32, device="cuda")
+            low.flash_attn_with_kvcache(q[:b], k, v, o, table[:b], lens, b, s, 1, 1, d, page, width, 1.0 / np.sqrt(d))
+        else:
+            low.flash_attn(q[:b], k[:b], v[:b], o, b, s, s, 1, 1, d, 0, 1.0 / np.sqrt(d))
+        torch.cuda.synchronize()
+        assert ffi.last_path() == "prefill_tcgen05" and ffi.device_status() == 0
+        outs.append(o)
+    assert torch.equal(outs[0], outs[1][:len(outs[0])])
+    kk, vv = ((x[table[-1].long()].reshape(1, -1, 1, d)[:, :s] if paged else x[-1:]) for x in (k, v))
+    assert torch.equal(outs[1][-1:], high.flash_attn_func(q[-1:], kk.contiguous(), vv.contiguous()))
