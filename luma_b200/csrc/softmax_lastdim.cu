@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kStreamThreads) softmax_stream_kernel(const T*
     const T* src = in + (long long)blockIdx.x * n;
     T* dst = out + (long long)blockIdx.x * n;
     float m = -INFINITY, s = 0.0f;
-    for (int c = threadIdx.x * V; c < n; c += kStreamThreads * V) {
+    for (unsigned c = threadIdx.x * V; c < (unsigned)n; c += kStreamThreads * V) {   // (up to a stride beyond n, which may be near 2^31)
         float x[V];
         load_vec<T, V>(src + c, x);
         float mv = x[0];
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kStreamThreads) softmax_stream_kernel(const T*
     s = lane < kStreamThreads / 32 ? sh_s[lane] : 0.0f;
     warp_merge(m, s);
     const float ml = m * kLog2e, inv = 1.0f / s;
-    for (int c = threadIdx.x * V; c < n; c += kStreamThreads * V) {
+    for (unsigned c = threadIdx.x * V; c < (unsigned)n; c += kStreamThreads * V) {
         float x[V];
         load_vec<T, V>(src + c, x);
 #pragma unroll

@@ -94,6 +94,25 @@ def test_softmax_rows_that_begin_anywhere(dt):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [2 ** 31 - 8])
+def test_softmax_of_a_row_near_the_longest(n):
+    """The largest row sizes of the signature: they are read twice like any long row, and a column counter passes 2^31."""
+    from luma_b200 import ffi, low
+    x = torch.zeros((1, n), device="cuda", dtype=torch.bfloat16)
+    tall = [0, 1, n // 2 + 1, n - 4097, n - 1]
+    x[0, tall] = 10.0
+    y = low.softmax_last_dim(x, out=x)
+    torch.cuda.synchronize()
+    assert ffi.last_path() == "softmax_stream"
+    total = len(tall) + (n - len(tall)) * np.exp(-10.0)
+    got = y[0, tall].double().cpu().numpy()
+    np.testing.assert_allclose(got, 1.0 / total, rtol=2.0 ** -8 + 1e-4)       # one rounding to 8 bits; whole counts below 2^24 in each thread's sum
+    y[0, tall] = float(y[0, 2])
+    assert bool((y == y[0, 2]).all())
+    np.testing.assert_allclose(float(y[0, 2]), np.exp(-10.0) / total, rtol=2.0 ** -8 + 1e-4)
+
+
+@pytest.mark.gpu
 def test_softmax_all_minus_inf_row_and_errors():
     import luma_b200 as L
     from luma_b200 import low
