@@ -304,6 +304,9 @@ int launch_softmax(const T* in, T* out, long long rows, int n, cudaStream_t stre
     // threads per SM, whose loads, arithmetic and stores then overlap; with 128 elements per thread
     // (one resident CTA) a bf16 row of 4096 reached 0.54 of the copy bandwidth
     constexpr int P = 32 / V;
+    constexpr int kWide = 16 / (int)sizeof(T);
+    // the longest row of one CTA: 32 elements for each of 1024 threads, of which a row that begins anywhere may leave kWide - 1 unused ahead of it
+    constexpr int kLongest = 32768 - (V == kWide ? 0 : kWide - 1);
     const int vecs = n / V;
     const int warps = 8;
     const unsigned grid = (unsigned)rows;
@@ -317,8 +320,8 @@ int launch_softmax(const T* in, T* out, long long rows, int n, cudaStream_t stre
         else if (vecs <= 32 * (P / 2)) per_warp(softmax_warp_kernel<T, V, P / 2, 2>, 2);
         else per_warp(softmax_warp_kernel<T, V, P, 1>, 1);
         note_path("softmax_warp", 1);
-    } else if (V * sizeof(T) == 16 ? n <= 32768 : (n + 30 / (int)sizeof(T)) / (16 / (int)sizeof(T)) <= 32768 / (16 / (int)sizeof(T))) {
-        if constexpr (V * sizeof(T) == 16) {
+    } else if (n <= kLongest) {
+        if constexpr (V == kWide) {
             if (vecs <= 64 * P) softmax_block_kernel<T, false, P, 64><<<grid, 64, 0, stream>>>(in, out, n);
             else if (vecs <= 128 * P) softmax_block_kernel<T, false, P, 128><<<grid, 128, 0, stream>>>(in, out, n);
             else if (vecs <= 256 * P) softmax_block_kernel<T, false, P, 256><<<grid, 256, 0, stream>>>(in, out, n);
@@ -329,7 +332,7 @@ int launch_softmax(const T* in, T* out, long long rows, int n, cudaStream_t stre
             // (60000 rows), one of 1413 86 and 57 (f16, 46713 rows). CTAs of just as many warps as a row needs: in CTAs of a power of two,
             // lengths just above one had twice the threads. Two CTAs of more than 512 threads do not fit an SM's registers: up to an eighth
             // above, each thread takes a vector more (8000 rows of 16383 bf16: 105 us, 155 without).
-            constexpr int kWide = 16 / (int)sizeof(T), kEach = 32 / kWide;
+            constexpr int kEach = 32 / kWide;
             const unsigned all = (unsigned)(n + 2 * kWide - 2) / kWide;   // (a row begins up to kWide - 1 elements into its first vector)
             auto fit = [&](unsigned each) { return (all + each * 32 - 1) / (each * 32) * 32; };
             const unsigned threads = fit(kEach);

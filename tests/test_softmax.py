@@ -94,9 +94,9 @@ def test_softmax_rows_that_begin_anywhere(dt):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [2 ** 31 - 8])
+@pytest.mark.parametrize("n", [2 ** 31 - 8, 2 ** 31 - 2])
 def test_softmax_of_a_row_near_the_longest(n):
-    """The largest row sizes of the signature: they are read twice like any long row, and a column counter passes 2^31."""
+    """The largest row sizes of the signature, on and off the 16-byte grid: they are read twice like any long row, and a column counter passes 2^31."""
     from luma_b200 import ffi, low
     x = torch.zeros((1, n), device="cuda", dtype=torch.bfloat16)
     tall = [0, 1, n // 2 + 1, n - 4097, n - 1]
