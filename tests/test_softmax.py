@@ -94,6 +94,21 @@ def test_softmax_rows_that_begin_anywhere(dt):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("n", [162, 1413, 4099, 16383, 32761, 33001])
+def test_softmax_in_place_of_rows_that_begin_anywhere(n, dt):
+    """A row's first and last words also hold its neighbours' ends, which other CTAs write meanwhile: the same bits as into another tensor."""
+    from luma_b200 import low
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn((1500, n), generator=g, device="cuda", dtype=H.TORCH_DT[dt])
+    want = low.softmax_last_dim(x)
+    for _ in range(3):
+        y = x.clone()
+        low.softmax_last_dim(y, out=y)
+        assert torch.equal(y, want)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n", [2 ** 31 - 8, 2 ** 31 - 2])
 def test_softmax_of_a_row_near_the_longest(n):
     """The largest row sizes of the signature, on and off the 16-byte grid: they are read twice like any long row, and a column counter passes 2^31."""

@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 import torch
 
-from luma_b200 import ffi, low
+from luma_b200 import ffi, high, low
 from oracle import binding as ob
 from tests import helpers as H
 
@@ -207,3 +207,28 @@ def test_row_counts_end_the_tensor_maps(lens, d, page):
         assert bool((o[t:] == -7.0).all()) and not bool(torch.isnan(o[:t]).any())
         got.append(o[:t])
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("d", [128, 64, 32])
+def test_an_output_that_is_only_16_byte_aligned(d):
+    # tiles that overhang their sequence go out from registers, in stores of 32 bytes where the output allows them and of 16 where not
+    lens, hq, hkv = [130, 17, 300, 128, 65], 4, 2
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(d)
+    q, k, v = (torch.randn((sum(lens), h, d), generator=g, device="cuda", dtype=torch.bfloat16) for h in (hq, hkv, hkv))
+    outs = []
+    for ahead in (16, 8):                              # 32 and 16 bytes
+        room = torch.full((q.numel() + 32,), -7.0, device="cuda", dtype=torch.bfloat16)
+        o = room[ahead:ahead + q.numel()].view(q.shape)
+        assert o.data_ptr() % 32 == (0 if ahead == 16 else 16)
+        low.flash_attn_varlen(q, k, v, o, cu, cu, len(lens), max(lens), max(lens), hq, hkv, d, 1.0 / np.sqrt(d), total_q=sum(lens), total_k=sum(lens))
+        torch.cuda.synchronize()
+        assert ffi.last_path() == "prefill_tcgen05" and ffi.device_status() == 0
+        assert bool((room[:ahead] == -7.0).all()) and bool((room[ahead + q.numel():] == -7.0).all())
+        outs.append(o)
+    assert torch.equal(*outs)
+    at = 0
+    for n in lens:
+        alone = high.flash_attn_func(q[None, at:at + n], k[None, at:at + n], v[None, at:at + n])
+        assert float((alone[0].float() - outs[1][at:at + n].float()).abs().max()) <= 2e-2     # one rounding of weights and result, other kernels for few rows
+        at += n
