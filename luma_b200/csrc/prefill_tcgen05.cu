@@ -971,7 +971,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     // producer/issuer warpgroup hands most of its share to the two softmax warpgroups, which
     // keep a whole 128-column score row per thread in registers.
     if (warp >= 8) {
-    // The packed buffers' ends that the tensor maps do not know.
+    // One instruction for the four warps, as the instruction wants it, and ahead of what they do first: the softmax warps wait for the registers that all four give back. Behind
+    // the K producer's first copies (which have no use for more than 88) 2 x 128, 32/8 heads took 7.2 us instead of 6.6 from a graph, 2 x 433 MHA 11.0 and 10.7.
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n");
+    // Packed buffers whose ends the tensor maps do not know.
     const bool q_open = packed && !a.q_bounded, kv_open = packed && !a.paged && !a.kv_bounded;
     Item w;                // K producer: the tile pair at hand
     bool begun = false;    // ... and whether the first one's first copies have been requested
@@ -994,6 +997,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 tma_load_4d(sm.q[1], &q_map, &sm.q_full[1], 0, w.t[1].head, w.sq.q_crow + w.t[1].row0, w.sq.q_cb);
                 if (D == 128) tma_load_4d(sm.q[1] + kHalfBytes, &q_map, &sm.q_full[1], 64, w.t[1].head, w.sq.q_crow + w.t[1].row0, w.sq.q_cb);
             }
+        }
+        if (lane == 0 && w.some) {   // (published here, the other roles have read it when the first scores come)
+            sm.item[0] = w;
+            mbar_arrive(&sm.item_full[0]);
         }
         __syncwarp();
     } else if (warp == kLoadWarpV) {
@@ -1028,9 +1035,6 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         asm volatile("barrier.cta.arrive 1, 96;\n" ::: "memory");    // the producers
         asm volatile("barrier.cta.arrive 2, 320;\n" ::: "memory");   // issuer and softmax warps, which wait for tensor memory as well
     }
-    // One instruction for the four warps, as the instruction wants it. The softmax warps get the registers that all four give back: none before the first copies have been
-    // requested, and there is nothing to do for them before.
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n");
     if (warp == kLoadWarp) {
         // ------------------------------ tile pairs, Q and K tiles ------------------------------
         // The warps run their loops whole; lane 0 issues the bulk copies (a paged tile: a lane per page), and all lanes share the
@@ -1058,6 +1062,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             ++requests;
             FA_TRACE_EVENT(3, (int)requests, 0);
         };
+        const bool have = w.some;            // the CTA's own tile pair is published
         bool owed = false;                   // the arrival that the last step of the pair before waits for, in place of another K tile
         auto owed_commit = [&]() { return (g & 1) ? k_free1 : k_free0; };
         for (unsigned it = 0;; ++it) {
@@ -1093,7 +1098,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 if (!alive) break;
             }
             if (!w.some) w.t[0].n_kv = w.t[1].n_kv = 0;
-            if (lane == 0 && (!kOnePair || it == 0)) {
+            if (lane == 0 && (kOnePair ? it == 0 && !w.some : it > 0 || !have)) {
                 sm.item[it & 1u] = w;
                 mbar_arrive(&sm.item_full[it & 1u]);
             }
@@ -1886,13 +1891,13 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
         grid = dim3((unsigned)ctas);
     }
     // Where the grid has no more CTAs than the device has SMs there is no pair to take over, and such a call runs without the loop over pairs, whose counters and cases cost the
-    // first copies, the step (2 to 3 %) and, over pages, the producers' registers. us with the loop and without, from a graph: 1 x 658, 32/8 heads 15.6 and 15.3; 2 x 433 MHA 11.4 and
-    // 11.0; 1 x 4096, 4/4 heads 52.4 and 51.6; 3 x 5 tokens over 46-747 18.9 and 17.7; 16 x 64 tokens over 1024-8192, 8/8 heads 108 and 100. Not asking for a pair alone, in the same
+    // step (up to 2 %) and, over pages, the producers' registers. us with the loop and without, from a graph: 1 x 658, 32/8 heads 15.2 and 14.9; 2 x 433 MHA 11.4 and
+    // 10.9; 1 x 4096, 4/4 heads 52.2 and 51.2; 3 x 5 tokens over 46-747 18.7 and 17.7; 16 x 64 tokens over 1024-8192, 8/8 heads 104 and 101.6. Not asking for a pair alone, in the same
     // code, gave 0.1 us. Nor has a call in order much to take over: a CTA that has asked starts a pair about 2 us later, and those that start by themselves take
-    // the next one just as well (4 chunks of 512 over 1024-8192 142 and 139.5, 4 of 300 over 2048-8192 125.5 and 122.6, 8 of 512 247 either way). With few-row sequences left out
-    // a grid in order has empty CTAs, which are cheaper to take over (serve steps of 4 chunks with 32 tokens 225 and 229, 6 with 40 308 and 317), and so are short pairs at head size
-    // 64 (8 x 200 over 512-4096, 32/8 heads 69 and 71). Contiguous K/V at head size 64: no difference (1 x 449, 64/8 heads of 32 11.6 either way; 1 x 2048, 8/8 heads 26.8 and 27.3), and
-    // none is built.
+    // the next one just as well (4 chunks of 512 over 1024-8192 140 and 138, 4 of 300 over 2048-8192 124.8 and 123.4, 8 of 512 246 and 247). With few-row sequences left out
+    // a grid in order has empty CTAs, which are cheaper to take over (serve steps of 4 chunks with 32 tokens 226 and 228, 6 with 40 310 and 318), and so are short pairs at head size
+    // 64 (8 x 200 over 512-4096, 32/8 heads 68.5 and 69.6). Contiguous K/V at head size 64: no difference (1 x 449, 64/8 heads of 32 11.6 either way; 1 x 2048, 8/8 heads 26.8 and
+    // 27.3), and none is built.
     constexpr bool kOneWave = D == 128 || kPaged;
     const bool one_pair = kOneWave && ((long long)grid.x * grid.y * grid.z <= sm_count() || (D == 128 && a.ordered && a.skip_rows == 0));
     const auto kernel = one_pair ? prefill_tcgen05_kernel<T, D, kMask, kPaged, kOneWave> : prefill_tcgen05_kernel<T, D, kMask, kPaged, false>;
