@@ -11,7 +11,8 @@
 // One CTA (384 threads, 1 per SM) works on a pair of query tiles of 128 rows that share a batch
 // element and a KV head — two query heads of one GQA group at the same row block, or two
 // consecutive row blocks of one head when the group is 1 (tile 0 the later one) — and streams that KV head's K/V tiles
-// (128 keys) past both; then it takes over the pair of a CTA of the grid that has not started (clusterlaunchcontrol), until none is left:
+// (128 keys) past both; then it takes over the pair of a CTA of the grid that has not started (clusterlaunchcontrol), until none is left
+// (an instantiation of one pair for grids where that wins nothing, see launch_variant):
 //   warps 0-3 / 4-7 : softmax warpgroup of query tile 0 / 1 — one thread per query row: read S
 //                     from tensor memory (tcgen05.ld), running max / sum in registers (exp2 with
 //                     the scale folded in), write P as packed 16-bit back over S (tcgen05.st),
@@ -53,7 +54,7 @@ constexpr int kBlockN = 128;   // keys per K/V tile
 // head size D (64 or 128) is a template parameter of the kernel
 constexpr int kStages = 2;     // depth of the K and V rings
 static_assert(kStages == 2, "step_full and step_done have an entry per stage, found by the parity of the step (j & 1, phase j >> 1) throughout the kernel");
-// A third V stage fits the shared memory and measured 5 % slower on every prefill workload (1165
+// A third V stage measured 5 % slower on every prefill workload when there was room for one, without the softmax warps' output rows (1165
 // against 1228 TFLOP/s at S = 8192); the issuer does not wait for the copies.
 constexpr int kThreads = 384;   // three warpgroups: softmax 0, softmax 1, and producers + issuer (+ an idle warp)
 constexpr int kLoadWarp = 8;
@@ -976,9 +977,12 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n");
     // Packed buffers whose ends the tensor maps do not know.
     const bool q_open = packed && !a.q_bounded, kv_open = packed && !a.paged && !a.kv_bounded;
-    Item w;                // K producer: the tile pair at hand
-    bool begun = false;    // ... and whether the first one's first copies have been requested
     if (warp == kLoadWarp) {
+        // ------------------------------ tile pairs, Q and K tiles ------------------------------
+        // The warps run their loops whole; lane 0 issues the bulk copies (a paged tile: a lane per page), and all lanes share the
+        // plain-load copy of a tile at the very end of a packed buffer.
+        Item w;
+        bool begun = false;   // the first tile pair's first copies have been requested
         // The CTA's own tile pair, and its first copies at once, in as few instructions as that takes: all of them come in for the first time here, and
         // in the loop below, with its waits and cases, the first S came 1600 to 2300 clocks later (a fifth of a call of one short wave).
         w.some = find_pair<kPaged>(a, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, lane, w);
@@ -1003,42 +1007,6 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             mbar_arrive(&sm.item_full[0]);
         }
         __syncwarp();
-    } else if (warp == kLoadWarpV) {
-        asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
-    } else if (warp != kMmaWarp) {
-        // Set-up, by the warp that has nothing else to do, while the K producer finds out what the CTA's first tile pair is.
-        if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&q_map) : "memory");
-            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&k_map) : "memory");
-            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&v_map) : "memory");
-            sm.abort_flag = 0;
-            sm.left_out = 0;
-            for (int i = 0; i < 2; ++i) {
-                mbar_init(&sm.item_full[i], 1);
-                mbar_init(&sm.item_empty[i], 10);
-                mbar_init(&sm.q_full[i], 1);
-                mbar_init(&sm.s_full[i], 1);
-                mbar_init(&sm.o_full[i], 1);
-                mbar_init(&sm.p_ready[0][i], 128);
-                mbar_init(&sm.p_ready[1][i], 128);
-                mbar_init(&sm.step_full[i], 2);
-            }
-            for (int i = 0; i < kDone; ++i) mbar_init(&sm.step_done[i], 1);
-            mbar_init(&sm.answered, 1);
-            mbar_init(&sm.k_first, 1);
-            mbar_init(&sm.v_tail, 1);
-            mbar_init(&sm.drain, 1);
-            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        }
-        __syncwarp();
-        asm volatile("barrier.cta.arrive 1, 96;\n" ::: "memory");    // the producers
-        asm volatile("barrier.cta.arrive 2, 320;\n" ::: "memory");   // issuer and softmax warps, which wait for tensor memory as well
-    }
-    if (warp == kLoadWarp) {
-        // ------------------------------ tile pairs, Q and K tiles ------------------------------
-        // The warps run their loops whole; lane 0 issues the bulk copies (a paged tile: a lane per page), and all lanes share the
-        // plain-load copy of a tile at the very end of a packed buffer.
         const long long tot_q = q_open ? (long long)a.cu_q[a.batch] : 0;
         const long long tot_k = kv_open ? (long long)a.cu_k[a.batch] : 0;
         int g = 0, commits = 0;              // steps and commits on step_done of the tile pairs before this one
@@ -1210,6 +1178,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         // ------------------------------ V tiles ------------------------------
         // A producer of its own: with a paged cache a tile is one copy per page and 64-column half plus a block-table read per page, and a single
         // thread issuing both rings cannot keep up with the tensor pipe at small page sizes.
+        asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
         const long long tot_k = kv_open ? (long long)a.cu_k[a.batch] : 0;
         int g = 0, commits = 0;
         int v_free0 = -1, v_free1 = -1;
@@ -1296,6 +1265,36 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         }
 #endif
         issue_products<T, D, kOnePair>(smem_u32(&sm), sm.tmem_base, a.status, a.wait_ns FA_TRACE_ARG(trace));
+    } else {
+        // ------------------------------ set-up ------------------------------
+        // By the warp that has nothing else to do, while the K producer finds out what the CTA's first tile pair is.
+        if (lane == 0) {
+            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&q_map) : "memory");
+            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&k_map) : "memory");
+            asm volatile("prefetch.tensormap [%0];\n" ::"l"(&v_map) : "memory");
+            sm.abort_flag = 0;
+            sm.left_out = 0;
+            for (int i = 0; i < 2; ++i) {
+                mbar_init(&sm.item_full[i], 1);
+                mbar_init(&sm.item_empty[i], 10);
+                mbar_init(&sm.q_full[i], 1);
+                mbar_init(&sm.s_full[i], 1);
+                mbar_init(&sm.o_full[i], 1);
+                mbar_init(&sm.p_ready[0][i], 128);
+                mbar_init(&sm.p_ready[1][i], 128);
+                mbar_init(&sm.step_full[i], 2);
+            }
+            for (int i = 0; i < kDone; ++i) mbar_init(&sm.step_done[i], 1);
+            mbar_init(&sm.answered, 1);
+            mbar_init(&sm.k_first, 1);
+            mbar_init(&sm.v_tail, 1);
+            mbar_init(&sm.drain, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        }
+        __syncwarp();
+        asm volatile("barrier.cta.arrive 1, 96;\n" ::: "memory");    // the producers
+        asm volatile("barrier.cta.arrive 2, 320;\n" ::: "memory");   // issuer and softmax warps, which wait for tensor memory as well
     }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 208;\n");

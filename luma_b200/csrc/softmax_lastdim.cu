@@ -330,8 +330,9 @@ int launch_softmax(const T* in, T* out, long long rows, int n, cudaStream_t stre
         } else {
             // Rows as long as this pay for aligned vectors with masked ends; in single elements a bf16 row of 4099 took 415 us where this takes 189
             // (60000 rows), one of 1413 86 and 57 (f16, 46713 rows). CTAs of just as many warps as a row needs: in CTAs of a power of two,
-            // lengths just above one had twice the threads. Two CTAs of more than 512 threads do not fit an SM's registers: up to an eighth
-            // above, each thread takes a vector more (8000 rows of 16383 bf16: 105 us, 155 without).
+            // lengths just above one had twice the threads. Two CTAs of more than 512 threads do not fit an SM's registers: just
+            // above, each thread takes a vector more, five instead of four in 16 bits (up to a quarter above), nine instead of eight in f32 (up to an eighth):
+            // 8000 rows of 16383 bf16 105 us, 155 without.
             constexpr int kEach = 32 / kWide;
             const unsigned all = (unsigned)(n + 2 * kWide - 2) / kWide;   // (a row begins up to kWide - 1 elements into its first vector)
             auto fit = [&](unsigned each) { return (all + each * 32 - 1) / (each * 32) * 32; };
