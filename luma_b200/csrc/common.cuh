@@ -123,6 +123,32 @@ __host__ __device__ inline int launch_rank(int by, int w, int m) {
     return by;
 }
 
+// Division of n < 2^31 by a divisor the host knows, as a product with its rounded-up inverse (Granlund and Montgomery, "Division by
+// invariant integers using multiplication"): a product, a sum and a shift. With the division operator, a CTA made ten divisions by run-time values one after
+// the other before its first copy was requested, and knew its extents 1700 clocks from its start (timeline), on an SM with nothing else to do.
+struct FastDiv {
+    unsigned mul, shift;
+    int d;
+    FastDiv() = default;
+    __host__ explicit FastDiv(int divisor) : mul(0), shift(0), d(divisor) {
+        while ((1u << shift) < (unsigned)d) ++shift;
+        mul = (unsigned)((((1ULL << shift) - (unsigned)d) << 32) / (unsigned)d) + 1u;
+    }
+    __device__ __forceinline__ int div(int n) const { return (int)((__umulhi((unsigned)n, mul) + (unsigned)n) >> shift); }
+};
+
+// Query heads of a GQA group that share a tile of the tensor-core prefill kernel: the largest power of two, up to the 32 rows that a warp
+// stores at a time, that divides the group.
+__host__ __device__ inline int pack_of(int group) {
+    const int low = group & -group;
+    return low < 32 ? low : 32;
+}
+// Pairs of 128-row tiles that q_len query tokens make for a KV head there.
+__host__ __device__ inline long long prefill_pairs(int group, long long q_len) {
+    const int pack = pack_of(group);
+    return ((long long)(group / pack) * ((q_len * pack + 127) / 128) + 1) / 2;
+}
+
 template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
@@ -190,6 +216,8 @@ struct RowsPlan {
 // family supports (the dispatcher then tries the next one).
 int launch_tile_simt(const AttnParams& p, cudaStream_t stream);
 int launch_tile_f32(const AttnParams& p, cudaStream_t stream);
+// (what launch_tile_f32 has found to be its own, with enough rows for a tile of 128)
+int launch_tile_f32_tcgen05(const AttnParams& p, cudaStream_t stream);
 int launch_decode_splitk(const AttnParams& p, cudaStream_t stream);
 // The same kernel for a few query rows per sequence through any entry point, where it is the faster one.
 int launch_few_rows(const AttnParams& p, bool prefill_takes_it, cudaStream_t stream);
@@ -220,6 +248,7 @@ int launch_kv_append(int elem_bytes, const void* k_new, const void* v_new, void*
 // was satisfied; otherwise the code of a wait that expired). The word is in mapped host memory:
 // prefill_take_status() only looks at it, prefill_device_status() synchronises the device first.
 int prefill_take_status();
+int* prefill_status_word();   // where a kernel whose bounded wait ran out leaves the wait's code; null: not to be had
 int prefill_device_status();
 // Copies the per-device debug area (status word, then from byte 256 the optional kernel timeline)
 // to host memory; returns the bytes copied or -1.

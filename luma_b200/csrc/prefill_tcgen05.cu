@@ -9,9 +9,12 @@
 // (kernels/flash_attn_varlen_func.cu:35-199), one-thread-per-query-row scalar kernels.
 //
 // One CTA (384 threads, 1 per SM) works on a pair of query tiles of 128 rows that share a batch
-// element and a KV head — two query heads of one GQA group at the same row block, or two
-// consecutive row blocks of one head when the group is 1 (tile 0 the later one) — and streams that KV head's K/V tiles
-// (128 keys) past both; then it takes over the pair of a CTA of the grid that has not started (clusterlaunchcontrol), until none is left
+// element and a KV head — two consecutive row blocks of the heads that share a tile (tile 0 the later one) — and streams that KV head's K/V tiles
+// (128 keys) past both. The rows of a tile are query token x head of the GQA group (as many heads as a power of two divides the group by, see pack_of): a tile
+// of 128 rows is 32 tokens of four heads, so that a sequence's last tile is partly empty once and not once for every head, and a few tokens fill one
+// tile together. A tile of 128 tokens for each head, and so (us): 1 x 658, 32/8 heads 15.0 and 13.7; 6 x 450-900 padded prompts at head size 64 76.2 and 68.5; 64 x 16
+// tokens over 4096 keys, 32/8 heads 400 and 189; 24 packed prompts of 17-2000, head size 64 250 and 243; row counts that fill the tiles either way, the same within 1 %. Then
+// it takes over the pair of a CTA of the grid that has not started (clusterlaunchcontrol), until none is left
 // (an instantiation of one pair for grids where that wins nothing, see launch_variant):
 //   warps 0-3 / 4-7 : softmax warpgroup of query tile 0 / 1 — one thread per query row: read S
 //                     from tensor memory (tcgen05.ld), running max / sum in registers (exp2 with
@@ -44,6 +47,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace fa {
 
@@ -81,8 +85,8 @@ struct SeqExtent {
 
 struct TileInfo {
     int valid;    // this query tile exists
-    int head;     // query head
-    int row0;     // first query row
+    int head;     // query head, the first of those that share the tile
+    int row0;     // first row, in rows of query token x head of the tile
     int n_kv;     // K/V tiles it needs
 };
 
@@ -132,20 +136,6 @@ constexpr int kCtaLogEntries = 2048;
 #endif
 constexpr unsigned long long kWaitLimitNs = 2000000000ULL;   // default bound of every mbarrier wait
 
-// Division of n < 2^31 by a divisor the host knows, as a product with its rounded-up inverse (Granlund and Montgomery, "Division by
-// invariant integers using multiplication"): a product, a sum and a shift. With the division operator, a CTA made ten divisions by run-time values one after
-// the other before its first copy was requested, and knew its extents 1700 clocks from its start (timeline), on an SM with nothing else to do.
-struct FastDiv {
-    unsigned mul, shift;
-    int d;
-    FastDiv() = default;
-    __host__ explicit FastDiv(int divisor) : mul(0), shift(0), d(divisor) {
-        while ((1u << shift) < (unsigned)d) ++shift;
-        mul = (unsigned)((((1ULL << shift) - (unsigned)d) << 32) / (unsigned)d) + 1u;
-    }
-    __device__ __forceinline__ int div(int n) const { return (int)((__umulhi((unsigned)n, mul) + (unsigned)n) >> shift); }
-};
-
 struct PrefillArgs {
     // Output: n_out buffers of (batch, q_seq_len, o_heads, 128), each receiving this launch's heads
     // at head offset o_head0. n_out == 1 with o_heads == q_heads is the ordinary call; with n_out > 1
@@ -170,7 +160,8 @@ struct PrefillArgs {
 #endif
     int batch, q_seq_len, kv_seq_len, q_heads, kv_heads, start_pos;
     int d_real;     // head size of the tensors: D, or 32 when the D = 64 kernel runs a head size of 32 on zero-padded tiles
-    FastDiv by_group, by_kv_heads, by_band;   // query heads per KV head; KV heads; band
+    int pack_log2;          // of the query heads that share a tile (pack_of): row r is query token r >> pack_log2, head r % pack of them
+    FastDiv by_packs, by_kv_heads, by_band;   // groups of `pack` query heads per KV head; KV heads; band
     int streams_z;  // (batch, KV head) streams per blockIdx.z
     int band;       // tile pairs of one (batch, KV head) that sit next to each other in blockIdx.x
     // Launch order of the bands (blockIdx.y), heaviest = 0. spread_w == 0: heaviest first. Otherwise the
@@ -196,57 +187,6 @@ struct PrefillArgs {
 };
 
 // ---- PTX wrappers -------------------------------------------------------------------------
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
-    asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
-    asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}\n" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait_at(unsigned bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_test_at(unsigned bar, unsigned parity) {   // (does not suspend)
-    unsigned ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) { return mbar_try_wait_at(smem_u32(bar), parity); }
-__device__ __forceinline__ bool shared_flag(unsigned addr) {
-    int f;
-    asm volatile("ld.volatile.shared.s32 %0, [%1];\n" : "=r"(f) : "r"(addr) : "memory");
-    return f != 0;
-}
-__device__ __forceinline__ int shared_int(unsigned addr) {
-    int f;
-    asm volatile("ld.shared.s32 %0, [%1];\n" : "=r"(f) : "r"(addr) : "memory");
-    return f;
-}
-__device__ __forceinline__ void mbar_arrive_at(unsigned bar) {
-    asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void set_shared_flag(unsigned addr) { asm volatile("st.volatile.shared.s32 [%0], 1;\n" ::"r"(addr) : "memory"); }
-__device__ __forceinline__ unsigned long long global_timer_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t));
-    return t;
-}
-
 // Bounded wait. Returns false when the wait was abandoned (time limit, or another thread of the
 // CTA already gave up); the caller then falls through to the end of the kernel.
 // The bound is counted in SM clocks (cheap to read, unlike the global nanosecond timer): wait_ns x 2 clocks, i.e. at least
@@ -392,63 +332,6 @@ __device__ __forceinline__ void store_32(void* to, const unsigned (&w)[8], bool 
     }
 }
 
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-
-// The products as the issuer warp runs them: the whole warp executes the instruction stream
-// converged and one elected lane issues. Keeping the warp uniform lets the descriptors live in
-// uniform registers; an election for each group of products instead of each product, and operands that the compiler can see to be the same for the
-// whole warp, take moves between the register files out (times at issue_products).
-__device__ __forceinline__ bool elect_one() {
-    unsigned e;
-    asm volatile("{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\nselp.u32 %0, 1, 0, e;\n}\n" : "=r"(e));
-    return e != 0;
-}
-// D[tmem] (+)= A[smem] * B[smem]
-__device__ __forceinline__ void tc_mma_ss(unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc, bool accumulate) {
-    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc),
-                 "r"(idesc), "r"((unsigned)accumulate)
-                 : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void tc_mma_ts(unsigned d_tmem, unsigned a_tmem, unsigned long long b_desc, unsigned idesc, bool accumulate) {
-    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc),
-                 "r"(idesc), "r"((unsigned)accumulate)
-                 : "memory");
-}
-// 32 lanes x 32 consecutive 32-bit columns: thread i of the warp <-> TMEM lane (base + i)
-__device__ __forceinline__ void tc_ld32(unsigned taddr, float (&r)[32]) {
-    unsigned* u = reinterpret_cast<unsigned*>(r);
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-        : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
-          "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]), "=r"(u[16]),
-          "=r"(u[17]), "=r"(u[18]), "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]), "=r"(u[24]),
-          "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tc_st32(unsigned taddr, const unsigned (&u)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};\n" ::"r"(
-            taddr),
-        "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]), "r"(u[9]),
-        "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15]), "r"(u[16]), "r"(u[17]), "r"(u[18]),
-        "r"(u[19]), "r"(u[20]), "r"(u[21]), "r"(u[22]), "r"(u[23]), "r"(u[24]), "r"(u[25]), "r"(u[26]), "r"(u[27]),
-        "r"(u[28]), "r"(u[29]), "r"(u[30]), "r"(u[31])
-        : "memory");
-}
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
-
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Maxima that are NaN where an operand is.
 __device__ __forceinline__ float max_nan(float a, float b) {
     float d;
@@ -504,45 +387,6 @@ __device__ __forceinline__ void ex2_fma2(float x0, float x1, float& p0, float& p
     p1 = __int_as_float(max(__float_as_int(q1) + (__float_as_int(t1) << 23), 0));
 }
 
-template <typename T> __device__ __forceinline__ unsigned pack16(float lo, float hi);
-template <> __device__ __forceinline__ unsigned pack16<__nv_bfloat16>(float lo, float hi) {
-    __nv_bfloat162 t = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<unsigned*>(&t);
-}
-template <> __device__ __forceinline__ unsigned pack16<__half>(float lo, float hi) {
-    __half2 t = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<unsigned*>(&t);
-}
-
-// Shared-memory matrix descriptor (tcgen05): 128-byte swizzle, descriptor version 1.
-//   bits [0,14)  start address >> 4      bits [16,30) leading byte offset >> 4
-//   bits [32,46) stride byte offset >> 4 bits [46,48) version = 1      bits [61,64) layout = 2 (SWIZZLE_128B)
-__device__ __forceinline__ unsigned long long make_desc(unsigned smem_addr, unsigned lbo_bytes, unsigned sbo_bytes) {
-    unsigned long long d = 0;
-    d |= (unsigned long long)((smem_addr & 0x3FFFFu) >> 4);
-    d |= (unsigned long long)((lbo_bytes >> 4) & 0x3FFFu) << 16;
-    d |= (unsigned long long)((sbo_bytes >> 4) & 0x3FFFu) << 32;
-    d |= 1ULL << 46;
-    d |= 2ULL << 61;
-    return d;
-}
-
-// Instruction descriptor, kind::f16: f32 accumulate, A/B both f16 or both bf16, M = 128, N = n.
-//   bits [4,6) D format (1 = f32)  [7,10) A format  [10,13) B format (0 = f16, 1 = bf16)
-//   bit 15 A major, bit 16 B major (0 = K-major, 1 = MN-major)  [17,23) N >> 3  [24,29) M >> 4
-template <typename T>
-__device__ __forceinline__ unsigned make_idesc(bool b_mn_major, int n) {
-    const unsigned fmt = sizeof(T) == 2 && std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
-    unsigned d = 0;
-    d |= 1u << 4;
-    d |= fmt << 7;
-    d |= fmt << 10;
-    d |= (b_mn_major ? 1u : 0u) << 16;
-    d |= (unsigned)(n >> 3) << 17;
-    d |= (unsigned)(kBlockM >> 4) << 24;
-    return d;
-}
-
 // Timeline slots: role (0/1 = softmax warpgroup, 2 = MMA issuer, 3 = K producer, by tile pair) x step of the CTA, over its tile pairs (< 60) x event (< 8).
 // Compiled in with -DFA_TRACE only; the default build carries none of it.
 [[maybe_unused]] constexpr int kTraceSteps = 60;
@@ -578,21 +422,24 @@ __device__ __forceinline__ SeqExtent seq_extent(const PrefillArgs& a, int s) {
     return e;
 }
 
-__device__ __forceinline__ TileInfo tile_info(const SeqExtent& a, int pair, int t, int kvh, const FastDiv& by_group, int num_mb) {
+// Tiles that the query tokens of a sequence fill for `pack` heads.
+static_assert(kBlockM == 1 << 7, "rows of a tile");
+__host__ __device__ __forceinline__ int row_blocks(int q_len, int pack_log2) { return (q_len + (kBlockM >> pack_log2) - 1) >> (7 - pack_log2); }
+
+__device__ __forceinline__ TileInfo tile_info(const SeqExtent& a, int pair, int t, int kvh, const FastDiv& by_packs, int pack_log2, int num_mb) {
     TileInfo ti;
-    // Tile 0 takes the later index of the pair: where the pair is two consecutive row blocks of one head
-    // (group 1), that is the longer tile, and tile 0 is the one whose copies are requested first and whose
+    // Tile 0 takes the later index of the pair: where the pair is two consecutive row blocks of the same heads,
+    // that is the longer tile, and tile 0 is the one whose copies are requested first and whose
     // products the issuer serves first in every step, so the tile that decides when the CTA ends is never
-    // the one that waits (S = 2048 MHA: 887-892 against 851 TFLOP/s; no difference for GQA pairs, whose
-    // two tiles are equally long).
+    // the one that waits (S = 2048 MHA: 887-892 against 851 TFLOP/s).
     const int idx = pair * 2 + (1 - t);
-    const int group = by_group.d;
-    ti.valid = idx < group * num_mb;
-    const int mb = ti.valid ? by_group.div(idx) : 0;
-    ti.head = kvh * group + (ti.valid ? idx - mb * group : 0);
+    const int packs = by_packs.d;
+    ti.valid = idx < packs * num_mb;
+    const int mb = ti.valid ? by_packs.div(idx) : 0;
+    ti.head = (kvh * packs + (ti.valid ? idx - mb * packs : 0)) << pack_log2;
     ti.row0 = mb * kBlockM;
-    const int last_row = min(ti.row0 + kBlockM, a.q_len) - 1;
-    const long long last_key = min((long long)a.kv_len - 1, (long long)a.pos_off + last_row);
+    const int last_token = (min(ti.row0 + kBlockM, a.q_len << pack_log2) - 1) >> pack_log2;
+    const long long last_key = min((long long)a.kv_len - 1, (long long)a.pos_off + last_token);
     ti.n_kv = (ti.valid && last_key >= 0) ? (int)(last_key / kBlockN) + 1 : 0;   // 0: the tile sees no key at all
     return ti;
 }
@@ -607,19 +454,20 @@ constexpr int kOrderMax = 32 * kOrderPerLane;
 constexpr int kOrderClasses = 8;
 
 // Tile pairs of one sequence whose longer tile sees at least w K/V tiles (w <= 0: all): pair p holds tiles 2p and
-// 2p + 1, tile i the row block i / group.
-__device__ __forceinline__ int pairs_from(int q_len, int kv_len, int group, int w) {
+// 2p + 1, tile i the row block i / packs.
+__device__ __forceinline__ int pairs_from(int q_len, int kv_len, int packs, int pack_log2, int w) {
     if (q_len <= 0) return 0;
-    const int pairs = (group * ((q_len + kBlockM - 1) / kBlockM) + 1) / 2;
+    const int pairs = (packs * row_blocks(q_len, pack_log2) + 1) / 2;
     if (w <= 0) return pairs;
     const long long key = (long long)(w - 1) * kBlockN;            // such a tile sees this key ...
-    const long long row = key - ((long long)kv_len - q_len);       // ... and so has this query row or a later one
-    if (key >= kv_len || row >= q_len) return 0;
-    return pairs - (int)(max(row, 0LL) / kBlockM) * group / 2;
+    const long long token = key - ((long long)kv_len - q_len);     // ... and so does this query token or a later one
+    if (key >= kv_len || token >= q_len) return 0;
+    return pairs - (int)((max(token, 0LL) << pack_log2) / kBlockM) * packs / 2;
 }
 
 // Returns {sequence or -1, KV head, pair}.
-__device__ __forceinline__ int3 find_item(const PrefillArgs& a, int group, int index, int lane) {
+__device__ __forceinline__ int3 find_item(const PrefillArgs& a, int index, int lane) {
+    const int packs = a.by_packs.d, pl = a.pack_log2, group = packs << pl;
     int ql[kOrderPerLane], kl[kOrderPerLane];
     const int per = (a.batch + 31) / 32;
     int most = 0;
@@ -632,7 +480,7 @@ __device__ __forceinline__ int3 find_item(const PrefillArgs& a, int group, int i
         const SeqExtent e = seq_extent(a, k);
         if (e.q_len <= 0 || e.q_len * group <= a.skip_rows) continue;
         // (a sequence longer than the call's max_seqlen_q has the grid's pairs and no more)
-        const int cut = max(0, e.q_len - (a.pairs * 2 + group - 1) / group * kBlockM);
+        const int cut = max(0, e.q_len - ((a.pairs * 2 + packs - 1) / packs * kBlockM >> pl));
         ql[i] = e.q_len - cut;
         kl[i] = e.kv_len - cut;
         most = max(most, kl[i] > 0 ? (kl[i] - 1) / kBlockN + 1 : 0);
@@ -645,7 +493,7 @@ __device__ __forceinline__ int3 find_item(const PrefillArgs& a, int group, int i
         for (int i = 0; i < kOrderPerLane; ++i) {
             x[i] = 0;
             if (i >= per) break;
-            x[i] = c < 0 ? 0 : min(a.pairs, pairs_from(ql[i], kl[i], group, c >= kOrderClasses ? 0 : most - (c + 1) * width + 1));
+            x[i] = c < 0 ? 0 : min(a.pairs, pairs_from(ql[i], kl[i], packs, pl, c >= kOrderClasses ? 0 : most - (c + 1) * width + 1));
             sum += x[i];
         }
         return __reduce_add_sync(0xffffffffu, sum) * a.kv_heads;
@@ -684,7 +532,7 @@ __device__ __forceinline__ int3 find_item(const PrefillArgs& a, int group, int i
             found = true;
             s = lane * per + i;
             kvh = rest / here;
-            const int pairs = min(a.pairs, pairs_from(ql[i], kl[i], group, 0));
+            const int pairs = min(a.pairs, pairs_from(ql[i], kl[i], packs, pl, 0));
             pair = pairs - 1 - before[i] - (rest - kvh * here);
         } else {
             rest -= here * a.kv_heads;
@@ -738,9 +586,9 @@ __device__ __forceinline__ void load_kv_tile(const PrefillArgs& a, int kv_crow, 
 // plain entry point 27 us, 23 so; 4 of 235-941, 8/2 heads, 39 and 31. (With the row counts given nothing comes this way, see q_open: 36 and 12 us, 38 and 22.)
 template <int D>
 __device__ __forceinline__ void edge_tile_copy(unsigned char* dst, const void* base, int heads, int head, long long row_start,
-                                               long long total_rows, unsigned long long* bar, int lane, int d_real) {
+                                               long long total_rows, unsigned long long* bar, int lane, int d_real, int pack_log2 = 0) {
     constexpr int kChunksPerRow = D / 8;   // 16-byte chunks per row of the tile (columns past d_real are zeros)
-    const long long left = total_rows - row_start;
+    const long long left = (total_rows - row_start) << pack_log2;   // rows of the tile: those of 1 << pack_log2 heads for each row of the buffer
     const int nrows = left < 0 ? 0 : (left > kBlockN ? kBlockN : (int)left);
     const unsigned char* src = static_cast<const unsigned char*>(base);
     const unsigned to = smem_u32(dst);
@@ -748,7 +596,7 @@ __device__ __forceinline__ void edge_tile_copy(unsigned char* dst, const void* b
     for (int idx = lane; idx < kBlockN * kChunksPerRow; idx += 32) {
         const int r = idx / kChunksPerRow, cc = idx % kChunksPerRow;
         const bool real = r < nrows && cc * 8 < d_real;
-        const unsigned char* from = real ? src + ((row_start + r) * heads + head) * (long long)(d_real * 2) + cc * 16 : src;
+        const unsigned char* from = real ? src + ((row_start + (r >> pack_log2)) * heads + head + (r & ((1 << pack_log2) - 1))) * (long long)(d_real * 2) + cc * 16 : src;
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to + (cc >> 3) * kHalfBytes + r * 128 + (((cc & 7) ^ (r & 7)) << 4)), "l"(from),
                      "r"(real ? 16 : 0)   // 0: nothing is read, zeros are written
                      : "memory");
@@ -913,10 +761,9 @@ __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int
 // The tile pair that CTA (bx, by, bz) of the grid stands for; false: there is none, or nothing to do for it. Run by one whole warp.
 template <bool kPaged>
 __device__ __forceinline__ bool find_pair(const PrefillArgs& a, int bx, int by, int bz, int lane, Item& w) {
-    const int group = a.by_group.d;
     int pair;
     if (kPaged && a.ordered) {
-        const int3 item = find_item(a, group, bx, lane);
+        const int3 item = find_item(a, bx, lane);
         w.seq = item.x; w.kv_head = item.y; pair = item.z;
         if (w.seq < 0) return false;
     } else {
@@ -935,10 +782,10 @@ __device__ __forceinline__ bool find_pair(const PrefillArgs& a, int bx, int by, 
         pair = ((int)gridDim.y - 1 - rank_y) * a.band + (a.band - 1 - (bx - x_band * a.band));
     }
     w.sq = seq_extent(a, w.seq);
-    if (w.sq.q_len * group <= a.skip_rows) return false;   // the few-row kernel's
-    const int num_mb = (w.sq.q_len + kBlockM - 1) / kBlockM;
-    w.t[0] = tile_info(w.sq, pair, 0, w.kv_head, a.by_group, num_mb);
-    w.t[1] = tile_info(w.sq, pair, 1, w.kv_head, a.by_group, num_mb);
+    if ((w.sq.q_len << a.pack_log2) * a.by_packs.d <= a.skip_rows) return false;   // the few-row kernel's
+    const int num_mb = row_blocks(w.sq.q_len, a.pack_log2);
+    w.t[0] = tile_info(w.sq, pair, 0, w.kv_head, a.by_packs, a.pack_log2, num_mb);
+    w.t[1] = tile_info(w.sq, pair, 1, w.kv_head, a.by_packs, a.pack_log2, num_mb);
     return w.t[0].valid || w.t[1].valid;   // (a sequence may be shorter than the grid's row range)
 }
 
@@ -992,14 +839,14 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             const int page = kPaged ? page_of_lane(a, w.sq.kv_len, w.seq, 0, lane) : -1;
             if (lane == 0 && w.t[0].n_kv > 0) {
                 mbar_expect_tx(&sm.q_full[0], TileBytes<D>::value);
-                tma_load_4d(sm.q[0], &q_map, &sm.q_full[0], 0, w.t[0].head, w.sq.q_crow + w.t[0].row0, w.sq.q_cb);
-                if (D == 128) tma_load_4d(sm.q[0] + kHalfBytes, &q_map, &sm.q_full[0], 64, w.t[0].head, w.sq.q_crow + w.t[0].row0, w.sq.q_cb);
+                tma_load_4d(sm.q[0], &q_map, &sm.q_full[0], 0, w.t[0].head, w.sq.q_crow + (w.t[0].row0 >> a.pack_log2), w.sq.q_cb);
+                if (D == 128) tma_load_4d(sm.q[0] + kHalfBytes, &q_map, &sm.q_full[0], 64, w.t[0].head, w.sq.q_crow + (w.t[0].row0 >> a.pack_log2), w.sq.q_cb);
             }
             load_kv_tile<D, kPaged>(a, w.sq.kv_crow, w.sq.kv_cb, w.kv_head, sm.k[0], &k_map, &sm.k_first, 0, page, lane);
             if (lane == 0 && w.t[1].n_kv > 0) {
                 mbar_expect_tx(&sm.q_full[1], TileBytes<D>::value);
-                tma_load_4d(sm.q[1], &q_map, &sm.q_full[1], 0, w.t[1].head, w.sq.q_crow + w.t[1].row0, w.sq.q_cb);
-                if (D == 128) tma_load_4d(sm.q[1] + kHalfBytes, &q_map, &sm.q_full[1], 64, w.t[1].head, w.sq.q_crow + w.t[1].row0, w.sq.q_cb);
+                tma_load_4d(sm.q[1], &q_map, &sm.q_full[1], 0, w.t[1].head, w.sq.q_crow + (w.t[1].row0 >> a.pack_log2), w.sq.q_cb);
+                if (D == 128) tma_load_4d(sm.q[1] + kHalfBytes, &q_map, &sm.q_full[1], 64, w.t[1].head, w.sq.q_crow + (w.t[1].row0 >> a.pack_log2), w.sq.q_cb);
             }
         }
         if (lane == 0 && w.some) {   // (published here, the other roles have read it when the first scores come)
@@ -1088,12 +935,12 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             }
             if (it > 0 && !q_open && lane == 0) {   // its Q on the way to L2 while the tiles before it are still in use
                 if (n0 > 0) {
-                    tma_prefetch_4d(&q_map, 0, w.t[0].head, w.sq.q_crow + w.t[0].row0, w.sq.q_cb);
-                    if (D == 128) tma_prefetch_4d(&q_map, 64, w.t[0].head, w.sq.q_crow + w.t[0].row0, w.sq.q_cb);
+                    tma_prefetch_4d(&q_map, 0, w.t[0].head, w.sq.q_crow + (w.t[0].row0 >> a.pack_log2), w.sq.q_cb);
+                    if (D == 128) tma_prefetch_4d(&q_map, 64, w.t[0].head, w.sq.q_crow + (w.t[0].row0 >> a.pack_log2), w.sq.q_cb);
                 }
                 if (n1 > 0) {
-                    tma_prefetch_4d(&q_map, 0, w.t[1].head, w.sq.q_crow + w.t[1].row0, w.sq.q_cb);
-                    if (D == 128) tma_prefetch_4d(&q_map, 64, w.t[1].head, w.sq.q_crow + w.t[1].row0, w.sq.q_cb);
+                    tma_prefetch_4d(&q_map, 0, w.t[1].head, w.sq.q_crow + (w.t[1].row0 >> a.pack_log2), w.sq.q_cb);
+                    if (D == 128) tma_prefetch_4d(&q_map, 64, w.t[1].head, w.sq.q_crow + (w.t[1].row0 >> a.pack_log2), w.sq.q_cb);
                 }
             }
             int page = kPaged ? page_of_lane(a, kv_len, seq, 0, lane) : -1;
@@ -1117,12 +964,13 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             auto load_q = [&](const TileInfo ti, unsigned char* to, unsigned long long* bar, unsigned& loads) {
                 if (ti.n_kv <= 0) return;
                 ++loads;
-                if (q_open && (long long)w.sq.q_crow + ti.row0 + kBlockM > tot_q) {
-                    edge_tile_copy<D>(to, a.q, a.q_heads, ti.head, (long long)w.sq.q_crow + ti.row0, tot_q, bar, lane, a.d_real);
+                const int token0 = ti.row0 >> a.pack_log2;
+                if (q_open && (long long)w.sq.q_crow + token0 + (kBlockM >> a.pack_log2) > tot_q) {
+                    edge_tile_copy<D>(to, a.q, a.q_heads, ti.head, (long long)w.sq.q_crow + token0, tot_q, bar, lane, a.d_real, a.pack_log2);
                 } else if (lane == 0) {
                     mbar_expect_tx(bar, TileBytes<D>::value);
-                    tma_load_4d(to, &q_map, bar, 0, ti.head, w.sq.q_crow + ti.row0, w.sq.q_cb);
-                    if (D == 128) tma_load_4d(to + kHalfBytes, &q_map, bar, 64, ti.head, w.sq.q_crow + ti.row0, w.sq.q_cb);
+                    tma_load_4d(to, &q_map, bar, 0, ti.head, w.sq.q_crow + token0, w.sq.q_cb);
+                    if (D == 128) tma_load_4d(to + kHalfBytes, &q_map, bar, 64, ti.head, w.sq.q_crow + token0, w.sq.q_cb);
                 }
             };
             // K tile 0 and the Q tiles: of the first pair in the order that the issuer wants them; else K first, which comes free first, then the Q tile that does, of
@@ -1323,8 +1171,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.item_empty[it & 1u]);
         if (!some) break;
-        const int row = ti.row0 + r;
-        const long long pos = (long long)sq.pos_off + row;      // global position of this query row
+        const int row = ti.row0 + r, pl = a.pack_log2;
+        const long long pos = (long long)sq.pos_off + (row >> pl);   // global position of this row's query token
+        // the last key that this row sees, and the last that every row of the tile sees (-1: none)
+        const int last_seen = (int)max(-1LL, min(pos, (long long)sq.kv_len - 1)), all_see = (int)max(-1LL, min((long long)sq.pos_off + (ti.row0 >> pl), (long long)sq.kv_len - 1));
         float m = -INFINITY;   // reference max, log2 domain (may lag the true max by <= 2^8)
         float l = 0.0f;
 
@@ -1336,9 +1186,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             tc_fence_after();
             const int key0 = j * kBlockN;
             // mask only where the causal diagonal or the end of K/V cuts through this tile
-            const long long limit_ll = min(pos, (long long)sq.kv_len - 1) - key0;
-            const bool need_mask = (long long)(key0 + kBlockN - 1) > min((long long)sq.pos_off + ti.row0, (long long)sq.kv_len - 1);
-            const int limit = need_mask ? (int)max(-1LL, min(limit_ll, (long long)kBlockN)) : kBlockN;
+            const bool need_mask = key0 + kBlockN - 1 > all_see;
+            const int limit = need_mask ? max(-1, min(last_seen - key0, kBlockN)) : kBlockN;
 
             // Masked scores become -inf, whose P is an exact zero from either exponential, so a masked tile runs the code of the others. (A form of its own
             // for the aligned diagonal, which left out the chunks of 32 keys that a warp does not see, and one for other masked tiles were straight-line
@@ -1443,7 +1292,8 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         FA_TRACE_EVENT(t, max(0, (int)steps - 1), 4);
         if (alive && ti.valid) {
             tc_fence_after();
-            const bool row_ok = row < sq.q_len;
+            const int rows_end = sq.q_len << pl, token = row >> pl, head = ti.head + (row & ((1 << pl) - 1));
+            const bool row_ok = row < rows_end;
             // with a padding mask a query row at a padded (or out-of-range) position outputs zeros (flash_attn_func.cu:77-84)
             bool q_ok = true;
             if (kMask) q_ok = row_ok && pos >= 0 && pos < (long long)sq.kv_len && a.mask[(long long)b * a.kv_seq_len + pos] != 0;
@@ -1458,7 +1308,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             constexpr bool staged_only = false;
 #endif
             unsigned char* const stage = sm.out[warp];
-            const bool bulk_ok = a.n_out == 1 && !a.multicast && !staged_only && (a.mode != MODE_VARLEN || ti.row0 + kBlockM <= sq.q_len);
+            const bool bulk_ok = a.n_out == 1 && !a.multicast && !staged_only && (a.mode != MODE_VARLEN || ti.row0 + kBlockM <= rows_end);
             if (bulk_ok) {
                 // Single output: the rows go out as bulk tensor stores. Each warp lays its 32 rows down in
                 // shared memory in the 128-byte-swizzled box layout, 64 columns at a time, and one lane issues one store of 32 rows x 64 columns. Plain 16-byte stores
@@ -1494,7 +1344,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");   // generic-proxy writes -> bulk copy reads
                     __syncwarp();
                     if (lane == 0) {
-                        tma_store_4d(&o_map, half, h * 64, a.o_head0 + ti.head, sq.q_crow + ti.row0 + (warp & 3) * 32, sq.q_cb);
+                        tma_store_4d(&o_map, half, h * 64, a.o_head0 + ti.head, sq.q_crow + ((ti.row0 + (warp & 3) * 32) >> pl), sq.q_cb);
                         asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
                     }
                 }
@@ -1506,7 +1356,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     __syncwarp();   // (lanes whose rows exist have stored)
                     tc_ld32(o_addr + c * 32, ov);
                     tc_wait_ld();
-                    T* const to = static_cast<T*>(a.o[0]) + ((sq.o_row0 + row) * a.o_heads + a.o_head0 + ti.head) * a.d_real + c * 32;
+                    T* const to = static_cast<T*>(a.o[0]) + ((sq.o_row0 + token) * a.o_heads + a.o_head0 + head) * a.d_real + c * 32;
                     if (row_ok && c * 32 < a.d_real) {
 #pragma unroll
                         for (int i = 0; i < 2; ++i) {
@@ -1561,9 +1411,9 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     for (int n = 0; n < kRowsAtOnce / kRowsPerStep; ++n) {
                         const int rr = n * kRowsPerStep + sub;
                         const int grow = part_row0 + rr;
-                        if (grow < sq.q_len && ch * 8 < a.d_real) {
+                        if (grow < rows_end && ch * 8 < a.d_real) {
                             const uint4 w = *reinterpret_cast<const uint4*>(stage + rr * kRowBytes + ((ch ^ (rr & (kChunks - 1))) << 4));
-                            const long long o_off = ((sq.o_row0 + grow) * a.o_heads + a.o_head0 + ti.head) * a.d_real + ch * 8;
+                            const long long o_off = ((sq.o_row0 + (grow >> pl)) * a.o_heads + a.o_head0 + ti.head + (grow & ((1 << pl) - 1))) * a.d_real + ch * 8;
                             // every GPU of a group starts its walk at a different buffer (peer0 = its own
                             // index + 1), so that at no time all of them store to the same GPU
                             if (a.multicast) {
@@ -1584,9 +1434,9 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             }
             if (row_ok && (a.lse != nullptr || a.n_lse > 0)) {
                 const float lse_val = seen ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
-                if (a.lse != nullptr) a.lse[((long long)b * a.q_heads + ti.head) * a.q_seq_len + row] = lse_val;
+                if (a.lse != nullptr) a.lse[((long long)b * a.q_heads + head) * a.q_seq_len + token] = lse_val;
                 // head-sharded call: the same value into the (batch, o_heads, q_seq_len) LSE of every GPU of the group
-                const long long g_off = ((long long)b * a.o_heads + a.o_head0 + ti.head) * a.q_seq_len + row;
+                const long long g_off = ((long long)b * a.o_heads + a.o_head0 + head) * a.q_seq_len + token;
                 for (int n = 0; n < a.n_lse; ++n) a.lse_peers[n][g_off] = lse_val;
             }
             FA_TRACE_EVENT(t, max(0, (int)steps - 1), 5);       // epilogue stores issued
@@ -1639,7 +1489,8 @@ EncodeFn get_encode_fn() {
 // (batch, seq, heads, 128) 16-bit tensor viewed as 4-D {d, head, seq, batch}; box = 64 x 1 x 128 x 1 (out: 64 x 1 x 32 x 1, what a softmax warp lays down at a time)
 // seq <= 0: a packed buffer whose row count the caller did not give (batch is 1 then). The row extent is
 // set beyond any buffer and the kernel never asks for a box that reaches past the real last row.
-bool encode_map(CUtensorMap* map, const void* base, int dtype, int d, int batch, int seq, int heads, bool out = false) {
+// pack: heads that share a tile, in neighbouring rows of a token: 64 x pack x 128 / pack x 1 (out: 64 x pack x 32 / pack x 1)
+bool encode_map(CUtensorMap* map, const void* base, int dtype, int d, int batch, int seq, int heads, int pack = 1, bool out = false) {
     EncodeFn fn = get_encode_fn();
     if (fn == nullptr) return false;
     const bool unbounded = seq <= 0;
@@ -1648,7 +1499,7 @@ bool encode_map(CUtensorMap* map, const void* base, int dtype, int d, int batch,
     // the stride of the batch axis is never used when batch is 1; it only has to be a legal value
     const cuuint64_t strides[3] = {(cuuint64_t)d * 2, (cuuint64_t)heads * d * 2,
                                    unbounded ? (cuuint64_t)heads * d * 2 * 128 : (cuuint64_t)seq * heads * d * 2};
-    const cuuint32_t box[4] = {64, 1, out ? 32u : (cuuint32_t)kBlockM, 1};
+    const cuuint32_t box[4] = {64, (cuuint32_t)pack, (out ? 32u : (cuuint32_t)kBlockM) / (cuuint32_t)pack, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUtensorMapDataType dt = dtype == DT_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     const CUresult rc = fn(map, dt, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1730,12 +1581,13 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     // head size 32 runs on the D = 64 kernel: the maps carry the real inner extent (32), the 64-column
     // boxes read zeros past it and bulk stores write nothing there
     const int d_real = p.head_size;
-    bool ok = encode_map(&qm, p.q, p.dtype, d_real, q_batch, q_rows, p.q_heads);
+    const int group = p.q_heads / p.kv_heads, pack = pack_of(group);
+    bool ok = encode_map(&qm, p.q, p.dtype, d_real, q_batch, q_rows, p.q_heads, pack);
     // The output as boxes of 32 rows. Bulk stores are used for a single, local output
     // only: a head-sharded call (n_out > 0) stores every copy with plain stores, and no tensor map is
     // ever made over another GPU's memory — the kernel's fourth map is then a second one over q, unused.
     if (p.n_out > 0) om = qm;
-    else ok = ok && encode_map(&om, p.o, p.dtype, d_real, q_batch, q_rows, p.q_heads, true);
+    else ok = ok && encode_map(&om, p.o, p.dtype, d_real, q_batch, q_rows, p.q_heads, pack, true);
     if (p.paged) {
         ok = ok && encode_paged_map(&km, p.k, p.dtype, d_real, p.block_size, p.kv_heads) &&
              encode_paged_map(&vm, p.v, p.dtype, d_real, p.block_size, p.kv_heads);
@@ -1802,9 +1654,9 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     a.kv_bounded = p.total_k > 0;
     a.scale_log2 = p.scale * 1.4426950408889634f;
 
-    const int group = p.q_heads / p.kv_heads;
-    const int num_mb = (p.q_seq_len + kBlockM - 1) / kBlockM;
-    const int pairs = (group * num_mb + 1) / 2;
+    const int packs = group / pack;
+    while ((1 << a.pack_log2) < pack) ++a.pack_log2;
+    const int pairs = (packs * row_blocks(p.q_seq_len, a.pack_log2) + 1) / 2;
     const size_t smem = sizeof(SharedStorage<D>) + 1024;
     // Band width: the pairs of a band start together, so their work must be about equal or the
     // heaviest-first order is lost (at S = 2048 without GQA, bands of 2 cost 13 %). A band of w
@@ -1820,7 +1672,7 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     a.band = band;
     a.by_band = FastDiv(band);
     a.by_kv_heads = FastDiv(p.kv_heads);
-    a.by_group = FastDiv(group);
+    a.by_packs = FastDiv(packs);
     // Head-sharded call (every CTA ends with stores to the other GPUs): heaviest-first makes the SMs end
     // their CTAs in waves, each wave a burst on the links that stalls every SM in it. A first wave that
     // mixes all weights staggers the SMs for the rest of the launch; the rest stays heaviest first, which
@@ -1875,11 +1727,12 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     // 512-2048, 32/32 heads (7 waves) 161-172 and 166-186; 4 chunks of 64 over 128-512 (less than a wave) 17-19 and 19-21.
     const long long kv_rows = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
     const PackedMix mix = packed_mix(p);
-    const double waves = (double)(mix.prompts * pairs + (a.skip_rows > 0 ? 0 : mix.few * ((group + 1) / 2))) * p.kv_heads / sm_count();
+    const long long few_pairs = (packs + 1) / 2;   // of a sequence whose rows fit one block
+    const double waves = (double)(mix.prompts * pairs + (a.skip_rows > 0 ? 0 : mix.few * few_pairs)) * p.kv_heads / sm_count();
     const long long all = (long long)p.num_seqs * p.kv_heads * pairs;
     long long ctas = all;
-    if (p.total_q > 0)   // a sequence of n rows has (group * ceil(n / 128) + 1) / 2 pairs
-        ctas = std::min(ctas, p.kv_heads * ((group * (((long long)p.total_q + 127LL * p.num_seqs) / 128) + p.num_seqs) / 2));
+    if (p.total_q > 0)   // a sequence of n tokens has (packs * ceil(n * pack / 128) + 1) / 2 pairs
+        ctas = std::min(ctas, p.kv_heads * ((packs * (((long long)p.total_q * pack + 127LL * p.num_seqs) / 128) + p.num_seqs) / 2));
     // ... and where most of the grid would be empty CTAs of sequences that are left to the few-row kernel: a launch in order has no more than
     // the rows can make (one chunk of 512 with 128 tokens over 128-2048, 32/8 heads: 8256 CTAs or 2644, 191 us or 153).
     const bool worth_ordering = (waves > 1.0 && (double)((kv_rows + kBlockN - 1) / kBlockN) > 5.0 * waves) || (a.skip_rows > 0 && all > 2 * ctas);
@@ -1920,6 +1773,8 @@ int launch_typed(const AttnParams& p, cudaStream_t stream) {
 }
 
 }  // namespace
+
+int* prefill_status_word() { return status_word(); }
 
 int prefill_take_status() {
     int* status = status_word();
@@ -1982,8 +1837,7 @@ int launch_prefill_tcgen05(const AttnParams& p, cudaStream_t stream) {
                       reinterpret_cast<uintptr_t>(p.v) | reinterpret_cast<uintptr_t>(p.o);
     for (int i = 0; i < p.n_out && i < 8; ++i) align |= reinterpret_cast<uintptr_t>(p.o_peers[i]);
     if (align & 15) return -1;
-    const long long pairs = ((long long)(p.q_heads / p.kv_heads) * ((p.q_seq_len + kBlockM - 1) / kBlockM) + 1) / 2;
-    if (pairs > 65535) return -1;
+    if (prefill_pairs(p.q_heads / p.kv_heads, p.q_seq_len) > 65535) return -1;
     if (p.head_size == 64 || p.head_size == 32) return p.dtype == DT_BF16 ? launch_typed<__nv_bfloat16, 64>(p, stream) : launch_typed<__half, 64>(p, stream);
     return p.dtype == DT_BF16 ? launch_typed<__nv_bfloat16, 128>(p, stream) : launch_typed<__half, 128>(p, stream);
 }
