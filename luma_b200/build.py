@@ -34,7 +34,7 @@ def host_path_file() -> Path:
     return LIB_DIR / f"_host.{sysconfig.get_config_var('SOABI')}.torch-{importlib.metadata.version('torch')}.so"
 
 
-SOURCES = ["api.cu", "tile_simt.cu", "tile_f32.cu", "decode_splitk.cu", "prefill_tcgen05.cu", "kv_append.cu", "softmax_lastdim.cu", "comm.cu", "host_pipe.cu"]
+SOURCES = ["api.cu", "tile_simt.cu", "tile_f32.cu", "tile_f32_tcgen05.cu", "decode_splitk.cu", "prefill_tcgen05.cu", "kv_append.cu", "softmax_lastdim.cu", "comm.cu", "host_pipe.cu"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

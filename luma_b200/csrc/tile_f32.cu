@@ -23,6 +23,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "tile_f32.cuh"
 
 namespace fa {
 
@@ -62,66 +63,6 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const unsigned (&a)[4], 
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// Two values -> three packed bf16 pairs whose sum is the pair (the differences are exact).
-__device__ __forceinline__ void split3(float x, float y, unsigned& hi, unsigned& mid, unsigned& lo) {
-    auto pack = [](float a, float b) {
-        __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
-        return *reinterpret_cast<unsigned*>(&t);
-    };
-    hi = pack(x, y);
-    const float x1 = x - __uint_as_float(hi << 16), y1 = y - __uint_as_float(hi & 0xffff0000u);
-    mid = pack(x1, y1);
-    lo = pack(x1 - __uint_as_float(mid << 16), y1 - __uint_as_float(mid & 0xffff0000u));
-}
-
-// The rows of a CTA that met a value that does not survive the split, one key at a time in plain f32, as tile_simt.cu
-// does it: a warp per row. An infinity minus itself, and infinity times the other operand's small terms, are NaN where the
-// product is not, and so is zero weight times a row that a query does not see; the same holds for a value that rounds
-// to a bf16 infinity. Each leaves a NaN in the sums that it reaches, which is where the kernel looks, once at its end.
-template <int D>
-__device__ __noinline__ void plain_rows(const AttnParams& p, int s, int kvh, int row0, int row_end) {
-    const SeqInfo si = seq_info(p, s);
-    const uint8_t* mask_row = p.mask ? p.mask + (long long)s * p.kv_seq_len : nullptr;
-    constexpr int E = D / 32;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = p.q_heads / p.kv_heads;
-    const float* kg = static_cast<const float*>(p.k);
-    const float* vg = static_cast<const float*>(p.v);
-    for (int r = row0 + warp; r < row_end; r += kWarps) {
-        const int t = r / group, h = kvh * group + r - t * group;
-        const long long pos = (long long)si.pos_off + t, at = ((si.q_row0 + t) * p.q_heads + h) * D;
-        const int end = (int)max(0LL, min((long long)si.kv_len, pos + 1));
-        float q[E], acc[E], m = -INFINITY, l = 0.0f;
-        for (int e = 0; e < E; ++e) {
-            q[e] = static_cast<const float*>(p.q)[at + lane + 32 * e];
-            acc[e] = 0.0f;
-        }
-        for (int j = 0; j < end; ++j) {
-            if (mask_row != nullptr && mask_row[j] == 0) continue;
-            const long long row = p.paged ? (long long)block_slot(p.block_tables, s, p.max_blocks, j, p.block_size) : si.kv_row0 + j;
-            const long long off = (row * p.kv_heads + kvh) * D + lane;
-            float part = 0.0f;
-            for (int e = 0; e < E; ++e) part = fmaf(q[e], kg[off + 32 * e], part);
-            for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-            const float sc = part * p.scale, m_new = fmaxf(m, sc);
-            const float alpha = __expf(m - m_new), pr = __expf(sc - m_new);
-            l = l * alpha + pr;
-            for (int e = 0; e < E; ++e) acc[e] = acc[e] * alpha + pr * vg[off + 32 * e];
-            m = m_new;
-        }
-        const bool ok = l > 0.0f && (mask_row == nullptr || (pos >= 0 && pos < si.kv_len && mask_row[pos] != 0));
-        const float inv = ok ? 1.0f / l : 0.0f;
-        for (int e = 0; e < E; ++e) static_cast<float*>(p.o)[at + lane + 32 * e] = acc[e] * inv;
-        if (p.lse != nullptr && lane == 0)
-            p.lse[((long long)s * p.q_heads + h) * p.q_seq_len + t] = ok ? m + __logf(l) : -INFINITY;
-    }
-}
-
 template <int D, int WR>
 __global__ void __launch_bounds__(kThreads, 2) tile_f32_kernel(const __grid_constant__ AttnParams p) {
     using S = Shape<D, WR>;
@@ -361,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, 2) tile_f32_kernel(const __grid_cons
 #pragma unroll
         for (int e = 0; e < 4; ++e) probe = fmaf(0.0f, acc[n][e], probe);
     if (__syncthreads_or(probe != 0.0f)) {
-        plain_rows<D>(p, s, kvh, row0, min(rows, row0 + S::kRows));
+        plain_rows<D, kWarps>(p, s, kvh, row0, min(rows, row0 + S::kRows));
         return;
     }
 
@@ -462,6 +403,8 @@ int launch_tile_f32(const AttnParams& p, cudaStream_t stream) {
         return -1;
     const long long rows = (long long)p.q_seq_len * (p.q_heads / p.kv_heads);
     if (rows > 0x7fffffffLL - 64) return -1;
+    const int rc = launch_tile_f32_tcgen05(p, stream);
+    if (rc >= 0) return rc;
     const bool large = (rows + 63) / 64 * p.kv_heads * p.num_seqs >= 2LL * sm_count();   // two CTAs per SM
     if (p.head_size == 128) return large ? launch_one<128, 4>(p, stream) : launch_one<128, 2>(p, stream);
     if (p.head_size == 64) return large ? launch_one<64, 4>(p, stream) : launch_one<64, 1>(p, stream);
