@@ -426,6 +426,13 @@ __device__ __forceinline__ SeqExtent seq_extent(const PrefillArgs& a, int s) {
 static_assert(kBlockM == 1 << 7, "rows of a tile");
 __host__ __device__ __forceinline__ int row_blocks(int q_len, int pack_log2) { return (q_len + (kBlockM >> pack_log2) - 1) >> (7 - pack_log2); }
 
+// One past the last query token of tile `idx` of a sequence, or of its last tile.
+__device__ __forceinline__ int tile_token_end(const SeqExtent& a, int idx, const FastDiv& by_packs, int pack_log2, int num_mb) {
+    const int mb = idx < by_packs.d * num_mb ? by_packs.div(idx) : num_mb - 1;
+    return min((mb + 1) * (kBlockM >> pack_log2), a.q_len);
+}
+
+template <bool kMask>
 __device__ __forceinline__ TileInfo tile_info(const SeqExtent& a, int pair, int t, int kvh, const FastDiv& by_packs, int pack_log2, int num_mb) {
     TileInfo ti;
     // Tile 0 takes the later index of the pair: where the pair is two consecutive row blocks of the same heads,
@@ -441,6 +448,7 @@ __device__ __forceinline__ TileInfo tile_info(const SeqExtent& a, int pair, int 
     const int last_token = (min(ti.row0 + kBlockM, a.q_len << pack_log2) - 1) >> pack_log2;
     const long long last_key = min((long long)a.kv_len - 1, (long long)a.pos_off + last_token);
     ti.n_kv = (ti.valid && last_key >= 0) ? (int)(last_key / kBlockN) + 1 : 0;   // 0: the tile sees no key at all
+    if (kMask && (long long)a.pos_off + (ti.row0 >> pack_log2) >= a.kv_len) ti.n_kv = 0;   // all its rows sit in padding
     return ti;
 }
 
@@ -758,8 +766,25 @@ __device__ __noinline__ void issue_products(unsigned sm_addr, unsigned tmem, int
     while (!mbar_try_wait_at(sm_addr + (unsigned)offsetof(Storage, drain), 0u) && global_timer_ns() - t_begin < 100000000ULL) {}
 }
 
+// One past the last key below `end` that the sequence's key-padding mask lets anybody see; 0: none. Run by one whole warp, 512 keys at a time from the end.
+__device__ __noinline__ int seen_below(const unsigned char* mask_row, int end, int lane) {
+#pragma unroll 1
+    for (; end > 0; end -= 512) {
+        int last = 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int key = end - 1 - lane - 32 * i;
+            const bool there = key >= 0 && mask_row[max(key, 0)] != 0;
+            last = max(last, there ? key + 1 : 0);
+        }
+        last = __reduce_max_sync(0xffffffffu, last);
+        if (last > 0) return last;
+    }
+    return 0;
+}
+
 // The tile pair that CTA (bx, by, bz) of the grid stands for; false: there is none, or nothing to do for it. Run by one whole warp.
-template <bool kPaged>
+template <bool kMask, bool kPaged>
 __device__ __forceinline__ bool find_pair(const PrefillArgs& a, int bx, int by, int bz, int lane, Item& w) {
     int pair;
     if (kPaged && a.ordered) {
@@ -784,8 +809,14 @@ __device__ __forceinline__ bool find_pair(const PrefillArgs& a, int bx, int by, 
     w.sq = seq_extent(a, w.seq);
     if ((w.sq.q_len << a.pack_log2) * a.by_packs.d <= a.skip_rows) return false;   // the few-row kernel's
     const int num_mb = row_blocks(w.sq.q_len, a.pack_log2);
-    w.t[0] = tile_info(w.sq, pair, 0, w.kv_head, a.by_packs, a.pack_log2, num_mb);
-    w.t[1] = tile_info(w.sq, pair, 1, w.kv_head, a.by_packs, a.pack_log2, num_mb);
+    if (kMask) {
+        // Padding behind a pair's last key that counts is not walked: the pair's keys end there, and a tile all of whose rows sit in padding (their output is zeros) sees none.
+        const int last = tile_token_end(w.sq, pair * 2 + 1, a.by_packs, a.pack_log2, num_mb);   // one past the pair's last query token
+        const long long end = min((long long)w.sq.kv_len, (long long)w.sq.pos_off + last);
+        if (end > 0) w.sq.kv_len = seen_below(a.mask + (long long)w.seq * a.kv_seq_len, (int)end, lane);
+    }
+    w.t[0] = tile_info<kMask>(w.sq, pair, 0, w.kv_head, a.by_packs, a.pack_log2, num_mb);
+    w.t[1] = tile_info<kMask>(w.sq, pair, 1, w.kv_head, a.by_packs, a.pack_log2, num_mb);
     return w.t[0].valid || w.t[1].valid;   // (a sequence may be shorter than the grid's row range)
 }
 
@@ -832,7 +863,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         bool begun = false;   // the first tile pair's first copies have been requested
         // The CTA's own tile pair, and its first copies at once, in as few instructions as that takes: all of them come in for the first time here, and
         // in the loop below, with its waits and cases, the first S came 1600 to 2300 clocks later (a fifth of a call of one short wave).
-        w.some = find_pair<kPaged>(a, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, lane, w);
+        w.some = find_pair<kMask, kPaged>(a, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, lane, w);
         asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
         begun = w.some && max(w.t[0].n_kv, w.t[1].n_kv) > 0 && !q_open && !kv_open && a.test_skip_k != 1;
         if (begun && (kPaged || lane == 0)) {
@@ -906,7 +937,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     const bool got = read_answer(sm.answer, bx, by, bz);
                     __syncwarp();
                     if (!got) break;   // every tile pair is taken
-                    w.some = find_pair<kPaged>(a, bx, by, bz, lane, w);
+                    w.some = find_pair<kMask, kPaged>(a, bx, by, bz, lane, w);
                     if (w.some) break;
                     ask();
                 }
