@@ -263,17 +263,21 @@ __device__ __forceinline__ void store_pair(const RowsOut& out, long long row, in
 
 // Merges the parts of a cut sequence: warp w takes rows w, w + 4, ..., RW of them, a lane D / 32 neighbouring
 // elements of each. The CTA runs alone at the end of its column here, so what counts is the number of dependent
-// trips to L2 (about 0.8 us each): one for every part's (m, l), then 16 rows of partials in flight per lane.
-// 22 parts of 8 rows: 10 us with one row and 8 partials at a time, 3 us so.
-template <int D, int RW, typename Finish>
-__device__ __forceinline__ void merge_parts(const float* acc0, const float2* ml0, float* scratch, int nrows, int c_first, int parts,
-                                            unsigned grid_x, int warp, int lane, const Finish& finish) {
+// trips to L2 (about 0.6 us each) and of instructions, which come in for the first time: the first partials are asked for together with every part's (m, l), in all 16 rows of
+// partials in flight per lane, and where a row goes is found by one lane and told to the others. With the partials asked for behind the weights, and
+// every lane finding each row's place, a merge of 13 parts of 4 rows took 2.1 us, of 2-5 parts of 16 rows 6 to 8 us, of which 0.65 and 3 to 5 behind the sums (device timer); 16 sequences
+// x 4 tokens over 512-8192 64.4 us a step, 8 x 4000 contiguous 28.7, one of 777 tokens 9.1.
+template <typename T, int D, int RW, bool kHalves>
+__device__ __forceinline__ void merge_parts(const RowsArgs& a, float* scratch, long long q_row0, int s, int kvh, int row0, int group, int nrows, int c_first, int parts, int warp, int lane) {
     constexpr int E = D / 32;
     constexpr int kAtOnce = 16 / RW;      // parts in flight per row
     constexpr int kChunk = 64;            // parts whose weights sit in shared memory at a time
     static_assert(kRows / 2 * (D + 2) <= kRows * Smem<D>::kMergePitch, "half of the rows fit the merge buffer whole");
     static_assert(kRows * kChunk * 4 <= Smem<D>::kMergeBytes, "weights of a chunk fit the merge buffer");
-    auto slot_of = [&](int c) { return (long long)c * grid_x * 2 + (c == c_first ? 1 : 0); };
+    const unsigned grid_x = gridDim.x;
+    const float* const acc0 = a.ws_acc + ((long long)blockIdx.x * (2 * kRows) + warp) * D + lane * E;   // of this warp's first row, slot 0 of column 0
+    const float2* const ml0 = a.ws_ml + (long long)blockIdx.x * (2 * kRows) + warp;
+    auto slot_of = [&](int c) { return (unsigned)c * grid_x * 2u + (c == c_first ? 1u : 0u); };   // (fits: the workspace has 2 kRows D floats for each)
     float o[RW][E], m[RW], l[RW];
 #pragma unroll
     for (int k = 0; k < RW; ++k) {
@@ -282,43 +286,20 @@ __device__ __forceinline__ void merge_parts(const float* acc0, const float2* ml0
 #pragma unroll
         for (int e = 0; e < E; ++e) o[k][e] = 0.0f;
     }
+#pragma unroll 1
     for (int p0 = 0; p0 < parts; p0 += kChunk) {
         const int n = min(kChunk, parts - p0);
+        float x[RW][kAtOnce][E];
+        auto ask = [&](int i0) {
 #pragma unroll
-        for (int k = 0; k < RW; ++k) {
-            const int r = warp + k * kWarps;
-            float2 x[2] = {make_float2(-INFINITY, 0.0f), make_float2(-INFINITY, 0.0f)};
-            if (r < nrows) {
-                if (lane < n) x[0] = __ldcg(&ml0[slot_of(c_first + p0 + lane) * kRows + r]);
-                if (lane + 32 < n) x[1] = __ldcg(&ml0[slot_of(c_first + p0 + 32 + lane) * kRows + r]);
-            }
-            float mx = fmaxf(x[0].x, x[1].x);
+            for (int i = 0; i < kAtOnce; ++i) {
+                const float* const part = acc0 + (unsigned long long)slot_of(c_first + p0 + i0 + i) * (kRows * D);
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-            mx = fmaxf(mx, m[k]);
-            const float before = m[k] == -INFINITY ? 0.0f : fast_exp2(m[k] - mx);
-            m[k] = mx;
-            l[k] *= before;
-#pragma unroll
-            for (int e = 0; e < E; ++e) o[k][e] *= before;
-            const float w0 = x[0].x == -INFINITY ? 0.0f : fast_exp2(x[0].x - mx);
-            const float w1 = x[1].x == -INFINITY ? 0.0f : fast_exp2(x[1].x - mx);
-            scratch[(k * kWarps + warp) * kChunk + lane] = w0;
-            scratch[(k * kWarps + warp) * kChunk + 32 + lane] = w1;
-            l[k] += w0 * x[0].y + w1 * x[1].y;   // this lane's share
-        }
-        __syncwarp();
-        for (int i0 = 0; i0 < n; i0 += kAtOnce) {
-            float x[RW][kAtOnce][E];
-#pragma unroll
-            for (int k = 0; k < RW; ++k) {
-                const int r = warp + k * kWarps;
-#pragma unroll
-                for (int i = 0; i < kAtOnce; ++i) {
+                for (int k = 0; k < RW; ++k) {
 #pragma unroll
                     for (int e = 0; e < E; ++e) x[k][i][e] = 0.0f;
-                    if (r < nrows && i0 + i < n) {
-                        const float* src = acc0 + (slot_of(c_first + p0 + i0 + i) * kRows + r) * D + lane * E;
+                    if (warp + k * kWarps < nrows && i0 + i < n) {
+                        const float* const src = part + k * kWarps * D;
                         if constexpr (E == 4) {
                             const float4 y = __ldcg(reinterpret_cast<const float4*>(src));
                             x[k][i][0] = y.x; x[k][i][1] = y.y; x[k][i][2] = y.z; x[k][i][3] = y.w;
@@ -331,22 +312,101 @@ __device__ __forceinline__ void merge_parts(const float* acc0, const float2* ml0
                     }
                 }
             }
+        };
+        float2 y[RW][2];
 #pragma unroll
-            for (int k = 0; k < RW; ++k)
+        for (int h = 0; h < 2; ++h) {
+            const float2* const part = ml0 + (unsigned long long)slot_of(c_first + p0 + h * 32 + lane) * kRows;
 #pragma unroll
-                for (int i = 0; i < kAtOnce; ++i) {
+            for (int k = 0; k < RW; ++k) {
+                y[k][h] = make_float2(-INFINITY, 0.0f);
+                if (warp + k * kWarps < nrows && h * 32 + lane < n) y[k][h] = __ldcg(part + k * kWarps);
+            }
+        }
+        ask(0);
+#pragma unroll
+        for (int k = 0; k < RW; ++k) {
+            float mx = fmaxf(y[k][0].x, y[k][1].x);
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+            mx = fmaxf(mx, m[k]);
+            const float before = m[k] == -INFINITY ? 0.0f : fast_exp2(m[k] - mx);
+            m[k] = mx;
+            l[k] *= before;
+#pragma unroll
+            for (int e = 0; e < E; ++e) o[k][e] *= before;
+            const float w0 = y[k][0].x == -INFINITY ? 0.0f : fast_exp2(y[k][0].x - mx);
+            const float w1 = y[k][1].x == -INFINITY ? 0.0f : fast_exp2(y[k][1].x - mx);
+            scratch[(k * kWarps + warp) * kChunk + lane] = w0;
+            scratch[(k * kWarps + warp) * kChunk + 32 + lane] = w1;
+            l[k] += w0 * y[k][0].y + w1 * y[k][1].y;   // this lane's share
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int i0 = 0;;) {
+#pragma unroll
+            for (int i = 0; i < kAtOnce; ++i)
+#pragma unroll
+                for (int k = 0; k < RW; ++k) {
                     const float w = scratch[(k * kWarps + warp) * kChunk + min(i0 + i, n - 1)];
 #pragma unroll
                     for (int e = 0; e < E; ++e) o[k][e] = fmaf(w, x[k][i][e], o[k][e]);
                 }
+            i0 += kAtOnce;
+            if (i0 >= n) break;
+            ask(i0);
         }
         __syncwarp();
     }
 #pragma unroll
-    for (int k = 0; k < RW; ++k) {
+    for (int off = 16; off > 0; off >>= 1)
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) l[k] += __shfl_xor_sync(0xffffffffu, l[k], off);
-        if (warp + k * kWarps < nrows) finish(warp + k * kWarps, o[k], m[k], l[k]);
+        for (int k = 0; k < RW; ++k) l[k] += __shfl_xor_sync(0xffffffffu, l[k], off);
+    // lane k, k + RW, ... : row k's place, maximum and sum
+    const int mine = lane & (RW - 1), r = warp + mine * kWarps, t = (row0 + r) / group, h = kvh * group + (row0 + r) - t * group;
+    const long long at = ((q_row0 + t) * a.out.o_heads + a.out.o_head0 + h) * D;
+    float m1 = m[0], l1 = l[0];
+#pragma unroll
+    for (int k = 1; k < RW; ++k)
+        if (mine == k) {
+            m1 = m[k];
+            l1 = l[k];
+        }
+    const float inv1 = l1 > 0.0f ? 1.0f / l1 : 0.0f;
+    if (a.out.lse != nullptr && lane < RW && r < nrows)
+        a.out.lse[((long long)s * a.q_heads + h) * a.q_seq_len + t] = l1 > 0.0f ? (m1 + log2f(l1)) * 0.6931471805599453f : -INFINITY;
+    unsigned both[RW][(E + 1) / 2];
+    long long to[RW];
+#pragma unroll
+    for (int k = 0; k < RW; ++k) {
+        const float inv = __shfl_sync(0xffffffffu, inv1, k);
+        to[k] = __shfl_sync(0xffffffffu, at, k) + lane * E;
+        if constexpr (E >= 2) {
+#pragma unroll
+            for (int e = 0; e < E; e += 2) both[k][e / 2] = pack2<T>(o[k][e] * inv, o[k][e + 1] * inv);
+        } else {
+            const float up = __shfl_down_sync(0xffffffffu, o[k][0], 1);
+            both[k][0] = pack2<T>(o[k][0] * inv, up * inv);   // (even lanes')
+        }
+    }
+    int pe = a.out.peer0;
+#pragma unroll 1
+    for (int n = 0; n < a.out.n_out; ++n) {
+        T* const base = static_cast<T*>(a.out.o[pe]);
+#pragma unroll
+        for (int k = 0; k < RW; ++k) {
+            if (warp + k * kWarps >= nrows || (E == 1 && (lane & 1) != 0)) continue;
+#pragma unroll
+            for (int e = 0; e < (E + 1) / 2; ++e) {
+                if (kHalves) {
+                    reinterpret_cast<unsigned short*>(base + to[k])[2 * e] = (unsigned short)both[k][e];
+                    reinterpret_cast<unsigned short*>(base + to[k])[2 * e + 1] = (unsigned short)(both[k][e] >> 16);
+                } else {
+                    reinterpret_cast<unsigned*>(base + to[k])[e] = both[k][e];
+                }
+            }
+        }
+        pe = pe + 1 == a.out.n_out ? 0 : pe + 1;
     }
 }
 
@@ -771,26 +831,10 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
             }
             __syncthreads();
             if (*last_flag) {
-                const float* acc0 = a.ws_acc + (long long)blockIdx.x * (2 * kRows * D);
-                const float2* ml0 = a.ws_ml + (long long)blockIdx.x * (2 * kRows);
-                auto finish = [&](int r, const float (&o)[D / 32], float m, float l) {
-                    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-                    const int t = (row0 + r) / group, h = kvh * group + (row0 + r) - t * group;
-                    if constexpr (D >= 64) {
-#pragma unroll
-                        for (int e = 0; e < D / 32; e += 2)
-                            store_pair<T, kHalves>(a.out, seq.q_row0 + t, h, D, lane * (D / 32) + e, pack2<T>(o[e] * inv, o[e + 1] * inv));
-                    } else {
-                        const float up = __shfl_down_sync(0xffffffffu, o[0], 1);
-                        if ((lane & 1) == 0) store_pair<T, kHalves>(a.out, seq.q_row0 + t, h, D, lane, pack2<T>(o[0] * inv, up * inv));
-                    }
-                    if (lane == 0 && a.out.lse != nullptr)
-                        a.out.lse[((long long)s * a.q_heads + h) * a.q_seq_len + t] = l > 0.0f ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
-                };
                 const int rows_per_warp = (nrows + kWarps - 1) / kWarps;
-                if (rows_per_warp == 1) merge_parts<D, 1>(acc0, ml0, merge, nrows, c_first, parts, gridDim.x, warp, lane, finish);
-                else if (rows_per_warp == 2) merge_parts<D, 2>(acc0, ml0, merge, nrows, c_first, parts, gridDim.x, warp, lane, finish);
-                else merge_parts<D, 4>(acc0, ml0, merge, nrows, c_first, parts, gridDim.x, warp, lane, finish);
+                if (rows_per_warp == 1) merge_parts<T, D, 1, kHalves>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
+                else if (rows_per_warp == 2) merge_parts<T, D, 2, kHalves>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
+                else merge_parts<T, D, 4, kHalves>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
                 __syncthreads();   // the merge buffer is written again by the next sequence
             }
         }
