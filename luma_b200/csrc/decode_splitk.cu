@@ -47,6 +47,7 @@ constexpr int kRows = 16;    // query rows served per CTA (M of the mma)
 struct RowsOut {
     void* o[8];
     int n_out, o_heads, o_head0, peer0;
+    int halves;      // a buffer is aligned to its 2-byte elements only: rows are stored element by element
     float* lse;      // MODE_BATCH: (num_seqs, q_heads, q_seq_len) or null
 };
 
@@ -72,6 +73,7 @@ struct RowsArgs {
     int max_rows;        // sequences with more query rows than this (per KV head) are not this launch's
     int behind_prefill;  // launched behind the prefill kernel of the same call, which it does not depend on
     int forced_units;    // > 0: units per column (option "decode_chunk_tokens"); 0: equal shares
+    int seq_cost;        // of a sequence, in units, beside its own units (see rows_span)
     float scale_log2;    // scale * log2(e)
     RowsOut out;
 };
@@ -172,16 +174,17 @@ struct RowsSeq {
     long long q_row0, kv_row0;
 };
 
+template <int kMode>
 __device__ __forceinline__ RowsSeq rows_seq(const RowsArgs& a, int s) {
     RowsSeq r;
-    if (a.mode == MODE_KVCACHE) {
+    if (kMode == MODE_KVCACHE) {
         r.q_len = a.q_seq_len;
         const int len = a.context_lens[s];
         r.kv_len = min(len, a.capacity);
         r.pos_off = len - r.q_len;
         r.q_row0 = (long long)s * a.q_seq_len;
         r.kv_row0 = 0;
-    } else if (a.mode == MODE_BATCH) {
+    } else if (kMode == MODE_BATCH) {
         r.q_len = a.q_seq_len;
         r.kv_len = a.kv_seq_len;
         r.pos_off = a.start_pos;
@@ -212,6 +215,13 @@ __device__ __forceinline__ int rows_units(const RowsArgs& a, const RowsSeq& r, i
     if (rows <= row0 || rows > a.max_rows) return 0;
     return max(1, (rows_visible(r) + kUnit - 1) / kUnit);
 }
+
+// What a sequence weighs in the cut: its units, and behind them `cost` units for what it costs a CTA to begin and to end one (its query rows, the merge of the warps' parts, the
+// count). Cut by the units alone, the CTAs with the end of a sequence in their share came to their own end 2 to 4 us behind the others (us, before and so: 8 x 4000 contiguous,
+// where eight of 37 columns hold one, 27.9 and 26.7; 8 x 512-2048 15.2 and 13.7; 16 x 7 tokens over 1217-4869, 8/2 heads 26.9 and 24.6; 16 x 91-367, 8 heads of 64 11.9 and 9.6).
+__device__ __forceinline__ unsigned rows_span(int units, int cost) { return units > 0 ? (unsigned)(units + cost) : 0u; }
+// Where the columns get little more than a unit each there is nothing to even out, and a cost would leave columns empty.
+__device__ __forceinline__ int rows_cost(const RowsArgs& a, unsigned total_units, int columns) { return total_units <= (unsigned)columns + (unsigned)columns / 8u ? 0 : a.seq_cost; }
 
 // The cut of `total` units into columns: the first `more` columns have share + 1 units, the others share
 // (or, forced, every column at least `forced` units). All in 32 bits: a 64-bit division here cost a microsecond of a small call.
@@ -245,13 +255,13 @@ __device__ __forceinline__ unsigned long long arrive_acq_rel(unsigned long long*
 }
 
 // Two finished neighbours of an output row, to every output buffer.
-template <typename T, bool kHalves>
+template <typename T>
 __device__ __forceinline__ void store_pair(const RowsOut& out, long long row, int head, int D, int d, unsigned both) {
     const long long off = (row * out.o_heads + out.o_head0 + head) * D + d;
     int pe = out.peer0;
     for (int n = 0; n < out.n_out; ++n) {
         T* const at = static_cast<T*>(out.o[pe]) + off;
-        if (kHalves) {
+        if (out.halves) {
             reinterpret_cast<unsigned short*>(at)[0] = (unsigned short)both;
             reinterpret_cast<unsigned short*>(at)[1] = (unsigned short)(both >> 16);
         } else {
@@ -267,7 +277,7 @@ __device__ __forceinline__ void store_pair(const RowsOut& out, long long row, in
 // partials in flight per lane, and where a row goes is found by one lane and told to the others. With the partials asked for behind the weights, and
 // every lane finding each row's place, a merge of 13 parts of 4 rows took 2.1 us, of 2-5 parts of 16 rows 6 to 8 us, of which 0.65 and 3 to 5 behind the sums (device timer); 16 sequences
 // x 4 tokens over 512-8192 64.4 us a step, 8 x 4000 contiguous 28.7, one of 777 tokens 9.1.
-template <typename T, int D, int RW, bool kHalves>
+template <typename T, int D, int RW>
 __device__ __forceinline__ void merge_parts(const RowsArgs& a, float* scratch, long long q_row0, int s, int kvh, int row0, int group, int nrows, int c_first, int parts, int warp, int lane) {
     constexpr int E = D / 32;
     constexpr int kAtOnce = 16 / RW;      // parts in flight per row
@@ -398,7 +408,7 @@ __device__ __forceinline__ void merge_parts(const RowsArgs& a, float* scratch, l
             if (warp + k * kWarps >= nrows || (E == 1 && (lane & 1) != 0)) continue;
 #pragma unroll
             for (int e = 0; e < (E + 1) / 2; ++e) {
-                if (kHalves) {
+                if (a.out.halves) {
                     reinterpret_cast<unsigned short*>(base + to[k])[2 * e] = (unsigned short)both[k][e];
                     reinterpret_cast<unsigned short*>(base + to[k])[2 * e + 1] = (unsigned short)(both[k][e] >> 16);
                 } else {
@@ -410,9 +420,9 @@ __device__ __forceinline__ void merge_parts(const RowsArgs& a, float* scratch, l
     }
 }
 
-// kHalves: an output buffer is aligned to its 2-byte elements only, rows are stored element by element (a separate instantiation: the
-// branch at each store, and a minimum with the table's capacity at each mask, cost 1 us of the 18 of one sequence with 16 rows to merge).
-template <typename T, int D, bool kHalves>
+// kMode: the entry point. With the three of them behind branches, every place that looks at a sequence had
+// the code of all three, which a small call brings in for the first time (1 x 777 tokens 8.7 us a step, 8.3 so; 2 x 62-250, 32 heads 10.1 and 9.1).
+template <typename T, int D, int kMode>
 __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_kernel(const __grid_constant__ RowsArgs a) {
     using S = Smem<D>;
     constexpr int kChunksPerRow = D / 8;          // 16-byte chunks per K/V row
@@ -446,10 +456,12 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
 
     // The cut: total units, this column's share of them, and the sequence its first unit lies in.
     unsigned total = 0, seq_first = 0;   // seq_first: unit at which sequence `s` begins
-    int s = 0;
+    int s = 0, cost = 0;
     unsigned u_begin, u_end;
-    if (a.mode == MODE_BATCH) {
-        const unsigned per = (unsigned)rows_units(a, rows_seq(a, 0), group, row0);
+    if (kMode == MODE_BATCH) {
+        const int units = rows_units(a, rows_seq<kMode>(a, 0), group, row0);
+        cost = rows_cost(a, (unsigned)units * (unsigned)a.num_seqs, columns);
+        const unsigned per = rows_span(units, cost);
         total = per * (unsigned)a.num_seqs;
         columns = (int)min((unsigned)columns, max(total, 1u));   // never an empty column between two others
         const Cut cut(total, (unsigned)columns, (unsigned)a.forced_units);
@@ -462,27 +474,39 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
         s = (int)(u_begin / per);
         seq_first = per * (unsigned)s;
     } else {
-        // four neighbouring sequences per lane, 128 at a time; the last 128's counts stay in registers
-        int mine[4], lane_sum = 0, upto = 0;
-        int s0 = 0;
-        for (;; s0 += 128) {
-            lane_sum = 0;
+        // four neighbouring sequences per lane, 128 at a time; the last 128's counts stay in registers: units, and sequences that have any
+        int mine[4], lane_sum = 0, upto = 0, lane_seqs = 0, upto_seqs = 0;
+        auto count = [&](int s0) {
+            lane_sum = lane_seqs = 0;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int si = s0 + lane * 4 + i;
-                mine[i] = si < a.num_seqs ? rows_units(a, rows_seq(a, si), group, row0) : 0;
+                mine[i] = si < a.num_seqs ? rows_units(a, rows_seq<kMode>(a, si), group, row0) : 0;
+                lane_sum += mine[i];
+                lane_seqs += mine[i] > 0 ? 1 : 0;
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) lane_sum += mine[i];
             upto = lane_sum;
+            upto_seqs = lane_seqs;
 #pragma unroll
             for (int off = 1; off < 32; off <<= 1) {
-                const int o = __shfl_up_sync(0xffffffffu, upto, off);
-                if (lane >= off) upto += o;
+                const int o = __shfl_up_sync(0xffffffffu, upto, off), q = __shfl_up_sync(0xffffffffu, upto_seqs, off);
+                if (lane >= off) {
+                    upto += o;
+                    upto_seqs += q;
+                }
             }
+        };
+        int s0 = 0;
+        unsigned seqs = 0;
+#pragma unroll 1
+        for (;; s0 += 128) {
+            count(s0);
             total += (unsigned)__shfl_sync(0xffffffffu, upto, 31);
+            seqs += (unsigned)__shfl_sync(0xffffffffu, upto_seqs, 31);
             if (s0 + 128 >= a.num_seqs) break;
         }
+        cost = rows_cost(a, total, columns);
+        total += seqs * (unsigned)cost;
         columns = (int)min((unsigned)columns, max(total, 1u));   // never an empty column between two others
         const Cut cut(total, (unsigned)columns, (unsigned)a.forced_units);
         u_begin = cut.first(column);
@@ -493,35 +517,25 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
         }
         if (s0 > 0) s0 = 0;          // more than 128 sequences: walk them again from the start
         else s0 = -1;
+#pragma unroll 1
         for (;;) {
-            if (s0 >= 0) {
-                lane_sum = 0;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int si = s0 + lane * 4 + i;
-                    mine[i] = si < a.num_seqs ? rows_units(a, rows_seq(a, si), group, row0) : 0;
-                    lane_sum += mine[i];
-                }
-                upto = lane_sum;
-#pragma unroll
-                for (int off = 1; off < 32; off <<= 1) {
-                    const int o = __shfl_up_sync(0xffffffffu, upto, off);
-                    if (lane >= off) upto += o;
-                }
-            }
-            const unsigned past = __ballot_sync(0xffffffffu, seq_first + (unsigned)upto > u_begin);
+            if (s0 >= 0) count(s0);
+            const unsigned past = __ballot_sync(0xffffffffu, seq_first + (unsigned)(upto + upto_seqs * cost) > u_begin);
             if (past != 0u) {   // always before the sequences run out: u_begin < total
                 const int at = __ffs(past) - 1;
-                unsigned f = seq_first + (unsigned)(upto - lane_sum);
+                unsigned f = seq_first + (unsigned)(upto - lane_sum + (upto_seqs - lane_seqs) * cost);
                 int si = max(s0, 0) + lane * 4;
 #pragma unroll
                 for (int i = 0; i < 3; ++i)
-                    if (f + (unsigned)mine[i] <= u_begin && si == max(s0, 0) + lane * 4 + i) { f += (unsigned)mine[i]; ++si; }
+                    if (f + rows_span(mine[i], cost) <= u_begin && si == max(s0, 0) + lane * 4 + i) {
+                        f += rows_span(mine[i], cost);
+                        ++si;
+                    }
                 s = __shfl_sync(0xffffffffu, si, at);
                 seq_first = __shfl_sync(0xffffffffu, f, at);
                 break;
             }
-            seq_first += (unsigned)__shfl_sync(0xffffffffu, upto, 31);
+            seq_first += (unsigned)(__shfl_sync(0xffffffffu, upto, 31) + __shfl_sync(0xffffffffu, upto_seqs, 31) * cost);
             s0 += 128;
         }
     }
@@ -543,17 +557,32 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
     static_assert(kCopiesPerLane == kInstrPerTile, "a lane issues one 16-byte copy per instruction");
     const int cp_ch = lane % kChunksPerRow;
     const int cp_sub = lane / kChunksPerRow;
-    int cp_left = (int)(u_end - u_begin);
     int cp_s = s;
-    RowsSeq cp_seq = rows_seq(a, s);
+    unsigned cp_first = seq_first;                     // unit at which sequence cp_s begins
+    RowsSeq cp_seq = rows_seq<kMode>(a, s);
+    int cp_units = rows_units(a, cp_seq, group, row0);
     int cp_vis = rows_visible(cp_seq);
-    int cp_tok = (int)(u_begin - seq_first) * kUnit;   // first token of the unit to copy next
-    int cp_end = rows_units(a, cp_seq, group, row0) * kUnit;
+    int cp_tok = (int)(u_begin - seq_first) * kUnit;   // first token of the unit to look up next
+    int cp_end = (int)min((unsigned)cp_units, u_end - cp_first) * kUnit;   // tokens of it that are this CTA's
+    int cp_looked = 0, cp_issued = 0;                  // units looked up and asked for
+    // on to the next sequence that has units here
+    auto cp_next_seq = [&]() {
+        while (cp_tok >= cp_end) {
+            cp_first += rows_span(cp_units, cost);
+            if (cp_first >= u_end) return;
+            cp_seq = rows_seq<kMode>(a, ++cp_s);
+            cp_units = rows_units(a, cp_seq, group, row0);
+            cp_vis = rows_visible(cp_seq);
+            cp_tok = 0;
+            cp_end = (int)min((unsigned)cp_units, u_end - cp_first) * kUnit;
+        }
+    };
+    cp_next_seq();
     auto look_up = [&]() -> long long {   // element offset of this lane's token row in the caches, -1 past the visible keys
         const int j = cp_tok + warp * kTile + (lane & 15);
         if (j >= cp_vis) return -1;
         long long slot;
-        if (a.paged) {
+        if (kMode == MODE_KVCACHE || (kMode == MODE_VARLEN && a.paged)) {
             const int page = a.block_shift >= 0 ? j >> a.block_shift : j / a.block_size;
             slot = a.block_tables[cp_s * a.max_blocks + page] * a.block_size + (j - page * a.block_size);
         } else {
@@ -561,28 +590,19 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
         }
         return slot * kv_pitch + (long long)kvh * D;
     };
-    int cp_ahead = (int)(u_end - u_begin);   // units whose slots have not been looked up yet
     auto look_up_next = [&]() -> long long {
-        if (cp_ahead <= 0) return -1;
+        if (cp_tok >= cp_end) return -1;
         const long long off = look_up();
-        if (--cp_ahead > 0) {
-            cp_tok += kUnit;
-            if (cp_tok >= cp_end) {   // on to the next sequence that has rows here
-                do {
-                    cp_seq = rows_seq(a, ++cp_s);
-                    cp_end = rows_units(a, cp_seq, group, row0) * kUnit;
-                } while (cp_end == 0);
-                cp_vis = rows_visible(cp_seq);
-                cp_tok = 0;
-            }
-        }
+        ++cp_looked;
+        cp_tok += kUnit;
+        if (cp_tok >= cp_end) cp_next_seq();
         return off;
     };
     long long cp_off = look_up_next();
     long long cp_off2 = look_up_next();
     int cp_stage = 0;
     auto issue = [&]() {
-        if (cp_left > 0) {
+        if (cp_issued < cp_looked) {
             unsigned char* kst = ring + cp_stage * S::kStageBytes;
             unsigned char* vst = kst + S::kTileBytes;
 #pragma unroll
@@ -596,7 +616,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
                 cp_async_16(vst + dst, vg + src, valid);
             }
             cp_stage = cp_stage + 1 == kStages ? 0 : cp_stage + 1;
-            --cp_left;
+            ++cp_issued;
             cp_off = cp_off2;
             cp_off2 = look_up_next();
         }
@@ -613,11 +633,13 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
     int stage = 0;
     unsigned u = u_begin;
     while (u < u_end) {
-        RowsSeq seq = rows_seq(a, s);
-        int units = rows_units(a, seq, group, row0);
-        while (units == 0) {   // not this launch's
-            seq = rows_seq(a, ++s);
-            units = rows_units(a, seq, group, row0);
+        const RowsSeq seq = rows_seq<kMode>(a, s);
+        const int units = rows_units(a, seq, group, row0);
+        if (u >= seq_first + (unsigned)units) {   // not this launch's, or ended
+            seq_first += rows_span(units, cost);
+            u = max(u, seq_first);
+            ++s;
+            continue;
         }
         const int vis = rows_visible(seq);
         const int nrows = min(kRows, seq.q_len * group - row0);   // query rows served here
@@ -803,7 +825,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
                         const float inv = l > 0.0f ? 1.0f / l : 0.0f;   // reference: flash_attn_with_kvcache.cu:109
                         const int t = (row0 + r) / group, h = kvh * group + (row0 + r) - t * group;
                         const unsigned w2 = pack2<T>(ox * inv, oy * inv);
-                        store_pair<T, kHalves>(a.out, seq.q_row0 + t, h, D, dd, w2);
+                        store_pair<T>(a.out, seq.q_row0 + t, h, D, dd, w2);
                         if (dd == 0 && a.out.lse != nullptr)
                             a.out.lse[((long long)s * a.q_heads + h) * a.q_seq_len + t] = l > 0.0f ? (mstar + log2f(l)) * 0.6931471805599453f : -INFINITY;
                     } else {
@@ -832,15 +854,11 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
             __syncthreads();
             if (*last_flag) {
                 const int rows_per_warp = (nrows + kWarps - 1) / kWarps;
-                if (rows_per_warp == 1) merge_parts<T, D, 1, kHalves>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
-                else if (rows_per_warp == 2) merge_parts<T, D, 2, kHalves>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
-                else merge_parts<T, D, 4, kHalves>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
+                if (rows_per_warp == 1) merge_parts<T, D, 1>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
+                else if (rows_per_warp == 2) merge_parts<T, D, 2>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
+                else merge_parts<T, D, 4>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
                 __syncthreads();   // the merge buffer is written again by the next sequence
             }
-        }
-        if (ends) {
-            seq_first += (unsigned)units;
-            ++s;
         }
     }
     cp_async_wait<0>();
@@ -881,17 +899,21 @@ RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, b
 
 std::atomic<unsigned long long> g_calls{0};   // launches of this kernel, of any type and on any device
 
-template <typename T, int D, bool kHalves>
+template <typename T, int D, int kMode>
 int launch_rows_as(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
     using S = Smem<D>;
     static_assert(kMaxColumns < (1 << kCountBits), "the parts of a sequence fit the count");
     a.row_blocks = plan.row_blocks;
     a.forced_units = plan.forced_units;
+    // (us for costs of 0, 2, 3, 4, 6: 64 x 512-8192 180.4, 180.3, 180.7-182, 181.2, 186; 8 x 4000 contiguous 27.9, 27.3, 26.7, 26.2, 25.9; 4 x 2369 15.9, 13.2, 13.8, 13.9, 13.9; with 16
+    // rows 43 x 4 tokens over 200-3000 67.0, 63.6, 62.6, 61.1, 59.5; 64 x 2 over 100-1600, 64/8 heads 59.3, 56.7, 54.4, 53.3, 51.6; 16 x 4 over 512-8192 58.6, 58.2, 58.9, 57.5, 58.4)
+    const int rows = a.max_rows < kRows ? a.max_rows : kRows;
+    a.seq_cost = plan.forced_units > 0 ? 0 : rows > 8 ? 5 : 3;
     static std::atomic<unsigned long long> ready{0};   // devices whose copy of this kernel has its shared-memory limit raised
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err == cudaSuccess && (dev >= 64 || !((ready.load(std::memory_order_acquire) >> dev) & 1ULL))) {
-        err = cudaFuncSetAttribute(decode_splitk_kernel<T, D, kHalves>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
+        err = cudaFuncSetAttribute(decode_splitk_kernel<T, D, kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
         if (err == cudaSuccess && dev < 64) ready.fetch_or(1ULL << dev, std::memory_order_release);
     }
     if (err != cudaSuccess) {
@@ -909,16 +931,17 @@ int launch_rows_as(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, decode_splitk_kernel<T, D, kHalves>, a);
+    cudaLaunchKernelEx(&cfg, decode_splitk_kernel<T, D, kMode>, a);
     return check_launch("decode_splitk_kernel");
 }
 
 template <typename T, int D>
 int launch_rows(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
     a.call = (g_calls.fetch_add(1, std::memory_order_relaxed) + 1) << kCountBits;
-    bool halves = false;
-    for (int i = 0; i < a.out.n_out; ++i) halves |= (reinterpret_cast<uintptr_t>(a.out.o[i]) & 3) != 0;
-    return halves ? launch_rows_as<T, D, true>(a, plan, stream) : launch_rows_as<T, D, false>(a, plan, stream);
+    for (int i = 0; i < a.out.n_out; ++i) a.out.halves |= (reinterpret_cast<uintptr_t>(a.out.o[i]) & 3) != 0;
+    return a.mode == MODE_KVCACHE ? launch_rows_as<T, D, MODE_KVCACHE>(a, plan, stream)
+           : a.mode == MODE_BATCH ? launch_rows_as<T, D, MODE_BATCH>(a, plan, stream)
+                                  : launch_rows_as<T, D, MODE_VARLEN>(a, plan, stream);
 }
 
 int log2_or_minus1(int v) {
