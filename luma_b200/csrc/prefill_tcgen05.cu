@@ -94,6 +94,7 @@ struct TileInfo {
 struct Item {
     int some;            // 0: nothing is left, the CTA ends
     int seq, kv_head;
+    int first_key;       // where the CTA's share of the keys begins (a multiple of a tile); kv_len, pos_off and kv_crow of `sq` count from there
     SeqExtent sq;
     TileInfo t[2];
 };
@@ -162,6 +163,7 @@ struct PrefillArgs {
     int d_real;     // head size of the tensors: D, or 32 when the D = 64 kernel runs a head size of 32 on zero-padded tiles
     int pack_log2;          // of the query heads that share a tile (pack_of): row r is query token r >> pack_log2, head r % pack of them
     FastDiv by_packs, by_kv_heads, by_band;   // groups of `pack` query heads per KV head; KV heads; band
+    int parts;      // CTAs (of a cluster) that share the keys of a tile pair; 1: the pair has a CTA of its own
     int streams_z;  // (batch, KV head) streams per blockIdx.z
     int band;       // tile pairs of one (batch, KV head) that sit next to each other in blockIdx.x
     // Launch order of the bands (blockIdx.y), heaviest = 0. spread_w == 0: heaviest first. Otherwise the
@@ -558,10 +560,10 @@ __device__ __forceinline__ int3 find_item(const PrefillArgs& a, int index, int l
 // that the request follows the release at once. Looked up and requested page by page by one thread after the release,
 // a tile came about a thousand clocks later, which the two-stage rings do not hide: 3.6 % of a step of 4 chunks of 512 over
 // 1024-8192 tokens (page 16).
-__device__ __forceinline__ int page_of_lane(const PrefillArgs& a, int kv_len, int s, int j, int lane) {
+__device__ __forceinline__ int page_of_lane(const PrefillArgs& a, int kv_len, int s, int j, int lane, int first_key) {
     const int per_tile = kBlockN / a.block_size;
     const int pg = j * per_tile + lane;
-    return lane < per_tile && pg < (kv_len + a.block_size - 1) / a.block_size ? a.block_tables[(long long)s * a.max_blocks + pg] : -1;
+    return lane < per_tile && pg < (kv_len + a.block_size - 1) / a.block_size ? a.block_tables[(long long)s * a.max_blocks + first_key / a.block_size + pg] : -1;
 }
 
 // Contiguous K/V: called by one lane.
@@ -820,13 +822,149 @@ __device__ __forceinline__ bool find_pair(const PrefillArgs& a, int bx, int by, 
     return w.t[0].valid || w.t[1].valid;   // (a sequence may be shorter than the grid's row range)
 }
 
+// The share of a pair's keys that is this CTA's, of `parts` equal ones in whole tiles.
+__device__ __forceinline__ void take_share(Item& w, int parts, int rank) {
+    const int per = (max(w.t[0].n_kv, w.t[1].n_kv) + parts - 1) / parts;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) w.t[t].n_kv = max(0, min(per, w.t[t].n_kv - rank * per));
+    w.first_key = rank * per * kBlockN;
+    w.sq.kv_len -= w.first_key;
+    w.sq.pos_off -= w.first_key;
+    w.sq.kv_crow += w.first_key;
+}
+
+// Clusters: every thread of its CTAs takes part in every phase, and all waits of all roles end, so these do.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
+__device__ __forceinline__ unsigned peer_addr(const void* p, int rank) {   // the same place in another CTA's shared memory
+    unsigned at;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"(smem_u32(p)), "r"(rank));
+    return at;
+}
+
+// The end of a pair whose keys are shared out over a cluster: every CTA has O over its share, unnormalised, and each row's reference and sum, lays them down where K and V were, and
+// finishes 128 / parts rows of either tile from what all CTAs have: the rows' weights first, a thread a row, then a warp's lanes along the rows, 16 bytes each, eight loads in flight. What counts
+// is the number of instructions, which come in for the first time at some 24 clocks each, and of trips to the other CTAs (some 800 clocks): two full tiles of 128 columns took
+// 8 us by stores of 16 bytes into the other CTAs' rows, 7 with 16 loads in flight and the weights found by every lane, 4 so (device timer, clusters of two).
+// Run by the eight softmax warps. `have`: the CTA has a pair, and this thread's tile is final.
+template <typename T, int D, bool kMask>
+__device__ __forceinline__ void split_rows(const PrefillArgs& a, SharedStorage<D>& sm, bool have, int t, int r, int warp, int lane, unsigned o_addr, int n_kv, float m, float l) {
+    const int parts = a.parts, rank = (int)blockIdx.x & (parts - 1), share = kBlockM / parts;
+    float* const rows = reinterpret_cast<float*>(sm.k[0]);   // K's and V's rings: (tile, row, D), 16-byte chunks swizzled by the row
+    static_assert(offsetof(SharedStorage<D>, v) == offsetof(SharedStorage<D>, k) + sizeof(sm.k) && sizeof(sm.k) + sizeof(sm.v) >= 2 * kBlockM * D * 4, "the rings hold the rows of both tiles");
+    float2* const ml = reinterpret_cast<float2*>(sm.out[0]);   // (tile, row)
+    float* const weights = reinterpret_cast<float*>(sm.out[1]);   // (tile, row of the share, CTA)
+    static_assert(sizeof(float2) * 2 * kBlockM <= kOutBytes && sizeof(float) * 2 * kBlockM / 2 * 8 <= kOutBytes, "fit");
+    asm volatile("barrier.cta.sync 3, 256;\n" ::: "memory");   // the products of both tiles have finished, nobody reads K or V any more
+    ml[t * kBlockM + r] = have ? make_float2(m, l) : make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));   // (else a wait ran out: the rows are undefined)
+    const Item& w = sm.item[0];
+    const int pl = a.pack_log2;
+    if (have && n_kv > 0 && w.t[t].row0 + (warp & 3) * 32 < w.sq.q_len << pl) {   // (a warp whose rows exist)
+        tc_fence_after();
+        float* const mine = rows + (t * kBlockM + r) * D;
+#pragma unroll 1
+        for (int c = 0; c < D / 32; ++c) {
+            float ov[32];
+            tc_ld32(o_addr + c * 32, ov);
+            tc_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                *reinterpret_cast<float4*>(mine + (((c * 8 + i) ^ (r & 7)) << 2)) = make_float4(ov[4 * i], ov[4 * i + 1], ov[4 * i + 2], ov[4 * i + 3]);
+        }
+    }
+    cluster_arrive();
+    cluster_wait();
+    const bool some = w.some && w.t[t].valid;
+    const int rows_left = some ? (w.sq.q_len << pl) - w.t[t].row0 - rank * share : 0;   // rows of this share that exist
+    if (r < share && r < rows_left) {
+        const int row = w.t[t].row0 + rank * share + r, token = row >> pl, head = w.t[t].head + (row & ((1 << pl) - 1));
+        float2 y[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            y[c] = make_float2(-INFINITY, 0.0f);
+            if (c < parts) asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(y[c].x), "=f"(y[c].y) : "r"(peer_addr(ml + t * kBlockM + rank * share + r, c)) : "memory");
+        }
+        // the row's reference and sum over all keys: the sum is NaN where one of the shares saw a NaN or +inf, as in a tile of one CTA
+        float top = y[0].x, sum = 0.0f;
+#pragma unroll
+        for (int c = 1; c < 8; ++c) top = max_nan(top, y[c].x);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            y[c].x = y[c].x == -INFINITY ? 0.0f : ex2(y[c].x - top);
+            sum = fmaf(y[c].x, y[c].y, sum);
+        }
+        bool q_ok = true;
+        if (kMask) {
+            const long long pos = (long long)w.sq.pos_off + w.first_key + token;
+            q_ok = pos >= 0 && pos < (long long)w.sq.kv_len + w.first_key && a.mask[(long long)w.seq * a.kv_seq_len + pos] != 0;
+        }
+        const bool seen = sum > 0.0f && top < INFINITY && q_ok;
+        // (a share whose reference moved on behind its NaN has it in its sum and its O alone)
+        const float inv = seen ? 1.0f / sum : sum != sum ? sum : 0.0f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+            if (c < parts) weights[(t * share + r) * parts + c] = y[c].x * inv;
+        if (a.lse != nullptr) a.lse[((long long)w.seq * a.q_heads + head) * a.q_seq_len + token] = seen ? (top + log2f(sum)) * 0.6931471805599453f : -INFINITY;
+    }
+    asm volatile("barrier.cta.sync 3, 256;\n" ::: "memory");   // the weights are there
+    if (rows_left > 0) {
+        constexpr int kLanes = D / 4, kRows = 32 / kLanes, kDeep = 4;   // lanes to a row; rows of a warp's load; loads of a part in flight
+        const int col = (lane % kLanes) * 4;
+#pragma unroll 1
+        for (int i0 = (warp & 3) * kRows + lane / kLanes; i0 < share; i0 += 4 * kRows * kDeep) {
+            float4 o[kDeep];
+#pragma unroll
+            for (int k = 0; k < kDeep; ++k) o[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+            for (int c = 0; c < parts; c += 2) {
+                float4 x[2][kDeep];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const unsigned from = peer_addr(rows + (t * kBlockM + rank * share) * D, c + h);
+#pragma unroll
+                    for (int k = 0; k < kDeep; ++k) {
+                        const int i = min(i0 + k * 4 * kRows, share - 1);
+                        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                                     : "=f"(x[h][k].x), "=f"(x[h][k].y), "=f"(x[h][k].z), "=f"(x[h][k].w)
+                                     : "r"(from + i * (D * 4) + (((lane % kLanes) ^ ((rank * share + i) & 7)) << 4))
+                                     : "memory");
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int k = 0; k < kDeep; ++k) {
+                        const float by = weights[(t * share + min(i0 + k * 4 * kRows, share - 1)) * parts + c + h];
+                        if (by != 0.0f) {   // (where a share saw no key, what lies there is nothing of ours)
+                            o[k].x = fmaf(by, x[h][k].x, o[k].x);
+                            o[k].y = fmaf(by, x[h][k].y, o[k].y);
+                            o[k].z = fmaf(by, x[h][k].z, o[k].z);
+                            o[k].w = fmaf(by, x[h][k].w, o[k].w);
+                        }
+                    }
+            }
+#pragma unroll
+            for (int k = 0; k < kDeep; ++k) {
+                const int i = i0 + k * 4 * kRows, row = w.t[t].row0 + rank * share + i;
+                if (i < min(share, rows_left) && col < a.d_real) {
+                    const long long at = ((w.sq.o_row0 + (row >> pl)) * a.o_heads + a.o_head0 + w.t[t].head + (row & ((1 << pl) - 1))) * a.d_real + col;
+                    *reinterpret_cast<uint2*>(static_cast<T*>(a.o[0]) + at) = make_uint2(pack16<T>(o[k].x, o[k].y), pack16<T>(o[k].z, o[k].w));
+                }
+            }
+        }
+    }
+    cluster_arrive();   // nobody's shared memory goes while another reads it
+    cluster_wait();
+}
+
 // kMask: the call carries a key-padding mask (a separate instantiation, so that calls without one
 // pay nothing for it in the softmax loop)
 // kPaged: paged K/V, whose tiles are gathered page by page and whose tile pairs may be ordered on the device (a separate instantiation as
 // well: with the code of the two in it the contiguous calls' kernel took 375 us for 24 prompts of 17-2000 tokens at d = 64,
 // 364 without; 2 x 8192 GQA 1047 against 1027)
 // kOnePair: a CTA works on its own tile pair and no other; nobody looks for a next one.
-template <typename T, int D, bool kMask, bool kPaged, bool kOnePair>
+// kSplit (of those): the CTAs of a cluster share the keys of a tile pair and merge their rows through distributed shared memory.
+template <typename T, int D, bool kMask, bool kPaged, bool kOnePair, bool kSplit>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                        const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap o_map, const PrefillArgs a) {
@@ -863,11 +1001,12 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         bool begun = false;   // the first tile pair's first copies have been requested
         // The CTA's own tile pair, and its first copies at once, in as few instructions as that takes: all of them come in for the first time here, and
         // in the loop below, with its waits and cases, the first S came 1600 to 2300 clocks later (a fifth of a call of one short wave).
-        w.some = find_pair<kMask, kPaged>(a, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, lane, w);
+        w.some = find_pair<kMask, kPaged>(a, kSplit ? (int)blockIdx.x / a.parts : (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, lane, w);
+        if (kSplit && w.some) take_share(w, a.parts, (int)blockIdx.x % a.parts);
         asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
         begun = w.some && max(w.t[0].n_kv, w.t[1].n_kv) > 0 && !q_open && !kv_open && a.test_skip_k != 1;
         if (begun && (kPaged || lane == 0)) {
-            const int page = kPaged ? page_of_lane(a, w.sq.kv_len, w.seq, 0, lane) : -1;
+            const int page = kPaged ? page_of_lane(a, w.sq.kv_len, w.seq, 0, lane, kSplit ? w.first_key : 0) : -1;
             if (lane == 0 && w.t[0].n_kv > 0) {
                 mbar_expect_tx(&sm.q_full[0], TileBytes<D>::value);
                 tma_load_4d(sm.q[0], &q_map, &sm.q_full[0], 0, w.t[0].head, w.sq.q_crow + (w.t[0].row0 >> a.pack_log2), w.sq.q_cb);
@@ -974,7 +1113,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     if (D == 128) tma_prefetch_4d(&q_map, 64, w.t[1].head, w.sq.q_crow + (w.t[1].row0 >> a.pack_log2), w.sq.q_cb);
                 }
             }
-            int page = kPaged ? page_of_lane(a, kv_len, seq, 0, lane) : -1;
+            int page = kPaged ? page_of_lane(a, kv_len, seq, 0, lane, kSplit ? w.first_key : 0) : -1;
             auto load_k = [&](int j) {   // K tile j of the pair is what step g + j - 1 reads besides its V tile, and arrives on its barrier (tile 0: on its own)
                 const int e = (g + j) & 1;
                 unsigned long long* const bar = j == 0 ? &sm.k_first : &sm.step_full[e ^ 1];
@@ -989,7 +1128,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 (e ? k_free1 : k_free0) = commits + j;
                 if (j > 0) given = g + j;
                 else if (!skip) ++firsts;
-                if (kPaged && j + 1 < n_max) page = page_of_lane(a, kv_len, seq, j + 1, lane);
+                if (kPaged && j + 1 < n_max) page = page_of_lane(a, kv_len, seq, j + 1, lane, kSplit ? w.first_key : 0);
             };
             // (a tile that sees no key needs no Q: the issuer leaves it out)
             auto load_q = [&](const TileInfo ti, unsigned char* to, unsigned long long* bar, unsigned& loads) {
@@ -1012,7 +1151,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 firsts = 1;
                 q_loads0 = n0 > 0;
                 q_loads1 = n1 > 0;
-                if (kPaged && n_max > 1) page = page_of_lane(a, kv_len, seq, 1, lane);
+                if (kPaged && n_max > 1) page = page_of_lane(a, kv_len, seq, 1, lane, kSplit ? w.first_key : 0);
             } else
 #pragma unroll 1
             for (int n = 0; n < 3; ++n) {
@@ -1086,7 +1225,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             // ring's barrier with a plain arrival. (Garbage in K is harmless: the score mask is a select.)
             const bool tail_fix = (a.paged || packed) && (sq.kv_len % kBlockN) != 0;
             const int tail_j = sq.kv_len > 0 ? (sq.kv_len - 1) / kBlockN : -1;
-            int page = kPaged ? page_of_lane(a, sq.kv_len, w.seq, 0, lane) : -1;
+            int page = kPaged ? page_of_lane(a, sq.kv_len, w.seq, 0, lane, kSplit ? w.first_key : 0) : -1;
             for (int j = 0; j < n_max; ++j) {
                 const int e = (g + j) & 1;
                 const int c = e ? v_free1 : v_free0;
@@ -1099,7 +1238,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 else if (kPaged || lane == 0)
                     load_kv_tile<D, kPaged>(a, sq.kv_crow, sq.kv_cb, w.kv_head, sm.v[e], &v_map, bar, j, page, lane);
                 (e ? v_free1 : v_free0) = commits + j + 1;
-                if (kPaged && j + 1 < n_max) page = page_of_lane(a, sq.kv_len, w.seq, j + 1, lane);
+                if (kPaged && j + 1 < n_max) page = page_of_lane(a, sq.kv_len, w.seq, j + 1, lane, kSplit ? w.first_key : 0);
                 if (!fix) {
                     given = g + j + 1;
                     continue;
@@ -1187,6 +1326,9 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         const unsigned s_addr = tmem + lane_base + t * 128;
         const unsigned o_addr = tmem + lane_base + 256 + t * 128;
         unsigned steps = 0, tiles = 0;    // of this query tile so far: steps, and tiles with a step
+        [[maybe_unused]] bool have = false;
+        [[maybe_unused]] int last_n = 0;
+        [[maybe_unused]] float last_m = 0.0f, last_l = 0.0f;
         bool alive = true;
 #ifdef FA_TRACE
         long long* trace = (a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == (unsigned)a.trace_y && blockIdx.z == 0 && lane == 0 && (warp & 3) == 0) ? a.trace : nullptr;
@@ -1202,6 +1344,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.item_empty[it & 1u]);
         if (!some) break;
+        const int first_key = kSplit ? sm.item[it & 1u].first_key : 0;
         const int row = ti.row0 + r, pl = a.pack_log2;
         const long long pos = (long long)sq.pos_off + (row >> pl);   // global position of this row's query token
         // the last key that this row sees, and the last that every row of the tile sees (-1: none)
@@ -1233,7 +1376,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 for (int c = 0; c < 4; ++c) {
                     const int kk = key0 + c * 32 + lane;
                     const bool real = kk < sq.kv_len;
-                    valid[c] = __ballot_sync(0xffffffffu, real && a.mask[(long long)b * a.kv_seq_len + (real ? kk : 0)] != 0);
+                    valid[c] = __ballot_sync(0xffffffffu, real && a.mask[(long long)b * a.kv_seq_len + first_key + (real ? kk : 0)] != 0);
                     masked = masked || valid[c] != __ballot_sync(0xffffffffu, real);
                 }
             }
@@ -1321,6 +1464,13 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         if (alive && ti.n_kv > 0)
             alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.o_full[t], tiles++ & 1u, a, 30 + t));
         FA_TRACE_EVENT(t, max(0, (int)steps - 1), 4);
+        if constexpr (kSplit) {
+            have = alive;
+            last_n = ti.n_kv;
+            last_m = m;
+            last_l = l;
+            break;
+        }
         if (alive && ti.valid) {
             tc_fence_after();
             const int rows_end = sq.q_len << pl, token = row >> pl, head = ti.head + (row & ((1 << pl) - 1));
@@ -1473,7 +1623,14 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             FA_TRACE_EVENT(t, max(0, (int)steps - 1), 5);       // epilogue stores issued
         }
         }
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // shared memory stays valid until read
+        if constexpr (kSplit) split_rows<T, D, kMask>(a, sm, have, t, r, warp, lane, o_addr, last_n, last_m, last_l);
+        else if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // shared memory stays valid until read
+    }
+    if (kSplit && warp >= 8) {   // the phases of split_rows, where every thread of a cluster is counted
+        cluster_arrive();
+        cluster_wait();
+        cluster_arrive();
+        cluster_wait();
     }
 
     tc_fence_before();
@@ -1781,9 +1938,48 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     // a grid in order has empty CTAs, which are cheaper to take over (serve steps of 4 chunks with 32 tokens 226 and 228, 6 with 40 310 and 318), and so are short pairs at head size
     // 64 (8 x 200 over 512-4096, 32/8 heads 68.5 and 69.6). Contiguous K/V at head size 64: no difference (1 x 449, 64/8 heads of 32 11.6 either way; 1 x 2048, 8/8 heads 26.8 and
     // 27.3), and none is built.
+    // Where the tile pairs leave SMs without one, a cluster of 2, 4 or 8 CTAs shares the keys of each, as many as find room at the same time (one CTA to an SM; 33 clusters of four and 15
+    // of eight, as the SMs lie) and two tiles for each, for a cluster of eight four. It takes 2 us (a few rows) to 7 (full tiles of 128 columns and eight CTAs) more, a tile 1.5. us from a graph,
+    // alone and shared by 2, 4, 8: 1 x 512 tokens over 8192, 32/8 heads 108, 70; 1 x 64 over 8192 105, 64, 41, 31; 5 x 84 over 339-5439, 8 heads of 64 57, 36; 1 x 2048, 8 heads 28.7, 23.6; 2 x 64 over
+    // 30000, 32/8 heads of 64 354, 192, 103, 115 (16 clusters of eight, in two rounds); 8 x 1 token over 1022, 8/2 heads 15.0, 12.6, 9.8; 4 x 1 over 544, 32/8 heads of 64 10.0, 9.8.
+    // More than a few rows over at most 12 tiles stay alone: their results have the bits of the same rows in a call that fills the device.
+    int parts = 1;
+    const long long tiles = (kv_rows + kBlockN - 1) / kBlockN, rows = (long long)p.q_seq_len * group;
+    if (p.n_out == 0 && a.skip_rows == 0 && (tiles > 12 || rows <= 16)) {
+        if (2 * all <= sm_count() && tiles >= 4) parts = 2;
+        if (9 * all <= 2 * sm_count() && tiles >= 8) parts = 4;
+        if (21 * all <= 2 * sm_count() && tiles >= (rows > 16 ? 32 : 16)) parts = 8;
+    }
+    a.parts = parts;
+    if (parts > 1) {
+        const auto kernel = prefill_tcgen05_kernel<T, D, kMask, kPaged, true, true>;
+        cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (err == cudaSuccess) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(grid.x * (unsigned)parts, grid.y, grid.z);
+            cfg.blockDim = dim3(kThreads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = stream;
+            cudaLaunchAttribute attr{};
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = (unsigned)parts;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            cudaLaunchKernelEx(&cfg, kernel, qm, km, vm, om, a);
+        }
+        if (err != cudaSuccess) {
+            set_last_errorf("prefill_tcgen05_kernel: %s", cudaGetErrorString(err));
+            cudaGetLastError();
+            return FLASH_ATTN_ERR_CUDA;
+        }
+        const int rc = check_launch("prefill_tcgen05_kernel");
+        if (rc == FLASH_ATTN_OK) note_path("prefill_tcgen05", 1);
+        return rc;
+    }
     constexpr bool kOneWave = D == 128 || kPaged;
     const bool one_pair = kOneWave && ((long long)grid.x * grid.y * grid.z <= sm_count() || (D == 128 && a.ordered && a.skip_rows == 0));
-    const auto kernel = one_pair ? prefill_tcgen05_kernel<T, D, kMask, kPaged, kOneWave> : prefill_tcgen05_kernel<T, D, kMask, kPaged, false>;
+    const auto kernel = one_pair ? prefill_tcgen05_kernel<T, D, kMask, kPaged, kOneWave, false> : prefill_tcgen05_kernel<T, D, kMask, kPaged, false, false>;
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) {
         set_last_errorf("prefill_tcgen05_kernel: %s", cudaGetErrorString(err));
