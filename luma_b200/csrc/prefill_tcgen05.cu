@@ -77,7 +77,7 @@ __device__ __forceinline__ constexpr bool fma_pipe_exp(int i) { return (i & 7) =
 // Extents of one sequence. Query row i sits at global position pos_off + i and sees keys
 // j < kv_len with j <= pos_off + i (bottom-right aligned for the varlen and kv-cache entry points).
 struct SeqExtent {
-    int q_len, kv_len, pos_off;
+    int q_len, kv_len, pos_off;   // (positions fit 32 bits: the last one is below kv_len or, batched, kv_seq_len + q_seq_len; see start_pos)
     long long o_row0;     // first row of this sequence in o (rows of o_heads * 128 elements)
     int q_crow, q_cb;     // TMA coordinates (row, batch) of the sequence's first q row
     int kv_crow, kv_cb;   // same for contiguous K/V (unused when paged)
@@ -448,9 +448,9 @@ __device__ __forceinline__ TileInfo tile_info(const SeqExtent& a, int pair, int 
     ti.head = (kvh * packs + (ti.valid ? idx - mb * packs : 0)) << pack_log2;
     ti.row0 = mb * kBlockM;
     const int last_token = (min(ti.row0 + kBlockM, a.q_len << pack_log2) - 1) >> pack_log2;
-    const long long last_key = min((long long)a.kv_len - 1, (long long)a.pos_off + last_token);
-    ti.n_kv = (ti.valid && last_key >= 0) ? (int)(last_key / kBlockN) + 1 : 0;   // 0: the tile sees no key at all
-    if (kMask && (long long)a.pos_off + (ti.row0 >> pack_log2) >= a.kv_len) ti.n_kv = 0;   // all its rows sit in padding
+    const int last_key = min(a.kv_len - 1, a.pos_off + last_token);
+    ti.n_kv = ti.valid && last_key >= 0 ? last_key / kBlockN + 1 : 0;   // 0: the tile sees no key at all
+    if (kMask && a.pos_off + (ti.row0 >> pack_log2) >= a.kv_len) ti.n_kv = 0;   // all its rows sit in padding
     return ti;
 }
 
@@ -814,8 +814,8 @@ __device__ __forceinline__ bool find_pair(const PrefillArgs& a, int bx, int by, 
     if (kMask) {
         // Padding behind a pair's last key that counts is not walked: the pair's keys end there, and a tile all of whose rows sit in padding (their output is zeros) sees none.
         const int last = tile_token_end(w.sq, pair * 2 + 1, a.by_packs, a.pack_log2, num_mb);   // one past the pair's last query token
-        const long long end = min((long long)w.sq.kv_len, (long long)w.sq.pos_off + last);
-        if (end > 0) w.sq.kv_len = seen_below(a.mask + (long long)w.seq * a.kv_seq_len, (int)end, lane);
+        const int end = min(w.sq.kv_len, w.sq.pos_off + last);
+        if (end > 0) w.sq.kv_len = seen_below(a.mask + (long long)w.seq * a.kv_seq_len, end, lane);
     }
     w.t[0] = tile_info<kMask>(w.sq, pair, 0, w.kv_head, a.by_packs, a.pack_log2, num_mb);
     w.t[1] = tile_info<kMask>(w.sq, pair, 1, w.kv_head, a.by_packs, a.pack_log2, num_mb);
@@ -895,8 +895,8 @@ __device__ __forceinline__ void split_rows(const PrefillArgs& a, SharedStorage<D
         }
         bool q_ok = true;
         if (kMask) {
-            const long long pos = (long long)w.sq.pos_off + w.first_key + token;
-            q_ok = pos >= 0 && pos < (long long)w.sq.kv_len + w.first_key && a.mask[(long long)w.seq * a.kv_seq_len + pos] != 0;
+            const int pos = w.sq.pos_off + w.first_key + token;
+            q_ok = pos >= 0 && pos < w.sq.kv_len + w.first_key && a.mask[(long long)w.seq * a.kv_seq_len + pos] != 0;
         }
         const bool seen = sum > 0.0f && top < INFINITY && q_ok;
         // (a share whose reference moved on behind its NaN has it in its sum and its O alone)
@@ -1346,9 +1346,9 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         if (!some) break;
         const int first_key = kSplit ? sm.item[it & 1u].first_key : 0;
         const int row = ti.row0 + r, pl = a.pack_log2;
-        const long long pos = (long long)sq.pos_off + (row >> pl);   // global position of this row's query token
+        const int pos = sq.pos_off + (row >> pl);   // global position of this row's query token
         // the last key that this row sees, and the last that every row of the tile sees (-1: none)
-        const int last_seen = (int)max(-1LL, min(pos, (long long)sq.kv_len - 1)), all_see = (int)max(-1LL, min((long long)sq.pos_off + (ti.row0 >> pl), (long long)sq.kv_len - 1));
+        const int last_seen = max(-1, min(pos, sq.kv_len - 1)), all_see = max(-1, min(sq.pos_off + (ti.row0 >> pl), sq.kv_len - 1));
         float m = -INFINITY;   // reference max, log2 domain (may lag the true max by <= 2^8)
         float l = 0.0f;
 
@@ -1477,7 +1477,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             const bool row_ok = row < rows_end;
             // with a padding mask a query row at a padded (or out-of-range) position outputs zeros (flash_attn_func.cu:77-84)
             bool q_ok = true;
-            if (kMask) q_ok = row_ok && pos >= 0 && pos < (long long)sq.kv_len && a.mask[(long long)b * a.kv_seq_len + pos] != 0;
+            if (kMask) q_ok = row_ok && pos >= 0 && pos < sq.kv_len && a.mask[(long long)b * a.kv_seq_len + pos] != 0;
             const bool seen = l > 0.0f && m < INFINITY && q_ok;   // (false where a score was NaN, l NaN, or +inf, m +inf: 0 times that row's NaN or infinity is NaN)
             const float inv = seen ? 1.0f / l : 0.0f;
             // a bulk store writes every row of its box that lies inside the tensor: in a packed buffer the
@@ -1824,7 +1824,7 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     a.kv_seq_len = p.kv_seq_len;
     a.q_heads = p.q_heads;
     a.kv_heads = p.kv_heads;
-    a.start_pos = p.start_pos;
+    a.start_pos = std::min(p.start_pos, p.kv_seq_len);   // (behind the keys there is nothing more to see)
     a.d_real = d_real;
     a.mode = p.mode;
     a.q = p.q;
