@@ -149,6 +149,14 @@ __host__ __device__ inline long long prefill_pairs(int group, long long q_len) {
     return ((long long)(group / pack) * ((q_len * pack + 127) / 128) + 1) / 2;
 }
 
+// CTAs that share the keys of a tile pair there: of `pairs` pairs in all over up to `tiles` K/V tiles (`exact`: over as many), `rows` rows per KV head and sequence (rule and times
+// where it is launched).
+inline int prefill_parts(long long pairs, long long tiles, bool exact, long long rows, int sms) {
+    if (tiles <= (rows <= 16 && exact ? 7 : 12)) return 1;
+    if (21 * pairs <= 2 * sms && tiles >= (rows > 16 ? 32 : 16)) return 8;
+    return 9 * pairs <= 2 * sms ? 4 : 2 * pairs <= sms ? 2 : 1;
+}
+
 template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }

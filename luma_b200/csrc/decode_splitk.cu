@@ -25,6 +25,7 @@
 // Token -> slot arithmetic is that of block_slot() in common.cuh (reference: kernels/common.cuh:89-108).
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <mutex>
 #include <type_traits>
 
@@ -1069,21 +1070,31 @@ static double rows_us(const AttnParams& p, long long seqs, long long rows) {
     return 4.4 + ((rows > kRows ? 0.91 : 1.04) * units + 2.2 + 0.15 * nrows) * blocks_per_slot + (units > 1.0 ? 0.6 * nrows : 0.0);
 }
 
-// Up to four row blocks of 16 (query token x group head) rows, each of which reads the K/V rows again, from L2. The prefill kernel's one or two
-// tiles per CTA are almost empty, but it reads K/V once: over up to 12 tiles in one wave of its CTAs (25 us at most) it keeps the call,
-// else the estimates decide. Both kernels over the 235 of 298 shapes that get this far (1-64 sequences x 1-64 tokens, 64-8192 keys, groups of 1, 4
-// and 8): the choice is at most 5 % slower than the prefill kernel and at most 9 % slower than this one. 64 rows:
-// 64 x 64 tokens x 1600 keys, 32 heads without GQA 275 us on the prefill kernel, 743 here; 1 x 16 x 8192, 32/8 heads 110 and 31. 16 rows: 16 x 4 x
-// 8192, 32/8: 180 and 63. With the prefill kernel as it is now, 135 calls drawn anew: the 102 that get this far at most 0.1 % slower than it and
-// 2.5 % slower than this one; of the 33 that it keeps for their short K/V the slowest takes 27 us where this kernel would take 11 (4 x 1 token over 256-1024, 64/8
-// heads).
+// Prefill kernel, the few rows of a sequence in one tile for as many heads as share one, clusters for the keys where they find room: 4 us a wave and 1.4 us per 128 keys, 4 more for a cluster.
+static double prefill_few_rows_us(const AttnParams& p, long long rows) {
+    const long long pairs = prefill_pairs(p.q_heads / p.kv_heads, p.q_seq_len) * p.kv_heads * p.num_seqs, tiles = (longest_keys(p) + 127) / 128;
+    const int parts = prefill_parts(pairs, tiles, p.mode == MODE_BATCH, rows, sm_count());
+    const double waves = std::max(1.0, (double)pairs / sm_count());
+    return std::ceil(waves) * 4.0 + waves * 1.4 * (double)((tiles + parts - 1) / parts) + (parts > 1 ? 4.0 : 0.0);
+}
+
+// Up to four row blocks of 16 (query token x group head) rows, each of which reads the K/V rows again, from L2; the prefill kernel reads K/V once and has them in one tile
+// where the heads of a group share it. Both kernels over 154 shapes of 1-64 sequences x 1-32 tokens, 64-32768 keys, groups of 1, 4 and 8: the choice takes on average 6 % more than the
+// faster kernel for each (9 % with a tile for every head in the estimate, and with all calls of one wave over up to 12 tiles left to the prefill kernel). us there and here:
+// 32 x 12 tokens over 1031-4126, 32/8 heads 81 and 139; 41 x 8 over 1375, 64/8 78 and 142; 16 x 4 over 216, 64/8 9.6 and 17.3; 8 x 2 over 1010, 32/8 17.7 and 13.3; 16 x 8 over 400,
+// 8 heads of 64 12.9 and 10.6; 16 x 4 over 8192, 32/8 96 and 92. The estimate has to say half for the prefill kernel: it does not know the lengths, and equal shares suit unequal ones.
+// Two groups of calls stay with one kernel whatever the estimates say, because programs and tests know them there: up to 64 pairs, counted by heads, over up to 12 tiles with the prefill
+// kernel (4 x 1 over 544, 32/8 heads of 64 9.6 and 6.0), and up to 4 sequences by the estimates of a tile for every head (1 x 64 over 8192, 32 heads 33 and 68).
 int launch_few_rows(const AttnParams& p, bool prefill_takes_it, cudaStream_t stream) {
     if (p.n_out > 0 || !rows_kernel_takes(p)) return -1;
     const long long rows = (long long)p.q_seq_len * (p.q_heads / p.kv_heads);
     if (rows <= 0 || rows > 4 * kRows) return -1;
     const double pairs = (double)tile_pairs(p, p.q_seq_len) * p.num_seqs;
-    if (longest_keys(p) <= 12 * 128 && pairs <= sm_count()) return -1;
-    if (prefill_takes_it && rows_us(p, p.num_seqs, rows) >= prefill_us(p, pairs)) return -1;
+    if (longest_keys(p) <= 12 * 128 && pairs <= 64) return -1;
+    if (prefill_takes_it) {
+        const double here = rows_us(p, p.num_seqs, rows);
+        if (p.num_seqs > 4 ? prefill_few_rows_us(p, rows) < 0.575 * here : here >= prefill_us(p, pairs)) return -1;
+    }
     RowsPlan plan;
     Workspace ws;
     if (prepare_rows(p, (int)rows, stream, plan, ws) != FLASH_ATTN_OK) return -1;   // the prefill kernel needs no memory of the library's

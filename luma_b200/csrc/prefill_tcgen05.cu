@@ -95,6 +95,7 @@ struct Item {
     int some;            // 0: nothing is left, the CTA ends
     int seq, kv_head;
     int first_key;       // where the CTA's share of the keys begins (a multiple of a tile); kv_len, pos_off and kv_crow of `sq` count from there
+    int shared;          // the CTAs of the cluster share the keys (0: there are too few, or there is no pair)
     SeqExtent sq;
     TileInfo t[2];
 };
@@ -822,9 +823,16 @@ __device__ __forceinline__ bool find_pair(const PrefillArgs& a, int bx, int by, 
     return w.t[0].valid || w.t[1].valid;   // (a sequence may be shorter than the grid's row range)
 }
 
-// The share of a pair's keys that is this CTA's, of `parts` equal ones in whole tiles.
+// The share of a pair's keys that is this CTA's, of `parts` equal ones in whole tiles. A pair of up to five tiles stays whole, with the first CTA (the host knows a bound only: 2 x 147 tokens
+// over 609 keys with room for 2048, 8/2 heads, shared by four 18.9 us, alone 17.5).
 __device__ __forceinline__ void take_share(Item& w, int parts, int rank) {
-    const int per = (max(w.t[0].n_kv, w.t[1].n_kv) + parts - 1) / parts;
+    const int most = max(w.t[0].n_kv, w.t[1].n_kv), per = (most + parts - 1) / parts;
+    w.first_key = 0;
+    w.shared = most > 5;
+    if (!w.shared) {
+        w.some = rank == 0;
+        return;
+    }
 #pragma unroll
     for (int t = 0; t < 2; ++t) w.t[t].n_kv = max(0, min(per, w.t[t].n_kv - rank * per));
     w.first_key = rank * per * kBlockN;
@@ -855,7 +863,6 @@ __device__ __forceinline__ void split_rows(const PrefillArgs& a, SharedStorage<D
     float2* const ml = reinterpret_cast<float2*>(sm.out[0]);   // (tile, row)
     float* const weights = reinterpret_cast<float*>(sm.out[1]);   // (tile, row of the share, CTA)
     static_assert(sizeof(float2) * 2 * kBlockM <= kOutBytes && sizeof(float) * 2 * kBlockM / 2 * 8 <= kOutBytes, "fit");
-    asm volatile("barrier.cta.sync 3, 256;\n" ::: "memory");   // the products of both tiles have finished, nobody reads K or V any more
     ml[t * kBlockM + r] = have ? make_float2(m, l) : make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));   // (else a wait ran out: the rows are undefined)
     const Item& w = sm.item[0];
     const int pl = a.pack_log2;
@@ -1002,7 +1009,10 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         // The CTA's own tile pair, and its first copies at once, in as few instructions as that takes: all of them come in for the first time here, and
         // in the loop below, with its waits and cases, the first S came 1600 to 2300 clocks later (a fifth of a call of one short wave).
         w.some = find_pair<kMask, kPaged>(a, kSplit ? (int)blockIdx.x / a.parts : (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, lane, w);
-        if (kSplit && w.some) take_share(w, a.parts, (int)blockIdx.x % a.parts);
+        if (kSplit) {
+            w.shared = 0;
+            if (w.some) take_share(w, a.parts, (int)blockIdx.x % a.parts);
+        }
         asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
         begun = w.some && max(w.t[0].n_kv, w.t[1].n_kv) > 0 && !q_open && !kv_open && a.test_skip_k != 1;
         if (begun && (kPaged || lane == 0)) {
@@ -1464,7 +1474,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         if (alive && ti.n_kv > 0)
             alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.o_full[t], tiles++ & 1u, a, 30 + t));
         FA_TRACE_EVENT(t, max(0, (int)steps - 1), 4);
-        if constexpr (kSplit) {
+        if (kSplit && sm.item[0].shared) {
             have = alive;
             last_n = ti.n_kv;
             last_m = m;
@@ -1623,14 +1633,20 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             FA_TRACE_EVENT(t, max(0, (int)steps - 1), 5);       // epilogue stores issued
         }
         }
-        if constexpr (kSplit) split_rows<T, D, kMask>(a, sm, have, t, r, warp, lane, o_addr, last_n, last_m, last_l);
-        else if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // shared memory stays valid until read
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // shared memory stays valid until read
+        if constexpr (kSplit) {
+            __syncthreads();   // the products of both tiles have finished, nobody reads K or V any more
+            if (sm.item[0].shared) split_rows<T, D, kMask>(a, sm, have, t, r, warp, lane, tmem + lane_base + 256 + t * 128, last_n, last_m, last_l);
+        }
     }
-    if (kSplit && warp >= 8) {   // the phases of split_rows, where every thread of a cluster is counted
-        cluster_arrive();
-        cluster_wait();
-        cluster_arrive();
-        cluster_wait();
+    if (kSplit && warp >= 8) {
+        __syncthreads();           // (every role has ended: what the K producer found out is there, and the same in all CTAs of the cluster)
+        if (sm.item[0].shared) {   // the phases of split_rows, where every thread of a cluster is counted
+            cluster_arrive();
+            cluster_wait();
+            cluster_arrive();
+            cluster_wait();
+        }
     }
 
     tc_fence_before();
@@ -1939,17 +1955,12 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     // 64 (8 x 200 over 512-4096, 32/8 heads 68.5 and 69.6). Contiguous K/V at head size 64: no difference (1 x 449, 64/8 heads of 32 11.6 either way; 1 x 2048, 8/8 heads 26.8 and
     // 27.3), and none is built.
     // Where the tile pairs leave SMs without one, a cluster of 2, 4 or 8 CTAs shares the keys of each, as many as find room at the same time (one CTA to an SM; 33 clusters of four and 15
-    // of eight, as the SMs lie) and two tiles for each, for a cluster of eight four. It takes 2 us (a few rows) to 7 (full tiles of 128 columns and eight CTAs) more, a tile 1.5. us from a graph,
+    // of eight, as the SMs lie), for a cluster of eight with four tiles for each. It takes 2 us (a few rows) to 7 (full tiles of 128 columns and eight CTAs) more, a tile 1.5. us from a graph,
     // alone and shared by 2, 4, 8: 1 x 512 tokens over 8192, 32/8 heads 108, 70; 1 x 64 over 8192 105, 64, 41, 31; 5 x 84 over 339-5439, 8 heads of 64 57, 36; 1 x 2048, 8 heads 28.7, 23.6; 2 x 64 over
     // 30000, 32/8 heads of 64 354, 192, 103, 115 (16 clusters of eight, in two rounds); 8 x 1 token over 1022, 8/2 heads 15.0, 12.6, 9.8; 4 x 1 over 544, 32/8 heads of 64 10.0, 9.8.
-    // More than a few rows over at most 12 tiles stay alone: their results have the bits of the same rows in a call that fills the device.
-    int parts = 1;
-    const long long tiles = (kv_rows + kBlockN - 1) / kBlockN, rows = (long long)p.q_seq_len * group;
-    if (p.n_out == 0 && a.skip_rows == 0 && (tiles > 12 || rows <= 16)) {
-        if (2 * all <= sm_count() && tiles >= 4) parts = 2;
-        if (9 * all <= 2 * sm_count() && tiles >= 8) parts = 4;
-        if (21 * all <= 2 * sm_count() && tiles >= (rows > 16 ? 32 : 16)) parts = 8;
-    }
+    // More than a few rows over at most 12 tiles stay alone: their results have the bits of the same rows in a call that fills the device. So do a few rows where there may be no more than 12 (over
+    // pages, whose lengths the host does not know: 2 x 6 over 361 with room for 1024, 32 heads 13.0 alone, 14.8 as a cluster that finds too few to share) or are no more than 7 tiles.
+    const int parts = p.n_out > 0 || a.skip_rows > 0 ? 1 : prefill_parts(all, (kv_rows + kBlockN - 1) / kBlockN, p.mode == MODE_BATCH, (long long)p.q_seq_len * group, sm_count());
     a.parts = parts;
     if (parts > 1) {
         const auto kernel = prefill_tcgen05_kernel<T, D, kMask, kPaged, true, true>;

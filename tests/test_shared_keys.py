@@ -33,7 +33,7 @@ def _twice(call, want, what):
     (3, 129, 2100, 4, 4, 1971, False),     # 4; a pair with one row in its second tile
     (2, 1700, 1700, 6, 2, 0, False),       # 2; early rows see few of the shares
     (1, 300, 1800, 3, 3, 0, False),        # keys that nobody sees
-    (2, 200, 2000, 4, 2, 1800, True), (4, 1, 1100, 8, 2, 1099, True), (3, 4, 700, 4, 1, 696, True),
+    (2, 200, 2000, 4, 2, 1800, True), (4, 1, 1100, 8, 2, 1099, True), (3, 4, 1000, 4, 1, 996, True),
 ])
 def test_batched(b, sq, skv, hq, hkv, sp, masked, d, dt):
     q, k, v = (H.round_to(H.normal(s, x), dt) for s, x in (((b, sq, hq, d), 1), ((b, skv, hkv, d), 2), ((b, skv, hkv, d), 3)))
