@@ -68,11 +68,12 @@ constexpr int kHalfBytes = kBlockN * 64 * 2;   // 16 KiB: one 64-column half, 12
 template <int D> struct TileBytes { static constexpr int value = kBlockN * D * 2; };   // one half at D = 64, two at D = 128
 constexpr float kRescaleThreshold = 8.0f;            // log2 units
 
-// Which element pairs take their exponential on the FMA pipe (a quintic) instead of the special-function unit: one in eight. It costs issue slots
-// and registers that the special-function unit's time does not buy back at a larger share where CTAs are short. us a pass for a share of 1/16, 1/8,
-// 1/6, 1/4: 2 x 8192 GQA 932, 903, 895, 881; 4 x 2048 MHA 155.0, 151.6, 148.9, 148.1; 24 packed prompts at head size 64 337, 335, 329, 332; 4 chunks of 512
-// 145.1, 142.5, 143.8, 144.7; chunks with 32 decoding sequences 225.9, 225.0, 226.8, 230.4; 7 packed prompts of 7-125 tokens 27.4, 27.0, 27.3, 28.1.
-__device__ __forceinline__ constexpr bool fma_pipe_exp(int i) { return (i & 7) == 7; }
+// Which element pairs take their exponential on the FMA pipe (a quintic) instead of the special-function unit: one in six at head size 128, one in eight at 64. It costs issue slots
+// and registers that the special-function unit's time does not buy back at a larger share, at head size 64 at that already. us from a graph for a share of 1/8, 1/7, 1/6, 1/5: 2 x 8192 GQA 807.6, 802.7, 797.7,
+// 807.8; 4 x 2048 MHA 129.4, 128.7, 128.1, 129.3; 4 chunks of 512 137.8, 136.2, 136.5, 135.8, with 32 decoding sequences 219.1, 218.4, 215.6, 216.2; 24 packed prompts of 1000 225.8, 227.8,
+// 227.9, 230.1. At head size 64, 1/8, 1/6, 1/5, 1/4: 2 x 4096 189.7, 195.6, 191.8, 197.7; 8 x 1000 65.3, 67.0, 66.4, 70.6; 24 packed prompts of 17-2000 250.8, 256.8, 256.7, 261.6. The error of the
+// log-sum-exp against 64 bits is the same for 1/8 and 1/6 (rms 2.1-3.9e-7 over 100-4096 tokens).
+template <int D> __device__ __forceinline__ constexpr bool fma_pipe_exp(int i) { return D == 128 ? i % 6 == 5 : (i & 7) == 7; }
 
 // Extents of one sequence. Query row i sits at global position pos_off + i and sees keys
 // j < kv_len with j <= pos_off + i (bottom-right aligned for the varlen and kv-cache entry points).
@@ -1449,7 +1450,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     const int ii = (i & 15) * 2;
                     float x0, x1, e0, e1;
                     unpack2(fma2(pack2(x[ii], x[ii + 1]), scale2, neg_m2), x0, x1);
-                    if (fma_pipe_exp(i)) {
+                    if (fma_pipe_exp<D>(i)) {
                         ex2_fma2(x0, x1, e0, e1);
                     } else {
                         e0 = ex2(x0);
