@@ -217,6 +217,7 @@ Workspace decode_workspace(cudaStream_t stream, size_t bytes, size_t counter_byt
 // How the split-K kernel runs a call.
 struct RowsPlan {
     int row_blocks = 0, columns = 0, forced_units = 0;
+    int wide = 0;   // CTAs of eight warps, one to an SM
     size_t partial_bytes = 0, counter_bytes = 0, acc_bytes = 0;
 };
 

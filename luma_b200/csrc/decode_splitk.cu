@@ -35,10 +35,10 @@ namespace fa {
 
 namespace {
 
-constexpr int kWarps = 4;
-constexpr int kThreads = kWarps * 32;
+constexpr int kFour = 4;     // warps of a CTA (kWarps below)
+constexpr int kWide = 8;     // ... of a launch that has part of the SMs to itself, one CTA to each (see prepare_mixed_few_rows)
 constexpr int kTile = 16;    // tokens per tile (one mma K step for P.V, two N blocks for Q.K^T)
-constexpr int kUnit = kWarps * kTile;   // tokens that the CTA's warps take at a time, the unit of the cut
+template <int kWarps> constexpr int unit_of = kWarps * kTile;   // tokens that the CTA's warps take at a time, the unit of the cut
 constexpr int kStages = 3;   // tiles in flight per warp
 constexpr int kRows = 16;    // query rows served per CTA (M of the mma)
 
@@ -72,6 +72,7 @@ struct RowsArgs {
     int row_blocks;      // blocks of kRows query rows per KV head (blockIdx.x = KV head x row block)
     int capacity;        // keys that a sequence's row of the block table has room for; contiguous K/V: no limit
     int max_rows;        // sequences with more query rows than this (per KV head) are not this launch's
+    int ahead_of_prefill;   // launched ahead of the prefill kernel of the same call, on part of the SMs
     int behind_prefill;  // launched behind the prefill kernel of the same call, which it does not depend on
     int forced_units;    // > 0: units per column (option "decode_chunk_tokens"); 0: equal shares
     int seq_cost;        // of a sequence, in units, beside its own units (see rows_span)
@@ -151,7 +152,7 @@ __device__ __forceinline__ float fast_exp2(float x) {
 //          ldmatrix bank conflicts
 //   merge: the warps' partials of a finished sequence, up to 8 rows whole or 16 rows kMergeCols columns at a time — beside
 //          the ring, which already holds tiles of the next sequence by then
-template <int D>
+template <int D, int kWarps>
 struct Smem {
     static constexpr int kRowBytes = D * 2;
     static constexpr int kSwz = (D / 8 - 1) < 7 ? (D / 8 - 1) : 7;   // XOR mask of the 16-byte chunk index: stays inside the row
@@ -164,7 +165,8 @@ struct Smem {
     static constexpr int kMergeBytes = kWarps * kRows * kMergePitch * 4;
     static constexpr int kBytes = kRingBytes + kMergeBytes + 16;
     // CTAs per SM by shared memory (228 KiB, 1 KiB of it reserved per CTA) and registers
-    static constexpr int kCtasPerSm = D == 128 ? 2 : (D == 64 ? 3 : 4);
+    static constexpr int kCtasPerSm = kWarps == kWide ? 1 : D == 128 ? 2 : (D == 64 ? 3 : 4);
+    static_assert(kBytes <= 232448, "fits the shared memory of an SM");
 };
 
 // Extents of one sequence: its query rows and the keys it sees. Query token i sits at global position
@@ -211,7 +213,9 @@ __device__ __forceinline__ int rows_visible(const RowsSeq& r) {
 
 // Units of the sequence for the row block that starts at query row `row0`; 0: nothing to do there. A sequence
 // whose rows see no key has one unit all the same: somebody has to write its zeros.
+template <int kWarps>
 __device__ __forceinline__ int rows_units(const RowsArgs& a, const RowsSeq& r, int group, int row0) {
+    constexpr int kUnit = unit_of<kWarps>;
     const int rows = r.q_len * group;
     if (rows <= row0 || rows > a.max_rows) return 0;
     return max(1, (rows_visible(r) + kUnit - 1) / kUnit);
@@ -278,13 +282,13 @@ __device__ __forceinline__ void store_pair(const RowsOut& out, long long row, in
 // partials in flight per lane, and where a row goes is found by one lane and told to the others. With the partials asked for behind the weights, and
 // every lane finding each row's place, a merge of 13 parts of 4 rows took 2.1 us, of 2-5 parts of 16 rows 6 to 8 us, of which 0.65 and 3 to 5 behind the sums (device timer); 16 sequences
 // x 4 tokens over 512-8192 64.4 us a step, 8 x 4000 contiguous 28.7, one of 777 tokens 9.1.
-template <typename T, int D, int RW>
+template <typename T, int D, int RW, int kWarps>
 __device__ __forceinline__ void merge_parts(const RowsArgs& a, float* scratch, long long q_row0, int s, int kvh, int row0, int group, int nrows, int c_first, int parts, int warp, int lane) {
     constexpr int E = D / 32;
     constexpr int kAtOnce = 16 / RW;      // parts in flight per row
     constexpr int kChunk = 64;            // parts whose weights sit in shared memory at a time
-    static_assert(kRows / 2 * (D + 2) <= kRows * Smem<D>::kMergePitch, "half of the rows fit the merge buffer whole");
-    static_assert(kRows * kChunk * 4 <= Smem<D>::kMergeBytes, "weights of a chunk fit the merge buffer");
+    static_assert(kRows / 2 * (D + 2) <= kRows * Smem<D, kWarps>::kMergePitch, "half of the rows fit the merge buffer whole");
+    static_assert(kRows * kChunk * 4 <= Smem<D, kWarps>::kMergeBytes, "weights of a chunk fit the merge buffer");
     const unsigned grid_x = gridDim.x;
     const float* const acc0 = a.ws_acc + ((long long)blockIdx.x * (2 * kRows) + warp) * D + lane * E;   // of this warp's first row, slot 0 of column 0
     const float2* const ml0 = a.ws_ml + (long long)blockIdx.x * (2 * kRows) + warp;
@@ -423,9 +427,10 @@ __device__ __forceinline__ void merge_parts(const RowsArgs& a, float* scratch, l
 
 // kMode: the entry point. With the three of them behind branches, every place that looks at a sequence had
 // the code of all three, which a small call brings in for the first time (1 x 777 tokens 8.7 us a step, 8.3 so; 2 x 62-250, 32 heads 10.1 and 9.1).
-template <typename T, int D, int kMode>
-__global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_kernel(const __grid_constant__ RowsArgs a) {
-    using S = Smem<D>;
+template <typename T, int D, int kMode, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, Smem<D, kWarps>::kCtasPerSm) decode_splitk_kernel(const __grid_constant__ RowsArgs a) {
+    using S = Smem<D, kWarps>;
+    constexpr int kThreads = kWarps * 32, kUnit = unit_of<kWarps>;
     constexpr int kChunksPerRow = D / 8;          // 16-byte chunks per K/V row
     constexpr int kCopiesPerLane = kChunksPerRow / 2;  // a lane copies half a row of K and of V
     constexpr int kKSteps = D / 16;
@@ -444,8 +449,11 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
     // the SMs that they leave: what both read was written before the prefill kernel began. Every CTA then waits at
     // its end instead, so that this grid's completion stands for both.
     const bool behind = a.behind_prefill != 0;
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    // Ahead of a prefill kernel of the same call, which does not wait for this one but for what came before both: that has finished when it may start.
+    const bool ahead = a.ahead_of_prefill != 0;
+    if (!ahead) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     if (!behind) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    if (ahead) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 
     // KV heads vary fastest across the grid: the CTAs that read the adjacent 256-byte slices of the
     // same token rows (one slice per KV head) are launched together, which keeps DRAM pages open.
@@ -460,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
     int s = 0, cost = 0;
     unsigned u_begin, u_end;
     if (kMode == MODE_BATCH) {
-        const int units = rows_units(a, rows_seq<kMode>(a, 0), group, row0);
+        const int units = rows_units<kWarps>(a, rows_seq<kMode>(a, 0), group, row0);
         cost = rows_cost(a, (unsigned)units * (unsigned)a.num_seqs, columns);
         const unsigned per = rows_span(units, cost);
         total = per * (unsigned)a.num_seqs;
@@ -482,7 +490,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int si = s0 + lane * 4 + i;
-                mine[i] = si < a.num_seqs ? rows_units(a, rows_seq<kMode>(a, si), group, row0) : 0;
+                mine[i] = si < a.num_seqs ? rows_units<kWarps>(a, rows_seq<kMode>(a, si), group, row0) : 0;
                 lane_sum += mine[i];
                 lane_seqs += mine[i] > 0 ? 1 : 0;
             }
@@ -561,7 +569,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
     int cp_s = s;
     unsigned cp_first = seq_first;                     // unit at which sequence cp_s begins
     RowsSeq cp_seq = rows_seq<kMode>(a, s);
-    int cp_units = rows_units(a, cp_seq, group, row0);
+    int cp_units = rows_units<kWarps>(a, cp_seq, group, row0);
     int cp_vis = rows_visible(cp_seq);
     int cp_tok = (int)(u_begin - seq_first) * kUnit;   // first token of the unit to look up next
     int cp_end = (int)min((unsigned)cp_units, u_end - cp_first) * kUnit;   // tokens of it that are this CTA's
@@ -572,7 +580,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
             cp_first += rows_span(cp_units, cost);
             if (cp_first >= u_end) return;
             cp_seq = rows_seq<kMode>(a, ++cp_s);
-            cp_units = rows_units(a, cp_seq, group, row0);
+            cp_units = rows_units<kWarps>(a, cp_seq, group, row0);
             cp_vis = rows_visible(cp_seq);
             cp_tok = 0;
             cp_end = (int)min((unsigned)cp_units, u_end - cp_first) * kUnit;
@@ -635,7 +643,7 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
     unsigned u = u_begin;
     while (u < u_end) {
         const RowsSeq seq = rows_seq<kMode>(a, s);
-        const int units = rows_units(a, seq, group, row0);
+        const int units = rows_units<kWarps>(a, seq, group, row0);
         if (u >= seq_first + (unsigned)units) {   // not this launch's, or ended
             seq_first += rows_span(units, cost);
             u = max(u, seq_first);
@@ -855,9 +863,9 @@ __global__ void __launch_bounds__(kThreads, Smem<D>::kCtasPerSm) decode_splitk_k
             __syncthreads();
             if (*last_flag) {
                 const int rows_per_warp = (nrows + kWarps - 1) / kWarps;
-                if (rows_per_warp == 1) merge_parts<T, D, 1>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
-                else if (rows_per_warp == 2) merge_parts<T, D, 2>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
-                else merge_parts<T, D, 4>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
+                if (rows_per_warp == 1) merge_parts<T, D, 1, kWarps>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
+                else if (rows_per_warp == 2) merge_parts<T, D, 2, kWarps>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
+                else merge_parts<T, D, 4, kWarps>(a, merge, seq.q_row0, s, kvh, row0, group, nrows, c_first, parts, warp, lane);
                 __syncthreads();   // the merge buffer is written again by the next sequence
             }
         }
@@ -877,15 +885,18 @@ int num_columns(int per_column, int ctas_per_sm, int sms) {
 }
 
 // `rows`: query rows per KV head at most; `max_tokens`: upper bound of a sequence's visible keys.
+// `wide_sms` > 0: a launch of wide CTAs on about so many SMs.
 template <int D>
-RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, bool allow_forced) {
+RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, bool allow_forced, int wide_sms = 0) {
     RowsPlan r;
     r.row_blocks = (rows + kRows - 1) / kRows;
     const long long per_column = (long long)kv_heads * r.row_blocks;
     if (per_column > 0x7fffffffLL) return r;   // columns == 0: not this kernel's
-    r.columns = num_columns((int)per_column, Smem<D>::kCtasPerSm, sm_count());
+    const int kUnit = wide_sms > 0 ? unit_of<kWide> : unit_of<kFour>;
+    r.wide = wide_sms > 0 ? 1 : 0;
+    r.columns = r.wide ? (int)std::max(1LL, wide_sms / per_column) : num_columns((int)per_column, Smem<D, kFour>::kCtasPerSm, sm_count());
     const long long most_units = (long long)num_seqs * std::max(1LL, (max_tokens + kUnit - 1) / kUnit);
-    if (allow_forced && get_option_decode_chunk() > 0) {
+    if (!r.wide && allow_forced && get_option_decode_chunk() > 0) {
         r.forced_units = (get_option_decode_chunk() + kUnit - 1) / kUnit;
         while ((most_units + r.forced_units - 1) / r.forced_units > 4096) r.forced_units *= 2;
         r.columns = (int)((most_units + r.forced_units - 1) / r.forced_units);
@@ -900,9 +911,9 @@ RowsPlan plan_rows(int num_seqs, int kv_heads, int rows, long long max_tokens, b
 
 std::atomic<unsigned long long> g_calls{0};   // launches of this kernel, of any type and on any device
 
-template <typename T, int D, int kMode>
+template <typename T, int D, int kMode, int kWarps>
 int launch_rows_as(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
-    using S = Smem<D>;
+    using S = Smem<D, kWarps>;
     static_assert(kMaxColumns < (1 << kCountBits), "the parts of a sequence fit the count");
     a.row_blocks = plan.row_blocks;
     a.forced_units = plan.forced_units;
@@ -914,7 +925,7 @@ int launch_rows_as(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err == cudaSuccess && (dev >= 64 || !((ready.load(std::memory_order_acquire) >> dev) & 1ULL))) {
-        err = cudaFuncSetAttribute(decode_splitk_kernel<T, D, kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
+        err = cudaFuncSetAttribute(decode_splitk_kernel<T, D, kMode, kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
         if (err == cudaSuccess && dev < 64) ready.fetch_or(1ULL << dev, std::memory_order_release);
     }
     if (err != cudaSuccess) {
@@ -924,7 +935,7 @@ int launch_rows_as(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
     }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(a.kv_heads * plan.row_blocks), (unsigned)plan.columns);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(kWarps * 32);
     cfg.dynamicSmemBytes = S::kBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr{};
@@ -932,7 +943,7 @@ int launch_rows_as(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, decode_splitk_kernel<T, D, kMode>, a);
+    cudaLaunchKernelEx(&cfg, decode_splitk_kernel<T, D, kMode, kWarps>, a);
     return check_launch("decode_splitk_kernel");
 }
 
@@ -940,9 +951,11 @@ template <typename T, int D>
 int launch_rows(RowsArgs& a, const RowsPlan& plan, cudaStream_t stream) {
     a.call = (g_calls.fetch_add(1, std::memory_order_relaxed) + 1) << kCountBits;
     for (int i = 0; i < a.out.n_out; ++i) a.out.halves |= (reinterpret_cast<uintptr_t>(a.out.o[i]) & 3) != 0;
-    return a.mode == MODE_KVCACHE ? launch_rows_as<T, D, MODE_KVCACHE>(a, plan, stream)
-           : a.mode == MODE_BATCH ? launch_rows_as<T, D, MODE_BATCH>(a, plan, stream)
-                                  : launch_rows_as<T, D, MODE_VARLEN>(a, plan, stream);
+    if constexpr (D >= 64)
+        if (plan.wide) return launch_rows_as<T, D, MODE_VARLEN, kWide>(a, plan, stream);
+    return a.mode == MODE_KVCACHE ? launch_rows_as<T, D, MODE_KVCACHE, kFour>(a, plan, stream)
+           : a.mode == MODE_BATCH ? launch_rows_as<T, D, MODE_BATCH, kFour>(a, plan, stream)
+                                  : launch_rows_as<T, D, MODE_VARLEN, kFour>(a, plan, stream);
 }
 
 int log2_or_minus1(int v) {
@@ -954,12 +967,12 @@ int log2_or_minus1(int v) {
 // What can fail before anything is launched: the plan and its workspace. -1: not this kernel's; FLASH_ATTN_ERR_CUDA (no
 // message yet): no memory for it, which is a failure only where no other kernel can take the call.
 template <int D>
-int prepare_typed(const AttnParams& p, int rows, cudaStream_t stream, RowsPlan& plan, Workspace& ws) {
+int prepare_typed(const AttnParams& p, int rows, cudaStream_t stream, RowsPlan& plan, Workspace& ws, int wide_sms) {
     const long long max_tokens = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
     if (max_tokens <= 0) return -1;
     // (behind a prefill kernel, whose SMs come free one after the other, smaller shares were no faster: 4 chunks of 512 with 32
     // decoding sequences 248-252 us with one share per CTA slot, 256 with two, 253-257 with three)
-    plan = plan_rows<D>(p.num_seqs, p.kv_heads, rows, max_tokens, true);
+    plan = plan_rows<D>(p.num_seqs, p.kv_heads, rows, max_tokens, true, wide_sms);
     if (plan.columns <= 0) return -1;
     ws = decode_workspace(stream, plan.partial_bytes, plan.counter_bytes);
     return ws.partials != nullptr ? FLASH_ATTN_OK : FLASH_ATTN_ERR_CUDA;
@@ -968,7 +981,8 @@ int prepare_typed(const AttnParams& p, int rows, cudaStream_t stream, RowsPlan& 
 template <typename T, int D>
 int launch_typed(const AttnParams& p, int max_rows, bool behind_prefill, const RowsPlan& plan, const Workspace& ws, cudaStream_t stream) {
     RowsArgs a{};
-    a.behind_prefill = behind_prefill ? 1 : 0;
+    a.behind_prefill = behind_prefill && !plan.wide ? 1 : 0;
+    a.ahead_of_prefill = plan.wide;
     a.q = p.q; a.k = p.k; a.v = p.v;
     a.block_tables = p.block_tables;
     a.context_lens = p.context_lens;
@@ -1021,10 +1035,10 @@ bool rows_kernel_takes(const AttnParams& p) {
     return (reinterpret_cast<uintptr_t>(p.q) & 3) == 0;
 }
 
-int prepare_rows(const AttnParams& p, int rows, cudaStream_t stream, RowsPlan& plan, Workspace& ws) {
-    return p.head_size == 128 ? prepare_typed<128>(p, rows, stream, plan, ws)
-           : p.head_size == 64 ? prepare_typed<64>(p, rows, stream, plan, ws)
-                               : prepare_typed<32>(p, rows, stream, plan, ws);
+int prepare_rows(const AttnParams& p, int rows, cudaStream_t stream, RowsPlan& plan, Workspace& ws, int wide_sms = 0) {
+    return p.head_size == 128 ? prepare_typed<128>(p, rows, stream, plan, ws, wide_sms)
+           : p.head_size == 64 ? prepare_typed<64>(p, rows, stream, plan, ws, wide_sms)
+                               : prepare_typed<32>(p, rows, stream, plan, ws, 0);
 }
 
 int launch_prepared(const AttnParams& p, int max_rows, bool behind_prefill, const RowsPlan& plan, const Workspace& ws, cudaStream_t stream) {
@@ -1064,7 +1078,8 @@ static double prefill_us(const AttnParams& p, double pairs, double setup = 6.6) 
 // + 0.15 us a row per sequence, most of it the merge of its warps' parts; some sequence of more than one unit is always cut, and the merge of its
 // parts is another 0.6 us a row.
 static double rows_us(const AttnParams& p, long long seqs, long long rows) {
-    const long long slots = (long long)sm_count() * (p.head_size == 128 ? Smem<128>::kCtasPerSm : p.head_size == 64 ? Smem<64>::kCtasPerSm : Smem<32>::kCtasPerSm);
+    const long long slots = (long long)sm_count() * (p.head_size == 128 ? Smem<128, kFour>::kCtasPerSm : p.head_size == 64 ? Smem<64, kFour>::kCtasPerSm : Smem<32, kFour>::kCtasPerSm);
+    constexpr int kUnit = unit_of<kFour>;
     const double units = (double)((longest_keys(p) + kUnit - 1) / kUnit), nrows = (double)std::min<long long>(kRows, rows);
     const double blocks_per_slot = (double)(seqs * p.kv_heads * ((rows + kRows - 1) / kRows)) / (double)slots;
     return 4.4 + ((rows > kRows ? 0.91 : 1.04) * units + 2.2 + 0.15 * nrows) * blocks_per_slot + (units > 1.0 ? 0.6 * nrows : 0.0);
@@ -1129,6 +1144,30 @@ static bool mixed_few_rows_are_better(const AttnParams& p) {
     return prefill_us(p, prompts + few, 14.0) > 1.15 * (prefill_us(p, prompts, 14.0) + rows_us(p, m.few, p.q_heads / p.kv_heads));
 }
 
+// A mixed batch's two kernels side by side: the few-row kernel first, in CTAs of eight warps on part of the SMs, the prefill kernel behind it without waiting, on the others and then on all. How
+// many SMs, and whether at all (0: behind, on all of them), by estimates from what the host knows: tile pairs of 6.6 us and 1.5 us per 128 keys; a wide CTA reads 50 GB/s (each warp's chain of products and
+// exponentials), all SMs 6.3 TB/s. One after the other the two leave the memory idle, then the tensor cores. us behind and ahead: 4 chunks of 512 with 32 tokens over 512-8192, 32/8 heads 220 and
+// 210; 2 x 512 with 8 over 512-8192 141 and 117; 2 x 300 with 64 over 300-4800 174 and 150; one of 67 with 15 over 338-5418, 64/8 heads 113 and 80; one of 329 with 72 over 162-2593, 8/2 heads 73 and 47; one
+// of 113 with 19 over 15-240, 32 heads of 64 28 and 21. On fewer SMs than the estimate says the few rows come last and alone (the first with 40 instead of 64 254). Over the shortest contexts the launch
+// that has to come first costs more than it wins (5 of up to 83 with 13 over 5-83, 32/8 heads 16 and 26; 4 of up to 169 with 9 over 10-169 19 and 22).
+static int wide_sms(const AttnParams& p) {
+    if (p.head_size < 64 || p.total_q <= 0 || longest_keys(p) < 192) return 0;
+    const PackedMix m = packed_mix(p);
+    const double keys = (double)longest_keys(p), sms = sm_count();
+    const double pair = 6.6 + 1.5 * std::ceil(keys / 128.0), pairs = (double)m.prompts * (double)prefill_pairs(p.q_heads / p.kv_heads, p.q_seq_len) * p.kv_heads;
+    const double bytes = (double)m.few * keys * p.kv_heads * p.head_size * 4.0, rate = 50e3 * p.head_size / 128.0;   // bytes, and bytes per us of a wide CTA
+    double best = 1.02 * (std::max(1.0, pairs / sms) * pair + bytes / 6.3e6);
+    int n = 0;
+    for (int k = p.kv_heads; k <= 2 * (int)sms / 3; k += p.kv_heads) {
+        const double few = bytes / std::min(k * rate, 6.3e6), all = std::max(std::max(few, pair), (pairs * pair + k * few) / sms);
+        if (all < best) {
+            best = all;
+            n = k;
+        }
+    }
+    return n;
+}
+
 MixedFewRows prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {
     MixedFewRows few;
     if (p.mode != MODE_VARLEN || p.num_seqs < 2 || p.n_out > 0 || !rows_kernel_takes(p)) return few;
@@ -1136,7 +1175,7 @@ MixedFewRows prepare_mixed_few_rows(const AttnParams& p, cudaStream_t stream) {
     // one row block: the CTA slots are shared out before anybody knows how many rows the sequences have
     // prompts packed back to back with their own K/V: few rows would see few keys
     if (group > kRows || (!p.paged && p.kv_seq_len <= p.q_seq_len) || !mixed_few_rows_are_better(p)) return few;
-    if (prepare_rows(p, kRows, stream, few.plan, few.ws) == FLASH_ATTN_OK) few.max_rows = kRows;
+    if (prepare_rows(p, kRows, stream, few.plan, few.ws, wide_sms(p)) == FLASH_ATTN_OK) few.max_rows = kRows;
     return few;
 }
 

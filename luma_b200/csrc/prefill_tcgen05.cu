@@ -186,6 +186,7 @@ struct PrefillArgs {
     const int* block_tables;    // paged K/V: (batch, max_blocks) logical -> physical block
     int paged, block_size, max_blocks;
     int q_bounded, kv_bounded;  // MODE_VARLEN: the caller gave the packed buffers' rows, their tensor maps end there
+    int behind_few;             // the few-row kernel was launched ahead: this one does not wait for it, but ends behind it
     int skip_rows;              // MODE_VARLEN: sequences of at most this many (query token, group head) rows are not this launch's; 0: none
     float scale_log2;
 };
@@ -987,7 +988,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // (the same for the whole warp, which the compiler sees only so)
     const int lane = threadIdx.x & 31;
     // A few-row kernel launched behind this one may start once every tile pair here is taken: it fills the SMs that run out of them.
-    if (a.skip_rows > 0) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    if (a.skip_rows > 0 && !a.behind_few) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     // Packed buffers end at row cu_seqlens[num_seqs]; where the tensor map does not end with the buffer, a tile that reaches past that row is not asked
     // of the copy engine but fetched by the producer warp (see edge_tile_copy). A map that does gives zeros there like any other.
     const bool packed = a.mode == MODE_VARLEN;
@@ -1652,6 +1653,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 
     tc_fence_before();
     __syncthreads();
+    if (a.behind_few && threadIdx.x == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");   // (this grid's completion stands for both)
     if (warp == kMmaWarp) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(sm.tmem_base) : "memory");
@@ -1990,7 +1992,7 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
         return rc;
     }
     constexpr bool kOneWave = D == 128 || kPaged;
-    const bool one_pair = kOneWave && ((long long)grid.x * grid.y * grid.z <= sm_count() || (D == 128 && a.ordered && a.skip_rows == 0));
+    const bool one_pair = kOneWave && !(few.plan.wide && a.skip_rows > 0) && ((long long)grid.x * grid.y * grid.z <= sm_count() || (D == 128 && a.ordered && a.skip_rows == 0));
     const auto kernel = one_pair ? prefill_tcgen05_kernel<T, D, kMask, kPaged, kOneWave, false> : prefill_tcgen05_kernel<T, D, kMask, kPaged, false, false>;
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) {
@@ -1998,9 +2000,22 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
         cudaGetLastError();
         return FLASH_ATTN_ERR_CUDA;
     }
-    kernel<<<grid, kThreads, smem, stream>>>(qm, km, vm, om, a);
-    int rc = check_launch("prefill_tcgen05_kernel");
-    if (rc == FLASH_ATTN_OK && a.skip_rows > 0) rc = launch_mixed_few_rows(p, few, stream);
+    a.behind_few = a.skip_rows > 0 && few.plan.wide;
+    int rc = a.behind_few ? launch_mixed_few_rows(p, few, stream) : FLASH_ATTN_OK;
+    if (rc != FLASH_ATTN_OK) return rc;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = a.behind_few ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, qm, km, vm, om, a);
+    rc = check_launch("prefill_tcgen05_kernel");
+    if (rc == FLASH_ATTN_OK && a.skip_rows > 0 && !a.behind_few) rc = launch_mixed_few_rows(p, few, stream);
     if (rc == FLASH_ATTN_OK) note_path("prefill_tcgen05", a.skip_rows > 0 ? 2 : 1);
     return rc;
 }
