@@ -1152,7 +1152,7 @@ static bool mixed_few_rows_are_better(const AttnParams& p) {
 // 15-240, 32 heads of 64 24.6 and 22.8; estimated well above a fifth, and left: 5 of 72 with 43 over 113-1822, 32 heads of 64 102 (122-173 beside). Over the shortest contexts the launch that has to
 // come first costs more than it wins (5 of up to 83 with 13 over 5-83, 32/8 heads from a graph 16 and 26; 4 of up to 169 with 9 over 10-169 19 and 22).
 static int wide_sms(const AttnParams& p) {
-    if (p.head_size < 64 || p.total_q <= 0 || longest_keys(p) < 192) return 0;
+    if (p.head_size < 64 || p.total_q <= 0 || longest_keys(p) < 192 || get_option_decode_chunk() > 0) return 0;
     const PackedMix m = packed_mix(p);
     const double keys = (double)longest_keys(p), sms = sm_count();
     const double pair = 6.6 + 1.5 * std::ceil(keys / 128.0), pairs = (double)m.prompts * (double)prefill_pairs(p.q_heads / p.kv_heads, p.q_seq_len) * p.kv_heads;
