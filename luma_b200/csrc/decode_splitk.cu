@@ -1146,21 +1146,24 @@ static bool mixed_few_rows_are_better(const AttnParams& p) {
 
 // A mixed batch's two kernels side by side: the few-row kernel first, in CTAs of eight warps on part of the SMs, the prefill kernel behind it without waiting, on the others and then on all. How
 // many SMs, and whether at all (0: behind, on all of them), by estimates from what the host knows: tile pairs of 6.6 us and 1.5 us per 128 keys; a wide CTA reads 42 GB/s (each warp's chain of products and
-// exponentials), all SMs 6.3 TB/s. One after the other the two leave the memory idle, then the tensor cores, and a last wave half empty, so that side by side is the faster up to an
+// exponentials) and takes 2 us for the end of each sequence, all SMs read 6.3 TB/s. One after the other the two leave the memory idle, then the tensor cores, and a last wave half empty, so that side by side is the faster up to an
 // estimate a fifth above. us a pass, behind and beside: 4 chunks of 512 with 32 tokens over 512-8192, 32/8 heads 236.6 and 231.9 (on 80 SMs; 72 238, 56 244, 48 260, 96 250); 2 of 512 with 8 over
 // 512-8192 139 and 116; 2 of 300 with 64 over 300-4800 173 and 161; one of 67 with 15 over 338-5418, 64/8 heads 118 and 79; one of 329 with 72 over 162-2593, 8/2 heads 76 and 46; one of 113 with 19 over
 // 15-240, 32 heads of 64 24.6 and 22.8; estimated well above a fifth, and left: 5 of 72 with 43 over 113-1822, 32 heads of 64 102 (122-173 beside). Over the shortest contexts the launch that has to
-// come first costs more than it wins (5 of up to 83 with 13 over 5-83, 32/8 heads from a graph 16 and 26; 4 of up to 169 with 9 over 10-169 19 and 22).
+// come first costs more than it wins (5 of up to 83 with 13 over 5-83, 32/8 heads from a graph 16 and 26; 4 of up to 169 with 9 over 10-169 19 and 22). Short sequences over many KV heads are ends above
+// all: 3 of up to 200 with 40 over 12-200, 32/32 heads 37 behind, 49 beside on the SMs that the rate alone would give, 39 so; one of 128 with 16 over 16-260, 32/8 heads of 64 15.7, 18.6, 14.1. 160 mixes of
+// contexts up to 200-900, from a graph: 0.949 of behind on average, 0.957 without the ends, 0.960 with 3 us; the slowest against behind 1.07, 1.33 and 1.06.
 static int wide_sms(const AttnParams& p) {
     if (p.head_size < 64 || p.total_q <= 0 || longest_keys(p) < 192 || get_option_decode_chunk() > 0) return 0;
     const PackedMix m = packed_mix(p);
     const double keys = (double)longest_keys(p), sms = sm_count();
     const double pair = 6.6 + 1.5 * std::ceil(keys / 128.0), pairs = (double)m.prompts * (double)prefill_pairs(p.q_heads / p.kv_heads, p.q_seq_len) * p.kv_heads;
     const double bytes = (double)m.few * keys * p.kv_heads * p.head_size * 4.0, rate = 42e3 * p.head_size / 128.0;   // bytes, and bytes per us of a wide CTA
-    double best = 1.2 * (std::max(1.0, pairs / sms) * pair + bytes / 6.3e6);
+    const double ends = 2.0 * m.few * p.kv_heads;   // us of a CTA
+    double best = 1.2 * (std::max(1.0, pairs / sms) * pair + bytes / 6.3e6 + ends / (2 * sms));
     int n = 0;
     for (int k = p.kv_heads; k <= 2 * (int)sms / 3; k += p.kv_heads) {
-        const double few = bytes / std::min(k * rate, 6.3e6), all = std::max(std::max(few, pair), (pairs * pair + k * few) / sms);
+        const double few = bytes / std::min(k * rate, 6.3e6) + ends / k, all = std::max(std::max(few, pair), (pairs * pair + k * few) / sms);
         if (all < best) {
             best = all;
             n = k;

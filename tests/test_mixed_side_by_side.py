@@ -30,6 +30,7 @@ def _batch(seed, decoding, prompts, longest, hq, hkv, d, dt, page=16, several=Fa
 
 @pytest.mark.parametrize("decoding,prompts,longest,hq,hkv,d,dt,several", [
     (200, 1, 1500, 8, 2, 128, "bf16", False), (200, 1, 1500, 8, 2, 128, "f16", True), (80, 2, 1300, 8, 2, 64, "bf16", False), (120, 3, 1100, 8, 8, 128, "bf16", True), (300, 2, 700, 8, 2, 128, "f16", False),
+    (40, 3, 200, 32, 32, 128, "bf16", False), (16, 1, 260, 32, 8, 64, "bf16", False),   # the ends of short sequences: fewer or more SMs than the keys alone ask for
 ])
 def test_rows_of_both_kernels(decoding, prompts, longest, hq, hkv, d, dt, several):
     dev, o, args, want = _batch(decoding, decoding, prompts, longest, hq, hkv, d, dt, several=several)
