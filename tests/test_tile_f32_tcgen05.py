@@ -31,6 +31,7 @@ def _close(o, want, what):
     (1, 5, 1025, 2, 2, 64, 1020), (1, 1, 4000, 4, 1, 128, 3999), (1, 3, 449, 1, 1, 32, 446),  # few rows over many keys
     (1, 43, 300, 9, 3, 64, 257), (1, 64, 257, 4, 2, 64, 193),                                # 129 and 128 rows
     (1, 300, 200, 4, 2, 64, 0), (1, 200, 300, 6, 2, 128, 0),                                  # more tokens than keys, and keys that nobody sees
+    (3, 160, 160, 8, 8, 32, 0), (4, 96, 96, 16, 4, 32, 0), (4, 128, 128, 8, 8, 32, 0),          # both sides of the line to the warp-wide products
     (4, 400, 400, 16, 8, 64, 0), (2, 513, 513, 24, 24, 32, 0), (3, 330, 330, 12, 12, 128, 0),  # a CTA to a block
 ])
 def test_batched_with_lse(b, sq, skv, hq, hkv, d, sp):
