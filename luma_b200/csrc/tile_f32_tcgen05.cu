@@ -30,6 +30,9 @@ constexpr int kThreads = kWorkers + 32;     // and the warp that issues the prod
 constexpr int kM = 128;                     // rows of a CTA: query token x head of the GQA group
 constexpr int kN = 64;                      // keys of a tile
 constexpr int kBlock = kN * 128;            // bytes of 64 rows of 64 columns of one term
+// A row's maxima by the tile's parity: behind the barrier of its rows' warps (tile j) a warp may run on and write the next tile's maximum, while another has not yet read this one's (nothing
+// else that it waits for needs that read). It writes into the same half again behind the barrier of tile j + 1, which the other reaches after its reads of tile j.
+constexpr int kMaxBuffers = 2;
 
 // A product of three terms by three, without the three products below 2^-24, is one matrix instruction for each term of A, on neighbouring blocks of B: A's leading term times
 // B's (leading, middle, last) adds into the sums of (order 0, 1, 2), its middle term times (leading, middle) into (1, 2), its last term
@@ -42,7 +45,7 @@ struct Plan {
     static constexpr int kQHalf = kM * 128, kQPlane = kHalves * kQHalf;
     // K: by half and term (the three terms of 64 columns are neighbouring rows), V: by term and half (neighbouring columns)
     static constexpr int kK = 3 * kQPlane, kV = kK + 3 * kHalves * kBlock, kRed = kV + 3 * kHalves * kBlock;
-    static constexpr int kVis = kRed + kShares * kM * 4, kMl = kVis + 2 * kN, kAt = kMl + kM * 8, kBar = kAt + kM * 8, kBytes = kBar + 80 + 1024;   // (1024: the planes are aligned to that)
+    static constexpr int kVis = kRed + kMaxBuffers * kShares * kM * 4, kMl = kVis + 2 * kN, kAt = kMl + kM * 8, kBar = kAt + kM * 8, kBytes = kBar + 80 + 1024;   // (1024: the planes are aligned to that)
     // Tensor memory: the scores' three orders, the weights' three terms, O's orders. At head size 128 the weights lie over the scores, and O's small orders share a sum.
     static constexpr bool kOver = D == 128;
     static constexpr int kP = kOver ? 0 : 3 * kN, kO = kOver ? 3 * kN : 3 * kN + 3 * kN / 2, kOrders = kOver ? 2 : 3;
@@ -396,9 +399,10 @@ __global__ void __launch_bounds__(kThreads, 1) tile_f32_tcgen05_kernel(const __g
 #pragma unroll
             for (int i = 0; i < kKeys; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], sc[i]);
             float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            red[part][r] = mx;
+            float(*const maxima)[kM] = red + (j & 1) * kShares;
+            maxima[part][r] = mx;
             asm volatile("barrier.cta.sync %0, 128;\n" ::"r"(1 + quad) : "memory");   // the warps of these rows (which have read their scores)
-            mx = fmaxf(fmaxf(red[0][r], red[1][r]), fmaxf(red[2][r], red[3][r]));
+            mx = fmaxf(fmaxf(maxima[0][r], maxima[1][r]), fmaxf(maxima[2][r], maxima[3][r]));
             const float before = u, by = alpha;
             u = mx == -INFINITY ? 0.0f : __fmul_rn(mx, scale);
             alpha = m == -INFINITY ? 0.0f : ex2(before - u);   // 1 exactly while the maximum stays
