@@ -33,6 +33,9 @@ constexpr int kBlock = kN * 128;            // bytes of 64 rows of 64 columns of
 // A row's maxima by the tile's parity: behind the barrier of its rows' warps (tile j) a warp may run on and write the next tile's maximum, while another has not yet read this one's (nothing
 // else that it waits for needs that read). It writes into the same half again behind the barrier of tile j + 1, which the other reaches after its reads of tile j.
 constexpr int kMaxBuffers = 2;
+// Tiles of mask bytes: the two warps that bring tile j + 1 are behind the scores of tile j, that is behind what every warp did before it gave K of tile j. Warps of another quad may then still read
+// the mask of tile j - 1 (at head sizes 32 and 64), not that of tile j - 2. Four and not three: the index is a mask.
+constexpr int kMaskBuffers = 4;
 
 // A product of three terms by three, without the three products below 2^-24, is one matrix instruction for each term of A, on neighbouring blocks of B: A's leading term times
 // B's (leading, middle, last) adds into the sums of (order 0, 1, 2), its middle term times (leading, middle) into (1, 2), its last term
@@ -45,7 +48,7 @@ struct Plan {
     static constexpr int kQHalf = kM * 128, kQPlane = kHalves * kQHalf;
     // K: by half and term (the three terms of 64 columns are neighbouring rows), V: by term and half (neighbouring columns)
     static constexpr int kK = 3 * kQPlane, kV = kK + 3 * kHalves * kBlock, kRed = kV + 3 * kHalves * kBlock;
-    static constexpr int kVis = kRed + kMaxBuffers * kShares * kM * 4, kMl = kVis + 2 * kN, kAt = kMl + kM * 8, kBar = kAt + kM * 8, kBytes = kBar + 80 + 1024;   // (1024: the planes are aligned to that)
+    static constexpr int kVis = kRed + kMaxBuffers * kShares * kM * 4, kMl = kVis + kMaskBuffers * kN, kAt = kMl + kM * 8, kBar = kAt + kM * 8, kBytes = kBar + 80 + 1024;   // (1024: the planes are aligned to that)
     // Tensor memory: the scores' three orders, the weights' three terms, O's orders. At head size 128 the weights lie over the scores, and O's small orders share a sum.
     static constexpr bool kOver = D == 128;
     static constexpr int kP = kOver ? 0 : 3 * kN, kO = kOver ? 3 * kN : 3 * kN + 3 * kN / 2, kOrders = kOver ? 2 : 3;
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_f32_tcgen05_kernel(const __g
             for (int i = 0; i < kLoads; ++i) put(base + S::kV + half_of * kBlock, S::kHalves * kBlock, at_row + i * kStep, x[i]);
         };
         auto put_vis = [&](int tile) {
-            if (mask_row != nullptr && tid < kN) vis[(tile & 1) * kN + tid] = tile * kN + tid < kv_end ? mask_row[tile * kN + tid] : 0;
+            if (mask_row != nullptr && tid < kN) vis[(tile & (kMaskBuffers - 1)) * kN + tid] = tile * kN + tid < kv_end ? mask_row[tile * kN + tid] : 0;
         };
         auto tell = [&](unsigned long long* bar) {   // what this warp has done before is seen by the issuer and the products
             __syncwarp();
@@ -393,7 +396,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_f32_tcgen05_kernel(const __g
             if (tile * kN + kN > all_see || mask_row != nullptr) {
 #pragma unroll
                 for (int i = 0; i < kKeys; ++i)
-                    if (key0 + i > lim || (mask_row != nullptr && vis[(tile & 1) * kN + part * kKeys + i] == 0)) sc[i] = -INFINITY;
+                    if (key0 + i > lim || (mask_row != nullptr && vis[(tile & (kMaskBuffers - 1)) * kN + part * kKeys + i] == 0)) sc[i] = -INFINITY;
             }
             float mx4[4] = {m, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll

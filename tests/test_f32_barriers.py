@@ -12,8 +12,10 @@ import pytest
 SOURCE = (Path(__file__).resolve().parent.parent / "luma_b200" / "csrc" / "tile_f32_tcgen05.cu").read_text()
 QUADS, PARTS = 3, 2
 WARPS = QUADS * PARTS
+WRITERS = 2
 MISTAKES = {
     "one buffer for the maxima": "a warp of the quad runs on and writes the next tile's maximum where another has not read this one's",
+    "two buffers for the mask": "the warps that bring the next tile's mask are behind what others did two tiles ago only",
     "a tile's K before its scores are there": "the planes are written again under the product that reads them",
 }
 
@@ -48,6 +50,8 @@ class Cta:
         self.quad_at = [0] * WARPS                       # barriers of its quad that a warp has come to
         self.k, self.v = [None] * WARPS, [None] * WARPS  # the tile whose rows a warp has laid down
         self.red = [[[None] * PARTS for _ in range(QUADS)] for _ in range(self.reds)]
+        self.masks = 2 if mistake == "two buffers for the mask" else _buffers("kMaskBuffers")
+        self.vis = [[None] * WRITERS for _ in range(self.masks)]
         self.s = None                                    # scores in tensor memory: tile
         self.s_read = [None] * WARPS
         self.p = [None] * WARPS                          # weights
@@ -135,6 +139,8 @@ class Cta:
     def worker(self, w):
         quad, part = w % QUADS, w // QUADS
         self.k[w] = 0
+        if w < WRITERS:
+            self.vis[0][w] = 0
         yield
         self.k_ready.arrive()
         for j in range(self.n):
@@ -149,10 +155,15 @@ class Cta:
                 self.s_free.arrive()
             yield
             if j + 1 < self.n:
+                if w < WRITERS:
+                    self.vis[(j + 1) % self.masks][w] = j + 1
                 self.k[w] = j + 1
                 yield
                 self.k_ready.arrive()
             yield
+            self.check(self.vis[j % self.masks] == [j] * WRITERS, "mask", j, self.vis)
+            yield
+            self.check(self.vis[j % self.masks] == [j] * WRITERS, "mask", j, self.vis)
             red = self.red[j % self.reds][quad]
             red[part] = j
             yield from self.quad_barrier(w)
