@@ -405,6 +405,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_f32_tcgen05_kernel(const __g
             float(*const maxima)[kM] = red + (j & 1) * kShares;
             maxima[part][r] = mx;
             asm volatile("barrier.cta.sync %0, 128;\n" ::"r"(1 + quad) : "memory");   // the warps of these rows (which have read their scores)
+            if (S::kOver) tc_fence_after();   // their loads come before this warp's weights, which go where the scores lie (tile 0 has no other fence until then)
             mx = fmaxf(fmaxf(maxima[0][r], maxima[1][r]), fmaxf(maxima[2][r], maxima[3][r]));
             const float before = u, by = alpha;
             u = mx == -INFINITY ? 0.0f : __fmul_rn(mx, scale);

@@ -224,3 +224,11 @@ def test_the_model_finds_a_planted_mistake(mistake):
             if found == 3:
                 return
     raise AssertionError(f"{mistake}: {MISTAKES[mistake]}: found {found} times")
+
+
+def test_weights_over_scores_are_stored_behind_a_fence():
+    """At head size 128 a warp's weights go over the scores that the other warps of its rows have loaded: loads, tcgen05.fence::before_thread_sync, barrier,
+    tcgen05.fence::after_thread_sync, stores, in the first tile as well (the later ones have the fence of their wait for O besides)."""
+    loop = SOURCE[SOURCE.index("wait_warp(s_full, phase, 70);"):SOURCE.index("tell(pv_ready);")]
+    at = [loop.index(x) for x in ("tc_ld16(mine + part * kKeys, sc);", "tc_fence_before();", "barrier.cta.sync %0, 128;", "if (S::kOver) tc_fence_after();", "if (j > 0) {", "tc_st8(")]
+    assert at == sorted(at)
