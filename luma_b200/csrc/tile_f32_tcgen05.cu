@@ -37,10 +37,12 @@ constexpr int kMaxBuffers = 2;
 // the mask of tile j - 1 (at head sizes 32 and 64), not that of tile j - 2. Four and not three: the index is a mask.
 constexpr int kMaskBuffers = 4;
 
-// A product of three terms by three, without the three products below 2^-24, is one matrix instruction for each term of A, on neighbouring blocks of B: A's leading term times
-// B's (leading, middle, last) adds into the sums of (order 0, 1, 2), its middle term times (leading, middle) into (1, 2), its last term
-// times the leading one into (2). The sums of an order stay apart, and are added in f32 when they are read, the smallest first. Half as many instructions as one for each of the
-// six products, which took the issuing warp longer than the tensor cores.
+// A product of three terms by three, without the three products below 2^-24, is six matrix products, into sums by their order (0: leading times leading; 1: leading times middle; 2: the others),
+// which are added in f32 when they are read, the smallest first. Products are promised to add in the order of their issue where accumulator and shape are the same (PTX ISA, pipelined
+// tcgen05 instructions), so no two of them that differ in shape share a column. The scores' leading term times K's leading and middle one is one product of both sums; the other four
+// go to the third, with the middle term times the leading one, which belongs to order 1: what the tensor cores cut off there is 2^-8 of what they cut off in order 0. One instruction for each term
+// of A on neighbouring blocks of B, in shapes of 192, 128 and 64 columns that overlapped, had a quarter less to read from shared memory, and no promise (us from a graph, so and now: 1 x 256, 8 heads of 64 9.31 and 9.42;
+// 2 x 979 37.7 and 36.4; 4 x 1000, 8 of 32 46.4 and 47.0; 1 x 1024, 16/4 of 128 101.3 and 103.9; six products of one shape for the scores 9.5, 36.6, 47.1, 106.1).
 template <int D>
 struct Plan {
     static constexpr int kHalves = D == 128 ? 2 : 1;               // blocks of 64 columns (head size 32: half of one, zeros behind)
@@ -49,7 +51,7 @@ struct Plan {
     // K: by half and term (the three terms of 64 columns are neighbouring rows), V: by term and half (neighbouring columns)
     static constexpr int kK = 3 * kQPlane, kV = kK + 3 * kHalves * kBlock, kRed = kV + 3 * kHalves * kBlock;
     static constexpr int kVis = kRed + kMaxBuffers * kShares * kM * 4, kMl = kVis + kMaskBuffers * kN, kAt = kMl + kM * 8, kBar = kAt + kM * 8, kBytes = kBar + 80 + 1024;   // (1024: the planes are aligned to that)
-    // Tensor memory: the scores' three orders, the weights' three terms, O's orders. At head size 128 the weights lie over the scores, and O's small orders share a sum.
+    // Tensor memory: the scores' three sums, the weights' three terms, O's sums. At head size 128 the weights lie over the scores, and O's small orders share one.
     static constexpr bool kOver = D == 128;
     static constexpr int kP = kOver ? 0 : 3 * kN, kO = kOver ? 3 * kN : 3 * kN + 3 * kN / 2, kOrders = kOver ? 2 : 3;
     static_assert(kO + kOrders * kCols <= 512, "fits tensor memory");
@@ -107,6 +109,52 @@ __device__ __forceinline__ void cluster_sync() {
 __device__ __forceinline__ float quotient(float x, float y, float inv) {
     const float q = x * inv;
     return fmaf(fmaf(-q, y, x), inv, q);
+}
+
+__device__ __forceinline__ void commit(unsigned long long* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// The issuer's products, in functions of their own: unrolled among the workers' code their descriptors cost everybody registers (head size 128: 1164 bytes of spill stores, 916 rolled up, 840 so).
+template <int D>
+__device__ __noinline__ void issue_scores(unsigned tmem, unsigned long long dq, unsigned long long dk, unsigned long long* s_full) {
+    using S = Plan<D>;
+    const unsigned x = tmem, z = tmem + 2 * kN;
+    tc_fence_after();
+    if (elect_one()) {
+#pragma unroll
+        for (int t = 0; t < 3; ++t)
+#pragma unroll
+            for (int kk = 0; kk < D / 16; ++kk) {
+                const unsigned long long q = dq + ((t * S::kQPlane + (kk >> 2) * S::kQHalf + (kk & 3) * 32) >> 4), k = dk + (((kk >> 2) * 3 * kBlock + (kk & 3) * 32) >> 4);
+                if (t == 0) tc_mma_ss(x, q, k, make_idesc<__nv_bfloat16>(false, 2 * kN), kk > 0);
+#pragma unroll
+                for (int u = t == 0 ? 2 : 0; t + u < 3; ++u) tc_mma_ss(z, q, k + (u * kBlock >> 4), make_idesc<__nv_bfloat16>(false, kN), t + kk > 0);
+            }
+        commit(s_full);
+    }
+    __syncwarp();
+}
+template <int D>
+__device__ __noinline__ void issue_sums(unsigned tmem, unsigned long long dv, unsigned long long* o_full) {
+    using S = Plan<D>;
+    const unsigned o0 = tmem + S::kO, o1 = tmem + S::kO + S::kCols, o2 = tmem + S::kO + (S::kOrders - 1) * S::kCols;
+    tc_fence_after();
+    if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            const unsigned p = tmem + S::kP + kk * 8, p1 = p + kN / 2, p2 = p + kN;
+            const unsigned long long v = dv + (kk * 2048 >> 4), v1 = v + (S::kHalves * kBlock >> 4), v2 = v + (2 * S::kHalves * kBlock >> 4);
+            tc_mma_ts(o0, p, v, make_idesc<__nv_bfloat16>(true, S::kCols), kk > 0);
+            tc_mma_ts(o1, p, v1, make_idesc<__nv_bfloat16>(true, S::kCols), kk > 0);
+            tc_mma_ts(o1, p1, v, make_idesc<__nv_bfloat16>(true, S::kCols), true);
+            tc_mma_ts(o2, p, v2, make_idesc<__nv_bfloat16>(true, S::kCols), kk > 0 || S::kOrders == 2);
+            tc_mma_ts(o2, p1, v1, make_idesc<__nv_bfloat16>(true, S::kCols), true);
+            tc_mma_ts(o2, p2, v, make_idesc<__nv_bfloat16>(true, S::kCols), true);
+        }
+        commit(o_full);
+    }
+    __syncwarp();
 }
 
 // kPlain: contiguous K/V and no key-padding mask (look-ups and mask in the loop cost it registers and a tenth of its instructions).
@@ -169,9 +217,6 @@ __global__ void __launch_bounds__(kThreads, 1) tile_f32_tcgen05_kernel(const __g
         }
         return true;
     };
-    auto commit = [&](unsigned long long* bar) {
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-    };
 
     float acc[kOut], m = -INFINITY, l = 0.0f;   // of this thread's row: its columns of O, the maximum of the raw scores so far, the sum over its keys
     float u = 0.0f;                             // the reference: that maximum, scaled and rounded (0 until a key has been seen)
@@ -201,45 +246,8 @@ __global__ void __launch_bounds__(kThreads, 1) tile_f32_tcgen05_kernel(const __g
         tc_fence_after();
         const unsigned tmem = __shfl_sync(0xffffffffu, *tmem_base, 0), base = __shfl_sync(0xffffffffu, smem_u32(sm), 0);
         const unsigned long long dq = make_desc(base, 16, 1024), dk = make_desc(base + S::kK, 16, 1024), dv = make_desc(base + S::kV, kBlock, 1024);
-        auto scores = [&]() {
-            tc_fence_after();
-            if (elect_one()) {
-#pragma unroll
-                for (int t = 0; t < 3; ++t)
-#pragma unroll
-                    for (int kk = 0; kk < D / 16; ++kk)
-                        tc_mma_ss(tmem + t * kN, dq + ((t * S::kQPlane + (kk >> 2) * S::kQHalf + (kk & 3) * 32) >> 4), dk + (((kk >> 2) * 3 * kBlock + (kk & 3) * 32) >> 4),
-                                  make_idesc<__nv_bfloat16>(false, (3 - t) * kN), t + kk > 0);
-                commit(s_full);
-            }
-            __syncwarp();
-        };
-        auto sums = [&]() {
-            tc_fence_after();
-            if (elect_one()) {
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk) {
-                    const unsigned at = tmem + S::kP + kk * 8;
-                    const unsigned long long v = dv + kk * (2048 >> 4);
-                    if (S::kOrders == 3) {
-#pragma unroll
-                        for (int t = 0; t < 3; ++t)
-                            tc_mma_ts(tmem + S::kO + t * S::kCols, at + t * (kN / 2), v, make_idesc<__nv_bfloat16>(true, (3 - t) * S::kCols), t + kk > 0);
-                    } else {
-                        constexpr unsigned long long kTerm = (unsigned long long)(S::kHalves * kBlock) >> 4;
-                        const unsigned one = make_idesc<__nv_bfloat16>(true, S::kCols);
-                        const unsigned o1 = tmem + S::kO + S::kCols;
-                        tc_mma_ts(tmem + S::kO, at, v, make_idesc<__nv_bfloat16>(true, 2 * S::kCols), kk > 0);
-                        tc_mma_ts(o1, at + kN / 2, v, one, true);
-                        tc_mma_ts(o1, at, v + 2 * kTerm, one, true);
-                        tc_mma_ts(o1, at + kN / 2, v + kTerm, one, true);
-                        tc_mma_ts(o1, at + kN, v, one, true);
-                    }
-                }
-                commit(o_full);
-            }
-            __syncwarp();
-        };
+        auto scores = [&]() { issue_scores<D>(tmem, dq, dk, s_full); };
+        auto sums = [&]() { issue_sums<D>(tmem, dv, o_full); };
         bool alive = n == 0 || __all_sync(0xffffffffu, wait(k_ready, 0u, 60));
         if (alive && n > 0) scores();
 #pragma unroll 1

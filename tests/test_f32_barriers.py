@@ -232,3 +232,28 @@ def test_weights_over_scores_are_stored_behind_a_fence():
     loop = SOURCE[SOURCE.index("wait_warp(s_full, phase, 70);"):SOURCE.index("tell(pv_ready);")]
     at = [loop.index(x) for x in ("tc_ld16(mine + part * kKeys, sc);", "tc_fence_before();", "barrier.cta.sync %0, 128;", "if (S::kOver) tc_fence_after();", "if (j > 0) {", "tc_st8(")]
     assert at == sorted(at)
+
+
+@pytest.mark.parametrize("d", [32, 64, 128])
+def test_products_that_share_columns_have_the_same_accumulator_and_shape(d):
+    """The order of issue is promised for products of one accumulator and shape only. From the source: first column and columns of every product, for each head size."""
+    plan = SOURCE[SOURCE.index("struct Plan {"):]
+    plan = plan[:plan.index("};")]
+    env = dict(D=d, kN=64, kM=128, tmem=0)
+    for name, value in re.findall(r"(k[A-Z]\w*) = ([^,;]+)[,;]", plan):
+        value = re.sub(r"(.+) \? (.+) : (.+)", r"(\2) if (\1) else (\3)", value.replace("/", "//"))
+        if name in ("kHalves", "kCols", "kOver", "kP", "kO", "kOrders"):
+            env[name] = eval(value, {}, env)
+    found = 0
+    for function in ("issue_scores", "issue_sums"):
+        body = SOURCE[SOURCE.index(f"__noinline__ void {function}("):]
+        body = body[:body.index("__syncwarp();")].replace("S::", "")
+        places = dict(re.findall(r"(\w+) = (tmem[^,;]*)[,;]", body))
+        shapes = set()
+        for to, columns in re.findall(r"tc_mma_[st]s\((\w+), .*?make_idesc<__nv_bfloat16>\(\w+, ([^)]*)\)", body):
+            shapes.add((eval(places[to], {}, env), eval(columns, {}, env)))
+            found += 1
+        shapes = sorted(shapes)
+        assert all(a + n <= b for (a, n), (b, _) in zip(shapes, shapes[1:])), (function, shapes)
+        assert all(a + n <= 512 for a, n in shapes)
+    assert found == 8
