@@ -41,7 +41,7 @@ constexpr int kMaskBuffers = 4;
 // which are added in f32 when they are read, the smallest first. Products are promised to add in the order of their issue where accumulator and shape are the same (PTX ISA, pipelined
 // tcgen05 instructions), so no two of them that differ in shape share a column. The scores' leading term times K's leading and middle one is one product of both sums; the other four
 // go to the third, with the middle term times the leading one, which belongs to order 1: what the tensor cores cut off there is 2^-8 of what they cut off in order 0. One instruction for each term
-// of A on neighbouring blocks of B, in shapes of 192, 128 and 64 columns that overlapped, had a quarter less to read from shared memory, and no promise (us from a graph, so and now: 1 x 256, 8 heads of 64 9.31 and 9.42;
+// of A on neighbouring blocks of B, in shapes of 192, 128 and 64 columns that overlapped, had a quarter less to read from shared memory, and no promise (us from a graph, so and with these: 1 x 256, 8 heads of 64 9.31 and 9.42;
 // 2 x 979 37.7 and 36.4; 4 x 1000, 8 of 32 46.4 and 47.0; 1 x 1024, 16/4 of 128 101.3 and 103.9; six products of one shape for the scores 9.5, 36.6, 47.1, 106.1).
 template <int D>
 struct Plan {
@@ -51,9 +51,9 @@ struct Plan {
     // K: by half and term (the three terms of 64 columns are neighbouring rows), V: by term and half (neighbouring columns)
     static constexpr int kK = 3 * kQPlane, kV = kK + 3 * kHalves * kBlock, kRed = kV + 3 * kHalves * kBlock;
     static constexpr int kVis = kRed + kMaxBuffers * kShares * kM * 4, kMl = kVis + kMaskBuffers * kN, kAt = kMl + kM * 8, kBar = kAt + kM * 8, kBytes = kBar + 80 + 1024;   // (1024: the planes are aligned to that)
-    // Tensor memory: the scores' three sums, the weights' three terms, O's sums. At head size 128 the weights lie over the scores, and O's small orders share one.
+    // Tensor memory: the scores' three sums, the weights' three terms, O's sums. At head size 128 the weights lie over the scores' third sum and behind it, and O's small orders share one.
     static constexpr bool kOver = D == 128;
-    static constexpr int kP = kOver ? 0 : 3 * kN, kO = kOver ? 3 * kN : 3 * kN + 3 * kN / 2, kOrders = kOver ? 2 : 3;
+    static constexpr int kP = kOver ? 2 * kN : 3 * kN, kO = kOver ? 4 * kN : 3 * kN + 3 * kN / 2, kOrders = kOver ? 2 : 3;
     static_assert(kO + kOrders * kCols <= 512, "fits tensor memory");
 };
 
@@ -115,23 +115,45 @@ __device__ __forceinline__ void commit(unsigned long long* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// What follows the first look of a wait, which suspends for some 8000 clocks: false when the limit has run out, here or for somebody else of the CTA. The wait's code goes to the status word, and
+// nobody in the CTA waits any more. A function, or in line where registers come out better so, which is what decides (us from a graph, in line and as a function: 4 x 2048, 8 heads of 128 528.8 and 506; 1 x 1024,
+// shared by two CTAs, 56.0 and 57.0; 4 x 1000, 8 of 32 47.1 and 44.8; 2 x 979, 8 of 64 36.4 and 37.3; 8 x 1024 102.4 and 105.0).
+__device__ __forceinline__ bool wait_in_line(unsigned bar, unsigned parity, unsigned given_up, long long limit, int* status, int where) {
+    const long long t0 = clock64();
+#pragma unroll 1
+    for (unsigned spin = 1; !mbar_try_wait_at(bar, parity); ++spin) {
+        if ((spin & 63u) != 0u) continue;
+        if (shared_flag(given_up)) return false;
+        if (clock64() - t0 > limit) {
+            set_shared_flag(given_up);
+            *reinterpret_cast<volatile int*>(status) = where;
+            __threadfence_system();
+            return false;
+        }
+    }
+    return true;
+}
+__device__ __noinline__ bool wait_called(unsigned bar, unsigned parity, unsigned given_up, long long limit, int* status, int where) {
+    return wait_in_line(bar, parity, given_up, limit, status, where);
+}
 // The issuer's products, in functions of their own: unrolled among the workers' code their descriptors cost everybody registers (head size 128: 1164 bytes of spill stores, 916 rolled up, 840 so).
-template <int D>
+template <int D, bool kFirst, bool kSmall>   // the first two sums, the third
 __device__ __noinline__ void issue_scores(unsigned tmem, unsigned long long dq, unsigned long long dk, unsigned long long* s_full) {
     using S = Plan<D>;
     const unsigned x = tmem, z = tmem + 2 * kN;
     tc_fence_after();
     if (elect_one()) {
 #pragma unroll
-        for (int t = 0; t < 3; ++t)
+        for (int t = 0; t < (kSmall ? 3 : 1); ++t)
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
                 const unsigned long long q = dq + ((t * S::kQPlane + (kk >> 2) * S::kQHalf + (kk & 3) * 32) >> 4), k = dk + (((kk >> 2) * 3 * kBlock + (kk & 3) * 32) >> 4);
-                if (t == 0) tc_mma_ss(x, q, k, make_idesc<__nv_bfloat16>(false, 2 * kN), kk > 0);
+                if (kFirst && t == 0) tc_mma_ss(x, q, k, make_idesc<__nv_bfloat16>(false, 2 * kN), kk > 0);
+                if (!kSmall) continue;
 #pragma unroll
                 for (int u = t == 0 ? 2 : 0; t + u < 3; ++u) tc_mma_ss(z, q, k + (u * kBlock >> 4), make_idesc<__nv_bfloat16>(false, kN), t + kk > 0);
             }
-        commit(s_full);
+        if (kSmall) commit(s_full);   // (the same lane is elected every time: its products before are behind the barrier as well)
     }
     __syncwarp();
 }
@@ -201,21 +223,11 @@ __global__ void __launch_bounds__(kThreads, 1) tile_f32_tcgen05_kernel(const __g
     const float scale = p.scale * 1.4426950408889634f;
 
     // Bounded: the wait's code goes to the status word, and nobody in the CTA waits any more.
+    constexpr bool kWaitInLine = D == 64 || (D == 128 && kCluster);
     auto wait = [&](unsigned long long* bar, unsigned parity, int where) {
         if (mbar_try_wait(bar, parity)) return true;
-        const long long t0 = clock64(), limit = (long long)(a.wait_ns * 2ULL);
-#pragma unroll 1
-        for (unsigned spin = 1; !mbar_try_wait(bar, parity); ++spin) {
-            if ((spin & 63u) != 0u) continue;
-            if (*given_up) return false;
-            if (clock64() - t0 > limit) {
-                *given_up = 1;
-                *reinterpret_cast<volatile int*>(a.status) = where;
-                __threadfence_system();
-                return false;
-            }
-        }
-        return true;
+        const auto on = kWaitInLine ? wait_in_line : wait_called;
+        return on(smem_u32(bar), parity, smem_u32((const void*)given_up), (long long)(a.wait_ns * 2ULL), a.status, where);
     };
 
     float acc[kOut], m = -INFINITY, l = 0.0f;   // of this thread's row: its columns of O, the maximum of the raw scores so far, the sum over its keys
@@ -246,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_f32_tcgen05_kernel(const __g
         tc_fence_after();
         const unsigned tmem = __shfl_sync(0xffffffffu, *tmem_base, 0), base = __shfl_sync(0xffffffffu, smem_u32(sm), 0);
         const unsigned long long dq = make_desc(base, 16, 1024), dk = make_desc(base + S::kK, 16, 1024), dv = make_desc(base + S::kV, kBlock, 1024);
-        auto scores = [&]() { issue_scores<D>(tmem, dq, dk, s_full); };
+        auto scores = [&]() { issue_scores<D, true, true>(tmem, dq, dk, s_full); };
         auto sums = [&]() { issue_sums<D>(tmem, dv, o_full); };
         bool alive = n == 0 || __all_sync(0xffffffffu, wait(k_ready, 0u, 60));
         if (alive && n > 0) scores();
@@ -263,9 +275,16 @@ __global__ void __launch_bounds__(kThreads, 1) tile_f32_tcgen05_kernel(const __g
             if (!alive) break;
             sums();
             if (S::kOver && more) {
-                alive = __all_sync(0xffffffffu, wait(k_ready, phase ^ 1u, 64));
+                // The third sum goes over the weights that sums() reads, and no order is promised there: it waits for their product. Behind the first two sums' products, or in a cluster with
+                // them (us from a graph: 4 x 2048, 8 heads 506 and 517; 1 x 1024, shared by two CTAs, 57.7 and 56.9; without the wait 523 with more spills, and 55.2)
+                alive = __all_sync(0xffffffffu, wait(k_ready, phase ^ 1u, 64) && (!kCluster || wait(o_full, phase, 65)));
                 if (!alive) break;
-                scores();
+                if (!kCluster) {
+                    issue_scores<D, true, false>(tmem, dq, dk, s_full);
+                    alive = __all_sync(0xffffffffu, wait(o_full, phase, 65));
+                    if (!alive) break;
+                }
+                issue_scores<D, kCluster, true>(tmem, dq, dk, s_full);
             }
         }
     } else {

@@ -1,7 +1,7 @@
 """The barriers between the warps of the f32 kernel on the tensor cores (csrc/tile_f32_tcgen05.cu), as a model on the CPU: worker warps (three quads of rows, two parts of
 keys and columns; the first two also write a tile's mask) and the issuer are coroutines that make the kernel's waits, arrivals and accesses in the kernel's order, and
-they and the products are interleaved at random. A product reads its operands at its begin and at its end; products end in the order in which
-they were issued. Checked: every wait is satisfied by the phase that it is for, no role waits for good, also where a wait runs out, and whatever is read, in shared memory and in tensor
+they and the products are interleaved at random. A product reads its operands at its begin and at its end; products into one sum end in the order in which
+they were issued, others in any. Checked: every wait is satisfied by the phase that it is for, no role waits for good, also where a wait runs out, and whatever is read, in shared memory and in tensor
 memory, is what was meant for that tile. How many buffers there are is read from the source; mistakes planted in the model show that it finds them."""
 import random
 import re
@@ -13,9 +13,11 @@ SOURCE = (Path(__file__).resolve().parent.parent / "luma_b200" / "csrc" / "tile_
 QUADS, PARTS = 3, 2
 WARPS = QUADS * PARTS
 WRITERS = 2
+WAITS_FOR_O = "wait(o_full, phase, 65)" in SOURCE
 MISTAKES = {
     "one buffer for the maxima": "a warp of the quad runs on and writes the next tile's maximum where another has not read this one's",
     "two buffers for the mask": "the warps that bring the next tile's mask are behind what others did two tiles ago only",
+    "scores without a wait for O": "at head size 128 the third sum of the scores lies over the weights, whose product may still run",
     "a tile's K before its scores are there": "the planes are written again under the product that reads them",
 }
 
@@ -52,11 +54,11 @@ class Cta:
         self.red = [[[None] * PARTS for _ in range(QUADS)] for _ in range(self.reds)]
         self.masks = 2 if mistake == "two buffers for the mask" else _buffers("kMaskBuffers")
         self.vis = [[None] * WRITERS for _ in range(self.masks)]
-        self.s = None                                    # scores in tensor memory: tile
+        self.s = [None, None]                            # the tile of the scores in tensor memory: first sums and third
         self.s_read = [None] * WARPS
         self.p = [None] * WARPS                          # weights
         self.o, self.o_read = None, [None] * WARPS
-        self.products = []                               # [check at begin and end, what it writes, begun], and commits
+        self.products = []                               # [where to, check at begin and end, what it writes, begun], and commits
         self.abort = False
 
     def check(self, what, *say):
@@ -74,14 +76,27 @@ class Cta:
         return True
 
     # -- products
-    def scores(self, j):
+    def product(self, to, reads, writes):
+        self.products.append([to, reads, writes, False])
+
+    def first_scores(self, j):
         def reads():
             self.check(all(x == j for x in self.k), "K", j, self.k)
             self.check(all(x == j - 1 for x in self.s_read) or j == 0, "scores over scores that have not been read", j, self.s_read)
 
         def writes():
-            self.s = j
-        self.products.append([reads, writes, False])
+            self.s[0] = j
+        self.product("first scores", reads, writes)
+
+    def small_scores(self, j):
+        def reads():
+            self.check(all(x == j for x in self.k), "K", j, self.k)
+            self.check(all(x == j - 1 for x in self.s_read) or j == 0, "scores over scores that have not been read", j, self.s_read)
+            self.check(not self.over or j == 0 or self.o == j - 1, "scores over weights that are still in use", j, self.o)
+
+        def writes():
+            self.s[1] = j
+        self.product("small scores", reads, writes)
         self.products.append(self.s_full)
 
     def sums(self, j):
@@ -91,35 +106,44 @@ class Cta:
 
         def writes():
             self.o = j
-        self.products.append([reads, writes, False])
+        self.product("O", reads, writes)
         self.products.append(self.o_full)
 
     def compute(self):
-        """The product at the head begins or ends, or its commit arrives."""
+        """A product begins or ends, or a commit behind products that have all ended arrives."""
         items = self.products
         if not isinstance(items[0], list):
             items.pop(0).arrive()
             return
-        reads, writes, begun = items[0]
+        able, places = [], set()
+        for i, x in enumerate(items):
+            if isinstance(x, list) and x[0] not in places:
+                places.add(x[0])
+                able.append(i)
+        i = self.rng.choice(able)
+        _, reads, writes, begun = items[i]
         reads()
         if begun:
             writes()
-            items.pop(0)
+            items.pop(i)
         else:
-            items[0][2] = True
+            items[i][3] = True
 
     # -- roles
     def issuer(self):
         if not (yield from self.wait(self.k_ready, 0)):
             return
-        self.scores(0)
+        self.first_scores(0)
+        self.small_scores(0)
         for j in range(self.n):
             more = j + 1 < self.n
             if not self.over and more:
                 for bar, x in ((self.k_ready, j + 1), (self.s_free, j)):
                     if not (yield from self.wait(bar, x)):
                         return
-                self.scores(j + 1)
+                self.first_scores(j + 1)
+                yield
+                self.small_scores(j + 1)
                 yield
             if not (yield from self.wait(self.pv_ready, j)):
                 return
@@ -128,7 +152,11 @@ class Cta:
             if self.over and more:
                 if not (yield from self.wait(self.k_ready, j + 1)):
                     return
-                self.scores(j + 1)
+                self.first_scores(j + 1)
+                yield
+                if WAITS_FOR_O and self.mistake != "scores without a wait for O" and not (yield from self.wait(self.o_full, j)):
+                    return
+                self.small_scores(j + 1)
                 yield
 
     def quad_barrier(self, w):
@@ -147,9 +175,9 @@ class Cta:
             if self.mistake == "a tile's K before its scores are there" and j + 1 < self.n:
                 self.k[w] = j + 1
             yield from self.wait(self.s_full, j)
-            self.check(self.s == j, "scores", j, self.s)
+            self.check(self.s == [j, j], "scores", j, self.s)
             yield
-            self.check(self.s == j, "scores", j, self.s)
+            self.check(self.s == [j, j], "scores", j, self.s)
             self.s_read[w] = j
             if not self.over:
                 self.s_free.arrive()
@@ -218,7 +246,7 @@ def test_the_model_finds_a_planted_mistake(mistake):
     found = 0
     for seed in range(1500):
         try:
-            Cta(5, False, seed, mistake=mistake).run()
+            Cta(5, mistake == "scores without a wait for O", seed, mistake=mistake).run()
         except AssertionError:
             found += 1
             if found == 3:
@@ -256,4 +284,6 @@ def test_products_that_share_columns_have_the_same_accumulator_and_shape(d):
         shapes = sorted(shapes)
         assert all(a + n <= b for (a, n), (b, _) in zip(shapes, shapes[1:])), (function, shapes)
         assert all(a + n <= 512 for a, n in shapes)
+    if d == 128:   # the weights over the third sum alone, and not over O
+        assert 2 * 64 <= env["kP"] and env["kP"] + 3 * 64 // 2 <= env["kO"]
     assert found == 8
