@@ -95,10 +95,14 @@ struct TileInfo {
 struct Item {
     int some;            // 0: nothing is left, the CTA ends
     int seq, kv_head;
-    int first_key;       // where the CTA's share of the keys begins (a multiple of a tile); kv_len, pos_off and kv_crow of `sq` count from there
-    int shared;          // the CTAs of the cluster share the keys (0: there are too few, or there is no pair)
     SeqExtent sq;
     TileInfo t[2];
+};
+
+// ... and its share of the keys, where a cluster has the pair. Not in Item, which the other instantiations carry in the registers of a producer that has none left.
+struct Share {
+    int first_key;       // where it begins (a multiple of a tile); kv_len, pos_off and kv_crow of the pair's `sq` count from there
+    int some;            // the CTAs of the cluster share the keys (0: there are too few, or there is no pair)
 };
 
 constexpr int kOutBytes = 4096;     // a softmax warp's rows on their way out: 32 of 128 bytes
@@ -112,6 +116,7 @@ struct SharedStorage {
     alignas(1024) unsigned char out[8][kOutBytes];
     alignas(16) unsigned char answer[16];   // what the request for another tile pair brought (written by the hardware)
     Item item[2];                   // tile pair i of the CTA in entry i & 1
+    Share share;                    // of item[0]
     alignas(8) unsigned long long item_full[2];   // K producer -> all roles: the entry holds the next tile pair
     unsigned long long item_empty[2];   // V producer, issuer, softmax warps -> K producer: it has been read
     unsigned long long answered;    // hardware -> K producer: `answer` is there
@@ -827,20 +832,19 @@ __device__ __forceinline__ bool find_pair(const PrefillArgs& a, int bx, int by, 
 
 // The share of a pair's keys that is this CTA's, of `parts` equal ones in whole tiles. A pair of up to five tiles stays whole, with the first CTA (the host knows a bound only: 2 x 147 tokens
 // over 609 keys with room for 2048, 8/2 heads, shared by four 18.9 us, alone 17.5).
-__device__ __forceinline__ void take_share(Item& w, int parts, int rank) {
+__device__ __forceinline__ Share take_share(Item& w, int parts, int rank) {
     const int most = max(w.t[0].n_kv, w.t[1].n_kv), per = (most + parts - 1) / parts;
-    w.first_key = 0;
-    w.shared = most > 5;
-    if (!w.shared) {
-        w.some = rank == 0;
-        return;
+    if (most <= 5) {
+        w.some = w.some && rank == 0;
+        return Share{0, 0};
     }
 #pragma unroll
     for (int t = 0; t < 2; ++t) w.t[t].n_kv = max(0, min(per, w.t[t].n_kv - rank * per));
-    w.first_key = rank * per * kBlockN;
-    w.sq.kv_len -= w.first_key;
-    w.sq.pos_off -= w.first_key;
-    w.sq.kv_crow += w.first_key;
+    const int first_key = rank * per * kBlockN;
+    w.sq.kv_len -= first_key;
+    w.sq.pos_off -= first_key;
+    w.sq.kv_crow += first_key;
+    return Share{first_key, 1};
 }
 
 // Clusters: every thread of its CTAs takes part in every phase, and all waits of all roles end, so these do.
@@ -904,8 +908,8 @@ __device__ __forceinline__ void split_rows(const PrefillArgs& a, SharedStorage<D
         }
         bool q_ok = true;
         if (kMask) {
-            const int pos = w.sq.pos_off + w.first_key + token;
-            q_ok = pos >= 0 && pos < w.sq.kv_len + w.first_key && a.mask[(long long)w.seq * a.kv_seq_len + pos] != 0;
+            const int pos = w.sq.pos_off + sm.share.first_key + token;
+            q_ok = pos >= 0 && pos < w.sq.kv_len + sm.share.first_key && a.mask[(long long)w.seq * a.kv_seq_len + pos] != 0;
         }
         const bool seen = sum > 0.0f && top < INFINITY && q_ok;
         // (a share whose reference moved on behind its NaN has it in its sum and its O alone)
@@ -1011,14 +1015,15 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         // The CTA's own tile pair, and its first copies at once, in as few instructions as that takes: all of them come in for the first time here, and
         // in the loop below, with its waits and cases, the first S came 1600 to 2300 clocks later (a fifth of a call of one short wave).
         w.some = find_pair<kMask, kPaged>(a, kSplit ? (int)blockIdx.x / a.parts : (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, lane, w);
+        Share share{0, 0};
         if (kSplit) {
-            w.shared = 0;
-            if (w.some) take_share(w, a.parts, (int)blockIdx.x % a.parts);
+            if (w.some) share = take_share(w, a.parts, (int)blockIdx.x % a.parts);
+            if (lane == 0) sm.share = share;   // (with the pair, or with the word that there is none)
         }
         asm volatile("barrier.cta.sync 1, 96;\n" ::: "memory");   // the barriers have been initialised
         begun = w.some && max(w.t[0].n_kv, w.t[1].n_kv) > 0 && !q_open && !kv_open && a.test_skip_k != 1;
         if (begun && (kPaged || lane == 0)) {
-            const int page = kPaged ? page_of_lane(a, w.sq.kv_len, w.seq, 0, lane, kSplit ? w.first_key : 0) : -1;
+            const int page = kPaged ? page_of_lane(a, w.sq.kv_len, w.seq, 0, lane, share.first_key) : -1;
             if (lane == 0 && w.t[0].n_kv > 0) {
                 mbar_expect_tx(&sm.q_full[0], TileBytes<D>::value);
                 tma_load_4d(sm.q[0], &q_map, &sm.q_full[0], 0, w.t[0].head, w.sq.q_crow + (w.t[0].row0 >> a.pack_log2), w.sq.q_cb);
@@ -1125,7 +1130,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     if (D == 128) tma_prefetch_4d(&q_map, 64, w.t[1].head, w.sq.q_crow + (w.t[1].row0 >> a.pack_log2), w.sq.q_cb);
                 }
             }
-            int page = kPaged ? page_of_lane(a, kv_len, seq, 0, lane, kSplit ? w.first_key : 0) : -1;
+            int page = kPaged ? page_of_lane(a, kv_len, seq, 0, lane, share.first_key) : -1;
             auto load_k = [&](int j) {   // K tile j of the pair is what step g + j - 1 reads besides its V tile, and arrives on its barrier (tile 0: on its own)
                 const int e = (g + j) & 1;
                 unsigned long long* const bar = j == 0 ? &sm.k_first : &sm.step_full[e ^ 1];
@@ -1140,7 +1145,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 (e ? k_free1 : k_free0) = commits + j;
                 if (j > 0) given = g + j;
                 else if (!skip) ++firsts;
-                if (kPaged && j + 1 < n_max) page = page_of_lane(a, kv_len, seq, j + 1, lane, kSplit ? w.first_key : 0);
+                if (kPaged && j + 1 < n_max) page = page_of_lane(a, kv_len, seq, j + 1, lane, share.first_key);
             };
             // (a tile that sees no key needs no Q: the issuer leaves it out)
             auto load_q = [&](const TileInfo ti, unsigned char* to, unsigned long long* bar, unsigned& loads) {
@@ -1163,7 +1168,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 firsts = 1;
                 q_loads0 = n0 > 0;
                 q_loads1 = n1 > 0;
-                if (kPaged && n_max > 1) page = page_of_lane(a, kv_len, seq, 1, lane, kSplit ? w.first_key : 0);
+                if (kPaged && n_max > 1) page = page_of_lane(a, kv_len, seq, 1, lane, share.first_key);
             } else
 #pragma unroll 1
             for (int n = 0; n < 3; ++n) {
@@ -1219,6 +1224,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             alive = __all_sync(0xffffffffu, producer_wait(sm, &sm.item_full[it & 1u], (it >> 1) & 1u, a, 7));
             if (!alive) break;
             const Item w = sm.item[it & 1u];
+            const Share share = kSplit ? sm.share : Share{0, 0};
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.item_empty[it & 1u]);
             if (!w.some) break;
@@ -1237,7 +1243,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             // ring's barrier with a plain arrival. (Garbage in K is harmless: the score mask is a select.)
             const bool tail_fix = (a.paged || packed) && (sq.kv_len % kBlockN) != 0;
             const int tail_j = sq.kv_len > 0 ? (sq.kv_len - 1) / kBlockN : -1;
-            int page = kPaged ? page_of_lane(a, sq.kv_len, w.seq, 0, lane, kSplit ? w.first_key : 0) : -1;
+            int page = kPaged ? page_of_lane(a, sq.kv_len, w.seq, 0, lane, share.first_key) : -1;
             for (int j = 0; j < n_max; ++j) {
                 const int e = (g + j) & 1;
                 const int c = e ? v_free1 : v_free0;
@@ -1250,7 +1256,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 else if (kPaged || lane == 0)
                     load_kv_tile<D, kPaged>(a, sq.kv_crow, sq.kv_cb, w.kv_head, sm.v[e], &v_map, bar, j, page, lane);
                 (e ? v_free1 : v_free0) = commits + j + 1;
-                if (kPaged && j + 1 < n_max) page = page_of_lane(a, sq.kv_len, w.seq, j + 1, lane, kSplit ? w.first_key : 0);
+                if (kPaged && j + 1 < n_max) page = page_of_lane(a, sq.kv_len, w.seq, j + 1, lane, share.first_key);
                 if (!fix) {
                     given = g + j + 1;
                     continue;
@@ -1356,7 +1362,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.item_empty[it & 1u]);
         if (!some) break;
-        const int first_key = kSplit ? sm.item[it & 1u].first_key : 0;
+        const int first_key = kSplit ? sm.share.first_key : 0;
         const int row = ti.row0 + r, pl = a.pack_log2;
         const int pos = sq.pos_off + (row >> pl);   // global position of this row's query token
         // the last key that this row sees, and the last that every row of the tile sees (-1: none)
@@ -1476,7 +1482,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         if (alive && ti.n_kv > 0)
             alive = __all_sync(0xffffffffu, mbar_wait(sm, &sm.o_full[t], tiles++ & 1u, a, 30 + t));
         FA_TRACE_EVENT(t, max(0, (int)steps - 1), 4);
-        if (kSplit && sm.item[0].shared) {
+        if (kSplit && sm.share.some) {
             have = alive;
             last_n = ti.n_kv;
             last_m = m;
@@ -1638,12 +1644,12 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");   // shared memory stays valid until read
         if constexpr (kSplit) {
             __syncthreads();   // the products of both tiles have finished, nobody reads K or V any more
-            if (sm.item[0].shared) split_rows<T, D, kMask>(a, sm, have, t, r, warp, lane, tmem + lane_base + 256 + t * 128, last_n, last_m, last_l);
+            if (sm.share.some) split_rows<T, D, kMask>(a, sm, have, t, r, warp, lane, tmem + lane_base + 256 + t * 128, last_n, last_m, last_l);
         }
     }
     if (kSplit && warp >= 8) {
         __syncthreads();           // (every role has ended: what the K producer found out is there, and the same in all CTAs of the cluster)
-        if (sm.item[0].shared) {   // the phases of split_rows, where every thread of a cluster is counted
+        if (sm.share.some) {   // the phases of split_rows, where every thread of a cluster is counted
             cluster_arrive();
             cluster_wait();
             cluster_arrive();
