@@ -137,7 +137,9 @@ __device__ __noinline__ bool wait_called(unsigned bar, unsigned parity, unsigned
     return wait_in_line(bar, parity, given_up, limit, status, where);
 }
 // The issuer's products, in functions of their own: unrolled among the workers' code their descriptors cost everybody registers (head size 128: 1164 bytes of spill stores, 916 rolled up, 840 so).
-template <int D, bool kFirst, bool kSmall>   // the first two sums, the third
+// At head size 64 rolled up where they come in for the first time (the scores of clusters, whose CTAs have a tile or two; what reads inputs anew every time: 1 x 256, 8 heads 10.94 us and 10.83) or where that is the
+// faster form (the sums; 8 x 1024, 8 heads 102.6 and 101.8; with the scores rolled up as well 104.0).
+template <int D, bool kFirst, bool kSmall, bool kRolled>   // the first two sums, the third
 __device__ __noinline__ void issue_scores(unsigned tmem, unsigned long long dq, unsigned long long dk, unsigned long long* s_full) {
     using S = Plan<D>;
     const unsigned x = tmem, z = tmem + 2 * kN;
@@ -145,7 +147,7 @@ __device__ __noinline__ void issue_scores(unsigned tmem, unsigned long long dq, 
     if (elect_one()) {
 #pragma unroll
         for (int t = 0; t < (kSmall ? 3 : 1); ++t)
-#pragma unroll
+#pragma unroll (kRolled ? 1 : D / 16)
             for (int kk = 0; kk < D / 16; ++kk) {
                 const unsigned long long q = dq + ((t * S::kQPlane + (kk >> 2) * S::kQHalf + (kk & 3) * 32) >> 4), k = dk + (((kk >> 2) * 3 * kBlock + (kk & 3) * 32) >> 4);
                 if (kFirst && t == 0) tc_mma_ss(x, q, k, make_idesc<__nv_bfloat16>(false, 2 * kN), kk > 0);
@@ -163,7 +165,7 @@ __device__ __noinline__ void issue_sums(unsigned tmem, unsigned long long dv, un
     const unsigned o0 = tmem + S::kO, o1 = tmem + S::kO + S::kCols, o2 = tmem + S::kO + (S::kOrders - 1) * S::kCols;
     tc_fence_after();
     if (elect_one()) {
-#pragma unroll
+#pragma unroll (D == 64 ? 1 : 4)
         for (int kk = 0; kk < 4; ++kk) {
             const unsigned p = tmem + S::kP + kk * 8, p1 = p + kN / 2, p2 = p + kN;
             const unsigned long long v = dv + (kk * 2048 >> 4), v1 = v + (S::kHalves * kBlock >> 4), v2 = v + (2 * S::kHalves * kBlock >> 4);
@@ -258,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_f32_tcgen05_kernel(const __g
         tc_fence_after();
         const unsigned tmem = __shfl_sync(0xffffffffu, *tmem_base, 0), base = __shfl_sync(0xffffffffu, smem_u32(sm), 0);
         const unsigned long long dq = make_desc(base, 16, 1024), dk = make_desc(base + S::kK, 16, 1024), dv = make_desc(base + S::kV, kBlock, 1024);
-        auto scores = [&]() { issue_scores<D, true, true>(tmem, dq, dk, s_full); };
+        auto scores = [&]() { issue_scores<D, true, true, D == 64 && kCluster>(tmem, dq, dk, s_full); };
         auto sums = [&]() { issue_sums<D>(tmem, dv, o_full); };
         bool alive = n == 0 || __all_sync(0xffffffffu, wait(k_ready, 0u, 60));
         if (alive && n > 0) scores();
@@ -280,11 +282,11 @@ __global__ void __launch_bounds__(kThreads, 1) tile_f32_tcgen05_kernel(const __g
                 alive = __all_sync(0xffffffffu, wait(k_ready, phase ^ 1u, 64) && (!kCluster || wait(o_full, phase, 65)));
                 if (!alive) break;
                 if (!kCluster) {
-                    issue_scores<D, true, false>(tmem, dq, dk, s_full);
+                    issue_scores<D, true, false, false>(tmem, dq, dk, s_full);
                     alive = __all_sync(0xffffffffu, wait(o_full, phase, 65));
                     if (!alive) break;
                 }
-                issue_scores<D, kCluster, true>(tmem, dq, dk, s_full);
+                issue_scores<D, kCluster, true, false>(tmem, dq, dk, s_full);
             }
         }
     } else {
