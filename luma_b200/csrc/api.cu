@@ -21,6 +21,7 @@ namespace fa {
 namespace {
 thread_local char g_last_error[256] = {0};
 thread_local const char* g_last_path = "";
+thread_local const char* g_last_form = "";
 thread_local int g_last_launches = 0;
 // Option knobs: written by flash_attn_set_option on any thread, read by launches on any thread.
 std::atomic<int> g_force_generic{0};
@@ -43,8 +44,9 @@ void set_last_errorf(const char* fmt, ...) {
     va_end(ap);
 }
 
-void note_path(const char* name, int launches) {
+void note_path(const char* name, int launches, const char* form) {
     g_last_path = name;
+    g_last_form = form;
     g_last_launches = launches;
 }
 
@@ -735,6 +737,7 @@ extern "C" {
 const char* flash_attn_last_error(void) { return fa::g_last_error; }
 const char* flash_attn_version(void) { return "luma-b200-flash-attn 0.1.0 (sm_100a)"; }
 const char* flash_attn_last_path(void) { return fa::g_last_path; }
+const char* flash_attn_last_form(void) { return fa::g_last_form; }
 int flash_attn_last_launches(void) { return fa::g_last_launches; }
 
 int flash_attn_device_status(void) {

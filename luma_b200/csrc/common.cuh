@@ -173,7 +173,7 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
 int release_host_pipes();   // host_pipe.cu: frees the staging buffers of flash_attn_host_<T>; returns how many devices held some
 void set_last_error(const char* msg);
 void set_last_errorf(const char* fmt, ...);
-void note_path(const char* name, int launches);   // records flash_attn_last_path / _launches
+void note_path(const char* name, int launches, const char* form = "");   // records flash_attn_last_path / _launches / _form
 int get_option_force_generic();
 int get_option_decode_chunk();
 int get_option_prefill_trace();

@@ -1994,7 +1994,7 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
             return FLASH_ATTN_ERR_CUDA;
         }
         const int rc = check_launch("prefill_tcgen05_kernel");
-        if (rc == FLASH_ATTN_OK) note_path("prefill_tcgen05", 1);
+        if (rc == FLASH_ATTN_OK) note_path("prefill_tcgen05", 1, parts == 8 ? "cluster 8" : parts == 4 ? "cluster 4" : "cluster 2");
         return rc;
     }
     constexpr bool kOneWave = D == 128 || kPaged;
@@ -2022,7 +2022,7 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     cudaLaunchKernelEx(&cfg, kernel, qm, km, vm, om, a);
     rc = check_launch("prefill_tcgen05_kernel");
     if (rc == FLASH_ATTN_OK && a.skip_rows > 0 && !a.behind_few) rc = launch_mixed_few_rows(p, few, stream);
-    if (rc == FLASH_ATTN_OK) note_path("prefill_tcgen05", a.skip_rows > 0 ? 2 : 1);
+    if (rc == FLASH_ATTN_OK) note_path("prefill_tcgen05", a.skip_rows > 0 ? 2 : 1, a.behind_few ? "few rows ahead" : a.skip_rows > 0 ? "few rows behind" : one_pair ? "one pair" : "pairs");
     return rc;
 }
 

@@ -389,7 +389,7 @@ int launch_one(const AttnParams& p, cudaStream_t stream) {
     dim3 grid((unsigned)((rows + S::kRows - 1) / S::kRows), (unsigned)p.kv_heads, (unsigned)p.num_seqs);
     tile_f32_kernel<D, WR><<<grid, kThreads, S::kBytes, stream>>>(p);
     const int rc = check_launch("tile_f32_kernel");
-    if (rc == FLASH_ATTN_OK) note_path("tile_f32", 1);
+    if (rc == FLASH_ATTN_OK) note_path("tile_f32", 1, "mma");
     return rc;
 }
 

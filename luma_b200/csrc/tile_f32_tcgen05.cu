@@ -625,7 +625,7 @@ int launch_one(const AttnParams& p, int clusters, cudaStream_t stream) {
     cfg.numAttrs = kCluster ? 1 : 0;
     cudaLaunchKernelEx(&cfg, tile_f32_tcgen05_kernel<D, kCluster, kPlain>, a);
     const int rc = check_launch("tile_f32_tcgen05_kernel");
-    if (rc == FLASH_ATTN_OK) note_path("tile_f32", 1);
+    if (rc == FLASH_ATTN_OK) note_path("tile_f32", 1, clusters == 8 ? "tcgen05 cluster 8" : clusters == 4 ? "tcgen05 cluster 4" : clusters == 2 ? "tcgen05 cluster 2" : "tcgen05");
     return rc;
 }
 

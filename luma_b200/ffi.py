@@ -48,7 +48,7 @@ EXPORTED_SYMBOLS = (
        "flash_attn_release_workspaces", "flash_attn_debug_launch_rank", "flash_attn_host_steps"]
     + [f"flash_attn_host_{s}" for s in DTYPE_SUFFIX]
     + [f"luma_softmax_{s}" for s in DTYPE_SUFFIX]   # include/luma_nn_kernels.h
-    + ["flash_attn_debug_block_slots", "flash_attn_version", "flash_attn_device_status", "flash_attn_debug_read", "flash_attn_last_path",
+    + ["flash_attn_debug_block_slots", "flash_attn_version", "flash_attn_device_status", "flash_attn_debug_read", "flash_attn_last_path", "flash_attn_last_form",
        "flash_attn_last_launches", "flash_attn_set_option"]
     # include/luma_dist_comm.h
     + ["luma_comm_unique_id", "luma_comm_from_rank", "luma_comm_from_devices", "luma_comm_rank", "luma_comm_world_size",
@@ -133,6 +133,8 @@ lib.flash_attn_debug_read.argtypes = [c_void_p, c_int]
 lib.flash_attn_debug_read.restype = c_int
 lib.flash_attn_last_path.argtypes = []
 lib.flash_attn_last_path.restype = c_char_p
+lib.flash_attn_last_form.argtypes = []
+lib.flash_attn_last_form.restype = c_char_p
 lib.flash_attn_last_launches.argtypes = []
 lib.flash_attn_last_launches.restype = c_int
 lib.flash_attn_set_option.argtypes = [c_char_p, c_int]
@@ -150,6 +152,10 @@ def last_error() -> str:
 def last_path() -> str:
     p = lib.flash_attn_last_path()
     return "" if p is None else p.decode()
+
+
+def last_form() -> str:
+    return lib.flash_attn_last_form().decode()
 
 
 def device_status() -> int:
