@@ -13,6 +13,7 @@
 #include <utility>
 
 #include "../../include/flash_attn.h"
+#include "shares.cuh"
 
 namespace fa {
 
@@ -121,40 +122,6 @@ __host__ __device__ inline int launch_rank(int by, int w, int m) {
     if (by < w) return by * m;
     if (by - w < w * (m - 1)) return ((by - w) / (m - 1)) * m + 1 + (by - w) % (m - 1);
     return by;
-}
-
-// Division of n < 2^31 by a divisor the host knows, as a product with its rounded-up inverse (Granlund and Montgomery, "Division by
-// invariant integers using multiplication"): a product, a sum and a shift. With the division operator, a CTA made ten divisions by run-time values one after
-// the other before its first copy was requested, and knew its extents 1700 clocks from its start (timeline), on an SM with nothing else to do.
-struct FastDiv {
-    unsigned mul, shift;
-    int d;
-    FastDiv() = default;
-    __host__ explicit FastDiv(int divisor) : mul(0), shift(0), d(divisor) {
-        while ((1u << shift) < (unsigned)d) ++shift;
-        mul = (unsigned)((((1ULL << shift) - (unsigned)d) << 32) / (unsigned)d) + 1u;
-    }
-    __device__ __forceinline__ int div(int n) const { return (int)((__umulhi((unsigned)n, mul) + (unsigned)n) >> shift); }
-};
-
-// Query heads of a GQA group that share a tile of the tensor-core prefill kernel: the largest power of two, up to the 32 rows that a warp
-// stores at a time, that divides the group.
-__host__ __device__ inline int pack_of(int group) {
-    const int low = group & -group;
-    return low < 32 ? low : 32;
-}
-// Pairs of 128-row tiles that q_len query tokens make for a KV head there.
-__host__ __device__ inline long long prefill_pairs(int group, long long q_len) {
-    const int pack = pack_of(group);
-    return ((long long)(group / pack) * ((q_len * pack + 127) / 128) + 1) / 2;
-}
-
-// CTAs that share the keys of a tile pair there: of `pairs` pairs in all over up to `tiles` K/V tiles (`exact`: over as many), `rows` rows per KV head and sequence (rule and times
-// where it is launched).
-inline int prefill_parts(long long pairs, long long tiles, bool exact, long long rows, int sms) {
-    if (tiles <= (rows <= 16 && exact ? 7 : 12)) return 1;
-    if (21 * pairs <= 2 * sms && tiles >= (rows > 16 ? 32 : 16)) return 8;
-    return 9 * pairs <= 2 * sms ? 4 : 2 * pairs <= sms ? 2 : 1;
 }
 
 template <typename T> __device__ __forceinline__ float to_f32(T v);

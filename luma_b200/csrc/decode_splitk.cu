@@ -221,32 +221,6 @@ __device__ __forceinline__ int rows_units(const RowsArgs& a, const RowsSeq& r, i
     return max(1, (rows_visible(r) + kUnit - 1) / kUnit);
 }
 
-// What a sequence weighs in the cut: its units, and behind them `cost` units for what it costs a CTA to begin and to end one (its query rows, the merge of the warps' parts, the
-// count). Cut by the units alone, the CTAs with the end of a sequence in their share came to their own end 2 to 4 us behind the others (us, before and so: 8 x 4000 contiguous,
-// where eight of 37 columns hold one, 27.9 and 26.7; 8 x 512-2048 15.2 and 13.7; 16 x 7 tokens over 1217-4869, 8/2 heads 26.9 and 24.6; 16 x 91-367, 8 heads of 64 11.9 and 9.6).
-__device__ __forceinline__ unsigned rows_span(int units, int cost) { return units > 0 ? (unsigned)(units + cost) : 0u; }
-// Where the columns get little more than a unit each there is nothing to even out, and a cost would leave columns empty.
-__device__ __forceinline__ int rows_cost(const RowsArgs& a, unsigned total_units, int columns) { return total_units <= (unsigned)columns + (unsigned)columns / 8u ? 0 : a.seq_cost; }
-
-// The cut of `total` units into columns: the first `more` columns have share + 1 units, the others share
-// (or, forced, every column at least `forced` units). All in 32 bits: a 64-bit division here cost a microsecond of a small call.
-struct Cut {
-    unsigned share, more;
-    __device__ __forceinline__ Cut(unsigned total, unsigned columns, unsigned forced) {
-        share = total / columns;
-        more = total - share * columns;
-        if (share < forced || (share == forced && more == 0u)) {   // (never less than covers them all, whatever bound the host had)
-            share = forced;
-            more = 0u;
-        }
-    }
-    __device__ __forceinline__ unsigned first(unsigned c) const { return share * c + min(c, more); }
-    __device__ __forceinline__ unsigned column_of(unsigned unit) const {
-        const unsigned split = more * (share + 1u);
-        return unit < split ? unit / (share + 1u) : more + (unit - split) / share;
-    }
-};
-
 // One arrival; returns how many came before it. Everything the CTA's threads wrote before their last barrier is visible to
 // whoever sees the count (release), and what earlier arrivals published is visible to this CTA after its next barrier (acquire).
 // Whatever an earlier call left there (calls that overlapped on one buffer, which spoils their results, leave counts that are
@@ -469,7 +443,7 @@ __global__ void __launch_bounds__(kWarps * 32, Smem<D, kWarps>::kCtasPerSm) deco
     unsigned u_begin, u_end;
     if (kMode == MODE_BATCH) {
         const int units = rows_units<kWarps>(a, rows_seq<kMode>(a, 0), group, row0);
-        cost = rows_cost(a, (unsigned)units * (unsigned)a.num_seqs, columns);
+        cost = rows_cost((unsigned)units * (unsigned)a.num_seqs, columns, a.seq_cost);
         const unsigned per = rows_span(units, cost);
         total = per * (unsigned)a.num_seqs;
         columns = (int)min((unsigned)columns, max(total, 1u));   // never an empty column between two others
@@ -514,7 +488,7 @@ __global__ void __launch_bounds__(kWarps * 32, Smem<D, kWarps>::kCtasPerSm) deco
             seqs += (unsigned)__shfl_sync(0xffffffffu, upto_seqs, 31);
             if (s0 + 128 >= a.num_seqs) break;
         }
-        cost = rows_cost(a, total, columns);
+        cost = rows_cost(total, columns, a.seq_cost);
         total += seqs * (unsigned)cost;
         columns = (int)min((unsigned)columns, max(total, 1u));   // never an empty column between two others
         const Cut cut(total, (unsigned)columns, (unsigned)a.forced_units);

@@ -53,8 +53,6 @@ namespace fa {
 
 namespace {
 
-constexpr int kBlockM = 128;   // query rows per tile
-constexpr int kBlockN = 128;   // keys per K/V tile
 // head size D (64 or 128) is a template parameter of the kernel
 constexpr int kStages = 2;     // depth of the K and V rings
 static_assert(kStages == 2, "step_full and step_done have an entry per stage, found by the parity of the step (j & 1, phase j >> 1) throughout the kernel");
@@ -74,36 +72,6 @@ constexpr float kRescaleThreshold = 8.0f;            // log2 units
 // 227.9, 230.1. At head size 64, 1/8, 1/6, 1/5, 1/4: 2 x 4096 189.7, 195.6, 191.8, 197.7; 8 x 1000 65.3, 67.0, 66.4, 70.6; 24 packed prompts of 17-2000 250.8, 256.8, 256.7, 261.6. The error of the
 // log-sum-exp against 64 bits is the same for 1/8 and 1/6 (rms 2.1-3.9e-7 over 100-4096 tokens).
 template <int D> __device__ __forceinline__ constexpr bool fma_pipe_exp(int i) { return D == 128 ? i % 6 == 5 : (i & 7) == 7; }
-
-// Extents of one sequence. Query row i sits at global position pos_off + i and sees keys
-// j < kv_len with j <= pos_off + i (bottom-right aligned for the varlen and kv-cache entry points).
-struct SeqExtent {
-    int q_len, kv_len, pos_off;   // (positions fit 32 bits: the last one is below kv_len or, batched, kv_seq_len + q_seq_len; see start_pos)
-    long long o_row0;     // first row of this sequence in o (rows of o_heads * 128 elements)
-    int q_crow, q_cb;     // TMA coordinates (row, batch) of the sequence's first q row
-    int kv_crow, kv_cb;   // same for contiguous K/V (unused when paged)
-};
-
-struct TileInfo {
-    int valid;    // this query tile exists
-    int head;     // query head, the first of those that share the tile
-    int row0;     // first row, in rows of query token x head of the tile
-    int n_kv;     // K/V tiles it needs
-};
-
-// One tile pair, as the CTA's roles find it in shared memory.
-struct Item {
-    int some;            // 0: nothing is left, the CTA ends
-    int seq, kv_head;
-    SeqExtent sq;
-    TileInfo t[2];
-};
-
-// ... and its share of the keys, where a cluster has the pair. Not in Item, which the other instantiations carry in the registers of a producer that has none left.
-struct Share {
-    int first_key;       // where it begins (a multiple of a tile); kv_len, pos_off and kv_crow of the pair's `sq` count from there
-    int some;            // the CTAs of the cluster share the keys (0: there are too few, or there is no pair)
-};
 
 constexpr int kOutBytes = 4096;     // a softmax warp's rows on their way out: 32 of 128 bytes
 constexpr int kDone = 4;            // entries of step_done, see there
@@ -432,36 +400,6 @@ __device__ __forceinline__ SeqExtent seq_extent(const PrefillArgs& a, int s) {
     return e;
 }
 
-// Tiles that the query tokens of a sequence fill for `pack` heads.
-static_assert(kBlockM == 1 << 7, "rows of a tile");
-__host__ __device__ __forceinline__ int row_blocks(int q_len, int pack_log2) { return (q_len + (kBlockM >> pack_log2) - 1) >> (7 - pack_log2); }
-
-// One past the last query token of tile `idx` of a sequence, or of its last tile.
-__device__ __forceinline__ int tile_token_end(const SeqExtent& a, int idx, const FastDiv& by_packs, int pack_log2, int num_mb) {
-    const int mb = idx < by_packs.d * num_mb ? by_packs.div(idx) : num_mb - 1;
-    return min((mb + 1) * (kBlockM >> pack_log2), a.q_len);
-}
-
-template <bool kMask>
-__device__ __forceinline__ TileInfo tile_info(const SeqExtent& a, int pair, int t, int kvh, const FastDiv& by_packs, int pack_log2, int num_mb) {
-    TileInfo ti;
-    // Tile 0 takes the later index of the pair: where the pair is two consecutive row blocks of the same heads,
-    // that is the longer tile, and tile 0 is the one whose copies are requested first and whose
-    // products the issuer serves first in every step, so the tile that decides when the CTA ends is never
-    // the one that waits (S = 2048 MHA: 887-892 against 851 TFLOP/s).
-    const int idx = pair * 2 + (1 - t);
-    const int packs = by_packs.d;
-    ti.valid = idx < packs * num_mb;
-    const int mb = ti.valid ? by_packs.div(idx) : 0;
-    ti.head = (kvh * packs + (ti.valid ? idx - mb * packs : 0)) << pack_log2;
-    ti.row0 = mb * kBlockM;
-    const int last_token = (min(ti.row0 + kBlockM, a.q_len << pack_log2) - 1) >> pack_log2;
-    const int last_key = min(a.kv_len - 1, a.pos_off + last_token);
-    ti.n_kv = ti.valid && last_key >= 0 ? last_key / kBlockN + 1 : 0;   // 0: the tile sees no key at all
-    if (kMask && a.pos_off + (ti.row0 >> pack_log2) >= a.kv_len) ti.n_kv = 0;   // all its rows sit in padding
-    return ti;
-}
-
 // The launch order of chunks of prompts over long contexts, whose lengths the host does not know: CTA `index`
 // of the grid takes the index-th tile pair of the call, heaviest first (K/V tiles, in classes of an eighth of the longest
 // range, so that the pairs of one K/V stream stay neighbours and meet in L2). In grid order (sequences as they
@@ -470,18 +408,6 @@ __device__ __forceinline__ TileInfo tile_info(const SeqExtent& a, int pair, int 
 constexpr int kOrderPerLane = 8;
 constexpr int kOrderMax = 32 * kOrderPerLane;
 constexpr int kOrderClasses = 8;
-
-// Tile pairs of one sequence whose longer tile sees at least w K/V tiles (w <= 0: all): pair p holds tiles 2p and
-// 2p + 1, tile i the row block i / packs.
-__device__ __forceinline__ int pairs_from(int q_len, int kv_len, int packs, int pack_log2, int w) {
-    if (q_len <= 0) return 0;
-    const int pairs = (packs * row_blocks(q_len, pack_log2) + 1) / 2;
-    if (w <= 0) return pairs;
-    const long long key = (long long)(w - 1) * kBlockN;            // such a tile sees this key ...
-    const long long token = key - ((long long)kv_len - q_len);     // ... and so does this query token or a later one
-    if (key >= kv_len || token >= q_len) return 0;
-    return pairs - (int)((max(token, 0LL) << pack_log2) / kBlockM) * packs / 2;
-}
 
 // Returns {sequence or -1, KV head, pair}.
 __device__ __forceinline__ int3 find_item(const PrefillArgs& a, int index, int lane) {
@@ -828,23 +754,6 @@ __device__ __forceinline__ bool find_pair(const PrefillArgs& a, int bx, int by, 
     w.t[0] = tile_info<kMask>(w.sq, pair, 0, w.kv_head, a.by_packs, a.pack_log2, num_mb);
     w.t[1] = tile_info<kMask>(w.sq, pair, 1, w.kv_head, a.by_packs, a.pack_log2, num_mb);
     return w.t[0].valid || w.t[1].valid;   // (a sequence may be shorter than the grid's row range)
-}
-
-// The share of a pair's keys that is this CTA's, of `parts` equal ones in whole tiles. A pair of up to five tiles stays whole, with the first CTA (the host knows a bound only: 2 x 147 tokens
-// over 609 keys with room for 2048, 8/2 heads, shared by four 18.9 us, alone 17.5).
-__device__ __forceinline__ Share take_share(Item& w, int parts, int rank) {
-    const int most = max(w.t[0].n_kv, w.t[1].n_kv), per = (most + parts - 1) / parts;
-    if (most <= 5) {
-        w.some = w.some && rank == 0;
-        return Share{0, 0};
-    }
-#pragma unroll
-    for (int t = 0; t < 2; ++t) w.t[t].n_kv = max(0, min(per, w.t[t].n_kv - rank * per));
-    const int first_key = rank * per * kBlockN;
-    w.sq.kv_len -= first_key;
-    w.sq.pos_off -= first_key;
-    w.sq.kv_crow += first_key;
-    return Share{first_key, 1};
 }
 
 // Clusters: every thread of its CTAs takes part in every phase, and all waits of all roles end, so these do.
