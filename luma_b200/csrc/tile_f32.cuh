@@ -24,6 +24,14 @@ __device__ __forceinline__ void split3(float x, float y, unsigned& hi, unsigned&
     lo = pack16<__nv_bfloat16>(rest.x, rest.y);
 }
 
+// x / y for many x, given 1 / y rounded to nearest: a product, its remainder and one correction (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990), which
+// round to nearest while nothing underflows: the bits of the division operator, whose code at the end of a kernel, for 16 or 32 columns of a row, takes longer (tile_f32_tcgen05.cu, us: 1 x 256, 8 heads of 64
+// 11.08 and 10.77 so; 4 x 2048, 8 of 128 523 and 506).
+__host__ __device__ __forceinline__ float quotient(float x, float y, float inv) {
+    const float q = x * inv;
+    return fmaf(fmaf(-q, y, x), inv, q);
+}
+
 // The rows of a CTA that met a value that does not survive the split, one key at a time in plain f32, as tile_simt.cu
 // does it: a warp per row (the CTA's first kWarps). An infinity minus itself, and infinity times the other operand's small terms, are NaN where the
 // product is not, and so is zero weight times a row that a query does not see; the same holds for a value that rounds

@@ -105,12 +105,6 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
 }
 
-// x / y, given 1 / y rounded.
-__device__ __forceinline__ float quotient(float x, float y, float inv) {
-    const float q = x * inv;
-    return fmaf(fmaf(-q, y, x), inv, q);
-}
-
 __device__ __forceinline__ void commit(unsigned long long* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
