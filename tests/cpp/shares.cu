@@ -1,4 +1,4 @@
-// The arithmetic by which CTAs share work (luma_b200/csrc/shares.cuh) for tests/test_cut_model.py, which calls it on the host.
+// The arithmetic by which CTAs share work (luma_b200/csrc/shares.cuh) for tests/test_cut_code.py, which calls it on the host.
 #include "../../luma_b200/csrc/shares.cuh"
 
 using namespace fa;

@@ -15,12 +15,12 @@ from tests import helpers as H
 pytestmark = pytest.mark.gpu
 
 
-def _twice(call, want, what, *forms):
+def _twice(call, want, what):
     first = None
     for _ in range(2):
         o = call()
         torch.cuda.synchronize()
-        assert ffi.last_path() == "prefill_tcgen05" and ffi.last_form() in forms and ffi.device_status() == 0
+        assert ffi.last_path() == "prefill_tcgen05" and ffi.device_status() == 0
         H.assert_bf16_close(H.to_np(o), want, what)
         assert first is None or torch.equal(first, o)
         first = o
@@ -28,15 +28,14 @@ def _twice(call, want, what, *forms):
 
 
 @pytest.mark.parametrize("d,dt", [(128, "bf16"), (64, "f16"), (32, "bf16")])
-@pytest.mark.parametrize("b,sq,skv,hq,hkv,sp,masked,ctas", [
-    (1, 70, 4500, 2, 1, 4430, False, 8),
-    (3, 129, 2100, 4, 4, 1971, False, 4),     # a pair with one row in its second tile
-    (1, 1700, 1700, 6, 2, 0, False, 2),       # early rows see few of the shares
-    (2, 1700, 1700, 6, 2, 0, False, 1),       # too many pairs
-    (1, 300, 1800, 3, 3, 0, False, 4),        # keys that nobody sees
-    (2, 200, 2000, 4, 2, 1800, True, 4), (4, 1, 1100, 8, 2, 1099, True, 4), (3, 4, 1000, 4, 1, 996, True, 4), (3, 400, 1700, 10, 5, 1300, True, 2),
+@pytest.mark.parametrize("b,sq,skv,hq,hkv,sp,masked", [
+    (1, 70, 4500, 2, 1, 4430, False),      # 8 CTAs to a pair
+    (3, 129, 2100, 4, 4, 1971, False),     # 4; a pair with one row in its second tile
+    (2, 1700, 1700, 6, 2, 0, False),       # 2; early rows see few of the shares
+    (1, 300, 1800, 3, 3, 0, False),        # keys that nobody sees
+    (2, 200, 2000, 4, 2, 1800, True), (4, 1, 1100, 8, 2, 1099, True), (3, 4, 1000, 4, 1, 996, True),
 ])
-def test_batched(b, sq, skv, hq, hkv, sp, masked, ctas, d, dt):
+def test_batched(b, sq, skv, hq, hkv, sp, masked, d, dt):
     q, k, v = (H.round_to(H.normal(s, x), dt) for s, x in (((b, sq, hq, d), 1), ((b, skv, hkv, d), 2), ((b, skv, hkv, d), 3)))
     mask = None
     if masked:
@@ -52,16 +51,16 @@ def test_batched(b, sq, skv, hq, hkv, sp, masked, ctas, d, dt):
         lse.fill_(float("nan"))
         low.flash_attn(*dev, o, b, sq, skv, hq, hkv, d, sp, 1.0 / math.sqrt(d), None if mask is None else torch.from_numpy(mask).cuda(), None, lse)
         return o
-    _twice(call, want, f"{b} x {sq} over {skv}", *([f"cluster {ctas}"] if ctas > 1 else ["pairs", "one pair"]))
+    _twice(call, want, f"{b} x {sq} over {skv}")
     got, there = lse.cpu().numpy(), np.isfinite(lse_want)
     assert np.array_equal(np.isfinite(got), there) and np.abs(got[there] - lse_want[there]).max() <= 1e-3
 
 
 @pytest.mark.parametrize("d", [128, 64])
-@pytest.mark.parametrize("sq,hq,hkv,page,lens,ctas", [
-    (100, 4, 1, 16, [4200, 100, 130], 8), (130, 3, 1, 32, [1800, 0, 131, 40], 4), (65, 16, 2, 128, [2900, 600], 4), (70, 8, 8, 8, [1700, 70, 1000], 4), (200, 16, 8, 16, [1700, 200, 1000], 2),
+@pytest.mark.parametrize("sq,hq,hkv,page,lens", [
+    (100, 4, 1, 16, [4200, 100, 130]), (130, 3, 1, 32, [1800, 0, 131, 40]), (65, 16, 2, 128, [2900, 600]), (70, 8, 8, 8, [1700, 70, 1000]),
 ])
-def test_chunks_over_pages(sq, hq, hkv, page, lens, ctas, d):
+def test_chunks_over_pages(sq, hq, hkv, page, lens, d):
     dt = "bf16"
     kc, vc, table = H.make_paged_cache(lens, page, hkv, d, seed=sq)
     kc, vc, q = H.round_to(kc, dt), H.round_to(vc, dt), H.round_to(H.normal((len(lens), sq, hq, d), 4), dt)
@@ -73,7 +72,7 @@ def test_chunks_over_pages(sq, hq, hkv, page, lens, ctas, d):
         o = torch.full_like(dev[0], float("nan"))
         low.flash_attn_with_kvcache(*dev, o, tab, cl, len(lens), sq, hq, hkv, d, page, table.shape[1], 1.0 / math.sqrt(d))
         return o
-    o = _twice(call, want, f"{sq} over {lens}", f"cluster {ctas}")
+    o = _twice(call, want, f"{sq} over {lens}")
     for name, value in ((b"prefill_order", 2), (b"prefill_band", 1)):
         ffi.lib.flash_attn_set_option(name, value)
         try:
@@ -83,13 +82,10 @@ def test_chunks_over_pages(sq, hq, hkv, page, lens, ctas, d):
 
 
 @pytest.mark.parametrize("paged", [False, True])
-@pytest.mark.parametrize("hq,hkv,ql,total,form", [
-    (4, 2, [200, 17, 0, 129, 64], True, "cluster 4"), (32, 1, [40, 17, 0, 33, 8], True, "cluster 4"), (32, 1, [40, 17, 0, 33, 8], False, "cluster 4"),
-    (4, 2, [200, 17, 0, 129, 64], False, "few rows behind"),     # (some of its sequences may have few rows, for all that the host knows)
-])
-def test_packed(paged, hq, hkv, ql, total, form):
-    dt, d, page = "f16", 128, 16
-    kl = [1900, 17, 0, 2500, 300]
+@pytest.mark.parametrize("total", [False, True])
+def test_packed(paged, total):
+    dt, d, page, hq, hkv = "f16", 128, 16, 4, 2
+    ql, kl = [200, 17, 0, 129, 64], [1900, 17, 0, 2500, 300]
     cu_q, cu_k = (np.concatenate([[0], np.cumsum(x)]).astype(np.int32) for x in (ql, kl))
     q = H.round_to(H.normal((sum(ql), hq, d), 5), dt)
     if paged:
@@ -106,7 +102,7 @@ def test_packed(paged, hq, hkv, ql, total, form):
         low.flash_attn_varlen(*dev, o, cq, ck, len(ql), max(ql), max(kl), hq, hkv, d, 1.0 / math.sqrt(d), torch.from_numpy(table).cuda() if paged else None, page if paged else 1,
                               total_q=sum(ql) if total else None, total_k=sum(kl) if total and not paged else None)
         return o
-    _twice(call, want, "packed", form)
+    _twice(call, want, "packed")
 
 
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
@@ -121,7 +117,7 @@ def test_scores_that_are_not_finite(value):
         o, lse = torch.empty_like(q), torch.empty((b, hq, sq), device="cuda")
         low.flash_attn(q, k, v, o, b, sq, skv, hq, hkv, d, skv - sq, 1.0 / math.sqrt(d), None, None, lse)
         torch.cuda.synchronize()
-        assert ffi.last_path() == "prefill_tcgen05" and ffi.last_form() == "cluster 4" and ffi.device_status() == 0
+        assert ffi.last_path() == "prefill_tcgen05" and ffi.device_status() == 0
         return o, lse
     clean, clean_lse = call()
     at = skv - sq + 100
@@ -144,7 +140,6 @@ def test_a_wait_that_runs_out(tile, d):
     call = lambda: low.flash_attn(q, k, v, o, b, sq, skv, h, h, d, skv - sq, 1.0 / math.sqrt(d))
     call()
     torch.cuda.synchronize()
-    assert ffi.last_form() == "cluster 8"
     want = o.clone()
     try:
         ffi.set_option("prefill_wait_us", 1000)
