@@ -38,12 +38,22 @@ __host__ __device__ inline long long prefill_pairs(int group, long long q_len) {
     return ((long long)(group / pack) * ((q_len * pack + 127) / 128) + 1) / 2;
 }
 
+// Whether n clusters find room at the same time, with one CTA to an SM: as the SMs lie, 33 clusters of four and 15 of eight do on 148.
+inline bool clusters_fit(long long n, int ctas, int sms) { return (ctas == 8 ? 21 : ctas == 4 ? 9 : 4) * n <= 2LL * sms; }
+
 // CTAs that share the keys of a tile pair there: of `pairs` pairs in all over up to `tiles` K/V tiles (`exact`: over as many), `rows` rows per KV head and sequence (rule and times
 // where it is launched).
 inline int prefill_parts(long long pairs, long long tiles, bool exact, long long rows, int sms) {
     if (tiles <= (rows <= 16 && exact ? 7 : 12)) return 1;
-    if (21 * pairs <= 2 * sms && tiles >= (rows > 16 ? 32 : 16)) return 8;
-    return 9 * pairs <= 2 * sms ? 4 : 2 * pairs <= sms ? 2 : 1;
+    if (clusters_fit(pairs, 8, sms) && tiles >= (rows > 16 ? 32 : 16)) return 8;
+    return clusters_fit(pairs, 4, sms) ? 4 : clusters_fit(pairs, 2, sms) ? 2 : 1;
+}
+
+// CTAs that share the keys of a row block of the f32 kernel on the tensor cores: of `blocks` in all over `tiles` K/V tiles (tile_f32_tcgen05.cu).
+inline int f32_parts(long long blocks, long long tiles, int sms) {
+    int c = 1;
+    while (c < 8 && clusters_fit(blocks, 2 * c, sms) && tiles >= c * 2) c *= 2;
+    return c;
 }
 
 // ---- few-row calls (decode_splitk.cu) ----

@@ -629,10 +629,10 @@ int launch_for(const AttnParams& p, cudaStream_t stream) {
     const long long blocks = (rows + kM - 1) / kM * streams;
     const long long keys = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
     const long long tiles = (keys + kN - 1) / kN;
-    // Few blocks: the keys of each are shared out over a cluster of 2, 4 or 8 CTAs, as long as there are SMs for them and two tiles for each. us with
-    // one CTA to a block and so: 1 x 256, 8 heads of 64 15.5 and 9.2; 1 x 512, 8 of 32 19.2 and 9.6; 3 x 552, 8/2 heads of 64 (54 blocks, 9 tiles) 26.3 either way.
-    int c = 1;
-    while (c < 8 && blocks * c * 2 <= sm_count() && tiles >= c * 2) c *= 2;
+    // Few blocks: the keys of each are shared out over a cluster of 2, 4 or 8 CTAs, as long as all clusters find room at the same time, with a tile for each CTA. us with
+    // one CTA to a block and so: 1 x 256, 8 heads of 64 15.5 and 9.2; 1 x 512, 8 of 32 19.2 and 9.6; 3 x 552, 8/2 heads of 64 (54 blocks, 9 tiles) 26.3 either way. 36 blocks in clusters of four, some of which
+    // had to wait for a place, and of two: 1 x 280, 16/4 heads of 64 17.8 and 13.7, of 32 14.4 and 10.8.
+    const int c = f32_parts(blocks, tiles, sm_count());
     // The other kernel (tile_f32.cu) keeps what leaves this one's 128 rows empty with a CTA to a block (us there and here: 32 x 1 token over 600, 8 heads of 64 29 and 52; 64 x 4 over
     // 512 81 and 94; 1 x 4 over 4096, 32/8 heads, shared by 8 CTAs 123 and 23), and problems of up to three tiles that give it a CTA of 16 rows (32 at head size 128) for
     // about every SM, which have no time to win back this one's set-up (2 x 113, 8/2 heads of 64 7.9 and 9.4; 1 x 192, 8 of 64 10.4 and 11.3; 2 x 91, 16/4 of 128 14.0 and

@@ -20,6 +20,7 @@ def code(tmp_path_factory):
     lib.cut_span.restype = lib.cut_column_of.restype = ctypes.c_uint
     lib.pair_count.restype = ctypes.c_longlong
     lib.pair_count.argtypes = [ctypes.c_int, ctypes.c_longlong]
+    lib.f32_pair_parts.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
     lib.pair_parts.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
     return lib
 
@@ -178,3 +179,10 @@ def test_clusters_have_room(code):
                     for exact in (0, 1):
                         parts = code.pair_parts(pairs, tiles, exact, rows, sms)
                         assert parts in (1, 2, 4, 8) and (parts == 1 or parts * pairs <= sms and tiles >= parts and tiles > 7)
+
+
+def test_clusters_of_the_f32_kernel_have_room(code):
+    for blocks in range(1, 200):
+        for tiles in range(1, 70):
+            parts = code.f32_pair_parts(blocks, tiles, 148)
+            assert parts == 1 or tiles >= parts and blocks <= {2: 74, 4: 33, 8: 15}[parts]     # at the same time: as the SMs lie
