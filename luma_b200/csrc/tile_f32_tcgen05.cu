@@ -637,8 +637,12 @@ int launch_for(const AttnParams& p, cudaStream_t stream) {
     // 512 81 and 94; 1 x 4 over 4096, 32/8 heads, shared by 8 CTAs 123 and 23), and problems of up to three tiles that give it a CTA of 16 rows (32 at head size 128) for
     // about every SM, which have no time to win back this one's set-up (2 x 113, 8/2 heads of 64 7.9 and 9.4; 1 x 192, 8 of 64 10.4 and 11.3; 2 x 91, 16/4 of 128 14.0 and
     // 14.5; at head size 32 up to 2.2 for an SM: 4 x 128, 8 heads 6.4 and 7.9; 4 x 73, 16/4 6.7 and 7.8; 4 x 160, 8/2 8.7 and 9.2, 8/8 9.7 and 8.8; 3 x 160 7.7 and 10.0; 3 x 95, 16/4 6.4 and 7.8; 4 x 96, 2.6 of them, 9.3 and 8.0; but 4 x 130, 16/4 of 64, 3.5 CTAs for an SM, 17.4 and 11.5; 1 x 160, 8 of 128 19.9 and 18.7).
-    const long long small = (rows + (D == 128 ? 31 : 15)) / (D == 128 ? 32 : 16) * streams;
-    if ((rows <= 16 && c == 1) || (tiles <= 3 && 20 * small <= (D == 32 ? 44LL : 30LL) * sm_count() && (D < 128 || tiles <= 2))) return -1;
+    // Two tiles of head size 64 up to 1.65 for an SM (3 x 80, 16/4 9.3 and 9.8; with 1.7 of them 4 x 128, 8 heads the same; with 2 of them 3 x 97, 16/4 11.0 and 9.8), one tile up to as many rounds of two CTAs to an SM there as of one here
+    // (4 x 64, 16/4 of 64 7.2 and 8.3; 24 x 48, 8 of 64 12.6 and 14.0, of 32 8.3 and 10.8), and at head size 32 up to five tiles where it has a CTA for each SM at most (1 x 200, 8 heads 7.0 and 7.7; 1 x 256 7.8 and 8.0; 1 x 280, 8/2 8.8 and 9.3; but with 160 of its CTAs 1 x 320, 8 heads 10.4 and 9.3, with 200
+    // 1 x 200, 16/4 9.0 and 8.0).
+    const long long small = (rows + (D == 128 ? 31 : 15)) / (D == 128 ? 32 : 16) * streams, sms = sm_count();
+    const bool one_round = 20 * small <= (D == 32 ? 44 : D == 64 && tiles == 2 ? 33 : 30) * sms;
+    if ((rows <= 16 && c == 1) || (tiles <= (D < 128 ? 3 : 2) && one_round) || (D < 128 && tiles == 1 && (small + 2 * sms - 1) / (2 * sms) <= (blocks + sms - 1) / sms) || (D == 32 && tiles <= 5 && small <= sms)) return -1;
     const bool plain = p.mask == nullptr && !p.paged;
     if (c > 1) return plain ? launch_one<D, true, true>(p, c, stream) : launch_one<D, true, false>(p, c, stream);
     return plain ? launch_one<D, false, true>(p, 1, stream) : launch_one<D, false, false>(p, 1, stream);

@@ -17,10 +17,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("b,sq,skv,hq,hkv,d,sp,form", [
-    (1, 256, 256, 8, 8, 64, 0, "tcgen05 cluster 4"), (2, 257, 257, 4, 4, 32, 0, "tcgen05 cluster 4"), (1, 193, 193, 2, 2, 128, 0, "tcgen05 cluster 4"),
+    (1, 256, 256, 8, 8, 64, 0, "tcgen05 cluster 4"), (2, 257, 257, 4, 4, 32, 0, "mma"), (1, 193, 193, 2, 2, 128, 0, "tcgen05 cluster 4"),
     (1, 1000, 1000, 8, 8, 128, 0, "tcgen05 cluster 2"), (2, 500, 500, 8, 4, 64, 0, "tcgen05 cluster 2"), (2, 400, 400, 9, 9, 32, 0, "tcgen05 cluster 2"),
     (1, 5, 1025, 2, 2, 64, 1020, "tcgen05 cluster 8"), (1, 1, 4000, 4, 1, 128, 3999, "tcgen05 cluster 8"), (1, 3, 449, 1, 1, 32, 446, "tcgen05 cluster 8"),
     (1, 43, 300, 9, 3, 64, 257, "tcgen05 cluster 4"), (1, 64, 257, 4, 2, 64, 193, "tcgen05 cluster 4"), (1, 300, 200, 4, 2, 64, 0, "tcgen05 cluster 4"), (1, 200, 300, 6, 2, 128, 0, "tcgen05 cluster 4"),
+    (1, 280, 280, 16, 4, 64, 0, "tcgen05 cluster 2"), (1, 320, 320, 8, 8, 32, 0, "tcgen05 cluster 4"), (1, 256, 256, 8, 2, 32, 0, "mma"), (1, 200, 200, 16, 4, 32, 0, "tcgen05 cluster 4"),
+    (4, 64, 64, 16, 4, 64, 0, "mma"), (3, 80, 80, 16, 4, 64, 0, "mma"), (24, 33, 33, 8, 8, 64, 0, "mma"), (5, 80, 80, 16, 4, 64, 0, "tcgen05 cluster 2"), (24, 64, 64, 8, 8, 64, 0, "tcgen05"),
     (3, 160, 160, 8, 8, 32, 0, "mma"), (4, 96, 96, 16, 4, 32, 0, "tcgen05 cluster 2"), (4, 128, 128, 8, 8, 32, 0, "mma"),   # both sides of the line
     (4, 400, 400, 16, 8, 64, 0, "tcgen05"), (2, 513, 513, 24, 24, 32, 0, "tcgen05"), (3, 330, 330, 12, 12, 128, 0, "tcgen05"),
 ])
@@ -31,7 +33,7 @@ def test_f32(b, sq, skv, hq, hkv, d, sp, form):
 
 @pytest.mark.parametrize("d", [32, 64, 128])
 def test_f32_with_a_mask_and_over_pages(d):
-    for b, form in ((1, "tcgen05 cluster 4"), (30, "tcgen05")):
+    for b, form in ((1, "mma" if d == 32 else "tcgen05 cluster 4"), (2, "tcgen05 cluster 2"), (30, "tcgen05")):
         f32.test_padding_mask(b, d)
         assert ffi.last_form() == form
     for bs in (0, 5, 16):
