@@ -1074,6 +1074,9 @@ static double prefill_few_rows_us(const AttnParams& p, long long rows) {
 // 8 heads of 64 12.9 and 10.6; 16 x 4 over 8192, 32/8 96 and 92. The estimate has to say half for the prefill kernel: it does not know the lengths, and equal shares suit unequal ones.
 // Two groups of calls stay with one kernel whatever the estimates say, because programs and tests know them there: up to 64 pairs, counted by heads, over up to 12 tiles with the prefill
 // kernel (4 x 1 over 544, 32/8 heads of 64 9.6 and 6.0), and up to 4 sequences by the estimates of a tile for every head (1 x 64 over 8192, 32 heads 33 and 68).
+// Of the calls of one wave of pairs, counted by heads, over up to 12 tiles, four row blocks and, without GQA, short ranges stay with the prefill kernel too, where the estimates are not fine enough: 1008 shapes of 3-37 sequences x 1-16
+// tokens over 66-1500 keys take 0.79 of what the prefill kernel takes for all, but of 635 that came here these were up to a quarter slower (there and here: 9 x 16 over 1200, 32/8 heads of 64 20.3 and 25.3; 3 x 8 over 500,
+// 32 of 64 9.6 and 11.9; 12 x 8 over 200, 8 of 128 7.9 and 9.1) and the others at most 12 % (18 x 16 over 1500, 8 of 128 23.7 and 26.5).
 int launch_few_rows(const AttnParams& p, bool prefill_takes_it, cudaStream_t stream) {
     if (p.n_out > 0 || !rows_kernel_takes(p)) return -1;
     const long long rows = (long long)p.q_seq_len * (p.q_heads / p.kv_heads);
@@ -1081,6 +1084,7 @@ int launch_few_rows(const AttnParams& p, bool prefill_takes_it, cudaStream_t str
     const double pairs = (double)tile_pairs(p, p.q_seq_len) * p.num_seqs;
     if (longest_keys(p) <= 12 * 128 && pairs <= 64) return -1;
     if (prefill_takes_it) {
+        if (longest_keys(p) <= 12 * 128 && pairs <= sm_count() && (rows > 3 * kRows || (p.q_heads == p.kv_heads && longest_keys(p) <= (p.num_seqs > 4 ? 3 : 4) * 128))) return -1;
         const double here = rows_us(p, p.num_seqs, rows);
         if (p.num_seqs > 4 ? prefill_few_rows_us(p, rows) < 0.575 * here : here >= prefill_us(p, pairs)) return -1;
     }

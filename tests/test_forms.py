@@ -1,11 +1,12 @@
 """Which form of a kernel ran (flash_attn_last_form), at the sizes of the tests that are there for that form and at more where those leave one out: the f32 kernels with warp-wide products and on
-the tensor cores, tile pairs with a CTA and with a cluster, few rows ahead of the prompts of a packed batch and behind them. Each call is compared with the f64 oracle as well."""
+the tensor cores, tile pairs with a CTA and with a cluster, few rows ahead of the prompts of a packed batch and behind them, which kernel takes few rows. Each call is compared with the f64 oracle as well."""
 import math
 
 import numpy as np
 import pytest
 import torch
 
+import tests.test_few_rows_routes as routes
 import tests.test_mixed_side_by_side as mixed
 import tests.test_shared_keys as shared
 import tests.test_tile_f32_tcgen05 as f32
@@ -94,3 +95,11 @@ def test_shared_keys_of_packed_buffers(paged, total):
 def test_mixed_batches(decoding, prompts, longest, hq, hkv, d, dt, several, form):
     mixed.test_rows_of_both_kernels(decoding, prompts, longest, hq, hkv, d, dt, several)
     assert ffi.last_form() == f"few rows {form}"
+
+
+@pytest.mark.parametrize("b,s,kv,hq,hkv,d,path", [
+    (9, 16, 1200, 32, 8, 64, "prefill_tcgen05"), (9, 12, 1200, 32, 8, 64, "decode_splitk"), (3, 8, 500, 32, 32, 64, "prefill_tcgen05"), (3, 8, 513, 32, 32, 64, "decode_splitk"),
+    (12, 8, 300, 8, 8, 64, "prefill_tcgen05"), (12, 8, 385, 8, 8, 64, "decode_splitk"),
+])
+def test_few_rows_of_one_wave(b, s, kv, hq, hkv, d, path):
+    routes.test_sides_of_the_line(b, s, kv, hq, hkv, d, path)
