@@ -1780,17 +1780,24 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     while ((1 << a.pack_log2) < pack) ++a.pack_log2;
     const int pairs = (packs * row_blocks(p.q_seq_len, a.pack_log2) + 1) / 2;
     const size_t smem = sizeof(SharedStorage<D>) + 1024;
+    const MixedFewRows few = prepare_mixed_few_rows(p, stream);   // its workspace is this call's until both kernels are launched
+    a.skip_rows = few.max_rows;
+    const long long kv_rows = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;   // upper bound per sequence
+    const long long all = (long long)p.num_seqs * p.kv_heads * pairs;
+    // Where the tile pairs leave SMs without one, a cluster of 2, 4 or 8 CTAs shares the keys of each, as many as find room at the same time (one CTA to an SM; 33 clusters of four and 15
+    // of eight, as the SMs lie), for a cluster of eight with four tiles for each. It takes 2 us (a few rows) to 7 (full tiles of 128 columns and eight CTAs) more, a tile 1.5. us from a graph,
+    // alone and shared by 2, 4, 8: 1 x 512 tokens over 8192, 32/8 heads 108, 70; 1 x 64 over 8192 105, 64, 41, 31; 5 x 84 over 339-5439, 8 heads of 64 57, 36; 1 x 2048, 8 heads 28.7, 23.6; 2 x 64 over
+    // 30000, 32/8 heads of 64 354, 192, 103, 115 (16 clusters of eight, in two rounds); 8 x 1 token over 1022, 8/2 heads 15.0, 12.6, 9.8; 4 x 1 over 544, 32/8 heads of 64 10.0, 9.8.
+    // More than a few rows over at most 12 tiles stay alone: their results have the bits of the same rows in a call that fills the device. So do a few rows where there may be no more than 12 (over
+    // pages, whose lengths the host does not know: 2 x 6 over 361 with room for 1024, 32 heads 13.0 alone, 14.8 as a cluster that finds too few to share) or are no more than 7 tiles.
+    const int parts = p.n_out > 0 || a.skip_rows > 0 ? 1 : prefill_parts(all, (kv_rows + kBlockN - 1) / kBlockN, p.mode == MODE_BATCH, (long long)p.q_seq_len * group, sm_count());
+    a.parts = parts;
     // Band width: the pairs of a band start together, so their work must be about equal or the
     // heaviest-first order is lost (at S = 2048 without GQA, bands of 2 cost 13 %). A band of w
     // pairs spans 2w / group row blocks, i.e. that many K/V tiles of difference between its lightest
-    // and heaviest pair: keep that within an eighth of the longest K/V range, at most 8 pairs (16 measured no better).
-    int band = 1;
-    {
-        const int kv_rows = p.mode == MODE_KVCACHE ? p.max_blocks * p.block_size : p.kv_seq_len;   // upper bound per sequence
-        const int kv_tiles = std::max(1, (kv_rows + kBlockN - 1) / kBlockN);
-        while (band < 8 && band * 2 <= pairs && (long long)(band * 2) * 2 * 8 <= (long long)kv_tiles * group) band *= 2;
-        if (get_option_prefill_band() > 0) band = std::min(get_option_prefill_band(), pairs);
-    }
+    // and heaviest pair: keep that within an eighth of the longest K/V range, at most 8 pairs (16 measured no better). Clusters all run at the same time, and a band that the pairs do not fill would be clusters without
+    // any, for which there may be no room (3 x 65 tokens over 640, 64/8 heads, 72 clusters of two for the 3 pairs of each KV head: with bands of two another 24 17.8 us, a CTA to a pair 14.6).
+    const int band = get_option_prefill_band() > 0 ? std::min(get_option_prefill_band(), pairs) : prefill_band(pairs, std::max(1LL, (kv_rows + kBlockN - 1) / kBlockN), group, parts);
     a.band = band;
     a.by_band = FastDiv(band);
     a.by_kv_heads = FastDiv(p.kv_heads);
@@ -1820,7 +1827,7 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
         const long long kv_bytes_per_stream = 2LL * (p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len) * D * 2;
         const long long budget = 16LL << 20;
         if (get_option_prefill_groups() > 0) groups = get_option_prefill_groups();
-        else if (band == 1 && pairs > 1 && p.n_out <= 1 && streams * kv_bytes_per_stream > 2 * budget)
+        else if (parts == 1 && band == 1 && pairs > 1 && p.n_out <= 1 && streams * kv_bytes_per_stream > 2 * budget)
             groups = (int)std::min<long long>(streams, (streams * kv_bytes_per_stream + budget - 1) / budget);
         else if (band > 1 && p.n_out <= 1 && (p.mode == MODE_BATCH || p.mode == MODE_VARLEN) && p.num_seqs >= 2 &&
                  streams * kv_bytes_per_stream > (48LL << 20) * (p.mode == MODE_VARLEN ? 2 : 1)) {
@@ -1840,18 +1847,14 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     a.streams_z = streams_per_group;
     dim3 grid(streams_per_group * band, (pairs + band - 1) / band, groups);
     a.pairs = pairs;
-    const MixedFewRows few = prepare_mixed_few_rows(p, stream);   // its workspace is this call's until both kernels are launched
-    a.skip_rows = few.max_rows;
     // Ordered: chunks of prompts, at most half as long as the context may be. Whole prompts keep grid order, which is heaviest
     // first for them already. Finding its pair costs a CTA 1 to 2 us; what it wins is one late long pair, about a fifth of the longest pair's
     // 1.5 to 1.7 us per K/V tile, and nothing where all pairs start at once. So: more than one wave of pairs, and at least five tiles in the longest for
     // each. 4 chunks of 300 over 2048-8192 keys (the longest last), 32/8 heads (1.3 waves) 138-152 us in grid order, 110 ordered; 16 chunks of 300 over
     // 512-2048, 32/32 heads (7 waves) 161-172 and 166-186; 4 chunks of 64 over 128-512 (less than a wave) 17-19 and 19-21.
-    const long long kv_rows = p.mode == MODE_KVCACHE ? (long long)p.max_blocks * p.block_size : p.kv_seq_len;
     const PackedMix mix = packed_mix(p);
     const long long few_pairs = (packs + 1) / 2;   // of a sequence whose rows fit one block
     const double waves = (double)(mix.prompts * pairs + (a.skip_rows > 0 ? 0 : mix.few * few_pairs)) * p.kv_heads / sm_count();
-    const long long all = (long long)p.num_seqs * p.kv_heads * pairs;
     long long ctas = all;
     if (p.total_q > 0)   // a sequence of n tokens has (packs * ceil(n * pack / 128) + 1) / 2 pairs
         ctas = std::min(ctas, p.kv_heads * ((packs * (((long long)p.total_q * pack + 127LL * p.num_seqs) / 128) + p.num_seqs) / 2));
@@ -1872,14 +1875,6 @@ int launch_variant(const AttnParams& p, cudaStream_t stream) {
     // a grid in order has empty CTAs, which are cheaper to take over (serve steps of 4 chunks with 32 tokens 226 and 228, 6 with 40 310 and 318), and so are short pairs at head size
     // 64 (8 x 200 over 512-4096, 32/8 heads 68.5 and 69.6). Contiguous K/V at head size 64: no difference (1 x 449, 64/8 heads of 32 11.6 either way; 1 x 2048, 8/8 heads 26.8 and
     // 27.3), and none is built.
-    // Where the tile pairs leave SMs without one, a cluster of 2, 4 or 8 CTAs shares the keys of each, as many as find room at the same time (one CTA to an SM; 33 clusters of four and 15
-    // of eight, as the SMs lie), for a cluster of eight with four tiles for each. It takes 2 us (a few rows) to 7 (full tiles of 128 columns and eight CTAs) more, a tile 1.5. us from a graph,
-    // alone and shared by 2, 4, 8: 1 x 512 tokens over 8192, 32/8 heads 108, 70; 1 x 64 over 8192 105, 64, 41, 31; 5 x 84 over 339-5439, 8 heads of 64 57, 36; 1 x 2048, 8 heads 28.7, 23.6; 2 x 64 over
-    // 30000, 32/8 heads of 64 354, 192, 103, 115 (16 clusters of eight, in two rounds); 8 x 1 token over 1022, 8/2 heads 15.0, 12.6, 9.8; 4 x 1 over 544, 32/8 heads of 64 10.0, 9.8.
-    // More than a few rows over at most 12 tiles stay alone: their results have the bits of the same rows in a call that fills the device. So do a few rows where there may be no more than 12 (over
-    // pages, whose lengths the host does not know: 2 x 6 over 361 with room for 1024, 32 heads 13.0 alone, 14.8 as a cluster that finds too few to share) or are no more than 7 tiles.
-    const int parts = p.n_out > 0 || a.skip_rows > 0 ? 1 : prefill_parts(all, (kv_rows + kBlockN - 1) / kBlockN, p.mode == MODE_BATCH, (long long)p.q_seq_len * group, sm_count());
-    a.parts = parts;
     if (parts > 1) {
         const auto kernel = prefill_tcgen05_kernel<T, D, kMask, kPaged, true, true>;
         cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

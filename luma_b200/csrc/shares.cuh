@@ -49,6 +49,13 @@ inline int prefill_parts(long long pairs, long long tiles, bool exact, long long
     return clusters_fit(pairs, 4, sms) ? 4 : clusters_fit(pairs, 2, sms) ? 2 : 1;
 }
 
+// Tile pairs of a stream (sequence, KV head) that sit next to each other in the grid there.
+inline int prefill_band(int pairs, long long kv_tiles, int group, int parts) {
+    int band = 1;
+    while (parts == 1 && band < 8 && band * 2 <= pairs && (long long)(band * 2) * 2 * 8 <= kv_tiles * group) band *= 2;
+    return band;
+}
+
 // CTAs that share the keys of a row block of the f32 kernel on the tensor cores: of `blocks` in all over `tiles` K/V tiles (tile_f32_tcgen05.cu).
 inline int f32_parts(long long blocks, long long tiles, int sms) {
     int c = 1;

@@ -52,4 +52,5 @@ void pair_share(int n0, int n1, int kv_len, int pos_off, int parts, int rank, in
 }
 int pair_parts(long long pairs, long long tiles, int exact, long long rows, int sms) { return prefill_parts(pairs, tiles, exact != 0, rows, sms); }
 int f32_pair_parts(long long blocks, long long tiles, int sms) { return f32_parts(blocks, tiles, sms); }
+int pair_band(int pairs, long long tiles, int group, int parts) { return prefill_band(pairs, tiles, group, parts); }
 }

@@ -21,6 +21,7 @@ def code(tmp_path_factory):
     lib.pair_count.restype = ctypes.c_longlong
     lib.pair_count.argtypes = [ctypes.c_int, ctypes.c_longlong]
     lib.f32_pair_parts.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
+    lib.pair_band.argtypes = [ctypes.c_int, ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
     lib.pair_parts.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
     return lib
 
@@ -186,3 +187,14 @@ def test_clusters_of_the_f32_kernel_have_room(code):
         for tiles in range(1, 70):
             parts = code.f32_pair_parts(blocks, tiles, 148)
             assert parts == 1 or tiles >= parts and blocks <= {2: 74, 4: 33, 8: 15}[parts]     # at the same time: as the SMs lie
+
+
+def test_a_grid_of_clusters_has_no_more_than_its_pairs(code):
+    for group in GROUPS:
+        for pairs in range(1, 75):
+            for tiles in (8, 13, 16, 32, 64, 256):
+                for streams in (1, 2, 3, 8, 24, 37):
+                    parts = code.pair_parts(pairs * streams, tiles, 0, 4096, 148)
+                    band = code.pair_band(pairs, tiles, group, parts)
+                    assert 1 <= band <= min(8, pairs)
+                    assert parts == 1 or -(-pairs // band) * band * streams * parts <= 148
