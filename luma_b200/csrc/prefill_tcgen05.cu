@@ -901,7 +901,7 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // (the same for the whole warp, which the compiler sees only so)
     const int lane = threadIdx.x & 31;
     // A few-row kernel launched behind this one may start once every tile pair here is taken: it fills the SMs that run out of them.
-    if (a.skip_rows > 0 && !a.behind_few) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    if (a.skip_rows > 0 && (kOnePair || !a.behind_few)) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     // Packed buffers end at row cu_seqlens[num_seqs]; where the tensor map does not end with the buffer, a tile that reaches past that row is not asked
     // of the copy engine but fetched by the producer warp (see edge_tile_copy). A map that does gives zeros there like any other.
     const bool packed = a.mode == MODE_VARLEN;
@@ -1240,6 +1240,9 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         __syncwarp();
         asm volatile("barrier.cta.arrive 1, 96;\n" ::: "memory");    // the producers
         asm volatile("barrier.cta.arrive 2, 320;\n" ::: "memory");   // issuer and softmax warps, which wait for tensor memory as well
+        // This grid's completion stands for the few-row kernel's that was launched ahead of it (whose CTAs have all started when this one begins), so its CTAs end behind that. In this warp, which has nothing else to do: at the
+        // end of every CTA the look whether there is one took 0.1 us of each call. Calls of one pair to a CTA never have one (see launch_variant).
+        if (!kOnePair && a.behind_few) asm volatile("griddepcontrol.wait;\n" ::: "memory");
     }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 208;\n");
@@ -1568,7 +1571,6 @@ prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 
     tc_fence_before();
     __syncthreads();
-    if (a.behind_few && threadIdx.x == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");   // (this grid's completion stands for both)
     if (warp == kMmaWarp) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(sm.tmem_base) : "memory");
