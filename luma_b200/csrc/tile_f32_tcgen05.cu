@@ -10,9 +10,10 @@
 // tensor memory; a seventeenth warp issues the products. The scores of the next tile are computed beside this tile's softmax (at head size 128 behind its weights' product: tensor
 // memory has no room for both), a tile's weights times V beside the next tile's softmax. Where blocks are few, a cluster of CTAs shares the keys of each and merges through
 // distributed shared memory. Sums start from zero for every tile and are added to the running output in f32, since the tensor cores truncate when they accumulate: relative error
-// against 64 bits over 64-1500 keys, N(0,1), 1.0-1.8e-7, log-sum-exp 1.9-3.1e-7 rms; the warp-wide products 1.1-1.8e-7 and 2.1-3.3e-7.
-// What bounds it: issue slots of the workers (700 instructions a warp and step, half of them the splitting), 4400 clocks a tile; the products take 1600. us a call, warp-wide products -> this:
-// 1 x 256, 8 heads of 64 12.0 -> 9.2; 2 x 979, 8 of 64 99 -> 38.7; 3 x 552, 8/2 of 64 51 -> 24.5; 3 x 301, 16/4 of 32 25.8 -> 12.1; 1 x 1024, 16/4 of 128 162 -> 104.
+// against 64 bits, causal, N(0,1), 256-1500 tokens, norm by norm over all rows: 1.0-1.8e-7, log-sum-exp 2.3-3.2e-7 rms; the warp-wide products 1.1-1.9e-7 and 2.5-3.3e-7.
+// What bounds it: issue slots of the workers (650 instructions a warp and step, half of them the splitting), 4000 clocks a tile; the products take 1600. 17 warps leave 96 registers a thread: 108-372 bytes of spill stores
+// at head size 64, 376-924 at 128 (-Xptxas -v). us a call, warp-wide products -> this: 1 x 256, 8 heads of 64 11.9 -> 9.4; 2 x 979, 8 of 64 97 -> 36.5; 3 x 552, 8/2 of 64 50.5 -> 23.7; 3 x 301, 16/4 of 32
+// 26.0 -> 12.0; 1 x 1024, 16/4 of 128 158 -> 100; 4 x 2048, 8 of 128 875 -> 507.
 #include <atomic>
 
 #include "common.cuh"
